@@ -135,6 +135,13 @@ xlb_status xlb_rel_is_canonical(const xlb_rel* rel, int* canonical);
  * Copies min(rows, cap_rows) rows into the host arrays and reports the logical row count. */
 xlb_status xlb_rel_to_host(xlb_ctx* ctx, const xlb_rel* rel, void* const* cols, uint64_t cap_rows,
                            uint64_t* rows);
+/* Page-locked host memory for results, from a bounded pool that the process shares: copies of
+ * xlb_rel_to_host into it run at the bus's rate, where fresh pageable memory takes a page fault per
+ * page (any other memory works as well).  `*out` is aligned to a huge page; hand it back with
+ * xlb_host_free.  XLB_ERR_RESOURCE_EXHAUSTED when the pool's bound is reached: use memory of your
+ * own then.  Both may be called from any thread; they need no context. */
+xlb_status xlb_host_alloc(uint64_t bytes, void** out);
+void xlb_host_free(void* block);
 /* clone_buffer (relational.rs:6113). */
 xlb_status xlb_rel_clone(xlb_ctx* ctx, const xlb_rel* rel, xlb_rel** out);
 void xlb_rel_free(xlb_rel* rel);

@@ -164,6 +164,8 @@ pub mod ffi {
         pub fn xlb_rel_schema(rel: *const xlb_rel, schema: *mut xlb_schema) -> c_int;
         pub fn xlb_rel_is_canonical(rel: *const xlb_rel, canonical: *mut c_int) -> c_int;
         pub fn xlb_rel_to_host(ctx: *mut xlb_ctx, rel: *const xlb_rel, cols: *const *mut c_void, cap_rows: u64, rows: *mut u64) -> c_int;
+        pub fn xlb_host_alloc(bytes: u64, out: *mut *mut c_void) -> c_int;
+        pub fn xlb_host_free(block: *mut c_void);
         pub fn xlb_rel_clone(ctx: *mut xlb_ctx, rel: *const xlb_rel, out: *mut *mut xlb_rel) -> c_int;
         pub fn xlb_rel_free(rel: *mut xlb_rel);
         pub fn xlb_rel_checksum(ctx: *mut xlb_ctx, rel: *const xlb_rel, digest: *mut u64) -> c_int;

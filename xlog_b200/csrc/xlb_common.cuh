@@ -354,6 +354,8 @@ struct xlb_ctx {
     unsigned long long* h_scalar = nullptr;  // 64 words
     unsigned long long* h_scalar_dev = nullptr;  // the same words as the device sees them (mapped): a kernel can leave counts there
     unsigned long long publish_seq = 0;          // number of the last set of counts a kernel was asked to leave there
+    char* h_stage = nullptr;      // page-locked staging of small results (made on first use) ...
+    char* h_stage_dev = nullptr;  // ... as the device sees it
     DevStatus* d_status = nullptr;
     int sm_count = 148;
     // executor state

@@ -1,0 +1,6 @@
+// Page-locked host memory for results (see xlb_host.cu).
+#pragma once
+#include <cstdint>
+
+void host_pool_context_opened();
+void host_pool_context_closed();

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "xlb_host.h"
 #include "xlb_kernels.cuh"
 #include "xlb_ops.h"
 
@@ -39,6 +40,32 @@ __global__ void gather_pair_k(const T* __restrict__ in, const uint64_t* __restri
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t p = pairs[i];
         out[i] = in[half == 0 ? (p >> 32) : (p & 0xFFFFFFFFull)];
+    }
+}
+
+// Columns written into page-locked host memory (16-byte aligned on both sides).
+constexpr uint64_t STAGE_BYTES = 256ull << 10;
+struct StageCols {
+    const void* from[XLB_MAX_ARITY];
+    void* to[XLB_MAX_ARITY];
+    uint64_t bytes[XLB_MAX_ARITY];
+    int n;
+};
+__global__ void cols_stage_k(StageCols sc) {
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (int c = 0; c < sc.n; ++c) {
+        const uint64_t words = sc.bytes[c] / 4;
+        for (uint64_t i = first; i < words; i += step) ((uint32_t*)sc.to[c])[i] = ((const uint32_t*)sc.from[c])[i];
+        if (first < (sc.bytes[c] & 3)) ((uint8_t*)sc.to[c])[words * 4 + first] = ((const uint8_t*)sc.from[c])[words * 4 + first];
+    }
+}
+__global__ void unpack_stage_k(const uint64_t* __restrict__ in, uint64_t n, uint32_t* c0, uint32_t* c1) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t k = in[i];
+        if (c1) {
+            c0[i] = (uint32_t)(k >> 32);
+            c1[i] = (uint32_t)k;
+        } else c0[i] = (uint32_t)k;
     }
 }
 
@@ -1086,6 +1113,7 @@ extern "C" xlb_status xlb_ctx_create(const xlb_config* cfg, xlb_ctx** out) {
         cudaDeviceProp prop;
         CUDA_OK(cudaGetDeviceProperties(&prop, dev));
         c->sm_count = prop.multiProcessorCount;
+        host_pool_context_opened();
         *out = c;
     } catch (const XlbError& e) {
         g_create_error = e.msg;
@@ -1102,7 +1130,9 @@ extern "C" void xlb_ctx_destroy(xlb_ctx* c) {
     cudaSetDevice(c->device);
     xlb_exec_teardown(c);
     cudaStreamSynchronize(c->stream);
+    host_pool_context_closed();
     if (c->h_scalar) cudaFreeHost(c->h_scalar);
+    if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->d_status) cudaFree(c->d_status);
     c->arena.destroy();
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1195,15 +1225,46 @@ extern "C" xlb_status xlb_rel_to_host(xlb_ctx* c, const xlb_rel* r, void* const*
     if (!c || !r) return XLB_ERR_INVALID;
     API_BEGIN(c)
     uint64_t n = std::min(r->rows, cap_rows);
-    if (n && r->schema.arity) {
+    const uint32_t arity = r->schema.arity;
+    uint64_t offset[XLB_MAX_ARITY + 1] = {0};
+    for (uint32_t i = 0; i < arity; ++i) offset[i + 1] = offset[i] + (n * type_width(r->schema.types[i]) + 15) / 16 * 16;
+    if (n && arity) {
         if (!cols) xlb_fail(XLB_ERR_INVALID, "column pointers missing");
-        ops_rel_columns(c, r);
-        for (uint32_t i = 0; i < r->schema.arity; ++i) {
+        for (uint32_t i = 0; i < arity; ++i)
             if (!cols[i]) xlb_fail(XLB_ERR_INVALID, "column %u pointer is null", i);
-            CUDA_OK(cudaMemcpyAsync(cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost, c->stream));
-        }
     }
-    CUDA_OK(cudaStreamSynchronize(c->stream));
+    if (n && arity && offset[arity] <= STAGE_BYTES) {
+        // A small result: one kernel writes all columns into page-locked staging memory across the
+        // bus (a copy per column cost 12 us each), the host copies them out of it.
+        if (!c->h_stage) {
+            CUDA_OK(cudaHostAlloc((void**)&c->h_stage, STAGE_BYTES, cudaHostAllocMapped));
+            CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_stage_dev, c->h_stage, 0));
+        }
+        const unsigned grid = (unsigned)std::min<uint64_t>((offset[arity] / 4 + BLOCK - 1) / BLOCK, (uint64_t)c->sm_count);
+        prof_begin(c, "to_host", offset[arity]);
+        if (!r->cols[0]) {
+            unpack_stage_k<<<grid, BLOCK, 0, c->stream>>>(r->packed->as<uint64_t>(), n, (uint32_t*)c->h_stage_dev, arity == 2 ? (uint32_t*)(c->h_stage_dev + offset[1]) : nullptr);
+        } else {
+            StageCols sc{};
+            sc.n = (int)arity;
+            for (uint32_t i = 0; i < arity; ++i) {
+                sc.from[i] = r->cols[i]->p;
+                sc.bytes[i] = n * type_width(r->schema.types[i]);
+                sc.to[i] = c->h_stage_dev + offset[i];
+            }
+            cols_stage_k<<<grid, BLOCK, 0, c->stream>>>(sc);
+        }
+        check_launch(c, "to_host");
+        stream_wait(c);
+        for (uint32_t i = 0; i < arity; ++i) memcpy(cols[i], c->h_stage + offset[i], n * type_width(r->schema.types[i]));
+    } else if (n && arity) {
+        ops_rel_columns(c, r);
+        for (uint32_t i = 0; i < arity; ++i)
+            CUDA_OK(cudaMemcpyAsync(cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost, c->stream));
+        CUDA_OK(cudaStreamSynchronize(c->stream));
+    } else {
+        CUDA_OK(cudaStreamSynchronize(c->stream));
+    }
     if (rows) *rows = r->rows;
     API_END()
 }

@@ -29,6 +29,8 @@ PROTOTYPES = {
     "xlb_rel_schema": (C.c_int, [P, C.POINTER(A.Schema)]),
     "xlb_rel_is_canonical": (C.c_int, [P, C.POINTER(C.c_int)]),
     "xlb_rel_to_host": (C.c_int, [P, P, C.POINTER(P), C.c_uint64, C.POINTER(C.c_uint64)]),
+    "xlb_host_alloc": (C.c_int, [C.c_uint64, C.POINTER(P)]),
+    "xlb_host_free": (None, [P]),
     "xlb_rel_clone": (C.c_int, [P, P, C.POINTER(P)]),
     "xlb_rel_free": (None, [P]),
     "xlb_rel_checksum": (C.c_int, [P, P, C.POINTER(C.c_uint64)]),
