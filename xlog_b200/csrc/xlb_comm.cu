@@ -191,11 +191,11 @@ void comm_allgather_words(xlb_ctx* c, const uint64_t* mine, uint32_t k, uint64_t
     unsigned long long* dev = cm->counts_dev->as<unsigned long long>();
     unsigned long long* send = cm->h_stage + (size_t)W * STAGE_ROW;
     for (uint32_t i = 0; i < k; ++i) send[i] = mine[i];
-    CUDA_OK(cudaMemcpyAsync(dev + (size_t)c->comm_rank * k, send, (size_t)k * 8, cudaMemcpyHostToDevice, c->stream));
+    CUDA_OK(copy_async(c, dev + (size_t)c->comm_rank * k, send, (size_t)k * 8, cudaMemcpyHostToDevice));
     const double tr0 = c->trace_on ? trace_now() : 0;
     NCCL_OK(api().AllGather(dev + (size_t)c->comm_rank * k, dev, k, ncclUint64, cm->comm, c->stream));
     trace_note(c, "ncclAllGather (enqueue)", tr0);
-    CUDA_OK(cudaMemcpyAsync(cm->h_stage, dev, (size_t)W * k * 8, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_OK(copy_async(c, cm->h_stage, dev, (size_t)W * k * 8, cudaMemcpyDeviceToHost));
     comm_wait(c);
     for (size_t i = 0; i < (size_t)W * k; ++i) all[i] = cm->h_stage[i];
 }
@@ -246,7 +246,7 @@ Keys comm_allgather_keys(xlb_ctx* c, const Keys& in) {
     for (uint32_t r = 0; r < W; ++r) {
         const uint64_t n = all[2 * r];
         if (r == c->comm_rank) {
-            if (n) CUDA_OK(cudaMemcpyAsync(out.buf->as<uint64_t>() + at, in.ptr(), n * 8, cudaMemcpyDeviceToDevice, c->stream));
+            if (n) CUDA_OK(copy_async(c, out.buf->as<uint64_t>() + at, in.ptr(), n * 8, cudaMemcpyDeviceToDevice));
         } else {
             if (in.n) NCCL_OK(api().Send(in.ptr(), in.n, ncclUint64, (int)r, cm->comm, c->stream));
             if (n) NCCL_OK(api().Recv(out.buf->as<uint64_t>() + at, n, ncclUint64, (int)r, cm->comm, c->stream));
@@ -275,11 +275,11 @@ Keys comm_repartition(xlb_ctx* c, const Keys& in, int keysel, bool sorted_unique
     unsigned long long* send_tail = cm->h_stage + (size_t)W * STAGE_ROW;
     send_tail[0] = in.n ? in.bound : 0;
     send_tail[1] = in.n;
-    CUDA_OK(cudaMemcpyAsync(mine + W, send_tail, 16, cudaMemcpyHostToDevice, c->stream));
+    CUDA_OK(copy_async(c, mine + W, send_tail, 16, cudaMemcpyHostToDevice));
     const double tr0 = c->trace_on ? trace_now() : 0;
     NCCL_OK(api().AllGather(mine, dev, RW, ncclUint64, cm->comm, c->stream));
     trace_note(c, "ncclAllGather (enqueue)", tr0);
-    CUDA_OK(cudaMemcpyAsync(cm->h_stage, dev, (size_t)W * RW * 8, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_OK(copy_async(c, cm->h_stage, dev, (size_t)W * RW * 8, cudaMemcpyDeviceToHost));
     comm_wait(c);
     const unsigned long long* all = cm->h_stage;
     std::vector<uint64_t> send(W), recv(W);
@@ -305,7 +305,7 @@ Keys comm_repartition(xlb_ctx* c, const Keys& in, int keysel, bool sorted_unique
     uint64_t so = 0, ro = 0;
     for (uint32_t r = 0; r < W; ++r) {
         if (r == c->comm_rank) {
-            if (send[r]) CUDA_OK(cudaMemcpyAsync(out.buf->as<uint64_t>() + ro, part.ptr() + so, send[r] * 8, cudaMemcpyDeviceToDevice, c->stream));
+            if (send[r]) CUDA_OK(copy_async(c, out.buf->as<uint64_t>() + ro, part.ptr() + so, send[r] * 8, cudaMemcpyDeviceToDevice));
         } else {
             if (send[r]) NCCL_OK(api().Send(part.ptr() + so, send[r], ncclUint64, (int)r, cm->comm, c->stream));
             if (recv[r]) NCCL_OK(api().Recv(out.buf->as<uint64_t>() + ro, recv[r], ncclUint64, (int)r, cm->comm, c->stream));

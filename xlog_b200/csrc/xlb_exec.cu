@@ -1615,8 +1615,8 @@ static void frontier_loop(xlb_ctx* c, const FrontierPlan& fp, const std::string&
     Buf cand = make_buf(c, bitmap_bytes);
     Buf counts = make_buf(c, (uint64_t)max_launches * 32 + 16);  // and, behind the counters, the step kernel's count of finished blocks
     unsigned int* visited = ds->visited->as<unsigned int>();
-    CUDA_OK(cudaMemcpyAsync(cand->p, visited, words * 4, cudaMemcpyDeviceToDevice, c->stream));
-    CUDA_OK(cudaMemsetAsync(counts->p, 0, (uint64_t)max_launches * 32 + 16, c->stream));
+    CUDA_OK(copy_async(c, cand->p, visited, words * 4, cudaMemcpyDeviceToDevice));
+    CUDA_OK(set_async(c, counts->p, 0, (uint64_t)max_launches * 32 + 16));
     unsigned int* ticket = reinterpret_cast<unsigned int*>(counts->as<unsigned long long>() + 4 * max_launches);
     struct Flight {
         unsigned long long seq = 0;  // the number the step kernel writes beside the counts it leaves in pinned memory
@@ -2206,7 +2206,6 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
     if (!c || !plan) return XLB_ERR_INVALID;
     RunState rs;
     EncodedRun enc;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
     uint64_t launches0 = c->launches, syncs0 = c->syncs;
     double wait0 = c->ms_sync_wait, alloc0 = c->ms_alloc;
     auto host_t0 = std::chrono::steady_clock::now();
@@ -2217,9 +2216,9 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
     xlb_status result = XLB_OK;
     try {
         CUDA_OK(cudaSetDevice(c->device));
-        CUDA_OK(cudaEventCreate(&e0));
-        CUDA_OK(cudaEventCreate(&e1));
-        CUDA_OK(cudaEventRecord(e0, c->stream));
+        if (!c->plan_e0) CUDA_OK(cudaEventCreate(&c->plan_e0));
+        if (!c->plan_e1) CUDA_OK(cudaEventCreate(&c->plan_e1));
+        CUDA_OK(cudaEventRecord(c->plan_e0, c->stream));
         if (!plan->sccs && plan->n_sccs) xlb_fail(XLB_ERR_INVALID, "plan has no SCC array");
         std::set<std::string> heads;
         const xlb_plan* run = enc.begin(c, plan);
@@ -2228,11 +2227,12 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
             for (uint32_t i = 0; i < run->sccs[s].n_rules; ++i) heads.insert(run->sccs[s].rules[i].head);
         }
         enc.finish();
-        check_dev_status(c);
-        CUDA_OK(cudaEventRecord(e1, c->stream));
-        CUDA_OK(cudaStreamSynchronize(c->stream));  // executor/mod.rs:1463
+        CUDA_OK(cudaEventRecord(c->plan_e1, c->stream));
+        c->drained = false;
+        check_dev_status(c);  // waits for everything above (executor/mod.rs:1463)
+        CUDA_OK(cudaEventSynchronize(c->plan_e1));
         float ms = 0;
-        CUDA_OK(cudaEventElapsedTime(&ms, e0, e1));
+        CUDA_OK(cudaEventElapsedTime(&ms, c->plan_e0, c->plan_e1));
         rs.st.ms_total = ms;
         uint64_t derived = 0;
         for (auto& h : heads) derived += store_get(c, h)->rows;
@@ -2255,8 +2255,6 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
         }
     }
     xlb_resolve_phase_timers(c);
-    if (e0) cudaEventDestroy(e0);
-    if (e1) cudaEventDestroy(e1);
     rs.st.kernel_launches = c->launches - launches0;
     rs.st.host_syncs = c->syncs - syncs0;
     rs.st.ms_host_wait = c->ms_sync_wait - wait0;

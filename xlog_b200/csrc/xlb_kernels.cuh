@@ -222,7 +222,7 @@ struct LoadLow32 {  // low half of a u64 word (the match length of a probe resul
 template <class Load, class Tout>
 void exclusive_scan(xlb_ctx* c, Load load, uint64_t n, Tout* out, Tout* d_total) {
     if (n == 0) {
-        CUDA_OK(cudaMemsetAsync(d_total, 0, sizeof(Tout), c->stream));
+        CUDA_OK(set_async(c, d_total, 0, sizeof(Tout)));
         return;
     }
     uint64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
@@ -382,7 +382,7 @@ uint64_t select_unordered(xlb_ctx* c, Pred pred, Emit emit, uint64_t n, const ch
     if (n == 0) return 0;
     uint64_t ntiles = (n + SA_TILE - 1) / SA_TILE;
     Buf total = make_buf(c, 8);
-    CUDA_OK(cudaMemsetAsync(total->p, 0, 8, c->stream));
+    CUDA_OK(set_async(c, total->p, 0, 8));
     prof_begin(c, name, bytes);
     select_append_k<Pred, Emit><<<(unsigned)ntiles, SA_BLOCK, 0, c->stream>>>(pred, emit, n, total->as<unsigned long long>());
     check_launch(c, name);
@@ -810,8 +810,8 @@ struct SortPlan {
 inline SortPlan plan_sort(xlb_ctx* c, const uint64_t* keys, uint64_t n) {
     SortPlan p;
     Buf oa = make_buf(c, 16);
-    CUDA_OK(cudaMemsetAsync(oa->p, 0, 8, c->stream));
-    CUDA_OK(cudaMemsetAsync((char*)oa->p + 8, 0xFF, 8, c->stream));
+    CUDA_OK(set_async(c, oa->p, 0, 8));
+    CUDA_OK(set_async(c, (char*)oa->p + 8, 0xFF, 8));
     prof_begin(c, "radix_bits", n * 8ull);
     radix_bits_k<<<grid_for(c, n, BLOCK * 8), BLOCK, 0, c->stream>>>(keys, n, oa->as<unsigned long long>());
     check_launch(c, "radix_bits");
@@ -844,7 +844,7 @@ inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned di
         unsigned int* ghist = gh->as<unsigned int>();
         unsigned int* bases = ghist + 8 * 256;
         unsigned long long* varies = (unsigned long long*)(bases + 8 * 256);
-        CUDA_OK(cudaMemsetAsync(ghist, 0, 8 * 256 * 4, c->stream));
+        CUDA_OK(set_async(c, ghist, 0, 8 * 256 * 4));
         unsigned want = digit_mask & 0xFFu;
         if (known_bound != ~0ull)
             for (int d = 0; d < 8; ++d)
@@ -868,11 +868,11 @@ inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned di
         if (np == 0) return;
         uint64_t status_words = (uint64_t)ntiles * 256;
         Buf status = make_buf(c, (status_words * np + 8) * 4);  // per pass: tile status; then 8 tile counters
-        CUDA_OK(cudaMemsetAsync(status->p, 0, (status_words * np + 8) * 4, c->stream));
+        CUDA_OK(set_async(c, status->p, 0, (status_words * np + 8) * 4));
         unsigned int* counters = status->as<unsigned int>() + status_words * np;
         if (c->lb_first_tile) {  // test knob: tiles take their numbers from here on, so tile 0 never publishes
             for (int q = 0; q < 8; ++q) ((unsigned int*)&c->h_scalar[56])[q] = c->lb_first_tile;
-            CUDA_OK(cudaMemcpyAsync(counters, &c->h_scalar[56], 8 * 4, cudaMemcpyHostToDevice, c->stream));
+            CUDA_OK(copy_async(c, counters, &c->h_scalar[56], 8 * 4, cudaMemcpyHostToDevice));
         }
         for (int q = 0; q < np; ++q) {
             int d = digits[q];
@@ -1052,7 +1052,7 @@ inline Buf set_difference(xlb_ctx* c, const uint64_t* A, uint64_t na, const uint
         Buf o = make_buf(c, na * 8);
         if (a_has_dups) *n_out = dedup_sorted(c, A, na, o->as<uint64_t>());
         else {
-            CUDA_OK(cudaMemcpyAsync(o->p, A, na * 8, cudaMemcpyDeviceToDevice, c->stream));
+            CUDA_OK(copy_async(c, o->p, A, na * 8, cudaMemcpyDeviceToDevice));
             *n_out = na;
         }
         return o;
@@ -1073,7 +1073,7 @@ inline Buf set_difference(xlb_ctx* c, const uint64_t* A, uint64_t na, const uint
 inline Buf merge_disjoint(xlb_ctx* c, const uint64_t* A, uint64_t na, const uint64_t* B, uint64_t nb) {
     Buf o = make_buf(c, (na + nb) * 8);
     if (na == 0 || nb == 0) {
-        if (na + nb) CUDA_OK(cudaMemcpyAsync(o->p, na ? A : B, (na + nb) * 8, cudaMemcpyDeviceToDevice, c->stream));
+        if (na + nb) CUDA_OK(copy_async(c, o->p, na ? A : B, (na + nb) * 8, cudaMemcpyDeviceToDevice));
         return o;
     }
     uint64_t ntiles = (na + nb + MP_TILE - 1) / MP_TILE;
@@ -1489,7 +1489,7 @@ inline Buf mix_and_group(xlb_ctx* c, const uint64_t* in, uint64_t n) {
     unsigned int* ghist = gh->as<unsigned int>();
     unsigned int* bases = ghist + 8 * 256;
     unsigned long long* varies = (unsigned long long*)(bases + 8 * 256);
-    CUDA_OK(cudaMemsetAsync(ghist, 0, 8 * 256 * 4, c->stream));
+    CUDA_OK(set_async(c, ghist, 0, 8 * 256 * 4));
     prof_begin(c, "mix", n * 16ull);
     mix_hist_k<<<grid_for(c, n, BLOCK * 8), BLOCK, 0, c->stream>>>(in, words->as<uint64_t>(), n, ghist + 7 * 256);
     check_launch(c, "mix");
@@ -1498,11 +1498,11 @@ inline Buf mix_and_group(xlb_ctx* c, const uint64_t* in, uint64_t n) {
     check_launch(c, "radix_bases");
     const uint64_t status_words = (uint64_t)ntiles * 256;
     Buf status = make_buf(c, (status_words + 8) * 4);
-    CUDA_OK(cudaMemsetAsync(status->p, 0, (status_words + 8) * 4, c->stream));
+    CUDA_OK(set_async(c, status->p, 0, (status_words + 8) * 4));
     unsigned int* counters = status->as<unsigned int>() + status_words;
     if (c->lb_first_tile) {
         for (int q = 0; q < 8; ++q) ((unsigned int*)&c->h_scalar[56])[q] = c->lb_first_tile;
-        CUDA_OK(cudaMemcpyAsync(counters, &c->h_scalar[56], 8 * 4, cudaMemcpyHostToDevice, c->stream));
+        CUDA_OK(copy_async(c, counters, &c->h_scalar[56], 8 * 4, cudaMemcpyHostToDevice));
     }
     prof_begin(c, "radix_scatter", n * 16ull);
     radix_scatter_k<false, true><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(words->as<uint64_t>(), out->as<uint64_t>(), nullptr, nullptr, n, 56, bases + 7 * 256, ntiles, counters,

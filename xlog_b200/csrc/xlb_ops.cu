@@ -329,6 +329,7 @@ PhaseTimer::~PhaseTimer() {
     g_phase_recs.push_back({e0, e1, acc});
 }
 void xlb_resolve_phase_timers(xlb_ctx* c) {
+    if (g_phase_recs.empty() && c->prof.empty()) return;
     cudaStreamSynchronize(c->stream);
     for (auto& r : g_phase_recs) {
         float ms = 0;
@@ -386,7 +387,7 @@ static Keys rel_packed(xlb_ctx* c, const xlb_rel* r, int fcol, uint32_t fval, Ke
         // pack and, in the same sweep, reduce the OR of all rows: later sorts of anything derived
         // from this relation plan their digits from it without a read-back
         Buf oa = make_buf(c, 16);
-        CUDA_OK(cudaMemsetAsync(oa->p, 0, 16, c->stream));
+        CUDA_OK(set_async(c, oa->p, 0, 16));
         prof_begin(c, "pack", r->rows * (materialize ? 16ull : 8ull));
         const bool fuse = filtered && r->schema.arity == 2 && fcol >= 0 && fcol < 2;
         if (fuse) filtered->buf = make_buf(c, r->rows * 8);  // at most every row; trimmed below
@@ -460,7 +461,7 @@ Keys ops_copy(xlb_ctx* c, const Keys& in) {
     o.n = in.n;
     o.bound = in.bound;
     o.buf = make_buf(c, in.n * 8);
-    if (in.n) CUDA_OK(cudaMemcpyAsync(o.buf->p, in.buf->p, in.n * 8, cudaMemcpyDeviceToDevice, c->stream));
+    if (in.n) CUDA_OK(copy_async(c, o.buf->p, in.buf->p, in.n * 8, cudaMemcpyDeviceToDevice));
     return o;
 }
 
@@ -473,7 +474,7 @@ Keys ops_from_host(xlb_ctx* c, const uint64_t* rows, uint64_t n) {
     o.buf = make_buf(c, n * 8);
     for (uint64_t i = 0; i < n; ++i) c->h_scalar[40 + i] = rows[i];  // pinned staging words
     if (n) {
-        CUDA_OK(cudaMemcpyAsync(o.buf->p, &c->h_scalar[40], n * 8, cudaMemcpyHostToDevice, c->stream));
+        CUDA_OK(copy_async(c, o.buf->p, &c->h_scalar[40], n * 8, cudaMemcpyHostToDevice));
         stream_wait(c);  // the staging words are reused by the next call
     }
     return o;
@@ -484,7 +485,7 @@ Keys ops_slice(xlb_ctx* c, const Keys& in, uint64_t lo, uint64_t hi) {
     o.n = hi - lo;
     o.bound = in.bound;
     o.buf = make_buf(c, o.n * 8);
-    if (o.n) CUDA_OK(cudaMemcpyAsync(o.buf->p, in.ptr() + lo, o.n * 8, cudaMemcpyDeviceToDevice, c->stream));
+    if (o.n) CUDA_OK(copy_async(c, o.buf->p, in.ptr() + lo, o.n * 8, cudaMemcpyDeviceToDevice));
     return o;
 }
 
@@ -498,7 +499,7 @@ Keys ops_concat(xlb_ctx* c, const std::vector<Keys>& parts) {
     o.buf = make_buf(c, o.n * 8);
     uint64_t at = 0;
     for (auto& p : parts) {
-        if (p.n) CUDA_OK(cudaMemcpyAsync(o.buf->as<uint64_t>() + at, p.buf->p, p.n * 8, cudaMemcpyDeviceToDevice, c->stream));
+        if (p.n) CUDA_OK(copy_async(c, o.buf->as<uint64_t>() + at, p.buf->p, p.n * 8, cudaMemcpyDeviceToDevice));
         at += p.n;
     }
     return o;
@@ -547,7 +548,7 @@ DenseSet ops_dense_begin(xlb_ctx* c, int hi_bits, int lo_bits) {
     const uint64_t bitmap_bytes = (d.words * 4 + 7) & ~7ull;
     d.bitmap = make_buf(c, bitmap_bytes + 24);
     d.counts = (uint64_t*)((char*)d.bitmap->p + bitmap_bytes);
-    CUDA_OK(cudaMemsetAsync(d.bitmap->p, 0, bitmap_bytes + 24, c->stream));
+    CUDA_OK(set_async(c, d.bitmap->p, 0, bitmap_bytes + 24));
     return d;
 }
 
@@ -559,8 +560,8 @@ DenseSet ops_dense_begin_from(xlb_ctx* c, int hi_bits, int lo_bits, unsigned int
     const uint64_t bitmap_bytes = (d.words * 4 + 7) & ~7ull;
     d.bitmap = make_buf(c, bitmap_bytes + 24);
     d.counts = (uint64_t*)((char*)d.bitmap->p + bitmap_bytes);
-    CUDA_OK(cudaMemcpyAsync(d.bitmap->p, visited, d.words * 4, cudaMemcpyDeviceToDevice, c->stream));
-    CUDA_OK(cudaMemsetAsync((char*)d.bitmap->p + d.words * 4, 0, bitmap_bytes + 24 - d.words * 4, c->stream));
+    CUDA_OK(copy_async(c, d.bitmap->p, visited, d.words * 4, cudaMemcpyDeviceToDevice));
+    CUDA_OK(set_async(c, (char*)d.bitmap->p + d.words * 4, 0, bitmap_bytes + 24 - d.words * 4));
     d.visited = visited;
     d.seeded = true;
     return d;
@@ -577,8 +578,8 @@ DenseSet ops_dense_begin_state(xlb_ctx* c, DenseState& s) {
     d.bitmap = s.marks;
     d.counts_buf = make_buf(c, 24);
     d.counts = d.counts_buf->as<uint64_t>();
-    CUDA_OK(cudaMemsetAsync(d.counts_buf->p, 0, 24, c->stream));
-    CUDA_OK(cudaMemsetAsync(s.touched->p, 0, s.touched->bytes, c->stream));
+    CUDA_OK(set_async(c, d.counts_buf->p, 0, 24));
+    CUDA_OK(set_async(c, s.touched->p, 0, s.touched->bytes));
     d.touched = s.touched->as<unsigned char>();
     d.visited = s.visited->as<unsigned int>();
     d.seeded = true;
@@ -645,7 +646,7 @@ void ops_dense_state_build(xlb_ctx* c, DenseState& s, int hi_bits, int lo_bits, 
     s.lo_bits = lo_bits;
     s.words = ((1ull << (hi_bits + lo_bits)) + 31) / 32;
     s.visited = make_buf(c, s.words * 4);
-    CUDA_OK(cudaMemsetAsync(s.visited->p, 0, s.words * 4, c->stream));
+    CUDA_OK(set_async(c, s.visited->p, 0, s.words * 4));
     for (const Keys* k : {&full, &novel}) {
         if (!k->n) continue;
         prof_begin(c, "dense_mark", k->n * 8ull);
@@ -656,7 +657,7 @@ void ops_dense_state_build(xlb_ctx* c, DenseState& s, int hi_bits, int lo_bits, 
     s.touched = nullptr;
     if (s.words >= DENSE_WIDE_WORDS && s.words % (32 * DW_WPL) == 0) {
         s.marks = make_buf(c, s.words * 4);
-        CUDA_OK(cudaMemcpyAsync(s.marks->p, s.visited->p, s.words * 4, cudaMemcpyDeviceToDevice, c->stream));
+        CUDA_OK(copy_async(c, s.marks->p, s.visited->p, s.words * 4, cudaMemcpyDeviceToDevice));
         s.touched = make_buf(c, s.words / (32 * DW_WPL));
     }
     s.rows = full.n + novel.n;
@@ -671,7 +672,7 @@ Keys ops_dense_state_rows(xlb_ctx* c, const DenseState& s, uint64_t bound) {
     d.bitmap = s.visited;
     d.bound = bound;
     Buf counts = make_buf(c, 24);
-    CUDA_OK(cudaMemsetAsync(counts->p, 0, 24, c->stream));
+    CUDA_OK(set_async(c, counts->p, 0, 24));
     d.counts = counts->as<uint64_t>();
     Keys none;
     return dense_finish(c, d, none, &s.rows);  // nothing to subtract, no second bitmap: every set bit comes out, s.rows of them
@@ -682,8 +683,8 @@ static void tuple_set_alloc(xlb_ctx* c, TupleSet& s, uint64_t tuples) {
     while ((1ull << s.log2cap) < 2 * tuples) ++s.log2cap;
     s.cap = 1ull << s.log2cap;
     s.table = make_buf(c, s.cap * 8 + 8);
-    CUDA_OK(cudaMemsetAsync(s.table->p, 0xFF, s.cap * 8, c->stream));
-    CUDA_OK(cudaMemsetAsync((char*)s.table->p + s.cap * 8, 0, 8, c->stream));
+    CUDA_OK(set_async(c, s.table->p, 0xFF, s.cap * 8));
+    CUDA_OK(set_async(c, (char*)s.table->p + s.cap * 8, 0, 8));
 }
 
 static unsigned int* tuple_set_flag(const TupleSet& s) { return (unsigned int*)((char*)s.table->p + s.cap * 8); }
@@ -741,7 +742,7 @@ Keys ops_tuple_set_novel(xlb_ctx* c, TupleSet& s, const Keys& cand) {
         const uint64_t need = s.rows + cand.n;
         tuple_set_alloc(c, s, need < (1ull << 27) ? 2 * need : need);  // (a table of gigabytes grows to what is needed only)
         tuple_set_fill(c, s, old.table->as<uint64_t>(), old.cap, true);
-        CUDA_OK(cudaMemcpyAsync(tuple_set_flag(s), tuple_set_flag(old), 4, cudaMemcpyDeviceToDevice, c->stream));
+        CUDA_OK(copy_async(c, tuple_set_flag(s), tuple_set_flag(old), 4, cudaMemcpyDeviceToDevice));
     }
     Buf words = tuple_set_words(c, s, cand.ptr(), cand.n);
     Buf out = make_buf(c, cand.n * 8);
@@ -843,7 +844,7 @@ Index ops_index_build(xlb_ctx* c, Buf S, uint64_t n, int key_shift, Buf pay) {
     while (cap < 2 * nu) cap <<= 1;
     ix.mask = cap - 1;
     ix.table = make_buf(c, cap * 16);
-    CUDA_OK(cudaMemsetAsync(ix.table->p, 0, cap * 16, c->stream));
+    CUDA_OK(set_async(c, ix.table->p, 0, cap * 16));
     if (nu) {
         prof_begin(c, "hash_insert", 0);
         hash_insert_k<<<grid_for(c, nu), BLOCK, 0, c->stream>>>(S->as<uint64_t>(), n, key_shift, starts->as<uint32_t>(), nu, ix.table->as<ulonglong2>(), ix.mask, c->d_status);
@@ -861,7 +862,7 @@ Index ops_index_build_direct(xlb_ctx* c, const Keys& rows, int keysel, int key_b
     const uint64_t other = keysel == SRC_HI ? (rows.bound & 0xFFFFFFFFull) : (rows.bound >> 32);
     ix.pay_bound = rows.bound == ~0ull ? 0xFFFFFFFFull : other;
     Buf cnt = make_buf(c, ix.domain * 4);
-    CUDA_OK(cudaMemsetAsync(cnt->p, 0, ix.domain * 4, c->stream));
+    CUDA_OK(set_async(c, cnt->p, 0, ix.domain * 4));
     ix.cursor = make_buf(c, ix.domain * 8);
     ix.pay = make_buf(c, rows.n * 4);
     Buf total = make_buf(c, 8);
@@ -906,7 +907,7 @@ Buf ops_keyset(xlb_ctx* c, const Keys& bag, int keysel, int key_bits) {
     const uint64_t domain = 1ull << key_bits;
     const uint64_t bytes = std::max<uint64_t>(domain / 8, 16);  // whole 16-byte words: the streaming kernel copies it that way
     Buf keyset = make_buf(c, bytes);
-    CUDA_OK(cudaMemsetAsync(keyset->p, 0, bytes, c->stream));
+    CUDA_OK(set_async(c, keyset->p, 0, bytes));
     if (bag.n) {
         prof_begin(c, "keyset_mark", bag.n * 8ull);
         keyset_mark_k<<<grid_for(c, bag.n), BLOCK, 0, c->stream>>>(bag.ptr(), bag.n, keysel, keyset->as<unsigned int>(), domain, c->d_status);
@@ -1047,7 +1048,7 @@ Keys ops_partition_by_owner_dev(xlb_ctx* c, const Keys& in, int keysel, uint32_t
     out.n = in.n;
     out.buf = make_buf(c, in.n * 8);
     if (world > 64) xlb_fail(XLB_ERR_UNSUPPORTED, "at most 64 ranks");
-    CUDA_OK(cudaMemsetAsync(counts, 0, (size_t)world * 8, c->stream));
+    CUDA_OK(set_async(c, counts, 0, (size_t)world * 8));
     if (in.n == 0) return out;
     Buf cur = make_buf(c, 64 * 8);
     unsigned long long* cursors = cur->as<unsigned long long>();
@@ -1105,9 +1106,9 @@ extern "C" xlb_status xlb_ctx_create(const xlb_config* cfg, xlb_ctx** out) {
         c->max_iterations = cfg && cfg->max_iterations ? cfg->max_iterations : 1000000ull;
         c->join_chunk = cfg ? cfg->join_chunk_tuples : 0;
         c->flags = cfg ? cfg->flags : 0;
-        CUDA_OK(cudaHostAlloc((void**)&c->h_scalar, 64 * 8, cudaHostAllocMapped));
+        CUDA_OK(cudaHostAlloc((void**)&c->h_scalar, SCALAR_WORDS * 8, cudaHostAllocMapped));
         CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_scalar_dev, c->h_scalar, 0));
-        memset(c->h_scalar, 0, 64 * 8);
+        memset(c->h_scalar, 0, SCALAR_WORDS * 8);
         CUDA_OK(cudaMalloc(&c->d_status, sizeof(DevStatus)));
         CUDA_OK(cudaMemset(c->d_status, 0, sizeof(DevStatus)));
         cudaDeviceProp prop;
@@ -1134,6 +1135,8 @@ extern "C" void xlb_ctx_destroy(xlb_ctx* c) {
     if (c->h_scalar) cudaFreeHost(c->h_scalar);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->d_status) cudaFree(c->d_status);
+    if (c->plan_e0) cudaEventDestroy(c->plan_e0);
+    if (c->plan_e1) cudaEventDestroy(c->plan_e1);
     c->arena.destroy();
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -1188,7 +1191,7 @@ extern "C" xlb_status xlb_rel_from_host(xlb_ctx* c, const xlb_schema* s, const v
         r->cols[i] = make_buf(c, bytes);
         if (bytes) {
             if (!cols[i]) xlb_fail(XLB_ERR_INVALID, "column %u pointer is null", i);
-            CUDA_OK(cudaMemcpyAsync(r->cols[i]->p, cols[i], bytes, cudaMemcpyHostToDevice, c->stream));
+            CUDA_OK(copy_async(c, r->cols[i]->p, cols[i], bytes, cudaMemcpyHostToDevice));
         }
     }
     CUDA_OK(cudaStreamSynchronize(c->stream));
@@ -1260,7 +1263,7 @@ extern "C" xlb_status xlb_rel_to_host(xlb_ctx* c, const xlb_rel* r, void* const*
     } else if (n && arity) {
         ops_rel_columns(c, r);
         for (uint32_t i = 0; i < arity; ++i)
-            CUDA_OK(cudaMemcpyAsync(cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost, c->stream));
+            CUDA_OK(copy_async(c, cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost));
         CUDA_OK(cudaStreamSynchronize(c->stream));
     } else {
         CUDA_OK(cudaStreamSynchronize(c->stream));
@@ -1284,7 +1287,7 @@ static xlb_rel* rel_clone(xlb_ctx* c, const xlb_rel* r) {
         for (uint32_t i = 0; i < r->schema.arity; ++i) {
             uint64_t bytes = r->rows * type_width(r->schema.types[i]);
             o->cols[i] = make_buf(c, bytes);
-            if (bytes) CUDA_OK(cudaMemcpyAsync(o->cols[i]->p, r->cols[i]->p, bytes, cudaMemcpyDeviceToDevice, c->stream));
+            if (bytes) CUDA_OK(copy_async(c, o->cols[i]->p, r->cols[i]->p, bytes, cudaMemcpyDeviceToDevice));
         }
     }
     return o.release();
@@ -1304,7 +1307,7 @@ extern "C" xlb_status xlb_rel_checksum(xlb_ctx* c, const xlb_rel* r, uint64_t di
     if (!c || !r || !digest) return XLB_ERR_INVALID;
     API_BEGIN(c)
     Buf acc = make_buf(c, 16);
-    CUDA_OK(cudaMemsetAsync(acc->p, 0, 16, c->stream));
+    CUDA_OK(set_async(c, acc->p, 0, 16));
     if (r->rows && r->schema.arity) {
         prof_begin(c, "digest", 0);
         if (rel_packable(r->schema)) {
@@ -1514,7 +1517,7 @@ xlb_rel* rel_concat(xlb_ctx* c, const xlb_rel* const* ins, uint32_t n) {
         for (uint32_t i = 0; i < n; ++i) {
             if (ins[i]->rows) {
                 ops_rel_columns(c, ins[i]);
-                CUDA_OK(cudaMemcpyAsync((char*)o->cols[col]->p + at * w, ins[i]->cols[col]->p, ins[i]->rows * w, cudaMemcpyDeviceToDevice, c->stream));
+                CUDA_OK(copy_async(c, (char*)o->cols[col]->p + at * w, ins[i]->cols[col]->p, ins[i]->rows * w, cudaMemcpyDeviceToDevice));
             }
             at += ins[i]->rows;
         }
