@@ -1272,32 +1272,15 @@ extern "C" xlb_status xlb_rel_to_host(xlb_ctx* c, const xlb_rel* r, void* const*
     API_END()
 }
 
-static xlb_rel* rel_clone(xlb_ctx* c, const xlb_rel* r) {
-    std::unique_ptr<xlb_rel> o(new xlb_rel);
-    o->ctx = c;
-    o->schema = r->schema;
-    o->rows = r->rows;
-    o->canonical = r->canonical;
-    if (r->packed) {
-        Keys k;
-        k.buf = r->packed;
-        k.n = r->rows;
-        o->packed = ops_copy(c, k).buf;
-    } else {
-        for (uint32_t i = 0; i < r->schema.arity; ++i) {
-            uint64_t bytes = r->rows * type_width(r->schema.types[i]);
-            o->cols[i] = make_buf(c, bytes);
-            if (bytes) CUDA_OK(copy_async(c, o->cols[i]->p, r->cols[i]->p, bytes, cudaMemcpyDeviceToDevice));
-        }
-    }
-    return o.release();
-}
+xlb_rel* rel_view(xlb_ctx* c, const xlb_rel* r);
+// Relations are immutable and their buffers counted, so a clone shares what its original holds now;
+// what either materialises later (a packed copy, columns) is its own.
+static xlb_rel* rel_clone(xlb_ctx* c, const xlb_rel* r) { return rel_view(c, r); }
 
 extern "C" xlb_status xlb_rel_clone(xlb_ctx* c, const xlb_rel* r, xlb_rel** out) {
     if (!c || !r || !out) return XLB_ERR_INVALID;
     API_BEGIN(c)
     *out = rel_clone(c, r);
-    CUDA_OK(cudaStreamSynchronize(c->stream));
     API_END()
 }
 
