@@ -1,0 +1,108 @@
+"""The delta loop (linear recursive rules run to their fixpoint by one kernel) against the oracle and
+against the general loop: iterations of one row and of many, rows with more matches than a warp
+takes, two joined relations, several rules, a log that has to grow, the iteration limit."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from xlog_b200 import _abi as A
+from xlog_b200 import programs, workloads
+from xlog_b200.executor import run_program
+from xlog_b200.lib import XlbError
+from xlog_b200.plan import CompiledRule, ExecutionPlan, Join, Project, Scan, Scc
+from xlog_b200.provider import KernelProvider
+
+pytestmark = pytest.mark.gpu
+U2 = (A.U32, A.U32)
+
+
+def both(plan, inputs, out, monkeypatch):
+    res = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("XLB_NO_DELTA_LOOP", "1")
+        else:
+            monkeypatch.delenv("XLB_NO_DELTA_LOOP", raising=False)
+        p = KernelProvider(device=0)
+        got, stats = run_program(p, plan, inputs, [out])
+        p.close()
+        res.append((got[out], stats["iterations"], stats["candidate_tuples"]))
+    for a, b in zip(res[0][0], res[1][0]):
+        assert np.array_equal(a, b)
+    assert res[0][1:] == res[1][1:]
+    return res[0]
+
+
+def star(hub, leaves):
+    """hub -> leaves -> hub' -> leaves': rows with `leaves` matches."""
+    l0 = np.arange(10, 10 + leaves, dtype=np.uint32)
+    return [np.concatenate([np.full(leaves, hub), l0]).astype(np.uint32), np.concatenate([l0, np.full(leaves, hub + 1)]).astype(np.uint32)]
+
+
+def chain(n):
+    return [np.arange(n - 1, dtype=np.uint32), np.arange(1, n, dtype=np.uint32)]
+
+
+@pytest.mark.parametrize("edge", [chain(2), chain(3), chain(300), star(1, 1023), star(1, 1025), star(1, 40000)], ids=["one", "two", "chain", "row1023", "row1025", "row40000"])
+@pytest.mark.parametrize("program", [programs.transitive_closure, programs.transitive_closure_left_linear, programs.transitive_closure_swapped_head])
+def test_closure(edge, program, monkeypatch):
+    got, _, _ = both(program(), {"edge": edge}, "reach", monkeypatch)
+    want, _ = O.run_program(program(), {"edge": edge}, ["reach"])
+    for g, w in zip(got, want["reach"]):
+        assert np.array_equal(g, w)
+
+
+def test_many_long_rows(monkeypatch):
+    # 70 sources with 1100 matches each twice over: the list of long rows is used by many warps at once
+    src = np.repeat(np.arange(70, dtype=np.uint32), 1100)
+    mid = np.tile(np.arange(100, 1200, dtype=np.uint32), 70)
+    back = [np.arange(100, 1200, dtype=np.uint32), np.arange(1100, dtype=np.uint32) % 70]
+    both(programs.transitive_closure(), {"edge": [np.concatenate([src, back[0]]), np.concatenate([mid, back[1]])]}, "reach", monkeypatch)
+
+
+@pytest.mark.parametrize("nodes", [40, 701])
+def test_same_generation(nodes, monkeypatch):
+    c0, c1, _ = workloads.tree_dag(nodes, 0.05)
+    got, _, _ = both(programs.same_generation(), {"edge": [c0, c1]}, "sg", monkeypatch)
+    want, _ = O.run_program(programs.same_generation(), {"edge": [c0, c1]}, ["sg"])
+    for g, w in zip(got, want["sg"]):
+        assert np.array_equal(g, w)
+
+
+def test_two_recursive_rules_and_wide_domain(monkeypatch):
+    # p(X,Y) :- e(X,Y).  p(X,Z) :- p(X,Y), e(Y,Z).  p(X,Z) :- f(X,Y), p(Y,Z).  ids up to 2^15: 30 bits
+    ids = {"e": 0, "f": 1, "p": 2}
+    plan = ExecutionPlan([Scc(0, True, [
+        CompiledRule("p", Scan(0), U2),
+        CompiledRule("p", Project(Join(Scan(2), Scan(0), [1], [0]), [0, 3]), U2),
+        CompiledRule("p", Project(Join(Scan(1), Scan(2), [1], [0]), [0, 3]), U2)])], ids)
+    rng = np.random.default_rng(3)
+    e = [rng.integers(0, 1 << 15, 3000).astype(np.uint32) for _ in range(2)]
+    f = [rng.integers(0, 1 << 15, 3000).astype(np.uint32), e[0][rng.integers(0, 3000, 3000)]]
+    both(plan, {"e": e, "f": f}, "p", monkeypatch)
+
+
+def test_log_grows(monkeypatch):
+    # 4500 nodes in one cycle-rich component: 20 M tuples over a domain of 2^26, more than the first log holds
+    c = workloads.uniform_digraph(4500, 18000)
+    got, _, _ = both(programs.transitive_closure(), {"edge": list(c)}, "reach", monkeypatch)
+    assert len(got[0]) > 1 << 24
+
+
+def test_iteration_limit():
+    for n, fits in [(6, True), (7, False)]:  # a chain of n nodes takes n - 1 iterations, the last of which finds nothing
+        p = KernelProvider(device=0, max_iterations=5)
+        if fits:
+            got, stats = run_program(p, programs.transitive_closure(), {"edge": chain(n)}, ["reach"])
+            assert len(got["reach"][0]) == n * (n - 1) // 2 and stats["iterations"] == 5
+        else:
+            with pytest.raises(XlbError) as e:
+                run_program(p, programs.transitive_closure(), {"edge": chain(n)}, ["reach"])
+            assert e.value.status == A.ERR_ITER_LIMIT
+        p.close()
+
+
+def test_one_column_head_after_the_frontier_loop(monkeypatch):
+    # a path longer than the frontier loop follows: the rest of it runs in the delta loop
+    got, it, _ = both(programs.reach_from_source(0), {"edge": chain(500)}, "r", monkeypatch)
+    assert len(got[0]) == 499 and it == 499

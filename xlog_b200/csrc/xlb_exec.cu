@@ -1740,6 +1740,198 @@ static void frontier_loop(xlb_ctx* c, const FrontierPlan& fp, const std::string&
     }
 }
 
+// ------------------------------------------------------------------------------ delta loop
+// A component of one head whose recursive rules hold one recursive atom each, joined with one or two
+// stored relations on its columns — closure in either direction, same generation, copies — runs to
+// its fixpoint on the device (ops_delta_run).  Heads of up to 32 bits: above the 27 bits that the
+// launch-by-launch bitmap route starts with, too, since nothing here passes over the whole bitmap per
+// iteration (a clear and one pass to read the result off, 0.3 ms at 2^32).
+struct DeltaPlan {
+    struct One {
+        const FlatRule* fr;
+        int joins = 0;
+        size_t atom[2];
+        int kc[2], key_src[2];
+        int hi_src, lo_src;
+    };
+    std::vector<One> rec;
+    std::vector<const FlatRule*> seeds;
+};
+constexpr size_t DELTA_RULES_MAX = 4;
+
+static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const std::vector<std::string>& preds, const std::set<std::string>& rec,
+                        const std::map<std::string, xlb_schema>& schema, DeltaPlan* plan) {
+    if (c->world != 1 || c->comm_world != 1 || (c->flags & (XLB_FLAG_NO_DENSE | XLB_FLAG_KEEP_DELTAS)) || getenv("XLB_NO_DELTA_LOOP")) return false;
+    if (preds.size() != 1) return false;
+    const uint32_t arity = schema.at(preds[0]).arity;
+    for (auto& fr : rules) {
+        int at = -1, nrec = 0;
+        for (size_t i = 0; i < fr.atoms.size(); ++i)
+            if (rec.count(fr.atoms[i].rel)) {
+                ++nrec;
+                at = (int)i;
+            }
+        for (auto& k : fr.checks)
+            if (rec.count(k.rel)) return false;
+        if (nrec == 0) {
+            plan->seeds.push_back(&fr);
+            continue;
+        }
+        if (nrec != 1 || !fr.filters.empty() || !fr.checks.empty() || fr.atoms.size() < 2 || fr.atoms.size() > 3) return false;
+        const Atom& d = fr.atoms[at];
+        if (d.arity != arity || (arity == 2 && d.var[0] == d.var[1])) return false;
+        const int hi = arity == 2 ? d.var[0] : -1, lo = d.var[arity - 1];
+        DeltaPlan::One one;
+        one.fr = &fr;
+        int other[2] = {-2, -2};
+        for (size_t i = 0; i < fr.atoms.size(); ++i) {
+            if ((int)i == at) continue;
+            const Atom& a = fr.atoms[i];
+            if (a.arity != 2 || a.var[0] == a.var[1]) return false;
+            const bool b0 = a.var[0] == hi || a.var[0] == lo, b1 = a.var[1] == hi || a.var[1] == lo;
+            if (b0 == b1) return false;
+            const int k = one.joins++;
+            one.atom[k] = i;
+            one.kc[k] = b0 ? 0 : 1;
+            one.key_src[k] = a.var[one.kc[k]] == hi ? SRC_HI : SRC_LO;
+            other[k] = a.var[1 - one.kc[k]];
+        }
+        if (other[0] == other[1]) return false;  // the two matches would have to agree
+        auto src = [&](int v) { return v == hi && hi >= 0 ? 0 : v == lo ? 1 : v == other[0] ? 2 : v == other[1] ? 3 : -1; };
+        one.hi_src = fr.head_vars.size() == 2 ? src(fr.head_vars[0]) : 4;
+        one.lo_src = src(fr.head_vars.back());
+        if (one.hi_src < 0 || one.lo_src < 0) return false;
+        plan->rec.push_back(one);
+    }
+    return !plan->rec.empty() && plan->rec.size() <= DELTA_RULES_MAX;
+}
+
+// OR bounds of the head's two halves over everything the component can derive, from the bounds of the
+// relations it reads and of the rows the head starts with.  False: some bound is not known.
+static bool delta_bounds(xlb_ctx* c, const std::vector<FlatRule>& rules, const std::string& p, RunState& rs, uint64_t start, uint64_t* bound) {
+    uint64_t hi = start >> 32, lo = start & 0xFFFFFFFFull;
+    std::map<std::string, uint64_t> known;
+    for (auto& fr : rules)
+        for (auto& a : fr.atoms)
+            if (a.rel != p && !known.count(a.rel)) {
+                const Keys k = packed_for_rules(c, a.rel, rules, rs);
+                if (k.n && k.bound == ~0ull) return false;
+                known[a.rel] = k.n ? k.bound : 0;
+            }
+    for (bool grew = true; grew;) {  // (bits are only ever added)
+        grew = false;
+        for (auto& fr : rules) {
+            auto var_bound = [&](int v) {  // a value is in every column its variable stands for
+                uint64_t b = 0xFFFFFFFFull;
+                for (auto& a : fr.atoms)
+                    for (uint32_t j = 0; j < a.arity; ++j) {
+                        if (a.var[j] != v) continue;
+                        const bool high = a.arity == 2 && j == 0;
+                        b &= a.rel == p ? (high ? hi : lo) : (high ? known[a.rel] >> 32 : known[a.rel] & 0xFFFFFFFFull);
+                    }
+                return b;
+            };
+            const uint64_t h = hi | (fr.head_vars.size() == 2 ? var_bound(fr.head_vars[0]) : 0), l = lo | var_bound(fr.head_vars.back());
+            grew |= h != hi || l != lo;
+            hi = h;
+            lo = l;
+        }
+    }
+    *bound = (hi << 32) | lo;
+    return true;
+}
+
+// Seeds the component (unless `from_store`: then the stored head and "__delta_<head>" are where it
+// stands) and runs it to its fixpoint.  False: not taken, nothing changed.
+static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<FlatRule>& rules, const std::string& p, const xlb_schema& hs, bool from_store, RunState& rs,
+                       uint64_t& it, bool& fix) {
+    const xlb_run_stats before = rs.st;
+    try {
+        Keys full = from_store ? full_view(c, rs, p) : Keys(), delta;
+        if (from_store) {
+            delta = ops_rel_packed(c, store_get(c, "__delta_" + p));
+            if (!delta.n || !full.n || full.bound == ~0ull || it >= c->max_iterations) return false;
+            full = real_full(c, rs, p);
+        }
+        uint64_t bound = 0;
+        if (!delta_bounds(c, rules, p, rs, full.n ? full.bound : 0, &bound)) return false;
+        const int hb = bit_len(bound >> 32), lb = std::max(bit_len(bound & 0xFFFFFFFFull), 1);
+        if (hb + lb > WIDE_DENSE_BITS) return false;
+        const uint64_t bitmap = (1ull << (hb + lb)) / 8;
+        if (c->budget && c->allocated + 3 * bitmap > c->budget) return false;
+        DeltaLoop d = ops_delta_begin(c, hb, lb);
+        if (from_store) {
+            PhaseTimer t(c, &rs.st.ms_join);
+            ops_delta_append(c, d, delta);
+            ops_delta_known(c, d, full);
+        }
+        for (const FlatRule* fr : from_store ? std::vector<const FlatRule*>() : plan.seeds) {
+            bool any_empty = false;
+            for (auto& a : fr->atoms) {
+                xlb_rel* r = store_get(c, a.rel);
+                if (!r || r->rows == 0) any_empty = true;
+            }
+            if (any_empty) continue;
+            const size_t start = pick_seed_start(c, *fr);
+            xlb_rel* sr = store_get(c, fr->atoms[start].rel);
+            const Keys rows = ops_rel_packed(c, sr);
+            const uint64_t limit = chunk_limit(c);
+            for (uint64_t at = 0, chunk = rows.n; at < rows.n;) {  // in chunks, so that no join output exceeds the configured bound
+                const uint64_t hi = std::min(rows.n, at + chunk);
+                const Keys part = at == 0 && hi == rows.n ? rows : ops_slice(c, rows, at, hi);
+                Keys cand;
+                try {
+                    cand = run_pipeline(c, *fr, start, part, sr->canonical, -1, limit, rs);
+                } catch (const ChunkTooBig&) {
+                    chunk = std::max<uint64_t>((hi - at) / 2, 1);
+                    continue;
+                }
+                at = hi;
+                rs.st.candidate_tuples += cand.n;
+                PhaseTimer t(c, &rs.st.ms_setops);
+                ops_delta_seed(c, d, cand);
+            }
+        }
+        std::vector<DeltaRule> run;
+        for (auto& one : plan.rec) {
+            DeltaRule r;
+            r.joins = one.joins;
+            r.hi_src = one.hi_src;
+            r.lo_src = one.lo_src;
+            bool empty = false;
+            for (int k = 0; k < one.joins; ++k) {
+                r.ix[k] = &get_index(c, one.fr->atoms[one.atom[k]].rel, one.kc[k], rs);
+                r.key_src[k] = one.key_src[k];
+                empty |= r.ix[k]->n == 0;
+            }
+            if (!empty) run.push_back(r);
+        }
+        DeltaResult res;
+        {
+            PhaseTimer t(c, &rs.st.ms_join);
+            if (!ops_delta_run(c, d, run, c->max_iterations - it, full, &res)) check_dev_status(c);
+        }
+        it += res.iterations;
+        rs.st.iterations += res.iterations;
+        rs.st.candidate_tuples += res.candidates;
+        fix = res.fix;
+        d.log.reset();
+        PhaseTimer t(c, &rs.st.ms_setops);
+        DenseState ds;
+        ds.visited = d.visited;
+        ds.words = d.words;
+        ds.hi_bits = hb;
+        ds.lo_bits = lb;
+        ds.rows = full.n + res.rows - delta.n;  // (a delta taken from the store is part of the stored head)
+        install_full(c, p, hs, ops_dense_state_rows(c, ds, bound), nullptr, rs);
+        return true;
+    } catch (const XlbError& e) {
+        if (e.st != XLB_ERR_RESOURCE_EXHAUSTED) throw;
+        rs.st = before;  // not enough memory for a bitmap and a log: the routes that work in pieces take over
+        return false;
+    }
+}
+
 static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
     if (!scc.rules && scc.n_rules) xlb_fail(XLB_ERR_INVALID, "SCC %u has no rule array", scc.id);
     std::vector<std::string> preds;
@@ -1870,6 +2062,18 @@ static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
         xlb_rel* d = store_get(c, "__delta_" + p);
         if (!d || !rel_packable(d->schema) || d->schema.arity != schema[p].arity) resume = false;
     }
+    bool fix = false;
+    uint64_t it = 0;
+    DeltaPlan deltas;
+    const bool delta_ok = scc.is_recursive && delta_shape(c, rules, preds, rec, schema, &deltas);
+    auto limit_reached = [&]() { xlb_fail(XLB_ERR_ITER_LIMIT, "Recursive SCC iteration limit (%llu) exceeded", (unsigned long long)c->max_iterations); };
+    if (delta_ok && !resume && store_get(c, preds[0])->rows == 0) {
+        FrontierPlan fp;  // (a frontier that streams over an unindexed relation needs no index at all)
+        if (!frontier_shape(c, rules, preds, rec, schema, rs, &fp) && delta_loop(c, deltas, rules, preds[0], schema[preds[0]], false, rs, it, fix)) {
+            if (!fix) limit_reached();
+            return;
+        }
+    }
     if (resume) {
         for (auto& p : preds) {
             // both are handed to the loop as it keeps them: sorted and unique
@@ -1885,7 +2089,6 @@ static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
     }
     if (!scc.is_recursive) return;
 
-    bool fix = false;
     // A failure inside the loop (memory budget, a device status) must not leave deltas behind: a
     // later call would take them for a saved state and resume from them, over a full relation
     // that may lack merges still put off.  Without them the next call seeds again from the stored
@@ -1907,12 +2110,12 @@ static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
             }
         }
     } guard{c, rs, preds};
-    uint64_t it = 0;
     {
         FrontierPlan fp;
         if (frontier_shape(c, rules, preds, rec, schema, rs, &fp)) frontier_loop(c, fp, preds[0], schema[preds[0]], rs, it, fix);
     }
-    for (; !fix && it < c->max_iterations; ++it) {  // recursive.rs:619-937
+    const bool by_loop = delta_ok && !fix && delta_loop(c, deltas, rules, preds[0], schema[preds[0]], true, rs, it, fix);
+    for (; !by_loop && !fix && it < c->max_iterations; ++it) {  // recursive.rs:619-937
         rs.st.iterations++;
         rs.bag_novel.clear();
         std::map<std::string, Keys> novel;
@@ -2010,7 +2213,7 @@ static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
             c->store.erase(it);
         }
     }
-    if (!fix) xlb_fail(XLB_ERR_ITER_LIMIT, "Recursive SCC iteration limit (%llu) exceeded", (unsigned long long)c->max_iterations);
+    if (!fix) limit_reached();
 }
 
 // ---- plans over wide or typed columns ------------------------------------------------------------

@@ -186,6 +186,35 @@ void ops_frontier_scan(xlb_ctx* c, const ScanRows& src, int rel_keysel, int bits
                        unsigned long long* count_marked, const unsigned long long* keys_in_frontier, uint64_t* live_out, unsigned long long* live_count);
 void ops_frontier_step(xlb_ctx* c, const unsigned int* mark_parts, uint32_t parts, uint64_t words, unsigned int* own, unsigned int* visited, unsigned int* next_frontier,
                        unsigned long long* counts, unsigned int* ticket, unsigned long long* publish_to, unsigned long long seq);
+// Delta loop (xlb_delta.cu): a recursive component over one head of at most 32 bits whose recursive
+// rules join the delta with one or two stored relations, run to its fixpoint by one kernel.
+struct DeltaRule {
+    const Index* ix[2] = {nullptr, nullptr};
+    int key_src[2] = {SRC_LO, SRC_LO};  // half of the delta row that probes the index
+    int joins = 1;
+    int hi_src = 4, lo_src = 4;         // 0 / 1: the delta row's high / low half, 2 / 3: other column of the first / second match, 4: zero
+};
+struct DeltaLoop {
+    Buf visited;            // the head as a bitmap
+    uint64_t words = 0;
+    int hi_bits = 0, lo_bits = 0;
+    Buf log;                // derived tuples in the order they were found; the last ones are the delta
+    uint64_t cap = 0, room = 0;  // tuples the log can hold; that may be in it
+    Buf ctl;
+};
+struct DeltaResult {
+    uint64_t rows = 0;      // tuples in the log: what was derived beyond the known rows
+    uint64_t iterations = 0, candidates = 0;
+    bool fix = false;       // an iteration found nothing (else the iteration limit was reached)
+};
+DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits);
+void ops_delta_known(xlb_ctx* c, DeltaLoop& d, const Keys& rows);   // rows the head holds that are not part of the delta
+void ops_delta_seed(xlb_ctx* c, DeltaLoop& d, const Keys& bag);     // candidates: what the head lacks joins it and the delta
+void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows);  // a delta as it is (known to the head already); before any seed
+// To the fixpoint.  `known`: what ops_delta_known was given (unique, disjoint from the seeds).
+// False: a kernel reported a failure (check_dev_status says which).
+bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, uint64_t max_iterations, const Keys& known, DeltaResult* res);
+
 // rows of `bag` whose key has (semi) or lacks (anti) a match in the index, in bag order
 // (pkeys, when given, holds the key word of every bag row instead of a half named by keysel)
 Keys ops_semi_filter(xlb_ctx* c, const Keys& bag, int keysel, const Index& ix, bool anti, const uint64_t* pkeys = nullptr);
