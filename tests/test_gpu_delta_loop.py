@@ -106,3 +106,36 @@ def test_one_column_head_after_the_frontier_loop(monkeypatch):
     # a path longer than the frontier loop follows: the rest of it runs in the delta loop
     got, it, _ = both(programs.reach_from_source(0), {"edge": chain(500)}, "r", monkeypatch)
     assert len(got[0]) == 499 and it == 499
+
+
+@pytest.mark.parametrize("nodes,edges", [(2, 1), (31, 60), (33, 70), (500, 900), (4000, 4200)])
+def test_two_recursive_atoms(nodes, edges, monkeypatch):
+    c = workloads.uniform_digraph(nodes, edges, 5)
+    both(programs.transitive_closure_nonlinear(), {"edge": list(c)}, "reach", monkeypatch)
+
+
+@pytest.mark.parametrize("scale", [0.00001, 0.0001, 0.0004])
+def test_points_to(scale, monkeypatch):
+    rels = {k: list(v) for k, v in workloads.andersen_program(scale, 11).items()}
+    # stored values no derived tuple ever has: beyond the head's domain
+    rels["store"] = [np.append(rels["store"][0], 3).astype(np.uint32), np.append(rels["store"][1], 1 << 20).astype(np.uint32)]
+    got, _, _ = both(programs.andersen(), rels, "pt", monkeypatch)
+    want, _ = O.run_program(programs.andersen(), rels, ["pt"])
+    for g, w in zip(got, want["pt"]):
+        assert np.array_equal(g, w)
+
+
+def test_transposed_partner_and_composed_relation(monkeypatch):
+    # p(X,Z) :- p(X,Y), p(Z,Y), g(X,Z)-free: the partner by its second column; q-shaped: p(Z,Y) :- g(Z,X), p(X,W), p(W,Y)
+    ids = {"e": 0, "g": 1, "p": 2}
+    plan = ExecutionPlan([Scc(0, True, [
+        CompiledRule("p", Scan(0), U2),
+        CompiledRule("p", Project(Join(Scan(2), Scan(2), [1], [1]), [0, 2]), U2),
+        CompiledRule("p", Project(Join(Join(Scan(1), Scan(2), [1], [0]), Scan(2), [3], [0]), [0, 5]), U2)])], ids)
+    rng = np.random.default_rng(9)
+    e = [rng.integers(0, 300, 200).astype(np.uint32) for _ in range(2)]
+    g = [rng.integers(0, 300, 150).astype(np.uint32) for _ in range(2)]
+    got, _, _ = both(plan, {"e": e, "g": g}, "p", monkeypatch)
+    want, _ = O.run_program(plan, {"e": e, "g": g}, ["p"])
+    for a, w in zip(got, want["p"]):
+        assert np.array_equal(a, w)

@@ -45,14 +45,44 @@ struct Rules {
     Rule r[DL_RULES];
     int n;
 };
-enum Phase { PH_ROWS = 0, PH_HEAVY = 1, PH_SOLO = 2, PH_DONE = 3 };
+// Rules with two recursive atoms (`square` components).  The partner of the delta is the head itself as
+// the iteration found it, kept as a bitmap and its transpose: a row of either is the partner's side of
+// the join, 32 candidates a word, and what the head holds already is masked out of it word by word
+// before any single candidate is looked at.
+constexpr int SQ_VARIANTS = 8, SQ_AUX = 2, SQ_UNROLL = 4;
+struct Variant {
+    Ix a;              // list step on a stored relation, keyed on a delta half (a_key), or none (a_key < 0)
+    int a_key;
+    const unsigned int* rows;   // bit rows joined with: the head, its transpose, or a composite
+    int row_key;       // the row: 0 / 1 the delta's high / low half, 2 the list step's value
+    int fixed;         // the output half that does not come from the bit row: 0 / 1 / 2 likewise
+    int bits_are_hi;   // the bit row's value is the output's high half
+    const unsigned long long* counts;  // composite: candidates a row stands for (its bits are a set, the join a bag)
+};
+// Composite of the head with a stored relation joined on the head's column that the output drops:
+// rows[key] = values of the stored rows joined with the head rows of that key.  Kept up to date by
+// the delta's rows.
+struct Composite {
+    Ix ix;
+    int list_key, row_key;  // halves of a head row: 0 high, 1 low
+    unsigned int* rows;
+    unsigned long long* counts;
+};
+struct Square {
+    Variant v[SQ_VARIANTS];
+    Composite aux[SQ_AUX];
+    int n, n_aux;
+    unsigned int *known_t, *full, *full_t;  // transpose of the head's bitmap; the head and its transpose as the iteration found them
+    int bits;                               // of a value
+};
+enum Phase { PH_ROWS = 0, PH_HEAVY = 1, PH_SOLO = 2, PH_DONE = 3, PH_FULL = 4 };
 struct Ctl {
     unsigned long long tail;        // tuples appended to the log so far (may pass its capacity: see overflow)
     unsigned long long start, end;  // the delta at hand: log[start, end)
     unsigned long long iterations, candidates, fix, overflow;
     unsigned long long cand_before; // candidates when the iteration began
     unsigned arrived;               // grid barrier: blocks that wait ...
-    unsigned sync;                  // ... for this word to change: (generation << 2) | phase, always written as one
+    unsigned sync;                  // ... for this word to change: (generation << 3) | phase, always written as one
     unsigned next_chunk;            // rows are taken in chunks
     unsigned heavy_n, next_heavy;
     unsigned abort;
@@ -97,6 +127,7 @@ struct Out {
     uint64_t cap;
     Ctl* ctl;
     DevStatus* st;
+    unsigned int* visited_t;  // square components: the transpose, brought along
 };
 
 // A warp's collected tuples go to the log: one reservation, coalesced stores.
@@ -110,6 +141,11 @@ __device__ __forceinline__ void flush(const Out& o, uint64_t* stage, unsigned& s
         if (at + i < o.cap) __stcg(&o.log[at + i], stage[i]);  // beyond the capacity: found again from the bitmap by the host
     __syncwarp();
     staged = 0;
+}
+
+__device__ __forceinline__ void mark_transposed(const Out& o, uint64_t t) {
+    const uint32_t h = (uint32_t)(t >> 32);
+    atomicOr(&o.visited_t[((uint32_t)t << (o.lo_bits - 5)) | (h >> 5)], 1u << (h & 31));
 }
 
 // What the warp's rows are, lane by lane (lane i: row i).
@@ -168,6 +204,10 @@ __device__ __forceinline__ void emit(const Out& o, const Rule& ru, const Lane& m
             const unsigned bit = 1u << (x[u] & 31);
             on[u] = on[u] && !(word[u] & bit) && !(atomicOr(&o.visited[x[u] >> 5], bit) & bit);
         }
+        if (o.visited_t)
+#pragma unroll
+            for (int u = 0; u < DL_UNROLL; ++u)
+                if (on[u]) mark_transposed(o, tup[u]);
         if (staged + DL_STEP > DL_STAGE) flush(o, stage, staged);
 #pragma unroll
         for (int u = 0; u < DL_UNROLL; ++u) {
@@ -237,6 +277,93 @@ __device__ __forceinline__ void take_rows(const Out& o, const Rules& rules, uint
     }
 }
 
+// One delta row under every variant of the rules with two recursive atoms, by the whole warp.
+__device__ __forceinline__ void square_row(const Out& o, const Square& sq, uint64_t row, uint64_t* stage, unsigned& staged, unsigned long long& cand) {
+    const unsigned lane = lane_id(), row_words = 1u << (sq.bits - 5);
+    for (int q = 0; q < sq.n; ++q) {
+        const Variant& v = sq.v[q];
+        uint32_t s = 0, len = 1;
+        if (v.a_key >= 0) find(v.a, v.a_key == 0 ? (uint32_t)(row >> 32) : (uint32_t)row, s, len);
+        for (uint32_t i = 0; i < len; i += SQ_UNROLL) {
+            uint32_t fixed[SQ_UNROLL];
+            bool on_row[SQ_UNROLL];
+            const unsigned int *from[SQ_UNROLL], *known[SQ_UNROLL];
+#pragma unroll
+            for (int k = 0; k < SQ_UNROLL; ++k) {
+                uint32_t e = 0;
+                if (v.a_key >= 0 && i + k < len) e = other_of(v.a, s + i + k);
+                const uint32_t key = pick(v.row_key, row, e, 0);
+                fixed[k] = pick(v.fixed, row, e, 0);
+                // (a stored value beyond the head's domain has no row in it)
+                on_row[k] = i + k < len && !(key >> sq.bits);
+                if (on_row[k] && fixed[k] >> sq.bits) {
+                    set_status(o.st, XLB_ERR_CAPACITY, 16, fixed[k]);
+                    on_row[k] = false;
+                }
+                from[k] = v.rows + ((uint64_t)key << (sq.bits - 5));
+                known[k] = (v.bits_are_hi ? sq.known_t : o.visited) + ((uint64_t)fixed[k] << (sq.bits - 5));
+                if (v.counts && lane == 0 && on_row[k]) cand += __ldcg(&v.counts[key]);
+            }
+            for (unsigned w0 = 0; w0 < row_words; w0 += 32) {
+                const unsigned w = w0 + lane;
+                unsigned m[SQ_UNROLL];
+#pragma unroll
+                for (int k = 0; k < SQ_UNROLL; ++k) {
+                    m[k] = on_row[k] && w < row_words ? __ldcg(&from[k][w]) : 0u;  // (what the last iteration left: never from the L1)
+                    if (!v.counts) cand += __popc(m[k]);
+                }
+#pragma unroll
+                for (int k = 0; k < SQ_UNROLL; ++k)
+                    if (m[k]) m[k] &= ~known[k][w];  // (a stale line only costs an atomic)
+#pragma unroll
+                for (int k = 0; k < SQ_UNROLL; ++k)
+                    while (__any_sync(FULL, m[k] != 0)) {  // what is left is new, or was found a moment ago
+                        bool on = m[k] != 0;
+                        uint64_t t = 0;
+                        if (on) {
+                            const uint32_t x = (w << 5) | (__ffs(m[k]) - 1);
+                            m[k] &= m[k] - 1;
+                            t = v.bits_are_hi ? ((uint64_t)x << 32) | fixed[k] : ((uint64_t)fixed[k] << 32) | x;
+                            const uint32_t at = ((uint32_t)(t >> 32) << sq.bits) | (uint32_t)t;
+                            const unsigned bit = 1u << (at & 31);
+                            on = !(atomicOr(&o.visited[at >> 5], bit) & bit);
+                            if (on) mark_transposed(o, t);
+                        }
+                        const unsigned b = __ballot_sync(FULL, on);
+                        if (staged + 32 > DL_STAGE) flush(o, stage, staged);
+                        if (on) stage[staged + __popc(b & lanemask_lt())] = t;
+                        staged += __popc(b);
+                        __syncwarp();
+                    }
+            }
+        }
+    }
+}
+// A row of the delta joins the head as the iteration finds it, and the composites over it.
+__device__ __forceinline__ void square_full(const Out& o, const Square& sq, uint64_t row) {
+    const uint32_t h = (uint32_t)(row >> 32), l = (uint32_t)row;
+    atomicOr(&sq.full[(h << (sq.bits - 5)) | (l >> 5)], 1u << (l & 31));
+    atomicOr(&sq.full_t[(l << (sq.bits - 5)) | (h >> 5)], 1u << (h & 31));
+    for (int q = 0; q < sq.n_aux; ++q) {
+        const Composite& x = sq.aux[q];
+        uint32_t s, len;
+        find(x.ix, x.list_key == 0 ? h : l, s, len);
+        if (!len) continue;
+        const uint32_t key = x.row_key == 0 ? h : l;
+        atomicAdd(&x.counts[key], (unsigned long long)len);
+        for (uint32_t i = 0; i < len; ++i) {
+            const uint32_t m = other_of(x.ix, s + i);
+            if (m >> sq.bits) {
+                set_status(o.st, XLB_ERR_CAPACITY, 17, m);
+                continue;
+            }
+            unsigned int* word = &x.rows[(key << (sq.bits - 5)) | (m >> 5)];
+            const unsigned bit = 1u << (m & 31);
+            if (!(__ldcg(word) & bit)) atomicOr(word, bit);
+        }
+    }
+}
+
 // One piece of a long row, by all warps of the block.
 __device__ __forceinline__ void take_piece(const Out& o, const Rules& rules, const Heavy& h, uint64_t* stage, unsigned& staged) {
     if (h.rule >= (unsigned)rules.n) return;
@@ -260,7 +387,7 @@ __device__ __forceinline__ void take_piece(const Out& o, const Rules& rules, con
 
 // The end of an iteration: its new tuples become the delta.  (One thread, everybody else waiting.)
 // Returns what comes next.
-__device__ unsigned next_iteration(const Out& o, uint64_t max_iterations) {
+__device__ unsigned next_iteration(const Out& o, uint64_t max_iterations, bool square) {
     Ctl* c = o.ctl;
     volatile Ctl* v = c;
     const uint64_t tail = v->tail, end = v->end, rows = end - v->start, cands = v->candidates - v->cand_before;
@@ -275,10 +402,12 @@ __device__ unsigned next_iteration(const Out& o, uint64_t max_iterations) {
     if (next == 0) v->fix = 1;
     else if (tail > o.cap) v->overflow = 1;
     if (next == 0 || tail > o.cap || v->iterations >= max_iterations) return PH_DONE;
+    if (square) return PH_FULL;
     return next <= DL_SOLO_ROWS && cands * next <= DL_SOLO_OUTPUTS * rows ? PH_SOLO : PH_ROWS;
 }
 
-__global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules, Heavy* heavy, uint64_t max_iterations) {
+template <bool SQUARE>
+__global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules, Heavy* heavy, uint64_t max_iterations, Square sq) {
     extern __shared__ uint64_t stage_s[];
     __shared__ uint64_t range_s[2];
     __shared__ unsigned phase_s, item_s, go_s;
@@ -294,8 +423,8 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
         if (threadIdx.x == 0) {
             const unsigned w = v->sync;
             __threadfence();
-            generation = w >> 2;
-            phase_s = w & 3;
+            generation = w >> 3;
+            phase_s = w & 7;
             range_s[0] = v->start;
             range_s[1] = v->end;
         }
@@ -303,11 +432,11 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
     };
     auto publish = [&](unsigned phase) {
         __threadfence();
-        v->sync = ((generation + 1) << 2) | phase;
+        v->sync = ((generation + 1) << 3) | phase;
     };
     // Thread 0 waits until the generation has passed; false: it never did.
     auto wait_next = [&]() {
-        for (unsigned polls = 0; v->sync >> 2 == generation; ++polls) {
+        for (unsigned polls = 0; v->sync >> 3 == generation; ++polls) {
             if (polls > DL_SPIN_LIMIT || v->abort) {
                 v->abort = 1;
                 set_status(o.st, XLB_ERR_TIMEOUT, 14, generation);
@@ -347,17 +476,21 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
         if (phase == PH_ROWS) {
             // rows of the delta in chunks: few rows per warp while there are few of them
             const uint64_t warps = (uint64_t)gridDim.x * DL_WARPS;
-            const unsigned per = (unsigned)(n >= warps * 32 ? 32 : (n + warps - 1) / warps);
+            // (a row of a square component can stand for any amount of work: smaller chunks)
+            const unsigned most = SQUARE ? 8 : 32, per = (unsigned)(n >= warps * most ? most : (n + warps - 1) / warps);
             for (uint64_t chunk = (uint64_t)warp * gridDim.x + blockIdx.x; chunk * per < n;) {
                 const uint64_t at = chunk * per;
-                take_rows(o, rules, start + at, (unsigned)(n - at < per ? n - at : per), heavy, stage, staged, cand);
+                const unsigned rows = (unsigned)(n - at < per ? n - at : per);
+                take_rows(o, rules, start + at, rows, heavy, stage, staged, cand);
+                if (SQUARE)
+                    for (unsigned r = 0; r < rows; ++r) square_row(o, sq, __ldcg(&o.log[start + at + r]), stage, staged, cand);
                 if (n <= warps * per) break;
                 unsigned next = 0;
                 if (lane == 0) next = atomicAdd(&ctl->next_chunk, 1u);
                 chunk = warps + __shfl_sync(FULL, next, 0);
             }
             end_warp(cand);
-            if (!barrier([&]() -> unsigned { return v->heavy_n ? (unsigned)PH_HEAVY : next_iteration(o, max_iterations); })) return;
+            if (!barrier([&]() -> unsigned { return v->heavy_n ? (unsigned)PH_HEAVY : next_iteration(o, max_iterations, SQUARE); })) return;
         } else if (phase == PH_HEAVY) {
             const unsigned listed = v->heavy_n, pieces = listed < DL_HEAVY_MAX ? listed : (unsigned)DL_HEAVY_MAX;
             for (;;) {
@@ -373,8 +506,11 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
                 take_piece(o, rules, h, stage, staged);
             }
             end_warp(0);
-            if (!barrier([&] { return next_iteration(o, max_iterations); })) return;
-        } else {  // PH_SOLO
+            if (!barrier([&] { return next_iteration(o, max_iterations, SQUARE); })) return;
+        } else if (SQUARE && phase == PH_FULL) {
+            for (uint64_t i = (uint64_t)blockIdx.x * DL_THREADS + threadIdx.x; i < n; i += (uint64_t)gridDim.x * DL_THREADS) square_full(o, sq, __ldcg(&o.log[start + i]));
+            if (!barrier([&]() -> unsigned { return PH_ROWS; })) return;
+        } else if (!SQUARE) {  // PH_SOLO
             if (blockIdx.x == 0) {
                 const unsigned per = (unsigned)((n + DL_WARPS - 1) / DL_WARPS);  // at most 32 (DL_SOLO_ROWS)
                 if ((uint64_t)warp * per < n) {
@@ -385,7 +521,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
                 __syncthreads();
                 if (threadIdx.x == 0) {
                     __threadfence();
-                    const unsigned next = v->heavy_n ? (unsigned)PH_HEAVY : next_iteration(o, max_iterations);
+                    const unsigned next = v->heavy_n ? (unsigned)PH_HEAVY : next_iteration(o, max_iterations, SQUARE);
                     if (next != PH_SOLO) publish(next);  // everybody again
                 }
             } else {
@@ -416,6 +552,7 @@ __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict
         }
         const unsigned bit = 1u << (at & 31);
         on = on && !(o.visited[at >> 5] & bit) && !(atomicOr(&o.visited[at >> 5], bit) & bit);
+        if (on && o.visited_t) mark_transposed(o, k);
         const unsigned b = __ballot_sync(FULL, on);
         if (on) stage[staged + __popc(b & lanemask_lt())] = k;
         staged += __popc(b);
@@ -425,7 +562,7 @@ __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict
     flush(o, stage, staged);
 }
 
-__global__ void delta_begin_k(Ctl* c) {
+__global__ void delta_begin_k(Ctl* c, bool square) {
     const unsigned long long n = c->tail;
     c->start = 0;
     c->end = n;
@@ -433,30 +570,37 @@ __global__ void delta_begin_k(Ctl* c) {
         c->iterations = 1;
         c->fix = 1;
     }
-    c->sync = n == 0 ? PH_DONE : PH_ROWS;  // (never solo: a block that starts late would miss it)
+    c->sync = n == 0 ? PH_DONE : square ? PH_FULL : PH_ROWS;  // (never solo: a block that starts late would miss it)
 }
 
 // On with the delta at hand, once the log has the room for it.
-__global__ void delta_resume_k(Ctl* c, uint64_t max_iterations) {
+__global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
     c->overflow = 0;
-    c->sync = c->iterations >= max_iterations ? PH_DONE : PH_ROWS;
+    c->sync = c->iterations >= max_iterations ? PH_DONE : square ? PH_FULL : PH_ROWS;
 }
 
 }  // namespace
 
 static Out out_of(xlb_ctx* c, const DeltaLoop& d) {
-    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, d.ctl->as<Ctl>(), c->d_status};
+    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, d.ctl->as<Ctl>(), c->d_status, d.visited_t ? d.visited_t->as<unsigned int>() : nullptr};
 }
 
-DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits) {
+DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square) {
     DeltaLoop d;
     d.hi_bits = hi_bits;
     d.lo_bits = lo_bits;
     d.words = ((1ull << (hi_bits + lo_bits)) + 31) / 32;
-    d.visited = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
+    const uint64_t bytes = std::max<uint64_t>(d.words * 4, 16);
+    d.visited = make_buf(c, bytes);
     d.ctl = make_buf(c, sizeof(Ctl));
-    CUDA_OK(set_async(c, d.visited->p, 0, d.visited->bytes));
+    CUDA_OK(set_async(c, d.visited->p, 0, bytes));
     CUDA_OK(set_async(c, d.ctl->p, 0, sizeof(Ctl)));
+    if (square) {
+        d.visited_t = make_buf(c, bytes);
+        d.full = make_buf(c, 2 * bytes);
+        CUDA_OK(set_async(c, d.visited_t->p, 0, bytes));
+        CUDA_OK(set_async(c, d.full->p, 0, 2 * bytes));
+    }
     return d;
 }
 
@@ -498,10 +642,53 @@ void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows) {
     stream_wait(c);  // (the staging word is used again)
 }
 
-bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, uint64_t max_iterations, const Keys& known, DeltaResult* res) {
-    if (rules.size() > DL_RULES) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules in a delta loop", rules.size());
-    if (!c->delta_attr_set) CUDA_OK(cudaFuncSetAttribute(delta_loop_k, cudaFuncAttributeMaxDynamicSharedMemorySize, DL_WARPS * DL_STAGE * 8));
+static Ix view_of(const Index& ix) {
+    return Ix{ix.cursor ? ix.cursor->as<unsigned long long>() : nullptr, ix.domain, ix.table ? ix.table->as<ulonglong2>() : nullptr, ix.mask,
+              ix.S ? ix.S->as<uint64_t>() : nullptr, ix.pay ? ix.pay->as<uint32_t>() : nullptr};
+}
+
+bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
+                   DeltaResult* res) {
+    if (rules.size() > DL_RULES || variants.size() > SQ_VARIANTS) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules and %zu variants in a delta loop", rules.size(), variants.size());
+    if (!c->delta_attr_set) {
+        CUDA_OK(cudaFuncSetAttribute(delta_loop_k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DL_WARPS * DL_STAGE * 8));
+        CUDA_OK(cudaFuncSetAttribute(delta_loop_k<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DL_WARPS * DL_STAGE * 8));
+    }
     c->delta_attr_set = true;
+    const bool square = d.visited_t != nullptr;
+    Square sq{};
+    std::vector<Buf> composites;
+    if (square) {
+        const uint64_t bytes = d.visited->bytes;
+        sq.bits = d.lo_bits;
+        sq.known_t = d.visited_t->as<unsigned int>();
+        sq.full = d.full->as<unsigned int>();
+        sq.full_t = sq.full + bytes / 4;
+        for (auto& in : variants) {
+            Variant& v = sq.v[sq.n++];
+            v.a_key = in.list ? in.list_key : -1;
+            if (in.list) v.a = view_of(*in.list);
+            v.row_key = in.row_key;
+            v.fixed = in.fixed;
+            v.bits_are_hi = in.bits_are_hi;
+            if (in.rows == DeltaVariant::HEAD) v.rows = sq.full;
+            else if (in.rows == DeltaVariant::HEAD_T) v.rows = sq.full_t;
+            else {
+                if (sq.n_aux == SQ_AUX) xlb_fail(XLB_ERR_INVALID, "internal: too many composites in a delta loop");
+                Buf b = make_buf(c, bytes + (8ull << d.lo_bits));
+                CUDA_OK(set_async(c, b->p, 0, b->bytes));
+                composites.push_back(b);
+                Composite& x = sq.aux[sq.n_aux++];
+                x.ix = view_of(*in.composed);
+                x.list_key = in.composed_list_key;
+                x.row_key = in.composed_row_key;
+                x.rows = b->as<unsigned int>();
+                x.counts = (unsigned long long*)(x.rows + bytes / 4);
+                v.rows = x.rows;
+                v.counts = x.counts;
+            }
+        }
+    }
     log_room(c, d, 0);
     Rules rs{};
     rs.n = (int)rules.size();
@@ -511,21 +698,19 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         r.hi_src = rules[q].hi_src;
         r.lo_src = rules[q].lo_src;
         for (int k = 0; k < r.joins; ++k) {
-            const Index& ix = *rules[q].ix[k];
             r.key_src[k] = rules[q].key_src[k];
-            r.ix[k] = Ix{ix.cursor ? ix.cursor->as<unsigned long long>() : nullptr, ix.domain, ix.table ? ix.table->as<ulonglong2>() : nullptr, ix.mask,
-                         ix.S ? ix.S->as<uint64_t>() : nullptr, ix.pay ? ix.pay->as<uint32_t>() : nullptr};
+            r.ix[k] = view_of(*rules[q].ix[k]);
         }
     }
     Buf heavy = make_buf(c, (uint64_t)DL_HEAVY_MAX * sizeof(Heavy));
-    delta_begin_k<<<1, 1, 0, c->stream>>>(d.ctl->as<Ctl>());
+    delta_begin_k<<<1, 1, 0, c->stream>>>(d.ctl->as<Ctl>(), square);
     check_launch(c, "delta_begin");
     for (;;) {
         Out o = out_of(c, d);
         Heavy* hp = heavy->as<Heavy>();
-        void* args[] = {&o, &rs, &hp, &max_iterations};
+        void* args[] = {&o, &rs, &hp, &max_iterations, &sq};
         prof_begin(c, "expand_mark", 0);
-        CUDA_OK(cudaLaunchCooperativeKernel((const void*)delta_loop_k, dim3((unsigned)c->sm_count), dim3(DL_THREADS), args, (size_t)DL_WARPS * DL_STAGE * 8, c->stream));
+        CUDA_OK(cudaLaunchCooperativeKernel(square ? (const void*)delta_loop_k<true> : (const void*)delta_loop_k<false>, dim3((unsigned)c->sm_count), dim3(DL_THREADS), args, (size_t)DL_WARPS * DL_STAGE * 8, c->stream));
         check_launch(c, "expand_mark");
         unsigned long long w[7];  // tail, start, end, iterations, candidates, fix, overflow
         read_words(c, d.ctl->p, 7, w);
@@ -568,7 +753,7 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         log_room(c, d, tail);
         CUDA_OK(copy_async(c, d.log->as<uint64_t>() + stored, rows.ptr(), rows.n * 8, cudaMemcpyDeviceToDevice));
         d.room = tail;
-        delta_resume_k<<<1, 1, 0, c->stream>>>(d.ctl->as<Ctl>(), max_iterations);
+        delta_resume_k<<<1, 1, 0, c->stream>>>(d.ctl->as<Ctl>(), max_iterations, square);
         check_launch(c, "delta_resume");
     }
 }

@@ -1743,7 +1743,10 @@ static void frontier_loop(xlb_ctx* c, const FrontierPlan& fp, const std::string&
 // ------------------------------------------------------------------------------ delta loop
 // A component of one head whose recursive rules hold one recursive atom each, joined with one or two
 // stored relations on its columns — closure in either direction, same generation, copies — runs to
-// its fixpoint on the device (ops_delta_run).  Heads of up to 32 bits: above the 27 bits that the
+// its fixpoint on the device (ops_delta_run).  So does one whose rules hold two recursive atoms and at
+// most one stored one (points-to analysis, closure by doubling), while values have at most SQUARE_BITS
+// bits: such a rule is evaluated on bit rows of the head, 2^bits / 32 words per delta row and stored
+// match, which at 13 bits is what the launch-by-launch route costs where rows are nearly empty.  Heads of up to 32 bits: above the 27 bits that the
 // launch-by-launch bitmap route starts with, too, since nothing here passes over the whole bitmap per
 // iteration (a clear and one pass to read the result off, 0.3 ms at 2^32).
 struct DeltaPlan {
@@ -1754,10 +1757,86 @@ struct DeltaPlan {
         int kc[2], key_src[2];
         int hi_src, lo_src;
     };
+    // a variant of a rule with two recursive atoms (see DeltaVariant); atom indices, -1: none
+    struct Two {
+        const FlatRule* fr;
+        int list = -1, list_kc = 0, list_key = SRC_HI;
+        DeltaVariant::Rows rows = DeltaVariant::HEAD;
+        int row_key = 0, fixed = 0;
+        bool bits_are_hi = false;
+        int composed = -1, composed_kc = 0, composed_list_key = 0, composed_row_key = 0;
+    };
     std::vector<One> rec;
+    std::vector<Two> square;
     std::vector<const FlatRule*> seeds;
 };
-constexpr size_t DELTA_RULES_MAX = 4;
+constexpr size_t DELTA_RULES_MAX = 4, DELTA_VARIANTS_MAX = 8, DELTA_COMPOSED_MAX = 2;
+constexpr int SQUARE_BITS = 13;
+
+// The variants of a rule with two recursive atoms, the delta at atom `at`.
+static bool square_variant(const FlatRule& fr, size_t at, const std::set<std::string>& rec, DeltaPlan* plan) {
+    const Atom& d = fr.atoms[at];
+    int head = -1, stored = -1;
+    for (size_t i = 0; i < fr.atoms.size(); ++i) {
+        if (i == at) continue;
+        const Atom& a = fr.atoms[i];
+        if (a.arity != 2 || a.var[0] == a.var[1]) return false;
+        int& slot = rec.count(a.rel) ? head : stored;
+        if (slot >= 0) return false;
+        slot = (int)i;
+    }
+    if (head < 0 || fr.head_vars.size() != 2 || d.arity != 2 || d.var[0] == d.var[1]) return false;
+    const Atom& h = fr.atoms[head];
+    auto in_delta = [&](int v) { return v == d.var[0] || v == d.var[1]; };
+    auto delta_half = [&](int v) { return v == d.var[0] ? 0 : 1; };
+    DeltaPlan::Two two;
+    two.fr = &fr;
+    int list_value = -1;  // variable a list step brings
+    const int h_in = (in_delta(h.var[0]) ? 1 : 0) + (in_delta(h.var[1]) ? 1 : 0);
+    if (stored >= 0) {
+        const Atom& s = fr.atoms[stored];
+        const bool s0 = in_delta(s.var[0]), s1 = in_delta(s.var[1]);
+        if (s0 != s1) {  // delta -> stored list
+            two.list = stored;
+            two.list_kc = s0 ? 0 : 1;
+            two.list_key = delta_half(s.var[two.list_kc]) == 0 ? SRC_HI : SRC_LO;
+            list_value = s.var[1 - two.list_kc];
+        } else if (!s0 && !s1 && h_in == 1) {  // delta -> head -> stored: composed
+            const int joined = in_delta(h.var[0]) ? 1 : 0, key = 1 - joined;  // columns of the head atom
+            const int kc = s.var[0] == h.var[joined] ? 0 : s.var[1] == h.var[joined] ? 1 : -1;
+            if (kc < 0) return false;
+            const int out = s.var[1 - kc];
+            for (int v : fr.head_vars)
+                if (v == h.var[joined]) return false;
+            const bool hi = fr.head_vars[0] == out, lo = fr.head_vars[1] == out;
+            if (hi == lo || !in_delta(fr.head_vars[hi ? 1 : 0])) return false;
+            two.rows = DeltaVariant::COMPOSED;
+            two.composed = stored;
+            two.composed_kc = kc;
+            two.composed_list_key = joined;
+            two.composed_row_key = key;
+            two.row_key = delta_half(h.var[key]);
+            two.bits_are_hi = hi;
+            two.fixed = delta_half(fr.head_vars[hi ? 1 : 0]);
+            plan->square.push_back(two);
+            return true;
+        } else return false;
+    }
+    auto bound = [&](int v) { return in_delta(v) || (list_value >= 0 && v == list_value); };
+    const bool b0 = bound(h.var[0]), b1 = bound(h.var[1]);
+    if (b0 == b1) return false;
+    const int key = h.var[b0 ? 0 : 1], bits = h.var[b0 ? 1 : 0];
+    two.rows = b0 ? DeltaVariant::HEAD : DeltaVariant::HEAD_T;
+    two.row_key = in_delta(key) ? delta_half(key) : 2;
+    const bool hi = fr.head_vars[0] == bits, lo = fr.head_vars[1] == bits;
+    if (hi == lo) return false;
+    const int other = fr.head_vars[hi ? 1 : 0];
+    if (!bound(other)) return false;
+    two.bits_are_hi = hi;
+    two.fixed = in_delta(other) ? delta_half(other) : 2;
+    plan->square.push_back(two);
+    return true;
+}
 
 static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const std::vector<std::string>& preds, const std::set<std::string>& rec,
                         const std::map<std::string, xlb_schema>& schema, DeltaPlan* plan) {
@@ -1775,6 +1854,11 @@ static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const st
             if (rec.count(k.rel)) return false;
         if (nrec == 0) {
             plan->seeds.push_back(&fr);
+            continue;
+        }
+        if (nrec == 2 && fr.filters.empty() && fr.checks.empty() && fr.atoms.size() <= 3) {
+            for (size_t i = 0; i < fr.atoms.size(); ++i)
+                if (rec.count(fr.atoms[i].rel) && !square_variant(fr, i, rec, plan)) return false;
             continue;
         }
         if (nrec != 1 || !fr.filters.empty() || !fr.checks.empty() || fr.atoms.size() < 2 || fr.atoms.size() > 3) return false;
@@ -1803,7 +1887,9 @@ static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const st
         if (one.hi_src < 0 || one.lo_src < 0) return false;
         plan->rec.push_back(one);
     }
-    return !plan->rec.empty() && plan->rec.size() <= DELTA_RULES_MAX;
+    size_t composed = 0;
+    for (auto& t : plan->square) composed += t.composed >= 0 ? 1 : 0;
+    return plan->rec.size() + plan->square.size() > 0 && plan->rec.size() <= DELTA_RULES_MAX && plan->square.size() <= DELTA_VARIANTS_MAX && composed <= DELTA_COMPOSED_MAX;
 }
 
 // OR bounds of the head's two halves over everything the component can derive, from the bounds of the
@@ -1855,11 +1941,17 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         }
         uint64_t bound = 0;
         if (!delta_bounds(c, rules, p, rs, full.n ? full.bound : 0, &bound)) return false;
-        const int hb = bit_len(bound >> 32), lb = std::max(bit_len(bound & 0xFFFFFFFFull), 1);
+        int hb = bit_len(bound >> 32), lb = std::max(bit_len(bound & 0xFFFFFFFFull), 1);
+        const bool square = !plan.square.empty();
+        if (square) {
+            // (a head that holds rows already would have to be brought into the transposed bitmaps as well)
+            hb = lb = std::max({hb, lb, 5});
+            if (from_store || hb > SQUARE_BITS) return false;
+        }
         if (hb + lb > WIDE_DENSE_BITS) return false;
         const uint64_t bitmap = (1ull << (hb + lb)) / 8;
-        if (c->budget && c->allocated + 3 * bitmap > c->budget) return false;
-        DeltaLoop d = ops_delta_begin(c, hb, lb);
+        if (c->budget && c->allocated + (square ? 8 : 3) * bitmap > c->budget) return false;
+        DeltaLoop d = ops_delta_begin(c, hb, lb, square);
         if (from_store) {
             PhaseTimer t(c, &rs.st.ms_join);
             ops_delta_append(c, d, delta);
@@ -1906,10 +1998,25 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
             }
             if (!empty) run.push_back(r);
         }
+        std::vector<DeltaVariant> variants;
+        for (auto& two : plan.square) {
+            DeltaVariant v;
+            v.list_key = two.list_key;
+            v.rows = two.rows;
+            v.row_key = two.row_key;
+            v.fixed = two.fixed;
+            v.bits_are_hi = two.bits_are_hi;
+            v.composed_list_key = two.composed_list_key;
+            v.composed_row_key = two.composed_row_key;
+            if (two.list >= 0) v.list = &get_index(c, two.fr->atoms[two.list].rel, two.list_kc, rs);
+            if (two.composed >= 0) v.composed = &get_index(c, two.fr->atoms[two.composed].rel, two.composed_kc, rs);
+            if ((v.list && v.list->n == 0) || (v.composed && v.composed->n == 0)) continue;
+            variants.push_back(v);
+        }
         DeltaResult res;
         {
             PhaseTimer t(c, &rs.st.ms_join);
-            if (!ops_delta_run(c, d, run, c->max_iterations - it, full, &res)) check_dev_status(c);
+            if (!ops_delta_run(c, d, run, variants, c->max_iterations - it, full, &res)) check_dev_status(c);
         }
         it += res.iterations;
         rs.st.iterations += res.iterations;

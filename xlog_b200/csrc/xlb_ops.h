@@ -194,6 +194,19 @@ struct DeltaRule {
     int joins = 1;
     int hi_src = 4, lo_src = 4;         // 0 / 1: the delta row's high / low half, 2 / 3: other column of the first / second match, 4: zero
 };
+// One variant of a rule with two recursive atoms: the delta at one of them, the head as the iteration
+// found it (a bitmap over 2^bits x 2^bits values) at the other.  A stored relation may take part in one of
+// two places: as a list step on a half of the delta row (`list`), or between the head and the output
+// (`composed`: the head's rows joined with it, the joining column dropped).
+struct DeltaVariant {
+    const Index* list = nullptr;
+    int list_key = SRC_HI;     // half of the delta row that probes `list`
+    enum Rows { HEAD, HEAD_T, COMPOSED } rows = HEAD;  // bit rows: low halves of the head by high half, the reverse, or composed
+    int row_key = 0, fixed = 0;  // the bit row's key and the output half that is no bit: 0 / 1 the delta row's high / low half, 2 the list's value
+    bool bits_are_hi = false;    // the bits are the output's high half
+    const Index* composed = nullptr;
+    int composed_list_key = 0, composed_row_key = 0;  // halves of a head row (0 high, 1 low): what probes `composed`, what keys its bit rows
+};
 struct DeltaLoop {
     Buf visited;            // the head as a bitmap
     uint64_t words = 0;
@@ -201,19 +214,22 @@ struct DeltaLoop {
     Buf log;                // derived tuples in the order they were found; the last ones are the delta
     uint64_t cap = 0, room = 0;  // tuples the log can hold; that may be in it
     Buf ctl;
+    Buf visited_t, full;    // square components: the head's transpose; the head and its transpose as an iteration finds them
 };
 struct DeltaResult {
     uint64_t rows = 0;      // tuples in the log: what was derived beyond the known rows
     uint64_t iterations = 0, candidates = 0;
     bool fix = false;       // an iteration found nothing (else the iteration limit was reached)
 };
-DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits);
+// square: for rules with two recursive atoms (hi_bits == lo_bits, at least 5)
+DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square);
 void ops_delta_known(xlb_ctx* c, DeltaLoop& d, const Keys& rows);   // rows the head holds that are not part of the delta
 void ops_delta_seed(xlb_ctx* c, DeltaLoop& d, const Keys& bag);     // candidates: what the head lacks joins it and the delta
 void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows);  // a delta as it is (known to the head already); before any seed
 // To the fixpoint.  `known`: what ops_delta_known was given (unique, disjoint from the seeds).
 // False: a kernel reported a failure (check_dev_status says which).
-bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, uint64_t max_iterations, const Keys& known, DeltaResult* res);
+bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
+                   DeltaResult* res);
 
 // rows of `bag` whose key has (semi) or lacks (anti) a match in the index, in bag order
 // (pkeys, when given, holds the key word of every bag row instead of a half named by keysel)
