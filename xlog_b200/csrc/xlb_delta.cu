@@ -17,13 +17,20 @@ using namespace xk;
 
 namespace {
 
+// (Measured on the cases the comment above names, 32 warps with 2 outputs a lane in flight against 24
+// warps, 16 warps, 4 outputs and 8 outputs: closure 299 us against 320 to 504, banded DAG 935 against
+// 993 to 1503, same generation 779 against 846 to 1300.  The loop is bound by the instructions and the
+// latency of short rows, not by bandwidth: more in flight per warp is work for rows that are not there.)
 constexpr int DL_THREADS = 1024, DL_WARPS = DL_THREADS / 32;
-constexpr int DL_UNROLL = 4, DL_STEP = 32 * DL_UNROLL;   // outputs a warp has in flight
-constexpr int DL_STAGE = 256;                            // new tuples a warp collects before it reserves room in the log
-constexpr unsigned DL_HEAVY = 1024;                      // a row with more outputs than this is shared by a block ...
-constexpr unsigned DL_PIECE = 16384;                     // ... in pieces of this many outputs
-constexpr unsigned DL_HEAVY_MAX = 1u << 16;              // pieces an iteration can list (rows beyond stay with their warp)
-constexpr uint64_t DL_SOLO_ROWS = 1024, DL_SOLO_OUTPUTS = 4096;  // iterations of at most this size run on one block
+constexpr int DL_UNROLL = 2;                             // outputs a lane has in flight
+constexpr int DL_STAGE = 128;                            // new tuples a warp collects before it reserves room in the log
+constexpr unsigned DL_HEAVY = 512;                       // a row with more outputs than this is taken apart
+constexpr unsigned DL_PIECE = 512;                       // ... into pieces that any warp can take
+constexpr unsigned DL_HEAVY_MAX = 1u << 18;              // pieces an iteration can list (rows beyond stay with their warp)
+constexpr uint64_t DL_SOLO_ROWS = 4096, DL_SOLO_OUTPUTS = 8192;  // iterations of at most this size run on one block
+constexpr unsigned SOLO_NEXT = 4096;                     // tuples of a solo iteration that stay in shared memory
+constexpr size_t DL_SMEM = std::max<size_t>((size_t)DL_WARPS * 2 * DL_STAGE * 8, 2 * SOLO_NEXT * 8);
+static_assert(2 * SOLO_NEXT * 8 <= DL_SMEM, "the solo phase uses the warps' stages");
 constexpr unsigned DL_SPIN_LIMIT = 1u << 26;             // polls of a barrier before a block gives up (tens of seconds)
 
 struct Ix {
@@ -31,8 +38,8 @@ struct Ix {
     uint64_t domain;
     const ulonglong2* table;           // hash form
     uint64_t mask;
-    const uint64_t* S;
-    const uint32_t* pay;
+    const uint32_t* other;             // the rows' other column: a payload array, or the low halves of packed rows (step 1)
+    int step;
 };
 struct Rule {
     Ix ix[2];
@@ -53,7 +60,7 @@ constexpr int SQ_VARIANTS = 8, SQ_AUX = 2, SQ_UNROLL = 4;
 struct Variant {
     Ix a;              // list step on a stored relation, keyed on a delta half (a_key), or none (a_key < 0)
     int a_key;
-    const unsigned int* rows;   // bit rows joined with: the head, its transpose, or a composite
+    uint32_t rows;     // bit rows joined with (head, transpose or a composite), as a word offset from the head's bitmap
     int row_key;       // the row: 0 / 1 the delta's high / low half, 2 the list step's value
     int fixed;         // the output half that does not come from the bit row: 0 / 1 / 2 likewise
     int bits_are_hi;   // the bit row's value is the output's high half
@@ -65,15 +72,17 @@ struct Variant {
 struct Composite {
     Ix ix;
     int list_key, row_key;  // halves of a head row: 0 high, 1 low
-    unsigned int* rows;
+    uint32_t rows;
     unsigned long long* counts;
 };
+// Bitmaps of `words` words each, back to back: the head, its transpose, the two as the iteration found
+// them, the composites.
 struct Square {
     Variant v[SQ_VARIANTS];
     Composite aux[SQ_AUX];
     int n, n_aux;
-    unsigned int *known_t, *full, *full_t;  // transpose of the head's bitmap; the head and its transpose as the iteration found them
-    int bits;                               // of a value
+    uint32_t words;
+    int bits;  // of a value
 };
 enum Phase { PH_ROWS = 0, PH_HEAVY = 1, PH_SOLO = 2, PH_DONE = 3, PH_FULL = 4 };
 struct Ctl {
@@ -85,6 +94,7 @@ struct Ctl {
     unsigned sync;                  // ... for this word to change: (generation << 3) | phase, always written as one
     unsigned next_chunk;            // rows are taken in chunks
     unsigned heavy_n, next_heavy;
+    unsigned check;                 // most candidates of the last iteration were known already
     unsigned abort;
 };
 struct Heavy {
@@ -114,7 +124,7 @@ __device__ __forceinline__ void find(const Ix& ix, uint32_t key, uint32_t& start
         h = (h + 1) & ix.mask;
     }
 }
-__device__ __forceinline__ uint32_t other_of(const Ix& ix, uint32_t at) { return ix.pay ? __ldg(&ix.pay[at]) : (uint32_t)__ldg(&ix.S[at]); }
+__device__ __forceinline__ uint32_t other_of(const Ix& ix, uint32_t at) { return __ldg(&ix.other[(uint64_t)at << ix.step]); }
 __device__ __forceinline__ uint32_t pick(int src, uint64_t row, uint32_t m1, uint32_t m2) {
     return src == 0 ? (uint32_t)(row >> 32) : src == 1 ? (uint32_t)row : src == 2 ? m1 : src == 3 ? m2 : 0u;
 }
@@ -130,23 +140,86 @@ struct Out {
     unsigned int* visited_t;  // square components: the transpose, brought along
 };
 
-// A warp's collected tuples go to the log: one reservation, coalesced stores.
-__device__ __forceinline__ void flush(const Out& o, uint64_t* stage, unsigned& staged) {
-    if (!staged) return;
-    unsigned long long at = 0;
-    if (lane_id() == 0) at = atomicAdd(&o.ctl->tail, (unsigned long long)staged);
-    at = __shfl_sync(FULL, at, 0);
-    __syncwarp();
-    for (unsigned i = lane_id(); i < staged; i += 32)
-        if (at + i < o.cap) __stcg(&o.log[at + i], stage[i]);  // beyond the capacity: found again from the bitmap by the host
-    __syncwarp();
-    staged = 0;
-}
-
 __device__ __forceinline__ void mark_transposed(const Out& o, uint64_t t) {
     const uint32_t h = (uint32_t)(t >> 32);
     atomicOr(&o.visited_t[((uint32_t)t << (o.lo_bits - 5)) | (h >> 5)], 1u << (h & 31));
 }
+
+// Where new tuples go.  A warp collects its own in shared memory and reserves room in the log for a
+// batch of them with one atomic add (added one warp step at a time, the queue on that one counter
+// held a same-generation closure at 24 G tuples/s); it does not wait for the reservation, but fills
+// the other half of its stage meanwhile.
+struct WarpSink {
+    const Out& o;
+    uint64_t* stage;  // two halves of DL_STAGE
+    unsigned staged = 0, pending = 0, half = 0;
+    unsigned long long at = 0;  // lane 0: where the pending half goes
+
+    __device__ __forceinline__ void finish() {
+        if (!pending) return;
+        const unsigned long long to = __shfl_sync(FULL, at, 0);
+        const uint64_t* from = stage + (half ^ 1) * DL_STAGE;
+        for (unsigned i = lane_id(); i < pending; i += 32)
+            if (to + i < o.cap) __stcg(&o.log[to + i], from[i]);  // beyond the capacity: found again from the bitmap by the host
+        __syncwarp();
+        pending = 0;
+    }
+    __device__ __forceinline__ void rotate() {
+        finish();
+        if (!staged) return;
+        __syncwarp();
+        if (lane_id() == 0) at = atomicAdd(&o.ctl->tail, (unsigned long long)staged);
+        pending = staged;
+        staged = 0;
+        half ^= 1;
+    }
+    __device__ __forceinline__ void write_left(unsigned long long to) {  // what is staged, to a place somebody else reserved
+        const uint64_t* from = stage + half * DL_STAGE;
+        for (unsigned i = lane_id(); i < staged; i += 32)
+            if (to + i < o.cap) __stcg(&o.log[to + i], from[i]);
+        staged = 0;
+        __syncwarp();
+    }
+    template <int N>
+    __device__ __forceinline__ void push(const bool (&on)[N], const uint64_t (&tup)[N]) {
+        if (staged + 32 * N > DL_STAGE) rotate();
+        uint64_t* to = stage + half * DL_STAGE;
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const unsigned b = __ballot_sync(FULL, on[u]);
+            if (on[u]) to[staged + __popc(b & lanemask_lt())] = tup[u];
+            staged += __popc(b);
+        }
+    }
+};
+// Block 0 alone: the next delta is built in shared memory; the log gets its copy on the side.
+struct SoloSink {
+    const Out& o;
+    uint64_t* next;
+    unsigned* count;
+    uint64_t base;  // the log's tail
+    template <int N>
+    __device__ __forceinline__ void push(const bool (&on)[N], const uint64_t (&tup)[N]) {
+        unsigned b[N], total = 0, at = 0;
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            b[u] = __ballot_sync(FULL, on[u]);
+            total += __popc(b[u]);
+        }
+        if (!total) return;
+        if (lane_id() == 0) at = atomicAdd(count, total);
+        at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const unsigned p = at + __popc(b[u] & lanemask_lt());
+            if (on[u]) {
+                if (p < SOLO_NEXT) next[p] = tup[u];
+                if (base + p < o.cap) __stcg(&o.log[base + p], tup[u]);
+            }
+            at += __popc(b[u]);
+        }
+    }
+};
 
 // What the warp's rows are, lane by lane (lane i: row i).
 struct Lane {
@@ -154,76 +227,95 @@ struct Lane {
     uint32_t s1, s2, l2, before;  // first matches, second join's length, outputs of the rows before
 };
 
-// Outputs [from, to) of the warp's rows: marked, and the new ones collected.  `single`: all of them
-// belong to lane 0's row.
-__device__ __forceinline__ void emit(const Out& o, const Rule& ru, const Lane& me, uint64_t incl, uint64_t from, uint64_t to, bool single, uint64_t* stage, unsigned& staged) {
+// Outputs of the warp's rows: marked, and the new ones handed to the sink.
+//   BALANCED  `count` outputs in all, dealt out over the lanes; `incl`: outputs up to and with lane's row
+//   SINGLE    `count` outputs of lane 0's row, from `first` on
+//   SERIAL    every lane its own row's `incl` outputs, at most `count`: no searching for owners, where
+//             the rows are about equally long
+// `check`: most of what an iteration finds is known already; then a look at the bitmap saves the
+// atomic, else it only delays it.
+enum Deal { BALANCED, SINGLE, SERIAL };
+template <Deal DEAL, int N, class Sink>
+__device__ __forceinline__ void emit(const Out& o, const Rule& ru, const Lane& me, uint32_t incl, uint64_t first, uint32_t count, bool check, Sink& sink) {
     const unsigned lane = lane_id();
-    for (uint64_t base = from; base < to; base += DL_STEP) {
-        uint64_t tup[DL_UNROLL];
-        uint32_t x[DL_UNROLL];
-        bool on[DL_UNROLL];
+    for (uint32_t base = 0; base < count; base += DEAL == SERIAL ? N : 32 * N) {
+        // (every load below is issued whether its lane has an output or not, from a place that exists:
+        // a branch around it would make each wait for the one before)
+        uint64_t tup[N];
+        uint32_t at1[N], at2[N], x[N];
+        bool on[N], bad = false;
 #pragma unroll
-        for (int u = 0; u < DL_UNROLL; ++u) {
-            const uint64_t t = base + u * 32 + lane;
-            on[u] = t < to;
-            int owner = 0;
-            if (!single) {  // the row whose outputs hold t: rows before it end at or before t
+        for (int u = 0; u < N; ++u) {
+            const uint32_t t = DEAL == SERIAL ? base + u : base + u * 32 + lane;
+            on[u] = t < (DEAL == SERIAL ? incl : count);
+            int owner = DEAL == SERIAL ? (int)lane : 0;
+            if (DEAL == BALANCED) {  // the row whose outputs hold t: rows before it end at or before t
 #pragma unroll
-                for (int d = 16; d; d >>= 1) {
-                    const uint64_t end = __shfl_sync(FULL, incl, owner + d - 1);
-                    if (end <= t) owner += d;
-                }
+                for (int d = 16; d; d >>= 1)
+                    if (__shfl_sync(FULL, incl, owner + d - 1) <= t) owner += d;
             }
-            const uint64_t row = __shfl_sync(FULL, me.row, owner);
-            const uint32_t s1 = __shfl_sync(FULL, me.s1, owner);
-            const uint32_t before = single ? 0u : __shfl_sync(FULL, me.before, owner);
-            uint32_t m1 = 0, m2 = 0;
+            tup[u] = DEAL == SERIAL ? me.row : __shfl_sync(FULL, me.row, owner);
+            const uint32_t s1 = DEAL == SERIAL ? me.s1 : __shfl_sync(FULL, me.s1, owner);
+            const uint64_t j = DEAL == SINGLE ? first + t : DEAL == SERIAL ? t : (uint64_t)(t - __shfl_sync(FULL, me.before, owner));
+            at1[u] = s1 + (uint32_t)j;
+            at2[u] = 0;
             if (ru.joins == 2) {
-                const uint32_t s2 = __shfl_sync(FULL, me.s2, owner), l2 = __shfl_sync(FULL, me.l2, owner);
-                if (on[u]) {
-                    const uint64_t j = t - before;
-                    const uint32_t a = j >> 32 ? (uint32_t)(j / l2) : (uint32_t)j / l2, b = (uint32_t)(j - (uint64_t)a * l2);
-                    m1 = other_of(ru.ix[0], s1 + a);
-                    m2 = other_of(ru.ix[1], s2 + b);
-                }
-            } else if (on[u]) m1 = other_of(ru.ix[0], s1 + (uint32_t)(t - before));
-            const uint32_t h = pick(ru.hi_src, row, m1, m2), l = pick(ru.lo_src, row, m1, m2);
+                const uint32_t s2 = DEAL == SERIAL ? me.s2 : __shfl_sync(FULL, me.s2, owner), l2 = max(DEAL == SERIAL ? me.l2 : __shfl_sync(FULL, me.l2, owner), 1u);
+                const uint32_t a = DEAL == SINGLE && j >> 32 ? (uint32_t)(j / l2) : (uint32_t)j / l2, b = (uint32_t)(j - (uint64_t)a * l2);
+                at1[u] = s1 + a;
+                at2[u] = s2 + b;
+            }
+            if (!on[u]) at1[u] = at2[u] = 0;
+        }
+        uint32_t m1[N], m2[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) m1[u] = other_of(ru.ix[0], at1[u]);
+#pragma unroll
+        for (int u = 0; u < N; ++u) m2[u] = ru.joins == 2 ? other_of(ru.ix[1], at2[u]) : 0u;
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const uint32_t h = pick(ru.hi_src, tup[u], m1[u], m2[u]), l = pick(ru.lo_src, tup[u], m1[u], m2[u]);
             tup[u] = ((uint64_t)h << 32) | l;
             const uint64_t at = ((uint64_t)h << o.lo_bits) | l;
             x[u] = (uint32_t)at;
-            if (on[u] && ((uint64_t)l >> o.lo_bits || (at >> 5) >= o.words)) {
-                set_status(o.st, XLB_ERR_CAPACITY, 13, tup[u]);  // outside the domain the host derived: report, never write
-                on[u] = false;
-            }
+            const bool outside = (uint64_t)l >> o.lo_bits || (at >> 5) >= o.words;
+            bad |= on[u] && outside;
+            on[u] = on[u] && !outside;
+            if (!on[u]) x[u] = 0;
         }
-        unsigned word[DL_UNROLL];
+        if (bad) set_status(o.st, XLB_ERR_CAPACITY, 13, tup[0]);  // outside the domain the host derived: reported, never written
+        if (check) {
+            unsigned word[N];
 #pragma unroll
-        for (int u = 0; u < DL_UNROLL; ++u) word[u] = on[u] ? o.visited[x[u] >> 5] : 0xFFFFFFFFu;  // (a stale line only costs an atomic)
+            for (int u = 0; u < N; ++u) word[u] = o.visited[x[u] >> 5];  // (a stale line only costs an atomic)
 #pragma unroll
-        for (int u = 0; u < DL_UNROLL; ++u) {
-            const unsigned bit = 1u << (x[u] & 31);
-            on[u] = on[u] && !(word[u] & bit) && !(atomicOr(&o.visited[x[u] >> 5], bit) & bit);
+            for (int u = 0; u < N; ++u) on[u] = on[u] && !((word[u] >> (x[u] & 31)) & 1u);
         }
+        unsigned old[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            old[u] = 0;
+            if (on[u]) old[u] = atomicOr(&o.visited[x[u] >> 5], 1u << (x[u] & 31));
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) on[u] = on[u] && !((old[u] >> (x[u] & 31)) & 1u);
         if (o.visited_t)
 #pragma unroll
-            for (int u = 0; u < DL_UNROLL; ++u)
+            for (int u = 0; u < N; ++u)
                 if (on[u]) mark_transposed(o, tup[u]);
-        if (staged + DL_STEP > DL_STAGE) flush(o, stage, staged);
-#pragma unroll
-        for (int u = 0; u < DL_UNROLL; ++u) {
-            const unsigned b = __ballot_sync(FULL, on[u]);
-            if (on[u]) stage[staged + __popc(b & lanemask_lt())] = tup[u];
-            staged += __popc(b);
-        }
-        __syncwarp();
+        sink.push(on, tup);
     }
 }
 
-// Rows log[at, at + rows) of the delta (rows <= 32) under every rule.
-__device__ __forceinline__ void take_rows(const Out& o, const Rules& rules, uint64_t at, unsigned rows, Heavy* heavy, uint64_t* stage, unsigned& staged, unsigned long long& cand) {
+// The warp's rows (lane i < rows: me_row of the delta) under every rule with one recursive atom.
+// `cand` += this lane's candidates (at most 512 a row and rule; those of longer rows are counted
+// in global memory).  Returns whether a long row was listed in pieces.
+template <class Sink>
+__device__ __forceinline__ bool take_rows(const Out& o, const Rules& rules, uint64_t me_row, unsigned rows, Heavy* heavy, bool check, Sink& sink, unsigned& cand) {
     const unsigned lane = lane_id();
+    bool any_listed = false;
     Lane me;
-    me.row = lane < rows ? __ldcg(&o.log[at + lane]) : 0;
+    me.row = me_row;
     for (int q = 0; q < rules.n; ++q) {
         const Rule& ru = rules.r[q];
         uint32_t l1 = 0;
@@ -237,8 +329,9 @@ __device__ __forceinline__ void take_rows(const Out& o, const Rules& rules, uint
                 cnt *= me.l2;
             }
         }
-        cand += cnt;
-        // long rows: listed for whole blocks; one that finds the list full stays here
+        if (cnt <= DL_HEAVY) cand += (unsigned)cnt;
+        else atomicAdd(&o.ctl->candidates, (unsigned long long)cnt);
+        // long rows: listed in pieces; one that finds the list full stays here
         unsigned alone = 0;
         if (cnt > DL_HEAVY) {
             const uint64_t pieces = (cnt + DL_PIECE - 1) / DL_PIECE;
@@ -252,18 +345,26 @@ __device__ __forceinline__ void take_rows(const Out& o, const Rules& rules, uint
                     for (unsigned k = h; k < DL_HEAVY_MAX; ++k) heavy[k] = {0, ~0u, 0};  // the room that was left: nothing to do there
                 }
             }
+            any_listed = true;  // (the count was raised either way)
             if (!listed) alone = 1;
         }
-        const uint64_t mine = cnt > DL_HEAVY ? 0 : cnt;
-        uint64_t incl = mine;
+        const uint32_t mine = cnt > DL_HEAVY ? 0 : (uint32_t)cnt, longest = __reduce_max_sync(FULL, mine), total = __reduce_add_sync(FULL, mine);
+        if (longest <= 1) {
+            if (longest) emit<SERIAL, 1>(o, ru, me, mine, 0, 1, check, sink);
+        } else if (longest * 16 <= total) {  // at least half of the lanes' steps would bring an output
+            emit<SERIAL, DL_UNROLL>(o, ru, me, mine, 0, longest, check, sink);
+        } else if (rows == 1) {
+            emit<SINGLE, DL_UNROLL>(o, ru, me, 0, 0, total, check, sink);
+        } else {
+            uint32_t incl = mine;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint64_t v = __shfl_up_sync(FULL, incl, d);
-            if (lane >= (unsigned)d) incl += v;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(FULL, incl, d);
+                if (lane >= (unsigned)d) incl += v;
+            }
+            me.before = incl - mine;
+            emit<BALANCED, DL_UNROLL>(o, ru, me, incl, 0, total, check, sink);
         }
-        me.before = (uint32_t)(incl - mine);
-        const uint64_t total = __shfl_sync(FULL, incl, 31);
-        if (total) emit(o, ru, me, incl, 0, total, rows == 1, stage, staged);
         for (unsigned left = __ballot_sync(FULL, alone); left; left &= left - 1) {
             const int r = __ffs(left) - 1;
             Lane one;
@@ -272,100 +373,15 @@ __device__ __forceinline__ void take_rows(const Out& o, const Rules& rules, uint
             one.s2 = __shfl_sync(FULL, me.s2, r);
             one.l2 = __shfl_sync(FULL, me.l2, r);
             one.before = 0;
-            emit(o, ru, one, 0, 0, __shfl_sync(FULL, cnt, r), true, stage, staged);
+            const uint64_t all = __shfl_sync(FULL, cnt, r);
+            for (uint64_t at = 0; at < all; at += 1u << 30) emit<SINGLE, DL_UNROLL>(o, ru, one, 0, at, (uint32_t)(all - at < (1u << 30) ? all - at : 1u << 30), check, sink);
         }
     }
+    return any_listed;
 }
 
-// One delta row under every variant of the rules with two recursive atoms, by the whole warp.
-__device__ __forceinline__ void square_row(const Out& o, const Square& sq, uint64_t row, uint64_t* stage, unsigned& staged, unsigned long long& cand) {
-    const unsigned lane = lane_id(), row_words = 1u << (sq.bits - 5);
-    for (int q = 0; q < sq.n; ++q) {
-        const Variant& v = sq.v[q];
-        uint32_t s = 0, len = 1;
-        if (v.a_key >= 0) find(v.a, v.a_key == 0 ? (uint32_t)(row >> 32) : (uint32_t)row, s, len);
-        for (uint32_t i = 0; i < len; i += SQ_UNROLL) {
-            uint32_t fixed[SQ_UNROLL];
-            bool on_row[SQ_UNROLL];
-            const unsigned int *from[SQ_UNROLL], *known[SQ_UNROLL];
-#pragma unroll
-            for (int k = 0; k < SQ_UNROLL; ++k) {
-                uint32_t e = 0;
-                if (v.a_key >= 0 && i + k < len) e = other_of(v.a, s + i + k);
-                const uint32_t key = pick(v.row_key, row, e, 0);
-                fixed[k] = pick(v.fixed, row, e, 0);
-                // (a stored value beyond the head's domain has no row in it)
-                on_row[k] = i + k < len && !(key >> sq.bits);
-                if (on_row[k] && fixed[k] >> sq.bits) {
-                    set_status(o.st, XLB_ERR_CAPACITY, 16, fixed[k]);
-                    on_row[k] = false;
-                }
-                from[k] = v.rows + ((uint64_t)key << (sq.bits - 5));
-                known[k] = (v.bits_are_hi ? sq.known_t : o.visited) + ((uint64_t)fixed[k] << (sq.bits - 5));
-                if (v.counts && lane == 0 && on_row[k]) cand += __ldcg(&v.counts[key]);
-            }
-            for (unsigned w0 = 0; w0 < row_words; w0 += 32) {
-                const unsigned w = w0 + lane;
-                unsigned m[SQ_UNROLL];
-#pragma unroll
-                for (int k = 0; k < SQ_UNROLL; ++k) {
-                    m[k] = on_row[k] && w < row_words ? __ldcg(&from[k][w]) : 0u;  // (what the last iteration left: never from the L1)
-                    if (!v.counts) cand += __popc(m[k]);
-                }
-#pragma unroll
-                for (int k = 0; k < SQ_UNROLL; ++k)
-                    if (m[k]) m[k] &= ~known[k][w];  // (a stale line only costs an atomic)
-#pragma unroll
-                for (int k = 0; k < SQ_UNROLL; ++k)
-                    while (__any_sync(FULL, m[k] != 0)) {  // what is left is new, or was found a moment ago
-                        bool on = m[k] != 0;
-                        uint64_t t = 0;
-                        if (on) {
-                            const uint32_t x = (w << 5) | (__ffs(m[k]) - 1);
-                            m[k] &= m[k] - 1;
-                            t = v.bits_are_hi ? ((uint64_t)x << 32) | fixed[k] : ((uint64_t)fixed[k] << 32) | x;
-                            const uint32_t at = ((uint32_t)(t >> 32) << sq.bits) | (uint32_t)t;
-                            const unsigned bit = 1u << (at & 31);
-                            on = !(atomicOr(&o.visited[at >> 5], bit) & bit);
-                            if (on) mark_transposed(o, t);
-                        }
-                        const unsigned b = __ballot_sync(FULL, on);
-                        if (staged + 32 > DL_STAGE) flush(o, stage, staged);
-                        if (on) stage[staged + __popc(b & lanemask_lt())] = t;
-                        staged += __popc(b);
-                        __syncwarp();
-                    }
-            }
-        }
-    }
-}
-// A row of the delta joins the head as the iteration finds it, and the composites over it.
-__device__ __forceinline__ void square_full(const Out& o, const Square& sq, uint64_t row) {
-    const uint32_t h = (uint32_t)(row >> 32), l = (uint32_t)row;
-    atomicOr(&sq.full[(h << (sq.bits - 5)) | (l >> 5)], 1u << (l & 31));
-    atomicOr(&sq.full_t[(l << (sq.bits - 5)) | (h >> 5)], 1u << (h & 31));
-    for (int q = 0; q < sq.n_aux; ++q) {
-        const Composite& x = sq.aux[q];
-        uint32_t s, len;
-        find(x.ix, x.list_key == 0 ? h : l, s, len);
-        if (!len) continue;
-        const uint32_t key = x.row_key == 0 ? h : l;
-        atomicAdd(&x.counts[key], (unsigned long long)len);
-        for (uint32_t i = 0; i < len; ++i) {
-            const uint32_t m = other_of(x.ix, s + i);
-            if (m >> sq.bits) {
-                set_status(o.st, XLB_ERR_CAPACITY, 17, m);
-                continue;
-            }
-            unsigned int* word = &x.rows[(key << (sq.bits - 5)) | (m >> 5)];
-            const unsigned bit = 1u << (m & 31);
-            if (!(__ldcg(word) & bit)) atomicOr(word, bit);
-        }
-    }
-}
-
-// One piece of a long row, by all warps of the block.
-__device__ __forceinline__ void take_piece(const Out& o, const Rules& rules, const Heavy& h, uint64_t* stage, unsigned& staged) {
+// One piece of a long row.
+__device__ __forceinline__ void take_piece(const Out& o, const Rules& rules, const Heavy& h, bool check, WarpSink& sink) {
     if (h.rule >= (unsigned)rules.n) return;
     const Rule& ru = rules.r[h.rule];
     Lane me;
@@ -379,18 +395,165 @@ __device__ __forceinline__ void take_piece(const Out& o, const Rules& rules, con
         find(ru.ix[1], ru.key_src[1] == 0 ? (uint32_t)(me.row >> 32) : (uint32_t)me.row, me.s2, me.l2);
         cnt *= me.l2;
     }
-    const uint64_t lo = (uint64_t)h.piece * DL_PIECE, hi = lo + DL_PIECE < cnt ? lo + DL_PIECE : cnt;
-    const uint64_t per = ((hi - lo + DL_WARPS - 1) / DL_WARPS + 31) & ~31ull;
-    const uint64_t from = lo + (threadIdx.x >> 5) * per, to = from + per < hi ? from + per : hi;
-    if (from < to) emit(o, ru, me, 0, from, to, true, stage, staged);
+    const uint64_t from = (uint64_t)h.piece * DL_PIECE;
+    if (from < cnt) emit<SINGLE, DL_UNROLL>(o, ru, me, 0, from, (uint32_t)(cnt - from < DL_PIECE ? cnt - from : DL_PIECE), check, sink);
+}
+
+// The warp's rows (lane i < rows: me_row) under every variant of the rules with two recursive atoms.  A variant
+// of a row stands for one bit row per stored match (or for one).  The warp looks the matches up
+// lane by lane for all rows and variants at once, then takes the bit rows SQ_UNROLL at a time, two
+// words per lane: what a single row costs is the latency of its loads, so they are kept in flight.
+__device__ __forceinline__ void take_square(const Out& o, const Square& sq, uint64_t me_row, unsigned rows, WarpSink& sink, unsigned long long& cand) {
+    const unsigned lane = lane_id(), shift = sq.bits - 5, row_words = 1u << shift, work = rows * sq.n;
+    const unsigned int* bits = o.visited;
+    for (unsigned t0 = 0; t0 < work; t0 += 32) {
+        const unsigned t = t0 + lane;
+        const uint64_t row = __shfl_sync(FULL, me_row, t / sq.n);
+        unsigned q = 0;
+        uint32_t s = 0, len = 0;
+        if (t < work) {
+            q = t % sq.n;
+            len = 1;
+            if (sq.v[q].a_key >= 0) find(sq.v[q].a, sq.v[q].a_key == 0 ? (uint32_t)(row >> 32) : (uint32_t)row, s, len);
+        }
+        uint64_t incl = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t v = __shfl_up_sync(FULL, incl, d);
+            if (lane >= (unsigned)d) incl += v;
+        }
+        const uint64_t total = __shfl_sync(FULL, incl, 31), before = incl - len;
+        for (uint64_t i0 = 0; i0 < total; i0 += 32) {
+            const uint64_t i = i0 + lane;
+            int owner = 0;
+#pragma unroll
+            for (int d = 16; d; d >>= 1)
+                if (__shfl_sync(FULL, incl, owner + d - 1) <= i) owner += d;
+            const uint64_t r = __shfl_sync(FULL, row, owner);
+            const unsigned vq = __shfl_sync(FULL, q, owner);
+            const uint32_t from_s = __shfl_sync(FULL, s, owner);
+            const uint64_t from_before = __shfl_sync(FULL, before, owner);
+            bool ok = i < total;
+            uint32_t from = 0, known = 0;
+            if (ok) {
+                const Variant& v = sq.v[vq];
+                const uint32_t e = v.a_key >= 0 ? other_of(v.a, from_s + (uint32_t)(i - from_before)) : 0;
+                const uint32_t key = pick(v.row_key, r, e, 0), fixed = pick(v.fixed, r, e, 0);
+                ok = !(key >> sq.bits);  // (a stored value beyond the head's domain has no row in it)
+                if (ok && fixed >> sq.bits) {
+                    set_status(o.st, XLB_ERR_CAPACITY, 16, fixed);
+                    ok = false;
+                }
+                from = v.rows + (key << shift);
+                known = (v.bits_are_hi ? sq.words : 0u) + (fixed << shift);
+                if (ok && v.counts) cand += __ldcg(&v.counts[key]);
+            }
+            for (unsigned left = __ballot_sync(FULL, ok); left;) {
+                uint32_t f[SQ_UNROLL], kn[SQ_UNROLL];
+                int items = 0;
+#pragma unroll
+                for (int k = 0; k < SQ_UNROLL; ++k) {
+                    const int src = left ? __ffs(left) - 1 : 0;
+                    items += left ? 1 : 0;
+                    f[k] = __shfl_sync(FULL, from, src);
+                    kn[k] = __shfl_sync(FULL, known, src);
+                    left &= left - 1;
+                }
+                for (unsigned w0 = 0; w0 < row_words; w0 += 64) {
+                    const unsigned w = w0 + 2 * lane;
+                    uint64_t m[SQ_UNROLL], have[SQ_UNROLL];
+#pragma unroll
+                    for (int k = 0; k < SQ_UNROLL; ++k) {
+                        const bool in = k < items && w < row_words;
+                        m[k] = in ? __ldcg(reinterpret_cast<const unsigned long long*>(bits + f[k] + w)) : 0ull;  // (what the last iteration left: never from the L1)
+                        have[k] = in ? *reinterpret_cast<const unsigned long long*>(bits + kn[k] + w) : 0ull;     // (a stale line only costs an atomic)
+                    }
+                    uint64_t any = 0;
+#pragma unroll
+                    for (int k = 0; k < SQ_UNROLL; ++k) {
+                        if (f[k] < 4 * sq.words) cand += __popcll(m[k]);
+                        m[k] &= ~have[k];
+                        any |= m[k];
+                    }
+                    while (__any_sync(FULL, any != 0)) {  // what is left is new, or was found a moment ago
+                        // a few bits of one word per lane and turn: their atomics are in flight together
+                        bool on[SQ_UNROLL];
+                        uint64_t tup[SQ_UNROLL];
+                        uint64_t mine = 0;
+                        uint32_t where = 0;
+#pragma unroll
+                        for (int k = SQ_UNROLL - 1; k >= 0; --k)
+                            if (m[k]) {
+                                mine = m[k];
+                                where = kn[k];
+                            }
+                        const bool hi = where >= sq.words;
+                        const uint32_t fixed = (hi ? where - sq.words : where) >> shift;
+                        unsigned old[SQ_UNROLL];
+                        uint64_t rest = mine;
+#pragma unroll
+                        for (int u = 0; u < SQ_UNROLL; ++u) {
+                            on[u] = rest != 0;
+                            const uint32_t x = (w << 5) + (on[u] ? __ffsll(rest) - 1 : 0);
+                            rest &= rest - 1;
+                            tup[u] = hi ? ((uint64_t)x << 32) | fixed : ((uint64_t)fixed << 32) | x;
+                            const uint32_t b = ((uint32_t)(tup[u] >> 32) << sq.bits) | (uint32_t)tup[u];
+                            old[u] = ~0u;
+                            if (on[u]) old[u] = atomicOr(&o.visited[b >> 5], 1u << (b & 31));
+                        }
+#pragma unroll
+                        for (int u = 0; u < SQ_UNROLL; ++u) {
+                            on[u] = on[u] && !((old[u] >> (hi ? fixed & 31 : (uint32_t)tup[u] & 31)) & 1u);
+                            if (on[u]) mark_transposed(o, tup[u]);
+                        }
+                        bool taken = mine == 0;
+                        any = 0;
+#pragma unroll
+                        for (int k = 0; k < SQ_UNROLL; ++k) {
+                            if (!taken && m[k]) {
+                                m[k] = rest;
+                                taken = true;
+                            }
+                            any |= m[k];
+                        }
+                        sink.push(on, tup);
+                    }
+                }
+            }
+        }
+    }
+}
+// A row of the delta joins the head as the iteration finds it, and the composites over it.
+__device__ __forceinline__ void square_full(const Out& o, const Square& sq, uint64_t row) {
+    const uint32_t h = (uint32_t)(row >> 32), l = (uint32_t)row, shift = sq.bits - 5;
+    atomicOr(&o.visited[2 * sq.words + ((h << shift) | (l >> 5))], 1u << (l & 31));
+    atomicOr(&o.visited[3 * sq.words + ((l << shift) | (h >> 5))], 1u << (h & 31));
+    for (int q = 0; q < sq.n_aux; ++q) {
+        const Composite& x = sq.aux[q];
+        uint32_t s, len;
+        find(x.ix, x.list_key == 0 ? h : l, s, len);
+        if (!len) continue;
+        const uint32_t key = x.row_key == 0 ? h : l;
+        atomicAdd(&x.counts[key], (unsigned long long)len);
+        for (uint32_t i = 0; i < len; ++i) {
+            const uint32_t m = other_of(x.ix, s + i);
+            if (m >> sq.bits) {
+                set_status(o.st, XLB_ERR_CAPACITY, 17, m);
+                continue;
+            }
+            unsigned int* word = &o.visited[x.rows + ((key << shift) | (m >> 5))];
+            const unsigned bit = 1u << (m & 31);
+            if (!(__ldcg(word) & bit)) atomicOr(word, bit);
+        }
+    }
 }
 
 // The end of an iteration: its new tuples become the delta.  (One thread, everybody else waiting.)
 // Returns what comes next.
 __device__ unsigned next_iteration(const Out& o, uint64_t max_iterations, bool square) {
-    Ctl* c = o.ctl;
-    volatile Ctl* v = c;
+    volatile Ctl* v = o.ctl;
     const uint64_t tail = v->tail, end = v->end, rows = end - v->start, cands = v->candidates - v->cand_before;
+    const uint64_t next = tail - end;
     v->iterations = v->iterations + 1;
     v->cand_before = v->candidates;
     v->start = end;
@@ -398,7 +561,7 @@ __device__ unsigned next_iteration(const Out& o, uint64_t max_iterations, bool s
     v->next_chunk = 0;
     v->heavy_n = 0;
     v->next_heavy = 0;
-    const uint64_t next = tail - end;
+    v->check = next * 2 < cands;
     if (next == 0) v->fix = 1;
     else if (tail > o.cap) v->overflow = 1;
     if (next == 0 || tail > o.cap || v->iterations >= max_iterations) return PH_DONE;
@@ -406,14 +569,92 @@ __device__ unsigned next_iteration(const Out& o, uint64_t max_iterations, bool s
     return next <= DL_SOLO_ROWS && cands * next <= DL_SOLO_OUTPUTS * rows ? PH_SOLO : PH_ROWS;
 }
 
+// Small iterations, by block 0 alone while the others wait: the delta, the next one and the counts
+// stay in shared memory, one block barrier per iteration.  Returns the phase that needs all blocks.
+struct SoloShared {
+    unsigned count[3], cand[3], listed;
+};
+__device__ __forceinline__ unsigned solo(const Out& o, const Rules& rules, Heavy* heavy, uint64_t max_iterations, uint64_t* buf, SoloShared& sh, uint64_t start, uint64_t base) {
+    volatile Ctl* v = o.ctl;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    unsigned n = (unsigned)(base - start), cur = 0;
+    bool thin = true;  // about one output a row: as few warps as hold the rows, each pays the whole chain of instructions
+    uint64_t iterations = v->iterations, before = 0;  // (candidates of the iterations that are over)
+    if (threadIdx.x < 3) {
+        sh.count[threadIdx.x] = 0;
+        sh.cand[threadIdx.x] = 0;
+    }
+    if (threadIdx.x == 0) sh.listed = 0;
+    for (unsigned i = threadIdx.x; i < n; i += DL_THREADS) buf[i] = __ldcg(&o.log[start + i]);
+    __syncthreads();
+    for (unsigned turn = 0;; turn = turn == 2 ? 0 : turn + 1) {
+        const unsigned after = turn == 2 ? 0 : turn + 1;  // (its counters were read last two barriers ago)
+        if (threadIdx.x == 0) {
+            sh.count[after] = 0;
+            sh.cand[after] = 0;
+        }
+        const unsigned per = thin || n >= DL_THREADS ? 32 : (n + DL_WARPS - 1) / DL_WARPS;
+        unsigned cand = 0;
+        for (unsigned at = warp * per; at < n; at += DL_WARPS * per) {
+            const unsigned rows = n - at < per ? n - at : per;
+            SoloSink sink{o, buf + (cur ^ 1) * SOLO_NEXT, &sh.count[turn], base};
+            if (take_rows(o, rules, lane < rows ? buf[cur * SOLO_NEXT + at + lane] : 0, rows, heavy, false, sink, cand)) sh.listed = 1;
+        }
+        cand = __reduce_add_sync(FULL, cand);
+        if (lane == 0 && cand) atomicAdd(&sh.cand[turn], cand);
+        __syncthreads();
+        const unsigned next = sh.count[turn];
+        const uint64_t cands = sh.cand[turn];
+        const uint64_t tail = base + next;
+        unsigned phase = PH_SOLO;
+        if (sh.listed) phase = PH_HEAVY;  // the iteration is not over
+        else {
+            ++iterations;
+            if (next == 0 || tail > o.cap || iterations >= max_iterations) phase = PH_DONE;
+            else if (next > DL_SOLO_ROWS || cands * next > DL_SOLO_OUTPUTS * n) phase = PH_ROWS;
+        }
+        if (phase != PH_SOLO) {
+            if (threadIdx.x == 0) {
+                v->tail = tail;
+                v->iterations = iterations;
+                const unsigned long long listed = v->candidates;  // what long rows have added
+                v->candidates = listed + before + cands;
+                if (phase == PH_HEAVY) {
+                    v->start = start;
+                    v->end = base;
+                    v->cand_before = v->cand_before + before;
+                } else {
+                    v->start = base;
+                    v->end = tail;
+                    v->cand_before = listed + before + cands;
+                    v->next_chunk = 0;
+                    v->check = next * 2ull < cands;
+                    if (next == 0) v->fix = 1;
+                    else if (tail > o.cap) v->overflow = 1;
+                }
+            }
+            return phase;
+        }
+        before += cands;
+        thin = cands <= 2ull * n;
+        start = base;
+        base = tail;
+        n = next;
+        cur ^= 1;
+    }
+}
+
 template <bool SQUARE>
-__global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules, Heavy* heavy, uint64_t max_iterations, Square sq) {
+__global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const __grid_constant__ Rules rules, Heavy* heavy, uint64_t max_iterations, const __grid_constant__ Square sq) {
     extern __shared__ uint64_t stage_s[];
     __shared__ uint64_t range_s[2];
-    __shared__ unsigned phase_s, item_s, go_s;
+    __shared__ unsigned phase_s, go_s, check_s;
+    __shared__ SoloShared solo_s;
+    __shared__ unsigned left_s[32];
+    __shared__ unsigned long long cand_s[32];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    uint64_t* stage = stage_s + warp * DL_STAGE;
-    unsigned staged = 0, generation = 0;
+    WarpSink sink{o, stage_s + warp * (2 * DL_STAGE)};
+    unsigned generation = 0;
     Ctl* ctl = o.ctl;
     volatile Ctl* v = ctl;
     // What thread 0 has seen of the sync word.  Between a barrier and the next, a solo phase may begin
@@ -427,6 +668,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
             phase_s = w & 7;
             range_s[0] = v->start;
             range_s[1] = v->end;
+            check_s = v->check;
         }
         __syncthreads();
     };
@@ -461,69 +703,106 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
         __syncthreads();
         return go_s != 0;
     };
-    auto end_warp = [&](unsigned long long cand) {
-        flush(o, stage, staged);
+    // The block's last tuples and its count of candidates go out with one atomic each (a warp with a
+    // tuple or two each would queue on them for longer than a small iteration takes).
+    auto end_block = [&](unsigned long long cand) {
+        sink.finish();
 #pragma unroll
         for (int d = 16; d; d >>= 1) cand += __shfl_xor_sync(FULL, cand, d);
-        if (lane == 0 && cand) atomicAdd(&ctl->candidates, cand);
+        if (lane == 0) {
+            left_s[warp] = sink.staged;
+            cand_s[warp] = cand;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned mine = lane < DL_WARPS ? left_s[lane] : 0;
+            unsigned incl = mine;
+            unsigned long long c = lane < DL_WARPS ? cand_s[lane] : 0, at = 0;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned x = __shfl_up_sync(FULL, incl, d);
+                if (lane >= (unsigned)d) incl += x;
+            }
+#pragma unroll
+            for (int d = 16; d; d >>= 1) c += __shfl_xor_sync(FULL, c, d);
+            const unsigned total = __shfl_sync(FULL, incl, 31);
+            if (lane == 0) {
+                if (total) at = atomicAdd(&ctl->tail, (unsigned long long)total);
+                if (c) atomicAdd(&ctl->candidates, c);
+            }
+            cand_s[lane] = __shfl_sync(FULL, at, 0) + incl - mine;
+        }
+        __syncthreads();
+        sink.write_left(cand_s[warp]);
     };
     read_phase();
     for (;;) {
         const unsigned phase = phase_s;
         const uint64_t start = range_s[0], n = range_s[1] - range_s[0];
+        const bool check = check_s != 0;
         if (phase == PH_DONE) return;
-        unsigned long long cand = 0;
         if (phase == PH_ROWS) {
-            // rows of the delta in chunks: few rows per warp while there are few of them
-            const uint64_t warps = (uint64_t)gridDim.x * DL_WARPS;
-            // (a row of a square component can stand for any amount of work: smaller chunks)
-            const unsigned most = SQUARE ? 8 : 32, per = (unsigned)(n >= warps * most ? most : (n + warps - 1) / warps);
-            for (uint64_t chunk = (uint64_t)warp * gridDim.x + blockIdx.x; chunk * per < n;) {
-                const uint64_t at = chunk * per;
-                const unsigned rows = (unsigned)(n - at < per ? n - at : per);
-                take_rows(o, rules, start + at, rows, heavy, stage, staged, cand);
-                if (SQUARE)
-                    for (unsigned r = 0; r < rows; ++r) square_row(o, sq, __ldcg(&o.log[start + at + r]), stage, staged, cand);
-                if (n <= warps * per) break;
-                unsigned next = 0;
-                if (lane == 0) next = atomicAdd(&ctl->next_chunk, 1u);
-                chunk = warps + __shfl_sync(FULL, next, 0);
+            unsigned long long cand = 0;
+            const uint64_t warps = (uint64_t)gridDim.x * DL_WARPS, me = (uint64_t)warp * gridDim.x + blockIdx.x;
+            if (SQUARE) {
+                // A row of a square component can stand for any amount of work, and rows of one hub lie
+                // side by side: every warp takes rows far apart, eight at a time.
+                for (uint64_t first = me; first < n; first += 8 * warps) {
+                    const unsigned rows = (unsigned)min((n - first + warps - 1) / warps, (uint64_t)8);
+                    const uint64_t row = lane < rows ? __ldcg(&o.log[start + first + lane * warps]) : 0;
+                    unsigned linear = 0;
+                    take_rows(o, rules, row, rows, heavy, check, sink, linear);
+                    cand += linear;
+                    take_square(o, sq, row, rows, sink, cand);
+                }
+            } else {
+                // Few rows per warp while there are few of them; many are taken in batches from a counter
+                // (32 at a time, 14 M rows queued on it for longer than their work took).
+                const unsigned per = (unsigned)(n >= warps * 32 ? 32 : (n + warps - 1) / warps);
+                uint64_t batch = n / (warps * 8) & ~31ull;
+                batch = per < 32 ? per : batch < 32 ? 32 : batch > 2048 ? 2048 : batch;
+                for (uint64_t at = me * batch; at < n;) {
+                    const uint64_t stop = at + batch < n ? at + batch : n;
+                    uint64_t row = at + lane < stop ? __ldcg(&o.log[start + at + lane]) : 0;
+                    for (; at < stop; at += per) {
+                        const unsigned rows = (unsigned)(stop - at < per ? stop - at : per);
+                        const uint64_t next_row = at + per + lane < stop ? __ldcg(&o.log[start + at + per + lane]) : 0;
+                        unsigned linear = 0;
+                        take_rows(o, rules, row, rows, heavy, check, sink, linear);
+                        cand += linear;
+                        row = next_row;
+                    }
+                    if (n <= warps * batch) break;
+                    unsigned next = 0;
+                    if (lane == 0) next = atomicAdd(&ctl->next_chunk, 1u);
+                    at = (warps + __shfl_sync(FULL, next, 0)) * batch;
+                }
             }
-            end_warp(cand);
+            end_block(cand);
             if (!barrier([&]() -> unsigned { return v->heavy_n ? (unsigned)PH_HEAVY : next_iteration(o, max_iterations, SQUARE); })) return;
         } else if (phase == PH_HEAVY) {
             const unsigned listed = v->heavy_n, pieces = listed < DL_HEAVY_MAX ? listed : (unsigned)DL_HEAVY_MAX;
             for (;;) {
-                __syncthreads();
-                if (threadIdx.x == 0) item_s = atomicAdd(&ctl->next_heavy, 1u);
-                __syncthreads();
-                const unsigned item = item_s;
+                unsigned item = 0;
+                if (lane == 0) item = atomicAdd(&ctl->next_heavy, 1u);
+                item = __shfl_sync(FULL, item, 0);
                 if (item >= pieces) break;
                 Heavy h;
                 h.row = __ldcg(&heavy[item].row);
                 h.rule = __ldcg(&heavy[item].rule);
                 h.piece = __ldcg(&heavy[item].piece);
-                take_piece(o, rules, h, stage, staged);
+                take_piece(o, rules, h, check, sink);
             }
-            end_warp(0);
+            end_block(0);
             if (!barrier([&] { return next_iteration(o, max_iterations, SQUARE); })) return;
         } else if (SQUARE && phase == PH_FULL) {
             for (uint64_t i = (uint64_t)blockIdx.x * DL_THREADS + threadIdx.x; i < n; i += (uint64_t)gridDim.x * DL_THREADS) square_full(o, sq, __ldcg(&o.log[start + i]));
             if (!barrier([&]() -> unsigned { return PH_ROWS; })) return;
         } else if (!SQUARE) {  // PH_SOLO
             if (blockIdx.x == 0) {
-                const unsigned per = (unsigned)((n + DL_WARPS - 1) / DL_WARPS);  // at most 32 (DL_SOLO_ROWS)
-                if ((uint64_t)warp * per < n) {
-                    const uint64_t at = (uint64_t)warp * per;
-                    take_rows(o, rules, start + at, (unsigned)(n - at < per ? n - at : per), heavy, stage, staged, cand);
-                }
-                end_warp(cand);
+                const unsigned next = solo(o, rules, heavy, max_iterations, stage_s, solo_s, start, start + n);
                 __syncthreads();
-                if (threadIdx.x == 0) {
-                    __threadfence();
-                    const unsigned next = v->heavy_n ? (unsigned)PH_HEAVY : next_iteration(o, max_iterations, SQUARE);
-                    if (next != PH_SOLO) publish(next);  // everybody again
-                }
+                if (threadIdx.x == 0) publish(next);  // everybody again
             } else {
                 if (threadIdx.x == 0) go_s = wait_next();
                 __syncthreads();
@@ -535,6 +814,17 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(Out o, Rules rules
     }
 }
 
+__device__ __forceinline__ void flush(const Out& o, const uint64_t* stage, unsigned& staged) {
+    if (!staged) return;
+    unsigned long long at = 0;
+    if (lane_id() == 0) at = atomicAdd(&o.ctl->tail, (unsigned long long)staged);
+    at = __shfl_sync(FULL, at, 0);
+    __syncwarp();
+    for (unsigned i = lane_id(); i < staged; i += 32)
+        if (at + i < o.cap) o.log[at + i] = stage[i];
+    __syncwarp();
+    staged = 0;
+}
 // Rows of a bag into the head: new ones (their bit was clear) are appended to the log.
 __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict__ rows, uint64_t n, Out o) {
     __shared__ uint64_t stage_s[BLOCK / 32][64];
@@ -564,6 +854,7 @@ __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict
 
 __global__ void delta_begin_k(Ctl* c, bool square) {
     const unsigned long long n = c->tail;
+    c->check = 1;
     c->start = 0;
     c->end = n;
     if (n == 0) {  // an iteration over nothing finds nothing
@@ -582,25 +873,19 @@ __global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
 }  // namespace
 
 static Out out_of(xlb_ctx* c, const DeltaLoop& d) {
-    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, d.ctl->as<Ctl>(), c->d_status, d.visited_t ? d.visited_t->as<unsigned int>() : nullptr};
+    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, d.ctl->as<Ctl>(), c->d_status, d.square ? d.visited->as<unsigned int>() + d.words : nullptr};
 }
 
-DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square) {
+DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square, int composites) {
     DeltaLoop d;
     d.hi_bits = hi_bits;
     d.lo_bits = lo_bits;
+    d.square = square;
     d.words = ((1ull << (hi_bits + lo_bits)) + 31) / 32;
-    const uint64_t bytes = std::max<uint64_t>(d.words * 4, 16);
-    d.visited = make_buf(c, bytes);
+    d.visited = make_buf(c, std::max<uint64_t>(d.words * 4, 16) * (square ? 4 + composites : 1));
     d.ctl = make_buf(c, sizeof(Ctl));
-    CUDA_OK(set_async(c, d.visited->p, 0, bytes));
+    CUDA_OK(set_async(c, d.visited->p, 0, d.visited->bytes));
     CUDA_OK(set_async(c, d.ctl->p, 0, sizeof(Ctl)));
-    if (square) {
-        d.visited_t = make_buf(c, bytes);
-        d.full = make_buf(c, 2 * bytes);
-        CUDA_OK(set_async(c, d.visited_t->p, 0, bytes));
-        CUDA_OK(set_async(c, d.full->p, 0, 2 * bytes));
-    }
     return d;
 }
 
@@ -616,8 +901,12 @@ static void log_room(xlb_ctx* c, DeltaLoop& d, uint64_t more) {
     const uint64_t need = d.room + more;
     d.room = need;
     if (d.log && d.cap >= need) return;
+    // Four times what is in it, and from the start as much as a large fixpoint derives where that is a
+    // small part of the free budget (running out costs a pass over the bitmap and a second launch);
+    // never more than the domain, beyond which nothing can be new.
     const uint64_t domain = 1ull << (d.hi_bits + d.lo_bits);
-    uint64_t cap = std::min<uint64_t>(domain, std::max<uint64_t>(4 * need, 1ull << 24));  // (beyond the domain nothing can be new)
+    const uint64_t spare = c->budget > c->allocated ? (c->budget - c->allocated) / 32 / 8 : 0;
+    const uint64_t cap = std::min<uint64_t>(domain, std::max<uint64_t>({4 * need, 1ull << 20, std::min<uint64_t>(spare, 1ull << 26)}));
     Buf log = make_buf(c, std::max<uint64_t>(cap, 1) * 8);
     if (d.log && need > more) CUDA_OK(copy_async(c, log->p, d.log->p, std::min(d.cap, need - more) * 8, cudaMemcpyDeviceToDevice));
     d.log = log;
@@ -644,26 +933,23 @@ void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows) {
 
 static Ix view_of(const Index& ix) {
     return Ix{ix.cursor ? ix.cursor->as<unsigned long long>() : nullptr, ix.domain, ix.table ? ix.table->as<ulonglong2>() : nullptr, ix.mask,
-              ix.S ? ix.S->as<uint64_t>() : nullptr, ix.pay ? ix.pay->as<uint32_t>() : nullptr};
+              ix.pay ? ix.pay->as<uint32_t>() : ix.S->as<uint32_t>(), ix.pay ? 0 : 1};
 }
 
 bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
                    DeltaResult* res) {
     if (rules.size() > DL_RULES || variants.size() > SQ_VARIANTS) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules and %zu variants in a delta loop", rules.size(), variants.size());
     if (!c->delta_attr_set) {
-        CUDA_OK(cudaFuncSetAttribute(delta_loop_k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DL_WARPS * DL_STAGE * 8));
-        CUDA_OK(cudaFuncSetAttribute(delta_loop_k<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DL_WARPS * DL_STAGE * 8));
+        CUDA_OK(cudaFuncSetAttribute(delta_loop_k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DL_SMEM));
+        CUDA_OK(cudaFuncSetAttribute(delta_loop_k<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DL_SMEM));
     }
     c->delta_attr_set = true;
-    const bool square = d.visited_t != nullptr;
+    const bool square = d.square;
     Square sq{};
-    std::vector<Buf> composites;
+    std::vector<Buf> counts;
     if (square) {
-        const uint64_t bytes = d.visited->bytes;
         sq.bits = d.lo_bits;
-        sq.known_t = d.visited_t->as<unsigned int>();
-        sq.full = d.full->as<unsigned int>();
-        sq.full_t = sq.full + bytes / 4;
+        sq.words = (uint32_t)d.words;
         for (auto& in : variants) {
             Variant& v = sq.v[sq.n++];
             v.a_key = in.list ? in.list_key : -1;
@@ -671,22 +957,20 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
             v.row_key = in.row_key;
             v.fixed = in.fixed;
             v.bits_are_hi = in.bits_are_hi;
-            if (in.rows == DeltaVariant::HEAD) v.rows = sq.full;
-            else if (in.rows == DeltaVariant::HEAD_T) v.rows = sq.full_t;
-            else {
-                if (sq.n_aux == SQ_AUX) xlb_fail(XLB_ERR_INVALID, "internal: too many composites in a delta loop");
-                Buf b = make_buf(c, bytes + (8ull << d.lo_bits));
-                CUDA_OK(set_async(c, b->p, 0, b->bytes));
-                composites.push_back(b);
-                Composite& x = sq.aux[sq.n_aux++];
-                x.ix = view_of(*in.composed);
-                x.list_key = in.composed_list_key;
-                x.row_key = in.composed_row_key;
-                x.rows = b->as<unsigned int>();
-                x.counts = (unsigned long long*)(x.rows + bytes / 4);
-                v.rows = x.rows;
-                v.counts = x.counts;
+            if (in.rows != DeltaVariant::COMPOSED) {
+                v.rows = (in.rows == DeltaVariant::HEAD ? 2 : 3) * sq.words;
+                continue;
             }
+            if (sq.n_aux == SQ_AUX || d.visited->bytes < (uint64_t)(5 + sq.n_aux) * sq.words * 4) xlb_fail(XLB_ERR_INVALID, "internal: too many composites in a delta loop");
+            Buf b = make_buf(c, 8ull << sq.bits);
+            CUDA_OK(set_async(c, b->p, 0, b->bytes));
+            counts.push_back(b);
+            Composite& x = sq.aux[sq.n_aux];
+            x.ix = view_of(*in.composed);
+            x.list_key = in.composed_list_key;
+            x.row_key = in.composed_row_key;
+            x.rows = v.rows = (4 + sq.n_aux++) * sq.words;
+            v.counts = x.counts = b->as<unsigned long long>();
         }
     }
     log_room(c, d, 0);
@@ -710,7 +994,7 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         Heavy* hp = heavy->as<Heavy>();
         void* args[] = {&o, &rs, &hp, &max_iterations, &sq};
         prof_begin(c, "expand_mark", 0);
-        CUDA_OK(cudaLaunchCooperativeKernel(square ? (const void*)delta_loop_k<true> : (const void*)delta_loop_k<false>, dim3((unsigned)c->sm_count), dim3(DL_THREADS), args, (size_t)DL_WARPS * DL_STAGE * 8, c->stream));
+        CUDA_OK(cudaLaunchCooperativeKernel(square ? (const void*)delta_loop_k<true> : (const void*)delta_loop_k<false>, dim3((unsigned)c->sm_count), dim3(DL_THREADS), args, DL_SMEM, c->stream));
         check_launch(c, "expand_mark");
         unsigned long long w[7];  // tail, start, end, iterations, candidates, fix, overflow
         read_words(c, d.ctl->p, 7, w);
@@ -727,7 +1011,7 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         Keys done;
         done.buf = d.log;
         done.n = stored;
-        Buf before = make_buf(c, d.visited->bytes);
+        Buf before = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
         CUDA_OK(set_async(c, before->p, 0, before->bytes));
         for (const Keys* k : {&known, (const Keys*)&done}) {
             if (!k->n) continue;

@@ -1945,13 +1945,15 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         const bool square = !plan.square.empty();
         if (square) {
             // (a head that holds rows already would have to be brought into the transposed bitmaps as well)
-            hb = lb = std::max({hb, lb, 5});
+            hb = lb = std::max({hb, lb, 6});
             if (from_store || hb > SQUARE_BITS) return false;
         }
         if (hb + lb > WIDE_DENSE_BITS) return false;
         const uint64_t bitmap = (1ull << (hb + lb)) / 8;
         if (c->budget && c->allocated + (square ? 8 : 3) * bitmap > c->budget) return false;
-        DeltaLoop d = ops_delta_begin(c, hb, lb, square);
+        int composed = 0;
+        for (auto& t : plan.square) composed += t.composed >= 0 ? 1 : 0;
+        DeltaLoop d = ops_delta_begin(c, hb, lb, square, composed);
         if (from_store) {
             PhaseTimer t(c, &rs.st.ms_join);
             ops_delta_append(c, d, delta);

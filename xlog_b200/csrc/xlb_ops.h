@@ -208,21 +208,21 @@ struct DeltaVariant {
     int composed_list_key = 0, composed_row_key = 0;  // halves of a head row (0 high, 1 low): what probes `composed`, what keys its bit rows
 };
 struct DeltaLoop {
-    Buf visited;            // the head as a bitmap
+    Buf visited;            // the head as a bitmap (square components: more of them behind it)
+    bool square = false;
     uint64_t words = 0;
     int hi_bits = 0, lo_bits = 0;
     Buf log;                // derived tuples in the order they were found; the last ones are the delta
     uint64_t cap = 0, room = 0;  // tuples the log can hold; that may be in it
     Buf ctl;
-    Buf visited_t, full;    // square components: the head's transpose; the head and its transpose as an iteration finds them
 };
 struct DeltaResult {
     uint64_t rows = 0;      // tuples in the log: what was derived beyond the known rows
     uint64_t iterations = 0, candidates = 0;
     bool fix = false;       // an iteration found nothing (else the iteration limit was reached)
 };
-// square: for rules with two recursive atoms (hi_bits == lo_bits, at least 5)
-DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square);
+// square: for rules with two recursive atoms (hi_bits == lo_bits, 6 to 13), `composites` of their variants composed
+DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square, int composites);
 void ops_delta_known(xlb_ctx* c, DeltaLoop& d, const Keys& rows);   // rows the head holds that are not part of the delta
 void ops_delta_seed(xlb_ctx* c, DeltaLoop& d, const Keys& bag);     // candidates: what the head lacks joins it and the delta
 void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows);  // a delta as it is (known to the head already); before any seed
