@@ -139,3 +139,23 @@ def test_transposed_partner_and_composed_relation(monkeypatch):
     want, _ = O.run_program(plan, {"e": e, "g": g}, ["p"])
     for a, w in zip(got, want["p"]):
         assert np.array_equal(a, w)
+
+
+@pytest.mark.parametrize("bits", [17, 24, 28, 29, 32])
+@pytest.mark.parametrize("values", [2, 500, 65536, 65537])
+def test_thinly_spread_values(bits, values, monkeypatch):
+    # ids of `bits` bits, `values` different ones: run on ranks (and on hash sets where there are too many)
+    if values >= 1 << bits:
+        return
+    rng = np.random.default_rng(bits)
+    ids = np.unique(np.concatenate([rng.integers(0, 1 << bits, 2 * values, dtype=np.uint64), [0, (1 << bits) - 1]]).astype(np.uint32))
+    ids = np.sort(np.concatenate([ids[[0, -1]], rng.permutation(ids[1:-1])[: values - 2]]))
+    assert len(ids) == values
+    n = min(values, 3000)
+    some = rng.permutation(ids)[:n]
+    u, v = rng.integers(0, n, n), rng.integers(0, n, n)
+    # the rest of the ids in pairs, so that every one of them is there
+    edge = [np.concatenate([some[u], ids[:-1:2]]), np.concatenate([some[v], ids[1::2]])]
+    if values % 2:
+        edge = [np.append(edge[0], ids[-1]), np.append(edge[1], ids[0])]
+    both(programs.transitive_closure(), {"edge": edge}, "reach", monkeypatch)

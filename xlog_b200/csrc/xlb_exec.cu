@@ -2335,9 +2335,17 @@ static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
 // columns and the sorted result are unchanged; constants of filters are translated to rank bounds.
 static bool rank32(uint8_t t) { return t == XLB_U32 || t == XLB_SYMBOL; }
 
+// Plans over 32-bit columns run on ranks, too, when the values are spread thin over a wide range (ids
+// that carry a kind or an address in their upper bits): a head of two columns of more than 16 bits has
+// no bitmap, and its candidates would each be hashed and grouped; where there are at most 2^16
+// different values, their ranks fit one.  Finding that out costs a pass over the relations and, above
+// 28 bits, a sort of their values: not worth it for a handful of rows.
+constexpr uint64_t SPARSE_VALUES = 1ull << 16, SPARSE_ROWS_MIN = 64, SPARSE_ROWS_MAX = 1ull << 26;
+
 struct EncodedRun {
     xlb_ctx* c = nullptr;
     Keys dict;
+    bool narrow = false;  // all columns are 32 bits wide: packed rows in, packed rows out
     std::deque<xlb_node> nodes;
     std::deque<std::vector<const xlb_node*>> lists;
     std::deque<std::vector<xlb_rule>> rules;
@@ -2389,6 +2397,34 @@ struct EncodedRun {
         return &m;
     }
 
+    // Is this a plan over thinly spread 32-bit values that a bitmap takes as ranks?  (Its dictionary is
+    // left in `dict` then.)
+    bool sparse(const xlb_plan* in, const std::vector<const xlb_rel*>& rels) {
+        if (c->world > 1 || c->comm_world > 1 || (c->flags & (XLB_FLAG_NO_DENSE | XLB_FLAG_KEEP_DELTAS | XLB_FLAG_GENERAL_ONLY)) || getenv("XLB_NO_DELTA_LOOP")) return false;
+        bool pair_head = false;
+        for (auto& h : head_types) {
+            if (h.second.arity < 1 || h.second.arity > 2 || store_get(c, "__delta_" + h.first)) return false;
+            pair_head |= h.second.arity == 2;
+        }
+        bool recursive = false;
+        for (uint32_t s = 0; s < in->n_sccs; ++s) recursive |= in->sccs[s].is_recursive != 0;
+        if (!pair_head || !recursive) return false;
+        uint64_t rows = 0, bound = 0;
+        for (const xlb_rel* r : rels) {
+            if (r->schema.arity < 1 || r->schema.arity > 2) return false;
+            rows += r->rows;
+        }
+        if (rows < SPARSE_ROWS_MIN || rows > SPARSE_ROWS_MAX) return false;
+        for (const xlb_rel* r : rels) {
+            if (!r->rows) continue;
+            const Keys k = ops_rel_packed(c, r);  // (kept: what the plan itself would start with)
+            if (k.bound == ~0ull) return false;
+            bound |= (k.bound >> 32) | (k.bound & 0xFFFFFFFFull);
+        }
+        const int bits = bit_len(bound);
+        return 2 * bits > WIDE_DENSE_BITS && ops_rank_build(c, rels, bits, SPARSE_VALUES, &dict);
+    }
+
     // Decide, and if the plan needs it swap the ranks in.  Returns the plan to run.
     const xlb_plan* begin(xlb_ctx* ctx, const xlb_plan* in) {
         c = ctx;
@@ -2413,7 +2449,10 @@ struct EncodedRun {
             rels.push_back(r);
             for (uint32_t k = 0; k < r->schema.arity; ++k) wide |= !rank32(r->schema.types[k]);
         }
-        if (!wide) return in;
+        if (!wide) {
+            if (!sparse(in, rels)) return in;
+            narrow = true;
+        }
         if (c->world > 1) xlb_fail(XLB_ERR_UNSUPPORTED, "plans over u64, signed or floating columns run on one GPU");
         if (c->flags & XLB_FLAG_KEEP_DELTAS) xlb_fail(XLB_ERR_UNSUPPORTED, "XLB_FLAG_KEEP_DELTAS with u64, signed or floating columns is not built");
         for (const xlb_rel* r : rels) {
@@ -2437,7 +2476,7 @@ struct EncodedRun {
                 for (uint32_t k = 0; k < h.second.arity; ++k) typed |= ordered(h.second.types[k]);
             if (typed) xlb_fail(XLB_ERR_UNSUPPORTED, "filters with constants over signed or floating columns are not built");
         }
-        dict = ops_dict_build(c, rels);
+        if (!narrow) dict = ops_dict_build(c, rels);
         std::vector<uint64_t> consts;
         for (const xlb_node* f : const_filters) consts.push_back(f->cmp_rhs);
         ops_dict_bounds(c, dict, consts, below, not_above);
@@ -2462,7 +2501,7 @@ struct EncodedRun {
         for (auto& n : names) {
             auto it = c->store.find(n);
             if (it == c->store.end()) continue;
-            xlb_rel* enc = ops_dict_encode(c, it->second, dict);
+            xlb_rel* enc = narrow ? ops_rank_encode(c, it->second, dict) : ops_dict_encode(c, it->second, dict);
             originals[n] = it->second;
             it->second = enc;
             c->versions[n]++;
@@ -2476,7 +2515,7 @@ struct EncodedRun {
         for (auto& h : head_types) {
             xlb_rel* ranks = store_get(c, h.first);
             if (!ranks) continue;
-            xlb_rel* decoded = ops_dict_decode(c, ranks, h.second, dict);
+            xlb_rel* decoded = narrow ? ops_rank_decode(c, ranks, h.second, dict) : ops_dict_decode(c, ranks, h.second, dict);
             store_put(c, h.first, decoded);  // frees the rank relation
             auto o = originals.find(h.first);
             if (o != originals.end()) {      // a head that held rows before: superseded by the result

@@ -1837,6 +1837,120 @@ void ops_dict_bounds(xlb_ctx* c, const Keys& dict, const std::vector<uint64_t>& 
     }
 }
 
+namespace {
+// every value of packed rows (both halves, or the low one) into a bitmap, or into a list
+__global__ void __launch_bounds__(BLOCK) rank_mark_k(const uint64_t* __restrict__ rows, uint64_t n, int halves, unsigned int* __restrict__ bitmap) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint64_t k = rows[i];
+        for (int h = 0; h < halves; ++h) {
+            const uint32_t v = h ? (uint32_t)(k >> 32) : (uint32_t)k;
+            const unsigned bit = 1u << (v & 31);
+            if (!(bitmap[v >> 5] & bit)) atomicOr(&bitmap[v >> 5], bit);
+        }
+    }
+}
+__global__ void __launch_bounds__(BLOCK) rank_list_k(const uint64_t* __restrict__ rows, uint64_t n, int halves, uint64_t* __restrict__ out) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint64_t k = rows[i];
+        out[i] = (uint32_t)k;
+        if (halves == 2) out[n + i] = k >> 32;
+    }
+}
+__global__ void __launch_bounds__(BLOCK) rank_encode_k(const uint64_t* __restrict__ rows, uint64_t n, int halves, const uint64_t* __restrict__ dict, uint64_t m,
+                                                      uint64_t* __restrict__ out, DevStatus* st) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint64_t k = rows[i];
+        uint64_t o = 0;
+        for (int h = 0; h < halves; ++h) {
+            const uint64_t v = h ? k >> 32 : (uint32_t)k, r = dict_below(dict, m, v);
+            if (r >= m || dict[r] != v) set_status(st, XLB_ERR_CAPACITY, 18, v);
+            o |= r << (32 * h);
+        }
+        out[i] = o;
+    }
+}
+__global__ void __launch_bounds__(BLOCK) rank_decode_k(const uint64_t* __restrict__ ranks, uint64_t n, const uint64_t* __restrict__ dict, uint64_t m, uint32_t* __restrict__ c0,
+                                                      uint32_t* __restrict__ c1, DevStatus* st) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint64_t k = ranks[i];
+        const uint32_t hi = (uint32_t)(k >> 32), lo = (uint32_t)k;
+        if (lo >= m || (c1 && hi >= m)) {
+            set_status(st, XLB_ERR_CAPACITY, 19, k);
+            continue;
+        }
+        if (c1) {
+            c0[i] = (uint32_t)dict[hi];
+            c1[i] = (uint32_t)dict[lo];
+        } else c0[i] = (uint32_t)dict[lo];
+    }
+}
+}  // namespace
+
+bool ops_rank_build(xlb_ctx* c, const std::vector<const xlb_rel*>& rels, int bits, uint64_t most, Keys* dict) {
+    uint64_t total = 0;
+    for (const xlb_rel* r : rels) total += r->rows * r->schema.arity;
+    const uint64_t all = bits >= 64 ? ~0ull : (1ull << bits) - 1;
+    if (bits <= 28) {
+        DenseSet d = ops_dense_begin(c, 0, bits);
+        d.bound = all;
+        for (const xlb_rel* r : rels) {
+            if (!r->rows) continue;
+            Keys k = ops_rel_packed(c, r);
+            prof_begin(c, "dict_image", k.n * 8ull);
+            rank_mark_k<<<grid_for(c, k.n), BLOCK, 0, c->stream>>>(k.ptr(), k.n, (int)r->schema.arity, d.bitmap->as<unsigned int>());
+            check_launch(c, "dict_image");
+        }
+        Keys none;
+        *dict = ops_dense_finish(c, d, none);
+    } else {
+        dict->n = total;
+        dict->bound = all;
+        dict->buf = make_buf(c, total * 8);
+        uint64_t at = 0;
+        for (const xlb_rel* r : rels) {
+            if (!r->rows) continue;
+            Keys k = ops_rel_packed(c, r);
+            prof_begin(c, "dict_image", k.n * 16ull);
+            rank_list_k<<<grid_for(c, k.n), BLOCK, 0, c->stream>>>(k.ptr(), k.n, (int)r->schema.arity, dict->buf->as<uint64_t>() + at);
+            check_launch(c, "dict_image");
+            at += k.n * r->schema.arity;
+        }
+        ops_sort(c, *dict);
+        ops_dedup_sorted(c, *dict);
+    }
+    return dict->n <= most;
+}
+
+xlb_rel* ops_rank_encode(xlb_ctx* c, const xlb_rel* r, const Keys& dict) {
+    Keys k = ops_rel_packed(c, r), o;
+    o.n = k.n;
+    o.buf = make_buf(c, k.n * 8);
+    const uint64_t ranks = (1ull << bit_length(dict.n ? dict.n - 1 : 0)) - 1;
+    o.bound = r->schema.arity == 2 ? (ranks << 32) | ranks : ranks;
+    if (k.n) {
+        prof_begin(c, "dict_rank", k.n * 16ull);
+        rank_encode_k<<<grid_for(c, k.n), BLOCK, 0, c->stream>>>(k.ptr(), k.n, (int)r->schema.arity, dict.ptr(), dict.n, o.buf->as<uint64_t>(), c->d_status);
+        check_launch(c, "dict_rank");
+    }
+    return ops_rel_from_keys(c, r->schema, o, r->canonical);  // ranks order as the values do
+}
+
+xlb_rel* ops_rank_decode(xlb_ctx* c, const xlb_rel* ranks, const xlb_schema& types, const Keys& dict) {
+    Keys k = ops_rel_packed(c, ranks);
+    std::unique_ptr<xlb_rel> o(new xlb_rel);
+    o->ctx = c;
+    o->rows = k.n;
+    o->schema = types;
+    o->canonical = ranks->canonical;
+    for (uint32_t i = 0; i < types.arity; ++i) o->cols[i] = make_buf(c, k.n * 4);
+    if (k.n) {
+        prof_begin(c, "dict_decode", k.n * (8ull + 4 * types.arity));
+        rank_decode_k<<<grid_for(c, k.n), BLOCK, 0, c->stream>>>(k.ptr(), k.n, dict.ptr(), dict.n, o->cols[0]->as<uint32_t>(), types.arity == 2 ? o->cols[1]->as<uint32_t>() : nullptr, c->d_status);
+        check_launch(c, "dict_decode");
+    }
+    return o.release();
+}
+
 // forward: a view of `r` whose typed columns are mapped to unsigned words (schema becomes
 // unsigned); inverse: `r` is an unsigned result, `types` the schema to restore.
 static xlb_rel* map_rel(xlb_ctx* c, const xlb_rel* r, const xlb_schema& types, bool inverse) {

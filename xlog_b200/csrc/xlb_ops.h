@@ -249,6 +249,13 @@ xlb_rel* ops_dict_decode(xlb_ctx* c, const xlb_rel* ranks, const xlb_schema& typ
 // number not above it (equal: the constant is absent).
 void ops_dict_bounds(xlb_ctx* c, const Keys& dict, const std::vector<uint64_t>& consts, std::vector<uint64_t>& below, std::vector<uint64_t>& not_above);
 
+// The same for relations of 32-bit columns whose values are spread thin over a wide range: `bits` = bit
+// length of the largest value.  The dictionary of at most `most` values is read off a bitmap of the
+// values (up to 28 bits) or sorted; false: there are more values.
+bool ops_rank_build(xlb_ctx* c, const std::vector<const xlb_rel*>& rels, int bits, uint64_t most, Keys* dict);
+xlb_rel* ops_rank_encode(xlb_ctx* c, const xlb_rel* r, const Keys& dict);
+xlb_rel* ops_rank_decode(xlb_ctx* c, const xlb_rel* ranks, const xlb_schema& types, const Keys& dict);
+
 // owner rank of every row by the half `keysel`; stable partition into `world` runs, whose lengths
 // are left in device memory at `counts_dev` (no read-back); returns the partitioned copy.
 Keys ops_partition_by_owner_dev(xlb_ctx* c, const Keys& in, int keysel, uint32_t world, unsigned long long* counts_dev);
