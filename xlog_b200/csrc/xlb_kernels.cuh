@@ -787,6 +787,123 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
     }
 }
 
+// A few thousand keys are sorted by one block in shared memory: all passes, histograms and the choice of
+// digits in one launch without a read-back.  (The one-sweep route takes two fills, two kernels, a
+// read-back and a launch per digit: 60 us for 2000 keys of three digits, against 9.)
+constexpr int SS_THREADS = 1024, SS_WARPS = SS_THREADS / 32, SS_MAX = SS_THREADS * 8;
+template <int IPT>
+static __global__ void __launch_bounds__(SS_THREADS) radix_small_k(const uint64_t* __restrict__ keys_in, uint64_t* __restrict__ keys_out, const uint32_t* __restrict__ vals_in,
+                                                                  uint32_t* __restrict__ vals_out, unsigned n, unsigned digit_mask) {
+    extern __shared__ __align__(16) unsigned char ss_smem[];
+    uint64_t* sk = reinterpret_cast<uint64_t*>(ss_smem);
+    uint32_t* sv = reinterpret_cast<uint32_t*>(sk + SS_THREADS * IPT);
+    unsigned short (*wh)[256] = reinterpret_cast<unsigned short (*)[256]>(sv + SS_THREADS * IPT);
+    __shared__ unsigned bits_s[4], base_s[256], warp_s[8];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5, first = warp * (32 * IPT) + lane;
+    uint64_t key[IPT];
+    uint32_t val[IPT];
+    if (threadIdx.x < 4) bits_s[threadIdx.x] = threadIdx.x < 2 ? 0u : ~0u;
+    __syncthreads();
+    uint64_t all_or = 0, all_and = ~0ull;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+        const unsigned i = first + j * 32;
+        key[j] = ~0ull;  // past the end: behind every key, in its place already
+        val[j] = 0;
+        if (i < n) {
+            key[j] = keys_in[i];
+            if (vals_in) val[j] = vals_in[i];
+            all_or |= key[j];
+            all_and &= key[j];
+        }
+    }
+    const unsigned o_lo = __reduce_or_sync(FULL, (unsigned)all_or), o_hi = __reduce_or_sync(FULL, (unsigned)(all_or >> 32));
+    const unsigned a_lo = __reduce_and_sync(FULL, (unsigned)all_and), a_hi = __reduce_and_sync(FULL, (unsigned)(all_and >> 32));
+    if (lane == 0) {
+        atomicOr(&bits_s[0], o_lo);
+        atomicOr(&bits_s[1], o_hi);
+        atomicAnd(&bits_s[2], a_lo);
+        atomicAnd(&bits_s[3], a_hi);
+    }
+    __syncthreads();
+    const uint64_t varying = (((uint64_t)bits_s[1] << 32) | bits_s[0]) & ~(((uint64_t)bits_s[3] << 32) | bits_s[2]);
+    for (int d = 0; d < 8; ++d) {
+        if (!((digit_mask >> d) & 1u) || !((varying >> (8 * d)) & 255)) continue;
+        for (unsigned i = threadIdx.x; i < SS_WARPS * 256 / 2; i += SS_THREADS) reinterpret_cast<unsigned*>(&wh[0][0])[i] = 0;
+        __syncthreads();
+        unsigned short rank[IPT];
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            const unsigned x = (unsigned)(key[j] >> (8 * d)) & 255, peers = match_digit(x), leader = __ffs(peers) - 1;
+            unsigned before = 0;
+            if (lane == leader) {
+                before = wh[warp][x];
+                wh[warp][x] = (unsigned short)(before + __popc(peers));
+            }
+            before = __shfl_sync(FULL, before, leader);
+            rank[j] = (unsigned short)(before + __popc(peers & lanemask_lt()));
+            __syncwarp();
+        }
+        __syncthreads();
+        unsigned run = 0, incl = 0;
+        if (threadIdx.x < 256) {  // per digit: prefix over the warps, then over the digits
+#pragma unroll
+            for (int w = 0; w < SS_WARPS; ++w) {
+                const unsigned v = wh[w][threadIdx.x];
+                wh[w][threadIdx.x] = (unsigned short)run;
+                run += v;
+            }
+            incl = run;
+#pragma unroll
+            for (int k = 1; k < 32; k <<= 1) {
+                const unsigned v = __shfl_up_sync(FULL, incl, k);
+                if (lane >= (unsigned)k) incl += v;
+            }
+            if (lane == 31) warp_s[warp] = incl;
+        }
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            unsigned before = 0;
+            for (unsigned w = 0; w < warp; ++w) before += warp_s[w];
+            base_s[threadIdx.x] = before + incl - run;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            const unsigned x = (unsigned)(key[j] >> (8 * d)) & 255, p = base_s[x] + wh[warp][x] + rank[j];
+            sk[p] = key[j];
+            sv[p] = val[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            key[j] = sk[first + j * 32];
+            val[j] = sv[first + j * 32];
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+        const unsigned i = first + j * 32;
+        if (i < n) {
+            keys_out[i] = key[j];
+            if (vals_out) vals_out[i] = val[j];
+        }
+    }
+}
+template <int IPT>
+inline void radix_small(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned digit_mask) {
+    constexpr size_t smem = (size_t)SS_THREADS * IPT * 12 + SS_WARPS * 512;
+    if (smem > (48u << 10)) CUDA_OK(cudaFuncSetAttribute(radix_small_k<IPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    Buf outk = make_buf(c, n * 8), outv = vals ? make_buf(c, n * 4) : Buf();
+    prof_begin(c, "radix_small", n * (vals ? 24ull : 16ull));
+    radix_small_k<IPT><<<1, SS_THREADS, smem, c->stream>>>(keys->as<uint64_t>(), outk->as<uint64_t>(), vals ? (*vals)->as<uint32_t>() : nullptr, vals ? outv->as<uint32_t>() : nullptr,
+                                                          (unsigned)n, digit_mask);
+    check_launch(c, "radix_small");
+    keys = outk;
+    if (vals) *vals = outv;
+}
+
 constexpr size_t SORT_SMEM = (size_t)SORT_TILE * 8 + SORT_WARPS * 1024 + 256 * 4 * 2 + 64 * 4;
 
 // The scatter kernel takes more than the 48 KB a launch gets by default: opt in once per context
@@ -834,6 +951,13 @@ inline SortPlan plan_sort(xlb_ctx* c, const uint64_t* keys, uint64_t n) {
 inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned digit_mask = 0xFFu, uint64_t known_bound = ~0ull, bool keep_input = false) {
     if (n <= 1) return;
     if (n >= (1ull << 32)) xlb_fail(XLB_ERR_CAPACITY, "sort of %llu keys exceeds the 2^32 limit of one sort", (unsigned long long)n);
+    if (n <= (uint64_t)SS_MAX && !c->lb_first_tile) {
+        if (n <= SS_THREADS) radix_small<1>(c, keys, vals, n, digit_mask);
+        else if (n <= 2 * SS_THREADS) radix_small<2>(c, keys, vals, n, digit_mask);
+        else if (n <= 4 * SS_THREADS) radix_small<4>(c, keys, vals, n, digit_mask);
+        else radix_small<8>(c, keys, vals, n, digit_mask);
+        return;
+    }
     radix_sort_setup(c);
     uint32_t ntiles = (uint32_t)((n + SORT_TILE - 1) / SORT_TILE);
     Buf tmpk = make_buf(c, n * 8);
