@@ -1,0 +1,88 @@
+"""Joins and aggregations at the sizes where their routes change hands: keys with one, a few and very
+many build rows, domains around the table limits, hub groups, row counts around tiles; and sorts
+around the sizes one block takes."""
+import numpy as np
+import pytest
+
+from xlog_b200 import _abi as A
+from xlog_b200.provider import KernelProvider
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def p():
+    prov = KernelProvider(device=0)
+    yield prov
+    prov.close()
+
+
+def inner(lk, rk):
+    """(left row, right row) pairs by left row, then right row."""
+    order = np.argsort(rk, kind="stable")
+    s = rk[order]
+    lo, hi = np.searchsorted(s, lk, "left"), np.searchsorted(s, lk, "right")
+    n = hi - lo
+    left = np.repeat(np.arange(len(lk)), n)
+    first = np.cumsum(n) - n
+    right = order[np.repeat(lo, n) + np.arange(len(left)) - np.repeat(first, n)]
+    return left, right
+
+
+@pytest.mark.parametrize("nl,nr,keys", [(1, 1, 1), (1, 64, 1), (3, 65, 1), (2047, 2049, 700), (2048, 513, 40), (2049, 100000, 60000), (70000, 3000, 1 << 31), (5000, 8192, 100)])
+@pytest.mark.parametrize("dtype", [np.uint32, np.uint64, "pair"])
+def test_joins(p, nl, nr, keys, dtype):
+    rng = np.random.default_rng(nl + nr)
+    draw = lambda n: rng.integers(0, keys, n)  # noqa: E731
+    if dtype == "pair":
+        lkc, rkc = [draw(nl).astype(np.uint32), (draw(nl) % 2).astype(np.uint32)], [draw(nr).astype(np.uint32), (draw(nr) % 2).astype(np.uint32)]
+        lk, rk = [(c[0].astype(np.uint64) << np.uint64(32)) | c[1] for c in (lkc, rkc)]
+    else:
+        scale = np.uint64(0x9E3779B97F4A7C15 if dtype is np.uint64 else 1)
+        with np.errstate(over="ignore"):
+            lkc, rkc = [(draw(nl).astype(np.uint64) * scale).astype(dtype)], [(draw(nr).astype(np.uint64) * scale).astype(dtype)]
+        lk, rk = lkc[0], rkc[0]
+    lv, rv = rng.integers(0, 1 << 60, nl, dtype=np.uint64), rng.integers(0, 255, nr).astype(np.float32)
+    L, R = p.create_buffer_from_slices(lkc + [lv]), p.create_buffer_from_slices([rv] + rkc)
+    nk = len(lkc)
+    got = p.download(p.hash_join_v2(L, R, list(range(nk)), list(range(1, nk + 1))))
+    left, right = inner(lk, rk)
+    want = [c[left] for c in lkc + [lv]] + [c[right] for c in [rv] + rkc]
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
+    has = np.isin(lk, rk)
+    for kind, keep in ((A.JOIN_SEMI, has), (A.JOIN_ANTI, ~has)):
+        for g, w in zip(p.download(p.hash_join_v2(L, R, list(range(nk)), list(range(1, nk + 1)), kind)), lkc + [lv]):
+            assert np.array_equal(g, w[keep])
+
+
+@pytest.mark.parametrize("n,groups,hub", [(1, 1, 0), (2048, 65536, 0), (2049, 65537, 0), (16385, 65537, 0), (100001, 30000, 50000), (200000, 10, 0), (200000, 3, 150000), (70001, 1 << 31, 0)])
+@pytest.mark.parametrize("nk", [1, 2])
+def test_groupby(p, n, groups, hub, nk):
+    rng = np.random.default_rng(n)
+    g = rng.integers(0, groups, n)
+    g[:hub] = groups - 1
+    g = rng.permutation(g).astype(np.uint32)
+    cols = [g, rng.integers(0, 3, n).astype(np.uint32)][:nk] + [rng.integers(0, 1 << 63, n, dtype=np.uint64), rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)]
+    b = p.create_buffer_from_slices(cols)
+    got = p.download(p.groupby_multi_agg(b, list(range(nk)), [(nk, A.AGG_SUM), (nk + 1, A.AGG_MIN), (nk, A.AGG_MAX), (0, A.AGG_COUNT), (nk + 1, A.AGG_SUM)]))
+    key = cols[0].astype(np.uint64) if nk == 1 else (cols[0].astype(np.uint64) << np.uint64(32)) | cols[1]
+    order = np.argsort(key, kind="stable")
+    u, at = np.unique(key[order], return_index=True)
+    v, w = cols[nk][order], cols[nk + 1][order]
+    want = ([u.astype(np.uint32)] if nk == 1 else [(u >> np.uint64(32)).astype(np.uint32), u.astype(np.uint32)]) + [
+        np.add.reduceat(v, at), np.minimum.reduceat(w, at), np.maximum.reduceat(v, at), np.diff(np.append(at, n)).astype(np.uint64), np.add.reduceat(w.astype(np.uint64), at)]
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [2, 31, 1023, 1024, 1025, 2048, 2049, 4097, 8191, 8192, 8193])
+def test_small_sorts(p, n):
+    rng = np.random.default_rng(n)
+    for cols in ([rng.integers(0, 1 << 63, n, dtype=np.uint64)], [rng.integers(0, 5, n).astype(np.uint32), rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)],
+                 [np.full(n, (1 << 64) - 1, np.uint64)]):
+        b = p.create_buffer_from_slices(cols + [np.arange(n, dtype=np.uint32)])
+        keys = list(range(len(cols)))
+        order = np.lexsort([c for c in reversed(cols)])
+        for g, c in zip(p.download(p.sort(b, keys)), cols + [np.arange(n, dtype=np.uint32)]):
+            assert np.array_equal(g, c[order])

@@ -2076,6 +2076,11 @@ extern "C" xlb_status xlb_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t*
         if (in->rows > 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "GroupBy supports at most %u rows, got %llu", 0xFFFFFFFFu, (unsigned long long)in->rows);
         ops_rel_columns(c, in);
         const uint64_t n = in->rows;
+        if (xlb_rel* o = query_groupby(c, in, key_cols, nk, agg_cols, agg_ops, na, os)) {
+            *out = o;
+            guard.deliver(c, out_final);
+            return XLB_OK;
+        }
         Buf idx = sort_permutation(c, in, key_cols, nk);
         // the key columns in sorted order, then the first row of every group
         xlb_rel keys_only;
@@ -2132,11 +2137,7 @@ static Buf join_keys(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_
     Buf kw = make_buf(c, r->rows * 8);
     if (!r->rows) return kw;
     int w0 = (int)type_width(r->schema.types[keys[0]]);
-    const void* c1 = nullptr;
-    if (nk == 2) {
-        if (w0 != 4 || type_width(r->schema.types[keys[1]]) != 4) xlb_fail(XLB_ERR_UNSUPPORTED, "two-column join keys must both be 32-bit");
-        c1 = r->cols[keys[1]]->p;
-    }
+    const void* c1 = nk == 2 ? r->cols[keys[1]]->p : nullptr;
     prof_begin(c, "build_key", 0);
     build_key_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(r->cols[keys[0]]->p, w0, c1, 4, nullptr, kw->as<uint64_t>(), r->rows);
     check_launch(c, "build_key");
@@ -2167,15 +2168,17 @@ xlb_rel* rel_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t
     if (l->rows >= (1ull << 32)) xlb_fail(XLB_ERR_CAPACITY, "join probe side exceeds the 2^32 row limit");
     ops_rel_columns(c, l);
     ops_rel_columns(c, r);
-    // build side: rows ordered by key word (stable, so equal keys keep right-row order)
+    if (nk == 2 && (type_width(l->schema.types[lk[0]]) != 4 || type_width(l->schema.types[lk[1]]) != 4 || type_width(r->schema.types[rk[0]]) != 4 || type_width(r->schema.types[rk[1]]) != 4))
+        xlb_fail(XLB_ERR_UNSUPPORTED, "two-column join keys must both be 32-bit");
+    if (type != XLB_JOIN_INNER) return query_exists(c, l, r, lk, rk, nk, type == XLB_JOIN_SEMI);
+    if (xlb_rel* o = query_join(c, l, r, lk, rk, nk, os)) return o;
+    // a key with many rows: order the build rows by key word (stable, so equal keys keep right-row order)
     Buf rkeys = join_keys(c, r, rk, nk);
     Buf ridx = make_buf(c, r->rows * 4);
-    if (r->rows) {
-        prof_begin(c, "iota", 0);
-        iota_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(ridx->as<uint32_t>(), r->rows);
-        check_launch(c, "iota");
-        radix_sort(c, rkeys, &ridx, r->rows);
-    }
+    prof_begin(c, "iota", 0);
+    iota_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(ridx->as<uint32_t>(), r->rows);
+    check_launch(c, "iota");
+    radix_sort(c, rkeys, &ridx, r->rows);
     Index ix = ops_index_build(c, rkeys, r->rows, 0, ridx);
     Buf lkeys = join_keys(c, l, lk, nk);
     Keys lrows;
@@ -2184,31 +2187,25 @@ xlb_rel* rel_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t
     prof_begin(c, "iota64", 0);
     iota64_k<<<grid_for(c, l->rows), BLOCK, 0, c->stream>>>(lrows.buf->as<uint64_t>(), l->rows);
     check_launch(c, "iota64");
-    if (type == XLB_JOIN_INNER) {
-        Keys pairs = ops_join_expand(c, lrows, SRC_LO, lkeys->as<uint64_t>(), ix, SRC_LO, SRC_OTHER);
-        std::unique_ptr<xlb_rel> o(new xlb_rel);
-        o->ctx = c;
-        o->schema = os;
-        o->rows = pairs.n;
-        for (uint32_t i = 0; i < os.arity; ++i) {
-            bool left = i < l->schema.arity;
-            const xlb_rel* src = left ? l : r;
-            uint32_t sc = left ? i : i - l->schema.arity;
-            uint32_t w = type_width(os.types[i]);
-            o->cols[i] = make_buf(c, pairs.n * w);
-            if (!pairs.n) continue;
-            prof_begin(c, "gather_pair", 0);
-            if (w == 4) gather_pair_k<uint32_t><<<grid_for(c, pairs.n), BLOCK, 0, c->stream>>>(src->cols[sc]->as<uint32_t>(), pairs.ptr(), left ? 0 : 1, o->cols[i]->as<uint32_t>(), pairs.n);
-            else if (w == 8) gather_pair_k<uint64_t><<<grid_for(c, pairs.n), BLOCK, 0, c->stream>>>(src->cols[sc]->as<uint64_t>(), pairs.ptr(), left ? 0 : 1, o->cols[i]->as<uint64_t>(), pairs.n);
-            else gather_pair_k<uint8_t><<<grid_for(c, pairs.n), BLOCK, 0, c->stream>>>(src->cols[sc]->as<uint8_t>(), pairs.ptr(), left ? 0 : 1, o->cols[i]->as<uint8_t>(), pairs.n);
-            check_launch(c, "gather_pair");
-        }
-        return o.release();
+    Keys pairs = ops_join_expand(c, lrows, SRC_LO, lkeys->as<uint64_t>(), ix, SRC_LO, SRC_OTHER);
+    std::unique_ptr<xlb_rel> o(new xlb_rel);
+    o->ctx = c;
+    o->schema = os;
+    o->rows = pairs.n;
+    for (uint32_t i = 0; i < os.arity; ++i) {
+        bool left = i < l->schema.arity;
+        const xlb_rel* src = left ? l : r;
+        uint32_t sc = left ? i : i - l->schema.arity;
+        uint32_t w = type_width(os.types[i]);
+        o->cols[i] = make_buf(c, pairs.n * w);
+        if (!pairs.n) continue;
+        prof_begin(c, "gather_pair", 0);
+        if (w == 4) gather_pair_k<uint32_t><<<grid_for(c, pairs.n), BLOCK, 0, c->stream>>>(src->cols[sc]->as<uint32_t>(), pairs.ptr(), left ? 0 : 1, o->cols[i]->as<uint32_t>(), pairs.n);
+        else if (w == 8) gather_pair_k<uint64_t><<<grid_for(c, pairs.n), BLOCK, 0, c->stream>>>(src->cols[sc]->as<uint64_t>(), pairs.ptr(), left ? 0 : 1, o->cols[i]->as<uint64_t>(), pairs.n);
+        else gather_pair_k<uint8_t><<<grid_for(c, pairs.n), BLOCK, 0, c->stream>>>(src->cols[sc]->as<uint8_t>(), pairs.ptr(), left ? 0 : 1, o->cols[i]->as<uint8_t>(), pairs.n);
+        check_launch(c, "gather_pair");
     }
-    Buf match = ops_probe_match(c, lrows, SRC_LO, lkeys->as<uint64_t>(), ix);
-    Buf sel = make_buf(c, l->rows * 4);
-    uint64_t m = select(c, PredFlag{match->as<uint64_t>(), type == XLB_JOIN_SEMI}, EmitIndex{sel->as<uint32_t>()}, l->rows);
-    return gather_rel(c, l, sel->as<uint32_t>(), m);
+    return o.release();
 }
 
 extern "C" xlb_status xlb_hash_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk,

@@ -283,3 +283,11 @@ xlb_rel* rel_distinct(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols, u
 xlb_rel* rel_union_many(xlb_ctx* c, const xlb_rel* const* ins, uint32_t n);
 xlb_rel* rel_difference(xlb_ctx* c, const xlb_rel* a, const xlb_rel* b);
 xlb_rel* rel_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, xlb_join_type type);
+
+// Joins and aggregation without sorting (xlb_query.cu); inputs as columns, checked by the callers.
+// Left rows that have (want) or lack a match, in left order.
+xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, bool want);
+// Inner join; null when a key of the build side has too many rows to be put in order one by one.
+xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, const xlb_schema& os);
+// Group-by over keys from a small domain; null when the domain is too large or a group too long.
+xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols, uint32_t nk, const uint32_t* agg_cols, const uint32_t* agg_ops, uint32_t na, const xlb_schema& os);

@@ -1,0 +1,500 @@
+// Joins and aggregation over column-major relations without sorting where no order is asked for:
+// semi and anti joins, inner joins (equal keys grouped by counting), group-by over small domains.
+#include <algorithm>
+
+#include "xlb_kernels.cuh"
+#include "xlb_ops.h"
+
+using namespace xk;
+
+namespace {
+
+// The key word of a row: a column's value, or (a << 32) | b for two 32-bit columns.
+struct KeyCols {
+    const void* c0;
+    const uint32_t* c1;
+    int w0;
+    __device__ __forceinline__ uint64_t operator()(uint64_t i) const {
+        if (c1) {
+            const uint32_t a = __ldg((const uint32_t*)c0 + i), b = __ldg(c1 + i);
+            return ((uint64_t)a << 32) | b;
+        }
+        if (w0 == 4) return __ldg((const uint32_t*)c0 + i);
+        return w0 == 8 ? (uint64_t)__ldg((const unsigned long long*)c0 + i) : (uint64_t)__ldg((const uint8_t*)c0 + i);
+    }
+};
+struct Cols {  // columns in and out, with the side a joined column comes from
+    const void* in[XLB_MAX_ARITY];
+    void* out[XLB_MAX_ARITY];
+    int width[XLB_MAX_ARITY];
+    int n, left;  // the first `left` columns come from the left side
+};
+__device__ __forceinline__ void copy_value(const Cols& c, int k, uint64_t from, uint64_t to) {
+    if (c.width[k] == 4) ((uint32_t*)c.out[k])[to] = __ldg((const uint32_t*)c.in[k] + from);
+    else if (c.width[k] == 8) ((unsigned long long*)c.out[k])[to] = __ldg((const unsigned long long*)c.in[k] + from);
+    else ((uint8_t*)c.out[k])[to] = __ldg((const uint8_t*)c.in[k] + from);
+}
+
+// ---- keys of the build side: open addressing, a slot names the first row (plus one) that brought its key
+__device__ __forceinline__ uint64_t claim(const KeyCols& keys, unsigned int* rep, uint64_t mask, uint64_t row, DevStatus* st) {
+    const uint64_t key = keys(row);
+    uint64_t h = mix64(key) & mask;
+    for (uint64_t probe = 0; probe <= mask; ++probe) {  // bounded by the table size
+        unsigned cur = rep[h];
+        if (cur == 0) {
+            cur = atomicCAS(&rep[h], 0u, (unsigned)row + 1);
+            if (cur == 0) return h;
+        }
+        if (keys(cur - 1) == key) return h;
+        h = (h + 1) & mask;
+    }
+    set_status(st, XLB_ERR_CAPACITY, 20, row);
+    return 0;
+}
+__global__ void __launch_bounds__(BLOCK) exists_build_k(KeyCols keys, uint64_t n, unsigned int* __restrict__ rep, uint64_t mask, DevStatus* st) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) claim(keys, rep, mask, i, st);
+}
+// One bit per probe row (has a match == want), and the rows selected per tile of SCAN_TILE.
+constexpr int QT_ROUNDS = SCAN_TILE / BLOCK;
+__global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t n, KeyCols keys, const unsigned int* __restrict__ rep, uint64_t mask, bool want,
+                                                       unsigned int* __restrict__ bits, uint32_t* __restrict__ tile_counts) {
+    __shared__ uint32_t sm[33];
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS;  // a warp's rows side by side
+    uint32_t cnt = 0;
+    uint64_t key[QT_ROUNDS];
+    unsigned cur[QT_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) {
+        const uint64_t i = base + r * 32 + lane_id();
+        key[r] = i < n ? probe(i) : 0;
+    }
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) cur[r] = __ldg(&rep[mix64(key[r]) & mask]);
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) {
+        const uint64_t i = base + r * 32 + lane_id();
+        bool found = false;
+        if (i < n && cur[r]) {
+            uint64_t h = mix64(key[r]) & mask;
+            unsigned c = cur[r];
+            for (uint64_t p = 0; p <= mask && c; ++p) {  // bounded by the table size
+                if (keys(c - 1) == key[r]) {
+                    found = true;
+                    break;
+                }
+                h = (h + 1) & mask;
+                c = __ldg(&rep[h]);
+            }
+        }
+        const unsigned b = __ballot_sync(FULL, i < n && found == want);
+        if (lane_id() == 0 && base + r * 32 < n) bits[(base + r * 32) >> 5] = b;
+        cnt += __popc(b);
+    }
+    uint32_t tot;
+    block_exclusive_scan<uint32_t>(lane_id() == 0 ? cnt : 0u, &tot, sm);
+    if (threadIdx.x == 0) tile_counts[blockIdx.x] = tot;
+}
+// The selected rows, all columns, in order.
+__global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned int* __restrict__ bits, uint64_t n, const uint64_t* __restrict__ tile_offs) {
+    __shared__ uint32_t sm[33];
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS;
+    unsigned w[QT_ROUNDS];
+    uint32_t cnt = 0;
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) {
+        w[r] = base + r * 32 < n ? bits[(base + r * 32) >> 5] : 0u;
+        cnt += __popc(w[r]);
+    }
+    uint32_t tot;
+    uint32_t ex = block_exclusive_scan<uint32_t>(lane_id() == 0 ? cnt : 0u, &tot, sm);
+    uint64_t pos = tile_offs[blockIdx.x] + __shfl_sync(FULL, ex, 0);
+    for (int r = 0; r < QT_ROUNDS; ++r) {
+        if ((w[r] >> lane_id()) & 1u) {
+            const uint64_t to = pos + __popc(w[r] & lanemask_lt());
+            for (int k = 0; k < cols.n; ++k) copy_value(cols, k, base + r * 32 + lane_id(), to);
+        }
+        pos += __popc(w[r]);
+    }
+}
+
+// ---- inner join: the build rows grouped by key
+// Every row finds its key's slot and takes a number in the group there; group starts are the prefix
+// sums of the counts.  The numbers come in no particular order, so each group's rows are put in row
+// order afterwards, which for the usual handful is a few compares.  A group above JOIN_GROUP_MAX rows
+// is reported, and the caller sorts instead.
+constexpr unsigned JOIN_GROUP_MAX = 64;
+__global__ void __launch_bounds__(BLOCK) group_count_k(KeyCols keys, uint64_t n, unsigned int* __restrict__ rep, unsigned int* __restrict__ count, uint64_t mask, uint2* __restrict__ place,
+                                                      DevStatus* st) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint64_t h = claim(keys, rep, mask, i, st);
+        place[i] = make_uint2((unsigned)h, atomicAdd(&count[h], 1u));
+    }
+}
+__global__ void __launch_bounds__(BLOCK) group_fill_k(const uint2* __restrict__ place, uint64_t n, const uint32_t* __restrict__ start, uint32_t* __restrict__ rows) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint2 p = place[i];
+        rows[start[p.x] + p.y] = (uint32_t)i;
+    }
+}
+__global__ void __launch_bounds__(BLOCK) group_order_k(KeyCols keys, const unsigned int* __restrict__ rep, const unsigned int* __restrict__ count, const uint32_t* __restrict__ start,
+                                                      uint64_t cap, uint32_t* __restrict__ rows, ulonglong2* __restrict__ table, unsigned int* __restrict__ too_long) {
+    for (uint64_t h = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; h < cap; h += (uint64_t)gridDim.x * BLOCK) {
+        const unsigned len = count[h], at = start[h];
+        table[h] = len ? make_ulonglong2(keys(rep[h] - 1), ((unsigned long long)at << 32) | len) : make_ulonglong2(0, 0);
+        if (len > JOIN_GROUP_MAX) {
+            *too_long = 1;
+            continue;
+        }
+        for (unsigned a = 1; a < len; ++a) {  // insertion sort in place
+            const uint32_t v = rows[at + a];
+            unsigned b = a;
+            while (b && rows[at + b - 1] > v) {
+                rows[at + b] = rows[at + b - 1];
+                --b;
+            }
+            rows[at + b] = v;
+        }
+    }
+}
+__global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n, const ulonglong2* __restrict__ table, uint64_t mask, uint64_t* __restrict__ match) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint64_t key = probe(i);
+        uint64_t h = mix64(key) & mask, m = 0;
+        for (uint64_t p = 0; p <= mask; ++p) {  // bounded by the table size
+            const ulonglong2 s = __ldg(&table[h]);
+            if (s.y == 0) break;
+            if (s.x == key) {
+                m = s.y;
+                break;
+            }
+            h = (h + 1) & mask;
+        }
+        match[i] = m;
+    }
+}
+// Load-balanced output of an inner join (the scheme of expand_k), all columns of both sides written
+// at once: the pairs of row numbers never touch memory.
+__global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict__ match, const uint64_t* __restrict__ off, uint64_t nrows, uint64_t total, const uint32_t* __restrict__ rows,
+                                                    Cols cols) {
+    __shared__ unsigned rel[EX_TILE + 2];
+    __shared__ uint64_t row_s[2];
+    const uint64_t o0 = (uint64_t)blockIdx.x * EX_TILE, o1 = o0 + EX_TILE < total ? o0 + EX_TILE : total;
+    if (threadIdx.x < 64) {
+        const uint64_t o = threadIdx.x < 32 ? o0 : o0 + EX_TILE;
+        const uint64_t ub = o < total ? warp_partition_point(nrows, [&](uint64_t i) { return off[i] <= o; }) : nrows + 1;
+        if (lane_id() == 0) row_s[threadIdx.x >> 5] = ub - 1;
+    }
+    __syncthreads();
+    const uint64_t r0 = row_s[0], r1 = row_s[1] < nrows ? row_s[1] : nrows - 1, span = r1 - r0 + 1;
+    const bool in_smem = span <= (uint64_t)(EX_TILE + 2);
+    if (in_smem)
+        for (unsigned i = threadIdx.x; i < (unsigned)span; i += BLOCK) {
+            const uint64_t at = off[r0 + i];
+            rel[i] = at <= o0 ? 0u : (at - o0 < (uint64_t)EX_TILE ? (unsigned)(at - o0) : (unsigned)EX_TILE);
+        }
+    const uint64_t skip0 = o0 - off[r0];
+    __syncthreads();
+    for (unsigned t = threadIdx.x; t < (unsigned)(o1 - o0); t += BLOCK) {
+        uint64_t lo = 0, hi = span, j;
+        if (in_smem) {
+            while (lo < hi) {
+                const uint64_t mid = (lo + hi) >> 1;
+                if (rel[mid] <= t) lo = mid + 1;
+                else hi = mid;
+            }
+            j = lo == 1 ? skip0 + t : (uint64_t)(t - rel[lo - 1]);
+        } else {
+            while (lo < hi) {
+                const uint64_t mid = (lo + hi) >> 1;
+                if (off[r0 + mid] <= o0 + t) lo = mid + 1;
+                else hi = mid;
+            }
+            j = o0 + t - off[r0 + lo - 1];
+        }
+        const uint64_t l = r0 + lo - 1, r = rows[(match[l] >> 32) + j];
+        for (int k = 0; k < cols.n; ++k) copy_value(cols, k, k < cols.left ? l : r, o0 + t);
+    }
+}
+
+// ---- group-by over a small domain of keys: tables indexed by the key itself
+// Rows per key (the tile's rows are combined in shared memory first: one hub key would serialise
+// the atomics), whose maximum tells whether the values may be added up by atomics as well.
+struct GroupKey {
+    KeyCols cols;
+    int lo_bits;  // two columns: index = (a << lo_bits) | b
+    __device__ __forceinline__ uint32_t operator()(uint64_t i) const {
+        const uint64_t k = cols(i);
+        return cols.c1 ? (uint32_t)(((k >> 32) << lo_bits) | (k & 0xFFFFFFFFull)) : (uint32_t)k;
+    }
+};
+__global__ void __launch_bounds__(BLOCK) group_bound_k(KeyCols keys, uint64_t n, unsigned long long* __restrict__ bound) {
+    uint64_t o = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) o |= keys(i);
+#pragma unroll
+    for (int d = 16; d; d >>= 1) o |= __shfl_xor_sync(FULL, o, d);
+    if (lane_id() == 0 && o) atomicOr(bound, (unsigned long long)o);
+}
+__global__ void __launch_bounds__(BLOCK) group_rows_k(GroupKey key, uint64_t n, unsigned int* __restrict__ count) {
+    __shared__ uint32_t skey[DX_SLOTS], scnt[DX_SLOTS];
+    const uint64_t ntiles = (n + DX_TILE - 1) / DX_TILE;
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        for (int s = threadIdx.x; s < DX_SLOTS; s += BLOCK) {
+            skey[s] = DX_EMPTY;
+            scnt[s] = 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < DX_IPT; ++k) {
+            const uint64_t i = tile * DX_TILE + (uint64_t)k * BLOCK + threadIdx.x;
+            if (i >= n) break;
+            const uint32_t x = key(i), h = dx_slot(skey, x);
+            if (h != DX_NONE) atomicAdd(&scnt[h], 1u);
+            else atomicAdd(&count[x], 1u);
+        }
+        __syncthreads();
+        for (int s = threadIdx.x; s < DX_SLOTS; s += BLOCK)
+            if (scnt[s]) atomicAdd(&count[skey[s]], scnt[s]);
+        __syncthreads();
+    }
+}
+__global__ void __launch_bounds__(BLOCK) group_tiles_k(const unsigned int* __restrict__ count, uint64_t domain, uint32_t* __restrict__ tile_groups, unsigned long long* __restrict__ longest) {
+    __shared__ uint32_t sm[33];
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
+    uint32_t groups = 0, most = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; ++k) {
+        const uint64_t x = base + (uint64_t)k * BLOCK + threadIdx.x;
+        const uint32_t c = x < domain ? count[x] : 0u;
+        groups += c != 0;
+        most = c > most ? c : most;
+    }
+    most = __reduce_max_sync(FULL, most);
+    if (lane_id() == 0 && most) atomicMax(longest, (unsigned long long)most);
+    uint32_t tot;
+    block_exclusive_scan<uint32_t>(groups, &tot, sm);
+    if (threadIdx.x == 0) tile_groups[blockIdx.x] = tot;
+}
+struct Aggs {
+    const void* val[XLB_MAX_ARITY];
+    unsigned long long* table[XLB_MAX_ARITY];  // null: a count, which the row counts hold
+    void* out[XLB_MAX_ARITY];
+    uint8_t op[XLB_MAX_ARITY], width[XLB_MAX_ARITY], out_width[XLB_MAX_ARITY];
+    int n;
+};
+__global__ void __launch_bounds__(BLOCK) group_add_k(GroupKey key, uint64_t n, Aggs a) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint32_t x = key(i);
+        for (int q = 0; q < a.n; ++q) {
+            unsigned long long* t = a.table[q];
+            if (!t) continue;
+            const unsigned long long v = a.width[q] == 4 ? __ldg((const uint32_t*)a.val[q] + i) : __ldg((const unsigned long long*)a.val[q] + i);
+            // (a look first: once a group has settled most values change nothing; a stale look only costs an atomic)
+            if (a.op[q] == XLB_AGG_SUM) atomicAdd(&t[x], v);
+            else if (a.op[q] == XLB_AGG_MIN) {
+                if (v < t[x]) atomicMin(&t[x], v);
+            } else if (v > t[x]) atomicMax(&t[x], v);
+        }
+    }
+}
+__global__ void __launch_bounds__(BLOCK) group_emit_k(const unsigned int* __restrict__ count, uint64_t domain, const uint64_t* __restrict__ tile_offs, Aggs a, int lo_bits, int w0, void* key0,
+                                                     uint32_t* key1) {
+    __shared__ uint32_t sm[33];
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_IPT;
+    uint32_t c[SCAN_IPT], groups = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; ++k) {
+        c[k] = base + k < domain ? count[base + k] : 0u;
+        groups += c[k] != 0;
+    }
+    uint32_t tot;
+    uint64_t pos = tile_offs[blockIdx.x] + block_exclusive_scan<uint32_t>(groups, &tot, sm);
+    for (int k = 0; k < SCAN_IPT; ++k) {
+        if (!c[k]) continue;
+        const uint64_t x = base + k;
+        if (key1) {
+            ((uint32_t*)key0)[pos] = (uint32_t)(x >> lo_bits);
+            key1[pos] = (uint32_t)(x & ((1ull << lo_bits) - 1));
+        } else if (w0 == 4) ((uint32_t*)key0)[pos] = (uint32_t)x;
+        else ((unsigned long long*)key0)[pos] = x;
+        for (int q = 0; q < a.n; ++q) {
+            const unsigned long long v = a.table[q] ? a.table[q][x] : c[k];
+            if (a.out_width[q] == 4) ((uint32_t*)a.out[q])[pos] = (uint32_t)v;
+            else ((unsigned long long*)a.out[q])[pos] = v;
+        }
+        ++pos;
+    }
+}
+
+KeyCols key_cols(const xlb_rel* r, const uint32_t* keys, uint32_t nk) {
+    KeyCols k{r->cols[keys[0]]->p, nullptr, (int)type_width(r->schema.types[keys[0]])};
+    if (nk == 2) k.c1 = r->cols[keys[1]]->as<uint32_t>();
+    return k;
+}
+int bit_length(uint64_t v) { return v ? 64 - __builtin_clzll(v) : 0; }
+// out: a fresh relation of `rows` rows with the columns of `from` in place `at` and after
+void add_columns(xlb_ctx* c, xlb_rel* out, Cols& cols, const xlb_rel* from, uint64_t rows) {
+    for (uint32_t i = 0; i < from->schema.arity; ++i) {
+        const int k = cols.n++;
+        cols.width[k] = (int)type_width(from->schema.types[i]);
+        out->cols[k] = make_buf(c, rows * cols.width[k]);
+        cols.in[k] = from->cols[i]->p;
+        cols.out[k] = out->cols[k]->p;
+    }
+}
+
+}  // namespace
+
+xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, bool want) {
+    if (r->rows >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)r->rows);
+    uint64_t cap = 1024;
+    while (cap < 2 * r->rows) cap <<= 1;
+    Buf rep = make_buf(c, cap * 4);
+    CUDA_OK(set_async(c, rep->p, 0, cap * 4));
+    const KeyCols build = key_cols(r, rk, nk), probe = key_cols(l, lk, nk);
+    if (r->rows) {
+        prof_begin(c, "hash_insert", 0);
+        exists_build_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(build, r->rows, rep->as<unsigned int>(), cap - 1, c->d_status);
+        check_launch(c, "hash_insert");
+    }
+    const uint64_t n = l->rows, tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+    Buf bits = make_buf(c, (n + 31) / 32 * 4), counts = make_buf(c, tiles * 4), offs = make_buf(c, tiles * 8), total = make_buf(c, 8);
+    prof_begin(c, "hash_probe", n * 12ull);
+    exists_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, n, build, rep->as<unsigned int>(), cap - 1, want, bits->as<unsigned int>(), counts->as<uint32_t>());
+    check_launch(c, "hash_probe");
+    exclusive_scan<LoadU32, uint64_t>(c, LoadU32{counts->as<uint32_t>()}, tiles, offs->as<uint64_t>(), total->as<uint64_t>());
+    unsigned long long m;
+    read_words(c, total->p, 1, &m);
+    std::unique_ptr<xlb_rel> o(new xlb_rel);
+    o->ctx = c;
+    o->schema = l->schema;
+    o->rows = m;
+    Cols cols{};
+    add_columns(c, o.get(), cols, l, m);
+    if (m) {
+        prof_begin(c, "select_rows", 0);
+        select_rows_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(cols, bits->as<unsigned int>(), n, offs->as<uint64_t>());
+        check_launch(c, "select_rows");
+    }
+    return o.release();
+}
+
+xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, const xlb_schema& os) {
+    const uint64_t n = r->rows;
+    if (n >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)n);
+    uint64_t cap = 1024;
+    while (cap < 2 * n) cap <<= 1;
+    const KeyCols build = key_cols(r, rk, nk), probe = key_cols(l, lk, nk);
+    Buf slots = make_buf(c, cap * 8), start = make_buf(c, cap * 4), place = make_buf(c, n * 8), rows = make_buf(c, n * 4), table = make_buf(c, cap * 16), words = make_buf(c, 24);
+    unsigned int *rep = slots->as<unsigned int>(), *count = rep + cap;
+    CUDA_OK(set_async(c, slots->p, 0, cap * 8));
+    CUDA_OK(set_async(c, words->p, 0, 24));  // [0] outputs, [1] a group is too long, [2] rows grouped
+    prof_begin(c, "hash_insert", n * 8ull);
+    group_count_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, rep, count, cap - 1, place->as<uint2>(), c->d_status);
+    check_launch(c, "hash_insert");
+    exclusive_scan<LoadU32, uint32_t>(c, LoadU32{count}, cap, start->as<uint32_t>(), (uint32_t*)(words->as<uint64_t>() + 2));
+    prof_begin(c, "group_fill", n * 16ull);
+    group_fill_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(place->as<uint2>(), n, start->as<uint32_t>(), rows->as<uint32_t>());
+    check_launch(c, "group_fill");
+    prof_begin(c, "group_order", cap * 24ull);
+    group_order_k<<<grid_for(c, cap), BLOCK, 0, c->stream>>>(build, rep, count, start->as<uint32_t>(), cap, rows->as<uint32_t>(), table->as<ulonglong2>(),
+                                                            (unsigned int*)(words->as<uint64_t>() + 1));
+    check_launch(c, "group_order");
+    Buf match = make_buf(c, l->rows * 8), off = make_buf(c, l->rows * 8);
+    prof_begin(c, "hash_probe", l->rows * 32ull);
+    join_probe_k<<<grid_for(c, l->rows), BLOCK, 0, c->stream>>>(probe, l->rows, table->as<ulonglong2>(), cap - 1, match->as<uint64_t>());
+    check_launch(c, "hash_probe");
+    exclusive_scan<LoadLow32, uint64_t>(c, LoadLow32{match->as<uint64_t>()}, l->rows, off->as<uint64_t>(), words->as<uint64_t>());
+    unsigned long long w[2];
+    read_words(c, words->p, 2, w);
+    if (w[1]) return nullptr;
+    std::unique_ptr<xlb_rel> o(new xlb_rel);
+    o->ctx = c;
+    o->schema = os;
+    o->rows = w[0];
+    Cols cols{};
+    cols.left = (int)l->schema.arity;
+    add_columns(c, o.get(), cols, l, w[0]);
+    add_columns(c, o.get(), cols, r, w[0]);
+    if (w[0]) {
+        prof_begin(c, "join_emit", 0);
+        join_emit_k<<<(unsigned)((w[0] + EX_TILE - 1) / EX_TILE), BLOCK, 0, c->stream>>>(match->as<uint64_t>(), off->as<uint64_t>(), l->rows, w[0], rows->as<uint32_t>(), cols);
+        check_launch(c, "join_emit");
+    }
+    return o.release();
+}
+
+// The tables cost a clear and a pass over the domain, four entries a row at most; groups of more
+// than 2^16 rows would queue their atomics for longer (80 us) than the sort of a few million rows takes.
+constexpr int GROUP_BITS_MAX = 26;
+constexpr uint64_t GROUP_DOMAIN_FREE = 1ull << 16, GROUP_ROWS_MAX = 1ull << 16;
+
+xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_in, uint32_t nk, const uint32_t* agg_cols, const uint32_t* agg_ops, uint32_t na, const xlb_schema& os) {
+    if (nk > 2 || (nk == 2 && (type_width(in->schema.types[key_cols_in[0]]) != 4 || type_width(in->schema.types[key_cols_in[1]]) != 4))) return nullptr;
+    const uint64_t n = in->rows;
+    GroupKey key{key_cols(in, key_cols_in, nk), 0};
+    Buf words = make_buf(c, 24);  // [0] key bound, [1] groups, [2] rows of the largest
+    CUDA_OK(set_async(c, words->p, 0, 24));
+    prof_begin(c, "group_bound", 0);
+    group_bound_k<<<grid_for(c, n, BLOCK * 4), BLOCK, 0, c->stream>>>(key.cols, n, words->as<unsigned long long>());
+    check_launch(c, "group_bound");
+    unsigned long long w[2];
+    read_words(c, words->p, 1, w);
+    int bits = bit_length(w[0]);
+    if (nk == 2) {
+        key.lo_bits = std::max(bit_length(w[0] & 0xFFFFFFFFull), 1);
+        bits = bit_length(w[0] >> 32) + key.lo_bits;
+    }
+    if (bits > GROUP_BITS_MAX || (1ull << bits) > std::max<uint64_t>(4 * n, GROUP_DOMAIN_FREE)) return nullptr;
+    const uint64_t domain = 1ull << bits, tiles = (domain + SCAN_TILE - 1) / SCAN_TILE;
+    Buf count = make_buf(c, domain * 4), tile_groups = make_buf(c, tiles * 4), offs = make_buf(c, tiles * 8);
+    CUDA_OK(set_async(c, count->p, 0, domain * 4));
+    prof_begin(c, "group_rows", 0);
+    group_rows_k<<<grid_for(c, n, DX_TILE), BLOCK, 0, c->stream>>>(key, n, count->as<unsigned int>());
+    check_launch(c, "group_rows");
+    prof_begin(c, "group_tiles", domain * 4ull);
+    group_tiles_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(count->as<unsigned int>(), domain, tile_groups->as<uint32_t>(), words->as<unsigned long long>() + 2);
+    check_launch(c, "group_tiles");
+    exclusive_scan<LoadU32, uint64_t>(c, LoadU32{tile_groups->as<uint32_t>()}, tiles, offs->as<uint64_t>(), words->as<uint64_t>() + 1);
+    read_words(c, words->as<uint64_t>() + 1, 2, w);
+    const uint64_t m = w[0];
+    uint32_t tables = 0;
+    for (uint32_t a = 0; a < na; ++a) tables += agg_ops[a] != XLB_AGG_COUNT;
+    if (tables && w[1] > GROUP_ROWS_MAX) return nullptr;
+    std::unique_ptr<xlb_rel> o(new xlb_rel);
+    o->ctx = c;
+    o->schema = os;
+    o->rows = m;
+    for (uint32_t i = 0; i < os.arity; ++i) o->cols[i] = make_buf(c, m * type_width(os.types[i]));
+    // sums and maxima start from zero, minima from all ones: two fills
+    Buf acc = make_buf(c, std::max<uint64_t>(tables * domain * 8, 8));
+    Aggs ag{};
+    ag.n = (int)na;
+    uint64_t at = 0, minima = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (uint32_t a = 0; a < na; ++a) {
+            if (agg_ops[a] == XLB_AGG_COUNT || (agg_ops[a] == XLB_AGG_MIN) != (pass == 1)) continue;
+            ag.table[a] = acc->as<unsigned long long>() + at;
+            at += domain;
+        }
+        if (pass == 0) minima = at;
+    }
+    if (minima) CUDA_OK(set_async(c, acc->p, 0, minima * 8));
+    if (at > minima) CUDA_OK(set_async(c, acc->as<uint64_t>() + minima, 0xFF, (at - minima) * 8));
+    for (uint32_t a = 0; a < na; ++a) {
+        ag.val[a] = in->cols[agg_cols[a]]->p;
+        ag.op[a] = (uint8_t)agg_ops[a];
+        ag.width[a] = (uint8_t)type_width(in->schema.types[agg_cols[a]]);
+        ag.out[a] = o->cols[nk + a]->p;
+        ag.out_width[a] = (uint8_t)type_width(os.types[nk + a]);
+    }
+    if (tables) {
+        prof_begin(c, "groupby_reduce", 0);
+        group_add_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(key, n, ag);
+        check_launch(c, "groupby_reduce");
+    }
+    prof_begin(c, "group_emit", 0);
+    group_emit_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(count->as<unsigned int>(), domain, offs->as<uint64_t>(), ag, key.lo_bits, (int)type_width(os.types[0]), o->cols[0]->p,
+                                                          nk == 2 ? o->cols[1]->as<uint32_t>() : nullptr);
+    check_launch(c, "group_emit");
+    return o.release();
+}
