@@ -465,7 +465,7 @@ __device__ __forceinline__ void take_square(const Out& o, const Square& sq, uint
 #pragma unroll
                     for (int k = 0; k < SQ_UNROLL; ++k) {
                         const bool in = k < items && w < row_words;
-                        m[k] = in ? __ldcg(reinterpret_cast<const unsigned long long*>(bits + f[k] + w)) : 0ull;  // (what the last iteration left: never from the L1)
+                        m[k] = in ? *reinterpret_cast<const unsigned long long*>(bits + f[k] + w) : 0ull;        // (the barrier's fence has emptied the L1)
                         have[k] = in ? *reinterpret_cast<const unsigned long long*>(bits + kn[k] + w) : 0ull;     // (a stale line only costs an atomic)
                     }
                     uint64_t any = 0;
@@ -664,11 +664,13 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
         if (threadIdx.x == 0) {
             const unsigned w = v->sync;
             __threadfence();
+            const unsigned long long a = v->start, b = v->end;
+            const unsigned c = v->check;
             generation = w >> 3;
             phase_s = w & 7;
-            range_s[0] = v->start;
-            range_s[1] = v->end;
-            check_s = v->check;
+            range_s[0] = a;
+            range_s[1] = b;
+            check_s = c;
         }
         __syncthreads();
     };
@@ -825,8 +827,18 @@ __device__ __forceinline__ void flush(const Out& o, const uint64_t* stage, unsig
     __syncwarp();
     staged = 0;
 }
+__device__ __forceinline__ void ready(Ctl* ctl, bool square) {
+    volatile Ctl* c = ctl;
+    const unsigned long long n = c->tail;
+    c->check = 1;
+    c->start = 0;
+    c->end = n;
+    c->iterations = n == 0 ? 1 : 0;  // an iteration over nothing finds nothing
+    c->fix = n == 0 ? 1 : 0;
+    c->sync = n == 0 ? PH_DONE : square ? PH_FULL : PH_ROWS;  // (never solo: a block that starts late would miss it)
+}
 // Rows of a bag into the head: new ones (their bit was clear) are appended to the log.
-__global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict__ rows, uint64_t n, Out o) {
+__global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict__ rows, uint64_t n, Out o, bool square) {
     __shared__ uint64_t stage_s[BLOCK / 32][64];
     uint64_t* stage = stage_s[threadIdx.x >> 5];
     const uint64_t step = (uint64_t)gridDim.x * BLOCK;
@@ -850,19 +862,19 @@ __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict
         if (staged > 32) flush(o, stage, staged);
     }
     flush(o, stage, staged);
+    // the block that finishes last leaves the loop ready to start on what has been seeded so far
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&o.ctl->arrived, 1u) == gridDim.x - 1) {
+            __threadfence();
+            o.ctl->arrived = 0;
+            ready(o.ctl, square);
+        }
+    }
 }
 
-__global__ void delta_begin_k(Ctl* c, bool square) {
-    const unsigned long long n = c->tail;
-    c->check = 1;
-    c->start = 0;
-    c->end = n;
-    if (n == 0) {  // an iteration over nothing finds nothing
-        c->iterations = 1;
-        c->fix = 1;
-    }
-    c->sync = n == 0 ? PH_DONE : square ? PH_FULL : PH_ROWS;  // (never solo: a block that starts late would miss it)
-}
+__global__ void delta_begin_k(Ctl* c, bool square) { ready(c, square); }
 
 // On with the delta at hand, once the log has the room for it.
 __global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
@@ -873,7 +885,7 @@ __global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
 }  // namespace
 
 static Out out_of(xlb_ctx* c, const DeltaLoop& d) {
-    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, d.ctl->as<Ctl>(), c->d_status, d.square ? d.visited->as<unsigned int>() + d.words : nullptr};
+    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, (Ctl*)d.ctl, c->d_status, d.square ? d.visited->as<unsigned int>() + d.words : nullptr};
 }
 
 DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square, int composites) {
@@ -882,10 +894,11 @@ DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square, int
     d.lo_bits = lo_bits;
     d.square = square;
     d.words = ((1ull << (hi_bits + lo_bits)) + 31) / 32;
-    d.visited = make_buf(c, std::max<uint64_t>(d.words * 4, 16) * (square ? 4 + composites : 1));
-    d.ctl = make_buf(c, sizeof(Ctl));
+    // the bitmaps, then the control block: one fill for both
+    const uint64_t bitmaps = std::max<uint64_t>(d.words * 4, 16) * (square ? 4 + composites : 1);
+    d.visited = make_buf(c, bitmaps + sizeof(Ctl));
+    d.ctl = (char*)d.visited->p + bitmaps;
     CUDA_OK(set_async(c, d.visited->p, 0, d.visited->bytes));
-    CUDA_OK(set_async(c, d.ctl->p, 0, sizeof(Ctl)));
     return d;
 }
 
@@ -917,7 +930,8 @@ void ops_delta_seed(xlb_ctx* c, DeltaLoop& d, const Keys& bag) {
     if (!bag.n) return;
     log_room(c, d, bag.n);
     prof_begin(c, "dense_mark", bag.n * 16ull);
-    delta_seed_k<<<grid_for(c, bag.n), BLOCK, 0, c->stream>>>(bag.ptr(), bag.n, out_of(c, d));
+    delta_seed_k<<<grid_for(c, bag.n), BLOCK, 0, c->stream>>>(bag.ptr(), bag.n, out_of(c, d), d.square);
+    d.seeded = true;
     check_launch(c, "dense_mark");
 }
 
@@ -927,7 +941,7 @@ void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows) {
     CUDA_OK(copy_async(c, d.log->as<uint64_t>() + (d.room - rows.n), rows.ptr(), rows.n * 8, cudaMemcpyDeviceToDevice));
     const unsigned long long tail = d.room;
     c->h_scalar[48] = tail;
-    CUDA_OK(copy_async(c, &d.ctl->as<Ctl>()->tail, &c->h_scalar[48], 8, cudaMemcpyHostToDevice));
+    CUDA_OK(copy_async(c, &((Ctl*)d.ctl)->tail, &c->h_scalar[48], 8, cudaMemcpyHostToDevice));
     stream_wait(c);  // (the staging word is used again)
 }
 
@@ -961,7 +975,7 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
                 v.rows = (in.rows == DeltaVariant::HEAD ? 2 : 3) * sq.words;
                 continue;
             }
-            if (sq.n_aux == SQ_AUX || d.visited->bytes < (uint64_t)(5 + sq.n_aux) * sq.words * 4) xlb_fail(XLB_ERR_INVALID, "internal: too many composites in a delta loop");
+            if (sq.n_aux == SQ_AUX || d.visited->bytes < (uint64_t)(5 + sq.n_aux) * sq.words * 4 + sizeof(Ctl)) xlb_fail(XLB_ERR_INVALID, "internal: too many composites in a delta loop");
             Buf b = make_buf(c, 8ull << sq.bits);
             CUDA_OK(set_async(c, b->p, 0, b->bytes));
             counts.push_back(b);
@@ -987,8 +1001,10 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         }
     }
     Buf heavy = make_buf(c, (uint64_t)DL_HEAVY_MAX * sizeof(Heavy));
-    delta_begin_k<<<1, 1, 0, c->stream>>>(d.ctl->as<Ctl>(), square);
-    check_launch(c, "delta_begin");
+    if (!d.seeded) {
+        delta_begin_k<<<1, 1, 0, c->stream>>>((Ctl*)d.ctl, square);
+        check_launch(c, "delta_begin");
+    }
     for (;;) {
         Out o = out_of(c, d);
         Heavy* hp = heavy->as<Heavy>();
@@ -997,7 +1013,7 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         CUDA_OK(cudaLaunchCooperativeKernel(square ? (const void*)delta_loop_k<true> : (const void*)delta_loop_k<false>, dim3((unsigned)c->sm_count), dim3(DL_THREADS), args, DL_SMEM, c->stream));
         check_launch(c, "expand_mark");
         unsigned long long w[7];  // tail, start, end, iterations, candidates, fix, overflow
-        read_words(c, d.ctl->p, 7, w);
+        read_words(c, d.ctl, 7, w);
         if (c->status_code) return false;
         res->rows = w[0];
         res->iterations = w[3];
@@ -1037,7 +1053,7 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         log_room(c, d, tail);
         CUDA_OK(copy_async(c, d.log->as<uint64_t>() + stored, rows.ptr(), rows.n * 8, cudaMemcpyDeviceToDevice));
         d.room = tail;
-        delta_resume_k<<<1, 1, 0, c->stream>>>(d.ctl->as<Ctl>(), max_iterations, square);
+        delta_resume_k<<<1, 1, 0, c->stream>>>((Ctl*)d.ctl, max_iterations, square);
         check_launch(c, "delta_resume");
     }
 }

@@ -271,6 +271,9 @@ struct RunState {
     // heads of 28 to 32 bits that moved from the hash set to bitmaps: an iteration brought more
     // candidates than a 256th of the domain, from where on passes over the bitmaps are the cheaper dedup
     std::set<std::string> wide_dense;
+    // something reads the packed rows of a finished head next (a later component, a decoding); without
+    // it the head is written out as the columns that it is fetched as
+    bool packed_results = false;
     std::set<std::string> keep_cols;  // stored relations a frontier loop will stream over as columns: not packed ahead of it
     // Several ranks.  Relations whose rows every rank holds in full while the running component is
     // evaluated: full copies of small stored relations (kept in the store under an alias name) and,
@@ -1723,7 +1726,10 @@ static void frontier_loop(xlb_ctx* c, const FrontierPlan& fp, const std::string&
     // back to lists: the head in order off its bitmap, and the last iteration's tuples as the delta
     {
         PhaseTimer t(c, &rs.st.ms_setops);
-        if (ds->rows != full.n) install_full(c, p, hs, ops_dense_state_rows(c, *ds, domain - 1), nullptr, rs);
+        if (ds->rows != full.n) {
+            if (fix && !rs.packed_results && !rs.repl.on) store_put(c, p, ops_dense_state_columns(c, *ds, hs));
+            else install_full(c, p, hs, ops_dense_state_rows(c, *ds, domain - 1), nullptr, rs);
+        }
         Keys d;
         d.buf = make_buf(c, 0);
         if (last_new) {
@@ -1894,13 +1900,18 @@ static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const st
 
 // OR bounds of the head's two halves over everything the component can derive, from the bounds of the
 // relations it reads and of the rows the head starts with.  False: some bound is not known.
-static bool delta_bounds(xlb_ctx* c, const std::vector<FlatRule>& rules, const std::string& p, RunState& rs, uint64_t start, uint64_t* bound) {
+static bool delta_bounds(xlb_ctx* c, const std::vector<FlatRule>& rules, const std::string& p, uint64_t start, uint64_t* bound) {
     uint64_t hi = start >> 32, lo = start & 0xFFFFFFFFull;
     std::map<std::string, uint64_t> known;
+    std::vector<const xlb_rel*> stored;
+    for (auto& fr : rules)
+        for (auto& a : fr.atoms)
+            if (a.rel != p) stored.push_back(store_get(c, a.rel));
+    ops_pack_all(c, stored);
     for (auto& fr : rules)
         for (auto& a : fr.atoms)
             if (a.rel != p && !known.count(a.rel)) {
-                const Keys k = packed_for_rules(c, a.rel, rules, rs);
+                const Keys k = ops_rel_packed(c, store_get(c, a.rel));
                 if (k.n && k.bound == ~0ull) return false;
                 known[a.rel] = k.n ? k.bound : 0;
             }
@@ -1940,7 +1951,7 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
             full = real_full(c, rs, p);
         }
         uint64_t bound = 0;
-        if (!delta_bounds(c, rules, p, rs, full.n ? full.bound : 0, &bound)) return false;
+        if (!delta_bounds(c, rules, p, full.n ? full.bound : 0, &bound)) return false;
         int hb = bit_len(bound >> 32), lb = std::max(bit_len(bound & 0xFFFFFFFFull), 1);
         const bool square = !plan.square.empty();
         if (square) {
@@ -2032,13 +2043,53 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         ds.hi_bits = hb;
         ds.lo_bits = lb;
         ds.rows = full.n + res.rows - delta.n;  // (a delta taken from the store is part of the stored head)
-        install_full(c, p, hs, ops_dense_state_rows(c, ds, bound), nullptr, rs);
+        if (rs.packed_results) install_full(c, p, hs, ops_dense_state_rows(c, ds, bound), nullptr, rs);
+        else store_put(c, p, ops_dense_state_columns(c, ds, hs));
         return true;
     } catch (const XlbError& e) {
         if (e.st != XLB_ERR_RESOURCE_EXHAUSTED) throw;
         rs.st = before;  // not enough memory for a bitmap and a log: the routes that work in pieces take over
         return false;
     }
+}
+
+// A component that ops_frontier_whole takes: the frontier rule, and seeds that filter the relation it
+// streams over by a constant.  True: done.  (Not when the caller wants the phases timed: one kernel has
+// none that could be told apart.)
+static bool frontier_whole(xlb_ctx* c, const std::vector<FlatRule>& rules, const FrontierPlan& fp, const std::string& p, const xlb_schema& hs, RunState& rs, bool& fix) {
+    const Atom& ea = fp.fr->atoms[fp.ei];
+    xlb_rel* er = store_get(c, ea.rel);
+    if (c->flags & XLB_FLAG_PROFILE) return false;
+    if (!er || er->packed || er->schema.arity != 2 || !rel_packable(er->schema)) return false;
+    std::vector<FrontierConst> seeds;
+    for (auto& fr : rules) {
+        if (&fr == fp.fr) continue;
+        int col;
+        uint64_t value;
+        size_t which;
+        if (fr.atoms.size() != 1 || fr.atoms[0].rel != ea.rel || fr.filters.size() != 1 || !fr.checks.empty() || fr.head_vars.size() != 1 ||
+            !single_atom_filter(fr, &col, &value, &which))
+            return false;
+        const int take = fr.head_vars[0] == fr.atoms[0].var[0] ? 0 : fr.head_vars[0] == fr.atoms[0].var[1] ? 1 : -1;
+        if (take < 0) return false;
+        seeds.push_back({col, take, (uint32_t)value});
+    }
+    FrontierWhole res;
+    {
+        PhaseTimer t(c, &rs.st.ms_join);
+        if (!ops_frontier_whole(c, er, fp.kc, fp.rel_lo == 0 ? fp.kc : 1 - fp.kc, seeds, c->max_iterations, &res)) return false;
+    }
+    rs.st.iterations += res.iterations;
+    rs.st.candidate_tuples += res.candidates;
+    fix = res.fix;
+    std::unique_ptr<xlb_rel> out(new xlb_rel);
+    out->ctx = c;
+    out->schema = hs;
+    out->rows = res.rows;
+    out->canonical = true;
+    out->cols[0] = res.values;
+    store_put(c, p, out.release());
+    return true;
 }
 
 static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
@@ -2176,6 +2227,13 @@ static void run_scc(xlb_ctx* c, const xlb_scc& scc, RunState& rs) {
     DeltaPlan deltas;
     const bool delta_ok = scc.is_recursive && delta_shape(c, rules, preds, rec, schema, &deltas);
     auto limit_reached = [&]() { xlb_fail(XLB_ERR_ITER_LIMIT, "Recursive SCC iteration limit (%llu) exceeded", (unsigned long long)c->max_iterations); };
+    if (scc.is_recursive && c->comm_world == 1 && !resume && preds.size() == 1 && store_get(c, preds[0])->rows == 0) {
+        FrontierPlan fp;
+        if (frontier_shape(c, rules, preds, rec, schema, rs, &fp) && frontier_whole(c, rules, fp, preds[0], schema[preds[0]], rs, fix)) {
+            if (!fix) limit_reached();
+            return;
+        }
+    }
     if (delta_ok && !resume && store_get(c, preds[0])->rows == 0) {
         FrontierPlan fp;  // (a frontier that streams over an unindexed relation needs no index at all)
         if (!frontier_shape(c, rules, preds, rec, schema, rs, &fp) && delta_loop(c, deltas, rules, preds[0], schema[preds[0]], false, rs, it, fix)) {
@@ -2415,9 +2473,10 @@ struct EncodedRun {
             rows += r->rows;
         }
         if (rows < SPARSE_ROWS_MIN || rows > SPARSE_ROWS_MAX) return false;
+        ops_pack_all(c, rels);  // (kept: what the plan itself would start with)
         for (const xlb_rel* r : rels) {
             if (!r->rows) continue;
-            const Keys k = ops_rel_packed(c, r);  // (kept: what the plan itself would start with)
+            const Keys k = ops_rel_packed(c, r);
             if (k.bound == ~0ull) return false;
             bound |= (k.bound >> 32) | (k.bound & 0xFFFFFFFFull);
         }
@@ -2573,6 +2632,7 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
         if (!plan->sccs && plan->n_sccs) xlb_fail(XLB_ERR_INVALID, "plan has no SCC array");
         std::set<std::string> heads;
         const xlb_plan* run = enc.begin(c, plan);
+        rs.packed_results = enc.narrow || run->n_sccs > 1;
         for (uint32_t s = 0; s < run->n_sccs; ++s) {
             run_scc(c, run->sccs[s], rs);
             for (uint32_t i = 0; i < run->sccs[s].n_rules; ++i) heads.insert(run->sccs[s].rules[i].head);

@@ -398,6 +398,48 @@ uint64_t select_unordered(xlb_ctx* c, Pred pred, Emit emit, uint64_t n, const ch
 // With `fcol` >= 0 the rows whose column fcol equals fval are also appended, packed, to `fout` in
 // no particular order (*fcount += their number): a rule that reads `rel(c, Y)` from a relation that
 // is packed for the first time gets its rows without a second pass over the relation.
+// (all threads of the block) acc joins *or_out: thousands of warps that each sent an atomic to the one
+// word queued on it for longer than the pass took, so a block sends one, and none once its bits are there
+__device__ __forceinline__ void block_or(uint64_t acc, unsigned long long* or_out) {
+    __shared__ unsigned or_s[2];
+    if (threadIdx.x < 2) or_s[threadIdx.x] = 0;
+    __syncthreads();
+    const unsigned lo = __reduce_or_sync(FULL, (unsigned)acc), hi = __reduce_or_sync(FULL, (unsigned)(acc >> 32));
+    if (lane_id() == 0) {
+        if (lo) atomicOr(&or_s[0], lo);
+        if (hi) atomicOr(&or_s[1], hi);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned long long all = ((unsigned long long)or_s[1] << 32) | or_s[0];
+        if ((*(volatile unsigned long long*)or_out & all) != all) atomicOr(or_out, all);
+    }
+}
+// Rows that match a constant, collected by the block in shared memory and appended to `fout` with one
+// atomic when it is done (a hub's 69 K rows, each with an atomic of its own, held the sweep over 16 M
+// rows at 54 us).  begin() and end() by all threads of the block, keep() by any.
+struct FilterStage {
+    static constexpr unsigned CAP = 512;  // more matches in one block go out one by one
+    uint64_t rows[CAP];
+    unsigned n;
+    unsigned long long base;
+    __device__ __forceinline__ void begin() {
+        if (threadIdx.x == 0) n = 0;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void keep(uint64_t row, uint64_t* fout, unsigned long long* fcount) {
+        const unsigned at = atomicAdd(&n, 1u);
+        if (at < CAP) rows[at] = row;
+        else fout[atomicAdd(fcount, 1ull)] = row;
+    }
+    __device__ __forceinline__ void end(uint64_t* fout, unsigned long long* fcount) {
+        __syncthreads();
+        const unsigned have = n < CAP ? n : CAP;
+        if (threadIdx.x == 0 && have) base = atomicAdd(fcount, (unsigned long long)have);
+        __syncthreads();
+        for (unsigned i = threadIdx.x; i < have; i += blockDim.x) fout[base + i] = rows[i];
+    }
+};
 static __global__ void pack2_k(const uint32_t* __restrict__ c0, const uint32_t* __restrict__ c1, uint64_t* __restrict__ out, uint64_t n, unsigned long long* or_out,
                                bool vec, int fcol = -1, uint32_t fval = 0, uint64_t* __restrict__ fout = nullptr, unsigned long long* fcount = nullptr) {
     uint64_t acc = 0;
@@ -405,8 +447,10 @@ static __global__ void pack2_k(const uint32_t* __restrict__ c0, const uint32_t* 
     const uint4* a4 = reinterpret_cast<const uint4*>(c0);
     const uint4* b4 = reinterpret_cast<const uint4*>(c1);
     ulonglong2* o2 = reinterpret_cast<ulonglong2*>(out);
+    __shared__ FilterStage stage;
+    if (fcol >= 0) stage.begin();
     auto keep = [&](uint32_t a, uint32_t b) {
-        if (fcol >= 0 && (fcol == 0 ? a : b) == fval) fout[atomicAdd(fcount, 1ull)] = ((uint64_t)a << 32) | b;  // a few rows out of millions
+        if (fcol >= 0 && (fcol == 0 ? a : b) == fval) stage.keep(((uint64_t)a << 32) | b, fout, fcount);
     };
     for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (uint64_t)gridDim.x * blockDim.x) {
         uint4 a = a4[q], b = b4[q];
@@ -436,9 +480,8 @@ static __global__ void pack2_k(const uint32_t* __restrict__ c0, const uint32_t* 
         acc |= k;
         keep(c0[i], c1[i]);
     }
-#pragma unroll
-    for (int d = 16; d; d >>= 1) acc |= __shfl_xor_sync(FULL, acc, d);
-    if (or_out && lane_id() == 0 && acc) atomicOr(or_out, (unsigned long long)acc);
+    if (fcol >= 0) stage.end(fout, fcount);
+    if (or_out) block_or(acc, or_out);
 }
 // The read-only sweep of a two-column relation that is not packed: OR of the packed rows into
 // *or_out, and with fcol >= 0 the rows whose column fcol equals fval appended, packed, to `fout`
@@ -447,8 +490,10 @@ static __global__ void pack2_k(const uint32_t* __restrict__ c0, const uint32_t* 
 static __global__ void __launch_bounds__(BLOCK) cols_or_filter_k(const uint32_t* __restrict__ c0, const uint32_t* __restrict__ c1, uint64_t n, unsigned long long* or_out, int fcol,
                                                             uint32_t fval, uint64_t* __restrict__ fout, unsigned long long* fcount) {
     uint32_t acc0 = 0, acc1 = 0;
+    __shared__ FilterStage stage;
+    if (fcol >= 0) stage.begin();
     auto keep = [&](uint32_t a, uint32_t b) {
-        if ((fcol == 0 ? a : b) == fval) fout[atomicAdd(fcount, 1ull)] = ((uint64_t)a << 32) | b;
+        if ((fcol == 0 ? a : b) == fval) stage.keep(((uint64_t)a << 32) | b, fout, fcount);
     };
     constexpr int V = 4;  // 16-byte words per column, thread and step
     const uint64_t per_step = (uint64_t)BLOCK * V * 4;
@@ -483,10 +528,9 @@ static __global__ void __launch_bounds__(BLOCK) cols_or_filter_k(const uint32_t*
         acc1 |= b;
         if (fcol >= 0) keep(a, b);
     }
+    if (fcol >= 0) stage.end(fout, fcount);
     uint64_t acc = ((uint64_t)acc0 << 32) | acc1;
-#pragma unroll
-    for (int d = 16; d; d >>= 1) acc |= __shfl_xor_sync(FULL, acc, d);
-    if (lane_id() == 0 && acc) atomicOr(or_out, (unsigned long long)acc);
+    block_or(acc, or_out);
 }
 static __global__ void pack1_k(const uint32_t* __restrict__ c0, uint64_t* __restrict__ out, uint64_t n, unsigned long long* or_out) {
     uint64_t acc = 0;
@@ -494,9 +538,7 @@ static __global__ void pack1_k(const uint32_t* __restrict__ c0, uint64_t* __rest
         out[i] = c0[i];
         acc |= c0[i];
     }
-#pragma unroll
-    for (int d = 16; d; d >>= 1) acc |= __shfl_xor_sync(FULL, acc, d);
-    if (or_out && lane_id() == 0 && acc) atomicOr(or_out, (unsigned long long)acc);
+    if (or_out) block_or(acc, or_out);
 }
 static __global__ void unpack2_k(const uint64_t* __restrict__ in, uint32_t* __restrict__ c0, uint32_t* __restrict__ c1, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -1263,7 +1305,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_count_k(const unsigned int
 constexpr int DENSE_FUSED_GROUPS = 8192;
 static __global__ void __launch_bounds__(BLOCK) dense_count_scan_k(const unsigned int* __restrict__ bitmap, uint64_t words, uint32_t* group_counts, uint64_t groups,
                                                               const unsigned int* __restrict__ visited, uint64_t* __restrict__ group_offs, uint64_t* total,
-                                                              unsigned int* ticket) {
+                                                              unsigned int* ticket, bool check, uint64_t expected, DevStatus* st) {
     __shared__ uint64_t sm[33];
     __shared__ bool last_s;
     uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1293,11 +1335,21 @@ static __global__ void __launch_bounds__(BLOCK) dense_count_scan_k(const unsigne
     if (threadIdx.x == 0) {
         *total = tot;
         *ticket = 0;
+        if (check && tot != expected) set_status(st, XLB_ERR_CAPACITY, 9, tot);
     }
+}
+// One tuple out: packed, or (out0 set) as a row of columns, which is what a result that is fetched
+// next is wanted as.
+__device__ __forceinline__ void dense_put(uint64_t x, int lo_bits, uint64_t lo_mask, uint64_t pos, uint64_t* out, uint32_t* out0, uint32_t* out1) {
+    if (!out0) out[pos] = ((x >> lo_bits) << 32) | (x & lo_mask);
+    else if (out1) {
+        out0[pos] = (uint32_t)(x >> lo_bits);
+        out1[pos] = (uint32_t)(x & lo_mask);
+    } else out0[pos] = (uint32_t)x;
 }
 static __global__ void __launch_bounds__(BLOCK) dense_emit_k(const unsigned int* __restrict__ bitmap, uint64_t words, const uint64_t* __restrict__ group_offs,
                                                            uint64_t groups, int lo_bits, uint64_t* __restrict__ out, unsigned int* __restrict__ visited,
-                                                           uint64_t cap, DevStatus* st) {
+                                                           uint64_t cap, DevStatus* st, uint32_t* __restrict__ out0 = nullptr, uint32_t* __restrict__ out1 = nullptr) {
     uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (g >= groups) return;
     const unsigned lane = lane_id();
@@ -1324,7 +1376,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_emit_k(const unsigned int*
             set_status(st, XLB_ERR_CAPACITY, 8, pos);
             break;
         }
-        out[pos++] = ((x >> lo_bits) << 32) | (x & lo_mask);
+        dense_put(x, lo_bits, lo_mask, pos++, out, out0, out1);
     }
 }
 
@@ -1358,7 +1410,8 @@ static __global__ void __launch_bounds__(BLOCK) dense_count_wide_k(const unsigne
 }
 static __global__ void __launch_bounds__(BLOCK) dense_emit_wide_k(const unsigned int* __restrict__ bitmap, const uint64_t* __restrict__ group_offs, uint64_t groups, int lo_bits,
                                                              uint64_t* __restrict__ out, unsigned int* __restrict__ visited, uint64_t cap, DevStatus* st,
-                                                             const unsigned char* __restrict__ touched) {
+                                                             const unsigned char* __restrict__ touched, uint32_t* __restrict__ out0 = nullptr,
+                                                             uint32_t* __restrict__ out1 = nullptr) {
     const uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (g >= groups) return;
     if (touched && !touched[g]) return;
@@ -1414,7 +1467,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_emit_wide_k(const unsigned
                 if (!word) continue;
                 if ((word >> lane) & 1u) {
                     const uint64_t x = ((((g * 32 + owner) * DW_WPL) + i) << 5) | lane;
-                    out[base + __popc(word & below)] = ((x >> lo_bits) << 32) | (x & lo_mask);
+                    dense_put(x, lo_bits, lo_mask, base + __popc(word & below), out, out0, out1);
                 }
                 base += __popc(word);
             }
@@ -1434,7 +1487,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_emit_wide_k(const unsigned
                 set_status(st, XLB_ERR_CAPACITY, 8, pos);
                 return;
             }
-            out[pos++] = ((x >> lo_bits) << 32) | (x & lo_mask);
+            dense_put(x, lo_bits, lo_mask, pos++, out, out0, out1);
         }
     }
 }
@@ -1777,6 +1830,41 @@ static __global__ void __launch_bounds__(BLOCK) direct_fill_k(const uint64_t* __
             if (pos < n) pay[pos] = other[k];
         }
         __syncthreads();
+    }
+}
+// A few thousand rows over a few thousand keys: counted, summed and filled by one block, instead of two
+// fills and three to five launches (18 us).
+constexpr int DS_THREADS = 1024, DS_BITS = 14;
+constexpr uint64_t DS_ROWS = 1ull << 14;
+static __global__ void __launch_bounds__(DS_THREADS) direct_small_k(const uint64_t* __restrict__ rows, unsigned n, int keysel, unsigned long long* __restrict__ cursor, unsigned domain,
+                                                                  uint32_t* __restrict__ pay, DevStatus* st) {
+    extern __shared__ unsigned ds_cnt[];
+    __shared__ unsigned sm[33];
+    for (unsigned k = threadIdx.x; k < domain; k += DS_THREADS) ds_cnt[k] = 0;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < n; i += DS_THREADS) {
+        const uint64_t t = rows[i];
+        const uint32_t key = keysel == 0 ? (uint32_t)(t >> 32) : (uint32_t)t;
+        if (key >= domain) set_status(st, XLB_ERR_CAPACITY, 5, key);
+        else atomicAdd(&ds_cnt[key], 1u);
+    }
+    __syncthreads();
+    const unsigned per = (domain + DS_THREADS - 1) / DS_THREADS, lo = threadIdx.x * per, hi = lo + per < domain ? lo + per : domain;
+    unsigned sum = 0;
+    for (unsigned k = lo; k < hi; ++k) sum += ds_cnt[k];
+    unsigned tot;
+    unsigned run = block_exclusive_scan<unsigned>(sum, &tot, sm);
+    for (unsigned k = lo; k < hi; ++k) {
+        const unsigned c = ds_cnt[k];
+        ds_cnt[k] = run;
+        run += c;
+        cursor[k] = run;
+    }
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < n; i += DS_THREADS) {
+        const uint64_t t = rows[i];
+        const uint32_t key = keysel == 0 ? (uint32_t)(t >> 32) : (uint32_t)t;
+        if (key < domain) pay[atomicAdd(&ds_cnt[key], 1u)] = keysel == 0 ? (uint32_t)t : (uint32_t)(t >> 32);
     }
 }
 // match[i] = (start << 32) | len, or 0 when the key has no rows (same form as hash_probe_k)

@@ -421,6 +421,39 @@ static Keys rel_packed(xlb_ctx* c, const xlb_rel* r, int fcol, uint32_t fval, Ke
     return k;
 }
 
+void ops_pack_all(xlb_ctx* c, const std::vector<const xlb_rel*>& rels) {
+    std::vector<const xlb_rel*> todo;
+    for (const xlb_rel* r : rels)
+        if (!r->packed && rel_packable(r->schema) && r->rows && std::find(todo.begin(), todo.end(), r) == todo.end()) todo.push_back(r);
+    for (size_t at = 0; at < todo.size(); at += READ_WORDS_MAX) {
+        const int k = (int)std::min<size_t>(READ_WORDS_MAX, todo.size() - at);
+        if (k == 1) {
+            rel_packed(c, todo[at], -1, 0, nullptr);
+            continue;
+        }
+        Buf bounds = make_buf(c, 8ull * k);
+        CUDA_OK(set_async(c, bounds->p, 0, bounds->bytes));
+        std::vector<Buf> out(k);
+        for (int i = 0; i < k; ++i) {
+            const xlb_rel* r = todo[at + i];
+            out[i] = make_buf(c, r->rows * 8);
+            unsigned long long* bound = bounds->as<unsigned long long>() + i;
+            prof_begin(c, "pack", r->rows * 16ull);
+            if (r->schema.arity == 2) {
+                const bool vec = (((uintptr_t)r->cols[0]->p | (uintptr_t)r->cols[1]->p | (uintptr_t)out[i]->p) & 15) == 0;
+                pack2_k<<<grid_for(c, r->rows, BLOCK * 4), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), r->cols[1]->as<uint32_t>(), out[i]->as<uint64_t>(), r->rows, bound, vec);
+            } else pack1_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), out[i]->as<uint64_t>(), r->rows, bound);
+            check_launch(c, "pack");
+        }
+        unsigned long long h[READ_WORDS_MAX];
+        read_words(c, bounds->p, k, h);
+        for (int i = 0; i < k; ++i) {
+            todo[at + i]->packed = out[i];
+            todo[at + i]->or_bound = h[i];
+        }
+    }
+}
+
 Keys ops_rel_packed(xlb_ctx* c, const xlb_rel* r) { return rel_packed(c, r, -1, 0, nullptr); }
 
 bool ops_rel_bound_filtered(xlb_ctx* c, const xlb_rel* r, int fcol, uint32_t fval, Keys* filtered) {
@@ -586,11 +619,12 @@ DenseSet ops_dense_begin_state(xlb_ctx* c, DenseState& s) {
     return d;
 }
 
-static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total);
+static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total, const Buf* cols = nullptr);
 Keys ops_dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full) { return dense_finish(c, d, full, nullptr); }
 
 // known_total: the number of rows that will come out, when the host knows it already (no read-back)
-static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total) {
+// cols: where they go as columns (the second may be null) instead of packed; needs known_total
+static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total, const Buf* cols) {
     Keys o;
     o.bound = d.bound;
     const uint64_t words = d.words;
@@ -611,7 +645,8 @@ static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64
         exclusive_scan<LoadU32, uint64_t>(c, LoadU32{gcnt->as<uint32_t>()}, groups, offs->as<uint64_t>(), d.counts);
     } else if (groups <= (uint64_t)DENSE_FUSED_GROUPS) {
         dense_count_scan_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, gcnt->as<uint32_t>(), groups, d.visited,
-                                                                                                  offs->as<uint64_t>(), d.counts, (unsigned int*)(d.counts + 2));
+                                                                                                  offs->as<uint64_t>(), d.counts, (unsigned int*)(d.counts + 2), known_total != nullptr,
+                                                                                                  known_total ? *known_total : 0, c->d_status);
         check_launch(c, "dense_count");
     } else {
         dense_count_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, gcnt->as<uint32_t>(), groups, d.visited);
@@ -620,7 +655,7 @@ static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64
     }
     unsigned long long both[2] = {known_total ? *known_total : 0ull, 0ull};
     if (!known_total) read_words(c, d.counts, 2, both);
-    else {
+    else if (wide || groups > (uint64_t)DENSE_FUSED_GROUPS) {
         verify_count_k<<<1, 1, 0, c->stream>>>(d.counts, *known_total, c->d_status);  // a mismatch surfaces as an error at the next status check
         check_launch(c, "verify_count");
     }
@@ -628,14 +663,17 @@ static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64
     d.marked = both[1];
     prof_add_bytes(c, "expand_mark", d.marked * 4ull);
     o.n = tot;
-    o.buf = make_buf(c, tot * 8);
+    uint32_t* c0 = cols ? cols[0]->as<uint32_t>() : nullptr;
+    uint32_t* c1 = cols && cols[1] ? cols[1]->as<uint32_t>() : nullptr;
+    if (!cols) o.buf = make_buf(c, tot * 8);
+    uint64_t* packed = cols ? nullptr : o.buf->as<uint64_t>();
     if (tot) {
         prof_begin(c, "dense_emit", words * 4ull + tot * 8ull);
         if (wide)
-            dense_emit_wide_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), offs->as<uint64_t>(), groups, d.lo_bits, o.buf->as<uint64_t>(),
-                                                                                                    d.visited, tot, c->d_status, d.touched);
+            dense_emit_wide_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), offs->as<uint64_t>(), groups, d.lo_bits, packed,
+                                                                                                    d.visited, tot, c->d_status, d.touched, c0, c1);
         else
-            dense_emit_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, offs->as<uint64_t>(), groups, d.lo_bits, o.buf->as<uint64_t>(), d.visited, tot, c->d_status);
+            dense_emit_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, offs->as<uint64_t>(), groups, d.lo_bits, packed, d.visited, tot, c->d_status, c0, c1);
         check_launch(c, "dense_emit");
     }
     return o;
@@ -664,18 +702,28 @@ void ops_dense_state_build(xlb_ctx* c, DenseState& s, int hi_bits, int lo_bits, 
     s.valid = true;
 }
 
-Keys ops_dense_state_rows(xlb_ctx* c, const DenseState& s, uint64_t bound) {
+static Keys dense_state_out(xlb_ctx* c, const DenseState& s, uint64_t bound, const Buf* cols) {
     DenseSet d;
     d.hi_bits = s.hi_bits;
     d.lo_bits = s.lo_bits;
     d.words = s.words;
     d.bitmap = s.visited;
     d.bound = bound;
-    Buf counts = make_buf(c, 24);
-    CUDA_OK(set_async(c, counts->p, 0, 24));
-    d.counts = counts->as<uint64_t>();
+    d.counts = (uint64_t*)(c->d_status + 1);  // (every use leaves the ticket clear and overwrites the total)
     Keys none;
-    return dense_finish(c, d, none, &s.rows);  // nothing to subtract, no second bitmap: every set bit comes out, s.rows of them
+    return dense_finish(c, d, none, &s.rows, cols);  // nothing to subtract, no second bitmap: every set bit comes out, s.rows of them
+}
+Keys ops_dense_state_rows(xlb_ctx* c, const DenseState& s, uint64_t bound) { return dense_state_out(c, s, bound, nullptr); }
+
+xlb_rel* ops_dense_state_columns(xlb_ctx* c, const DenseState& s, const xlb_schema& schema) {
+    std::unique_ptr<xlb_rel> o(new xlb_rel);
+    o->ctx = c;
+    o->schema = schema;
+    o->rows = s.rows;
+    o->canonical = true;
+    for (uint32_t i = 0; i < schema.arity; ++i) o->cols[i] = make_buf(c, s.rows * 4);
+    dense_state_out(c, s, 0, o->cols);
+    return o.release();
 }
 
 static void tuple_set_alloc(xlb_ctx* c, TupleSet& s, uint64_t tuples) {
@@ -861,10 +909,18 @@ Index ops_index_build_direct(xlb_ctx* c, const Keys& rows, int keysel, int key_b
     ix.bound = rows.bound;
     const uint64_t other = keysel == SRC_HI ? (rows.bound & 0xFFFFFFFFull) : (rows.bound >> 32);
     ix.pay_bound = rows.bound == ~0ull ? 0xFFFFFFFFull : other;
-    Buf cnt = make_buf(c, ix.domain * 4);
-    CUDA_OK(set_async(c, cnt->p, 0, ix.domain * 4));
     ix.cursor = make_buf(c, ix.domain * 8);
     ix.pay = make_buf(c, rows.n * 4);
+    if (rows.n && rows.n <= DS_ROWS && key_bits <= DS_BITS) {
+        if (!c->index_attr_set) CUDA_OK(cudaFuncSetAttribute(direct_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << DS_BITS));
+        c->index_attr_set = true;
+        prof_begin(c, "direct_fill", rows.n * 20ull);
+        direct_small_k<<<1, DS_THREADS, ix.domain * 4, c->stream>>>(rows.ptr(), (unsigned)rows.n, keysel, ix.cursor->as<unsigned long long>(), (unsigned)ix.domain, ix.pay->as<uint32_t>(), c->d_status);
+        check_launch(c, "direct_fill");
+        return ix;
+    }
+    Buf cnt = make_buf(c, ix.domain * 4);
+    CUDA_OK(set_async(c, cnt->p, 0, ix.domain * 4));
     Buf total = make_buf(c, 8);
     if (rows.n) {
         prof_begin(c, "direct_count", rows.n * 8ull);
@@ -1109,8 +1165,8 @@ extern "C" xlb_status xlb_ctx_create(const xlb_config* cfg, xlb_ctx** out) {
         CUDA_OK(cudaHostAlloc((void**)&c->h_scalar, SCALAR_WORDS * 8, cudaHostAllocMapped));
         CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_scalar_dev, c->h_scalar, 0));
         memset(c->h_scalar, 0, SCALAR_WORDS * 8);
-        CUDA_OK(cudaMalloc(&c->d_status, sizeof(DevStatus)));
-        CUDA_OK(cudaMemset(c->d_status, 0, sizeof(DevStatus)));
+        CUDA_OK(cudaMalloc(&c->d_status, sizeof(DevStatus) + 24));  // and behind it the count words of dense_state_out
+        CUDA_OK(cudaMemset(c->d_status, 0, sizeof(DevStatus) + 24));
         cudaDeviceProp prop;
         CUDA_OK(cudaGetDeviceProperties(&prop, dev));
         c->sm_count = prop.multiProcessorCount;

@@ -35,6 +35,7 @@ struct Index {
 };
 
 Keys ops_rel_packed(xlb_ctx* c, const xlb_rel* r);             // packed view (cached on the relation)
+void ops_pack_all(xlb_ctx* c, const std::vector<const xlb_rel*>& rels);  // the packed views of several relations, with one read-back
 // The same for a two-column relation that is not packed yet, with the rows whose column fcol equals
 // fval collected in the same pass (`filtered`, a bag).  False (nothing done): already packed.
 bool ops_rel_packed_filtered(xlb_ctx* c, const xlb_rel* r, int fcol, uint32_t fval, Keys* filtered);
@@ -118,6 +119,7 @@ void ops_tuple_set_build(xlb_ctx* c, TupleSet& s, const Keys& full, const Keys& 
 Keys ops_tuple_set_novel(xlb_ctx* c, TupleSet& s, const Keys& cand);
 void ops_dense_state_build(xlb_ctx* c, DenseState& s, int hi_bits, int lo_bits, const Keys& full, const Keys& novel);
 Keys ops_dense_state_rows(xlb_ctx* c, const DenseState& s, uint64_t bound);  // all its tuples, in order
+xlb_rel* ops_dense_state_columns(xlb_ctx* c, const DenseState& s, const xlb_schema& schema);  // the same as a relation of columns
 // A set whose bitmap starts as a copy of `visited` (same domain) instead of empty.
 DenseSet ops_dense_begin_from(xlb_ctx* c, int hi_bits, int lo_bits, unsigned int* visited);
 // The candidate set of one use of a head's bitmap state: its persistent marks when it keeps them, else a copy of the head.
@@ -214,7 +216,8 @@ struct DeltaLoop {
     int hi_bits = 0, lo_bits = 0;
     Buf log;                // derived tuples in the order they were found; the last ones are the delta
     uint64_t cap = 0, room = 0;  // tuples the log can hold; that may be in it
-    Buf ctl;
+    void* ctl = nullptr;    // behind the bitmaps
+    bool seeded = false;
 };
 struct DeltaResult {
     uint64_t rows = 0;      // tuples in the log: what was derived beyond the known rows
@@ -230,6 +233,25 @@ void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows);  // a delta a
 // False: a kernel reported a failure (check_dev_status says which).
 bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
                    DeltaResult* res);
+
+// A whole frontier fixpoint in one launch (xlb_frontier.cu): seeds are the rows of `rel` with a column
+// equal to a constant; from then on rows whose key_col holds a derived value derive their value_col.
+constexpr int FRONTIER_SEEDS = 4;
+struct FrontierConst {
+    int filter_col, take_col;
+    uint32_t constant;
+};
+struct FrontierSeed {
+    const uint32_t *filter, *take;
+    uint32_t constant;
+};
+struct FrontierWhole {
+    Buf values;  // sorted, unique
+    uint64_t rows = 0, iterations = 0, candidates = 0;
+    bool fix = false;
+};
+// False: not a relation for it (too many rows, values too large, too many iterations).
+bool ops_frontier_whole(xlb_ctx* c, const xlb_rel* rel, int key_col, int value_col, const std::vector<FrontierConst>& seeds, uint64_t max_iterations, FrontierWhole* out);
 
 // rows of `bag` whose key has (semi) or lacks (anti) a match in the index, in bag order
 // (pkeys, when given, holds the key word of every bag row instead of a half named by keysel)

@@ -230,9 +230,7 @@ struct GroupKey {
 __global__ void __launch_bounds__(BLOCK) group_bound_k(KeyCols keys, uint64_t n, unsigned long long* __restrict__ bound) {
     uint64_t o = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) o |= keys(i);
-#pragma unroll
-    for (int d = 16; d; d >>= 1) o |= __shfl_xor_sync(FULL, o, d);
-    if (lane_id() == 0 && o) atomicOr(bound, (unsigned long long)o);
+    block_or(o, bound);
 }
 __global__ void __launch_bounds__(BLOCK) group_rows_k(GroupKey key, uint64_t n, unsigned int* __restrict__ count) {
     __shared__ uint32_t skey[DX_SLOTS], scnt[DX_SLOTS];
