@@ -1,5 +1,5 @@
-"""Frontier fixpoints in one launch against the oracle: row counts around the limits of the one-block
-and the many-block kernel, paths longer than the latter follows, values at the edge of the domains,
+"""Frontier fixpoints in one launch against the oracle: row counts around the limits of the three
+kernels, paths longer than the latter follows, values at the edge of the domains,
 no seed at all, the iteration limit, both join columns."""
 import numpy as np
 import pytest
@@ -13,6 +13,7 @@ from xlog_b200.plan import CompiledRule, ExecutionPlan, Filter, Join, Project, S
 from xlog_b200.provider import KernelProvider
 
 pytestmark = pytest.mark.gpu
+LARGE = (1 << 21) + 101  # rows: the kernel that keeps lists of the rows still of use
 
 
 def check(plan, edge, out="r"):
@@ -32,16 +33,16 @@ def test_row_counts(n):
     check(programs.reach_from_source(0), [rng.integers(0, nodes, n).astype(np.uint32), rng.integers(0, nodes, n).astype(np.uint32)])
 
 
-@pytest.mark.parametrize("n,rows", [(2000, 2000), (47, 40000), (49, 40000), (400, 40000)])
+@pytest.mark.parametrize("n,rows", [(2000, 2000), (47, 40000), (49, 40000), (400, 40000), (47, LARGE), (60, LARGE)])
 def test_paths(n, rows):
     # a path of n nodes, and unrelated rows to make up the number
     edge = [np.arange(n - 1, dtype=np.uint32), np.arange(1, n, dtype=np.uint32)]
-    fill = np.arange(rows - n + 1, dtype=np.uint32) + n
+    fill = np.arange(rows - n + 1, dtype=np.uint32) % (1 << 19) + n
     assert check(programs.reach_from_source(0), [np.append(edge[0], fill), np.append(edge[1], fill)])["iterations"] == n - 1
 
 
-@pytest.mark.parametrize("top", [(1 << 18) - 1, (1 << 19) - 1, 1 << 19, (1 << 32) - 1])
-@pytest.mark.parametrize("rows", [100, 40000])
+@pytest.mark.parametrize("top", [(1 << 18) - 1, (1 << 19) - 1, 1 << 19, (1 << 20) - 1, 1 << 20, (1 << 32) - 1])
+@pytest.mark.parametrize("rows", [100, 40000, LARGE])
 def test_large_values(top, rows):
     rng = np.random.default_rng(rows)
     a, b = rng.integers(0, 500, rows).astype(np.uint32), rng.integers(0, 500, rows).astype(np.uint32)
@@ -60,14 +61,14 @@ def test_no_seed_other_column_and_two_seeds():
         CompiledRule("r", Project(Filter(Scan(0), A.EQ, 1, 5, True), [0]), u),
         CompiledRule("r", Project(Filter(Scan(0), A.EQ, 0, 9, True), [0]), u),
         CompiledRule("r", Project(Join(Scan(1), Scan(0), [0], [1]), [1]), u)])], ids)
-    for n in (9000, 40000):
+    for n in (9000, 40000, LARGE):
         check(plan, [rng.integers(1, 3000, n).astype(np.uint32), rng.integers(1, 3000, n).astype(np.uint32)])
 
 
-@pytest.mark.parametrize("rows", [10, 40000])
+@pytest.mark.parametrize("rows", [10, 40000, LARGE])
 def test_iteration_limit(rows):
     n = 10
-    fill = np.arange(rows - n + 1, dtype=np.uint32) + n
+    fill = np.arange(rows - n + 1, dtype=np.uint32) % (1 << 19) + n
     edge = [np.append(np.arange(n - 1, dtype=np.uint32), fill), np.append(np.arange(1, n, dtype=np.uint32), fill)]
     for limit, ok in ((n - 1, True), (n - 2, False)):
         p = KernelProvider(device=0, max_iterations=limit)

@@ -377,7 +377,7 @@ struct xlb_ctx {
     // bounded look-back of the one-sweep sort: polls before a tile gives up (XLB_ERR_TIMEOUT), and
     // the number the first tile takes (0; a test makes tile 0 never run so that the wait runs out)
     unsigned lb_spin_limit = 1u << 22, lb_first_tile = 0;
-    bool frontier_attr_set = false, frontier_many_attr_set = false;  // the same for frontier_one_k, frontier_many_k
+    bool frontier_attr_set = false, frontier_many_attr_set = false, frontier_large_attr_set = false;  // the same for the frontier kernels
     bool index_attr_set = false;  // the same for direct_small_k
     bool delta_attr_set = false;  // the same for the delta loop's kernel
     bool sort_attr_set = false;  // the scatter kernels' shared-memory opt-in was made on this context's device
