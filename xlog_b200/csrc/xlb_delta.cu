@@ -27,10 +27,10 @@ constexpr int DL_STAGE = 128;                            // new tuples a warp co
 constexpr unsigned DL_HEAVY = 512;                       // a row with more outputs than this is taken apart
 constexpr unsigned DL_PIECE = 512;                       // ... into pieces that any warp can take
 constexpr unsigned DL_HEAVY_MAX = 1u << 18;              // pieces an iteration can list (rows beyond stay with their warp)
-constexpr uint64_t DL_SOLO_ROWS = 4096, DL_SOLO_OUTPUTS = 8192;  // iterations of at most this size run on one block
-constexpr unsigned SOLO_NEXT = 4096;                     // tuples of a solo iteration that stay in shared memory
-constexpr size_t DL_SMEM = std::max<size_t>((size_t)DL_WARPS * 2 * DL_STAGE * 8, 2 * SOLO_NEXT * 8);
-static_assert(2 * SOLO_NEXT * 8 <= DL_SMEM, "the solo phase uses the warps' stages");
+constexpr uint64_t DL_SOLO_ROWS = 2048, DL_SOLO_OUTPUTS = 8192;  // iterations of at most this size run on one block
+constexpr unsigned SOLO_NEXT = 2048;                     // tuples of a solo iteration that stay in shared memory
+constexpr size_t DL_SMEM = std::max<size_t>((size_t)DL_WARPS * 2 * DL_STAGE * 8, 2 * SOLO_NEXT * 16);
+static_assert(2 * SOLO_NEXT * 16 <= DL_SMEM, "the solo phase uses the warps' stages");
 constexpr unsigned DL_SPIN_LIMIT = 1u << 26;             // polls of a barrier before a block gives up (tens of seconds)
 
 struct Ix {
@@ -85,17 +85,27 @@ struct Square {
     int bits;  // of a value
 };
 enum Phase { PH_ROWS = 0, PH_HEAVY = 1, PH_SOLO = 2, PH_DONE = 3, PH_FULL = 4 };
+// What the blocks share about one iteration.  Three are used in turn: while one is filled the next is
+// cleared, and the one before may still be read by a block that is late.
+struct Slot {
+    unsigned long long count, cand;  // tuples appended to the log; candidates
+    unsigned heavy_n, next_heavy;    // pieces of long rows listed, taken
+    unsigned next_chunk;             // rows are taken in batches
+    unsigned pad;
+};
 struct Ctl {
-    unsigned long long tail;        // tuples appended to the log so far (may pass its capacity: see overflow)
+    // in: where the loop stands; out: where it stopped (read by the host)
+    unsigned long long tail;        // tuples in the log (may pass its capacity: see overflow)
     unsigned long long start, end;  // the delta at hand: log[start, end)
     unsigned long long iterations, candidates, fix, overflow;
-    unsigned long long cand_before; // candidates when the iteration began
-    unsigned arrived;               // grid barrier: blocks that wait ...
-    unsigned sync;                  // ... for this word to change: (generation << 3) | phase, always written as one
-    unsigned next_chunk;            // rows are taken in chunks
-    unsigned heavy_n, next_heavy;
-    unsigned check;                 // most candidates of the last iteration were known already
+    unsigned phase, check;          // check: most candidates of the last iteration were known already
+    unsigned arrived;               // blocks that arrived at the grid barriers so far
     unsigned abort;
+    // what block 0 found when it ran on alone
+    unsigned solo_turns;            // solo phases that are over
+    unsigned solo_phase, solo_check, pad;
+    unsigned long long solo_start, solo_end, solo_iterations, solo_candidates;
+    Slot slot[3];
 };
 struct Heavy {
     uint64_t row;
@@ -151,35 +161,37 @@ __device__ __forceinline__ void mark_transposed(const Out& o, uint64_t t) {
 // the other half of its stage meanwhile.
 struct WarpSink {
     const Out& o;
-    uint64_t* stage;  // two halves of DL_STAGE
+    uint64_t* stage;              // two halves of DL_STAGE
+    Slot* slot = nullptr;         // of the iteration under way ...
+    uint64_t base = 0;            // ... whose tuples follow here in the log
     unsigned staged = 0, pending = 0, half = 0;
-    unsigned long long at = 0;  // lane 0: where the pending half goes
+    unsigned long long at = 0;    // lane 0: where the pending half goes
 
+    __device__ __forceinline__ void write(uint64_t to, const uint64_t* from, unsigned n) {
+        for (unsigned i = lane_id(); i < n; i += 32)
+            if (to + i < o.cap) o.log[to + i] = from[i];  // beyond the capacity: found again from the bitmap by the host
+        __syncwarp();
+    }
     __device__ __forceinline__ void finish() {
         if (!pending) return;
-        const unsigned long long to = __shfl_sync(FULL, at, 0);
-        const uint64_t* from = stage + (half ^ 1) * DL_STAGE;
-        for (unsigned i = lane_id(); i < pending; i += 32)
-            if (to + i < o.cap) __stcg(&o.log[to + i], from[i]);  // beyond the capacity: found again from the bitmap by the host
-        __syncwarp();
+        write(__shfl_sync(FULL, at, 0), stage + (half ^ 1) * DL_STAGE, pending);
         pending = 0;
     }
     __device__ __forceinline__ void rotate() {
         finish();
         if (!staged) return;
         __syncwarp();
-        if (lane_id() == 0) at = atomicAdd(&o.ctl->tail, (unsigned long long)staged);
+        if (lane_id() == 0) at = base + atomicAdd(&slot->count, (unsigned long long)staged);
         pending = staged;
         staged = 0;
         half ^= 1;
     }
-    __device__ __forceinline__ void write_left(unsigned long long to) {  // what is staged, to a place somebody else reserved
-        const uint64_t* from = stage + half * DL_STAGE;
-        for (unsigned i = lane_id(); i < staged; i += 32)
-            if (to + i < o.cap) __stcg(&o.log[to + i], from[i]);
+    __device__ __forceinline__ void write_left(uint64_t to) {  // what is staged, to a place somebody else reserved
+        write(to, stage + half * DL_STAGE, staged);
         staged = 0;
-        __syncwarp();
     }
+    template <int N>
+    __device__ __forceinline__ void look_ahead(const uint64_t (&)[N]) {}
     template <int N>
     __device__ __forceinline__ void push(const bool (&on)[N], const uint64_t (&tup)[N]) {
         if (staged + 32 * N > DL_STAGE) rotate();
@@ -192,12 +204,28 @@ struct WarpSink {
         }
     }
 };
-// Block 0 alone: the next delta is built in shared memory; the log gets its copy on the side.
+// Block 0 alone: the next delta is built in shared memory; the log gets its copy on the side.  With one
+// join a tuple's own matches are looked up while the atomic that decides about it is on its way, and
+// kept beside it.
+struct SoloShared {
+    unsigned count[3], cand[3], listed;
+};
+template <bool AHEAD>
 struct SoloSink {
     const Out& o;
+    const Rules& rules;
     uint64_t* next;
-    unsigned* count;
+    uint32_t *next_s, *next_l;
+    unsigned *count, *listed;
     uint64_t base;  // the log's tail
+    uint32_t s[DL_UNROLL], l[DL_UNROLL];
+    template <int N>
+    __device__ __forceinline__ void look_ahead(const uint64_t (&tup)[N]) {
+        if constexpr (AHEAD) {
+#pragma unroll
+            for (int u = 0; u < N; ++u) find(rules.r[0].ix[0], rules.r[0].key_src[0] == 0 ? (uint32_t)(tup[u] >> 32) : (uint32_t)tup[u], s[u], l[u]);
+        }
+    }
     template <int N>
     __device__ __forceinline__ void push(const bool (&on)[N], const uint64_t (&tup)[N]) {
         unsigned b[N], total = 0, at = 0;
@@ -213,8 +241,15 @@ struct SoloSink {
         for (int u = 0; u < N; ++u) {
             const unsigned p = at + __popc(b[u] & lanemask_lt());
             if (on[u]) {
-                if (p < SOLO_NEXT) next[p] = tup[u];
-                if (base + p < o.cap) __stcg(&o.log[base + p], tup[u]);
+                if (p < SOLO_NEXT) {
+                    next[p] = tup[u];
+                    if (AHEAD) {
+                        next_s[p] = s[u];
+                        next_l[p] = l[u];
+                        if (l[u] > DL_HEAVY) *listed = 1;  // a long row: not for one block
+                    }
+                }
+                if (base + p < o.cap) o.log[base + p] = tup[u];
             }
             at += __popc(b[u]);
         }
@@ -297,6 +332,7 @@ __device__ __forceinline__ void emit(const Out& o, const Rule& ru, const Lane& m
             old[u] = 0;
             if (on[u]) old[u] = atomicOr(&o.visited[x[u] >> 5], 1u << (x[u] & 31));
         }
+        sink.look_ahead(tup);
 #pragma unroll
         for (int u = 0; u < N; ++u) on[u] = on[u] && !((old[u] >> (x[u] & 31)) & 1u);
         if (o.visited_t)
@@ -307,11 +343,36 @@ __device__ __forceinline__ void emit(const Out& o, const Rule& ru, const Lane& m
     }
 }
 
+// Outputs of rows whose matches are known (lane's own: `mine`, none of them long) under one rule.
+template <class Sink>
+__device__ __forceinline__ void deal(const Out& o, const Rule& ru, Lane& me, uint32_t mine, unsigned rows, bool check, Sink& sink) {
+    const uint32_t longest = __reduce_max_sync(FULL, mine);
+    if (longest <= 1) {
+        if (longest) emit<SERIAL, 1>(o, ru, me, mine, 0, 1, check, sink);
+        return;
+    }
+    const uint32_t total = __reduce_add_sync(FULL, mine);
+    if (longest * 16 <= total) {  // at least half of the lanes' steps would bring an output
+        emit<SERIAL, DL_UNROLL>(o, ru, me, mine, 0, longest, check, sink);
+    } else if (rows == 1) {
+        emit<SINGLE, DL_UNROLL>(o, ru, me, 0, 0, total, check, sink);
+    } else {
+        uint32_t incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, incl, d);
+            if (lane_id() >= (unsigned)d) incl += v;
+        }
+        me.before = incl - mine;
+        emit<BALANCED, DL_UNROLL>(o, ru, me, incl, 0, total, check, sink);
+    }
+}
+
 // The warp's rows (lane i < rows: me_row of the delta) under every rule with one recursive atom.
 // `cand` += this lane's candidates (at most 512 a row and rule; those of longer rows are counted
 // in global memory).  Returns whether a long row was listed in pieces.
 template <class Sink>
-__device__ __forceinline__ bool take_rows(const Out& o, const Rules& rules, uint64_t me_row, unsigned rows, Heavy* heavy, bool check, Sink& sink, unsigned& cand) {
+__device__ __forceinline__ bool take_rows(const Out& o, const Rules& rules, uint64_t me_row, unsigned rows, Heavy* heavy, Slot* slot, bool check, Sink& sink, unsigned& cand) {
     const unsigned lane = lane_id();
     bool any_listed = false;
     Lane me;
@@ -330,14 +391,14 @@ __device__ __forceinline__ bool take_rows(const Out& o, const Rules& rules, uint
             }
         }
         if (cnt <= DL_HEAVY) cand += (unsigned)cnt;
-        else atomicAdd(&o.ctl->candidates, (unsigned long long)cnt);
+        else atomicAdd(&slot->cand, (unsigned long long)cnt);
         // long rows: listed in pieces; one that finds the list full stays here
         unsigned alone = 0;
         if (cnt > DL_HEAVY) {
             const uint64_t pieces = (cnt + DL_PIECE - 1) / DL_PIECE;
             bool listed = false;
             if (pieces <= DL_HEAVY_MAX) {
-                const unsigned h = atomicAdd(&o.ctl->heavy_n, (unsigned)pieces);
+                const unsigned h = atomicAdd(&slot->heavy_n, (unsigned)pieces);
                 if (h <= DL_HEAVY_MAX - pieces) {
                     for (unsigned k = 0; k < pieces; ++k) heavy[h + k] = {me.row, (unsigned)q, k};
                     listed = true;
@@ -348,23 +409,7 @@ __device__ __forceinline__ bool take_rows(const Out& o, const Rules& rules, uint
             any_listed = true;  // (the count was raised either way)
             if (!listed) alone = 1;
         }
-        const uint32_t mine = cnt > DL_HEAVY ? 0 : (uint32_t)cnt, longest = __reduce_max_sync(FULL, mine), total = __reduce_add_sync(FULL, mine);
-        if (longest <= 1) {
-            if (longest) emit<SERIAL, 1>(o, ru, me, mine, 0, 1, check, sink);
-        } else if (longest * 16 <= total) {  // at least half of the lanes' steps would bring an output
-            emit<SERIAL, DL_UNROLL>(o, ru, me, mine, 0, longest, check, sink);
-        } else if (rows == 1) {
-            emit<SINGLE, DL_UNROLL>(o, ru, me, 0, 0, total, check, sink);
-        } else {
-            uint32_t incl = mine;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t v = __shfl_up_sync(FULL, incl, d);
-                if (lane >= (unsigned)d) incl += v;
-            }
-            me.before = incl - mine;
-            emit<BALANCED, DL_UNROLL>(o, ru, me, incl, 0, total, check, sink);
-        }
+        deal(o, ru, me, cnt > DL_HEAVY ? 0 : (uint32_t)cnt, rows, check, sink);
         for (unsigned left = __ballot_sync(FULL, alone); left; left &= left - 1) {
             const int r = __ffs(left) - 1;
             Lane one;
@@ -548,45 +593,55 @@ __device__ __forceinline__ void square_full(const Out& o, const Square& sq, uint
     }
 }
 
-// The end of an iteration: its new tuples become the delta.  (One thread, everybody else waiting.)
-// Returns what comes next.
-__device__ unsigned next_iteration(const Out& o, uint64_t max_iterations, bool square) {
-    volatile Ctl* v = o.ctl;
-    const uint64_t tail = v->tail, end = v->end, rows = end - v->start, cands = v->candidates - v->cand_before;
-    const uint64_t next = tail - end;
-    v->iterations = v->iterations + 1;
-    v->cand_before = v->candidates;
-    v->start = end;
-    v->end = tail;
-    v->next_chunk = 0;
-    v->heavy_n = 0;
-    v->next_heavy = 0;
-    v->check = next * 2 < cands;
-    if (next == 0) v->fix = 1;
-    else if (tail > o.cap) v->overflow = 1;
-    if (next == 0 || tail > o.cap || v->iterations >= max_iterations) return PH_DONE;
-    if (square) return PH_FULL;
-    return next <= DL_SOLO_ROWS && cands * next <= DL_SOLO_OUTPUTS * rows ? PH_SOLO : PH_ROWS;
+// Where the loop stands, as every block works it out for itself.
+struct State {
+    uint64_t start, end, iterations, candidates;
+    unsigned phase, check, slot;
+    bool fix, overflow;
+};
+// The end of an iteration that appended `count` tuples: they become the delta.
+__device__ __forceinline__ void next_iteration(State& st, uint64_t count, uint64_t cands, uint64_t cap, uint64_t max_iterations, bool square) {
+    const uint64_t rows = st.end - st.start;
+    ++st.iterations;
+    st.candidates += cands;
+    st.start = st.end;
+    st.end += count;
+    st.check = count * 2 < cands;
+    st.fix = count == 0;
+    st.overflow = !st.fix && st.end > cap;
+    if (st.fix || st.overflow || st.iterations >= max_iterations) st.phase = PH_DONE;
+    else if (square) st.phase = PH_FULL;
+    else st.phase = count <= DL_SOLO_ROWS && cands * count <= DL_SOLO_OUTPUTS * rows ? PH_SOLO : PH_ROWS;
 }
 
 // Small iterations, by block 0 alone while the others wait: the delta, the next one and the counts
-// stay in shared memory, one block barrier per iteration.  Returns the phase that needs all blocks.
-struct SoloShared {
-    unsigned count[3], cand[3], listed;
-};
-__device__ __forceinline__ unsigned solo(const Out& o, const Rules& rules, Heavy* heavy, uint64_t max_iterations, uint64_t* buf, SoloShared& sh, uint64_t start, uint64_t base) {
-    volatile Ctl* v = o.ctl;
+// stay in shared memory, one block barrier per iteration.  Leaves `st` (of all threads) at what needs all
+// blocks.
+template <bool AHEAD>
+__device__ __forceinline__ void solo(const Out& o, const Rules& rules, Heavy* heavy, Slot* slot, uint64_t max_iterations, uint64_t* buf, SoloShared& sh, State& st) {
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    unsigned n = (unsigned)(base - start), cur = 0;
+    uint32_t *buf_s = reinterpret_cast<uint32_t*>(buf + 2 * SOLO_NEXT), *buf_l = buf_s + 2 * SOLO_NEXT;
+    unsigned n = (unsigned)(st.end - st.start), cur = 0;
     bool thin = true;  // about one output a row: as few warps as hold the rows, each pays the whole chain of instructions
-    uint64_t iterations = v->iterations, before = 0;  // (candidates of the iterations that are over)
     if (threadIdx.x < 3) {
         sh.count[threadIdx.x] = 0;
         sh.cand[threadIdx.x] = 0;
     }
     if (threadIdx.x == 0) sh.listed = 0;
-    for (unsigned i = threadIdx.x; i < n; i += DL_THREADS) buf[i] = __ldcg(&o.log[start + i]);
     __syncthreads();
+    for (unsigned i = threadIdx.x; i < n; i += DL_THREADS) {
+        const uint64_t row = __ldcg(&o.log[st.start + i]);
+        buf[i] = row;
+        if (AHEAD) {
+            find(rules.r[0].ix[0], rules.r[0].key_src[0] == 0 ? (uint32_t)(row >> 32) : (uint32_t)row, buf_s[i], buf_l[i]);
+            if (buf_l[i] > DL_HEAVY) sh.listed = 1;
+        }
+    }
+    __syncthreads();
+    if (AHEAD && sh.listed) {  // a long row: all blocks
+        st.phase = PH_ROWS;
+        return;
+    }
     for (unsigned turn = 0;; turn = turn == 2 ? 0 : turn + 1) {
         const unsigned after = turn == 2 ? 0 : turn + 1;  // (its counters were read last two barriers ago)
         if (threadIdx.x == 0) {
@@ -595,50 +650,38 @@ __device__ __forceinline__ unsigned solo(const Out& o, const Rules& rules, Heavy
         }
         const unsigned per = thin || n >= DL_THREADS ? 32 : (n + DL_WARPS - 1) / DL_WARPS;
         unsigned cand = 0;
+        const unsigned to = (cur ^ 1) * SOLO_NEXT, from = cur * SOLO_NEXT;
         for (unsigned at = warp * per; at < n; at += DL_WARPS * per) {
             const unsigned rows = n - at < per ? n - at : per;
-            SoloSink sink{o, buf + (cur ^ 1) * SOLO_NEXT, &sh.count[turn], base};
-            if (take_rows(o, rules, lane < rows ? buf[cur * SOLO_NEXT + at + lane] : 0, rows, heavy, false, sink, cand)) sh.listed = 1;
+            SoloSink<AHEAD> sink{o, rules, buf + to, buf_s + to, buf_l + to, &sh.count[turn], &sh.listed, st.end};
+            const uint64_t row = lane < rows ? buf[from + at + lane] : 0;
+            if (AHEAD) {
+                Lane me;
+                me.row = row;
+                me.s1 = lane < rows ? buf_s[from + at + lane] : 0;
+                me.s2 = me.l2 = 0;
+                const uint32_t mine = lane < rows ? buf_l[from + at + lane] : 0;
+                cand += mine;
+                deal(o, rules.r[0], me, mine, rows, false, sink);
+            } else if (take_rows(o, rules, row, rows, heavy, slot, false, sink, cand)) sh.listed = 1;
         }
         cand = __reduce_add_sync(FULL, cand);
         if (lane == 0 && cand) atomicAdd(&sh.cand[turn], cand);
         __syncthreads();
         const unsigned next = sh.count[turn];
         const uint64_t cands = sh.cand[turn];
-        const uint64_t tail = base + next;
-        unsigned phase = PH_SOLO;
-        if (sh.listed) phase = PH_HEAVY;  // the iteration is not over
-        else {
-            ++iterations;
-            if (next == 0 || tail > o.cap || iterations >= max_iterations) phase = PH_DONE;
-            else if (next > DL_SOLO_ROWS || cands * next > DL_SOLO_OUTPUTS * n) phase = PH_ROWS;
-        }
-        if (phase != PH_SOLO) {
+        if (!AHEAD && sh.listed) {  // the iteration is not over: its long rows are listed
             if (threadIdx.x == 0) {
-                v->tail = tail;
-                v->iterations = iterations;
-                const unsigned long long listed = v->candidates;  // what long rows have added
-                v->candidates = listed + before + cands;
-                if (phase == PH_HEAVY) {
-                    v->start = start;
-                    v->end = base;
-                    v->cand_before = v->cand_before + before;
-                } else {
-                    v->start = base;
-                    v->end = tail;
-                    v->cand_before = listed + before + cands;
-                    v->next_chunk = 0;
-                    v->check = next * 2ull < cands;
-                    if (next == 0) v->fix = 1;
-                    else if (tail > o.cap) v->overflow = 1;
-                }
+                slot->count = next;
+                atomicAdd(&slot->cand, (unsigned long long)cands);
             }
-            return phase;
+            st.phase = PH_HEAVY;
+            return;
         }
-        before += cands;
+        next_iteration(st, next, cands, o.cap, max_iterations, false);
+        if (AHEAD && sh.listed && st.phase == PH_SOLO) st.phase = PH_ROWS;
+        if (st.phase != PH_SOLO) return;
         thin = cands <= 2ull * n;
-        start = base;
-        base = tail;
         n = next;
         cur ^= 1;
     }
@@ -647,63 +690,47 @@ __device__ __forceinline__ unsigned solo(const Out& o, const Rules& rules, Heavy
 template <bool SQUARE>
 __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const __grid_constant__ Rules rules, Heavy* heavy, uint64_t max_iterations, const __grid_constant__ Square sq) {
     extern __shared__ uint64_t stage_s[];
-    __shared__ uint64_t range_s[2];
-    __shared__ unsigned phase_s, go_s, check_s;
+    __shared__ State state_s;
+    __shared__ unsigned go_s;
     __shared__ SoloShared solo_s;
     __shared__ unsigned left_s[32];
     __shared__ unsigned long long cand_s[32];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     WarpSink sink{o, stage_s + warp * (2 * DL_STAGE)};
-    unsigned generation = 0;
+    unsigned passed = 0, solo_turns = 0;
     Ctl* ctl = o.ctl;
-    volatile Ctl* v = ctl;
-    // What thread 0 has seen of the sync word.  Between a barrier and the next, a solo phase may begin
-    // and end without the other blocks: one that is late finds the word two generations on, never a
-    // phase that does not belong to the generation beside it.
-    auto read_phase = [&]() {
-        if (threadIdx.x == 0) {
-            const unsigned w = v->sync;
-            __threadfence();
-            const unsigned long long a = v->start, b = v->end;
-            const unsigned c = v->check;
-            generation = w >> 3;
-            phase_s = w & 7;
-            range_s[0] = a;
-            range_s[1] = b;
-            check_s = c;
-        }
-        __syncthreads();
-    };
-    auto publish = [&](unsigned phase) {
-        __threadfence();
-        v->sync = ((generation + 1) << 3) | phase;
-    };
-    // Thread 0 waits until the generation has passed; false: it never did.
-    auto wait_next = [&]() {
-        for (unsigned polls = 0; v->sync >> 3 == generation; ++polls) {
-            if (polls > DL_SPIN_LIMIT || v->abort) {
-                v->abort = 1;
-                set_status(o.st, XLB_ERR_TIMEOUT, 14, generation);
+    // A bounded wait (one thread): until `done` holds of the word.
+    auto wait_for = [&](const unsigned* word, unsigned sleep, auto done) {
+        unsigned v;
+        for (unsigned polls = 0;; ++polls) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+            if (done(v)) return true;
+            if (polls > DL_SPIN_LIMIT || *(volatile unsigned*)&ctl->abort) {
+                *(volatile unsigned*)&ctl->abort = 1;
+                set_status(o.st, XLB_ERR_TIMEOUT, 14, passed);
                 return false;
             }
-            __nanosleep(polls < 64 ? 20 : 100);
+            if (sleep) __nanosleep(sleep);
         }
-        return true;
     };
-    // All blocks arrive; the last one asks `then` what comes next and lets the others go.
+    // All blocks arrive; then thread 0 of each runs `then`, which all threads see the effects of.
     auto barrier = [&](auto then) {
         __syncthreads();
         if (threadIdx.x == 0) {
-            __threadfence();
-            go_s = 1;
-            if (atomicAdd(&ctl->arrived, 1u) == gridDim.x - 1) {
-                __threadfence();
-                v->arrived = 0;
-                publish(then());
-            } else go_s = wait_next();
+            passed += gridDim.x;
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->arrived) : "memory");
+            const unsigned want = passed;
+            go_s = wait_for(&ctl->arrived, 0, [want](unsigned v) { return (int)(v - want) >= 0; });
+            if (go_s) then(state_s);
         }
         __syncthreads();
         return go_s != 0;
+    };
+    auto end_iteration = [&](State& st) {
+        const Slot* s = &ctl->slot[st.slot];
+        const unsigned long long count = __ldcg(&s->count), cands = __ldcg(&s->cand);
+        next_iteration(st, count, cands, o.cap, max_iterations, SQUARE);
+        st.slot = st.slot == 2 ? 0 : st.slot + 1;
     };
     // The block's last tuples and its count of candidates go out with one atomic each (a warp with a
     // tuple or two each would queue on them for longer than a small iteration takes).
@@ -717,9 +744,9 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
         }
         __syncthreads();
         if (warp == 0) {
-            const unsigned mine = lane < DL_WARPS ? left_s[lane] : 0;
+            const unsigned mine = left_s[lane];
             unsigned incl = mine;
-            unsigned long long c = lane < DL_WARPS ? cand_s[lane] : 0, at = 0;
+            unsigned long long c = cand_s[lane], at = 0;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const unsigned x = __shfl_up_sync(FULL, incl, d);
@@ -729,21 +756,30 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
             for (int d = 16; d; d >>= 1) c += __shfl_xor_sync(FULL, c, d);
             const unsigned total = __shfl_sync(FULL, incl, 31);
             if (lane == 0) {
-                if (total) at = atomicAdd(&ctl->tail, (unsigned long long)total);
-                if (c) atomicAdd(&ctl->candidates, c);
+                if (total) at = atomicAdd(&sink.slot->count, (unsigned long long)total);
+                if (c) atomicAdd(&sink.slot->cand, c);
             }
-            cand_s[lane] = __shfl_sync(FULL, at, 0) + incl - mine;
+            cand_s[lane] = sink.base + __shfl_sync(FULL, at, 0) + incl - mine;
         }
         __syncthreads();
         sink.write_left(cand_s[warp]);
     };
-    read_phase();
+    static_assert(DL_WARPS == 32, "end_block adds up one value a lane");
+    if (threadIdx.x == 0) {
+        const Ctl* c = ctl;
+        state_s = State{__ldcg(&c->start), __ldcg(&c->end), __ldcg(&c->iterations), __ldcg(&c->candidates), __ldcg(&c->phase), __ldcg(&c->check), 0, __ldcg(&c->fix) != 0, false};
+    }
+    __syncthreads();
     for (;;) {
-        const unsigned phase = phase_s;
-        const uint64_t start = range_s[0], n = range_s[1] - range_s[0];
-        const bool check = check_s != 0;
-        if (phase == PH_DONE) return;
+        const unsigned phase = state_s.phase;
+        const uint64_t start = state_s.start, n = state_s.end - state_s.start;
+        const bool check = state_s.check != 0;
+        Slot* slot = &ctl->slot[state_s.slot];
+        sink.slot = slot;
+        sink.base = state_s.end;
+        if (phase == PH_DONE) break;
         if (phase == PH_ROWS) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) ctl->slot[state_s.slot == 2 ? 0 : state_s.slot + 1] = Slot{};
             unsigned long long cand = 0;
             const uint64_t warps = (uint64_t)gridDim.x * DL_WARPS, me = (uint64_t)warp * gridDim.x + blockIdx.x;
             if (SQUARE) {
@@ -751,9 +787,9 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
                 // side by side: every warp takes rows far apart, eight at a time.
                 for (uint64_t first = me; first < n; first += 8 * warps) {
                     const unsigned rows = (unsigned)min((n - first + warps - 1) / warps, (uint64_t)8);
-                    const uint64_t row = lane < rows ? __ldcg(&o.log[start + first + lane * warps]) : 0;
+                    const uint64_t row = lane < rows ? o.log[start + first + lane * warps] : 0;
                     unsigned linear = 0;
-                    take_rows(o, rules, row, rows, heavy, check, sink, linear);
+                    take_rows(o, rules, row, rows, heavy, slot, check, sink, linear);
                     cand += linear;
                     take_square(o, sq, row, rows, sink, cand);
                 }
@@ -765,28 +801,32 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
                 batch = per < 32 ? per : batch < 32 ? 32 : batch > 2048 ? 2048 : batch;
                 for (uint64_t at = me * batch; at < n;) {
                     const uint64_t stop = at + batch < n ? at + batch : n;
-                    uint64_t row = at + lane < stop ? __ldcg(&o.log[start + at + lane]) : 0;
+                    uint64_t row = at + lane < stop ? o.log[start + at + lane] : 0;
                     for (; at < stop; at += per) {
                         const unsigned rows = (unsigned)(stop - at < per ? stop - at : per);
-                        const uint64_t next_row = at + per + lane < stop ? __ldcg(&o.log[start + at + per + lane]) : 0;
+                        const uint64_t next_row = at + per + lane < stop ? o.log[start + at + per + lane] : 0;
                         unsigned linear = 0;
-                        take_rows(o, rules, row, rows, heavy, check, sink, linear);
+                        take_rows(o, rules, row, rows, heavy, slot, check, sink, linear);
                         cand += linear;
                         row = next_row;
                     }
                     if (n <= warps * batch) break;
                     unsigned next = 0;
-                    if (lane == 0) next = atomicAdd(&ctl->next_chunk, 1u);
+                    if (lane == 0) next = atomicAdd(&slot->next_chunk, 1u);
                     at = (warps + __shfl_sync(FULL, next, 0)) * batch;
                 }
             }
             end_block(cand);
-            if (!barrier([&]() -> unsigned { return v->heavy_n ? (unsigned)PH_HEAVY : next_iteration(o, max_iterations, SQUARE); })) return;
+            if (!barrier([&](State& st) {
+                    if (__ldcg(&slot->heavy_n)) st.phase = PH_HEAVY;
+                    else end_iteration(st);
+                }))
+                return;
         } else if (phase == PH_HEAVY) {
-            const unsigned listed = v->heavy_n, pieces = listed < DL_HEAVY_MAX ? listed : (unsigned)DL_HEAVY_MAX;
+            const unsigned listed = __ldcg(&slot->heavy_n), pieces = listed < DL_HEAVY_MAX ? listed : (unsigned)DL_HEAVY_MAX;
             for (;;) {
                 unsigned item = 0;
-                if (lane == 0) item = atomicAdd(&ctl->next_heavy, 1u);
+                if (lane == 0) item = atomicAdd(&slot->next_heavy, 1u);
                 item = __shfl_sync(FULL, item, 0);
                 if (item >= pieces) break;
                 Heavy h;
@@ -796,23 +836,54 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
                 take_piece(o, rules, h, check, sink);
             }
             end_block(0);
-            if (!barrier([&] { return next_iteration(o, max_iterations, SQUARE); })) return;
+            if (!barrier(end_iteration)) return;
         } else if (SQUARE && phase == PH_FULL) {
-            for (uint64_t i = (uint64_t)blockIdx.x * DL_THREADS + threadIdx.x; i < n; i += (uint64_t)gridDim.x * DL_THREADS) square_full(o, sq, __ldcg(&o.log[start + i]));
-            if (!barrier([&]() -> unsigned { return PH_ROWS; })) return;
+            for (uint64_t i = (uint64_t)blockIdx.x * DL_THREADS + threadIdx.x; i < n; i += (uint64_t)gridDim.x * DL_THREADS) square_full(o, sq, o.log[start + i]);
+            if (!barrier([&](State& st) { st.phase = PH_ROWS; })) return;
         } else if (!SQUARE) {  // PH_SOLO
             if (blockIdx.x == 0) {
-                const unsigned next = solo(o, rules, heavy, max_iterations, stage_s, solo_s, start, start + n);
+                State st = state_s;
+                if (rules.n == 1 && rules.r[0].joins == 1) solo<true>(o, rules, heavy, slot, max_iterations, stage_s, solo_s, st);
+                else solo<false>(o, rules, heavy, slot, max_iterations, stage_s, solo_s, st);
                 __syncthreads();
-                if (threadIdx.x == 0) publish(next);  // everybody again
+                if (threadIdx.x == 0) {  // everybody again
+                    state_s = st;
+                    volatile Ctl* v = ctl;
+                    v->solo_start = st.start;
+                    v->solo_end = st.end;
+                    v->solo_iterations = st.iterations;
+                    v->solo_candidates = st.candidates;
+                    v->solo_phase = st.phase;
+                    v->solo_check = st.check;
+                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&ctl->solo_turns), "r"(++solo_turns) : "memory");
+                }
+                __syncthreads();
             } else {
-                if (threadIdx.x == 0) go_s = wait_next();
+                if (threadIdx.x == 0) {
+                    const unsigned want = ++solo_turns;
+                    go_s = wait_for(&ctl->solo_turns, 100, [want](unsigned v) { return (int)(v - want) >= 0; });
+                    state_s.start = __ldcg(&ctl->solo_start);
+                    state_s.end = __ldcg(&ctl->solo_end);
+                    state_s.iterations = __ldcg(&ctl->solo_iterations);
+                    state_s.candidates = __ldcg(&ctl->solo_candidates);
+                    state_s.phase = __ldcg(&ctl->solo_phase);
+                    state_s.check = __ldcg(&ctl->solo_check);
+                }
                 __syncthreads();
                 if (!go_s) return;
             }
         }
-        __syncthreads();
-        read_phase();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        volatile Ctl* v = ctl;
+        v->tail = state_s.end;
+        v->start = state_s.start;
+        v->end = state_s.end;
+        v->iterations = state_s.iterations;
+        v->candidates = state_s.candidates;
+        v->fix = state_s.fix;
+        v->overflow = state_s.overflow;
+        v->check = state_s.check;
     }
 }
 
@@ -835,7 +906,7 @@ __device__ __forceinline__ void ready(Ctl* ctl, bool square) {
     c->end = n;
     c->iterations = n == 0 ? 1 : 0;  // an iteration over nothing finds nothing
     c->fix = n == 0 ? 1 : 0;
-    c->sync = n == 0 ? PH_DONE : square ? PH_FULL : PH_ROWS;  // (never solo: a block that starts late would miss it)
+    c->phase = n == 0 ? PH_DONE : square ? PH_FULL : PH_ROWS;  // (never solo: a block that starts late would miss it)
 }
 // Rows of a bag into the head: new ones (their bit was clear) are appended to the log.
 __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict__ rows, uint64_t n, Out o, bool square) {
@@ -879,7 +950,10 @@ __global__ void delta_begin_k(Ctl* c, bool square) { ready(c, square); }
 // On with the delta at hand, once the log has the room for it.
 __global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
     c->overflow = 0;
-    c->sync = c->iterations >= max_iterations ? PH_DONE : square ? PH_FULL : PH_ROWS;
+    c->arrived = 0;
+    c->solo_turns = 0;
+    for (int k = 0; k < 3; ++k) c->slot[k] = Slot{};
+    c->phase = c->iterations >= max_iterations ? PH_DONE : square ? PH_FULL : PH_ROWS;
 }
 
 }  // namespace
