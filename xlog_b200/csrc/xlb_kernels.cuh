@@ -30,12 +30,24 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
-// Lanes of the warp whose 8-bit value equals this lane's: eight ballots.  (The match.any
-// instruction does the same but its cost grows with the number of distinct values in the warp,
-// and radix digits are close to all-distinct.)
-__device__ __forceinline__ unsigned match_digit(unsigned d) {
-#ifdef XLB_RANK_MATCH
+// Lanes of the warp whose 8-bit value equals this lane's.  `table`: 256 clear words of the warp's own in
+// shared memory; every lane sets its bit in its value's word and reads the word back, two accesses
+// where eight ballots and their masks took some thirty instructions of a kernel that is bound by them.
+// One lane of each group clears the word again (match_clear) once all have read it.
+// (The match.any instruction costs more the more different values there are, and radix digits are
+// close to all different.)
+#ifndef XLB_RANK
+#define XLB_RANK 2
+#endif
+__device__ __forceinline__ unsigned match_digit(unsigned d, unsigned* table) {
+#if XLB_RANK == 1
     return __match_any_sync(FULL, d);
+#elif XLB_RANK == 2
+    atomicOr(&table[d], 1u << lane_id());
+    __syncwarp();
+    const unsigned peers = table[d];
+    __syncwarp();
+    return peers;
 #else
     unsigned peers = FULL;
 #pragma unroll
@@ -45,6 +57,11 @@ __device__ __forceinline__ unsigned match_digit(unsigned d) {
         peers &= bit ? vote : ~vote;
     }
     return peers;
+#endif
+}
+__device__ __forceinline__ void match_clear(unsigned d, unsigned* table) {
+#if XLB_RANK == 2
+    table[d] = 0;
 #endif
 }
 
@@ -580,6 +597,59 @@ constexpr int SORT_IPT = XLB_SORT_IPT;
 constexpr int SORT_TILE = SORT_THREADS * SORT_IPT;  // keys per tile
 constexpr int SORT_WARPS = SORT_THREADS / 32;
 
+// What a pass sorts by: up to eight bits of the key, from one or two places.  A packed pair has its bits
+// at 0.. and 32..: a digit may take the last bits of the low half and the first of the high one, so that a
+// pair of 12-bit values is sorted in three passes and not in four.
+struct Digit {
+    unsigned char s1 = 0, s2 = 0, b1 = 8;  // shifts of the two pieces, bits of the first
+    unsigned char m1 = 255, m2 = 0;        // their masks
+    __host__ __device__ __forceinline__ unsigned operator()(uint64_t k) const { return ((unsigned)(k >> s1) & m1) | (((unsigned)(k >> s2) & m2) << b1); }
+};
+inline Digit whole_digit(int d) {
+    Digit g;
+    g.s1 = (unsigned char)(8 * d);
+    return g;
+}
+struct Digits {
+    Digit d[8];
+    int n = 0;
+};
+// The digits of keys whose bits all lie within `bound`.
+inline Digits plan_digits(uint64_t bound) {
+    const int lb = (bound & 0xFFFFFFFFull) ? 64 - __builtin_clzll(bound & 0xFFFFFFFFull) : 0, hb = bound >> 32 ? 64 - __builtin_clzll(bound >> 32) : 0;
+    Digits p;
+    for (int at = 0; at < lb + hb; at += 8) {  // bits counted without the gap
+        Digit g;
+        const int first = std::max(0, std::min(8, lb - at)), second = std::min(8 - first, lb + hb - at - first);
+        if (first) {
+            g.s1 = (unsigned char)at;
+            g.b1 = (unsigned char)first;
+            g.m1 = (unsigned char)((1u << first) - 1);
+            g.s2 = 32;
+            g.m2 = (unsigned char)((1u << second) - 1);
+        } else {
+            g.s1 = (unsigned char)(32 + at - lb);
+            g.b1 = 8;
+            g.m1 = (unsigned char)((1u << second) - 1);
+            g.m2 = 0;
+        }
+        p.d[p.n++] = g;
+    }
+    return p;
+}
+
+// The digits of `bits` adjacent bits from bit `from` on.
+inline Digits run_of_digits(int from, int bits) {
+    Digits p;
+    for (int at = 0; at < bits; at += 8) {
+        Digit g;
+        g.s1 = (unsigned char)(from + at);
+        g.m1 = (unsigned char)((1u << std::min(8, bits - at)) - 1);
+        p.d[p.n++] = g;
+    }
+    return p;
+}
+
 // OR and AND of all keys in one read: a digit whose bits never vary needs no pass.
 static __global__ void __launch_bounds__(BLOCK) radix_bits_k(const uint64_t* __restrict__ keys, uint64_t n, unsigned long long* __restrict__ or_and /* [2] */) {
     uint64_t o = 0, a = ~0ull;
@@ -599,10 +669,9 @@ static __global__ void __launch_bounds__(BLOCK) radix_bits_k(const uint64_t* __r
     }
 }
 
-// Histograms of all eight digits in one read of the keys.  A digit on which a whole warp agrees
+// Histograms of all digits in one read of the keys.  A digit on which a whole warp agrees
 // (constant high bytes are the common case) costs one shared-memory add per warp.
-// `digits`: bit d set = digit d is wanted (the others are known constant or take no part).
-static __global__ void __launch_bounds__(BLOCK) radix_upfront_k(const uint64_t* __restrict__ keys, uint64_t n, unsigned int* __restrict__ ghist /* 8*256 */, unsigned digits) {
+static __global__ void __launch_bounds__(BLOCK) radix_upfront_k(const uint64_t* __restrict__ keys, uint64_t n, unsigned int* __restrict__ ghist /* 8*256 */, const Digits digits) {
     __shared__ unsigned int sh[8 * 256];
     for (int i = threadIdx.x; i < 8 * 256; i += BLOCK) sh[i] = 0;
     __syncthreads();
@@ -616,8 +685,8 @@ static __global__ void __launch_bounds__(BLOCK) radix_upfront_k(const uint64_t* 
         unsigned first_lane = __ffs(live) - 1;
 #pragma unroll
         for (int d = 0; d < 8; ++d) {
-            if (!((digits >> d) & 1u)) continue;
-            unsigned dig = (unsigned)((k >> (8 * d)) & 255);
+            if (d >= digits.n) break;
+            unsigned dig = digits.d[d](k);
             unsigned first = __shfl_sync(FULL, dig, first_lane);
             bool uni = __all_sync(FULL, !ok || dig == first);
             if (uni) {
@@ -688,7 +757,7 @@ constexpr unsigned LB_FLAG_AGG = 1u << 30, LB_FLAG_INC = 2u << 30, LB_MASK = (1u
 template <bool HAS_VALUES, bool LOOKBACK>
 static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scatter_k(const uint64_t* __restrict__ keys_in, uint64_t* __restrict__ keys_out,
                                                           const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ vals_out,
-                                                          uint64_t n, int shift, const uint32_t* __restrict__ offs, uint32_t ntiles,
+                                                          uint64_t n, const Digit digit, const uint32_t* __restrict__ offs, uint32_t ntiles,
                                                           unsigned int* __restrict__ tile_counter, volatile unsigned int* status, DevStatus* dst,
                                                           unsigned spin_limit) {
     extern __shared__ __align__(16) unsigned char sort_smem[];
@@ -698,6 +767,8 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
     unsigned int* glob_off = tile_start + 256;
     unsigned int* scan_sm = glob_off + 256;
 
+    // (the table of match_digit lies where the keys will be reordered)
+    unsigned int (*smatch)[256] = reinterpret_cast<unsigned int (*)[256]>(sort_smem);
     __shared__ unsigned int tile_s;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     unsigned tile = blockIdx.x;
@@ -711,7 +782,10 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
     const uint64_t rem = n - tile_base;
     const unsigned valid = rem < (uint64_t)SORT_TILE ? (unsigned)rem : (unsigned)SORT_TILE;
 
-    for (int i = threadIdx.x; i < SORT_WARPS * 256; i += SORT_THREADS) (&whist[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < SORT_WARPS * 256; i += SORT_THREADS) {
+        (&whist[0][0])[i] = 0;
+        (&smatch[0][0])[i] = 0;
+    }
     if (!LOOKBACK && threadIdx.x < 256) glob_off[threadIdx.x] = offs[(uint64_t)threadIdx.x * ntiles + tile];
 
     // warp-striped load: key j of lane l sits at warp*512 + j*32 + l (memory order = (j, l))
@@ -729,13 +803,14 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
 #pragma unroll
     for (int j = 0; j < SORT_IPT; ++j) {
         unsigned t = wbase + j * 32 + lane;
-        unsigned d = t < valid ? (unsigned)((key[j] >> shift) & 255) : 255u;
-        unsigned peers = match_digit(d);
+        unsigned d = t < valid ? digit(key[j]) : 255u;
+        const unsigned peers = match_digit(d, &smatch[warp][0]);
         unsigned leader = __ffs(peers) - 1;
         unsigned before = 0;
         if (lane == leader) {
             before = whist[warp][d];
             whist[warp][d] = before + __popc(peers);
+            match_clear(d, &smatch[warp][0]);
         }
         before = __shfl_sync(FULL, before, leader);
         rank[j] = (unsigned short)(before + __popc(peers & lanemask_lt()));
@@ -795,7 +870,7 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
 #pragma unroll
     for (int j = 0; j < SORT_IPT; ++j) {
         unsigned t = wbase + j * 32 + lane;
-        unsigned d = t < valid ? (unsigned)((key[j] >> shift) & 255) : 255u;
+        unsigned d = t < valid ? digit(key[j]) : 255u;
         unsigned p = tile_start[d] + whist[warp][d] + rank[j];
         pos[j] = (unsigned short)p;
         skeys[p] = key[j];
@@ -804,7 +879,7 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
     // coalesced runs: consecutive shared-memory slots of one digit go to consecutive addresses
     for (unsigned i = threadIdx.x; i < valid; i += SORT_THREADS) {
         uint64_t k = skeys[i];
-        unsigned d = (unsigned)((k >> shift) & 255);
+        unsigned d = digit(k);
         keys_out[(uint64_t)glob_off[d] + (i - tile_start[d])] = k;
     }
     if (HAS_VALUES) {
@@ -817,8 +892,8 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
         for (int j = 0; j < SORT_IPT; ++j) {
             unsigned t = wbase + j * 32 + lane;
             if (t < valid) {
-                sv[pos[j]] = vals_in[tile_base + t];
-                sd[pos[j]] = (uint8_t)((key[j] >> shift) & 255);
+                sv[pos[j]] = vals_in ? vals_in[tile_base + t] : (uint32_t)(tile_base + t);  // (none: row numbers)
+                sd[pos[j]] = (uint8_t)digit(key[j]);
             }
         }
         __syncthreads();
@@ -833,13 +908,14 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
 // digits in one launch without a read-back.  (The one-sweep route takes two fills, two kernels, a
 // read-back and a launch per digit: 60 us for 2000 keys of three digits, against 9.)
 constexpr int SS_THREADS = 1024, SS_WARPS = SS_THREADS / 32, SS_MAX = SS_THREADS * 8;
-template <int IPT>
-static __global__ void __launch_bounds__(SS_THREADS) radix_small_k(const uint64_t* __restrict__ keys_in, uint64_t* __restrict__ keys_out, const uint32_t* __restrict__ vals_in,
-                                                                  uint32_t* __restrict__ vals_out, unsigned n, unsigned digit_mask) {
+// `load(i, val)` gives key i and sets its payload, `store(i, key, val)` takes what ends at place i.
+template <int IPT, class Load, class Store>
+static __global__ void __launch_bounds__(SS_THREADS) radix_small_k(const Load load, const Store store, unsigned n, unsigned digit_mask) {
     extern __shared__ __align__(16) unsigned char ss_smem[];
     uint64_t* sk = reinterpret_cast<uint64_t*>(ss_smem);
     uint32_t* sv = reinterpret_cast<uint32_t*>(sk + SS_THREADS * IPT);
     unsigned short (*wh)[256] = reinterpret_cast<unsigned short (*)[256]>(sv + SS_THREADS * IPT);
+    unsigned (*smatch)[256] = reinterpret_cast<unsigned (*)[256]>(wh + SS_WARPS);
     __shared__ unsigned bits_s[4], base_s[256], warp_s[8];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5, first = warp * (32 * IPT) + lane;
     uint64_t key[IPT];
@@ -853,8 +929,7 @@ static __global__ void __launch_bounds__(SS_THREADS) radix_small_k(const uint64_
         key[j] = ~0ull;  // past the end: behind every key, in its place already
         val[j] = 0;
         if (i < n) {
-            key[j] = keys_in[i];
-            if (vals_in) val[j] = vals_in[i];
+            key[j] = load(i, val[j]);
             all_or |= key[j];
             all_and &= key[j];
         }
@@ -872,15 +947,17 @@ static __global__ void __launch_bounds__(SS_THREADS) radix_small_k(const uint64_
     for (int d = 0; d < 8; ++d) {
         if (!((digit_mask >> d) & 1u) || !((varying >> (8 * d)) & 255)) continue;
         for (unsigned i = threadIdx.x; i < SS_WARPS * 256 / 2; i += SS_THREADS) reinterpret_cast<unsigned*>(&wh[0][0])[i] = 0;
+        for (unsigned i = threadIdx.x; i < SS_WARPS * 256; i += SS_THREADS) (&smatch[0][0])[i] = 0;
         __syncthreads();
         unsigned short rank[IPT];
 #pragma unroll
         for (int j = 0; j < IPT; ++j) {
-            const unsigned x = (unsigned)(key[j] >> (8 * d)) & 255, peers = match_digit(x), leader = __ffs(peers) - 1;
+            const unsigned x = (unsigned)(key[j] >> (8 * d)) & 255, peers = match_digit(x, &smatch[warp][0]), leader = __ffs(peers) - 1;
             unsigned before = 0;
             if (lane == leader) {
                 before = wh[warp][x];
                 wh[warp][x] = (unsigned short)(before + __popc(peers));
+                match_clear(x, &smatch[warp][0]);
             }
             before = __shfl_sync(FULL, before, leader);
             rank[j] = (unsigned short)(before + __popc(peers & lanemask_lt()));
@@ -927,21 +1004,45 @@ static __global__ void __launch_bounds__(SS_THREADS) radix_small_k(const uint64_
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
         const unsigned i = first + j * 32;
-        if (i < n) {
-            keys_out[i] = key[j];
-            if (vals_out) vals_out[i] = val[j];
-        }
+        if (i < n) store(i, key[j], val[j]);
     }
 }
-template <int IPT>
-inline void radix_small(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned digit_mask) {
-    constexpr size_t smem = (size_t)SS_THREADS * IPT * 12 + SS_WARPS * 512;
-    if (smem > (48u << 10)) CUDA_OK(cudaFuncSetAttribute(radix_small_k<IPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    Buf outk = make_buf(c, n * 8), outv = vals ? make_buf(c, n * 4) : Buf();
-    prof_begin(c, "radix_small", n * (vals ? 24ull : 16ull));
-    radix_small_k<IPT><<<1, SS_THREADS, smem, c->stream>>>(keys->as<uint64_t>(), outk->as<uint64_t>(), vals ? (*vals)->as<uint32_t>() : nullptr, vals ? outv->as<uint32_t>() : nullptr,
-                                                          (unsigned)n, digit_mask);
+struct LoadKeys {
+    const uint64_t* keys;
+    const uint32_t* vals;
+    __device__ __forceinline__ uint64_t operator()(unsigned i, uint32_t& val) const {
+        val = vals ? vals[i] : i;  // (none: row numbers)
+        return keys[i];
+    }
+};
+struct StoreKeys {
+    uint64_t* keys;
+    uint32_t* vals;
+    __device__ __forceinline__ void operator()(unsigned i, uint64_t key, uint32_t val) const {
+        keys[i] = key;
+        if (vals) vals[i] = val;
+    }
+};
+template <int IPT, class Load, class Store>
+inline void launch_radix_small(xlb_ctx* c, const Load& load, const Store& store, uint64_t n, unsigned digit_mask) {
+    constexpr size_t smem = (size_t)SS_THREADS * IPT * 12 + SS_WARPS * 1536;
+    if (smem > (48u << 10)) CUDA_OK(cudaFuncSetAttribute(radix_small_k<IPT, Load, Store>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    prof_begin(c, "radix_small", n * 24ull);
+    radix_small_k<IPT><<<1, SS_THREADS, smem, c->stream>>>(load, store, (unsigned)n, digit_mask);
     check_launch(c, "radix_small");
+}
+// at most SS_MAX keys, with anything to read them from and anything to write them to
+template <class Load, class Store>
+inline void radix_small(xlb_ctx* c, const Load& load, const Store& store, uint64_t n, unsigned digit_mask) {
+    if (n <= SS_THREADS) launch_radix_small<1>(c, load, store, n, digit_mask);
+    else if (n <= 2 * SS_THREADS) launch_radix_small<2>(c, load, store, n, digit_mask);
+    else if (n <= 4 * SS_THREADS) launch_radix_small<4>(c, load, store, n, digit_mask);
+    else launch_radix_small<8>(c, load, store, n, digit_mask);
+}
+inline void radix_small_keys(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned digit_mask) {
+    Buf outk = make_buf(c, n * 8), outv = vals ? make_buf(c, n * 4) : Buf();
+    radix_small(c, LoadKeys{keys->as<uint64_t>(), vals && *vals ? (*vals)->as<uint32_t>() : nullptr}, StoreKeys{outk->as<uint64_t>(), vals ? outv->as<uint32_t>() : nullptr}, n,
+                digit_mask);
     keys = outk;
     if (vals) *vals = outv;
 }
@@ -983,21 +1084,22 @@ inline SortPlan plan_sort(xlb_ctx* c, const uint64_t* keys, uint64_t n) {
 }
 
 // Sorts `n` keys ascending (stable).  keys/vals are replaced by buffers holding the result;
-// vals may be empty.  n must be below 2^32.
+// vals may be null (keys only) or point to an empty buffer (the payload is then the row number).
+// n must be below 2^32.
 // `digit_mask` bit d set = digit d (bits 8d..8d+7) takes part in the order; a join index only
 // needs its rows grouped by the key half, i.e. digits 4..7.
 // `known_bound` != ~0: an upper bound of the OR of all keys that the host already holds; digits
 // outside it are constant, so the digit plan needs no read-back.
 // `keep_input`: the buffer `keys` names on entry is left untouched (it may belong to a stored
 // relation); the first pass reads it and later passes ping-pong between two fresh buffers.
-inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned digit_mask = 0xFFu, uint64_t known_bound = ~0ull, bool keep_input = false) {
-    if (n <= 1) return;
+// `plan`: the digits to sort by, where the caller knows them better (bits outside them take part only
+// where they cannot change the order: small sorts and those of 2^30 keys and more go by whole bytes).
+inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned digit_mask = 0xFFu, uint64_t known_bound = ~0ull, bool keep_input = false,
+                       const Digits* plan = nullptr) {
+    if (n == 0 || (n == 1 && !(vals && !*vals))) return;
     if (n >= (1ull << 32)) xlb_fail(XLB_ERR_CAPACITY, "sort of %llu keys exceeds the 2^32 limit of one sort", (unsigned long long)n);
     if (n <= (uint64_t)SS_MAX && !c->lb_first_tile) {
-        if (n <= SS_THREADS) radix_small<1>(c, keys, vals, n, digit_mask);
-        else if (n <= 2 * SS_THREADS) radix_small<2>(c, keys, vals, n, digit_mask);
-        else if (n <= 4 * SS_THREADS) radix_small<4>(c, keys, vals, n, digit_mask);
-        else radix_small<8>(c, keys, vals, n, digit_mask);
+        radix_small_keys(c, keys, vals, n, digit_mask);
         return;
     }
     radix_sort_setup(c);
@@ -1011,26 +1113,37 @@ inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned di
         unsigned int* bases = ghist + 8 * 256;
         unsigned long long* varies = (unsigned long long*)(bases + 8 * 256);
         CUDA_OK(set_async(c, ghist, 0, 8 * 256 * 4));
-        unsigned want = digit_mask & 0xFFu;
-        if (known_bound != ~0ull)
+        const bool known = plan || known_bound != ~0ull;
+        Digits digits;
+        if (plan) {
+            digits = *plan;
+        } else if (known) {
+            uint64_t keep = 0;
             for (int d = 0; d < 8; ++d)
-                if (!((known_bound >> (8 * d)) & 255)) want &= ~(1u << d);
-        if (want == 0) return;
+                if ((digit_mask >> d) & 1u) keep |= 255ull << (8 * d);
+            digits = plan_digits(known_bound & keep);
+        } else {
+            for (int d = 0; d < 8; ++d)
+                if ((digit_mask >> d) & 1u) digits.d[digits.n++] = whole_digit(d);
+        }
+        if (digits.n == 0 && vals && !*vals) digits.d[digits.n++] = whole_digit(0);  // no bit varies: the row numbers are still to be written
+        if (digits.n == 0) return;
         prof_begin(c, "radix_upfront", n * 8ull);
-        radix_upfront_k<<<grid_for(c, n, BLOCK * 8), BLOCK, 0, c->stream>>>(keys->as<uint64_t>(), n, ghist, want);
+        radix_upfront_k<<<grid_for(c, n, BLOCK * 8), BLOCK, 0, c->stream>>>(keys->as<uint64_t>(), n, ghist, digits);
         check_launch(c, "radix_upfront");
         prof_begin(c, "radix_bases", 0);
         radix_bases_k<<<1, BLOCK, 0, c->stream>>>(ghist, n, bases, varies);
         check_launch(c, "radix_bases");
-        unsigned long long v[8];
-        if (known_bound != ~0ull) {
-            for (int d = 0; d < 8; ++d) v[d] = (known_bound >> (8 * d)) & 255 ? 1 : 0;
+        int np = 0, pass[8];
+        if (known) {
+            for (int d = 0; d < digits.n; ++d) pass[np++] = d;
         } else {
+            unsigned long long v[8];
             read_words(c, varies, 8, v);
+            for (int d = 0; d < digits.n; ++d)
+                if (v[d]) pass[np++] = d;
         }
-        int np = 0, digits[8];
-        for (int d = 0; d < 8; ++d)
-            if (v[d] && ((digit_mask >> d) & 1u)) digits[np++] = d;
+        if (np == 0 && vals && !*vals) pass[np++] = 0;  // all keys equal: the row numbers are still to be written
         if (np == 0) return;
         uint64_t status_words = (uint64_t)ntiles * 256;
         Buf status = make_buf(c, (status_words * np + 8) * 4);  // per pass: tile status; then 8 tile counters
@@ -1041,19 +1154,22 @@ inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned di
             CUDA_OK(copy_async(c, counters, &c->h_scalar[56], 8 * 4, cudaMemcpyHostToDevice));
         }
         for (int q = 0; q < np; ++q) {
-            int d = digits[q];
+            const int d = pass[q];
             unsigned int* st = status->as<unsigned int>() + status_words * q;
             prof_begin(c, "radix_scatter", n * (vals ? 24ull : 16ull));
             if (vals)
-                radix_scatter_k<true, true><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), (*vals)->as<uint32_t>(), tmpv->as<uint32_t>(), n, 8 * d, bases + d * 256, ntiles, counters + q, st, c->d_status, c->lb_spin_limit);
+                radix_scatter_k<true, true><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), *vals ? (*vals)->as<uint32_t>() : nullptr, tmpv->as<uint32_t>(), n, digits.d[d], bases + d * 256, ntiles, counters + q, st, c->d_status, c->lb_spin_limit);
             else
-                radix_scatter_k<false, true><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), nullptr, nullptr, n, 8 * d, bases + d * 256, ntiles, counters + q, st, c->d_status, c->lb_spin_limit);
+                radix_scatter_k<false, true><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), nullptr, nullptr, n, digits.d[d], bases + d * 256, ntiles, counters + q, st, c->d_status, c->lb_spin_limit);
             check_launch(c, "radix_scatter");
             if (keep_input && q == 0) {
                 keys = tmpk;
                 tmpk = np > 1 ? make_buf(c, n * 8) : Buf();
             } else std::swap(keys, tmpk);
-            if (vals) std::swap(*vals, tmpv);
+            if (vals) {
+                std::swap(*vals, tmpv);
+                if (!tmpv && q + 1 < np) tmpv = make_buf(c, n * 4);
+            }
         }
         return;
     }
@@ -1062,6 +1178,7 @@ inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned di
     SortPlan p0 = plan_sort(c, keys->as<uint64_t>(), n), p;
     for (int q = 0; q < p0.npasses; ++q)
         if ((digit_mask >> (p0.shifts[q] / 8)) & 1u) p.shifts[p.npasses++] = p0.shifts[q];
+    if (p.npasses == 0 && vals && !*vals) p.shifts[p.npasses++] = 0;  // all keys equal: the row numbers are still to be written
     if (p.npasses == 0) return;
     Buf hist = make_buf(c, (uint64_t)256 * ntiles * 4);
     Buf offs = make_buf(c, (uint64_t)256 * ntiles * 4);
@@ -1074,15 +1191,18 @@ inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned di
         exclusive_scan<LoadU32, uint32_t>(c, LoadU32{hist->as<uint32_t>()}, (uint64_t)256 * ntiles, offs->as<uint32_t>(), total->as<uint32_t>());
         prof_begin(c, "radix_scatter", n * (vals ? 24ull : 16ull));
         if (vals)
-            radix_scatter_k<true, false><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), (*vals)->as<uint32_t>(), tmpv->as<uint32_t>(), n, shift, offs->as<uint32_t>(), ntiles, nullptr, nullptr, c->d_status, 0u);
+            radix_scatter_k<true, false><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), *vals ? (*vals)->as<uint32_t>() : nullptr, tmpv->as<uint32_t>(), n, whole_digit(shift / 8), offs->as<uint32_t>(), ntiles, nullptr, nullptr, c->d_status, 0u);
         else
-            radix_scatter_k<false, false><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), nullptr, nullptr, n, shift, offs->as<uint32_t>(), ntiles, nullptr, nullptr, c->d_status, 0u);
+            radix_scatter_k<false, false><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(keys->as<uint64_t>(), tmpk->as<uint64_t>(), nullptr, nullptr, n, whole_digit(shift / 8), offs->as<uint32_t>(), ntiles, nullptr, nullptr, c->d_status, 0u);
         check_launch(c, "radix_scatter");
         if (keep_input && q == 0) {
             keys = tmpk;
             tmpk = p.npasses > 1 ? make_buf(c, n * 8) : Buf();
         } else std::swap(keys, tmpk);
-        if (vals) std::swap(*vals, tmpv);
+        if (vals) {
+            std::swap(*vals, tmpv);
+            if (!tmpv && q + 1 < p.npasses) tmpv = make_buf(c, n * 4);
+        }
     }
 }
 
@@ -1682,7 +1802,7 @@ inline Buf mix_and_group(xlb_ctx* c, const uint64_t* in, uint64_t n) {
         CUDA_OK(copy_async(c, counters, &c->h_scalar[56], 8 * 4, cudaMemcpyHostToDevice));
     }
     prof_begin(c, "radix_scatter", n * 16ull);
-    radix_scatter_k<false, true><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(words->as<uint64_t>(), out->as<uint64_t>(), nullptr, nullptr, n, 56, bases + 7 * 256, ntiles, counters,
+    radix_scatter_k<false, true><<<ntiles, SORT_THREADS, SORT_SMEM, c->stream>>>(words->as<uint64_t>(), out->as<uint64_t>(), nullptr, nullptr, n, whole_digit(7), bases + 7 * 256, ntiles, counters,
                                                                                status->as<unsigned int>(), c->d_status, c->lb_spin_limit);
     check_launch(c, "radix_scatter");
     return out;

@@ -12,19 +12,15 @@ using namespace xk;
 // ------------------------------------------------------------------------------ small kernels
 namespace {
 
-__global__ void iota_k(uint32_t* out, uint64_t n) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) out[i] = (uint32_t)i;
-}
 __global__ void iota64_k(uint64_t* out, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) out[i] = i;
 }
 // key word of a row from up to two columns: (a << 32 | b) for two 32-bit columns, the value itself otherwise
-__global__ void build_key_k(const void* c0, int w0, const void* c1, int w1, const uint32_t* idx, uint64_t* out, uint64_t n) {
+__global__ void build_key_k(const void* c0, int w0, const void* c1, uint64_t* out, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t r = idx ? idx[i] : i;
-        uint64_t a = w0 == 4 ? ((const uint32_t*)c0)[r] : w0 == 8 ? ((const uint64_t*)c0)[r] : ((const uint8_t*)c0)[r];
+        uint64_t a = w0 == 4 ? ((const uint32_t*)c0)[i] : w0 == 8 ? ((const uint64_t*)c0)[i] : ((const uint8_t*)c0)[i];
         if (c1) {
-            uint64_t b = ((const uint32_t*)c1)[r];
+            uint64_t b = ((const uint32_t*)c1)[i];
             a = (a << 32) | b;
         }
         out[i] = a;
@@ -1427,67 +1423,42 @@ static ColSet colset_of(const xlb_rel* r) {
     return cs;
 }
 
-// Stable sort permutation by key columns (first key most significant): LSD over the key
-// columns, least significant first, each a stable (key word, row index) radix sort.
-static Buf sort_permutation(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_t nk) {
-    uint64_t n = r->rows;
-    Buf idx = make_buf(c, n * 4);
-    if (n == 0) return idx;
-    if (n >= (1ull << 32)) xlb_fail(XLB_ERR_CAPACITY, "sort of %llu rows exceeds the 2^32 row limit", (unsigned long long)n);
-    prof_begin(c, "iota", 0);
-    iota_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(idx->as<uint32_t>(), n);
-    check_launch(c, "iota");
-    int k = (int)nk - 1;
-    while (k >= 0) {
-        // fuse two adjacent 32-bit key columns into one 64-bit key word
-        int w1 = (int)type_width(r->schema.types[keys[k]]);
-        const void* lo = nullptr;
-        int hi_col = k;
-        if (w1 == 4 && k >= 1 && type_width(r->schema.types[keys[k - 1]]) == 4) {
-            lo = r->cols[keys[k]]->p;
-            hi_col = k - 1;
+struct GatherCols {
+    const void* from[XLB_MAX_ARITY];
+    void* to[XLB_MAX_ARITY];
+    int width[XLB_MAX_ARITY], n;
+};
+// all columns in one launch: the row numbers are read once
+static __global__ void gather_cols_k(const GatherCols g, const uint32_t* __restrict__ idx, uint64_t n) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t row = idx[i];
+        for (int k = 0; k < g.n; ++k) {
+            if (g.width[k] == 4) ((uint32_t*)g.to[k])[i] = __ldg((const uint32_t*)g.from[k] + row);
+            else if (g.width[k] == 8) ((unsigned long long*)g.to[k])[i] = __ldg((const unsigned long long*)g.from[k] + row);
+            else ((uint8_t*)g.to[k])[i] = __ldg((const uint8_t*)g.from[k] + row);
         }
-        Buf kw = make_buf(c, n * 8);
-        const xlb_rel* rr = r;
-        prof_begin(c, "build_key", 0);
-        build_key_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(rr->cols[keys[hi_col]]->p, (int)type_width(r->schema.types[keys[hi_col]]), lo, 4, idx->as<uint32_t>(), kw->as<uint64_t>(), n);
-        check_launch(c, "build_key");
-        radix_sort(c, kw, &idx, n);
-        k = hi_col - 1;
     }
-    return idx;
 }
-
 static xlb_rel* gather_rel(xlb_ctx* c, const xlb_rel* r, const uint32_t* idx, uint64_t n) {
     std::unique_ptr<xlb_rel> o(new xlb_rel);
     o->ctx = c;
     o->schema = r->schema;
     o->rows = n;
+    GatherCols g{};
+    g.n = (int)r->schema.arity;
     for (uint32_t i = 0; i < r->schema.arity; ++i) {
         uint32_t w = type_width(r->schema.types[i]);
         o->cols[i] = make_buf(c, n * w);
-        if (!n) continue;
+        g.from[i] = r->cols[i]->p;
+        g.to[i] = o->cols[i]->p;
+        g.width[i] = (int)w;
+    }
+    if (n && g.n) {
         prof_begin(c, "gather", 0);
-        if (w == 4) gather_k<uint32_t><<<grid_for(c, n), BLOCK, 0, c->stream>>>(r->cols[i]->as<uint32_t>(), idx, o->cols[i]->as<uint32_t>(), n);
-        else if (w == 8) gather_k<uint64_t><<<grid_for(c, n), BLOCK, 0, c->stream>>>(r->cols[i]->as<uint64_t>(), idx, o->cols[i]->as<uint64_t>(), n);
-        else gather_k<uint8_t><<<grid_for(c, n), BLOCK, 0, c->stream>>>(r->cols[i]->as<uint8_t>(), idx, o->cols[i]->as<uint8_t>(), n);
+        gather_cols_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(g, idx, n);
         check_launch(c, "gather");
     }
     return o.release();
-}
-
-static xlb_status sort_unsigned(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols, uint32_t nk, xlb_rel** out_final) {
-    if (!c || !in || !out_final) return XLB_ERR_INVALID;
-    API_BEGIN(c)
-    ResultGuard guard;
-    xlb_rel** out = &guard.r;
-    for (uint32_t i = 0; i < nk; ++i)
-        if (key_cols[i] >= in->schema.arity) xlb_fail(XLB_ERR_INVALID, "sort key column %u out of range", key_cols[i]);
-    ops_rel_columns(c, in);
-    Buf idx = sort_permutation(c, in, key_cols, nk);
-    *out = gather_rel(c, in, idx->as<uint32_t>(), in->rows);
-    guard.deliver(c, out_final);
-    API_END()
 }
 
 xlb_rel* rel_view(xlb_ctx* c, const xlb_rel* r) {
@@ -2078,7 +2049,13 @@ static xlb_status with_typed(xlb_ctx* c, const xlb_rel* const* ins, uint32_t n, 
 
 extern "C" xlb_status xlb_sort(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols, uint32_t nk, xlb_rel** out) {
     if (!c || !in || !out) return XLB_ERR_INVALID;
-    return with_typed(c, &in, 1, out, [&](const xlb_rel* const* v, xlb_rel** o) { return sort_unsigned(c, v[0], key_cols, nk, o); });
+    API_BEGIN(c)
+    ResultGuard guard;
+    for (uint32_t i = 0; i < nk; ++i)
+        if (key_cols[i] >= in->schema.arity) xlb_fail(XLB_ERR_INVALID, "sort key column %u out of range", key_cols[i]);
+    guard.r = sort_rows(c, in, key_cols, nk);
+    guard.deliver(c, out);
+    API_END()
 }
 extern "C" xlb_status xlb_dedup(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols, uint32_t nk, xlb_rel** out) {
     if (!c || !in || !out) return XLB_ERR_INVALID;
@@ -2195,7 +2172,7 @@ static Buf join_keys(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_
     int w0 = (int)type_width(r->schema.types[keys[0]]);
     const void* c1 = nk == 2 ? r->cols[keys[1]]->p : nullptr;
     prof_begin(c, "build_key", 0);
-    build_key_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(r->cols[keys[0]]->p, w0, c1, 4, nullptr, kw->as<uint64_t>(), r->rows);
+    build_key_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(r->cols[keys[0]]->p, w0, c1, kw->as<uint64_t>(), r->rows);
     check_launch(c, "build_key");
     return kw;
 }
@@ -2230,10 +2207,7 @@ xlb_rel* rel_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t
     if (xlb_rel* o = query_join(c, l, r, lk, rk, nk, os)) return o;
     // a key with many rows: order the build rows by key word (stable, so equal keys keep right-row order)
     Buf rkeys = join_keys(c, r, rk, nk);
-    Buf ridx = make_buf(c, r->rows * 4);
-    prof_begin(c, "iota", 0);
-    iota_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(ridx->as<uint32_t>(), r->rows);
-    check_launch(c, "iota");
+    Buf ridx;
     radix_sort(c, rkeys, &ridx, r->rows);
     Index ix = ops_index_build(c, rkeys, r->rows, 0, ridx);
     Buf lkeys = join_keys(c, l, lk, nk);

@@ -306,6 +306,10 @@ xlb_rel* rel_union_many(xlb_ctx* c, const xlb_rel* const* ins, uint32_t n);
 xlb_rel* rel_difference(xlb_ctx* c, const xlb_rel* a, const xlb_rel* b);
 xlb_rel* rel_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, xlb_join_type type);
 
+// Row order (xlb_sort.cu), stable, first key most significant, each type in its own order; `r` as columns.
+Buf sort_permutation(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_t nk);  // row numbers in order
+xlb_rel* sort_rows(xlb_ctx* c, const xlb_rel* in, const uint32_t* keys, uint32_t nk);
+
 // Joins and aggregation without sorting (xlb_query.cu); inputs as columns, checked by the callers.
 // Left rows that have (want) or lack a match, in left order.
 xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, bool want);
