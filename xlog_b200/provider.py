@@ -19,6 +19,7 @@ from .lib import XlbError, load
 
 _NP = {A.U32: np.uint32, A.SYMBOL: np.uint32, A.U64: np.uint64, A.I32: np.int32, A.I64: np.int64,
        A.F32: np.float32, A.F64: np.float64, A.BOOL: np.uint8}
+_DTYPE = {t: np.dtype(d) for t, d in _NP.items()}
 _CODE = {np.dtype(np.uint32): A.U32, np.dtype(np.uint64): A.U64, np.dtype(np.int32): A.I32, np.dtype(np.int64): A.I64,
          np.dtype(np.float32): A.F32, np.dtype(np.float64): A.F64, np.dtype(np.bool_): A.BOOL}
 
@@ -165,8 +166,8 @@ class KernelProvider:
     def download(self, buf: Buffer) -> list[np.ndarray]:
         schema = buf.schema()
         n = buf.num_rows()
-        cols = _host_columns(self._lib, n, [np.dtype(_NP[t]) for t in schema])
-        ptrs = (C.c_void_p * max(len(cols), 1))(*[c.ctypes.data for c in cols])
+        cols = _host_columns(self._lib, n, [_DTYPE[t] for t in schema])
+        ptrs = (C.c_void_p * max(len(cols), 1))(*[C.addressof(C.c_byte.from_buffer(c)) if n else None for c in cols])
         rows = C.c_uint64()
         self._check(self._lib.xlb_rel_to_host(self._ctx, buf._h, ptrs, n, C.byref(rows)))
         return cols
