@@ -230,6 +230,10 @@ struct LoadU32 {
     const uint32_t* p;
     __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return p[i]; }
 };
+struct LoadU64 {
+    const uint64_t* p;
+    __device__ __forceinline__ uint64_t operator()(uint64_t i) const { return p[i]; }
+};
 struct LoadLow32 {  // low half of a u64 word (the match length of a probe result)
     const uint64_t* p;
     __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return (uint32_t)p[i]; }
@@ -275,29 +279,98 @@ void exclusive_scan(xlb_ctx* c, Load load, uint64_t n, Tout* out, Tout* d_total)
 
 // ---------------------------------------------------------------------------------- select
 // Stable compaction: Pred(i) -> keep?, Emit(i, pos) stores row i at output position pos.
-template <class Pred>
-static __global__ void __launch_bounds__(BLOCK) select_count_k(Pred pred, uint64_t n, uint32_t* tile_counts) {
-    __shared__ uint32_t sm[33];
-    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_IPT; ++k) {
-        uint64_t i = base + (uint64_t)k * BLOCK + threadIdx.x;
-        if (i < n && pred(i)) s++;
+// One sweep: a tile takes its number from a ticket, leaves its count and gets the sum of all earlier
+// ones by looking back, 32 tiles at a time (they took earlier numbers, so they are running or done; the
+// wait is bounded).  Counting in one launch, scanning the counts and reading the rows again took
+// three launches: 29 us for 3 M rows.
+struct SelectTiles {
+    unsigned n = 1;
+    unsigned long long* state = nullptr;  // flag in the two top bits: 1 the tile's count, 2 the sum up to and with it
+    unsigned* ticket = nullptr;
+    DevStatus* st = nullptr;
+    unsigned spin_limit = 0;
+    const uint64_t* known = nullptr;  // the sums, for a caller without room for a status to wait with
+    // the number of this block's tile, for all its threads
+    __device__ __forceinline__ unsigned take(unsigned& shared) const {
+        if (n <= 1) return 0;
+        if (threadIdx.x == 0) shared = ticket ? atomicAdd(ticket, 1u) : blockIdx.x;
+        __syncthreads();
+        return shared;
     }
-    uint32_t tot;
-    block_exclusive_scan<uint32_t>(s, &tot, sm);
-    if (threadIdx.x == 0) tile_counts[blockIdx.x] = tot;
+    // (a whole warp; `count` is the tile's)
+    __device__ __forceinline__ uint64_t before(unsigned tile, uint64_t count) const {
+        constexpr unsigned long long VALUE = (1ull << 62) - 1;
+        volatile unsigned long long* s = state;
+        const unsigned lane = lane_id();
+        uint64_t sum = 0;
+        if (n <= 1) return 0;
+        if (known) return known[tile];
+        if (tile > 0) {
+            if (lane == 0) s[tile] = (1ull << 62) | count;
+            int64_t t = (int64_t)tile - 1;
+            for (unsigned spins = 0;;) {
+                const unsigned long long v = t >= (int64_t)lane ? (unsigned long long)s[t - lane] : 2ull << 62;
+                const unsigned ready = __ballot_sync(FULL, v >> 62), whole = __ballot_sync(FULL, v >> 63);
+                const unsigned need = whole ? (whole & (0u - whole)) * 2u - 1u : FULL;  // up to the first sum
+                if ((ready & need) != need) {
+                    if (++spins > spin_limit) {
+                        if (lane == 0) set_status(st, XLB_ERR_TIMEOUT, 21, tile);
+                        break;
+                    }
+                    __nanosleep(20);
+                    continue;
+                }
+                uint64_t x = (need >> lane) & 1u ? v & VALUE : 0ull;
+#pragma unroll
+                for (int d = 16; d; d >>= 1) x += __shfl_xor_sync(FULL, x, d);
+                sum += x;
+                if (whole) break;
+                t -= 32;
+            }
+        }
+        if (lane == 0) s[tile] = (2ull << 62) | (sum + count);
+        return sum;
+    }
+};
+
+// Sums before each tile, by one sweep or (no ticket) left as counts for a scan: with several waves of
+// blocks the waiting costs more than the scan's launch (a probe of 4 M rows: 20 us more), with one less.
+// For a whole warp.
+__device__ __forceinline__ void leave_tile(const SelectTiles& tiles, unsigned tile, uint64_t count, uint64_t* out, uint64_t* total) {
+    if (!tiles.ticket) {
+        if (lane_id() == 0) out[tile] = count;
+        return;
+    }
+    const uint64_t before = tiles.before(tile, count);
+    if (lane_id() == 0) {
+        out[tile] = before;
+        if (tile + 1 == tiles.n) *total = before + count;
+    }
+}
+
+// `zeroed`: sweep_words(tiles) clear words
+inline uint64_t sweep_words(uint64_t tiles) { return tiles + 1; }
+inline SelectTiles sweep_tiles(xlb_ctx* c, uint64_t* zeroed, uint64_t n) {
+    SelectTiles t;
+    t.n = (unsigned)n;
+    t.ticket = (unsigned*)zeroed;
+    t.state = (unsigned long long*)(zeroed + 1);
+    t.st = c->d_status;
+    t.spin_limit = c->lb_spin_limit;
+    return t;
 }
 
 // Each warp owns 256 consecutive rows and walks them 32 at a time, so reads are coalesced and
 // the predicate runs once per row; ballots give the stable position inside the warp.
 template <class Pred, class Emit>
-static __global__ void __launch_bounds__(BLOCK) select_write_k(Pred pred, Emit emit, uint64_t n, const uint64_t* tile_offsets, uint64_t* total) {
+static __global__ void __launch_bounds__(BLOCK) select_write_k(Pred pred, Emit emit, uint64_t n, SelectTiles tiles, uint64_t* total) {
     __shared__ uint32_t sm[33];
+    __shared__ unsigned tile_s;
+    __shared__ uint64_t before_s;
+    const unsigned tile = tiles.take(tile_s);
     constexpr int ROUNDS = SCAN_TILE / BLOCK;  // 8 rounds of 32 rows per warp
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    const uint64_t wbase = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)warp * (32 * ROUNDS);
+    const uint64_t wbase = (uint64_t)tile * SCAN_TILE + (uint64_t)warp * (32 * ROUNDS);
     unsigned flags[ROUNDS];
     uint32_t cnt = 0;
     bool f[ROUNDS];
@@ -315,14 +388,22 @@ static __global__ void __launch_bounds__(BLOCK) select_write_k(Pred pred, Emit e
     uint32_t tot;
     uint32_t ex = block_exclusive_scan<uint32_t>(lane == 0 ? cnt : 0u, &tot, sm);
     ex = __shfl_sync(FULL, ex, 0);
-    uint64_t pos = (tile_offsets ? tile_offsets[blockIdx.x] : 0ull) + ex;
+    uint64_t pos = ex;
+    if (tiles.n > 1) {
+        if (warp == 0) {
+            const uint64_t before = tiles.before(tile, tot);
+            if (lane == 0) before_s = before;
+        }
+        __syncthreads();
+        pos += before_s;
+    }
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         unsigned b = flags[r];
         if ((b >> lane) & 1u) emit(wbase + r * 32 + lane, pos + __popc(b & lanemask_lt()));
         pos += __popc(b);
     }
-    if (!tile_offsets && threadIdx.x == 0) *total = tot;
+    if (tile + 1 == tiles.n && threadIdx.x == 0) *total = (tiles.n > 1 ? before_s : 0ull) + tot;
 }
 
 // Returns the number of selected rows (one host read-back).
@@ -330,25 +411,19 @@ template <class Pred, class Emit>
 uint64_t select(xlb_ctx* c, Pred pred, Emit emit, uint64_t n) {
     if (n == 0) return 0;
     uint64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    Buf total = make_buf(c, 8);
-    unsigned long long h;
-    if (ntiles == 1) {
-        prof_begin(c, "select_write", 0);
-        select_write_k<Pred, Emit><<<1, BLOCK, 0, c->stream>>>(pred, emit, n, nullptr, total->as<uint64_t>());
-        check_launch(c, "select_write");
-        read_words(c, total->p, 1, &h);
-        return h;
+    if (ntiles > 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "selection from %llu rows", (unsigned long long)n);
+    Buf state = make_buf(c, 16 + (ntiles > 1 ? ntiles * 8 : 0));  // total | ticket | one word per tile
+    uint64_t* total = state->as<uint64_t>();
+    SelectTiles tiles;
+    if (ntiles > 1) {
+        CUDA_OK(set_async(c, state->p, 0, 16 + ntiles * 8));
+        tiles = sweep_tiles(c, total + 1, ntiles);
     }
-    Buf counts = make_buf(c, ntiles * 4);
-    Buf offs = make_buf(c, ntiles * 8);
-    prof_begin(c, "select_count", 0);
-    select_count_k<Pred><<<(unsigned)ntiles, BLOCK, 0, c->stream>>>(pred, n, counts->as<uint32_t>());
-    check_launch(c, "select_count");
-    exclusive_scan<LoadU32, uint64_t>(c, LoadU32{counts->as<uint32_t>()}, ntiles, offs->as<uint64_t>(), total->as<uint64_t>());
     prof_begin(c, "select_write", 0);
-    select_write_k<Pred, Emit><<<(unsigned)ntiles, BLOCK, 0, c->stream>>>(pred, emit, n, offs->as<uint64_t>(), nullptr);
+    select_write_k<Pred, Emit><<<(unsigned)ntiles, BLOCK, 0, c->stream>>>(pred, emit, n, tiles, total);
     check_launch(c, "select_write");
-    read_words(c, total->p, 1, &h);
+    unsigned long long h;
+    read_words(c, total, 1, &h);
     return h;
 }
 
@@ -839,6 +914,7 @@ static __global__ void __launch_bounds__(SORT_THREADS, XLB_SORT_MINB) radix_scat
                 *mine = cnt | LB_FLAG_INC;
             } else {
                 *mine = cnt | LB_FLAG_AGG;
+                // (asking eight earlier tiles at a time was slower: 70 us a pass over 4 M rows against 58)
                 int64_t t = (int64_t)tile - 1;
                 unsigned spins = 0;
                 while (t >= 0) {

@@ -54,12 +54,14 @@ __device__ __forceinline__ uint64_t claim(const KeyCols& keys, unsigned int* rep
 __global__ void __launch_bounds__(BLOCK) exists_build_k(KeyCols keys, uint64_t n, unsigned int* __restrict__ rep, uint64_t mask, DevStatus* st) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) claim(keys, rep, mask, i, st);
 }
-// One bit per probe row (has a match == want), and the rows selected per tile of SCAN_TILE.
+// One bit per probe row (has a match == want), and for each tile of SCAN_TILE rows how many were selected before it.
 constexpr int QT_ROUNDS = SCAN_TILE / BLOCK;
 __global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t n, KeyCols keys, const unsigned int* __restrict__ rep, uint64_t mask, bool want,
-                                                       unsigned int* __restrict__ bits, uint32_t* __restrict__ tile_counts) {
+                                                       unsigned int* __restrict__ bits, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total) {
     __shared__ uint32_t sm[33];
-    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS;  // a warp's rows side by side
+    __shared__ unsigned tile_s;
+    const unsigned tile = tiles.take(tile_s);
+    const uint64_t base = (uint64_t)tile * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS;  // a warp's rows side by side
     uint32_t cnt = 0;
     uint64_t key[QT_ROUNDS];
     unsigned cur[QT_ROUNDS];
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t 
     }
     uint32_t tot;
     block_exclusive_scan<uint32_t>(lane_id() == 0 ? cnt : 0u, &tot, sm);
-    if (threadIdx.x == 0) tile_counts[blockIdx.x] = tot;
+    if (threadIdx.x < 32) leave_tile(tiles, tile, tot, tile_offs, total);
 }
 // The selected rows, all columns, in order.
 __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned int* __restrict__ bits, uint64_t n, const uint64_t* __restrict__ tile_offs) {
@@ -130,19 +132,59 @@ __global__ void __launch_bounds__(BLOCK) group_count_k(KeyCols keys, uint64_t n,
         place[i] = make_uint2((unsigned)h, atomicAdd(&count[h], 1u));
     }
 }
-__global__ void __launch_bounds__(BLOCK) group_fill_k(const uint2* __restrict__ place, uint64_t n, const uint32_t* __restrict__ start, uint32_t* __restrict__ rows) {
-    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
-        const uint2 p = place[i];
-        rows[start[p.x] + p.y] = (uint32_t)i;
+// A slot's entry: its key, where its rows lie (start << 32) and how many they are.  Groups may lie in any
+// order: a block takes the room for its slots' rows with one atomic.
+__global__ void __launch_bounds__(BLOCK) group_start_k(KeyCols keys, const unsigned int* __restrict__ rep, const unsigned int* __restrict__ count, uint64_t cap, ulonglong2* __restrict__ table,
+                                                      unsigned int* __restrict__ used) {
+    __shared__ uint32_t sm[33], room_s;
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + threadIdx.x;
+    unsigned len[SCAN_IPT], mine = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; ++k) {
+        const uint64_t h = base + (uint64_t)k * BLOCK;
+        len[k] = h < cap ? count[h] : 0u;
+        mine += len[k];
+    }
+    uint32_t tot;
+    uint32_t at = block_exclusive_scan<uint32_t>(mine, &tot, sm);
+    if (threadIdx.x == 0) room_s = tot ? atomicAdd(used, tot) : 0u;
+    __syncthreads();
+    at += room_s;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; ++k) {
+        const uint64_t h = base + (uint64_t)k * BLOCK;
+        if (h >= cap) break;
+        table[h] = len[k] ? make_ulonglong2(keys(rep[h] - 1), ((unsigned long long)at << 32) | len[k]) : make_ulonglong2(0, 0);
+        at += len[k];
     }
 }
-__global__ void __launch_bounds__(BLOCK) group_order_k(KeyCols keys, const unsigned int* __restrict__ rep, const unsigned int* __restrict__ count, const uint32_t* __restrict__ start,
-                                                      uint64_t cap, uint32_t* __restrict__ rows, ulonglong2* __restrict__ table, unsigned int* __restrict__ too_long) {
+__global__ void __launch_bounds__(BLOCK) group_fill_k(const uint2* __restrict__ place, uint64_t n, const ulonglong2* __restrict__ table, uint32_t* __restrict__ rows) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
+        const uint2 p = place[i];
+        rows[(uint32_t)(table[p.x].y >> 32) + p.y] = (uint32_t)i;
+    }
+}
+__global__ void __launch_bounds__(BLOCK) group_order_k(const unsigned int* __restrict__ count, const ulonglong2* __restrict__ table, uint64_t cap, uint32_t* __restrict__ rows,
+                                                      unsigned int* __restrict__ too_long) {
     for (uint64_t h = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; h < cap; h += (uint64_t)gridDim.x * BLOCK) {
-        const unsigned len = count[h], at = start[h];
-        table[h] = len ? make_ulonglong2(keys(rep[h] - 1), ((unsigned long long)at << 32) | len) : make_ulonglong2(0, 0);
+        const unsigned len = count[h];
+        if (len < 2) continue;
         if (len > JOIN_GROUP_MAX) {
             *too_long = 1;
+            continue;
+        }
+        const unsigned at = (unsigned)(table[h].y >> 32);
+        if (len <= 4) {  // most groups: read at once, placed by rank (row numbers differ)
+            uint32_t v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = k < (int)len ? rows[at + k] : 0xFFFFFFFFu;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                unsigned rank = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) rank += q < (int)len && v[q] < v[k];
+                if (k < (int)len) rows[at + rank] = v[k];
+            }
             continue;
         }
         for (unsigned a = 1; a < len; ++a) {  // insertion sort in place
@@ -156,25 +198,58 @@ __global__ void __launch_bounds__(BLOCK) group_order_k(KeyCols keys, const unsig
         }
     }
 }
-__global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n, const ulonglong2* __restrict__ table, uint64_t mask, uint64_t* __restrict__ match) {
-    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
-        const uint64_t key = probe(i);
-        uint64_t h = mix64(key) & mask, m = 0;
-        for (uint64_t p = 0; p <= mask; ++p) {  // bounded by the table size
-            const ulonglong2 s = __ldg(&table[h]);
-            if (s.y == 0) break;
-            if (s.x == key) {
-                m = s.y;
-                break;
-            }
+// What each probe row meets (start << 32 | rows) and how many outputs come before it: in its tile, and before the tile.
+__global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n, const ulonglong2* __restrict__ table, uint64_t mask, uint64_t* __restrict__ match,
+                                                     uint32_t* __restrict__ in_tile, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total) {
+    __shared__ uint64_t sm[33];
+    __shared__ unsigned tile_s;
+    const unsigned tile = tiles.take(tile_s), lane = lane_id();
+    const uint64_t base = (uint64_t)tile * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS + lane;  // a warp's rows side by side
+    uint64_t key[QT_ROUNDS];
+    ulonglong2 m[QT_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) key[r] = base + r * 32 < n ? probe(base + r * 32) : 0;
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) m[r] = base + r * 32 < n ? __ldg(&table[mix64(key[r]) & mask]) : make_ulonglong2(0, 0);
+    uint64_t mine = 0;
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) {
+        uint64_t h = mix64(key[r]) & mask;
+        for (uint64_t p = 0; p < mask && m[r].y && m[r].x != key[r]; ++p) {  // bounded by the table size
             h = (h + 1) & mask;
+            m[r] = __ldg(&table[h]);
         }
-        match[i] = m;
+        if (m[r].x != key[r]) m[r].y = 0;
+        mine += (uint32_t)m[r].y;
+    }
+    for (int d = 16; d; d >>= 1) mine += __shfl_xor_sync(FULL, mine, d);
+    uint64_t tot;
+    uint64_t at = block_exclusive_scan<uint64_t>(lane == 0 ? mine : 0ull, &tot, sm);
+    if (threadIdx.x < 32) leave_tile(tiles, tile, tot, tile_offs, total);
+    at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r) {
+        uint32_t run = (uint32_t)m[r].y;  // (32 groups of at most JOIN_GROUP_MAX rows; longer ones are not used)
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, run, d);
+            if (lane >= (unsigned)d) run += v;
+        }
+        if (base + r * 32 < n) {
+            match[base + r * 32] = m[r].y;
+            in_tile[base + r * 32] = (uint32_t)at + run - (uint32_t)m[r].y;
+        }
+        at += __shfl_sync(FULL, run, 31);
     }
 }
+struct OutputsBefore {
+    const uint64_t* tile;
+    const uint32_t* in_tile;
+    __device__ __forceinline__ uint64_t operator[](uint64_t row) const { return tile[row / SCAN_TILE] + in_tile[row]; }
+};
 // Load-balanced output of an inner join (the scheme of expand_k), all columns of both sides written
 // at once: the pairs of row numbers never touch memory.
-__global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict__ match, const uint64_t* __restrict__ off, uint64_t nrows, uint64_t total, const uint32_t* __restrict__ rows,
+__global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict__ match, const OutputsBefore off, uint64_t nrows, uint64_t total, const uint32_t* __restrict__ rows,
                                                     Cols cols) {
     __shared__ unsigned rel[EX_TILE + 2];
     __shared__ uint64_t row_s[2];
@@ -255,9 +330,12 @@ __global__ void __launch_bounds__(BLOCK) group_rows_k(GroupKey key, uint64_t n, 
         __syncthreads();
     }
 }
-__global__ void __launch_bounds__(BLOCK) group_tiles_k(const unsigned int* __restrict__ count, uint64_t domain, uint32_t* __restrict__ tile_groups, unsigned long long* __restrict__ longest) {
+__global__ void __launch_bounds__(BLOCK) group_tiles_k(const unsigned int* __restrict__ count, uint64_t domain, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total,
+                                                      unsigned long long* __restrict__ longest) {
     __shared__ uint32_t sm[33];
-    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
+    __shared__ unsigned tile_s;
+    const unsigned tile = tiles.take(tile_s);
+    const uint64_t base = (uint64_t)tile * SCAN_TILE;
     uint32_t groups = 0, most = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_IPT; ++k) {
@@ -270,7 +348,7 @@ __global__ void __launch_bounds__(BLOCK) group_tiles_k(const unsigned int* __res
     if (lane_id() == 0 && most) atomicMax(longest, (unsigned long long)most);
     uint32_t tot;
     block_exclusive_scan<uint32_t>(groups, &tot, sm);
-    if (threadIdx.x == 0) tile_groups[blockIdx.x] = tot;
+    if (threadIdx.x < 32) leave_tile(tiles, tile, tot, tile_offs, total);
 }
 struct Aggs {
     const void* val[XLB_MAX_ARITY];
@@ -340,28 +418,52 @@ void add_columns(xlb_ctx* c, xlb_rel* out, Cols& cols, const xlb_rel* from, uint
     }
 }
 
+// The sums before each tile of a kernel that calls leave_tile: the kernel's own doing, or by a scan after it.
+struct Sweep {
+    SelectTiles tiles;
+    uint64_t* leave_at;
+    Sweep(xlb_ctx* c_, uint64_t n_, uint64_t* zeroed, uint64_t* offs_, uint64_t* total_) : leave_at(offs_), c(c_), n(n_), offs(offs_), total(total_) {
+        if (n <= 4ull * c->sm_count) tiles = sweep_tiles(c, zeroed, n);  // (four blocks of 256 threads and more fit an SM)
+        else {
+            tiles.n = (unsigned)n;
+            counts = make_buf(c, n * 8);
+            leave_at = counts->as<uint64_t>();
+        }
+    }
+    void finish() {
+        if (counts) exclusive_scan<LoadU64, uint64_t>(c, LoadU64{counts->as<uint64_t>()}, n, offs, total);
+    }
+
+   private:
+    xlb_ctx* c;
+    uint64_t n, *offs, *total;
+    Buf counts;
+};
+
 }  // namespace
 
 xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, bool want) {
     if (r->rows >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)r->rows);
     uint64_t cap = 1024;
     while (cap < 2 * r->rows) cap <<= 1;
-    Buf rep = make_buf(c, cap * 4);
-    CUDA_OK(set_async(c, rep->p, 0, cap * 4));
+    const uint64_t n = l->rows, tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+    Buf rep = make_buf(c, cap * 4 + sweep_words(tiles) * 8);
+    CUDA_OK(set_async(c, rep->p, 0, cap * 4 + sweep_words(tiles) * 8));
     const KeyCols build = key_cols(r, rk, nk), probe = key_cols(l, lk, nk);
     if (r->rows) {
         prof_begin(c, "hash_insert", 0);
         exists_build_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(build, r->rows, rep->as<unsigned int>(), cap - 1, c->d_status);
         check_launch(c, "hash_insert");
     }
-    const uint64_t n = l->rows, tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    Buf bits = make_buf(c, (n + 31) / 32 * 4), counts = make_buf(c, tiles * 4), offs = make_buf(c, tiles * 8), total = make_buf(c, 8);
+    Buf bits = make_buf(c, (n + 31) / 32 * 4), offs = make_buf(c, tiles * 8 + 8);
+    uint64_t* total = offs->as<uint64_t>() + tiles;
+    Sweep sweep(c, tiles, rep->as<uint64_t>() + cap / 2, offs->as<uint64_t>(), total);
     prof_begin(c, "hash_probe", n * 12ull);
-    exists_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, n, build, rep->as<unsigned int>(), cap - 1, want, bits->as<unsigned int>(), counts->as<uint32_t>());
+    exists_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, n, build, rep->as<unsigned int>(), cap - 1, want, bits->as<unsigned int>(), sweep.tiles, sweep.leave_at, total);
     check_launch(c, "hash_probe");
-    exclusive_scan<LoadU32, uint64_t>(c, LoadU32{counts->as<uint32_t>()}, tiles, offs->as<uint64_t>(), total->as<uint64_t>());
+    sweep.finish();
     unsigned long long m;
-    read_words(c, total->p, 1, &m);
+    read_words(c, total, 1, &m);
     std::unique_ptr<xlb_rel> o(new xlb_rel);
     o->ctx = c;
     o->schema = l->schema;
@@ -382,28 +484,31 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     uint64_t cap = 1024;
     while (cap < 2 * n) cap <<= 1;
     const KeyCols build = key_cols(r, rk, nk), probe = key_cols(l, lk, nk);
-    Buf slots = make_buf(c, cap * 8), start = make_buf(c, cap * 4), place = make_buf(c, n * 8), rows = make_buf(c, n * 4), table = make_buf(c, cap * 16), words = make_buf(c, 24);
+    const uint64_t tiles = (l->rows + SCAN_TILE - 1) / SCAN_TILE, clear = cap * 8 + (3 + sweep_words(tiles)) * 8;
+    Buf slots = make_buf(c, clear), place = make_buf(c, n * 8), rows = make_buf(c, n * 4), table = make_buf(c, cap * 16);
     unsigned int *rep = slots->as<unsigned int>(), *count = rep + cap;
-    CUDA_OK(set_async(c, slots->p, 0, cap * 8));
-    CUDA_OK(set_async(c, words->p, 0, 24));  // [0] outputs, [1] a group is too long, [2] rows grouped
+    uint64_t* words = slots->as<uint64_t>() + cap;  // [0] outputs, [1] a group is too long, [2] room taken for groups, then the sweep's
+    CUDA_OK(set_async(c, slots->p, 0, clear));
     prof_begin(c, "hash_insert", n * 8ull);
     group_count_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, rep, count, cap - 1, place->as<uint2>(), c->d_status);
     check_launch(c, "hash_insert");
-    exclusive_scan<LoadU32, uint32_t>(c, LoadU32{count}, cap, start->as<uint32_t>(), (uint32_t*)(words->as<uint64_t>() + 2));
+    prof_begin(c, "group_start", cap * 24ull);
+    group_start_k<<<(unsigned)((cap + SCAN_TILE - 1) / SCAN_TILE), BLOCK, 0, c->stream>>>(build, rep, count, cap, table->as<ulonglong2>(), (unsigned int*)(words + 2));
+    check_launch(c, "group_start");
     prof_begin(c, "group_fill", n * 16ull);
-    group_fill_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(place->as<uint2>(), n, start->as<uint32_t>(), rows->as<uint32_t>());
+    group_fill_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(place->as<uint2>(), n, table->as<ulonglong2>(), rows->as<uint32_t>());
     check_launch(c, "group_fill");
-    prof_begin(c, "group_order", cap * 24ull);
-    group_order_k<<<grid_for(c, cap), BLOCK, 0, c->stream>>>(build, rep, count, start->as<uint32_t>(), cap, rows->as<uint32_t>(), table->as<ulonglong2>(),
-                                                            (unsigned int*)(words->as<uint64_t>() + 1));
+    prof_begin(c, "group_order", cap * 4ull);
+    group_order_k<<<grid_for(c, cap), BLOCK, 0, c->stream>>>(count, table->as<ulonglong2>(), cap, rows->as<uint32_t>(), (unsigned int*)(words + 1));
     check_launch(c, "group_order");
-    Buf match = make_buf(c, l->rows * 8), off = make_buf(c, l->rows * 8);
+    Buf match = make_buf(c, l->rows * 8), in_tile = make_buf(c, l->rows * 4), offs = make_buf(c, tiles * 8);
+    Sweep sweep(c, tiles, words + 3, offs->as<uint64_t>(), words);
     prof_begin(c, "hash_probe", l->rows * 32ull);
-    join_probe_k<<<grid_for(c, l->rows), BLOCK, 0, c->stream>>>(probe, l->rows, table->as<ulonglong2>(), cap - 1, match->as<uint64_t>());
+    join_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, l->rows, table->as<ulonglong2>(), cap - 1, match->as<uint64_t>(), in_tile->as<uint32_t>(), sweep.tiles, sweep.leave_at, words);
     check_launch(c, "hash_probe");
-    exclusive_scan<LoadLow32, uint64_t>(c, LoadLow32{match->as<uint64_t>()}, l->rows, off->as<uint64_t>(), words->as<uint64_t>());
+    sweep.finish();
     unsigned long long w[2];
-    read_words(c, words->p, 2, w);
+    read_words(c, words, 2, w);
     if (w[1]) return nullptr;
     std::unique_ptr<xlb_rel> o(new xlb_rel);
     o->ctx = c;
@@ -415,7 +520,7 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     add_columns(c, o.get(), cols, r, w[0]);
     if (w[0]) {
         prof_begin(c, "join_emit", 0);
-        join_emit_k<<<(unsigned)((w[0] + EX_TILE - 1) / EX_TILE), BLOCK, 0, c->stream>>>(match->as<uint64_t>(), off->as<uint64_t>(), l->rows, w[0], rows->as<uint32_t>(), cols);
+        join_emit_k<<<(unsigned)((w[0] + EX_TILE - 1) / EX_TILE), BLOCK, 0, c->stream>>>(match->as<uint64_t>(), OutputsBefore{offs->as<uint64_t>(), in_tile->as<uint32_t>()}, l->rows, w[0], rows->as<uint32_t>(), cols);
         check_launch(c, "join_emit");
     }
     return o.release();
@@ -444,15 +549,17 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
     }
     if (bits > GROUP_BITS_MAX || (1ull << bits) > std::max<uint64_t>(4 * n, GROUP_DOMAIN_FREE)) return nullptr;
     const uint64_t domain = 1ull << bits, tiles = (domain + SCAN_TILE - 1) / SCAN_TILE;
-    Buf count = make_buf(c, domain * 4), tile_groups = make_buf(c, tiles * 4), offs = make_buf(c, tiles * 8);
-    CUDA_OK(set_async(c, count->p, 0, domain * 4));
+    const uint64_t clear = (domain * 4 + 7) / 8 * 8 + sweep_words(tiles) * 8;
+    Buf count = make_buf(c, clear), offs = make_buf(c, tiles * 8);
+    CUDA_OK(set_async(c, count->p, 0, clear));
     prof_begin(c, "group_rows", 0);
     group_rows_k<<<grid_for(c, n, DX_TILE), BLOCK, 0, c->stream>>>(key, n, count->as<unsigned int>());
     check_launch(c, "group_rows");
+    Sweep sweep(c, tiles, count->as<uint64_t>() + (domain * 4 + 7) / 8, offs->as<uint64_t>(), words->as<uint64_t>() + 1);
     prof_begin(c, "group_tiles", domain * 4ull);
-    group_tiles_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(count->as<unsigned int>(), domain, tile_groups->as<uint32_t>(), words->as<unsigned long long>() + 2);
+    group_tiles_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(count->as<unsigned int>(), domain, sweep.tiles, sweep.leave_at, words->as<uint64_t>() + 1, words->as<unsigned long long>() + 2);
     check_launch(c, "group_tiles");
-    exclusive_scan<LoadU32, uint64_t>(c, LoadU32{tile_groups->as<uint32_t>()}, tiles, offs->as<uint64_t>(), words->as<uint64_t>() + 1);
+    sweep.finish();
     read_words(c, words->as<uint64_t>() + 1, 2, w);
     const uint64_t m = w[0];
     uint32_t tables = 0;

@@ -74,24 +74,37 @@ struct OutCols {
     }
 };
 
-// Least image and the complement of the greatest one, per key column (from words of all ones).
+// Least image and the complement of the greatest one, per key column (from words of all ones).  A few
+// blocks per SM with several loads in flight each: one atomic per block and word is all that meets.
+template <int WIDTH>
+__device__ __forceinline__ void range_of(const KeyPart& p, uint64_t n, uint64_t& a, uint64_t& b) {
+    const uint64_t step = (uint64_t)gridDim.x * BLOCK;
+#pragma unroll 8
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += step) {
+        const uint64_t v = image_of(p.col, WIDTH, p.kind, i);
+        a = min(a, v);
+        b = min(b, ~v);
+    }
+}
 __global__ void __launch_bounds__(BLOCK) key_range_k(const KeyWord w, uint64_t n, unsigned long long* __restrict__ least) {
-    const uint64_t first = (uint64_t)blockIdx.x * BLOCK + threadIdx.x, step = (uint64_t)gridDim.x * BLOCK;
+    __shared__ unsigned long long s[2];
     for (int k = 0; k < w.n; ++k) {
         uint64_t a = ~0ull, b = ~0ull;
-        for (uint64_t i = first; i < n; i += step) {
-            const uint64_t v = image_of(w.p[k].col, w.p[k].width, w.p[k].kind, i);
-            a = min(a, v);
-            b = min(b, ~v);
-        }
+        if (threadIdx.x < 2) s[threadIdx.x] = ~0ull;
+        if (w.p[k].width == 4) range_of<4>(w.p[k], n, a, b);
+        else if (w.p[k].width == 8) range_of<8>(w.p[k], n, a, b);
+        else range_of<1>(w.p[k], n, a, b);
         for (int d = 16; d; d >>= 1) {
             a = min(a, (uint64_t)__shfl_xor_sync(FULL, a, d));
             b = min(b, (uint64_t)__shfl_xor_sync(FULL, b, d));
         }
+        __syncthreads();
         if (lane_id() == 0) {
-            atomicMin(&least[2 * k], (unsigned long long)a);
-            atomicMin(&least[2 * k + 1], (unsigned long long)b);
+            atomicMin(&s[0], (unsigned long long)a);
+            atomicMin(&s[1], (unsigned long long)b);
         }
+        __syncthreads();
+        if (threadIdx.x < 2) atomicMin(&least[2 * k + threadIdx.x], s[threadIdx.x]);
     }
 }
 __global__ void __launch_bounds__(BLOCK) key_word_k(const KeyWord w, const uint32_t* __restrict__ rows, uint64_t* __restrict__ out, uint64_t n) {
@@ -173,7 +186,7 @@ void order_rows(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_t nk,
         Buf least = make_buf(c, 16 * XLB_MAX_ARITY);
         CUDA_OK(set_async(c, least->p, 0xFF, 16 * XLB_MAX_ARITY));
         prof_begin(c, "key_range", n * 8ull * all.n);
-        key_range_k<<<grid_for(c, n, BLOCK * 8), BLOCK, 0, c->stream>>>(all, n, least->as<unsigned long long>());
+        key_range_k<<<std::min(grid_for(c, n, BLOCK * 8), 6u * c->sm_count), BLOCK, 0, c->stream>>>(all, n, least->as<unsigned long long>());
         check_launch(c, "key_range");
         unsigned long long range[2 * XLB_MAX_ARITY];
         read_words(c, least->p, 2 * all.n, range);

@@ -14,6 +14,21 @@
 
 using namespace xk;
 
+template <class Pred>
+static __global__ void __launch_bounds__(BLOCK) select_count_k(Pred pred, uint64_t n, uint32_t* tile_counts) {
+    __shared__ uint32_t sm[33];
+    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
+    uint32_t s = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; ++k) {
+        uint64_t i = base + (uint64_t)k * BLOCK + threadIdx.x;
+        if (i < n && pred(i)) s++;
+    }
+    uint32_t tot;
+    block_exclusive_scan<uint32_t>(s, &tot, sm);
+    if (threadIdx.x == 0) tile_counts[blockIdx.x] = tot;
+}
+
 // Largest input the fixed scratch serves: 2^26 keys (512 MiB of keys).
 static constexpr uint64_t STATIC_MAX_KEYS = 1ull << 26;
 static constexpr uint64_t STATIC_MAX_TILES = STATIC_MAX_KEYS / SCAN_TILE;                    // 32768 tiles of 2048 keys
@@ -86,7 +101,7 @@ extern "C" xlb_status xlb_dedup_sorted_u64_static(const uint64_t* d_sorted, uint
         EmitKey emit{d_sorted, d_unique};
         uint64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
         if (ntiles == 1) {
-            select_write_k<PredHead, EmitKey><<<1, BLOCK, 0, stream>>>(pred, emit, n, nullptr, d_count);
+            select_write_k<PredHead, EmitKey><<<1, BLOCK, 0, stream>>>(pred, emit, n, SelectTiles(), d_count);
         } else {
             // every scratch word that is read below is written first by these launches, so nothing
             // left behind by an earlier call is ever observed
@@ -100,9 +115,10 @@ extern "C" xlb_status xlb_dedup_sorted_u64_static(const uint64_t* d_sorted, uint
                 scan_spine_k<uint64_t><<<1, 1024, 0, stream>>>(spine, stiles, total);
                 scan_apply_k<LoadU32, uint64_t><<<(unsigned)stiles, BLOCK, 0, stream>>>(load, ntiles, spine, offs, nullptr);
             }
-            select_write_k<PredHead, EmitKey><<<(unsigned)ntiles, BLOCK, 0, stream>>>(pred, emit, n, offs, nullptr);
-            e = cudaMemcpyAsync(d_count, total, 8, cudaMemcpyDeviceToDevice, stream);
-            if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "cudaMemcpyAsync(count)", e);
+            SelectTiles tiles;
+            tiles.n = (unsigned)ntiles;
+            tiles.known = offs;
+            select_write_k<PredHead, EmitKey><<<(unsigned)ntiles, BLOCK, 0, stream>>>(pred, emit, n, tiles, d_count);
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "kernel launch", e);
