@@ -159,3 +159,48 @@ def test_thinly_spread_values(bits, values, monkeypatch):
     if values % 2:
         edge = [np.append(edge[0], ids[-1]), np.append(edge[1], ids[0])]
     both(programs.transitive_closure(), {"edge": edge}, "reach", monkeypatch)
+
+
+def _rows_graph(kind):
+    rng = np.random.default_rng(3)
+    if kind.startswith("values"):  # bits of the second column: a word, two words, 16 and 17 bits
+        n = int(kind[6:])
+        m = min(2 * n, 3000)
+        return [rng.integers(0, n, m, dtype=np.uint32), np.concatenate([rng.integers(0, n, m - 1, dtype=np.uint32), [n - 1]]).astype(np.uint32)]
+    if kind.startswith("front"):  # chains that run into a node with so many successors, which come together again
+        k = int(kind[5:])
+        leaves = np.arange(400, 400 + k, dtype=np.uint32)
+        a = [np.arange(50), np.full(k, 50), leaves, np.arange(100, 399)]
+        b = [np.arange(1, 51), leaves, np.full(k, 60), np.arange(101, 400)]
+        return [np.concatenate(x).astype(np.uint32) for x in (a, b)]
+    if kind == "all_wide":  # every row outgrows its queue
+        leaves = np.arange(4000, 20600, dtype=np.uint32)
+        src = np.arange(1500, dtype=np.uint32)
+        return [np.concatenate([src, np.full(16600, 3500)]).astype(np.uint32), np.concatenate([np.full(1500, 3500), leaves]).astype(np.uint32)]
+    n = 300  # every node next to every other: long rows
+    return [np.repeat(np.arange(n, dtype=np.uint32), n), np.tile(np.arange(n, dtype=np.uint32), n)]
+
+
+@pytest.mark.parametrize("kind", ["values31", "values32", "values33", "values65536", "values65537", "front16383", "front16384", "front16385", "all_wide", "dense"])
+def test_rows_apart(kind, monkeypatch):
+    edge = _rows_graph(kind)
+    got, _, _ = both(programs.transitive_closure(), {"edge": edge}, "reach", monkeypatch)
+    if kind not in ("dense", "all_wide"):
+        want, _ = O.run_program(programs.transitive_closure(), {"edge": edge}, ["reach"])
+        for g, w in zip(got, want["reach"]):
+            assert np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("nodes", [40, 1500])
+def test_rows_apart_two_rules(nodes, monkeypatch):
+    # p(X,Z) :- p(X,Y), a(Y,Z).  p(X,Z) :- p(X,Y), b(Y,Z).
+    ids = {"a": 0, "b": 1, "p": 2}
+    rules = [CompiledRule("p", Scan(0), U2)] + [CompiledRule("p", Project(Join(Scan(2), Scan(r), [1], [0]), [0, 3]), U2) for r in (0, 1)]
+    rng = np.random.default_rng(nodes)
+    pairs = lambda m: [rng.integers(0, nodes, m, dtype=np.uint32), rng.integers(0, nodes, m, dtype=np.uint32)]  # noqa: E731
+    both(ExecutionPlan([Scc(0, True, rules)], ids), {"a": pairs(nodes), "b": pairs(nodes // 2)}, "p", monkeypatch)
+
+
+def test_log_grows_left_linear(monkeypatch):
+    got, _, _ = both(programs.transitive_closure_left_linear(), {"edge": list(workloads.uniform_digraph())}, "reach", monkeypatch, memory_budget_bytes=200 << 20)
+    assert len(got[0]) > 1 << 21

@@ -106,6 +106,9 @@ struct Ctl {
     unsigned solo_phase, solo_check, pad;
     unsigned long long solo_start, solo_end, solo_iterations, solo_candidates;
     Slot slot[3];
+    // rows evaluated one warp each: what they came to, and what was given up (read by the host)
+    unsigned long long rows_tuples, rows_candidates, rows_levels, rows_left, rows_given_up, rows_seeds;
+    unsigned rows_ticket, rows_idle;
 };
 struct Heavy {
     uint64_t row;
@@ -956,6 +959,343 @@ __global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
     c->phase = c->iterations >= max_iterations ? PH_DONE : square ? PH_FULL : PH_ROWS;
 }
 
+// ---- rules that keep a column: a block (one warp or a few) for each value of it
+// Where every rule hands the head's first column on and joins on the second (a closure: reach(x, z) :-
+// reach(x, y), edge(y, z)), what is derived for one x depends on nothing derived for another.  A
+// block takes an x, holds its row of the head's bitmap and the frontier of its search in shared memory and
+// goes level by level to the end: no barrier between blocks, no atomics and no log in global memory.
+// Its levels are the iterations of the loop, and its candidates the loop's.  Latency of one instruction
+// after the other bounds it, not memory: hence several warps a row where rows are few, four outputs a
+// lane in flight, and a path of its own for a frontier of one value.  (Loop -> this, B200: chain of 1500
+// nodes 3279 -> 498 us, banded DAG of 2^14 nodes 961 -> 472, 2000 nodes of degree 5 276 -> 113, four
+// blocks of 128 nodes 181 -> 66; one warp a row with one output a lane in flight: 1089, 1238, 185, 698.)
+//   What a block is too slow for is left to the loop: a row is given up when its frontier outgrows its
+// queue, or when it is long and most blocks have nothing left to do; its seeds are all that remains
+// of it.  Once a quarter of the blocks have given one up, the rest of the rows are not tried.
+constexpr int RW_UNROLL = 4;
+constexpr int RW_BITS_MIN = 5, RW_BITS_MAX = 16;  // of the second column: a row is whole words, a value 16 bits
+constexpr unsigned RW_QUEUE = 16384;              // values the frontier of a row may hold (and the row's seeds)
+constexpr unsigned RW_LONG = 16384;               // candidates of a warp (some 50 us) from which a row may be given up
+constexpr unsigned RW_LIST = 64;                  // a value with so many matches is a warp's work by itself
+struct RowsShape {
+    unsigned rows, words;  // rows of the bitmap, words of each
+    unsigned queue;        // entries, a power of two
+    unsigned chunk;        // rows taken at a time
+};
+constexpr unsigned rows_queue(int bits) { return 1u << bits < RW_QUEUE ? 1u << bits : RW_QUEUE; }
+constexpr unsigned rows_bytes(int bits) { return (1u << bits) / 8 + rows_queue(bits) * 2; }
+struct RowsShared {
+    unsigned head, tail;  // of the queue's ring; the tail counts the row's tuples
+    unsigned failed, next;
+    unsigned long long level, cand, tuples, cands, levels;
+};
+template <int W>
+struct RowsWarp {
+    unsigned* seen;
+    unsigned short* queue;
+    uint2* match;  // of the warp's 32 values: start, length
+    RowsShared* sh;
+    unsigned mask, head;
+
+    // New values among z join the row and the queue.
+    template <int N>
+    __device__ __forceinline__ void offer(const Out& o, const uint32_t (&z)[N], bool (&on)[N]) {
+        unsigned word[N];
+        bool any = false, bad = false;
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            bad |= on[u] && z[u] >> o.lo_bits;
+            on[u] = on[u] && !(z[u] >> o.lo_bits);
+            word[u] = on[u] ? seen[z[u] >> 5] : ~0u;  // (a look first: most are known, and many lanes share a word)
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            on[u] = on[u] && !((word[u] >> (z[u] & 31)) & 1u);
+            any |= on[u];
+        }
+        if (bad) set_status(o.st, XLB_ERR_CAPACITY, 22, z[0]);  // outside the domain the host derived
+        if (!__any_sync(FULL, any)) return;
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+            if (on[u]) word[u] = atomicOr(&seen[z[u] >> 5], 1u << (z[u] & 31));
+        unsigned b[N], count = 0;
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            on[u] = on[u] && !((word[u] >> (z[u] & 31)) & 1u);
+            b[u] = __ballot_sync(FULL, on[u]);
+            count += __popc(b[u]);
+        }
+        if (!count) return;
+        unsigned to = 0;
+        if (lane_id() == 0) to = atomicAdd(&sh->tail, count);
+        to = __shfl_sync(FULL, to, 0);
+        if (to + count - head > mask + 1) {  // (the level at hand is still in the ring)
+            if (lane_id() == 0) sh->failed = 1;
+            return;
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            if (on[u]) queue[(to + __popc(b[u] & lanemask_lt())) & mask] = (unsigned short)z[u];
+            to += __popc(b[u]);
+        }
+    }
+    // The matches [at, at + len) of one value.
+    __device__ __forceinline__ void list(const Out& o, const Ix& ix, uint32_t at, uint32_t len) {
+        for (uint32_t base = 0; base < len; base += 32 * RW_UNROLL) {
+            uint32_t z[RW_UNROLL];
+            bool on[RW_UNROLL];
+#pragma unroll
+            for (int u = 0; u < RW_UNROLL; ++u) {
+                const uint32_t t = base + u * 32 + lane_id();
+                on[u] = t < len;
+                z[u] = other_of(ix, at + (on[u] ? t : 0u));
+            }
+            offer(o, z, on);
+        }
+    }
+    // `total` matches of the lanes' values, dealt out evenly; lanes below m have some, lane's first is output `before`.
+    template <int N>
+    __device__ __forceinline__ void dealt(const Out& o, const Ix& ix, uint32_t from, uint32_t total, unsigned m, uint32_t before, uint32_t shift) {
+        const unsigned lane = lane_id();
+        uint32_t z[N];
+        bool on[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const uint32_t base = from + u * 32, t = base + lane, d = before - base;
+            const unsigned starts = __reduce_or_sync(FULL, lane < m && before >= base && d < 32 ? 1u << d : 0u);
+            // the last lane whose outputs start at or before t
+            const unsigned owner = __popc(__ballot_sync(FULL, lane < m && before < base)) + __popc(starts & (lanemask_lt() | (1u << lane))) - 1;
+            const uint32_t at = __shfl_sync(FULL, shift, owner) + t;
+            on[u] = t < total;
+            z[u] = other_of(ix, on[u] ? at : 0u);
+        }
+        offer(o, z, on);
+    }
+    // All matches of up to 32 values by one rule; their number.
+    __device__ __forceinline__ uint32_t expand(const Out& o, const Ix& ix, bool on, unsigned y) {
+        const unsigned lane = lane_id();
+        uint32_t start = 0, len = 0;
+        if (on) find(ix, y, start, len);
+        uint32_t all = 0;
+        for (unsigned far = __ballot_sync(FULL, len >= RW_LIST); far; far &= far - 1) {
+            const uint32_t n = __shfl_sync(FULL, len, __ffs(far) - 1);
+            list(o, ix, __shfl_sync(FULL, start, __ffs(far) - 1), n);
+            all += n;
+        }
+        if (len >= RW_LIST) len = 0;
+        const unsigned some = __ballot_sync(FULL, len != 0), m = __popc(some);
+        if (!some) return all;
+        if (some & (some + 1)) {  // values without matches between others: closed up, so that every lane below m has outputs
+            if (len) match[__popc(some & lanemask_lt())] = make_uint2(start, len);
+            __syncwarp();
+            const uint2 p = lane < m ? match[lane] : make_uint2(0, 0);
+            __syncwarp();
+            start = p.x;
+            len = p.y;
+        }
+        uint32_t incl = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, incl, d);
+            if (lane >= (unsigned)d) incl += v;
+        }
+        const uint32_t total = __shfl_sync(FULL, incl, 31), before = incl - len, shift = start - before;
+        uint32_t from = 0;
+        for (; total - from > 64; from += 32 * RW_UNROLL) {
+            dealt<RW_UNROLL>(o, ix, from, total, m, before, shift);
+            if (total - from <= 32 * RW_UNROLL) return all + total;
+        }
+        for (; from < total; from += 32) dealt<1>(o, ix, from, total, m, before, shift);
+        return all + total;
+    }
+    // A frontier of one value, followed by one warp while it stays one: a value's matches are looked up
+    // while the test whether it is new is under way.  Leaves the ring's ends and the level in `sh`.
+    __device__ __forceinline__ void follow(const Out& o, const Ix& ix, uint64_t max_iterations) {
+        const unsigned lane = lane_id();
+        unsigned at = sh->head, y = queue[at & mask];
+        uint64_t cand = 0;
+        uint32_t start, len;
+        find(ix, y, start, len);
+        const unsigned levels = (unsigned)min((unsigned long long)(max_iterations - sh->level), 0xFFFFFFFFull);
+        unsigned more = 1, done = 0;  // values in the frontier; levels done
+        while (done < levels && len <= 32) {
+            ++done;
+            cand += len;
+            bool fresh = lane < len;
+            const uint32_t z = other_of(ix, fresh ? start + lane : 0u);
+            if (fresh && z >> o.lo_bits) {
+                set_status(o.st, XLB_ERR_CAPACITY, 22, z);
+                fresh = false;
+            }
+            uint32_t next = 0, next_len = 0;
+            unsigned word = ~0u;
+            if (fresh) {
+                word = seen[z >> 5];
+                find(ix, z, next, next_len);
+            }
+            const unsigned bit = 1u << (z & 31);
+            fresh = fresh && !(word & bit);
+            unsigned b = __ballot_sync(FULL, fresh);
+            if (b & (b - 1)) {  // several (or one more than once)
+                if (fresh) fresh = !(atomicOr(&seen[z >> 5], bit) & bit);
+                b = __ballot_sync(FULL, fresh);
+                more = __popc(b);
+                if (more > 1) {
+                    const unsigned to = at + 1 + __popc(b & lanemask_lt());
+                    if (fresh) queue[to & mask] = (unsigned short)z;  // (32 at most, and the one they came from is done with)
+                    break;
+                }
+            } else if (fresh) seen[z >> 5] = word | bit;
+            if (!b) {
+                more = 0;
+                break;
+            }
+            const unsigned from = __ffs(b) - 1;
+            y = __shfl_sync(FULL, z, from);
+            start = __shfl_sync(FULL, next, from);
+            len = __shfl_sync(FULL, next_len, from);
+            ++at;
+            __syncwarp();
+        }
+        __syncwarp();
+        if (lane == 0) {
+            const bool still = more == 1;  // one value, not looked at yet
+            if (still) queue[at & mask] = (unsigned short)y;
+            sh->head = still ? at : at + 1;
+            sh->tail = still ? at + 1 : at + 1 + more;
+            sh->level += done;
+            sh->cand += cand;
+        }
+    }
+};
+// The seeds of a row that is given up, for the loop.
+__device__ __noinline__ void rows_give_up(const Out& o, const RowsShape& sh, unsigned row) {
+    for (unsigned at = threadIdx.x; at < sh.words; at += blockDim.x) {
+        unsigned word = o.visited[(uint64_t)row * sh.words + at];
+        if (!word) continue;
+        unsigned long long to = atomicAdd(&o.ctl->rows_seeds, (unsigned long long)__popc(word));
+        for (; word; word &= word - 1, ++to)
+            if (to < o.cap) o.log[to] = ((uint64_t)row << 32) | (at * 32 + __ffs(word) - 1);
+    }
+    if (threadIdx.x == 0) atomicAdd(&o.ctl->rows_given_up, 1ull);
+}
+template <int W>
+__global__ void __launch_bounds__(W * 32) delta_rows_k(const Out o, const __grid_constant__ Rules rules, const RowsShape sh, uint64_t max_iterations) {
+    extern __shared__ __align__(16) unsigned char rw_smem[];
+    __shared__ RowsShared s;
+    __shared__ uint2 match_s[W][32];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    RowsWarp<W> w;
+    w.seen = reinterpret_cast<unsigned*>(rw_smem);
+    w.queue = reinterpret_cast<unsigned short*>(w.seen + sh.words);
+    w.match = match_s[warp];
+    w.sh = &s;
+    w.mask = sh.queue - 1;
+    volatile RowsShared* v = &s;
+    Ctl* ctl = o.ctl;
+    if (threadIdx.x == 0) s.tuples = s.cands = s.levels = 0;
+    bool left = false;
+    for (uint64_t chunk = blockIdx.x;;) {
+        const uint64_t first = chunk * sh.chunk;
+        if (first >= sh.rows) break;
+        if (threadIdx.x == 0) s.next = *(volatile unsigned long long*)&ctl->rows_given_up * 4 <= gridDim.x;
+        __syncthreads();
+        const bool tried = v->next;
+        for (unsigned row = (unsigned)first; row < sh.rows && row < first + sh.chunk; ++row) {
+            // the row's bits and the queue they start
+            unsigned mine = 0;
+            for (unsigned at = threadIdx.x; at < sh.words; at += W * 32) {
+                const unsigned word = o.visited[(uint64_t)row * sh.words + at];
+                w.seen[at] = word;
+                mine += __popc(word);
+            }
+            if (threadIdx.x == 0) {
+                s.head = s.tail = s.failed = 0;
+                s.level = s.cand = 0;
+            }
+            const int any = __syncthreads_or(mine != 0);
+            if (!any) continue;
+            if (mine) {
+                unsigned to = atomicAdd(&s.tail, mine);
+                for (unsigned at = threadIdx.x; at < sh.words; at += W * 32)
+                    for (unsigned word = w.seen[at]; word; word &= word - 1, ++to)
+                        if (to < sh.queue) w.queue[to] = (unsigned short)(at * 32 + __ffs(word) - 1);
+            }
+            __syncthreads();
+            unsigned head = 0, end = v->tail;
+            bool ok = tried && end <= sh.queue;
+            uint64_t level = 0, cand = 0, looked = RW_LONG;
+            while (ok && head != end && level < max_iterations) {
+                if (end - head == 1 && rules.n == 1) {
+                    if (warp == 0) w.follow(o, rules.r[0].ix[0], max_iterations);
+                    __syncthreads();
+                    head = v->head;
+                    end = v->tail;
+                    level = v->level;
+                    __syncthreads();
+                    if (head == end || level >= max_iterations) break;
+                }
+                ++level;
+                w.head = head;
+                const unsigned per = min(32u, (end - head + W - 1) / W);
+                for (unsigned at = head + warp * per; at - head < end - head; at += W * per) {
+                    const bool on = lane < per && end - at > lane;
+                    const unsigned y = on ? w.queue[(at + lane) & w.mask] : 0u;
+                    for (int q = 0; q < rules.n; ++q) cand += w.expand(o, rules.r[q].ix[0], on, y);
+                    if (cand > looked) {
+                        looked = cand + 4096;
+                        if (lane == 0 && *(volatile unsigned*)&ctl->rows_idle * 4ull > gridDim.x * 3ull) s.failed = 1;
+                    }
+                    if (__any_sync(FULL, v->failed)) break;
+                }
+                __syncthreads();
+                head = end;
+                end = v->tail;
+                ok = !v->failed;
+                if (threadIdx.x == 0) {
+                    s.head = head;
+                    s.level = level;
+                }
+                __syncthreads();
+            }
+            if (!ok) {
+                rows_give_up(o, sh, row);
+                __syncthreads();
+                continue;
+            }
+            if (lane == 0) atomicAdd(&s.cand, (unsigned long long)cand);
+            for (unsigned at = threadIdx.x; at < sh.words; at += W * 32) o.visited[(uint64_t)row * sh.words + at] = w.seen[at];
+            left |= head != end;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                s.tuples += end;
+                s.cands += s.cand;
+                s.levels = level > s.levels ? level : s.levels;
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s.next = atomicAdd(&ctl->rows_ticket, 1u);
+        __syncthreads();
+        chunk = (uint64_t)gridDim.x + v->next;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        atomicAdd(&ctl->rows_idle, 1u);
+        if (s.levels) {
+            atomicAdd(&ctl->rows_tuples, s.tuples);
+            atomicAdd(&ctl->rows_candidates, s.cands);
+            if (*(volatile unsigned long long*)&ctl->rows_levels < s.levels) atomicMax(&ctl->rows_levels, s.levels);
+        }
+        if (left) ctl->rows_left = 1;
+    }
+}
+// The loop starts over on what was given up.
+__global__ void delta_rows_left_k(Ctl* c) {
+    c->tail = c->rows_seeds;
+    ready(c, false);
+}
+
 }  // namespace
 
 static Out out_of(xlb_ctx* c, const DeltaLoop& d) {
@@ -1024,6 +1364,53 @@ static Ix view_of(const Index& ix) {
               ix.pay ? ix.pay->as<uint32_t>() : ix.S->as<uint32_t>(), ix.pay ? 0 : 1};
 }
 
+// Rules that keep the head's first column and join its second with one stored relation, from seeds alone.
+static bool rows_apart(const DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, const Keys& known) {
+    if (d.square || !d.seeded || known.n || rules.empty() || !variants.empty() || d.lo_bits < RW_BITS_MIN || d.lo_bits > RW_BITS_MAX || d.hi_bits > 31) return false;
+    for (auto& r : rules)
+        if (r.joins != 1 || r.hi_src != 0 || r.lo_src != 2 || r.key_src[0] != SRC_LO) return false;
+    return true;
+}
+static_assert(rows_bytes(RW_BITS_MAX) <= (46u << 10), "a row's shared memory needs no opt-in");
+static unsigned rows_per_sm(int lo_bits) { return std::min(32u, (220u << 10) / (rows_bytes(lo_bits) + 2048u)); }
+template <int W>
+static void launch_rows(xlb_ctx* c, const DeltaLoop& d, const Rules& rs, RowsShape sh, uint64_t max_iterations) {
+    const unsigned smem = rows_bytes(d.lo_bits);
+    const unsigned per_sm = std::min(2048u / (W * 32), rows_per_sm(d.lo_bits));
+    const unsigned blocks = std::min(per_sm * (unsigned)c->sm_count, sh.rows);
+    sh.chunk = std::max(1u, sh.rows / (blocks * 8));  // (a domain much larger than what is in use: few tickets)
+    delta_rows_k<W><<<blocks, W * 32, smem, c->stream>>>(out_of(c, d), rs, sh, max_iterations);
+}
+// False: rows are left for the loop, which is ready to start on them.
+static bool run_rows(xlb_ctx* c, DeltaLoop& d, const Rules& rs, uint64_t max_iterations, DeltaResult* res) {
+    RowsShape sh{};
+    sh.rows = 1u << d.hi_bits;
+    sh.words = 1u << (d.lo_bits - 5);
+    sh.queue = rows_queue(d.lo_bits);
+    Ctl* ctl = (Ctl*)d.ctl;
+    prof_begin(c, "expand_mark", 0);
+    // Four warps a row keep rows of a few thousand candidates short (one: twice the time); eight where an SM
+    // has few rows, or room for few.
+    if (std::min((sh.rows + (unsigned)c->sm_count - 1) / (unsigned)c->sm_count, rows_per_sm(d.lo_bits)) <= 6) launch_rows<8>(c, d, rs, sh, max_iterations);
+    else launch_rows<4>(c, d, rs, sh, max_iterations);
+    check_launch(c, "expand_mark");
+    unsigned long long w[6];  // tuples, candidates, levels, left, given up, seeds
+    read_words(c, &ctl->rows_tuples, 6, w);
+    res->rows = w[0];
+    res->candidates = w[1];
+    res->iterations = w[2];
+    res->fix = w[3] == 0;
+    prof_add_bytes(c, "expand_mark", w[1] * 4ull + d.words * 8ull);
+    if (w[4] == 0) {
+        res->iterations = std::max<uint64_t>(res->iterations, 1);  // an iteration over nothing finds nothing
+        return true;
+    }
+    delta_rows_left_k<<<1, 1, 0, c->stream>>>(ctl);
+    check_launch(c, "delta_begin");
+    d.room = w[5];
+    return false;
+}
+
 bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
                    DeltaResult* res) {
     if (rules.size() > DL_RULES || variants.size() > SQ_VARIANTS) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules and %zu variants in a delta loop", rules.size(), variants.size());
@@ -1074,6 +1461,15 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
             r.ix[k] = view_of(*rules[q].ix[k]);
         }
     }
+    Buf by_rows;  // the head after rows were evaluated one by one and some are left
+    if (rows_apart(d, rules, variants, known)) {
+        if (run_rows(c, d, rs, max_iterations, res)) return !c->status_code;
+        if (c->status_code) return false;
+        by_rows = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
+        CUDA_OK(copy_async(c, by_rows->p, d.visited->p, d.words * 4, cudaMemcpyDeviceToDevice));
+    }
+    DeltaResult rows_done = *res;
+    if (!by_rows) rows_done.fix = true;
     Buf heavy = make_buf(c, (uint64_t)DL_HEAVY_MAX * sizeof(Heavy));
     if (!d.seeded) {
         delta_begin_k<<<1, 1, 0, c->stream>>>((Ctl*)d.ctl, square);
@@ -1089,10 +1485,10 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         unsigned long long w[7];  // tail, start, end, iterations, candidates, fix, overflow
         read_words(c, d.ctl, 7, w);
         if (c->status_code) return false;
-        res->rows = w[0];
-        res->iterations = w[3];
-        res->candidates = w[4];
-        res->fix = w[5] != 0;
+        res->rows = rows_done.rows + w[0];
+        res->iterations = std::max<uint64_t>(rows_done.iterations, w[3]);
+        res->candidates = rows_done.candidates + w[4];
+        res->fix = rows_done.fix && w[5] != 0;
         prof_add_bytes(c, "expand_mark", w[4] * 4ull + w[0] * 16ull);
         if (!w[6]) return true;
         // The log was too short for the last iteration: its delta is what the head's bitmap holds
@@ -1102,7 +1498,8 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         done.buf = d.log;
         done.n = stored;
         Buf before = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
-        CUDA_OK(set_async(c, before->p, 0, before->bytes));
+        if (by_rows) CUDA_OK(copy_async(c, before->p, by_rows->p, d.words * 4, cudaMemcpyDeviceToDevice));
+        else CUDA_OK(set_async(c, before->p, 0, before->bytes));
         for (const Keys* k : {&known, (const Keys*)&done}) {
             if (!k->n) continue;
             prof_begin(c, "dense_mark", k->n * 8ull);
