@@ -360,7 +360,9 @@ struct xlb_ctx {
     DevStatus* d_status = nullptr;
     unsigned read_seq = 0;      // number of the last read-back (read_words)
     unsigned status_code = 0;   // device status as the last read-back found it ...
-    bool drained = false;       // ... and nothing was enqueued since: the stream is idle and the code is current
+    bool drained = false;       // ... and nothing was enqueued since: all of it has done its work and the code is current
+    bool leaving = false;       // the last kernel enqueued leaves the status itself (Publish), which nobody has read yet
+    unsigned* arrived = nullptr;  // its blocks that are done: zero between kernels
     cudaEvent_t plan_e0 = nullptr, plan_e1 = nullptr;  // around a plan (made on first use)
     int sm_count = 148;
     // executor state
@@ -476,7 +478,7 @@ inline Buf make_buf(xlb_ctx* c, uint64_t bytes) { return std::make_shared<DevBuf
 
 inline void check_launch(xlb_ctx* c, const char* what) {
     c->launches++;
-    c->drained = false;
+    c->drained = c->leaving = false;
     if (c->prof_open) {
         cudaEvent_t e1;
         cudaEventCreate(&e1);
@@ -490,11 +492,11 @@ inline void check_launch(xlb_ctx* c, const char* what) {
 
 // Copies and fills enqueued on the context's stream.
 inline cudaError_t copy_async(xlb_ctx* c, void* dst, const void* src, size_t n, cudaMemcpyKind kind) {
-    c->drained = false;
+    c->drained = c->leaving = false;
     return cudaMemcpyAsync(dst, src, n, kind, c->stream);
 }
 inline cudaError_t set_async(xlb_ctx* c, void* dst, int value, size_t n) {
-    c->drained = false;
+    c->drained = c->leaving = false;
     return cudaMemsetAsync(dst, value, n, c->stream);
 }
 
@@ -539,23 +541,62 @@ static __global__ void publish_words_k(const unsigned long long* __restrict__ sr
     *(volatile unsigned long long*)(dst + i) = ((unsigned long long)seq << 32) | half;
 }
 
-// Read `n` 64-bit words from device memory (everything enqueued before has run when this returns).
-inline void read_words(xlb_ctx* c, const void* dptr, int n, unsigned long long* out) {
-    static const bool spin = getenv("XLB_BLOCKING_WAIT") == nullptr;
-    if (c->wait_hook || !spin || n > READ_WORDS_MAX) {
-        if (n) CUDA_OK(copy_async(c, c->h_scalar, dptr, (size_t)n * 8, cudaMemcpyDeviceToHost));
-        CUDA_OK(copy_async(c, c->h_scalar + READ_WORDS_AT, c->d_status, 8, cudaMemcpyDeviceToHost));
-        stream_wait(c);
-        for (int i = 0; i < n; ++i) out[i] = c->h_scalar[i];
-        c->status_code = (unsigned)c->h_scalar[READ_WORDS_AT];
-        c->drained = true;
-        return;
+// The same by the kernel that computes the words: its last block to finish sends them, which saves the
+// launch of another (4 us).  For kernels of few blocks, which all pass publish_last at their end (the
+// arrivals queue on one counter); or publish_now, by one block that knows all others are done.
+struct Publish {
+    unsigned long long* dst = nullptr;  // null: not asked to
+    const unsigned long long* src = nullptr;
+    const DevStatus* st = nullptr;
+    unsigned* arrived = nullptr;
+    int n = 0;
+    unsigned seq = 0;
+};
+constexpr unsigned PUBLISH_BLOCKS_MAX = 1184;
+__device__ __forceinline__ void publish_now(const Publish& p) {  // all threads of a block
+    if (!p.dst) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i <= 2 * p.n; i += blockDim.x) {
+        const unsigned half = i == 2 * p.n ? __ldcg(&p.st->code) : (unsigned)(__ldcg(&p.src[i >> 1]) >> ((i & 1) * 32));
+        *(volatile unsigned long long*)(p.dst + i) = ((unsigned long long)p.seq << 32) | half;
     }
+}
+__device__ __forceinline__ void publish_last(const Publish& p) {  // all threads of all blocks
+    if (!p.dst) return;
+    __shared__ bool last_s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last_s = atomicAdd(p.arrived, 1u) == gridDim.x - 1;
+        if (last_s) {
+            *(volatile unsigned*)p.arrived = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (last_s) publish_now(p);
+}
+inline bool publish_ok(xlb_ctx* c, int n) {
+    static const bool spin = getenv("XLB_BLOCKING_WAIT") == nullptr;
+    return !c->wait_hook && spin && n <= READ_WORDS_MAX;
+}
+// What a kernel of `blocks` blocks gets so that it leaves `n` words from `dptr` (none: the status alone).
+inline Publish publish_by(xlb_ctx* c, uint64_t blocks, const void* dptr = nullptr, int n = 0) {
+    Publish p;
+    c->leaving = false;
+    if (blocks > PUBLISH_BLOCKS_MAX || !publish_ok(c, n)) return p;
+    if (++c->read_seq == 0) ++c->read_seq;  // 0 is what untouched words carry
+    p.dst = c->h_scalar_dev + READ_WORDS_AT;
+    p.src = (const unsigned long long*)dptr;
+    p.st = c->d_status;
+    p.arrived = c->arrived;
+    p.n = n;
+    p.seq = c->read_seq;
+    return p;
+}
+inline void poll_words(xlb_ctx* c, int n, unsigned long long* out) {
     const double tr0 = c->trace_on ? trace_now() : 0;
     auto t0 = std::chrono::steady_clock::now();
-    if (++c->read_seq == 0) ++c->read_seq;  // 0 is what untouched words carry
-    publish_words_k<<<1, 64, 0, c->stream>>>((const unsigned long long*)dptr, n, c->d_status, c->h_scalar_dev + READ_WORDS_AT, c->read_seq);
-    CUDA_OK(cudaGetLastError());
     const volatile unsigned long long* w = c->h_scalar + READ_WORDS_AT;
     uint64_t polls = 0;
     bool waited = false;
@@ -570,14 +611,42 @@ inline void read_words(xlb_ctx* c, const void* dptr, int n, unsigned long long* 
     for (int i = 0; i < n; ++i) out[i] = (w[2 * i] & 0xFFFFFFFFull) | (w[2 * i + 1] << 32);
     c->status_code = (unsigned)w[2 * n];
     c->drained = true;
+    c->leaving = false;
     c->ms_sync_wait += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     c->syncs++;
     trace_note(c, "wait (words)", tr0);
 }
 
+// Read `n` 64-bit words from device memory (everything enqueued before has run when this returns).
+inline void read_words(xlb_ctx* c, const void* dptr, int n, unsigned long long* out) {
+    if (!publish_ok(c, n)) {
+        if (n) CUDA_OK(copy_async(c, c->h_scalar, dptr, (size_t)n * 8, cudaMemcpyDeviceToHost));
+        CUDA_OK(copy_async(c, c->h_scalar + READ_WORDS_AT, c->d_status, 8, cudaMemcpyDeviceToHost));
+        stream_wait(c);
+        for (int i = 0; i < n; ++i) out[i] = c->h_scalar[i];
+        c->status_code = (unsigned)c->h_scalar[READ_WORDS_AT];
+        c->drained = true;
+        return;
+    }
+    if (++c->read_seq == 0) ++c->read_seq;
+    publish_words_k<<<1, 64, 0, c->stream>>>((const unsigned long long*)dptr, n, c->d_status, c->h_scalar_dev + READ_WORDS_AT, c->read_seq);
+    CUDA_OK(cudaGetLastError());
+    poll_words(c, n, out);
+}
+// After the launch of a kernel that got `p`: its words (by a read-back of their own where it was not asked).
+inline void read_published(xlb_ctx* c, const Publish& p, const void* dptr, int n, unsigned long long* out) {
+    if (p.dst) poll_words(c, n, out);
+    else read_words(c, dptr, n, out);
+}
+// The same for a kernel that may be the last of an operation: its status is read when one is asked for.
+inline void status_published(xlb_ctx* c, const Publish& p) { c->leaving = p.dst != nullptr; }
+
 // Fails with what a kernel reported, if one did; everything enqueued has run when this returns.
 inline void check_dev_status(xlb_ctx* c) {
-    if (!c->drained) read_words(c, nullptr, 0, nullptr);
+    if (!c->drained) {
+        if (c->leaving) poll_words(c, 0, nullptr);
+        else read_words(c, nullptr, 0, nullptr);
+    }
     if (c->status_code == 0) return;
     DevStatus s;
     CUDA_OK(copy_async(c, c->h_scalar, c->d_status, sizeof s, cudaMemcpyDeviceToHost));

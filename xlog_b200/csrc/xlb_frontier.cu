@@ -42,7 +42,7 @@ struct Args {
 };
 
 // One block: bitmaps in shared memory.
-__global__ void __launch_bounds__(F_THREADS, 1) frontier_one_k(const __grid_constant__ Args a) {
+__device__ __forceinline__ void frontier_one(const Args& a) {
     extern __shared__ unsigned bm[];
     __shared__ unsigned or_s, fresh_s[3], cand_s;
     __shared__ unsigned sm[33];
@@ -478,6 +478,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) frontier_large_k(const __grid_co
     }
 }
 
+__global__ void __launch_bounds__(F_THREADS, 1) frontier_one_k(const __grid_constant__ Args a, const Publish pub) {
+    frontier_one(a);
+    publish_now(pub);
+}
+
 }  // namespace
 
 bool ops_frontier_whole(xlb_ctx* c, const xlb_rel* rel, int key_col, int value_col, const std::vector<FrontierConst>& seeds, uint64_t max_iterations, FrontierWhole* out) {
@@ -504,12 +509,15 @@ bool ops_frontier_whole(xlb_ctx* c, const xlb_rel* rel, int key_col, int value_c
     Buf work = make_buf(c, 64 + (one ? 0 : 32 + 3 * bitmap)), lists[2];
     a.words = work->as<unsigned long long>();
     const char* name = large ? "scan_join_mark" : "dense_mark";
+    const unsigned grid = one ? 1u : (unsigned)std::min<uint64_t>({(uint64_t)c->sm_count, (n + 4 * F_THREADS - 1) / (4 * F_THREADS)});
+    Publish pub;
     prof_begin(c, name, large ? 0 : n * 8ull);
     if (one) {
         const int smem = 3 << (F1_BITS - 3);
         if (!c->frontier_attr_set) CUDA_OK(cudaFuncSetAttribute(frontier_one_k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         c->frontier_attr_set = true;
-        frontier_one_k<<<1, F_THREADS, smem, c->stream>>>(a);
+        pub = publish_by(c, grid, work->p, 5);
+        frontier_one_k<<<grid, F_THREADS, smem, c->stream>>>(a, pub);
     } else {
         a.sync = (unsigned*)((char*)work->p + 64);
         a.marks = a.sync + 8;
@@ -524,13 +532,12 @@ bool ops_frontier_whole(xlb_ctx* c, const xlb_rel* rel, int key_col, int value_c
                 lists[k] = make_buf(c, n * 8);
                 a.list[k] = lists[k]->as<uint64_t>();
             }
-        const unsigned grid = (unsigned)std::min<uint64_t>({(uint64_t)c->sm_count, (n + 4 * F_THREADS - 1) / (4 * F_THREADS)});
-        void* args[] = {&a};
+        void* args[] = {&a};  // (the words left by these two kernels themselves: 80 -> 89 us at 80 K rows)
         CUDA_OK(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(F_THREADS), args, smem, c->stream));
     }
     check_launch(c, name);
     unsigned long long w[5];
-    read_words(c, work->p, 5, w);
+    read_published(c, pub, work->p, 5, w);
     if (c->status_code) check_dev_status(c);
     if (large) prof_add_bytes(c, name, w[4] * 8ull);
     if (w[3] == 2 || (w[3] == 0 && one && max_iterations == 1u << 17)) return false;

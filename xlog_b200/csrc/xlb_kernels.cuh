@@ -363,7 +363,7 @@ inline SelectTiles sweep_tiles(xlb_ctx* c, uint64_t* zeroed, uint64_t n) {
 // Each warp owns 256 consecutive rows and walks them 32 at a time, so reads are coalesced and
 // the predicate runs once per row; ballots give the stable position inside the warp.
 template <class Pred, class Emit>
-static __global__ void __launch_bounds__(BLOCK) select_write_k(Pred pred, Emit emit, uint64_t n, SelectTiles tiles, uint64_t* total) {
+static __global__ void __launch_bounds__(BLOCK) select_write_k(Pred pred, Emit emit, uint64_t n, SelectTiles tiles, uint64_t* total, const Publish pub) {
     __shared__ uint32_t sm[33];
     __shared__ unsigned tile_s;
     __shared__ uint64_t before_s;
@@ -404,6 +404,7 @@ static __global__ void __launch_bounds__(BLOCK) select_write_k(Pred pred, Emit e
         pos += __popc(b);
     }
     if (tile + 1 == tiles.n && threadIdx.x == 0) *total = (tiles.n > 1 ? before_s : 0ull) + tot;
+    publish_last(pub);
 }
 
 // Returns the number of selected rows (one host read-back).
@@ -420,10 +421,11 @@ uint64_t select(xlb_ctx* c, Pred pred, Emit emit, uint64_t n) {
         tiles = sweep_tiles(c, total + 1, ntiles);
     }
     prof_begin(c, "select_write", 0);
-    select_write_k<Pred, Emit><<<(unsigned)ntiles, BLOCK, 0, c->stream>>>(pred, emit, n, tiles, total);
+    const Publish pub = publish_by(c, ntiles, total, 1);
+    select_write_k<Pred, Emit><<<(unsigned)ntiles, BLOCK, 0, c->stream>>>(pred, emit, n, tiles, total, pub);
     check_launch(c, "select_write");
     unsigned long long h;
-    read_words(c, total, 1, &h);
+    read_published(c, pub, total, 1, &h);
     return h;
 }
 
@@ -436,7 +438,7 @@ uint64_t select(xlb_ctx* c, Pred pred, Emit emit, uint64_t n) {
 // was slower: 94 us against 59.)
 constexpr int SA_BLOCK = 1024, SA_ROUNDS = 8, SA_TILE = SA_BLOCK * SA_ROUNDS;
 template <class Pred, class Emit>
-static __global__ void __launch_bounds__(SA_BLOCK) select_append_k(Pred pred, Emit emit, uint64_t n, unsigned long long* total) {
+static __global__ void __launch_bounds__(SA_BLOCK) select_append_k(Pred pred, Emit emit, uint64_t n, unsigned long long* total, const Publish pub) {
     __shared__ uint32_t sm[33];
     __shared__ unsigned long long base_s;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -466,6 +468,7 @@ static __global__ void __launch_bounds__(SA_BLOCK) select_append_k(Pred pred, Em
         if ((b >> lane) & 1u) emit(wbase + r * 32 + lane, pos + __popc(b & lanemask_lt()));
         pos += __popc(b);
     }
+    publish_last(pub);
 }
 
 // Returns the number of selected rows (one host read-back); output order unspecified.
@@ -476,10 +479,11 @@ uint64_t select_unordered(xlb_ctx* c, Pred pred, Emit emit, uint64_t n, const ch
     Buf total = make_buf(c, 8);
     CUDA_OK(set_async(c, total->p, 0, 8));
     prof_begin(c, name, bytes);
-    select_append_k<Pred, Emit><<<(unsigned)ntiles, SA_BLOCK, 0, c->stream>>>(pred, emit, n, total->as<unsigned long long>());
+    const Publish pub = publish_by(c, ntiles, total->p, 1);
+    select_append_k<Pred, Emit><<<(unsigned)ntiles, SA_BLOCK, 0, c->stream>>>(pred, emit, n, total->as<unsigned long long>(), pub);
     check_launch(c, name);
     unsigned long long h;
-    read_words(c, total->p, 1, &h);
+    read_published(c, pub, total->p, 1, &h);
     return h;
 }
 
@@ -533,7 +537,7 @@ struct FilterStage {
     }
 };
 static __global__ void pack2_k(const uint32_t* __restrict__ c0, const uint32_t* __restrict__ c1, uint64_t* __restrict__ out, uint64_t n, unsigned long long* or_out,
-                               bool vec, int fcol = -1, uint32_t fval = 0, uint64_t* __restrict__ fout = nullptr, unsigned long long* fcount = nullptr) {
+                               bool vec, int fcol = -1, uint32_t fval = 0, uint64_t* __restrict__ fout = nullptr, unsigned long long* fcount = nullptr, const Publish pub = Publish()) {
     uint64_t acc = 0;
     const uint64_t n4 = vec ? n / 4 : 0;
     const uint4* a4 = reinterpret_cast<const uint4*>(c0);
@@ -574,13 +578,14 @@ static __global__ void pack2_k(const uint32_t* __restrict__ c0, const uint32_t* 
     }
     if (fcol >= 0) stage.end(fout, fcount);
     if (or_out) block_or(acc, or_out);
+    publish_last(pub);
 }
 // The read-only sweep of a two-column relation that is not packed: OR of the packed rows into
 // *or_out, and with fcol >= 0 the rows whose column fcol equals fval appended, packed, to `fout`
 // (*fcount += their number; a match is rare).  Sixteen rows per thread and step: eight 16-byte
 // loads in flight (the columns are 16-byte aligned; the host checks).
 static __global__ void __launch_bounds__(BLOCK) cols_or_filter_k(const uint32_t* __restrict__ c0, const uint32_t* __restrict__ c1, uint64_t n, unsigned long long* or_out, int fcol,
-                                                            uint32_t fval, uint64_t* __restrict__ fout, unsigned long long* fcount) {
+                                                            uint32_t fval, uint64_t* __restrict__ fout, unsigned long long* fcount, const Publish pub) {
     uint32_t acc0 = 0, acc1 = 0;
     __shared__ FilterStage stage;
     if (fcol >= 0) stage.begin();
@@ -623,14 +628,16 @@ static __global__ void __launch_bounds__(BLOCK) cols_or_filter_k(const uint32_t*
     if (fcol >= 0) stage.end(fout, fcount);
     uint64_t acc = ((uint64_t)acc0 << 32) | acc1;
     block_or(acc, or_out);
+    publish_last(pub);
 }
-static __global__ void pack1_k(const uint32_t* __restrict__ c0, uint64_t* __restrict__ out, uint64_t n, unsigned long long* or_out) {
+static __global__ void pack1_k(const uint32_t* __restrict__ c0, uint64_t* __restrict__ out, uint64_t n, unsigned long long* or_out, const Publish pub) {
     uint64_t acc = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         out[i] = c0[i];
         acc |= c0[i];
     }
     if (or_out) block_or(acc, or_out);
+    publish_last(pub);
 }
 static __global__ void unpack2_k(const uint64_t* __restrict__ in, uint32_t* __restrict__ c0, uint32_t* __restrict__ c1, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -778,16 +785,18 @@ static __global__ void __launch_bounds__(BLOCK) radix_upfront_k(const uint64_t* 
 
 // Exclusive scan of each digit histogram (the digit bases of the sweep) and, per digit, whether
 // more than one bin is occupied.
-static __global__ void __launch_bounds__(BLOCK) radix_bases_k(const unsigned int* __restrict__ ghist, unsigned long long n, unsigned int* __restrict__ bases, unsigned long long* __restrict__ varies) {
+// (a block per digit: one block for all took 8 us)
+static __global__ void __launch_bounds__(BLOCK) radix_bases_k(const unsigned int* __restrict__ ghist, unsigned long long n, unsigned int* __restrict__ bases, unsigned long long* __restrict__ varies,
+                                                              const Publish pub) {
     __shared__ unsigned int sm[33];
-    for (int d = 0; d < 8; ++d) {
-        unsigned v = ghist[d * 256 + threadIdx.x];
-        unsigned tot;
-        unsigned ex = block_exclusive_scan<unsigned>(v, &tot, sm);
-        bases[d * 256 + threadIdx.x] = ex;
-        int constant = __syncthreads_or(v == n);
-        if (threadIdx.x == 0) varies[d] = constant ? 0ull : 1ull;
-    }
+    const int d = blockIdx.x;
+    const unsigned v = ghist[d * 256 + threadIdx.x];
+    unsigned tot;
+    const unsigned ex = block_exclusive_scan<unsigned>(v, &tot, sm);
+    bases[d * 256 + threadIdx.x] = ex;
+    const int constant = __syncthreads_or(v == n);
+    if (threadIdx.x == 0) varies[d] = constant ? 0ull : 1ull;
+    publish_last(pub);
 }
 
 // Per-tile histogram of one digit: hist[d * ntiles + tile].
@@ -1208,14 +1217,16 @@ inline void radix_sort(xlb_ctx* c, Buf& keys, Buf* vals, uint64_t n, unsigned di
         radix_upfront_k<<<grid_for(c, n, BLOCK * 8), BLOCK, 0, c->stream>>>(keys->as<uint64_t>(), n, ghist, digits);
         check_launch(c, "radix_upfront");
         prof_begin(c, "radix_bases", 0);
-        radix_bases_k<<<1, BLOCK, 0, c->stream>>>(ghist, n, bases, varies);
+        Publish pub;
+        if (!known) pub = publish_by(c, 8, varies, 8);
+        radix_bases_k<<<8, BLOCK, 0, c->stream>>>(ghist, n, bases, varies, pub);
         check_launch(c, "radix_bases");
         int np = 0, pass[8];
         if (known) {
             for (int d = 0; d < digits.n; ++d) pass[np++] = d;
         } else {
             unsigned long long v[8];
-            read_words(c, varies, 8, v);
+            read_published(c, pub, varies, 8, v);
             for (int d = 0; d < digits.n; ++d)
                 if (v[d]) pass[np++] = d;
         }
@@ -1322,7 +1333,7 @@ __device__ __forceinline__ uint64_t merge_path(const uint64_t* A, uint64_t na, c
 // MODE 1: out = merge of A and B (disjoint), out has na + nb entries.
 template <int MODE>
 static __global__ void __launch_bounds__(BLOCK) mp_tile_k(const uint64_t* __restrict__ A, uint64_t na, const uint64_t* __restrict__ B, uint64_t nb,
-                                                    uint8_t* __restrict__ keep, uint64_t* __restrict__ out) {
+                                                    uint8_t* __restrict__ keep, uint64_t* __restrict__ out, const Publish pub = Publish()) {
     __shared__ uint64_t sA[MP_TILE + 1];
     __shared__ uint64_t sB[MP_TILE + 2];
     __shared__ uint64_t split_s[2];
@@ -1380,6 +1391,7 @@ static __global__ void __launch_bounds__(BLOCK) mp_tile_k(const uint64_t* __rest
         __syncthreads();
         for (unsigned i = threadIdx.x; i < total; i += BLOCK) out[d0 + i] = sA[i];
     }
+    publish_last(pub);
 }
 
 struct PredKeep {
@@ -1440,8 +1452,10 @@ inline Buf merge_disjoint(xlb_ctx* c, const uint64_t* A, uint64_t na, const uint
     }
     uint64_t ntiles = (na + nb + MP_TILE - 1) / MP_TILE;
     prof_begin(c, "mp_union", (na + nb) * 16ull);
-    mp_tile_k<1><<<(unsigned)ntiles, BLOCK, 0, c->stream>>>(A, na, B, nb, nullptr, o->as<uint64_t>());
+    const Publish pub = publish_by(c, ntiles);
+    mp_tile_k<1><<<(unsigned)ntiles, BLOCK, 0, c->stream>>>(A, na, B, nb, nullptr, o->as<uint64_t>(), pub);
     check_launch(c, "mp_union");
+    status_published(c, pub);
     return o;
 }
 
@@ -1501,7 +1515,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_count_k(const unsigned int
 constexpr int DENSE_FUSED_GROUPS = 8192;
 static __global__ void __launch_bounds__(BLOCK) dense_count_scan_k(const unsigned int* __restrict__ bitmap, uint64_t words, uint32_t* group_counts, uint64_t groups,
                                                               const unsigned int* __restrict__ visited, uint64_t* __restrict__ group_offs, uint64_t* total,
-                                                              unsigned int* ticket, bool check, uint64_t expected, DevStatus* st) {
+                                                              unsigned int* ticket, bool check, uint64_t expected, DevStatus* st, const Publish pub) {
     __shared__ uint64_t sm[33];
     __shared__ bool last_s;
     uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1533,6 +1547,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_count_scan_k(const unsigne
         *ticket = 0;
         if (check && tot != expected) set_status(st, XLB_ERR_CAPACITY, 9, tot);
     }
+    publish_now(pub);
 }
 // One tuple out: packed, or (out0 set) as a row of columns, which is what a result that is fetched
 // next is wanted as.
@@ -1545,9 +1560,8 @@ __device__ __forceinline__ void dense_put(uint64_t x, int lo_bits, uint64_t lo_m
 }
 static __global__ void __launch_bounds__(BLOCK) dense_emit_k(const unsigned int* __restrict__ bitmap, uint64_t words, const uint64_t* __restrict__ group_offs,
                                                            uint64_t groups, int lo_bits, uint64_t* __restrict__ out, unsigned int* __restrict__ visited,
-                                                           uint64_t cap, DevStatus* st, uint32_t* __restrict__ out0 = nullptr, uint32_t* __restrict__ out1 = nullptr) {
+                                                           uint64_t cap, DevStatus* st, uint32_t* __restrict__ out0, uint32_t* __restrict__ out1, const Publish pub) {
     uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (g >= groups) return;
     const unsigned lane = lane_id();
     const uint64_t lo_mask = (1ull << lo_bits) - 1;
     uint64_t w = g * 32 + lane;
@@ -1563,7 +1577,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_emit_k(const unsigned int*
         unsigned o = __shfl_up_sync(FULL, incl, d);
         if (lane >= (unsigned)d) incl += o;
     }
-    uint64_t pos = group_offs[g] + (incl - cnt);
+    uint64_t pos = g < groups ? group_offs[g] + (incl - cnt) : 0;
     while (m) {
         unsigned b = __ffs(m) - 1;
         m &= m - 1;
@@ -1574,6 +1588,7 @@ static __global__ void __launch_bounds__(BLOCK) dense_emit_k(const unsigned int*
         }
         dense_put(x, lo_bits, lo_mask, pos++, out, out0, out1);
     }
+    publish_last(pub);
 }
 
 // The same two passes for bitmaps of a million words and more (domains of 2^25 bits and up): a
@@ -1867,7 +1882,7 @@ inline Buf mix_and_group(xlb_ctx* c, const uint64_t* in, uint64_t n) {
     mix_hist_k<<<grid_for(c, n, BLOCK * 8), BLOCK, 0, c->stream>>>(in, words->as<uint64_t>(), n, ghist + 7 * 256);
     check_launch(c, "mix");
     prof_begin(c, "radix_bases", 0);
-    radix_bases_k<<<1, BLOCK, 0, c->stream>>>(ghist, n, bases, varies);
+    radix_bases_k<<<8, BLOCK, 0, c->stream>>>(ghist, n, bases, varies, Publish());
     check_launch(c, "radix_bases");
     const uint64_t status_words = (uint64_t)ntiles * 256;
     Buf status = make_buf(c, (status_words + 8) * 4);

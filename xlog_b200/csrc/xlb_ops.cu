@@ -385,22 +385,29 @@ static Keys rel_packed(xlb_ctx* c, const xlb_rel* r, int fcol, uint32_t fval, Ke
         Buf oa = make_buf(c, 16);
         CUDA_OK(set_async(c, oa->p, 0, 16));
         prof_begin(c, "pack", r->rows * (materialize ? 16ull : 8ull));
+        Publish pub;
         const bool fuse = filtered && r->schema.arity == 2 && fcol >= 0 && fcol < 2;
         if (fuse) filtered->buf = make_buf(c, r->rows * 8);  // at most every row; trimmed below
         if (r->schema.arity == 2 && !materialize && (((uintptr_t)r->cols[0]->p | (uintptr_t)r->cols[1]->p) & 15) == 0) {
-            cols_or_filter_k<<<grid_for(c, r->rows, BLOCK * 16), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), r->cols[1]->as<uint32_t>(), r->rows, oa->as<unsigned long long>(),
+            const unsigned grid = grid_for(c, r->rows, BLOCK * 16);
+            pub = publish_by(c, grid, oa->p, 2);
+            cols_or_filter_k<<<grid, BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), r->cols[1]->as<uint32_t>(), r->rows, oa->as<unsigned long long>(),
                                                                                          fuse ? fcol : -1, fval, fuse ? filtered->buf->as<uint64_t>() : nullptr,
-                                                                                         oa->as<unsigned long long>() + 1);
+                                                                                         oa->as<unsigned long long>() + 1, pub);
         } else if (r->schema.arity == 2) {
             const bool vec = (((uintptr_t)r->cols[0]->p | (uintptr_t)r->cols[1]->p | (uintptr_t)b->p) & 15) == 0;
-            pack2_k<<<grid_for(c, r->rows, BLOCK * 4), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), r->cols[1]->as<uint32_t>(), materialize ? b->as<uint64_t>() : nullptr, r->rows,
+            const unsigned grid = grid_for(c, r->rows, BLOCK * 4);
+            pub = publish_by(c, grid, oa->p, 2);
+            pack2_k<<<grid, BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), r->cols[1]->as<uint32_t>(), materialize ? b->as<uint64_t>() : nullptr, r->rows,
                                                                               oa->as<unsigned long long>(), vec, fuse ? fcol : -1, fval,
-                                                                              fuse ? filtered->buf->as<uint64_t>() : nullptr, oa->as<unsigned long long>() + 1);
+                                                                              fuse ? filtered->buf->as<uint64_t>() : nullptr, oa->as<unsigned long long>() + 1, pub);
+        } else {
+            pub = publish_by(c, grid_for(c, r->rows), oa->p, 2);
+            pack1_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), b->as<uint64_t>(), r->rows, oa->as<unsigned long long>(), pub);
         }
-        else pack1_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), b->as<uint64_t>(), r->rows, oa->as<unsigned long long>());
         check_launch(c, "pack");
         unsigned long long h[2];
-        read_words(c, oa->p, 2, h);
+        read_published(c, pub, oa->p, 2, h);
         r->or_bound = h[0];
         if (fuse) {
             filtered->n = h[1];
@@ -430,19 +437,22 @@ void ops_pack_all(xlb_ctx* c, const std::vector<const xlb_rel*>& rels) {
         Buf bounds = make_buf(c, 8ull * k);
         CUDA_OK(set_async(c, bounds->p, 0, bounds->bytes));
         std::vector<Buf> out(k);
+        Publish pub;
         for (int i = 0; i < k; ++i) {
             const xlb_rel* r = todo[at + i];
+            const unsigned grid = grid_for(c, r->rows, r->schema.arity == 2 ? BLOCK * 4 : BLOCK);
+            if (i + 1 == k) pub = publish_by(c, grid, bounds->p, k);  // (the last one finds the others done)
             out[i] = make_buf(c, r->rows * 8);
             unsigned long long* bound = bounds->as<unsigned long long>() + i;
             prof_begin(c, "pack", r->rows * 16ull);
             if (r->schema.arity == 2) {
                 const bool vec = (((uintptr_t)r->cols[0]->p | (uintptr_t)r->cols[1]->p | (uintptr_t)out[i]->p) & 15) == 0;
-                pack2_k<<<grid_for(c, r->rows, BLOCK * 4), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), r->cols[1]->as<uint32_t>(), out[i]->as<uint64_t>(), r->rows, bound, vec);
-            } else pack1_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), out[i]->as<uint64_t>(), r->rows, bound);
+                pack2_k<<<grid, BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), r->cols[1]->as<uint32_t>(), out[i]->as<uint64_t>(), r->rows, bound, vec, -1, 0u, nullptr, nullptr, pub);
+            } else pack1_k<<<grid, BLOCK, 0, c->stream>>>(r->cols[0]->as<uint32_t>(), out[i]->as<uint64_t>(), r->rows, bound, pub);
             check_launch(c, "pack");
         }
         unsigned long long h[READ_WORDS_MAX];
-        read_words(c, bounds->p, k, h);
+        read_published(c, pub, bounds->p, k, h);
         for (int i = 0; i < k; ++i) {
             todo[at + i]->packed = out[i];
             todo[at + i]->or_bound = h[i];
@@ -635,14 +645,16 @@ static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64
     Buf gcnt = make_buf(c, groups * 4);
     Buf offs = make_buf(c, groups * 8);
     prof_begin(c, "dense_count", words * 4ull);
+    Publish pub;
     if (wide) {
         dense_count_wide_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), gcnt->as<uint32_t>(), groups, d.visited, d.touched);
         check_launch(c, "dense_count");
         exclusive_scan<LoadU32, uint64_t>(c, LoadU32{gcnt->as<uint32_t>()}, groups, offs->as<uint64_t>(), d.counts);
     } else if (groups <= (uint64_t)DENSE_FUSED_GROUPS) {
+        if (!known_total) pub = publish_by(c, 1, d.counts, 2);  // (its last block is one already)
         dense_count_scan_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, gcnt->as<uint32_t>(), groups, d.visited,
                                                                                                   offs->as<uint64_t>(), d.counts, (unsigned int*)(d.counts + 2), known_total != nullptr,
-                                                                                                  known_total ? *known_total : 0, c->d_status);
+                                                                                                  known_total ? *known_total : 0, c->d_status, pub);
         check_launch(c, "dense_count");
     } else {
         dense_count_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, gcnt->as<uint32_t>(), groups, d.visited);
@@ -650,7 +662,7 @@ static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64
         exclusive_scan<LoadU32, uint64_t>(c, LoadU32{gcnt->as<uint32_t>()}, groups, offs->as<uint64_t>(), d.counts);
     }
     unsigned long long both[2] = {known_total ? *known_total : 0ull, 0ull};
-    if (!known_total) read_words(c, d.counts, 2, both);
+    if (!known_total) read_published(c, pub, d.counts, 2, both);
     else if (wide || groups > (uint64_t)DENSE_FUSED_GROUPS) {
         verify_count_k<<<1, 1, 0, c->stream>>>(d.counts, *known_total, c->d_status);  // a mismatch surfaces as an error at the next status check
         check_launch(c, "verify_count");
@@ -665,12 +677,16 @@ static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64
     uint64_t* packed = cols ? nullptr : o.buf->as<uint64_t>();
     if (tot) {
         prof_begin(c, "dense_emit", words * 4ull + tot * 8ull);
+        const unsigned grid = (unsigned)((groups * 32 + BLOCK - 1) / BLOCK);
+        pub = Publish();
+        if (!wide) pub = publish_by(c, grid);
         if (wide)
             dense_emit_wide_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), offs->as<uint64_t>(), groups, d.lo_bits, packed,
                                                                                                     d.visited, tot, c->d_status, d.touched, c0, c1);
         else
-            dense_emit_k<<<(unsigned)((groups * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, offs->as<uint64_t>(), groups, d.lo_bits, packed, d.visited, tot, c->d_status, c0, c1);
+            dense_emit_k<<<grid, BLOCK, 0, c->stream>>>(d.bitmap->as<unsigned int>(), words, offs->as<uint64_t>(), groups, d.lo_bits, packed, d.visited, tot, c->d_status, c0, c1, pub);
         check_launch(c, "dense_emit");
+        status_published(c, pub);
     }
     return o;
 }
@@ -1161,8 +1177,9 @@ extern "C" xlb_status xlb_ctx_create(const xlb_config* cfg, xlb_ctx** out) {
         CUDA_OK(cudaHostAlloc((void**)&c->h_scalar, SCALAR_WORDS * 8, cudaHostAllocMapped));
         CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_scalar_dev, c->h_scalar, 0));
         memset(c->h_scalar, 0, SCALAR_WORDS * 8);
-        CUDA_OK(cudaMalloc(&c->d_status, sizeof(DevStatus) + 24));  // and behind it the count words of dense_state_out
-        CUDA_OK(cudaMemset(c->d_status, 0, sizeof(DevStatus) + 24));
+        CUDA_OK(cudaMalloc(&c->d_status, sizeof(DevStatus) + 24 + 8));  // and behind it the count words of dense_state_out, and Publish's counter
+        CUDA_OK(cudaMemset(c->d_status, 0, sizeof(DevStatus) + 24 + 8));
+        c->arrived = (unsigned*)((char*)c->d_status + sizeof(DevStatus) + 24);
         cudaDeviceProp prop;
         CUDA_OK(cudaGetDeviceProperties(&prop, dev));
         c->sm_count = prop.multiProcessorCount;

@@ -57,7 +57,8 @@ __global__ void __launch_bounds__(BLOCK) exists_build_k(KeyCols keys, uint64_t n
 // One bit per probe row (has a match == want), and for each tile of SCAN_TILE rows how many were selected before it.
 constexpr int QT_ROUNDS = SCAN_TILE / BLOCK;
 __global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t n, KeyCols keys, const unsigned int* __restrict__ rep, uint64_t mask, bool want,
-                                                       unsigned int* __restrict__ bits, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total) {
+                                                       unsigned int* __restrict__ bits, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total,
+                                                       const Publish pub) {
     __shared__ uint32_t sm[33];
     __shared__ unsigned tile_s;
     const unsigned tile = tiles.take(tile_s);
@@ -95,9 +96,10 @@ __global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t 
     uint32_t tot;
     block_exclusive_scan<uint32_t>(lane_id() == 0 ? cnt : 0u, &tot, sm);
     if (threadIdx.x < 32) leave_tile(tiles, tile, tot, tile_offs, total);
+    publish_last(pub);
 }
 // The selected rows, all columns, in order.
-__global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned int* __restrict__ bits, uint64_t n, const uint64_t* __restrict__ tile_offs) {
+__global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned int* __restrict__ bits, uint64_t n, const uint64_t* __restrict__ tile_offs, const Publish pub) {
     __shared__ uint32_t sm[33];
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS;
     unsigned w[QT_ROUNDS];
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned
         }
         pos += __popc(w[r]);
     }
+    publish_last(pub);
 }
 
 // ---- inner join: the build rows grouped by key
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(BLOCK) group_order_k(const unsigned int* __res
 }
 // What each probe row meets (start << 32 | rows) and how many outputs come before it: in its tile, and before the tile.
 __global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n, const ulonglong2* __restrict__ table, uint64_t mask, uint64_t* __restrict__ match,
-                                                     uint32_t* __restrict__ in_tile, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total) {
+                                                     uint32_t* __restrict__ in_tile, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total, const Publish pub) {
     __shared__ uint64_t sm[33];
     __shared__ unsigned tile_s;
     const unsigned tile = tiles.take(tile_s), lane = lane_id();
@@ -241,6 +244,7 @@ __global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n,
         }
         at += __shfl_sync(FULL, run, 31);
     }
+    publish_last(pub);
 }
 struct OutputsBefore {
     const uint64_t* tile;
@@ -250,7 +254,7 @@ struct OutputsBefore {
 // Load-balanced output of an inner join (the scheme of expand_k), all columns of both sides written
 // at once: the pairs of row numbers never touch memory.
 __global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict__ match, const OutputsBefore off, uint64_t nrows, uint64_t total, const uint32_t* __restrict__ rows,
-                                                    Cols cols) {
+                                                    Cols cols, const Publish pub) {
     __shared__ unsigned rel[EX_TILE + 2];
     __shared__ uint64_t row_s[2];
     const uint64_t o0 = (uint64_t)blockIdx.x * EX_TILE, o1 = o0 + EX_TILE < total ? o0 + EX_TILE : total;
@@ -289,6 +293,7 @@ __global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict_
         const uint64_t l = r0 + lo - 1, r = rows[(match[l] >> 32) + j];
         for (int k = 0; k < cols.n; ++k) copy_value(cols, k, k < cols.left ? l : r, o0 + t);
     }
+    publish_last(pub);
 }
 
 // ---- group-by over a small domain of keys: tables indexed by the key itself
@@ -302,10 +307,11 @@ struct GroupKey {
         return cols.c1 ? (uint32_t)(((k >> 32) << lo_bits) | (k & 0xFFFFFFFFull)) : (uint32_t)k;
     }
 };
-__global__ void __launch_bounds__(BLOCK) group_bound_k(KeyCols keys, uint64_t n, unsigned long long* __restrict__ bound) {
+__global__ void __launch_bounds__(BLOCK) group_bound_k(KeyCols keys, uint64_t n, unsigned long long* __restrict__ bound, const Publish pub) {
     uint64_t o = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) o |= keys(i);
     block_or(o, bound);
+    publish_last(pub);
 }
 __global__ void __launch_bounds__(BLOCK) group_rows_k(GroupKey key, uint64_t n, unsigned int* __restrict__ count) {
     __shared__ uint32_t skey[DX_SLOTS], scnt[DX_SLOTS];
@@ -331,7 +337,7 @@ __global__ void __launch_bounds__(BLOCK) group_rows_k(GroupKey key, uint64_t n, 
     }
 }
 __global__ void __launch_bounds__(BLOCK) group_tiles_k(const unsigned int* __restrict__ count, uint64_t domain, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total,
-                                                      unsigned long long* __restrict__ longest) {
+                                                      unsigned long long* __restrict__ longest, const Publish pub) {
     __shared__ uint32_t sm[33];
     __shared__ unsigned tile_s;
     const unsigned tile = tiles.take(tile_s);
@@ -349,6 +355,7 @@ __global__ void __launch_bounds__(BLOCK) group_tiles_k(const unsigned int* __res
     uint32_t tot;
     block_exclusive_scan<uint32_t>(groups, &tot, sm);
     if (threadIdx.x < 32) leave_tile(tiles, tile, tot, tile_offs, total);
+    publish_last(pub);
 }
 struct Aggs {
     const void* val[XLB_MAX_ARITY];
@@ -373,7 +380,7 @@ __global__ void __launch_bounds__(BLOCK) group_add_k(GroupKey key, uint64_t n, A
     }
 }
 __global__ void __launch_bounds__(BLOCK) group_emit_k(const unsigned int* __restrict__ count, uint64_t domain, const uint64_t* __restrict__ tile_offs, Aggs a, int lo_bits, int w0, void* key0,
-                                                     uint32_t* key1) {
+                                                     uint32_t* key1, const Publish pub) {
     __shared__ uint32_t sm[33];
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_IPT;
     uint32_t c[SCAN_IPT], groups = 0;
@@ -399,6 +406,7 @@ __global__ void __launch_bounds__(BLOCK) group_emit_k(const unsigned int* __rest
         }
         ++pos;
     }
+    publish_last(pub);
 }
 
 KeyCols key_cols(const xlb_rel* r, const uint32_t* keys, uint32_t nk) {
@@ -430,6 +438,8 @@ struct Sweep {
             leave_at = counts->as<uint64_t>();
         }
     }
+    // For the kernel to leave `words` words from `from` (the total among them) when it places its tiles itself.
+    Publish publish(const void* from, int words) const { return counts ? Publish() : publish_by(c, n, from, words); }
     void finish() {
         if (counts) exclusive_scan<LoadU64, uint64_t>(c, LoadU64{counts->as<uint64_t>()}, n, offs, total);
     }
@@ -459,11 +469,12 @@ xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint
     uint64_t* total = offs->as<uint64_t>() + tiles;
     Sweep sweep(c, tiles, rep->as<uint64_t>() + cap / 2, offs->as<uint64_t>(), total);
     prof_begin(c, "hash_probe", n * 12ull);
-    exists_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, n, build, rep->as<unsigned int>(), cap - 1, want, bits->as<unsigned int>(), sweep.tiles, sweep.leave_at, total);
+    const Publish pub = sweep.publish(total, 1);
+    exists_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, n, build, rep->as<unsigned int>(), cap - 1, want, bits->as<unsigned int>(), sweep.tiles, sweep.leave_at, total, pub);
     check_launch(c, "hash_probe");
     sweep.finish();
     unsigned long long m;
-    read_words(c, total, 1, &m);
+    read_published(c, pub, total, 1, &m);
     std::unique_ptr<xlb_rel> o(new xlb_rel);
     o->ctx = c;
     o->schema = l->schema;
@@ -472,8 +483,10 @@ xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint
     add_columns(c, o.get(), cols, l, m);
     if (m) {
         prof_begin(c, "select_rows", 0);
-        select_rows_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(cols, bits->as<unsigned int>(), n, offs->as<uint64_t>());
+        const Publish last = publish_by(c, tiles);
+        select_rows_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(cols, bits->as<unsigned int>(), n, offs->as<uint64_t>(), last);
         check_launch(c, "select_rows");
+        status_published(c, last);
     }
     return o.release();
 }
@@ -504,11 +517,12 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     Buf match = make_buf(c, l->rows * 8), in_tile = make_buf(c, l->rows * 4), offs = make_buf(c, tiles * 8);
     Sweep sweep(c, tiles, words + 3, offs->as<uint64_t>(), words);
     prof_begin(c, "hash_probe", l->rows * 32ull);
-    join_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, l->rows, table->as<ulonglong2>(), cap - 1, match->as<uint64_t>(), in_tile->as<uint32_t>(), sweep.tiles, sweep.leave_at, words);
+    const Publish pub = sweep.publish(words, 2);
+    join_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, l->rows, table->as<ulonglong2>(), cap - 1, match->as<uint64_t>(), in_tile->as<uint32_t>(), sweep.tiles, sweep.leave_at, words, pub);
     check_launch(c, "hash_probe");
     sweep.finish();
     unsigned long long w[2];
-    read_words(c, words, 2, w);
+    read_published(c, pub, words, 2, w);
     if (w[1]) return nullptr;
     std::unique_ptr<xlb_rel> o(new xlb_rel);
     o->ctx = c;
@@ -520,8 +534,10 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     add_columns(c, o.get(), cols, r, w[0]);
     if (w[0]) {
         prof_begin(c, "join_emit", 0);
-        join_emit_k<<<(unsigned)((w[0] + EX_TILE - 1) / EX_TILE), BLOCK, 0, c->stream>>>(match->as<uint64_t>(), OutputsBefore{offs->as<uint64_t>(), in_tile->as<uint32_t>()}, l->rows, w[0], rows->as<uint32_t>(), cols);
+        const Publish last = publish_by(c, (w[0] + EX_TILE - 1) / EX_TILE);
+        join_emit_k<<<(unsigned)((w[0] + EX_TILE - 1) / EX_TILE), BLOCK, 0, c->stream>>>(match->as<uint64_t>(), OutputsBefore{offs->as<uint64_t>(), in_tile->as<uint32_t>()}, l->rows, w[0], rows->as<uint32_t>(), cols, last);
         check_launch(c, "join_emit");
+        status_published(c, last);
     }
     return o.release();
 }
@@ -538,10 +554,12 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
     Buf words = make_buf(c, 24);  // [0] key bound, [1] groups, [2] rows of the largest
     CUDA_OK(set_async(c, words->p, 0, 24));
     prof_begin(c, "group_bound", 0);
-    group_bound_k<<<grid_for(c, n, BLOCK * 4), BLOCK, 0, c->stream>>>(key.cols, n, words->as<unsigned long long>());
+    const unsigned bound_grid = std::min(grid_for(c, n, BLOCK * 4), PUBLISH_BLOCKS_MAX);
+    const Publish bound_pub = publish_by(c, bound_grid, words->p, 1);
+    group_bound_k<<<bound_grid, BLOCK, 0, c->stream>>>(key.cols, n, words->as<unsigned long long>(), bound_pub);
     check_launch(c, "group_bound");
     unsigned long long w[2];
-    read_words(c, words->p, 1, w);
+    read_published(c, bound_pub, words->p, 1, w);
     int bits = bit_length(w[0]);
     if (nk == 2) {
         key.lo_bits = std::max(bit_length(w[0] & 0xFFFFFFFFull), 1);
@@ -557,10 +575,11 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
     check_launch(c, "group_rows");
     Sweep sweep(c, tiles, count->as<uint64_t>() + (domain * 4 + 7) / 8, offs->as<uint64_t>(), words->as<uint64_t>() + 1);
     prof_begin(c, "group_tiles", domain * 4ull);
-    group_tiles_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(count->as<unsigned int>(), domain, sweep.tiles, sweep.leave_at, words->as<uint64_t>() + 1, words->as<unsigned long long>() + 2);
+    const Publish pub = sweep.publish(words->as<uint64_t>() + 1, 2);
+    group_tiles_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(count->as<unsigned int>(), domain, sweep.tiles, sweep.leave_at, words->as<uint64_t>() + 1, words->as<unsigned long long>() + 2, pub);
     check_launch(c, "group_tiles");
     sweep.finish();
-    read_words(c, words->as<uint64_t>() + 1, 2, w);
+    read_published(c, pub, words->as<uint64_t>() + 1, 2, w);
     const uint64_t m = w[0];
     uint32_t tables = 0;
     for (uint32_t a = 0; a < na; ++a) tables += agg_ops[a] != XLB_AGG_COUNT;
@@ -598,8 +617,10 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
         check_launch(c, "groupby_reduce");
     }
     prof_begin(c, "group_emit", 0);
+    const Publish last = publish_by(c, tiles);
     group_emit_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(count->as<unsigned int>(), domain, offs->as<uint64_t>(), ag, key.lo_bits, (int)type_width(os.types[0]), o->cols[0]->p,
-                                                          nk == 2 ? o->cols[1]->as<uint32_t>() : nullptr);
+                                                          nk == 2 ? o->cols[1]->as<uint32_t>() : nullptr, last);
     check_launch(c, "group_emit");
+    status_published(c, last);
     return o.release();
 }

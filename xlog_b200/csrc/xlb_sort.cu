@@ -86,7 +86,7 @@ __device__ __forceinline__ void range_of(const KeyPart& p, uint64_t n, uint64_t&
         b = min(b, ~v);
     }
 }
-__global__ void __launch_bounds__(BLOCK) key_range_k(const KeyWord w, uint64_t n, unsigned long long* __restrict__ least) {
+__global__ void __launch_bounds__(BLOCK) key_range_k(const KeyWord w, uint64_t n, unsigned long long* __restrict__ least, const Publish pub) {
     __shared__ unsigned long long s[2];
     for (int k = 0; k < w.n; ++k) {
         uint64_t a = ~0ull, b = ~0ull;
@@ -106,15 +106,17 @@ __global__ void __launch_bounds__(BLOCK) key_range_k(const KeyWord w, uint64_t n
         __syncthreads();
         if (threadIdx.x < 2) atomicMin(&least[2 * k + threadIdx.x], s[threadIdx.x]);
     }
+    publish_last(pub);
 }
 __global__ void __launch_bounds__(BLOCK) key_word_k(const KeyWord w, const uint32_t* __restrict__ rows, uint64_t* __restrict__ out, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) out[i] = w(rows ? rows[i] : i);
 }
-__global__ void __launch_bounds__(BLOCK) rows_out_k(const OutCols out, const uint64_t* __restrict__ words, const uint32_t* __restrict__ rows, uint64_t row_mask, uint64_t n) {
+__global__ void __launch_bounds__(BLOCK) rows_out_k(const OutCols out, const uint64_t* __restrict__ words, const uint32_t* __restrict__ rows, uint64_t row_mask, uint64_t n, const Publish pub) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
         const uint64_t w = words ? words[i] : 0;
         out(i, w, rows ? rows[i] : row_mask ? (uint32_t)(w & row_mask) : (uint32_t)i);
     }
+    publish_last(pub);
 }
 
 // a few thousand rows: words made, sorted and (the last one) turned into columns in one launch each
@@ -186,10 +188,12 @@ void order_rows(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_t nk,
         Buf least = make_buf(c, 16 * XLB_MAX_ARITY);
         CUDA_OK(set_async(c, least->p, 0xFF, 16 * XLB_MAX_ARITY));
         prof_begin(c, "key_range", n * 8ull * all.n);
-        key_range_k<<<std::min(grid_for(c, n, BLOCK * 8), 6u * c->sm_count), BLOCK, 0, c->stream>>>(all, n, least->as<unsigned long long>());
+        const unsigned grid = std::min(grid_for(c, n, BLOCK * 8), 6u * c->sm_count);
+        const Publish pub = publish_by(c, grid, least->p, 2 * all.n);
+        key_range_k<<<grid, BLOCK, 0, c->stream>>>(all, n, least->as<unsigned long long>(), pub);
         check_launch(c, "key_range");
         unsigned long long range[2 * XLB_MAX_ARITY];
-        read_words(c, least->p, 2 * all.n, range);
+        read_published(c, pub, least->p, 2 * all.n, range);
         words = words_of(all, range);
     }
     bool rows_wanted = words.size() > 1;
@@ -244,8 +248,10 @@ void order_rows(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_t nk,
         radix_sort(c, last, rows_wanted && !row_bits ? &rows : nullptr, n, 0xFFu, ~0ull, false, &digits);
     }
     prof_begin(c, "rows_out", 0);
-    rows_out_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(out, last ? last->as<uint64_t>() : nullptr, rows ? rows->as<uint32_t>() : nullptr, row_mask, n);
+    const Publish pub = publish_by(c, grid_for(c, n));
+    rows_out_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(out, last ? last->as<uint64_t>() : nullptr, rows ? rows->as<uint32_t>() : nullptr, row_mask, n, pub);
     check_launch(c, "rows_out");
+    status_published(c, pub);
 }
 
 }  // namespace

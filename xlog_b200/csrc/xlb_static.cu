@@ -101,7 +101,7 @@ extern "C" xlb_status xlb_dedup_sorted_u64_static(const uint64_t* d_sorted, uint
         EmitKey emit{d_sorted, d_unique};
         uint64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
         if (ntiles == 1) {
-            select_write_k<PredHead, EmitKey><<<1, BLOCK, 0, stream>>>(pred, emit, n, SelectTiles(), d_count);
+            select_write_k<PredHead, EmitKey><<<1, BLOCK, 0, stream>>>(pred, emit, n, SelectTiles(), d_count, Publish());
         } else {
             // every scratch word that is read below is written first by these launches, so nothing
             // left behind by an earlier call is ever observed
@@ -118,7 +118,7 @@ extern "C" xlb_status xlb_dedup_sorted_u64_static(const uint64_t* d_sorted, uint
             SelectTiles tiles;
             tiles.n = (unsigned)ntiles;
             tiles.known = offs;
-            select_write_k<PredHead, EmitKey><<<(unsigned)ntiles, BLOCK, 0, stream>>>(pred, emit, n, tiles, d_count);
+            select_write_k<PredHead, EmitKey><<<(unsigned)ntiles, BLOCK, 0, stream>>>(pred, emit, n, tiles, d_count, Publish());
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "kernel launch", e);
