@@ -64,6 +64,25 @@ def test_sort_rows(prov, n, kinds, keys):
         assert g.tobytes() == c[order].tobytes()
 
 
+@pytest.mark.parametrize("n", [8193, 65536, 65537, 300007])
+@pytest.mark.parametrize("kind", ["spread", "run33", "run34", "run_of_equal", "few"])
+def test_rows_of_one_prefix(prov, n, kind):
+    """Sorted by the highest bits, the rest put in order afterwards: prefixes of a few rows, of as many as
+    that is done for, of more, and values that are too few for it."""
+    rng = np.random.default_rng(n)
+    key = rng.integers(0, 1 << 56, n, dtype=np.uint64)
+    k = {"run33": 33, "run34": 34, "run_of_equal": 500}.get(kind, 0)
+    if k:  # so many rows next to each other in the order, below the bits sorted by
+        key[rng.choice(n, k, replace=False)] = np.uint64(123 << 40) + (np.zeros(k, np.uint64) if kind == "run_of_equal" else rng.integers(0, 1 << 10, k, dtype=np.uint64))
+    if kind == "few":
+        key = key[rng.integers(0, 50, n)]
+    cols = [key, np.arange(n, dtype=np.uint32)]
+    got = prov.download(prov.sort(prov.create_buffer_from_slices(cols), [0]))
+    order = np.argsort(key, kind="stable")
+    for g, c in zip(got, cols):
+        assert np.array_equal(g, c[order])
+
+
 @pytest.mark.parametrize("bits", [(1, 1), (7, 9), (12, 12), (13, 20), (32, 3), (3, 32), (32, 32)])
 @pytest.mark.parametrize("n", [8192, 8193, 100001])
 def test_digits_across_the_halves_of_a_pair(prov, bits, n):

@@ -111,12 +111,55 @@ __global__ void __launch_bounds__(BLOCK) key_range_k(const KeyWord w, uint64_t n
 __global__ void __launch_bounds__(BLOCK) key_word_k(const KeyWord w, const uint32_t* __restrict__ rows, uint64_t* __restrict__ out, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) out[i] = w(rows ? rows[i] : i);
 }
-__global__ void __launch_bounds__(BLOCK) rows_out_k(const OutCols out, const uint64_t* __restrict__ words, const uint32_t* __restrict__ rows, uint64_t row_mask, uint64_t n, const Publish pub) {
+// Words that were sorted by their bits from `mend` on only: each row finds the others of its prefix next to
+// it and counts those that come before it.  *unmended: a prefix has more rows than that is done for.
+constexpr unsigned MEND_MAX = 32;
+template <bool MEND>
+__global__ void __launch_bounds__(BLOCK) rows_out_k(const OutCols out, const uint64_t* __restrict__ words, const uint32_t* __restrict__ rows, uint64_t row_mask, uint64_t n, int mend,
+                                                    unsigned long long* __restrict__ unmended, const Publish pub) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
         const uint64_t w = words ? words[i] : 0;
-        out(i, w, rows ? rows[i] : row_mask ? (uint32_t)(w & row_mask) : (uint32_t)i);
+        uint64_t to = i;
+        if (MEND) {
+            const uint64_t prefix = w >> mend;
+            unsigned left = 0, right = 0;
+            for (; left < MEND_MAX && left < i; ++left) {
+                const uint64_t v = words[i - left - 1];
+                if (v >> mend != prefix) break;
+                if (v > w) --to;
+            }
+            for (; right < MEND_MAX && i + right + 1 < n; ++right) {
+                const uint64_t v = words[i + right + 1];
+                if (v >> mend != prefix) break;
+                if (v < w) ++to;
+            }
+            if (left == MEND_MAX || right == MEND_MAX) *unmended = 1;
+        }
+        out(to, w, rows ? rows[i] : row_mask ? (uint32_t)(w & row_mask) : (uint32_t)i);
     }
     publish_last(pub);
+}
+// How often rows picked evenly meet one with the same bits from `mend` on.
+constexpr unsigned SAMPLE = 2048, SAMPLE_SLOTS = 4096, SAMPLE_MEET = SAMPLE / 16;
+__global__ void __launch_bounds__(1024) prefix_sample_k(const KeyWord w, uint64_t n, int mend, unsigned long long* __restrict__ met, const Publish pub) {
+    __shared__ unsigned long long table[SAMPLE_SLOTS];
+    __shared__ unsigned met_s;
+    for (unsigned i = threadIdx.x; i < SAMPLE_SLOTS; i += 1024) table[i] = ~0ull;  // (no prefix: mend > 0)
+    if (threadIdx.x == 0) met_s = 0;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < SAMPLE; i += 1024) {
+        const unsigned long long prefix = w(i * n / SAMPLE) >> mend;
+        unsigned h = (unsigned)mix64(prefix) & (SAMPLE_SLOTS - 1);
+        for (unsigned probe = 0; probe < SAMPLE_SLOTS; ++probe) {
+            const unsigned long long cur = atomicCAS(&table[h], ~0ull, prefix);
+            if (cur == prefix) atomicAdd(&met_s, 1u);
+            if (cur == ~0ull || cur == prefix) break;
+            h = (h + 1) & (SAMPLE_SLOTS - 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *met = met_s;
+    publish_now(pub);
 }
 
 // a few thousand rows: words made, sorted and (the last one) turned into columns in one launch each
@@ -136,6 +179,8 @@ struct StoreOut {
     OutCols out;
     __device__ __forceinline__ void operator()(unsigned i, uint64_t key, uint32_t val) const { out(i, key, val); }
 };
+
+int bits_of(uint64_t v) { return v ? 64 - __builtin_clzll(v) : 1; }
 
 // The key columns cut into words, least significant word first; a column that came before is no key again.
 // `range`: least and complement of the greatest image of each part, or null: all bits of the type.
@@ -229,27 +274,57 @@ void order_rows(xlb_ctx* c, const xlb_rel* r, const uint32_t* keys, uint32_t nk,
     }
     Buf last;
     uint64_t row_mask = 0;
-    for (size_t q = 0; q < words.size(); ++q) {
-        KeyWord& w = words[q];
-        int row_bits = 0;
-        if (words.size() == 1 && rows_wanted) {
-            row_bits = n > 1 ? 64 - __builtin_clzll(n - 1) : 1;
-            if (w.bits + row_bits > 64) row_bits = 0;
-            w.with_row = row_bits > 0;
-            row_mask = (1ull << row_bits) - 1;
-            for (int k = 0; k < w.n; ++k) w.p[k].shift = (unsigned char)(w.p[k].shift + row_bits);
-            for (int k = 0; k < out.n; ++k) out.c[k].shift = (unsigned char)(out.c[k].shift + row_bits);
-        }
+    int row_bits = 0;
+    if (words.size() == 1) {
+        KeyWord& w = words[0];
+        row_bits = rows_wanted ? bits_of(n - 1) : 0;
+        if (w.bits + row_bits > 64) row_bits = 0;
+        w.with_row = row_bits > 0;
+        row_mask = (1ull << row_bits) - 1;
+        for (int k = 0; k < w.n; ++k) w.p[k].shift = (unsigned char)(w.p[k].shift + row_bits);
+        for (int k = 0; k < out.n; ++k) out.c[k].shift = (unsigned char)(out.c[k].shift + row_bits);
+    }
+    const auto sort_word = [&](const KeyWord& w, int from, int bits) {
         last = make_buf(c, n * 8);
         prof_begin(c, "key_word", n * 8ull);
         key_word_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(w, rows ? rows->as<uint32_t>() : nullptr, last->as<uint64_t>(), n);
         check_launch(c, "key_word");
-        const Digits digits = run_of_digits(row_bits, w.bits);
+        const Digits digits = run_of_digits(from, bits);
         radix_sort(c, last, rows_wanted && !row_bits ? &rows : nullptr, n, 0xFFu, ~0ull, false, &digits);
+    };
+    const unsigned grid = grid_for(c, n);
+    // Many bits and values spread over them: the highest log2(n) bits tell nearly all rows apart, so only
+    // they are sorted by, and rows_out puts the few of one prefix in order.  A sample says whether they do
+    // (ids that are few or lie close together do not); a prefix of many rows that it missed costs the
+    // passes made so far.  (4 M rows of 59 bits: three passes of 50 us and not eight.)
+    if (words.size() == 1) {
+        const KeyWord& w = words[0];
+        const int high = (bits_of(n - 1) + 7) / 8 * 8, mend = row_bits + w.bits - high;
+        if ((w.bits + 7) / 8 > high / 8 + 1) {
+            Buf flags = make_buf(c, 16);
+            CUDA_OK(set_async(c, flags->p, 0, 16));
+            unsigned long long *met = flags->as<unsigned long long>(), *unmended = met + 1, h;
+            const Publish asked = publish_by(c, 1, met, 1);
+            prof_begin(c, "prefix_sample", 0);
+            prefix_sample_k<<<1, 1024, 0, c->stream>>>(w, n, mend, met, asked);
+            check_launch(c, "prefix_sample");
+            read_published(c, asked, met, 1, &h);
+            if (h <= SAMPLE_MEET) {
+                sort_word(w, mend, high);
+                const Publish pub = publish_by(c, grid, unmended, 1);
+                prof_begin(c, "rows_out", 0);
+                rows_out_k<true><<<grid, BLOCK, 0, c->stream>>>(out, last->as<uint64_t>(), rows ? rows->as<uint32_t>() : nullptr, row_mask, n, mend, unmended, pub);
+                check_launch(c, "rows_out");
+                read_published(c, pub, unmended, 1, &h);
+                if (!h) return;
+                rows.reset();
+            }
+        }
     }
+    for (const KeyWord& w : words) sort_word(w, row_bits, w.bits);
+    const Publish pub = publish_by(c, grid);
     prof_begin(c, "rows_out", 0);
-    const Publish pub = publish_by(c, grid_for(c, n));
-    rows_out_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(out, last ? last->as<uint64_t>() : nullptr, rows ? rows->as<uint32_t>() : nullptr, row_mask, n, pub);
+    rows_out_k<false><<<grid, BLOCK, 0, c->stream>>>(out, last ? last->as<uint64_t>() : nullptr, rows ? rows->as<uint32_t>() : nullptr, row_mask, n, 0, nullptr, pub);
     check_launch(c, "rows_out");
     status_published(c, pub);
 }
