@@ -1577,6 +1577,23 @@ static __global__ void __launch_bounds__(BLOCK) dense_emit_k(const unsigned int*
         if (lane >= (unsigned)d) incl += o;
     }
     uint64_t pos = g < groups ? group_offs[g] + (incl - cnt) : 0;
+    if (__reduce_max_sync(FULL, cnt) >= 12) {
+        // Dense: the warp walks its words in order and lane b writes bit b, so that a word's tuples go out side
+        // by side (each lane its own word: 56 us for 4 M tuples, against 16).
+        uint64_t base = __shfl_sync(FULL, pos, 0);
+        if (base + __shfl_sync(FULL, incl, 31) > cap) {  // more bits than the rows the host sized the output for
+            if (lane == 0) set_status(st, XLB_ERR_CAPACITY, 8, base);
+            m = 0;
+        }
+        const uint64_t first = w - lane;
+#pragma unroll 4
+        for (int owner = 0; owner < 32; ++owner) {
+            const unsigned word = __shfl_sync(FULL, m, owner);
+            if ((word >> lane) & 1u) dense_put(((first + owner) << 5) | lane, lo_bits, lo_mask, base + __popc(word & lanemask_lt()), out, out0, out1);
+            base += __popc(word);
+        }
+        m = 0;
+    }
     while (m) {
         unsigned b = __ffs(m) - 1;
         m &= m - 1;
