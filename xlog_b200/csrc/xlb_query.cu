@@ -29,10 +29,25 @@ struct Cols {  // columns in and out, with the side a joined column comes from
     int width[XLB_MAX_ARITY];
     int n, left;  // the first `left` columns come from the left side
 };
-__device__ __forceinline__ void copy_value(const Cols& c, int k, uint64_t from, uint64_t to) {
-    if (c.width[k] == 4) ((uint32_t*)c.out[k])[to] = __ldg((const uint32_t*)c.in[k] + from);
-    else if (c.width[k] == 8) ((unsigned long long*)c.out[k])[to] = __ldg((const unsigned long long*)c.in[k] + from);
-    else ((uint8_t*)c.out[k])[to] = __ldg((const uint8_t*)c.in[k] + from);
+// A row out: all columns are read before any is written, so that a row costs one trip and not one a column
+// (joined rows of five columns, 2.6 M of them: 80 us one by one, against 71; a selection of three columns 41, against 34).
+__device__ __forceinline__ void copy_row(const Cols& c, uint64_t left, uint64_t right, uint64_t to) {
+    unsigned long long v[XLB_MAX_ARITY];
+#pragma unroll
+    for (int k = 0; k < (int)XLB_MAX_ARITY; ++k) {
+        if (k >= c.n) break;
+        const uint64_t from = k < c.left ? left : right;
+        if (c.width[k] == 4) v[k] = __ldg((const uint32_t*)c.in[k] + from);
+        else if (c.width[k] == 8) v[k] = __ldg((const unsigned long long*)c.in[k] + from);
+        else v[k] = __ldg((const uint8_t*)c.in[k] + from);
+    }
+#pragma unroll
+    for (int k = 0; k < (int)XLB_MAX_ARITY; ++k) {
+        if (k >= c.n) break;
+        if (c.width[k] == 4) ((uint32_t*)c.out[k])[to] = (uint32_t)v[k];
+        else if (c.width[k] == 8) ((unsigned long long*)c.out[k])[to] = v[k];
+        else ((uint8_t*)c.out[k])[to] = (uint8_t)v[k];
+    }
 }
 
 // ---- keys of the build side: open addressing, a slot names the first row (plus one) that brought its key
@@ -72,21 +87,25 @@ __global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t 
         key[r] = i < n ? probe(i) : 0;
     }
 #pragma unroll
-    for (int r = 0; r < QT_ROUNDS; ++r) cur[r] = __ldg(&rep[mix64(key[r]) & mask]);
+    for (int r = 0; r < QT_ROUNDS; ++r) cur[r] = base + r * 32 + lane_id() < n ? __ldg(&rep[mix64(key[r]) & mask]) : 0u;
+    unsigned same = 0;  // (rounds whose first slot holds the key: all looked at together, 4 M probes 83 us -> 71)
+#pragma unroll
+    for (int r = 0; r < QT_ROUNDS; ++r)
+        if (cur[r] && keys(cur[r] - 1) == key[r]) same |= 1u << r;
 #pragma unroll
     for (int r = 0; r < QT_ROUNDS; ++r) {
         const uint64_t i = base + r * 32 + lane_id();
-        bool found = false;
-        if (i < n && cur[r]) {
+        bool found = (same >> r) & 1u;
+        if (cur[r] && !found) {
             uint64_t h = mix64(key[r]) & mask;
-            unsigned c = cur[r];
-            for (uint64_t p = 0; p <= mask && c; ++p) {  // bounded by the table size
+            for (uint64_t p = 0; p < mask; ++p) {  // bounded by the table size
+                h = (h + 1) & mask;
+                const unsigned c = __ldg(&rep[h]);
+                if (!c) break;
                 if (keys(c - 1) == key[r]) {
                     found = true;
                     break;
                 }
-                h = (h + 1) & mask;
-                c = __ldg(&rep[h]);
             }
         }
         const unsigned b = __ballot_sync(FULL, i < n && found == want);
@@ -115,7 +134,7 @@ __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned
     for (int r = 0; r < QT_ROUNDS; ++r) {
         if ((w[r] >> lane_id()) & 1u) {
             const uint64_t to = pos + __popc(w[r] & lanemask_lt());
-            for (int k = 0; k < cols.n; ++k) copy_value(cols, k, base + r * 32 + lane_id(), to);
+            copy_row(cols, base + r * 32 + lane_id(), base + r * 32 + lane_id(), to);
         }
         pos += __popc(w[r]);
     }
@@ -167,37 +186,49 @@ __global__ void __launch_bounds__(BLOCK) group_fill_k(const uint2* __restrict__ 
         rows[(uint32_t)(table[p.x].y >> 32) + p.y] = (uint32_t)i;
     }
 }
+// Four slots a thread at a time: a slot is a chain of three loads (60 us one at a time for 4 M slots, against 50).
 __global__ void __launch_bounds__(BLOCK) group_order_k(const unsigned int* __restrict__ count, const ulonglong2* __restrict__ table, uint64_t cap, uint32_t* __restrict__ rows,
                                                       unsigned int* __restrict__ too_long) {
-    for (uint64_t h = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; h < cap; h += (uint64_t)gridDim.x * BLOCK) {
-        const unsigned len = count[h];
-        if (len < 2) continue;
-        if (len > JOIN_GROUP_MAX) {
-            *too_long = 1;
-            continue;
-        }
-        const unsigned at = (unsigned)(table[h].y >> 32);
-        if (len <= 4) {  // most groups: read at once, placed by rank (row numbers differ)
-            uint32_t v[4];
+    constexpr int S = 4, SHORT = 4;
+    const uint64_t step = (uint64_t)gridDim.x * BLOCK;
+    for (uint64_t h0 = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; h0 < cap; h0 += S * step) {
+        unsigned len[S], at[S];
+        uint32_t v[S][SHORT];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) v[k] = k < (int)len ? rows[at + k] : 0xFFFFFFFFu;
+        for (int s = 0; s < S; ++s) len[s] = h0 + s * step < cap ? count[h0 + s * step] : 0u;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                unsigned rank = 0;
+        for (int s = 0; s < S; ++s) at[s] = len[s] > 1 ? (unsigned)(table[h0 + s * step].y >> 32) : 0u;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) rank += q < (int)len && v[q] < v[k];
-                if (k < (int)len) rows[at + rank] = v[k];
+        for (int s = 0; s < S; ++s)
+#pragma unroll
+            for (int k = 0; k < SHORT; ++k) v[s][k] = len[s] > 1 && len[s] <= SHORT && k < (int)len[s] ? rows[at[s] + k] : 0xFFFFFFFFu;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            if (len[s] < 2) continue;
+            if (len[s] <= SHORT) {  // most groups: placed by rank (row numbers differ)
+#pragma unroll
+                for (int k = 0; k < SHORT; ++k) {
+                    unsigned rank = 0;
+#pragma unroll
+                    for (int q = 0; q < SHORT; ++q) rank += v[s][q] < v[s][k];  // (what is past the end is above all)
+                    if (k < (int)len[s]) rows[at[s] + rank] = v[s][k];
+                }
+                continue;
             }
-            continue;
-        }
-        for (unsigned a = 1; a < len; ++a) {  // insertion sort in place
-            const uint32_t v = rows[at + a];
-            unsigned b = a;
-            while (b && rows[at + b - 1] > v) {
-                rows[at + b] = rows[at + b - 1];
-                --b;
+            if (len[s] > JOIN_GROUP_MAX) {
+                *too_long = 1;
+                continue;
             }
-            rows[at + b] = v;
+            uint32_t* g = rows + at[s];
+            for (unsigned a = 1; a < len[s]; ++a) {  // insertion sort in place
+                const uint32_t x = g[a];
+                unsigned b = a;
+                while (b && g[b - 1] > x) {
+                    g[b] = g[b - 1];
+                    --b;
+                }
+                g[b] = x;
+            }
         }
     }
 }
@@ -252,46 +283,66 @@ struct OutputsBefore {
     __device__ __forceinline__ uint64_t operator[](uint64_t row) const { return tile[row / SCAN_TILE] + in_tile[row]; }
 };
 // Load-balanced output of an inner join (the scheme of expand_k), all columns of both sides written
-// at once: the pairs of row numbers never touch memory.
+// at once: the pairs of row numbers never touch memory.  IPT outputs a thread, each step for all of them
+// before the next; one where that still leaves SMs without a block (1848 outputs: 22 us -> 14; 2.6 M: 71 -> 61).
+template <int IPT>
 __global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict__ match, const OutputsBefore off, uint64_t nrows, uint64_t total, const uint32_t* __restrict__ rows,
                                                     Cols cols, const Publish pub) {
-    __shared__ unsigned rel[EX_TILE + 2];
+    constexpr int TILE = BLOCK * IPT;
+    __shared__ unsigned rel[TILE + 2];
     __shared__ uint64_t row_s[2];
-    const uint64_t o0 = (uint64_t)blockIdx.x * EX_TILE, o1 = o0 + EX_TILE < total ? o0 + EX_TILE : total;
+    const uint64_t o0 = (uint64_t)blockIdx.x * TILE, o1 = o0 + TILE < total ? o0 + TILE : total;
     if (threadIdx.x < 64) {
-        const uint64_t o = threadIdx.x < 32 ? o0 : o0 + EX_TILE;
+        const uint64_t o = threadIdx.x < 32 ? o0 : o0 + TILE;
         const uint64_t ub = o < total ? warp_partition_point(nrows, [&](uint64_t i) { return off[i] <= o; }) : nrows + 1;
         if (lane_id() == 0) row_s[threadIdx.x >> 5] = ub - 1;
     }
     __syncthreads();
     const uint64_t r0 = row_s[0], r1 = row_s[1] < nrows ? row_s[1] : nrows - 1, span = r1 - r0 + 1;
-    const bool in_smem = span <= (uint64_t)(EX_TILE + 2);
+    const bool in_smem = span <= (uint64_t)(TILE + 2);
     if (in_smem)
         for (unsigned i = threadIdx.x; i < (unsigned)span; i += BLOCK) {
             const uint64_t at = off[r0 + i];
-            rel[i] = at <= o0 ? 0u : (at - o0 < (uint64_t)EX_TILE ? (unsigned)(at - o0) : (unsigned)EX_TILE);
+            rel[i] = at <= o0 ? 0u : (at - o0 < (uint64_t)TILE ? (unsigned)(at - o0) : (unsigned)TILE);
         }
     const uint64_t skip0 = o0 - off[r0];
     __syncthreads();
-    for (unsigned t = threadIdx.x; t < (unsigned)(o1 - o0); t += BLOCK) {
-        uint64_t lo = 0, hi = span, j;
+    uint64_t l[IPT], r[IPT];
+#pragma unroll
+    for (int u = 0; u < IPT; ++u) {
+        const unsigned t = u * BLOCK + threadIdx.x;
+        l[u] = r0;
+        r[u] = 0;
+        if (t >= (unsigned)(o1 - o0)) continue;
+        uint64_t lo = 0, hi = span;
         if (in_smem) {
             while (lo < hi) {
                 const uint64_t mid = (lo + hi) >> 1;
                 if (rel[mid] <= t) lo = mid + 1;
                 else hi = mid;
             }
-            j = lo == 1 ? skip0 + t : (uint64_t)(t - rel[lo - 1]);
+            r[u] = lo == 1 ? skip0 + t : (uint64_t)(t - rel[lo - 1]);
         } else {
             while (lo < hi) {
                 const uint64_t mid = (lo + hi) >> 1;
                 if (off[r0 + mid] <= o0 + t) lo = mid + 1;
                 else hi = mid;
             }
-            j = o0 + t - off[r0 + lo - 1];
+            r[u] = o0 + t - off[r0 + lo - 1];
         }
-        const uint64_t l = r0 + lo - 1, r = rows[(match[l] >> 32) + j];
-        for (int k = 0; k < cols.n; ++k) copy_value(cols, k, k < cols.left ? l : r, o0 + t);
+        l[u] = r0 + lo - 1;
+    }
+#pragma unroll
+    for (int u = 0; u < IPT; ++u) r[u] += match[l[u]] >> 32;
+#pragma unroll
+    for (int u = 0; u < IPT; ++u) {
+        const unsigned t = u * BLOCK + threadIdx.x;
+        if (t < (unsigned)(o1 - o0)) r[u] = rows[r[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < IPT; ++u) {
+        const unsigned t = u * BLOCK + threadIdx.x;
+        if (t < (unsigned)(o1 - o0)) copy_row(cols, l[u], r[u], o0 + t);
     }
     publish_last(pub);
 }
@@ -534,8 +585,12 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     add_columns(c, o.get(), cols, r, w[0]);
     if (w[0]) {
         prof_begin(c, "join_emit", 0);
-        const Publish last = publish_by(c, (w[0] + EX_TILE - 1) / EX_TILE);
-        join_emit_k<<<(unsigned)((w[0] + EX_TILE - 1) / EX_TILE), BLOCK, 0, c->stream>>>(match->as<uint64_t>(), OutputsBefore{offs->as<uint64_t>(), in_tile->as<uint32_t>()}, l->rows, w[0], rows->as<uint32_t>(), cols, last);
+        const bool few = w[0] <= (uint64_t)c->sm_count * BLOCK * 4;
+        const uint64_t tile = few ? BLOCK : BLOCK * 4, blocks = (w[0] + tile - 1) / tile;
+        const Publish last = publish_by(c, blocks);
+        const OutputsBefore before{offs->as<uint64_t>(), in_tile->as<uint32_t>()};
+        if (few) join_emit_k<1><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), before, l->rows, w[0], rows->as<uint32_t>(), cols, last);
+        else join_emit_k<4><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), before, l->rows, w[0], rows->as<uint32_t>(), cols, last);
         check_launch(c, "join_emit");
         status_published(c, last);
     }
