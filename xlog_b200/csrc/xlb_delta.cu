@@ -1223,6 +1223,7 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const Out o, const __grid
             }
             __syncthreads();
             unsigned head = 0, end = v->tail;
+            __syncthreads();  // (read by all before a warp adds to it)
             bool ok = tried && end <= sh.queue;
             uint64_t level = 0, cand = 0, looked = RW_LONG;
             while (ok && head != end && level < max_iterations) {
