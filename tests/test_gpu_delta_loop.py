@@ -161,6 +161,12 @@ def test_thinly_spread_values(bits, values, monkeypatch):
     both(programs.transitive_closure(), {"edge": edge}, "reach", monkeypatch)
 
 
+@pytest.mark.parametrize("bits", [14, 15, 16])
+@pytest.mark.parametrize("values", [64, 4096, 8191, 8193])
+def test_thinly_spread_values_of_16_bits(bits, values, monkeypatch):
+    test_thinly_spread_values(bits, values, monkeypatch)
+
+
 def _rows_graph(kind):
     rng = np.random.default_rng(3)
     if kind.startswith("values"):  # bits of the second column: a word, two words, 16 and 17 bits
