@@ -211,7 +211,7 @@ struct WarpSink {
 // join a tuple's own matches are looked up while the atomic that decides about it is on its way, and
 // kept beside it.
 struct SoloShared {
-    unsigned count[3], cand[3], listed;
+    unsigned count[3], cand[3], listed[3];  // of three turns: a fast warp is in the next one while a slow one still reads
 };
 template <bool AHEAD>
 struct SoloSink {
@@ -629,19 +629,19 @@ __device__ __forceinline__ void solo(const Out& o, const Rules& rules, Heavy* he
     if (threadIdx.x < 3) {
         sh.count[threadIdx.x] = 0;
         sh.cand[threadIdx.x] = 0;
+        sh.listed[threadIdx.x] = 0;
     }
-    if (threadIdx.x == 0) sh.listed = 0;
     __syncthreads();
     for (unsigned i = threadIdx.x; i < n; i += DL_THREADS) {
         const uint64_t row = __ldcg(&o.log[st.start + i]);
         buf[i] = row;
         if (AHEAD) {
             find(rules.r[0].ix[0], rules.r[0].key_src[0] == 0 ? (uint32_t)(row >> 32) : (uint32_t)row, buf_s[i], buf_l[i]);
-            if (buf_l[i] > DL_HEAVY) sh.listed = 1;
+            if (buf_l[i] > DL_HEAVY) sh.listed[2] = 1;
         }
     }
     __syncthreads();
-    if (AHEAD && sh.listed) {  // a long row: all blocks
+    if (AHEAD && sh.listed[2]) {  // a long row: all blocks
         st.phase = PH_ROWS;
         return;
     }
@@ -650,13 +650,14 @@ __device__ __forceinline__ void solo(const Out& o, const Rules& rules, Heavy* he
         if (threadIdx.x == 0) {
             sh.count[after] = 0;
             sh.cand[after] = 0;
+            sh.listed[after] = 0;
         }
         const unsigned per = thin || n >= DL_THREADS ? 32 : (n + DL_WARPS - 1) / DL_WARPS;
         unsigned cand = 0;
         const unsigned to = (cur ^ 1) * SOLO_NEXT, from = cur * SOLO_NEXT;
         for (unsigned at = warp * per; at < n; at += DL_WARPS * per) {
             const unsigned rows = n - at < per ? n - at : per;
-            SoloSink<AHEAD> sink{o, rules, buf + to, buf_s + to, buf_l + to, &sh.count[turn], &sh.listed, st.end};
+            SoloSink<AHEAD> sink{o, rules, buf + to, buf_s + to, buf_l + to, &sh.count[turn], &sh.listed[turn], st.end};
             const uint64_t row = lane < rows ? buf[from + at + lane] : 0;
             if (AHEAD) {
                 Lane me;
@@ -666,14 +667,14 @@ __device__ __forceinline__ void solo(const Out& o, const Rules& rules, Heavy* he
                 const uint32_t mine = lane < rows ? buf_l[from + at + lane] : 0;
                 cand += mine;
                 deal(o, rules.r[0], me, mine, rows, false, sink);
-            } else if (take_rows(o, rules, row, rows, heavy, slot, false, sink, cand)) sh.listed = 1;
+            } else if (take_rows(o, rules, row, rows, heavy, slot, false, sink, cand)) sh.listed[turn] = 1;
         }
         cand = __reduce_add_sync(FULL, cand);
         if (lane == 0 && cand) atomicAdd(&sh.cand[turn], cand);
         __syncthreads();
         const unsigned next = sh.count[turn];
         const uint64_t cands = sh.cand[turn];
-        if (!AHEAD && sh.listed) {  // the iteration is not over: its long rows are listed
+        if (!AHEAD && sh.listed[turn]) {  // the iteration is not over: its long rows are listed
             if (threadIdx.x == 0) {
                 slot->count = next;
                 atomicAdd(&slot->cand, (unsigned long long)cands);
@@ -682,7 +683,7 @@ __device__ __forceinline__ void solo(const Out& o, const Rules& rules, Heavy* he
             return;
         }
         next_iteration(st, next, cands, o.cap, max_iterations, false);
-        if (AHEAD && sh.listed && st.phase == PH_SOLO) st.phase = PH_ROWS;
+        if (AHEAD && sh.listed[turn] && st.phase == PH_SOLO) st.phase = PH_ROWS;
         if (st.phase != PH_SOLO) return;
         thin = cands <= 2ull * n;
         n = next;
