@@ -86,7 +86,9 @@ struct Square {
 };
 enum Phase { PH_ROWS = 0, PH_HEAVY = 1, PH_SOLO = 2, PH_DONE = 3, PH_FULL = 4 };
 // What the blocks share about one iteration.  Three are used in turn: while one is filled the next is
-// cleared, and the one before may still be read by a block that is late.
+// cleared (by block 0, in every phase that ends an iteration at a grid barrier: the rows and the pieces of
+// long rows, which a solo phase goes over to directly), and the one before may still be read by a block
+// that is late.  A solo phase that ends an iteration by itself touches none.
 struct Slot {
     unsigned long long count, cand;  // tuples appended to the log; candidates
     unsigned heavy_n, next_heavy;    // pieces of long rows listed, taken
@@ -736,6 +738,10 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
         next_iteration(st, count, cands, o.cap, max_iterations, SQUARE);
         st.slot = st.slot == 2 ? 0 : st.slot + 1;
     };
+    // (The next slot was last read by blocks that have since arrived at another barrier.)
+    auto clear_next = [&]() {
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->slot[state_s.slot == 2 ? 0 : state_s.slot + 1] = Slot{};
+    };
     // The block's last tuples and its count of candidates go out with one atomic each (a warp with a
     // tuple or two each would queue on them for longer than a small iteration takes).
     auto end_block = [&](unsigned long long cand) {
@@ -783,7 +789,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
         sink.base = state_s.end;
         if (phase == PH_DONE) break;
         if (phase == PH_ROWS) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) ctl->slot[state_s.slot == 2 ? 0 : state_s.slot + 1] = Slot{};
+            clear_next();
             unsigned long long cand = 0;
             const uint64_t warps = (uint64_t)gridDim.x * DL_WARPS, me = (uint64_t)warp * gridDim.x + blockIdx.x;
             if (SQUARE) {
@@ -827,6 +833,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
                 }))
                 return;
         } else if (phase == PH_HEAVY) {
+            clear_next();
             const unsigned listed = __ldcg(&slot->heavy_n), pieces = listed < DL_HEAVY_MAX ? listed : (unsigned)DL_HEAVY_MAX;
             for (;;) {
                 unsigned item = 0;
