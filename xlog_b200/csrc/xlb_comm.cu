@@ -99,7 +99,7 @@ static void comm_wait(xlb_ctx* c) {
     auto t0 = std::chrono::steady_clock::now();
     uint64_t polls = 0;
     for (;;) {
-        cudaError_t q = cudaStreamQuery(c->stream);
+        const cudaError_t q = cuda_take(cudaStreamQuery(c->stream));
         if (q == cudaSuccess) break;
         if (q != cudaErrorNotReady) xlb_fail(XLB_ERR_CUDA, "stream failed during an exchange: %s", cudaGetErrorString(q));
         if ((++polls & 15) == 0 && cm && cm->comm) {
@@ -124,7 +124,7 @@ static void comm_wait(xlb_ctx* c) {
 void comm_destroy(xlb_ctx* c) {
     if (!c->comm) return;
     if (c->comm->comm) api().CommDestroy(c->comm->comm);
-    if (c->comm->h_stage) cudaFreeHost(c->comm->h_stage);
+    if (c->comm->h_stage) CUDA_QUIET(cudaFreeHost(c->comm->h_stage));
     delete c->comm;
     c->comm = nullptr;
     c->wait_hook = nullptr;

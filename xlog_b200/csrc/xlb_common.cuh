@@ -7,7 +7,6 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
-#include <cstdarg>
 #include <cstring>
 #include <cstdint>
 #include <cstdio>
@@ -17,29 +16,7 @@
 #include <string>
 #include <vector>
 
-#include "../../include/xlb.h"
-
-struct XlbError {
-    xlb_status st;
-    std::string msg;
-};
-
-[[noreturn]] inline void xlb_fail(xlb_status st, const char* fmt, ...) {
-    char buf[512];
-    va_list ap;
-    va_start(ap, fmt);
-    vsnprintf(buf, sizeof buf, fmt, ap);
-    va_end(ap);
-    throw XlbError{st, buf};
-}
-
-#define CUDA_OK(expr)                                                                            \
-    do {                                                                                         \
-        cudaError_t e__ = (expr);                                                                \
-        if (e__ != cudaSuccess)                                                                  \
-            xlb_fail(e__ == cudaErrorMemoryAllocation ? XLB_ERR_RESOURCE_EXHAUSTED : XLB_ERR_CUDA, \
-                     "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e__), __FILE__, __LINE__); \
-    } while (0)
+#include "xlb_error.h"
 
 struct Comm;  // NCCL exchange layer (xlb_comm.cu)
 
@@ -72,12 +49,11 @@ struct VmmApi {
         VmmApi a;
         auto sym = [](const char* name, void** fn) {
             cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-            return cudaGetDriverEntryPoint(name, fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess && *fn != nullptr;
+            return cuda_take(cudaGetDriverEntryPoint(name, fn, cudaEnableDefault, &q)) == cudaSuccess && q == cudaDriverEntryPointSuccess && *fn != nullptr;
         };
         a.ok = sym("cuMemAddressReserve", (void**)&a.reserve) && sym("cuMemAddressFree", (void**)&a.addr_free) && sym("cuMemCreate", (void**)&a.create) &&
                sym("cuMemRelease", (void**)&a.release) && sym("cuMemMap", (void**)&a.map) && sym("cuMemUnmap", (void**)&a.unmap) &&
                sym("cuMemSetAccess", (void**)&a.set_access) && sym("cuMemGetAllocationGranularity", (void**)&a.granularity);
-        if (!a.ok) cudaGetLastError();
         return a;
     }
 };
@@ -147,18 +123,12 @@ struct Arena {
         if (getenv("XLB_ARENA_SLABS")) return false;
         const VmmApi& api = VmmApi::get();
         int supported = 0;
-        if (!api.ok || cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, device) != cudaSuccess || !supported) {
-            cudaGetLastError();
-            return false;
-        }
+        if (!api.ok || cuda_take(cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, device)) != cudaSuccess || !supported) return false;
         CUmemAllocationProp prop = vmm_prop();
         size_t g = 0;
         if (api.granularity(&g, &prop, CU_MEM_ALLOC_GRANULARITY_RECOMMENDED) != CUDA_SUCCESS || g == 0) return false;
         size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
+        if (cuda_take(cudaMemGetInfo(&free_b, &total_b)) != cudaSuccess) return false;
         gran = g;
         va_size = (total_b + gran - 1) / gran * gran;
         CUdeviceptr base = 0;
@@ -229,10 +199,7 @@ struct Arena {
     }
     bool add_slab(uint64_t size) {
         void* p = nullptr;
-        if (cudaMalloc(&p, size) != cudaSuccess) {
-            cudaGetLastError();  // clear the sticky-less allocation error
-            return false;
-        }
+        if (cuda_take(cudaMalloc(&p, size)) != cudaSuccess) return false;
         slabs.push_back({(char*)p, size});
         reserved += size;
         insert_free((char*)p, size);
@@ -240,7 +207,7 @@ struct Arena {
     }
     // Give back every part of the backing store that is entirely free (after the stream has drained).
     void trim(cudaStream_t stream) {
-        cudaStreamSynchronize(stream);
+        CUDA_QUIET(cudaStreamSynchronize(stream));
         if (vmm) {
             vmm_trim();
             return;
@@ -249,7 +216,7 @@ struct Arena {
             auto it = free_by_addr.find(slabs[i].base);
             if (it != free_by_addr.end() && it->second == slabs[i].size) {
                 erase_free(slabs[i].base, slabs[i].size);
-                cudaFree(slabs[i].base);
+                CUDA_QUIET(cudaFree(slabs[i].base));
                 reserved -= slabs[i].size;
                 slabs.erase(slabs.begin() + i);
             } else ++i;
@@ -316,7 +283,7 @@ struct Arena {
         return false;
     }
     void destroy() {
-        for (auto& s : slabs) cudaFree(s.base);
+        for (auto& s : slabs) CUDA_QUIET(cudaFree(s.base));
         slabs.clear();
         if (vmm) {
             const VmmApi& api = VmmApi::get();
@@ -393,6 +360,7 @@ struct xlb_ctx {
     std::string prof_filter;  // "" = off, "*" = every kernel, else kernel names separated by commas
     ProfEntry* prof_open = nullptr;
     cudaEvent_t prof_e0 = nullptr;
+    cudaError_t error_before = cudaSuccess;  // what was on the thread when the launch at hand began (nothing, if every call is checked)
     // host timeline of one plan execution (XLB_TRACE_HOST=1): every launch and every wait with its
     // wall-clock interval, printed to stderr when the plan is done
     struct TraceNote {
@@ -417,6 +385,7 @@ inline void trace_note(xlb_ctx* c, const char* what, double t0) {
 
 // Bracket one launch with CUDA events on the launching stream when its kernel is profiled.
 inline void prof_begin(xlb_ctx* c, const char* name, uint64_t bytes) {
+    c->error_before = cudaPeekAtLastError();
     if (c->trace_on) trace_note(c, name, trace_now());
     if (c->prof_filter.empty()) return;
     if (c->prof_filter != "*") {  // a kernel name, or several separated by commas
@@ -430,8 +399,8 @@ inline void prof_begin(xlb_ctx* c, const char* name, uint64_t bytes) {
     auto& e = c->prof[name];
     e.launches++;
     e.bytes += bytes;
-    cudaEventCreate(&c->prof_e0);
-    cudaEventRecord(c->prof_e0, c->stream);
+    CUDA_OK(cudaEventCreate(&c->prof_e0));
+    CUDA_OK(cudaEventRecord(c->prof_e0, c->stream));
     c->prof_open = &e;
 }
 
@@ -477,17 +446,21 @@ using Buf = std::shared_ptr<DevBuf>;
 inline Buf make_buf(xlb_ctx* c, uint64_t bytes) { return std::make_shared<DevBuf>(c, bytes); }
 
 inline void check_launch(xlb_ctx* c, const char* what) {
+    const cudaError_t launched = cudaGetLastError();  // (before anything else takes it)
     c->launches++;
     c->drained = c->leaving = false;
     if (c->prof_open) {
         cudaEvent_t e1;
-        cudaEventCreate(&e1);
-        cudaEventRecord(e1, c->stream);
+        CUDA_OK(cudaEventCreate(&e1));
+        CUDA_OK(cudaEventRecord(e1, c->stream));
         c->prof_open->pending.emplace_back(c->prof_e0, e1);
         c->prof_open = nullptr;
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) xlb_fail(XLB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
+    const cudaError_t before = c->error_before, e = launched;
+    c->error_before = cudaSuccess;
+    if (e == cudaSuccess) return;
+    if (before != cudaSuccess) xlb_fail(XLB_ERR_CUDA, "an error from before the launch of %s: %s", what, cudaGetErrorString(before));
+    xlb_fail(XLB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
 }
 
 // Copies and fills enqueued on the context's stream.
@@ -514,12 +487,12 @@ inline void stream_wait(xlb_ctx* c) {
     if (spin) {  // poll first: a fixpoint waits for a row count many times, and a blocked thread's wake-up
                  // costs milliseconds on a busy host; after 5 ms fall back to a blocking wait
         for (;;) {
-            cudaError_t q = cudaStreamQuery(c->stream);
+            const cudaError_t q = cuda_take(cudaStreamQuery(c->stream));
             if (q == cudaSuccess) {
                 done = true;
                 break;
             }
-            if (q != cudaErrorNotReady) CUDA_OK(q);
+            if (q != cudaErrorNotReady) xlb_fail(XLB_ERR_CUDA, "waiting for the stream: %s", cudaGetErrorString(q));
             if (std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count() > 5.0) break;
         }
     }

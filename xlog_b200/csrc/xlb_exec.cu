@@ -2646,8 +2646,8 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
         CUDA_OK(cudaEventRecord(c->plan_e1, c->stream));
         check_dev_status(c);  // waits for everything above (executor/mod.rs:1463)
         cudaError_t done;  // (all work is: the event is due at once, and waiting for it took 10 us)
-        for (int polls = 0; (done = cudaEventQuery(c->plan_e1)) == cudaErrorNotReady && polls < 1000;) ++polls;
-        if (done == cudaErrorNotReady) done = cudaEventSynchronize(c->plan_e1);
+        for (int polls = 0; (done = cuda_take(cudaEventQuery(c->plan_e1))) == cudaErrorNotReady && polls < 1000;) ++polls;
+        if (done == cudaErrorNotReady) done = cuda_take(cudaEventSynchronize(c->plan_e1));
         CUDA_OK(done);
         float ms = 0;
         CUDA_OK(cudaEventElapsedTime(&ms, c->plan_e0, c->plan_e1));
@@ -2660,7 +2660,7 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
     } catch (const XlbError& e) {
         c->last_error = e.msg;
         result = e.st;
-        cudaStreamSynchronize(c->stream);
+        CUDA_QUIET(cudaStreamSynchronize(c->stream));
     } catch (const std::bad_alloc&) {
         c->last_error = "host allocation failed";
         result = XLB_ERR_RESOURCE_EXHAUSTED;

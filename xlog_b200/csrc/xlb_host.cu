@@ -15,13 +15,15 @@
 #include <sys/mman.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <list>
 #include <mutex>
 #include <system_error>
 #include <thread>
 #include <unordered_map>
+#include <vector>
 
-#include "xlb_common.cuh"
+#include "xlb_error.h"
 #include "xlb_host.h"
 
 namespace {
@@ -36,7 +38,7 @@ struct HostPool {
     int contexts = 0;
 
     static void destroy(void* p, uint64_t size) {
-        cudaHostUnregister(p);
+        CUDA_QUIET(cudaHostUnregister(p));
         munmap(p, size);
     }
     static void* create(uint64_t size) {
@@ -62,8 +64,7 @@ struct HostPool {
         }
         touch(p, std::min(per, size));
         for (auto& t : helpers) t.join();
-        if (cudaHostRegister(p, size, cudaHostRegisterPortable) != cudaSuccess) {
-            cudaGetLastError();
+        if (cuda_take(cudaHostRegister(p, size, cudaHostRegisterPortable)) != cudaSuccess) {
             munmap(p, size);
             return nullptr;
         }

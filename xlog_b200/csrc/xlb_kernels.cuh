@@ -1138,10 +1138,10 @@ constexpr size_t SORT_SMEM = (size_t)SORT_TILE * 8 + SORT_WARPS * 1024 + 256 * 4
 inline void radix_sort_setup(xlb_ctx* c) {
     bool& done = c->sort_attr_set;
     if (done) return;
-    cudaFuncSetAttribute(radix_scatter_k<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM);
-    cudaFuncSetAttribute(radix_scatter_k<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM);
-    cudaFuncSetAttribute(radix_scatter_k<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM);
-    cudaFuncSetAttribute(radix_scatter_k<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM);
+    CUDA_OK((cudaFuncSetAttribute(radix_scatter_k<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM)));
+    CUDA_OK((cudaFuncSetAttribute(radix_scatter_k<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM)));
+    CUDA_OK((cudaFuncSetAttribute(radix_scatter_k<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM)));
+    CUDA_OK((cudaFuncSetAttribute(radix_scatter_k<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SORT_SMEM)));
     done = true;
 }
 

@@ -315,31 +315,31 @@ static thread_local std::vector<PhaseRec> g_phase_recs;
 
 PhaseTimer::PhaseTimer(xlb_ctx* ctx, double* into) : c(ctx), acc(into) {
     if (!(c->flags & XLB_FLAG_PROFILE) || !into) return;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, c->stream);
+    CUDA_OK(cudaEventCreate(&e0));
+    CUDA_OK(cudaEventCreate(&e1));
+    CUDA_OK(cudaEventRecord(e0, c->stream));
 }
 PhaseTimer::~PhaseTimer() {
     if (!e0) return;
-    cudaEventRecord(e1, c->stream);
+    CUDA_QUIET(cudaEventRecord(e1, c->stream));
     g_phase_recs.push_back({e0, e1, acc});
 }
 void xlb_resolve_phase_timers(xlb_ctx* c) {
     if (g_phase_recs.empty() && c->prof.empty()) return;
-    cudaStreamSynchronize(c->stream);
+    CUDA_QUIET(cudaStreamSynchronize(c->stream));
     for (auto& r : g_phase_recs) {
         float ms = 0;
-        if (cudaEventElapsedTime(&ms, r.e0, r.e1) == cudaSuccess) *r.acc += ms;
-        cudaEventDestroy(r.e0);
-        cudaEventDestroy(r.e1);
+        if (cuda_take(cudaEventElapsedTime(&ms, r.e0, r.e1)) == cudaSuccess) *r.acc += ms;
+        CUDA_QUIET(cudaEventDestroy(r.e0));
+        CUDA_QUIET(cudaEventDestroy(r.e1));
     }
     g_phase_recs.clear();
     for (auto& kv : c->prof) {
         for (auto& e : kv.second.pending) {
             float ms = 0;
-            if (cudaEventElapsedTime(&ms, e.first, e.second) == cudaSuccess) kv.second.ms += ms;
-            cudaEventDestroy(e.first);
-            cudaEventDestroy(e.second);
+            if (cuda_take(cudaEventElapsedTime(&ms, e.first, e.second)) == cudaSuccess) kv.second.ms += ms;
+            CUDA_QUIET(cudaEventDestroy(e.first));
+            CUDA_QUIET(cudaEventDestroy(e.second));
         }
         kv.second.pending.clear();
     }
@@ -1157,7 +1157,7 @@ extern "C" xlb_status xlb_ctx_create(const xlb_config* cfg, xlb_ctx** out) {
     xlb_ctx* c = nullptr;
     try {
         int ndev = 0;
-        cudaError_t e = cudaGetDeviceCount(&ndev);
+        const cudaError_t e = cuda_take(cudaGetDeviceCount(&ndev));
         if (e != cudaSuccess || ndev == 0)
             xlb_fail(XLB_ERR_CUDA, "no CUDA device: %s (this library has no CPU path)", cudaGetErrorString(e));
         c = new xlb_ctx;
@@ -1197,17 +1197,17 @@ void xlb_exec_teardown(xlb_ctx* c);  // xlb_exec.cu: store, indexes, communicato
 
 extern "C" void xlb_ctx_destroy(xlb_ctx* c) {
     if (!c) return;
-    cudaSetDevice(c->device);
+    CUDA_QUIET(cudaSetDevice(c->device));
     xlb_exec_teardown(c);
-    cudaStreamSynchronize(c->stream);
+    CUDA_QUIET(cudaStreamSynchronize(c->stream));
     host_pool_context_closed();
-    if (c->h_scalar) cudaFreeHost(c->h_scalar);
-    if (c->h_stage) cudaFreeHost(c->h_stage);
-    if (c->d_status) cudaFree(c->d_status);
-    if (c->plan_e0) cudaEventDestroy(c->plan_e0);
-    if (c->plan_e1) cudaEventDestroy(c->plan_e1);
+    if (c->h_scalar) CUDA_QUIET(cudaFreeHost(c->h_scalar));
+    if (c->h_stage) CUDA_QUIET(cudaFreeHost(c->h_stage));
+    if (c->d_status) CUDA_QUIET(cudaFree(c->d_status));
+    if (c->plan_e0) CUDA_QUIET(cudaEventDestroy(c->plan_e0));
+    if (c->plan_e1) CUDA_QUIET(cudaEventDestroy(c->plan_e1));
     c->arena.destroy();
-    if (c->stream) cudaStreamDestroy(c->stream);
+    if (c->stream) CUDA_QUIET(cudaStreamDestroy(c->stream));
     delete c;
 }
 
@@ -1381,7 +1381,7 @@ extern "C" xlb_status xlb_rel_checksum(xlb_ctx* c, const xlb_rel* r, uint64_t di
 
 extern "C" void xlb_rel_free(xlb_rel* r) {
     if (!r) return;
-    cudaSetDevice(r->ctx->device);
+    CUDA_QUIET(cudaSetDevice(r->ctx->device));
     delete r;
 }
 

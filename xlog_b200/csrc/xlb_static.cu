@@ -76,14 +76,14 @@ extern "C" xlb_status xlb_dedup_sorted_u64_static(const uint64_t* d_sorted, uint
     cudaError_t e = cudaPeekAtLastError();
     if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "a CUDA error was already pending when the call began", e);
     int dev = 0;
-    e = cudaGetDevice(&dev);
+    e = cuda_take(cudaGetDevice(&dev));
     if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "cudaGetDevice", e);
     if (dev < 0 || dev >= 64) return fail(XLB_ERR_UNSUPPORTED, "device ordinal above 63", cudaSuccess);
     unsigned char* base = g_scratch_ptr[dev].load(std::memory_order_acquire);
     if (!base) {
         // set-up, once per device, with that device current
         void* p = nullptr;
-        e = cudaGetSymbolAddress(&p, g_static_scratch);
+        e = cuda_take(cudaGetSymbolAddress(&p, g_static_scratch));
         if (e != cudaSuccess || !p) return fail(XLB_ERR_CUDA, "cudaGetSymbolAddress(g_static_scratch)", e);
         base = (unsigned char*)p;
         g_scratch_ptr[dev].store(base, std::memory_order_release);
@@ -94,7 +94,7 @@ extern "C" xlb_status xlb_dedup_sorted_u64_static(const uint64_t* d_sorted, uint
     uint64_t* spine = (uint64_t*)(base + OFF_SPINE);
 
     if (n == 0) {
-        e = cudaMemsetAsync(d_count, 0, 8, stream);
+        e = cuda_take(cudaMemsetAsync(d_count, 0, 8, stream));
         if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "cudaMemsetAsync", e);
     } else {
         PredHead pred{d_sorted};
@@ -123,7 +123,7 @@ extern "C" xlb_status xlb_dedup_sorted_u64_static(const uint64_t* d_sorted, uint
         e = cudaGetLastError();
         if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "kernel launch", e);
     }
-    e = cudaStreamSynchronize(stream);
+    e = cuda_take(cudaStreamSynchronize(stream));
     if (e != cudaSuccess) return fail(XLB_ERR_CUDA, "cudaStreamSynchronize", e);
     g_static_error[0] = 0;
     return XLB_OK;
