@@ -590,8 +590,15 @@ inline void poll_words(xlb_ctx* c, int n, unsigned long long* out) {
     trace_note(c, "wait (words)", tr0);
 }
 
-// Read `n` 64-bit words from device memory (everything enqueued before has run when this returns).
-inline void read_words(xlb_ctx* c, const void* dptr, int n, unsigned long long* out) {
+// Fails with the status that the last read-back brought, and clears it.
+[[noreturn]] inline void fail_with_status(xlb_ctx* c);
+// What a kernel reported ends an operation at its next read-back: what such a kernel left (a list that is not
+// sorted, counts that do not fit) is nothing to size buffers by or to search in.  (Not with several ranks: the others
+// are in the same exchanges, and hear of it when the plan is done.)
+inline void stop_on_status(xlb_ctx* c) {
+    if (c->status_code && !c->wait_hook) fail_with_status(c);
+}
+inline void read_words_only(xlb_ctx* c, const void* dptr, int n, unsigned long long* out) {
     if (!publish_ok(c, n)) {
         if (n) CUDA_OK(copy_async(c, c->h_scalar, dptr, (size_t)n * 8, cudaMemcpyDeviceToHost));
         CUDA_OK(copy_async(c, c->h_scalar + READ_WORDS_AT, c->d_status, 8, cudaMemcpyDeviceToHost));
@@ -606,10 +613,16 @@ inline void read_words(xlb_ctx* c, const void* dptr, int n, unsigned long long* 
     CUDA_OK(cudaGetLastError());
     poll_words(c, n, out);
 }
+// Read `n` 64-bit words from device memory (everything enqueued before has run when this returns).
+inline void read_words(xlb_ctx* c, const void* dptr, int n, unsigned long long* out) {
+    read_words_only(c, dptr, n, out);
+    stop_on_status(c);
+}
 // After the launch of a kernel that got `p`: its words (by a read-back of their own where it was not asked).
 inline void read_published(xlb_ctx* c, const Publish& p, const void* dptr, int n, unsigned long long* out) {
     if (p.dst) poll_words(c, n, out);
-    else read_words(c, dptr, n, out);
+    else read_words_only(c, dptr, n, out);
+    stop_on_status(c);
 }
 // The same for a kernel that may be the last of an operation: its status is read when one is asked for.
 inline void status_published(xlb_ctx* c, const Publish& p) { c->leaving = p.dst != nullptr; }
@@ -618,14 +631,17 @@ inline void status_published(xlb_ctx* c, const Publish& p) { c->leaving = p.dst 
 inline void check_dev_status(xlb_ctx* c) {
     if (!c->drained) {
         if (c->leaving) poll_words(c, 0, nullptr);
-        else read_words(c, nullptr, 0, nullptr);
+        else read_words_only(c, nullptr, 0, nullptr);
     }
-    if (c->status_code == 0) return;
+    if (c->status_code) fail_with_status(c);
+}
+inline void fail_with_status(xlb_ctx* c) {
     DevStatus s;
     CUDA_OK(copy_async(c, c->h_scalar, c->d_status, sizeof s, cudaMemcpyDeviceToHost));
     stream_wait(c);
     memcpy(&s, c->h_scalar, sizeof s);
     CUDA_OK(set_async(c, c->d_status, 0, sizeof s));
+    c->status_code = 0;
     xlb_fail((xlb_status)s.code, "device kernel reported status %u at site %u (detail %llu)", s.code, s.where, s.detail);
 }
 

@@ -1420,7 +1420,7 @@ static bool run_rows(xlb_ctx* c, DeltaLoop& d, const Rules& rs, uint64_t max_ite
     return false;
 }
 
-bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
+void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
                    DeltaResult* res) {
     if (rules.size() > DL_RULES || variants.size() > SQ_VARIANTS) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules and %zu variants in a delta loop", rules.size(), variants.size());
     if (!c->delta_attr_set) {
@@ -1472,8 +1472,7 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
     }
     Buf by_rows;  // the head after rows were evaluated one by one and some are left
     if (rows_apart(d, rules, variants, known)) {
-        if (run_rows(c, d, rs, max_iterations, res)) return !c->status_code;
-        if (c->status_code) return false;
+        if (run_rows(c, d, rs, max_iterations, res)) return;
         by_rows = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
         CUDA_OK(copy_async(c, by_rows->p, d.visited->p, d.words * 4, cudaMemcpyDeviceToDevice));
     }
@@ -1493,13 +1492,12 @@ bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         check_launch(c, "expand_mark");
         unsigned long long w[7];  // tail, start, end, iterations, candidates, fix, overflow
         read_words(c, d.ctl, 7, w);
-        if (c->status_code) return false;
         res->rows = rows_done.rows + w[0];
         res->iterations = std::max<uint64_t>(rows_done.iterations, w[3]);
         res->candidates = rows_done.candidates + w[4];
         res->fix = rows_done.fix && w[5] != 0;
         prof_add_bytes(c, "expand_mark", w[4] * 4ull + w[0] * 16ull);
-        if (!w[6]) return true;
+        if (!w[6]) return;
         // The log was too short for the last iteration: its delta is what the head's bitmap holds
         // beyond the known rows and the log before it.  A longer log takes up from there.
         const uint64_t tail = w[0], stored = d.cap;

@@ -2029,7 +2029,7 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         DeltaResult res;
         {
             PhaseTimer t(c, &rs.st.ms_join);
-            if (!ops_delta_run(c, d, run, variants, c->max_iterations - it, full, &res)) check_dev_status(c);
+            ops_delta_run(c, d, run, variants, c->max_iterations - it, full, &res);
         }
         it += res.iterations;
         rs.st.iterations += res.iterations;

@@ -538,7 +538,6 @@ bool ops_frontier_whole(xlb_ctx* c, const xlb_rel* rel, int key_col, int value_c
     check_launch(c, name);
     unsigned long long w[5];
     read_published(c, pub, work->p, 5, w);
-    if (c->status_code) check_dev_status(c);
     if (large) prof_add_bytes(c, name, w[4] * 8ull);
     if (w[3] == 2 || (w[3] == 0 && one && max_iterations == 1u << 17)) return false;
     out->rows = w[0];

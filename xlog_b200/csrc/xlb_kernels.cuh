@@ -834,7 +834,9 @@ static __global__ void __launch_bounds__(BLOCK) radix_tile_hist_k(const uint64_t
 // number from an atomic counter, publish their digit counts in `status` and obtain the sum over
 // all earlier tiles by a decoupled look-back, so the pass reads and writes every key once.
 // A tile only waits for tiles that took an earlier number, which are running already; every
-// wait is bounded and reports XLB_ERR_TIMEOUT through `dst` instead of spinning for ever.
+// wait is bounded and reports XLB_ERR_TIMEOUT through `dst` instead of spinning for ever.  What a pass
+// leaves then is incomplete, so that the keys of a later pass no longer fit its histogram: hence the
+// test against n before a key is stored.
 constexpr unsigned LB_FLAG_AGG = 1u << 30, LB_FLAG_INC = 2u << 30, LB_MASK = (1u << 30) - 1;
 
 template <bool HAS_VALUES, bool LOOKBACK>
@@ -964,7 +966,8 @@ static __global__ void __launch_bounds__(SORT_THREADS, SORT_BLOCKS) radix_scatte
     for (unsigned i = threadIdx.x; i < valid; i += SORT_THREADS) {
         uint64_t k = skeys[i];
         unsigned d = digit(k);
-        keys_out[(uint64_t)glob_off[d] + (i - tile_start[d])] = k;
+        const uint64_t to = (uint64_t)glob_off[d] + (i - tile_start[d]);
+        if (to < n) keys_out[to] = k;
     }
     if (HAS_VALUES) {
         // Payloads take the same route through the (now free) shared key array: slot p gets the
@@ -983,7 +986,8 @@ static __global__ void __launch_bounds__(SORT_THREADS, SORT_BLOCKS) radix_scatte
         __syncthreads();
         for (unsigned i = threadIdx.x; i < valid; i += SORT_THREADS) {
             unsigned d = sd[i];
-            vals_out[(uint64_t)glob_off[d] + (i - tile_start[d])] = sv[i];
+            const uint64_t to = (uint64_t)glob_off[d] + (i - tile_start[d]);
+            if (to < n) vals_out[to] = sv[i];
         }
     }
 }
@@ -1348,6 +1352,10 @@ static __global__ void __launch_bounds__(BLOCK) mp_tile_k(const uint64_t* __rest
     __syncthreads();
     uint64_t a0 = split_s[0], a1 = split_s[1];
     uint64_t b0 = d0 - a0, b1 = d1 - a1;
+    if (a1 < a0 || b1 < b0) {  // (only over lists that are not sorted: a sort gave up, and its status says so)
+        a1 = a0;
+        b1 = b0;
+    }
     unsigned la = (unsigned)(a1 - a0), lb = (unsigned)(b1 - b0);
     unsigned lbx = lb + ((b1 < nb) ? 1u : 0u);  // one look-ahead element of B for a match across the tile edge
     for (unsigned i = threadIdx.x; i < la; i += BLOCK) sA[i] = A[a0 + i];

@@ -230,8 +230,7 @@ void ops_delta_known(xlb_ctx* c, DeltaLoop& d, const Keys& rows);   // rows the 
 void ops_delta_seed(xlb_ctx* c, DeltaLoop& d, const Keys& bag);     // candidates: what the head lacks joins it and the delta
 void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows);  // a delta as it is (known to the head already); before any seed
 // To the fixpoint.  `known`: what ops_delta_known was given (unique, disjoint from the seeds).
-// False: a kernel reported a failure (check_dev_status says which).
-bool ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
+void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
                    DeltaResult* res);
 
 // A whole frontier fixpoint in one launch (xlb_frontier.cu): seeds are the rows of `rel` with a column

@@ -108,8 +108,11 @@ __global__ void __launch_bounds__(BLOCK) key_range_k(const KeyWord w, uint64_t n
     }
     publish_last(pub);
 }
+// A row number that came out of a sort.  One that gave up (its status says so) leaves places unwritten, and
+// this kernel runs before the host has read the status: no row is looked for outside the relation.
+__device__ __forceinline__ uint32_t row_of(uint32_t row, uint64_t n) { return row < n ? row : 0u; }
 __global__ void __launch_bounds__(BLOCK) key_word_k(const KeyWord w, const uint32_t* __restrict__ rows, uint64_t* __restrict__ out, uint64_t n) {
-    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) out[i] = w(rows ? rows[i] : i);
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) out[i] = w(rows ? row_of(rows[i], n) : i);
 }
 // Words that were sorted by their bits from `mend` on only: each row finds the others of its prefix next to
 // it and counts those that come before it.  *unmended: a prefix has more rows than that is done for.
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(BLOCK) rows_out_k(const OutCols out, const uin
             }
             if (left == MEND_MAX || right == MEND_MAX) *unmended = 1;
         }
-        out(to, w, rows ? rows[i] : row_mask ? (uint32_t)(w & row_mask) : (uint32_t)i);
+        out(to, w, row_of(rows ? rows[i] : row_mask ? (uint32_t)(w & row_mask) : (uint32_t)i, n));
     }
     publish_last(pub);
 }
