@@ -139,7 +139,8 @@ xlb_status xlb_rel_to_host(xlb_ctx* ctx, const xlb_rel* rel, void* const* cols, 
  * xlb_rel_to_host into it run at the bus's rate, where fresh pageable memory takes a page fault per
  * page (any other memory works as well).  `*out` is aligned to a huge page; hand it back with
  * xlb_host_free.  XLB_ERR_RESOURCE_EXHAUSTED when the pool's bound is reached: use memory of your
- * own then.  Both may be called from any thread; they need no context. */
+ * own then.  Both may be called from any thread and need no context.  While one is open, blocks are
+ * registered on its device, whichever device the calling thread has chosen or not. */
 xlb_status xlb_host_alloc(uint64_t bytes, void** out);
 void xlb_host_free(void* block);
 /* clone_buffer (relational.rs:6113). */

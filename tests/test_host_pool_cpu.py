@@ -1,0 +1,66 @@
+"""The pool of page-locked result memory with several devices, ranks and threads, over a stand-in for
+the CUDA runtime."""
+import ctypes as C
+import threading
+
+import pytest
+
+from test_cuda_errors_cpu import build
+
+OK, EXHAUSTED = 0, 3
+MB = 1 << 20
+
+
+@pytest.fixture()
+def pool(tmp_path):
+    lib = build(str(tmp_path), """
+extern "C" void opened(int d) { host_pool_context_opened(d); }
+extern "C" void closed(int d) { host_pool_context_closed(d); }
+extern "C" int last_device() { return fake.last_device; }
+extern "C" int touched_devices() { return fake.touched_devices.exchange(0); }
+extern "C" int registered() { return fake.registered; }
+extern "C" int device_here() { return fake_device; }
+extern "C" void device_is(int d) { fake_device = d; }
+extern "C" void registration_takes(int ms) { fake.register_ms = ms; }
+extern "C" void fail(int r, int u) { fake.fail_register = r; fake.fail_unregister = u; }
+""", "xlb_host.cu")
+    lib.xlb_host_alloc.argtypes = [C.c_uint64, C.POINTER(C.c_void_p)]
+    lib.xlb_host_free.argtypes = [C.c_void_p]
+    return lib
+
+
+def alloc(lib, size, status=OK):
+    p = C.c_void_p()
+    assert lib.xlb_host_alloc(size, C.byref(p)) == status
+    return p.value
+
+
+def in_thread(f):
+    got = []
+    t = threading.Thread(target=lambda: got.append(f()))
+    t.start()
+    t.join()
+    return got[0]
+
+
+def test_a_fresh_thread_uses_the_device_of_the_open_context(pool):
+    pool.device_is(5)
+    pool.opened(5)
+    a = alloc(pool, MB)                       # the rank's own thread
+    assert pool.last_device() == 5
+    b = in_thread(lambda: alloc(pool, MB))    # one that never chose a device
+    assert pool.last_device() == 5
+    for p in (a, b):
+        in_thread(lambda: pool.xlb_host_free(p))
+    in_thread(lambda: pool.closed(5))         # the last context: what is kept is given back
+    assert pool.last_device() == 5 and pool.registered() == 0
+    assert pool.touched_devices() == 1 << 5   # device 0 is nobody's here
+    assert in_thread(pool.device_here) == 0 and pool.device_here() == 5
+
+
+def test_without_a_context_the_thread_decides(pool):
+    pool.device_is(3)
+    p = alloc(pool, MB)
+    assert pool.last_device() == 3
+    pool.xlb_host_free(p)
+    assert pool.registered() == 0 and pool.touched_devices() == 1 << 3

@@ -11,7 +11,8 @@
 // 16 GB; xlb_host_alloc then gives nothing and the caller uses memory of its own), kept ones below
 // 1 GB; what is kept is given back when the last context of the process closes.  One lock guards the
 // lists; a block has one owner at a time and no device work refers to it once it is handed back
-// (xlb_rel_to_host returns when its copies are done).
+// (xlb_rel_to_host returns when its copies are done).  Blocks are registered on the device of an open
+// context, whatever thread asks for them, and usable by all (cudaHostRegisterPortable).
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -30,18 +31,42 @@ namespace {
 
 constexpr uint64_t HUGE_PAGE = 2ull << 20, IDLE_MAX = 1ull << 30, LIVE_MAX = 16ull << 30;
 
+struct Block {
+    void* p;
+    uint64_t size;
+    int device;  // that it was registered on, -1: the one its first user's thread had (no context was open)
+};
 struct HostPool {
     std::mutex mu;
-    std::unordered_map<void*, uint64_t> used;         // blocks handed out
-    std::list<std::pair<void*, uint64_t>> idle;       // blocks kept, the one kept longest first
+    std::unordered_map<void*, Block> used;            // blocks handed out
+    std::list<Block> idle;                            // blocks kept, the one kept longest first
     uint64_t used_bytes = 0, idle_bytes = 0, limit = 0;
-    int contexts = 0;
+    std::vector<int> devices;                         // of the open contexts
 
-    static void destroy(void* p, uint64_t size) {
-        CUDA_QUIET(cudaHostUnregister(p));
-        munmap(p, size);
+    // `f` with `device` current: on this thread where it is already, else on one of its own.  (The caller's
+    // current device stays what it is, and a device that no context is open on is not set up by a
+    // thread that never chose one.)  False: there is no thread to be had.
+    template <class F>
+    static bool with_device(int device, F f) {
+        int current = -1;
+        if (device < 0 || (cuda_take(cudaGetDevice(&current)) == cudaSuccess && current == device)) {
+            f();
+            return true;
+        }
+        try {
+            std::thread([&] {
+                if (cuda_take(cudaSetDevice(device)) == cudaSuccess) f();
+            }).join();
+        } catch (const std::system_error&) {
+            return false;
+        }
+        return true;
     }
-    static void* create(uint64_t size) {
+    static void destroy(const Block& b) {
+        if (!with_device(b.device, [&] { CUDA_QUIET(cudaHostUnregister(b.p)); })) CUDA_QUIET(cudaHostUnregister(b.p));
+        munmap(b.p, b.size);
+    }
+    static void* create(uint64_t size, int device) {
         char* raw = (char*)mmap(nullptr, size + HUGE_PAGE, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
         if (raw == (char*)MAP_FAILED) return nullptr;
         char* p = (char*)(((uintptr_t)raw + HUGE_PAGE - 1) & ~(uintptr_t)(HUGE_PAGE - 1));
@@ -64,7 +89,9 @@ struct HostPool {
         }
         touch(p, std::min(per, size));
         for (auto& t : helpers) t.join();
-        if (cuda_take(cudaHostRegister(p, size, cudaHostRegisterPortable)) != cudaSuccess) {
+        bool registered = false;
+        with_device(device, [&] { registered = cuda_take(cudaHostRegister(p, size, cudaHostRegisterPortable)) == cudaSuccess; });
+        if (!registered) {
             munmap(p, size);
             return nullptr;
         }
@@ -72,10 +99,10 @@ struct HostPool {
     }
     void trim(uint64_t keep) {
         while (idle_bytes > keep) {
-            auto b = idle.front();
+            const Block b = idle.front();
             idle.pop_front();
-            idle_bytes -= b.second;
-            destroy(b.first, b.second);
+            idle_bytes -= b.size;
+            destroy(b);
         }
     }
     void* take(uint64_t bytes) {
@@ -84,20 +111,21 @@ struct HostPool {
         if (!limit) limit = std::min<uint64_t>(LIVE_MAX, (uint64_t)sysconf(_SC_PHYS_PAGES) * (uint64_t)sysconf(_SC_PAGESIZE) / 8);
         auto best = idle.end();  // the smallest kept block that fits without wasting more than a quarter
         for (auto it = idle.begin(); it != idle.end(); ++it)
-            if (it->second >= size && it->second <= size + size / 4 + HUGE_PAGE && (best == idle.end() || it->second < best->second)) best = it;
+            if (it->size >= size && it->size <= size + size / 4 + HUGE_PAGE && (best == idle.end() || it->size < best->size)) best = it;
         if (best != idle.end()) {
-            auto b = *best;
+            const Block b = *best;
             idle.erase(best);
-            idle_bytes -= b.second;
-            used[b.first] = b.second;
-            used_bytes += b.second;
-            return b.first;
+            idle_bytes -= b.size;
+            used[b.p] = b;
+            used_bytes += b.size;
+            return b.p;
         }
         if (used_bytes + size > limit) return nullptr;
         if (used_bytes + idle_bytes + size > limit) trim(limit - used_bytes - size);
-        void* p = create(size);
+        const int device = devices.empty() ? -1 : devices.back();
+        void* p = create(size, device);
         if (!p) return nullptr;
-        used[p] = size;
+        used[p] = Block{p, size, device};
         used_bytes += size;
         return p;
     }
@@ -105,12 +133,12 @@ struct HostPool {
         std::lock_guard<std::mutex> g(mu);
         auto it = used.find(p);
         if (it == used.end()) return;
-        const uint64_t size = it->second;
+        const Block b = it->second;
         used.erase(it);
-        used_bytes -= size;
-        idle.emplace_back(p, size);
-        idle_bytes += size;
-        trim(contexts > 0 ? IDLE_MAX : 0);
+        used_bytes -= b.size;
+        idle.push_back(b);
+        idle_bytes += b.size;
+        trim(devices.empty() ? 0 : IDLE_MAX);
     }
 };
 HostPool& pool() {
@@ -120,13 +148,16 @@ HostPool& pool() {
 
 }  // namespace
 
-void host_pool_context_opened() {
+void host_pool_context_opened(int device) {
     std::lock_guard<std::mutex> g(pool().mu);
-    ++pool().contexts;
+    pool().devices.push_back(device);
 }
-void host_pool_context_closed() {
+void host_pool_context_closed(int device) {
     std::lock_guard<std::mutex> g(pool().mu);
-    if (--pool().contexts == 0) pool().trim(0);
+    auto& open = pool().devices;
+    const auto it = std::find(open.begin(), open.end(), device);
+    if (it != open.end()) open.erase(it);
+    if (open.empty()) pool().trim(0);
 }
 
 extern "C" xlb_status xlb_host_alloc(uint64_t bytes, void** out) {

@@ -2,5 +2,5 @@
 #pragma once
 #include <cstdint>
 
-void host_pool_context_opened();
-void host_pool_context_closed();
+void host_pool_context_opened(int device);
+void host_pool_context_closed(int device);

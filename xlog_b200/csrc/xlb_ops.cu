@@ -1183,7 +1183,7 @@ extern "C" xlb_status xlb_ctx_create(const xlb_config* cfg, xlb_ctx** out) {
         cudaDeviceProp prop;
         CUDA_OK(cudaGetDeviceProperties(&prop, dev));
         c->sm_count = prop.multiProcessorCount;
-        host_pool_context_opened();
+        host_pool_context_opened(dev);
         *out = c;
     } catch (const XlbError& e) {
         g_create_error = e.msg;
@@ -1200,7 +1200,7 @@ extern "C" void xlb_ctx_destroy(xlb_ctx* c) {
     CUDA_QUIET(cudaSetDevice(c->device));
     xlb_exec_teardown(c);
     CUDA_QUIET(cudaStreamSynchronize(c->stream));
-    host_pool_context_closed();
+    host_pool_context_closed(c->device);
     if (c->h_scalar) CUDA_QUIET(cudaFreeHost(c->h_scalar));
     if (c->h_stage) CUDA_QUIET(cudaFreeHost(c->h_stage));
     if (c->d_status) CUDA_QUIET(cudaFree(c->d_status));
