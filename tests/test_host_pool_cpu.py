@@ -1,6 +1,7 @@
 """The pool of page-locked result memory with several devices, ranks and threads, over a stand-in for
 the CUDA runtime."""
 import ctypes as C
+import os
 import threading
 
 import pytest
@@ -22,10 +23,13 @@ extern "C" int registered() { return fake.registered; }
 extern "C" int device_here() { return fake_device; }
 extern "C" void device_is(int d) { fake_device = d; }
 extern "C" void registration_takes(int ms) { fake.register_ms = ms; }
+extern "C" uint64_t most() { return host_pool_most(); }
+extern "C" void ranks(unsigned n) { host_pool_ranks(n); }
 extern "C" void fail(int r, int u) { fake.fail_register = r; fake.fail_unregister = u; }
 """, "xlb_host.cu")
     lib.xlb_host_alloc.argtypes = [C.c_uint64, C.POINTER(C.c_void_p)]
     lib.xlb_host_free.argtypes = [C.c_void_p]
+    lib.most.restype = C.c_uint64
     return lib
 
 
@@ -56,6 +60,24 @@ def test_a_fresh_thread_uses_the_device_of_the_open_context(pool):
     assert pool.last_device() == 5 and pool.registered() == 0
     assert pool.touched_devices() == 1 << 5   # device 0 is nobody's here
     assert in_thread(pool.device_here) == 0 and pool.device_here() == 5
+
+
+@pytest.mark.parametrize("said", [None, "8", "0", "many"])
+def test_ranks_share_the_bound(pool, said, monkeypatch):
+    memory = os.sysconf("SC_PHYS_PAGES") * os.sysconf("SC_PAGE_SIZE")
+    share = lambda ranks: min(16 << 30, memory // 8 // ranks)  # noqa: E731
+    monkeypatch.delenv("LOCAL_WORLD_SIZE", raising=False)
+    assert pool.most() == share(1)
+    if said is not None:
+        monkeypatch.setenv("LOCAL_WORLD_SIZE", said)
+    assert pool.most() == share(8 if said == "8" else 1)
+    pool.ranks(4)  # a communicator
+    assert pool.most() == share(8 if said == "8" else 4)
+    monkeypatch.setenv("LOCAL_WORLD_SIZE", str(memory // (64 * MB)))  # a share of 8 MB
+    alloc(pool, 6 * MB)
+    alloc(pool, 4 * MB, EXHAUSTED)
+    alloc(pool, 1 << 63, EXHAUSTED)
+    alloc(pool, (1 << 64) - 1, EXHAUSTED)
 
 
 def test_without_a_context_the_thread_decides(pool):

@@ -10,6 +10,7 @@
 #include <cstdlib>
 
 #include "xlb_comm.h"
+#include "xlb_host.h"
 
 namespace {
 
@@ -164,6 +165,7 @@ extern "C" xlb_status xlb_comm_init(xlb_ctx* c, const uint8_t id[XLB_UNIQUE_ID_B
         c->world = c->comm_world = world;
         cm->counts_dev = make_buf(c, (uint64_t)world * STAGE_ROW * 8);
         CUDA_OK(cudaHostAlloc((void**)&cm->h_stage, (size_t)(world + 1) * STAGE_ROW * 8, cudaHostAllocDefault));
+        host_pool_ranks(world);
         c->wait_hook = comm_wait;  // every host wait of this context now watches the communicator too
     } catch (const XlbError& e) {
         c->last_error = e.msg;

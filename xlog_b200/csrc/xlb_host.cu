@@ -7,9 +7,10 @@
 // (256 MB: 16 ms, against 97 ms by cudaHostAlloc and 121 ms for one pageable copy of that size):
 // even a block used once pays for itself.  Blocks that come back are kept for the next result.
 //
-// Bounds: blocks in use and kept together stay below an eighth of the machine's memory (at most
-// 16 GB; xlb_host_alloc then gives nothing and the caller uses memory of its own), kept ones below
-// 1 GB; what is kept is given back when the last context of the process closes.  One lock guards the
+// Bounds: blocks in use and kept together stay below this process's share of an eighth of the
+// machine's memory (at most 16 GB; xlb_host_alloc then gives nothing and the caller uses memory of its
+// own), kept ones below 1 GB.  Ranks on one machine share the eighth: their number is LOCAL_WORLD_SIZE
+// where the launcher says so, else that of the communicator; what is kept is given back when the last context of the process closes.  One lock guards the
 // lists; a block has one owner at a time and no device work refers to it once it is handed back
 // (xlb_rel_to_host returns when its copies are done).  Blocks are registered on the device of an open
 // context, whatever thread asks for them, and usable by all (cudaHostRegisterPortable).
@@ -17,6 +18,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <list>
 #include <mutex>
 #include <system_error>
@@ -40,7 +42,8 @@ struct HostPool {
     std::mutex mu;
     std::unordered_map<void*, Block> used;            // blocks handed out
     std::list<Block> idle;                            // blocks kept, the one kept longest first
-    uint64_t used_bytes = 0, idle_bytes = 0, limit = 0;
+    uint64_t used_bytes = 0, idle_bytes = 0;
+    unsigned ranks = 1;                               // of the communicators made in this process, the most
     std::vector<int> devices;                         // of the open contexts
 
     // `f` with `device` current: on this thread where it is already, else on one of its own.  (The caller's
@@ -105,10 +108,17 @@ struct HostPool {
             destroy(b);
         }
     }
+    uint64_t most() const {
+        const char* local = getenv("LOCAL_WORLD_SIZE");
+        const unsigned long said = local ? strtoul(local, nullptr, 10) : 0;
+        const uint64_t memory = (uint64_t)sysconf(_SC_PHYS_PAGES) * (uint64_t)sysconf(_SC_PAGESIZE);
+        return std::min<uint64_t>(LIVE_MAX, memory / 8 / (said ? said : ranks));
+    }
     void* take(uint64_t bytes) {
+        if (bytes > LIVE_MAX) return nullptr;
         const uint64_t size = (bytes + HUGE_PAGE - 1) / HUGE_PAGE * HUGE_PAGE;
         std::lock_guard<std::mutex> g(mu);
-        if (!limit) limit = std::min<uint64_t>(LIVE_MAX, (uint64_t)sysconf(_SC_PHYS_PAGES) * (uint64_t)sysconf(_SC_PAGESIZE) / 8);
+        const uint64_t limit = most();
         auto best = idle.end();  // the smallest kept block that fits without wasting more than a quarter
         for (auto it = idle.begin(); it != idle.end(); ++it)
             if (it->size >= size && it->size <= size + size / 4 + HUGE_PAGE && (best == idle.end() || it->size < best->size)) best = it;
@@ -158,6 +168,15 @@ void host_pool_context_closed(int device) {
     const auto it = std::find(open.begin(), open.end(), device);
     if (it != open.end()) open.erase(it);
     if (open.empty()) pool().trim(0);
+}
+
+void host_pool_ranks(unsigned ranks) {
+    std::lock_guard<std::mutex> g(pool().mu);
+    pool().ranks = std::max(pool().ranks, ranks);
+}
+uint64_t host_pool_most() {
+    std::lock_guard<std::mutex> g(pool().mu);
+    return pool().most();
 }
 
 extern "C" xlb_status xlb_host_alloc(uint64_t bytes, void** out) {
