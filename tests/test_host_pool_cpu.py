@@ -2,7 +2,9 @@
 the CUDA runtime."""
 import ctypes as C
 import os
+import random
 import threading
+import time
 
 import pytest
 
@@ -78,6 +80,53 @@ def test_ranks_share_the_bound(pool, said, monkeypatch):
     alloc(pool, 4 * MB, EXHAUSTED)
     alloc(pool, 1 << 63, EXHAUSTED)
     alloc(pool, (1 << 64) - 1, EXHAUSTED)
+
+
+def test_others_do_not_wait_while_a_block_is_made(pool):
+    pool.opened(0)
+    kept, held = alloc(pool, 4 * MB), alloc(pool, 16 * MB)
+    pool.xlb_host_free(kept)
+    pool.registration_takes(1500)
+    maker = threading.Thread(target=lambda: alloc(pool, 64 * MB))
+    maker.start()
+    time.sleep(0.3)
+    t = time.perf_counter()
+    pool.xlb_host_free(held)
+    assert alloc(pool, 4 * MB) == kept
+    assert time.perf_counter() - t < 0.5 and maker.is_alive()
+    maker.join()
+    assert pool.registered() == 3
+
+
+def test_many_threads(pool, monkeypatch):
+    # blocks of all sizes under a bound that they reach: nobody shares one, and all come back
+    monkeypatch.setenv("LOCAL_WORLD_SIZE", str(os.sysconf("SC_PHYS_PAGES") * os.sysconf("SC_PAGE_SIZE") // 8 // (48 * MB)))
+    pool.opened(0)
+    owned, lock, wrong = set(), threading.Lock(), []
+
+    def work(seed):
+        rng = random.Random(seed)
+        for _ in range(60):
+            p = C.c_void_p()
+            st = pool.xlb_host_alloc(rng.randint(1, 12 * MB), C.byref(p))
+            if st == EXHAUSTED:
+                continue
+            with lock:
+                if st != OK or p.value in owned:
+                    wrong.append((st, p.value))
+                owned.add(p.value)
+            with lock:
+                owned.discard(p.value)
+            pool.xlb_host_free(p)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    pool.closed(0)
+    assert pool.registered() == 0
 
 
 def test_without_a_context_the_thread_decides(pool):

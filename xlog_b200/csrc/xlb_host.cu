@@ -11,7 +11,7 @@
 // machine's memory (at most 16 GB; xlb_host_alloc then gives nothing and the caller uses memory of its
 // own), kept ones below 1 GB.  Ranks on one machine share the eighth: their number is LOCAL_WORLD_SIZE
 // where the launcher says so, else that of the communicator; what is kept is given back when the last context of the process closes.  One lock guards the
-// lists; a block has one owner at a time and no device work refers to it once it is handed back
+// lists, and is not held while a block is made or given back; a block has one owner at a time and no device work refers to it once it is handed back
 // (xlb_rel_to_host returns when its copies are done).  Blocks are registered on the device of an open
 // context, whatever thread asks for them, and usable by all (cudaHostRegisterPortable).
 #include <sys/mman.h>
@@ -19,9 +19,10 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <exception>
 #include <list>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -38,13 +39,15 @@ struct Block {
     uint64_t size;
     int device;  // that it was registered on, -1: the one its first user's thread had (no context was open)
 };
+using Blocks = std::list<Block>;
 struct HostPool {
     std::mutex mu;
-    std::unordered_map<void*, Block> used;            // blocks handed out
-    std::list<Block> idle;                            // blocks kept, the one kept longest first
-    uint64_t used_bytes = 0, idle_bytes = 0;
-    unsigned ranks = 1;                               // of the communicators made in this process, the most
-    std::vector<int> devices;                         // of the open contexts
+    Blocks used, idle;                                     // handed out; kept, the one kept longest first
+    std::unordered_map<void*, Blocks::iterator> used_at;
+    uint64_t used_bytes = 0, idle_bytes = 0;               // (used: with what is being made)
+    uint64_t leaving_bytes = 0;                            // no longer kept, not yet given back
+    unsigned ranks = 1;                                    // of the communicators made in this process, the most
+    std::vector<int> devices;                              // of the open contexts
 
     // `f` with `device` current: on this thread where it is already, else on one of its own.  (The caller's
     // current device stays what it is, and a device that no context is open on is not set up by a
@@ -60,14 +63,16 @@ struct HostPool {
             std::thread([&] {
                 if (cuda_take(cudaSetDevice(device)) == cudaSuccess) f();
             }).join();
-        } catch (const std::system_error&) {
+        } catch (const std::exception&) {
             return false;
         }
         return true;
     }
     static void destroy(const Block& b) {
-        if (!with_device(b.device, [&] { CUDA_QUIET(cudaHostUnregister(b.p)); })) CUDA_QUIET(cudaHostUnregister(b.p));
-        munmap(b.p, b.size);
+        bool done = false;
+        const auto unregister = [&] { done = cuda_take(cudaHostUnregister(b.p)) == cudaSuccess; };
+        if (!with_device(b.device, unregister)) unregister();
+        if (done) munmap(b.p, b.size);  // (else the device still knows the pages: not for anybody else)
     }
     static void* create(uint64_t size, int device) {
         char* raw = (char*)mmap(nullptr, size + HUGE_PAGE, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
@@ -81,14 +86,12 @@ struct HostPool {
         };
         const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
         const uint64_t pages = size / HUGE_PAGE, parts = std::min<uint64_t>({8, cores, (pages + 3) / 4});
-        std::vector<std::thread> helpers;
         const uint64_t per = (pages + parts - 1) / parts * HUGE_PAGE;
-        for (uint64_t at = per; at < size; at += per) {
-            try {
-                helpers.emplace_back(touch, p + at, std::min(per, size - at));
-            } catch (const std::system_error&) {  // no thread to be had: registering touches the pages then
-                break;
-            }
+        std::vector<std::thread> helpers;
+        try {
+            helpers.reserve(parts);
+            for (uint64_t at = per; at < size; at += per) helpers.emplace_back(touch, p + at, std::min(per, size - at));
+        } catch (const std::exception&) {  // no thread (or memory for one) to be had: registering touches the pages then
         }
         touch(p, std::min(per, size));
         for (auto& t : helpers) t.join();
@@ -100,13 +103,26 @@ struct HostPool {
         }
         return p;
     }
-    void trim(uint64_t keep) {
-        while (idle_bytes > keep) {
-            const Block b = idle.front();
-            idle.pop_front();
-            idle_bytes -= b.size;
-            destroy(b);
+    // Kept blocks to be given back until `enough` holds.  (Lock held; what comes out goes to give_back without it.)
+    template <class F>
+    Blocks pick(F enough) {
+        Blocks out;
+        while (!idle.empty() && !enough()) {
+            idle_bytes -= idle.front().size;
+            leaving_bytes += idle.front().size;
+            out.splice(out.end(), idle, idle.begin());
         }
+        return out;
+    }
+    void give_back(const Blocks& blocks) {
+        uint64_t bytes = 0;
+        for (const Block& b : blocks) {
+            destroy(b);
+            bytes += b.size;
+        }
+        if (!bytes) return;
+        std::lock_guard<std::mutex> g(mu);
+        leaving_bytes -= bytes;
     }
     uint64_t most() const {
         const char* local = getenv("LOCAL_WORLD_SIZE");
@@ -117,38 +133,68 @@ struct HostPool {
     void* take(uint64_t bytes) {
         if (bytes > LIVE_MAX) return nullptr;
         const uint64_t size = (bytes + HUGE_PAGE - 1) / HUGE_PAGE * HUGE_PAGE;
-        std::lock_guard<std::mutex> g(mu);
-        const uint64_t limit = most();
-        auto best = idle.end();  // the smallest kept block that fits without wasting more than a quarter
-        for (auto it = idle.begin(); it != idle.end(); ++it)
-            if (it->size >= size && it->size <= size + size / 4 + HUGE_PAGE && (best == idle.end() || it->size < best->size)) best = it;
-        if (best != idle.end()) {
-            const Block b = *best;
-            idle.erase(best);
-            idle_bytes -= b.size;
-            used[b.p] = b;
-            used_bytes += b.size;
-            return b.p;
+        Blocks one, out;
+        {
+            std::lock_guard<std::mutex> g(mu);
+            auto best = idle.end();  // the smallest kept block that fits without wasting more than a quarter
+            for (auto it = idle.begin(); it != idle.end(); ++it)
+                if (it->size >= size && it->size <= size + size / 4 + HUGE_PAGE && (best == idle.end() || it->size < best->size)) best = it;
+            if (best != idle.end()) {
+                used_at.emplace(best->p, best);
+                idle_bytes -= best->size;
+                used_bytes += best->size;
+                used.splice(used.end(), idle, best);
+                return best->p;
+            }
+            const uint64_t limit = most();
+            if (used_bytes + leaving_bytes + size > limit) return nullptr;
+            one.push_back(Block{nullptr, size, devices.empty() ? -1 : devices.back()});
+            const uint64_t gone = leaving_bytes;  // by other threads; what is picked here is gone before the new block is made
+            out = pick([&] { return used_bytes + idle_bytes + gone + size <= limit; });
+            used_bytes += size;
         }
-        if (used_bytes + size > limit) return nullptr;
-        if (used_bytes + idle_bytes + size > limit) trim(limit - used_bytes - size);
-        const int device = devices.empty() ? -1 : devices.back();
-        void* p = create(size, device);
-        if (!p) return nullptr;
-        used[p] = Block{p, size, device};
-        used_bytes += size;
-        return p;
+        // Making a block takes milliseconds: without the lock.
+        give_back(out);
+        one.front().p = create(size, one.front().device);
+        std::unique_lock<std::mutex> g(mu);
+        if (one.front().p) {
+            try {
+                used_at.emplace(one.front().p, one.begin());
+                used.splice(used.end(), one);
+                return used.back().p;
+            } catch (const std::bad_alloc&) {
+            }
+        }
+        used_bytes -= size;
+        g.unlock();
+        if (one.front().p) destroy(one.front());
+        return nullptr;
     }
     void give(void* p) {
-        std::lock_guard<std::mutex> g(mu);
-        auto it = used.find(p);
-        if (it == used.end()) return;
-        const Block b = it->second;
-        used.erase(it);
-        used_bytes -= b.size;
-        idle.push_back(b);
-        idle_bytes += b.size;
-        trim(devices.empty() ? 0 : IDLE_MAX);
+        Blocks out;
+        {
+            std::lock_guard<std::mutex> g(mu);
+            const auto at = used_at.find(p);
+            if (at == used_at.end()) return;
+            const auto it = at->second;
+            used_at.erase(at);
+            used_bytes -= it->size;
+            idle_bytes += it->size;
+            idle.splice(idle.end(), used, it);
+            const uint64_t keep = devices.empty() ? 0 : IDLE_MAX;
+            out = pick([&] { return idle_bytes <= keep; });
+        }
+        give_back(out);
+    }
+    void closed(int device) {
+        Blocks out;
+        {
+            std::lock_guard<std::mutex> g(mu);
+            const auto it = std::find(devices.begin(), devices.end(), device);
+            if (it != devices.end()) devices.erase(it);
+            if (devices.empty()) out = pick([] { return false; });
+        }
+        give_back(out);
     }
 };
 HostPool& pool() {
@@ -162,14 +208,7 @@ void host_pool_context_opened(int device) {
     std::lock_guard<std::mutex> g(pool().mu);
     pool().devices.push_back(device);
 }
-void host_pool_context_closed(int device) {
-    std::lock_guard<std::mutex> g(pool().mu);
-    auto& open = pool().devices;
-    const auto it = std::find(open.begin(), open.end(), device);
-    if (it != open.end()) open.erase(it);
-    if (open.empty()) pool().trim(0);
-}
-
+void host_pool_context_closed(int device) { pool().closed(device); }
 void host_pool_ranks(unsigned ranks) {
     std::lock_guard<std::mutex> g(pool().mu);
     pool().ranks = std::max(pool().ranks, ranks);
