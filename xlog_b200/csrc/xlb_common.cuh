@@ -346,6 +346,7 @@ struct xlb_ctx {
     // bounded look-back of the one-sweep sort: polls before a tile gives up (XLB_ERR_TIMEOUT), and
     // the number the first tile takes (0; a test makes tile 0 never run so that the wait runs out)
     unsigned lb_spin_limit = 1u << 22, lb_first_tile = 0;
+    unsigned delta_spin_limit = 1u << 26;  // polls (tens of seconds) for which a block of the delta loop waits without seeing anything go on
     bool frontier_attr_set = false, frontier_many_attr_set = false, frontier_large_attr_set = false;  // the same for the frontier kernels
     bool index_attr_set = false;  // the same for direct_small_k
     bool delta_attr_set = false;  // the same for the delta loop's kernel

@@ -31,7 +31,6 @@ constexpr uint64_t DL_SOLO_ROWS = 2048, DL_SOLO_OUTPUTS = 8192;  // iterations o
 constexpr unsigned SOLO_NEXT = 2048;                     // tuples of a solo iteration that stay in shared memory
 constexpr size_t DL_SMEM = std::max<size_t>((size_t)DL_WARPS * 2 * DL_STAGE * 8, 2 * SOLO_NEXT * 16);
 static_assert(2 * SOLO_NEXT * 16 <= DL_SMEM, "the solo phase uses the warps' stages");
-constexpr unsigned DL_SPIN_LIMIT = 1u << 26;             // polls of a barrier before a block gives up (tens of seconds)
 
 struct Ix {
     const unsigned long long* cursor;  // direct form: ends of the groups in `pay`, for keys below `domain`
@@ -105,7 +104,10 @@ struct Ctl {
     unsigned abort;
     // what block 0 found when it ran on alone
     unsigned solo_turns;            // solo phases that are over
-    unsigned solo_phase, solo_check, pad;
+    unsigned solo_phase, solo_check;
+    // Work that touches none of the slots' counters for long counts up here, so that those who wait for it
+    // can tell it from work that is not going on.
+    unsigned beat;
     unsigned long long solo_start, solo_end, solo_iterations, solo_candidates;
     Slot slot[3];
     // rows evaluated one warp each: what they came to, and what was given up (read by the host)
@@ -153,7 +155,10 @@ struct Out {
     Ctl* ctl;
     DevStatus* st;
     unsigned int* visited_t;  // square components: the transpose, brought along
+    unsigned spin_limit;      // polls without anything going on before a block gives up waiting
 };
+constexpr unsigned DL_BEAT_OUTPUTS = 1u << 22, DL_BEAT_ITEMS = 4096, DL_BEAT_GROUPS = 8, DL_BEAT_TURNS = 1024;  // work between two beats
+__device__ __forceinline__ void beat(const Out& o) { atomicAdd(&o.ctl->beat, 1u); }
 
 __device__ __forceinline__ void mark_transposed(const Out& o, uint64_t t) {
     const uint32_t h = (uint32_t)(t >> 32);
@@ -424,7 +429,10 @@ __device__ __forceinline__ bool take_rows(const Out& o, const Rules& rules, uint
             one.l2 = __shfl_sync(FULL, me.l2, r);
             one.before = 0;
             const uint64_t all = __shfl_sync(FULL, cnt, r);
-            for (uint64_t at = 0; at < all; at += 1u << 30) emit<SINGLE, DL_UNROLL>(o, ru, one, 0, at, (uint32_t)(all - at < (1u << 30) ? all - at : 1u << 30), check, sink);
+            for (uint64_t at = 0; at < all; at += DL_BEAT_OUTPUTS) {
+                emit<SINGLE, DL_UNROLL>(o, ru, one, 0, at, (uint32_t)(all - at < DL_BEAT_OUTPUTS ? all - at : DL_BEAT_OUTPUTS), check, sink);
+                if (lane == 0) beat(o);
+            }
         }
     }
     return any_listed;
@@ -474,6 +482,7 @@ __device__ __forceinline__ void take_square(const Out& o, const Square& sq, uint
         }
         const uint64_t total = __shfl_sync(FULL, incl, 31), before = incl - len;
         for (uint64_t i0 = 0; i0 < total; i0 += 32) {
+            if (i0 && i0 % DL_BEAT_ITEMS == 0 && lane == 0) beat(o);
             const uint64_t i = i0 + lane;
             int owner = 0;
 #pragma unroll
@@ -586,6 +595,7 @@ __device__ __forceinline__ void square_full(const Out& o, const Square& sq, uint
         const uint32_t key = x.row_key == 0 ? h : l;
         atomicAdd(&x.counts[key], (unsigned long long)len);
         for (uint32_t i = 0; i < len; ++i) {
+            if ((i + 1) % DL_BEAT_ITEMS == 0) beat(o);
             const uint32_t m = other_of(x.ix, s + i);
             if (m >> sq.bits) {
                 set_status(o.st, XLB_ERR_CAPACITY, 17, m);
@@ -648,6 +658,7 @@ __device__ __forceinline__ void solo(const Out& o, const Rules& rules, Heavy* he
         return;
     }
     for (unsigned turn = 0;; turn = turn == 2 ? 0 : turn + 1) {
+        if (threadIdx.x == 0 && st.iterations % DL_BEAT_TURNS == 0) beat(o);
         const unsigned after = turn == 2 ? 0 : turn + 1;  // (its counters were read last two barriers ago)
         if (threadIdx.x == 0) {
             sh.count[after] = 0;
@@ -705,17 +716,33 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
     WarpSink sink{o, stage_s + warp * (2 * DL_STAGE)};
     unsigned passed = 0, solo_turns = 0;
     Ctl* ctl = o.ctl;
-    // A bounded wait (one thread): until `done` holds of the word.
+    // A bounded wait (one thread): until `done` holds of the word.  An iteration may take any time, so
+    // what is bounded is the time in which nothing that the others do can be seen.
+    auto going_on = [&]() {
+        unsigned v = *(volatile unsigned*)&ctl->beat;
+        for (int k = 0; k < 3; ++k) {
+            const volatile Slot* s = &ctl->slot[k];
+            v += (unsigned)s->count + s->next_heavy + s->next_chunk;
+        }
+        return v;
+    };
     auto wait_for = [&](const unsigned* word, unsigned sleep, auto done) {
-        unsigned v;
+        unsigned v, seen = going_on();
         for (unsigned polls = 0;; ++polls) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
             if (done(v)) return true;
-            if (polls > DL_SPIN_LIMIT || *(volatile unsigned*)&ctl->abort) {
+            if (polls > o.spin_limit) {
+                const unsigned now = going_on();
+                if (now != seen) {
+                    seen = now;
+                    polls = 0;
+                    continue;
+                }
                 *(volatile unsigned*)&ctl->abort = 1;
                 set_status(o.st, XLB_ERR_TIMEOUT, 14, passed);
                 return false;
             }
+            if (*(volatile unsigned*)&ctl->abort) return false;
             if (sleep) __nanosleep(sleep);
         }
     };
@@ -795,7 +822,9 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
             if (SQUARE) {
                 // A row of a square component can stand for any amount of work, and rows of one hub lie
                 // side by side: every warp takes rows far apart, eight at a time.
+                unsigned groups = 0;
                 for (uint64_t first = me; first < n; first += 8 * warps) {
+                    if (++groups % DL_BEAT_GROUPS == 0 && lane == 0) beat(o);
                     const unsigned rows = (unsigned)min((n - first + warps - 1) / warps, (uint64_t)8);
                     const uint64_t row = lane < rows ? o.log[start + first + lane * warps] : 0;
                     unsigned linear = 0;
@@ -1308,7 +1337,7 @@ __global__ void delta_rows_left_k(Ctl* c) {
 }  // namespace
 
 static Out out_of(xlb_ctx* c, const DeltaLoop& d) {
-    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, (Ctl*)d.ctl, c->d_status, d.square ? d.visited->as<unsigned int>() + d.words : nullptr};
+    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, (Ctl*)d.ctl, c->d_status, d.square ? d.visited->as<unsigned int>() + d.words : nullptr, c->delta_spin_limit};
 }
 
 DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square, int composites) {

@@ -2029,7 +2029,13 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         DeltaResult res;
         {
             PhaseTimer t(c, &rs.st.ms_join);
-            ops_delta_run(c, d, run, variants, c->max_iterations - it, full, &res);
+            try {
+                ops_delta_run(c, d, run, variants, c->max_iterations - it, full, &res);
+            } catch (const XlbError& e) {
+                if (e.st != XLB_ERR_TIMEOUT) throw;
+                rs.st = before;  // a wait inside the loop ran out: the routes without one start over
+                return false;
+            }
         }
         it += res.iterations;
         rs.st.iterations += res.iterations;

@@ -1174,6 +1174,7 @@ extern "C" xlb_status xlb_ctx_create(const xlb_config* cfg, xlb_ctx** out) {
         c->max_iterations = cfg && cfg->max_iterations ? cfg->max_iterations : 1000000ull;
         c->join_chunk = cfg ? cfg->join_chunk_tuples : 0;
         c->flags = cfg ? cfg->flags : 0;
+        if (const char* polls = getenv("XLB_DELTA_POLLS")) c->delta_spin_limit = (unsigned)strtoul(polls, nullptr, 10);  // (tests)
         CUDA_OK(cudaHostAlloc((void**)&c->h_scalar, SCALAR_WORDS * 8, cudaHostAllocMapped));
         CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_scalar_dev, c->h_scalar, 0));
         memset(c->h_scalar, 0, SCALAR_WORDS * 8);
