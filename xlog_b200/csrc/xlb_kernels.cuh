@@ -314,7 +314,7 @@ struct SelectTiles {
                 const unsigned need = whole ? (whole & (0u - whole)) * 2u - 1u : FULL;  // up to the first sum
                 if ((ready & need) != need) {
                     if (++spins > spin_limit) {
-                        if (lane == 0) set_status(st, XLB_ERR_TIMEOUT, 21, tile);
+                        if (lane == 0) set_status(st, XLB_ERR_TIMEOUT, 23, tile);
                         break;
                     }
                     __nanosleep(20);
