@@ -90,9 +90,9 @@ enum Phase { PH_ROWS = 0, PH_HEAVY = 1, PH_SOLO = 2, PH_DONE = 3, PH_FULL = 4 };
 // that is late.  A solo phase that ends an iteration by itself touches none.
 struct Slot {
     unsigned long long count, cand;  // tuples appended to the log; candidates
-    unsigned heavy_n, next_heavy;    // pieces of long rows listed, taken
+    unsigned long long heavy_n;      // pieces of long rows, listed or not (rows that found the list full go on raising it)
+    unsigned next_heavy;             // pieces taken
     unsigned next_chunk;             // rows are taken in batches
-    unsigned pad;
 };
 struct Ctl {
     // in: where the loop stands; out: where it stopped (read by the host)
@@ -408,12 +408,12 @@ __device__ __forceinline__ bool take_rows(const Out& o, const Rules& rules, uint
             const uint64_t pieces = (cnt + DL_PIECE - 1) / DL_PIECE;
             bool listed = false;
             if (pieces <= DL_HEAVY_MAX) {
-                const unsigned h = atomicAdd(&slot->heavy_n, (unsigned)pieces);
+                const uint64_t h = atomicAdd(&slot->heavy_n, (unsigned long long)pieces);
                 if (h <= DL_HEAVY_MAX - pieces) {
                     for (unsigned k = 0; k < pieces; ++k) heavy[h + k] = {me.row, (unsigned)q, k};
                     listed = true;
                 } else {
-                    for (unsigned k = h; k < DL_HEAVY_MAX; ++k) heavy[k] = {0, ~0u, 0};  // the room that was left: nothing to do there
+                    for (uint64_t k = h; k < DL_HEAVY_MAX; ++k) heavy[k] = {0, ~0u, 0};  // the room that was left: nothing to do there
                 }
             }
             any_listed = true;  // (the count was raised either way)
@@ -863,7 +863,8 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
                 return;
         } else if (phase == PH_HEAVY) {
             clear_next();
-            const unsigned listed = __ldcg(&slot->heavy_n), pieces = listed < DL_HEAVY_MAX ? listed : (unsigned)DL_HEAVY_MAX;
+            const uint64_t listed = __ldcg(&slot->heavy_n);
+            const unsigned pieces = listed < DL_HEAVY_MAX ? (unsigned)listed : (unsigned)DL_HEAVY_MAX;
             for (;;) {
                 unsigned item = 0;
                 if (lane == 0) item = atomicAdd(&slot->next_heavy, 1u);
