@@ -2402,8 +2402,12 @@ static bool rank32(uint8_t t) { return t == XLB_U32 || t == XLB_SYMBOL; }
 // Plans over 32-bit columns run on ranks, too, when the values are spread thin over a wide range (ids
 // that carry a kind or an address in their upper bits): a head of two columns of more than 16 bits has
 // no bitmap, and its candidates would each be hashed and grouped; where there are at most 2^16
-// different values, their ranks fit one.  Finding that out costs a pass over the relations and, above
-// 28 bits, a sort of their values: not worth it for a handful of rows.
+// different values, their ranks fit one.  Finding that out costs a pass over the relations (above 28 bits
+// one that ends when there are more values than that): not worth it for a handful of rows.
+//   Where the line lies: a bitmap of 32 bits costs some 300 us to clear, read and write off whatever is in it.
+// Paths of 4 / 64 / 1024 nodes over 30 000 values of 28 bits (30 bits of bitmap): 409 / 1370 / 15 200 us on ranks,
+// 581 / 6475 / 101 700 on hash sets; over 60 000 (32 bits): 884 / 2900 / 31 000 against 597 / 6770 / 106 900.
+// How deep a program goes is not known here, and what 32 bits lose on the shallowest they win many times over.
 // Values of 15 and 16 bits have a bitmap, but one of 128 or 512 MB that is cleared, counted and read off
 // for whatever little is in it (closure of 1024 rows over 64 values of 16 bits: 573 us, on ranks 153): they
 // take ranks, too, where that makes the bitmap a sixteenth and the rows are few.

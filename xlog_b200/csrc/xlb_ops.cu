@@ -625,12 +625,13 @@ DenseSet ops_dense_begin_state(xlb_ctx* c, DenseState& s) {
     return d;
 }
 
-static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total, const Buf* cols = nullptr);
+static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total, const Buf* cols = nullptr, uint64_t at_most = ~0ull);
 Keys ops_dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full) { return dense_finish(c, d, full, nullptr); }
 
 // known_total: the number of rows that will come out, when the host knows it already (no read-back)
 // cols: where they go as columns (the second may be null) instead of packed; needs known_total
-static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total, const Buf* cols) {
+// at_most: with more rows than that only their number comes out
+static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64_t* known_total, const Buf* cols, uint64_t at_most) {
     Keys o;
     o.bound = d.bound;
     const uint64_t words = d.words;
@@ -671,6 +672,7 @@ static Keys dense_finish(xlb_ctx* c, DenseSet& d, const Keys& full, const uint64
     d.marked = both[1];
     prof_add_bytes(c, "expand_mark", d.marked * 4ull);
     o.n = tot;
+    if (tot > at_most) return o;
     uint32_t* c0 = cols ? cols[0]->as<uint32_t>() : nullptr;
     uint32_t* c1 = cols && cols[1] ? cols[1]->as<uint32_t>() : nullptr;
     if (!cols) o.buf = make_buf(c, tot * 8);
@@ -1931,6 +1933,50 @@ __global__ void __launch_bounds__(BLOCK) rank_list_k(const uint64_t* __restrict_
         if (halves == 2) out[n + i] = k >> 32;
     }
 }
+// Their set: a table of (value | 2^32), 0 where it is free, while there are at most `most` of them.  Blocks stop
+// adding when there are more; the table has room for what those under way still add.
+constexpr int RF_ROWS = 4, RF_SEEN = 1024;
+__global__ void __launch_bounds__(BLOCK) rank_find_k(const uint64_t* __restrict__ rows, uint64_t n, int halves, unsigned long long* table, uint64_t mask, volatile unsigned* found, unsigned most) {
+    __shared__ unsigned long long seen[RF_SEEN];  // values that some thread of the block is seeing to (a hub's many rows would queue for its slot)
+    for (int i = threadIdx.x; i < RF_SEEN; i += BLOCK) seen[i] = 0;
+    __syncthreads();
+    const uint64_t step = (uint64_t)gridDim.x * BLOCK;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i0 < n; i0 += RF_ROWS * step) {
+        uint64_t k[RF_ROWS];
+#pragma unroll
+        for (int u = 0; u < RF_ROWS; ++u) k[u] = i0 + u * step < n ? rows[i0 + u * step] : rows[i0];
+#pragma unroll
+        for (int u = 0; u < RF_ROWS; ++u)
+            for (int h = 0; h < halves; ++h) {
+                const unsigned long long v = (1ull << 32) | (h ? k[u] >> 32 : k[u] & 0xFFFFFFFFull);
+                const uint64_t x = mix64(v);
+                if (atomicExch(&seen[(x >> 40) & (RF_SEEN - 1)], v) == v) continue;
+                uint64_t at = x & mask;
+                for (uint64_t probe = 0; probe <= mask; ++probe) {  // bounded by the table size
+                    unsigned long long cur = table[at];
+                    if (!cur) {
+                        if (*found > most) return;
+                        cur = atomicCAS(&table[at], 0ull, v);
+                        if (!cur) {
+                            atomicAdd((unsigned*)found, 1u);
+                            break;
+                        }
+                    }
+                    if (cur == v) break;
+                    at = (at + 1) & mask;
+                }
+            }
+    }
+}
+struct PredSlot {
+    const uint64_t* table;
+    __device__ __forceinline__ bool operator()(uint64_t i) const { return table[i] != 0; }
+};
+struct EmitSlot {
+    const uint64_t* table;
+    uint64_t* out;
+    __device__ __forceinline__ void operator()(uint64_t i, uint64_t pos) const { out[pos] = (uint32_t)table[i]; }
+};
 __global__ void __launch_bounds__(BLOCK) rank_encode_k(const uint64_t* __restrict__ rows, uint64_t n, int halves, const uint64_t* __restrict__ dict, uint64_t m,
                                                       uint64_t* __restrict__ out, DevStatus* st) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
@@ -1961,6 +2007,7 @@ __global__ void __launch_bounds__(BLOCK) rank_decode_k(const uint64_t* __restric
 }
 }  // namespace
 
+constexpr uint64_t RANK_SORT_MAX = 1ull << 17;  // values
 bool ops_rank_build(xlb_ctx* c, const std::vector<const xlb_rel*>& rels, int bits, uint64_t most, Keys* dict) {
     uint64_t total = 0;
     for (const xlb_rel* r : rels) total += r->rows * r->schema.arity;
@@ -1976,7 +2023,28 @@ bool ops_rank_build(xlb_ctx* c, const std::vector<const xlb_rel*>& rels, int bit
             check_launch(c, "dict_image");
         }
         Keys none;
-        *dict = ops_dense_finish(c, d, none);
+        *dict = dense_finish(c, d, none, nullptr, nullptr, most);
+    } else if (total > RANK_SORT_MAX) {
+        // Their set first, and only that is sorted; or it turns out too large, and the search for it ends.  (Closure
+        // of paths of four nodes, ids of 30 bits: 1 M rows of as many values 1018 us when all were sorted to see
+        // how many there are, 912 so; 20 M rows of 2 M values 4496 -> 2793; 878 and 2794 on the route taken then.
+        // Few rows are sorted faster than looked up: 32 K values, 16 000 different, 284 against 305.)
+        uint64_t cap = 1ull << 18;
+        while (cap < 4 * most) cap <<= 1;
+        Buf table = make_buf(c, cap * 8 + 8);
+        CUDA_OK(set_async(c, table->p, 0, cap * 8 + 8));
+        for (const xlb_rel* r : rels) {
+            if (!r->rows) continue;
+            Keys k = ops_rel_packed(c, r);
+            prof_begin(c, "dict_image", k.n * 8ull);
+            rank_find_k<<<std::min(grid_for(c, k.n, BLOCK * RF_ROWS), 2u * c->sm_count), BLOCK, 0, c->stream>>>(k.ptr(), k.n, (int)r->schema.arity, table->as<unsigned long long>(), cap - 1,
+                                                                                                              (unsigned*)(table->as<uint64_t>() + cap), (unsigned)most);
+            check_launch(c, "dict_image");
+        }
+        dict->buf = make_buf(c, cap * 8);
+        dict->bound = all;
+        dict->n = select(c, PredSlot{table->as<uint64_t>()}, EmitSlot{table->as<uint64_t>(), dict->buf->as<uint64_t>()}, cap);
+        if (dict->n <= most) ops_sort(c, *dict);
     } else {
         dict->n = total;
         dict->bound = all;
