@@ -36,34 +36,14 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // One lane of each group clears the word again (match_clear) once all have read it.
 // (The match.any instruction costs more the more different values there are, and radix digits are
 // close to all different.)
-#ifndef XLB_RANK
-#define XLB_RANK 2
-#endif
 __device__ __forceinline__ unsigned match_digit(unsigned d, unsigned* table) {
-#if XLB_RANK == 1
-    return __match_any_sync(FULL, d);
-#elif XLB_RANK == 2
     atomicOr(&table[d], 1u << lane_id());
     __syncwarp();
     const unsigned peers = table[d];
     __syncwarp();
     return peers;
-#else
-    unsigned peers = FULL;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        bool bit = (d >> b) & 1u;
-        unsigned vote = __ballot_sync(FULL, bit);
-        peers &= bit ? vote : ~vote;
-    }
-    return peers;
-#endif
 }
-__device__ __forceinline__ void match_clear(unsigned d, unsigned* table) {
-#if XLB_RANK == 2
-    table[d] = 0;
-#endif
-}
+__device__ __forceinline__ void match_clear(unsigned d, unsigned* table) { table[d] = 0; }
 
 __device__ __forceinline__ void set_status(DevStatus* st, unsigned code, unsigned where, unsigned long long detail) {
     if (atomicCAS(&st->code, 0u, code) == 0u) {
@@ -1320,17 +1300,6 @@ __device__ __forceinline__ uint64_t warp_partition_point(uint64_t n, Pred pred) 
 // ------------------------------------------------------------------------------ merge path
 constexpr int MP_IPT = 8;
 constexpr int MP_TILE = BLOCK * MP_IPT;  // 2048 merged elements per tile
-
-// Number of A elements among the first `diag` merged elements (A first on ties).
-__device__ __forceinline__ uint64_t merge_path(const uint64_t* A, uint64_t na, const uint64_t* B, uint64_t nb, uint64_t diag) {
-    uint64_t lo = diag > nb ? diag - nb : 0, hi = diag < na ? diag : na;
-    while (lo < hi) {
-        uint64_t mid = (lo + hi) >> 1;
-        if (A[mid] <= B[diag - 1 - mid]) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
 
 // MODE 0: keep[i] = 1 iff A[i] is not in B (A, B sorted unique).
 // MODE 1: out = merge of A and B (disjoint), out has na + nb entries.
