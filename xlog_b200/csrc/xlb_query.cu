@@ -148,15 +148,15 @@ __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned
 //   The rows of a hub queue for its slot and on its count, some 10 ns each, so a build side of 2 JOIN_SAMPLE
 // rows and more is looked at first: while the other blocks clear the slots, one picks rows evenly and
 // reports a key that it meets far more often than one of JOIN_GROUP_MAX rows could be.  (2 M build rows, 4 M
-// probe rows, B200: one key of 1000 rows 951 -> 801 us, one of 1 M that no probe row asks for 1590 -> 690; the
-// sort alone, before there was this route, 768 and 673; keys of at most 64 rows 398 -> 404 for the sample.)
+// probe rows, B200: one key of 1000 rows 947 -> 797 us, one of 1 M that no probe row asks for 1592 -> 685; the
+// sort alone, before there was this route, 768 and 673; keys of at most 64 rows 393 -> 396 for the sample.)
 constexpr unsigned JOIN_GROUP_MAX = 64;
 constexpr unsigned JOIN_SAMPLE = 1024;  // (a row a thread: a chain of latencies as long as the clearing)
 __global__ void __launch_bounds__(JOIN_SAMPLE) group_clear_k(KeyCols keys, uint64_t n, uint4* __restrict__ slots, uint64_t slot_vecs, uint64_t* __restrict__ words, uint64_t nwords,
                                                             unsigned int* too_long) {
-    const unsigned clearing = gridDim.x - 1;  // blocks; the last one has the words and the sample
-    if (blockIdx.x < clearing) {
-        for (uint64_t i = (uint64_t)blockIdx.x * JOIN_SAMPLE + threadIdx.x; i < slot_vecs; i += (uint64_t)clearing * JOIN_SAMPLE) slots[i] = make_uint4(0, 0, 0, 0);
+    if (blockIdx.x > 0) {  // (the first block, which starts at once, has the words and the sample)
+        const uint64_t step = (uint64_t)(gridDim.x - 1) * JOIN_SAMPLE;
+        for (uint64_t i = (uint64_t)(blockIdx.x - 1) * JOIN_SAMPLE + threadIdx.x; i < slot_vecs; i += step) slots[i] = make_uint4(0, 0, 0, 0);
         return;
     }
     __shared__ uint64_t key_s[JOIN_SAMPLE];
@@ -594,7 +594,7 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     uint64_t* words = slots->as<uint64_t>() + cap;  // [0] outputs, [1] a group is too long, [2] room taken for groups, then the sweep's
     unsigned int* too_long = (unsigned int*)(words + 1);
     prof_begin(c, "group_clear", cap * 8ull);
-    group_clear_k<<<(unsigned)std::min<uint64_t>((cap / 2 + JOIN_SAMPLE - 1) / JOIN_SAMPLE, 4ull * c->sm_count) + 1, JOIN_SAMPLE, 0, c->stream>>>(build, n, slots->as<uint4>(), cap / 2, words, clear / 8 - cap, too_long);
+    group_clear_k<<<(unsigned)std::min<uint64_t>((cap / 2 + JOIN_SAMPLE - 1) / JOIN_SAMPLE, 2ull * c->sm_count) + 1, JOIN_SAMPLE, 0, c->stream>>>(build, n, slots->as<uint4>(), cap / 2, words, clear / 8 - cap, too_long);
     check_launch(c, "group_clear");
     prof_begin(c, "hash_insert", n * 8ull);
     group_count_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, rep, count, cap - 1, place->as<uint2>(), too_long, c->d_status);
