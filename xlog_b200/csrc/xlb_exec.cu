@@ -2409,7 +2409,7 @@ static bool rank32(uint8_t t) { return t == XLB_U32 || t == XLB_SYMBOL; }
 // 581 / 6475 / 101 700 on hash sets; over 60 000 (32 bits): 884 / 2900 / 31 000 against 597 / 6770 / 106 900.
 // How deep a program goes is not known here, and what 32 bits lose on the shallowest they win many times over.
 // Values of 15 and 16 bits have a bitmap, but one of 128 or 512 MB that is cleared, counted and read off
-// for whatever little is in it (closure of 1024 rows over 64 values of 16 bits: 573 us, on ranks 153): they
+// for whatever little is in it (closure of 1024 rows over 64 values of 16 bits: 573 us, on ranks 164): they
 // take ranks, too, where that makes the bitmap a sixteenth and the rows are few.
 constexpr uint64_t SPARSE_VALUES = 1ull << 16, SPARSE_ROWS_MIN = 64, SPARSE_ROWS_MAX = 1ull << 26, SPARSE_ROWS_FEW = 1ull << 22;
 constexpr int SPARSE_BITS_MIN = 15;
