@@ -19,8 +19,9 @@ namespace {
 
 // (Measured on the cases the comment above names, 32 warps with 2 outputs a lane in flight against 24
 // warps, 16 warps, 4 outputs and 8 outputs: closure 299 us against 320 to 504, banded DAG 935 against
-// 993 to 1503, same generation 779 against 846 to 1300.  The loop is bound by the instructions and the
-// latency of short rows, not by bandwidth: more in flight per warp is work for rows that are not there.)
+// 993 to 1503, same generation 779 against 846 to 1300.  The loop is bound by the latency of short rows'
+// chains and by warps that wait for the others at the barriers, not by bandwidth or issue slots, of which 17 to
+// 24 % are used: more in flight per warp is work for rows that are not there.)
 constexpr int DL_THREADS = 1024, DL_WARPS = DL_THREADS / 32;
 constexpr int DL_UNROLL = 2;                             // outputs a lane has in flight
 constexpr int DL_STAGE = 128;                            // new tuples a warp collects before it reserves room in the log
@@ -1002,8 +1003,9 @@ __global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
 // reach(x, y), edge(y, z)), what is derived for one x depends on nothing derived for another.  A
 // block takes an x, holds its row of the head's bitmap and the frontier of its search in shared memory and
 // goes level by level to the end: no barrier between blocks, no atomics and no log in global memory.
-// Its levels are the iterations of the loop, and its candidates the loop's.  Latency of one instruction
-// after the other bounds it, not memory: hence several warps a row where rows are few, four outputs a
+// Its levels are the iterations of the loop, and its candidates the loop's.  Instructions one after the
+// other bound it (issue slots 68 % used on 2000 nodes of degree 5; 20 % on a chain, where one warp of four has
+// something to do), not memory: hence several warps a row where rows are few, four outputs a
 // lane in flight, and a path of its own for a frontier of one value.  (Loop -> this, B200: chain of 1500
 // nodes 3279 -> 498 us, banded DAG of 2^14 nodes 961 -> 472, 2000 nodes of degree 5 276 -> 113, four
 // blocks of 128 nodes 181 -> 66; one warp a row with one output a lane in flight: 1089, 1238, 185, 698.)
