@@ -361,7 +361,7 @@ struct xlb_ctx {
     std::string prof_filter;  // "" = off, "*" = every kernel, else kernel names separated by commas
     ProfEntry* prof_open = nullptr;
     cudaEvent_t prof_e0 = nullptr;
-    cudaError_t error_before = cudaSuccess;  // what was on the thread when the launch at hand began (nothing, if every call is checked)
+    cudaError_t error_before = cudaSuccess;  // what was on the thread when the operation at hand began (nothing, if every call is checked)
     // host timeline of one plan execution (XLB_TRACE_HOST=1): every launch and every wait with its
     // wall-clock interval, printed to stderr when the plan is done
     struct TraceNote {
@@ -386,7 +386,6 @@ inline void trace_note(xlb_ctx* c, const char* what, double t0) {
 
 // Bracket one launch with CUDA events on the launching stream when its kernel is profiled.
 inline void prof_begin(xlb_ctx* c, const char* name, uint64_t bytes) {
-    c->error_before = cudaPeekAtLastError();
     if (c->trace_on) trace_note(c, name, trace_now());
     if (c->prof_filter.empty()) return;
     if (c->prof_filter != "*") {  // a kernel name, or several separated by commas
@@ -457,11 +456,9 @@ inline void check_launch(xlb_ctx* c, const char* what) {
         c->prof_open->pending.emplace_back(c->prof_e0, e1);
         c->prof_open = nullptr;
     }
-    const cudaError_t before = c->error_before, e = launched;
-    c->error_before = cudaSuccess;
-    if (e == cudaSuccess) return;
-    if (before != cudaSuccess) xlb_fail(XLB_ERR_CUDA, "an error from before the launch of %s: %s", what, cudaGetErrorString(before));
-    xlb_fail(XLB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
+    if (launched == cudaSuccess) return;
+    if (c->error_before != cudaSuccess) xlb_fail(XLB_ERR_CUDA, "an error from before the operation, found at the launch of %s: %s", what, cudaGetErrorString(c->error_before));
+    xlb_fail(XLB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(launched));
 }
 
 // Copies and fills enqueued on the context's stream.

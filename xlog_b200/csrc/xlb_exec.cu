@@ -2640,6 +2640,7 @@ extern "C" xlb_status xlb_execute_plan(xlb_ctx* c, const xlb_plan* plan, xlb_run
     c->peak = c->allocated;
     xlb_status result = XLB_OK;
     try {
+        c->error_before = cudaPeekAtLastError();
         CUDA_OK(cudaSetDevice(c->device));
         if (!c->plan_e0) CUDA_OK(cudaEventCreate(&c->plan_e0));
         if (!c->plan_e1) CUDA_OK(cudaEventCreate(&c->plan_e1));

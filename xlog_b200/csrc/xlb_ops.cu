@@ -1139,7 +1139,10 @@ Keys ops_partition_by_owner_dev(xlb_ctx* c, const Keys& in, int keysel, uint32_t
 #define API_BEGIN(ctxp) \
     xlb_ctx* ctx__ = (ctxp); \
     try {                    \
-        if (ctx__) CUDA_OK(cudaSetDevice(ctx__->device));
+        if (ctx__) {       \
+            ctx__->error_before = cudaPeekAtLastError(); \
+            CUDA_OK(cudaSetDevice(ctx__->device)); \
+        }
 #define API_END()                                  \
     }                                              \
     catch (const XlbError& e) {                    \
