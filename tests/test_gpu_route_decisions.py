@@ -19,8 +19,8 @@ def p():
     prov.close()
 
 
-# (the build side is sampled from 2048 rows on; a key of half of them is met there, one of 65 only when counted)
-@pytest.mark.parametrize("nr,longest", [(64, 64), (65, 65), (2047, 2047), (2048, 64), (2048, 65), (2048, 2048), (2049, 1025), (300_000, 64), (300_000, 65), (300_000, 4000), (300_000, 150_000), (300_000, 300_000)])
+# (the build side is sampled from 65536 rows on; a key of half of them is met there, one of 65 only when counted)
+@pytest.mark.parametrize("nr,longest", [(64, 64), (65, 65), (2049, 1025), (65_535, 65_535), (65_536, 64), (65_536, 65), (65_536, 65_536), (65_537, 32_769), (300_000, 64), (300_000, 65), (300_000, 4000), (300_000, 150_000), (300_000, 300_000)])
 @pytest.mark.parametrize("dtype", [np.uint32, np.uint64])
 def test_join_with_one_long_key(p, nr, longest, dtype):
     rng = np.random.default_rng(nr + longest)

@@ -145,13 +145,15 @@ __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned
 // sums of the counts.  The numbers come in no particular order, so each group's rows are put in row
 // order afterwards, which for the usual handful is a few compares.  A group above JOIN_GROUP_MAX rows
 // is reported when it is met, the launches behind end at once, and the caller sorts instead.
-//   The rows of a hub queue for its slot and on its count, some 10 ns each, so a build side of 2 JOIN_SAMPLE
+//   The rows of a hub queue for its slot and on its count, some 13 ns each, so a build side of JOIN_SAMPLED
 // rows and more is looked at first: while the other blocks clear the slots, one picks rows evenly and
-// reports a key that it meets far more often than one of JOIN_GROUP_MAX rows could be.  (2 M build rows, 4 M
-// probe rows, B200: one key of 1000 rows 947 -> 797 us, one of 1 M that no probe row asks for 1592 -> 685; the
-// sort alone, before there was this route, 768 and 673; keys of at most 64 rows 393 -> 396 for the sample.)
+// reports a key that it meets JOIN_OFTEN times, which one of JOIN_GROUP_MAX rows cannot be.  (2 M build rows,
+// 4 M probe rows, B200: one key of 1000 rows 947 -> 797 us, one of 1 M that no probe row asks for 1592 -> 685; the
+// sort alone, before there was this route, 768 and 673; keys of at most 64 rows 393 -> 396.  The sample costs
+// some 3 us of 200, so smaller build sides go without: 32 768 rows all of one key 122 us sampled, 138 counted.)
 constexpr unsigned JOIN_GROUP_MAX = 64;
-constexpr unsigned JOIN_SAMPLE = 1024;  // (a row a thread: a chain of latencies as long as the clearing)
+constexpr unsigned JOIN_SAMPLE = 1024, JOIN_OFTEN = 16;  // (a row a thread: a chain of latencies as long as the clearing)
+constexpr uint64_t JOIN_SAMPLED = 1ull << 16;
 __global__ void __launch_bounds__(JOIN_SAMPLE) group_clear_k(KeyCols keys, uint64_t n, uint4* __restrict__ slots, uint64_t slot_vecs, uint64_t* __restrict__ words, uint64_t nwords,
                                                             unsigned int* too_long) {
     if (blockIdx.x > 0) {  // (the first block, which starts at once, has the words and the sample)
@@ -162,17 +164,15 @@ __global__ void __launch_bounds__(JOIN_SAMPLE) group_clear_k(KeyCols keys, uint6
     __shared__ uint64_t key_s[JOIN_SAMPLE];
     __shared__ unsigned count_s[JOIN_SAMPLE], rep_s[2 * JOIN_SAMPLE];
     const unsigned me = threadIdx.x;
-    const bool sample = n >= 2 * JOIN_SAMPLE;
-    const uint64_t key = sample ? keys(me * n / JOIN_SAMPLE) : 0;
+    const uint64_t key = keys(me * n / JOIN_SAMPLE);
     for (uint64_t i = me; i < nwords; i += JOIN_SAMPLE) words[i] = 0;
     count_s[me] = rep_s[me] = rep_s[me + JOIN_SAMPLE] = 0;
     key_s[me] = key;
     __syncthreads();
-    if (!sample) return;
     for (unsigned h = (unsigned)mix64(key);; ++h) {  // (half of the slots stay free)
         const unsigned at = h & (2 * JOIN_SAMPLE - 1), cur = atomicCAS(&rep_s[at], 0u, me + 1);
         if (cur && key_s[cur - 1] != key) continue;
-        if (atomicAdd(&count_s[cur ? cur - 1 : me], 1u) >= 11 + (unsigned)(3 * JOIN_GROUP_MAX * JOIN_SAMPLE / n)) *too_long = 1;
+        if (atomicAdd(&count_s[cur ? cur - 1 : me], 1u) + 1 >= JOIN_OFTEN) *too_long = 1;
         break;
     }
 }
@@ -593,9 +593,13 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     unsigned int *rep = slots->as<unsigned int>(), *count = rep + cap;
     uint64_t* words = slots->as<uint64_t>() + cap;  // [0] outputs, [1] a group is too long, [2] room taken for groups, then the sweep's
     unsigned int* too_long = (unsigned int*)(words + 1);
-    prof_begin(c, "group_clear", cap * 8ull);
-    group_clear_k<<<(unsigned)std::min<uint64_t>((cap / 2 + JOIN_SAMPLE - 1) / JOIN_SAMPLE, 2ull * c->sm_count) + 1, JOIN_SAMPLE, 0, c->stream>>>(build, n, slots->as<uint4>(), cap / 2, words, clear / 8 - cap, too_long);
-    check_launch(c, "group_clear");
+    if (n < JOIN_SAMPLED) {
+        CUDA_OK(set_async(c, slots->p, 0, clear));
+    } else {
+        prof_begin(c, "group_clear", cap * 8ull);
+        group_clear_k<<<(unsigned)std::min<uint64_t>((cap / 2 + JOIN_SAMPLE - 1) / JOIN_SAMPLE, 2ull * c->sm_count) + 1, JOIN_SAMPLE, 0, c->stream>>>(build, n, slots->as<uint4>(), cap / 2, words, clear / 8 - cap, too_long);
+        check_launch(c, "group_clear");
+    }
     prof_begin(c, "hash_insert", n * 8ull);
     group_count_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, rep, count, cap - 1, place->as<uint2>(), too_long, c->d_status);
     check_launch(c, "hash_insert");
