@@ -52,6 +52,42 @@ def test_closure(edge, program, monkeypatch):
         assert np.array_equal(g, w)
 
 
+def paths(tail):
+    """A path of 33 to 70 edges that ends in nothing, in a loop back, in a branch that closes again (and a second path
+    behind it), in a value with 40 matches: what a row that is followed as a path can run into."""
+    a, b = list(range(70)), list(range(1, 71))
+    if tail == "loop":
+        a, b = a + [70], b + [3]
+    elif tail == "itself":
+        a, b = a + [70], b + [70]
+    elif tail == "branch":
+        a, b = a + [70, 70, 71, 72] + list(range(73, 140)), b + [71, 72, 73, 73] + list(range(74, 141))
+    elif tail == "fan":
+        a, b = a + [70] * 40, b + list(range(71, 111))
+    return np.array(a, np.uint32), np.array(b, np.uint32)
+
+
+# (ids up to 2^11 and 2^14: every value has an entry in a row's queue; up to 2^15: it has not)
+@pytest.mark.parametrize("top", [200, 2047, (1 << 14) - 1, (1 << 15) - 1])
+@pytest.mark.parametrize("tail", ["end", "loop", "itself", "branch", "fan"])
+def test_rows_that_follow_a_path(tail, top, monkeypatch):
+    edge = [np.where(x == 0, top, x).astype(np.uint32) for x in paths(tail)]
+    both(programs.transitive_closure(), {"edge": edge}, "reach", monkeypatch)
+
+
+@pytest.mark.parametrize("limit", [31, 32, 33, 34, 69, 70])
+def test_iteration_limit_on_a_path(limit):
+    p = KernelProvider(device=0, max_iterations=limit)
+    if limit == 70:  # 71 nodes
+        got, stats = run_program(p, programs.transitive_closure(), {"edge": list(paths("end"))}, ["reach"])
+        assert len(got["reach"][0]) == 71 * 70 // 2 and stats["iterations"] == 70 and stats["candidate_tuples"] == 71 * 70 // 2
+    else:
+        with pytest.raises(XlbError) as e:
+            run_program(p, programs.transitive_closure(), {"edge": list(paths("end"))}, ["reach"])
+        assert e.value.status == A.ERR_ITER_LIMIT
+    p.close()
+
+
 def test_many_long_rows(monkeypatch):
     # 70 sources with 1100 matches each twice over: the list of long rows is used by many warps at once
     src = np.repeat(np.arange(70, dtype=np.uint32), 1100)

@@ -1007,7 +1007,7 @@ __global__ void delta_resume_k(Ctl* c, uint64_t max_iterations, bool square) {
 // other bound it (issue slots 68 % used on 2000 nodes of degree 5; 20 % on a chain, where one warp of four has
 // something to do), not memory: hence several warps a row where rows are few, four outputs a
 // lane in flight, and a path of its own for a frontier of one value.  (Loop -> this, B200: chain of 1500
-// nodes 3279 -> 498 us, banded DAG of 2^14 nodes 961 -> 472, 2000 nodes of degree 5 276 -> 113, four
+// nodes 3279 -> 498 us (70 with `walk`), banded DAG of 2^14 nodes 961 -> 472, 2000 nodes of degree 5 276 -> 113, four
 // blocks of 128 nodes 181 -> 66; one warp a row with one output a lane in flight: 1089, 1238, 185, 698.)
 //   What a block is too slow for is left to the loop: a row is given up when its frontier outgrows its
 // queue, or when it is long and most blocks have nothing left to do; its seeds are all that remains
@@ -1017,6 +1017,8 @@ constexpr int RW_BITS_MIN = 5, RW_BITS_MAX = 16;  // of the second column: a row
 constexpr unsigned RW_QUEUE = 16384;              // values the frontier of a row may hold (and the row's seeds)
 constexpr unsigned RW_LONG = 16384;               // candidates of a warp (some 50 us) from which a row may be given up
 constexpr unsigned RW_LIST = 64;                  // a value with so many matches is a warp's work by itself
+constexpr unsigned RW_FOLLOW = 32;                // levels of one value each after which a row is taken for a path
+constexpr unsigned RW_SQUARED = 16;               // entries a thread of the path's table
 struct RowsShape {
     unsigned rows, words;  // rows of the bitmap, words of each
     unsigned queue;        // entries, a power of two
@@ -1148,15 +1150,16 @@ struct RowsWarp {
         for (; from < total; from += 32) dealt<1>(o, ix, from, total, m, before, shift);
         return all + total;
     }
-    // A frontier of one value, followed by one warp while it stays one: a value's matches are looked up
-    // while the test whether it is new is under way.  Leaves the ring's ends and the level in `sh`.
-    __device__ __forceinline__ void follow(const Out& o, const Ix& ix, uint64_t max_iterations) {
+    // A frontier of one value, followed by one warp while it stays one, for at most `most` levels: a value's
+    // matches are looked up while the test whether it is new is under way.  Leaves the ring's ends and the
+    // level in `sh`.
+    __device__ __forceinline__ void follow(const Out& o, const Ix& ix, uint64_t max_iterations, unsigned most) {
         const unsigned lane = lane_id();
         unsigned at = sh->head, y = queue[at & mask];
         uint64_t cand = 0;
         uint32_t start, len;
         find(ix, y, start, len);
-        const unsigned levels = (unsigned)min((unsigned long long)(max_iterations - sh->level), 0xFFFFFFFFull);
+        const unsigned levels = (unsigned)min((unsigned long long)(max_iterations - sh->level), (unsigned long long)most);
         unsigned more = 1, done = 0;  // values in the frontier; levels done
         while (done < levels && len <= 32) {
             ++done;
@@ -1206,6 +1209,73 @@ struct RowsWarp {
             sh->level += done;
             sh->cand += cand;
         }
+    }
+    // A path that has been followed for a while, by the whole block: the ring, which holds one value then, becomes
+    // a table of every value's only match.  Squared five times over it leads 32 matches on, and 32 lanes of one
+    // warp, which start on matches that follow one another, go down the path side by side: 32 levels for a
+    // look-up of the table and of the row's bits.  (A value a lane is squared in registers; where the
+    // table has more, one lane goes alone.)  Ends where a value has no or several matches (its level is not done),
+    // where a value is known, or at the limit.  What bounds `follow` is some 600 cycles of dependent instructions a
+    // level, one warp an SM partition; here 32 levels share them (chain of 1500 nodes, the whole kernel: 484 us
+    // with `follow` alone, 135 with one lane on the table, 70 with 32).
+    __device__ __forceinline__ void walk(const Out& o, const Ix& ix, uint64_t max_iterations) {
+        constexpr unsigned short STOP = 0xFFFF;  // (no value: the ring has fewer entries)
+        const unsigned lane = lane_id(), at = sh->head, values = 1u << o.lo_bits;
+        unsigned y = queue[at & mask];
+        __syncthreads();
+        for (unsigned v = threadIdx.x; v < values; v += W * 32) {
+            uint32_t start, len;
+            find(ix, v, start, len);
+            const uint32_t z = len == 1 ? other_of(ix, start) : ~0u;
+            queue[v] = z >> o.lo_bits ? STOP : (unsigned short)z;  // (a match outside the domain is left to the other paths to report)
+        }
+        __syncthreads();
+        const unsigned width = values <= RW_SQUARED * W * 32 ? 32 : 1;
+        unsigned z = queue[y];  // lane l's: the match l + 1 steps on
+        for (unsigned k = 1; k < width; k *= 2) {
+            const unsigned from = __shfl_up_sync(FULL, z, k);
+            if (lane >= k && lane < 2 * k) z = from == STOP ? STOP : queue[from];
+            unsigned short twice[RW_SQUARED];
+#pragma unroll
+            for (int i = 0; i < (int)RW_SQUARED; ++i) {
+                const unsigned v = threadIdx.x + i * W * 32, next = v < values ? queue[v] : STOP;
+                twice[i] = next == STOP ? STOP : queue[next];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < (int)RW_SQUARED; ++i)
+                if (threadIdx.x + i * W * 32 < values) queue[threadIdx.x + i * W * 32] = twice[i];
+            __syncthreads();
+        }
+        if (threadIdx.x >= 32) return;
+        const unsigned levels = (unsigned)min((unsigned long long)(max_iterations - sh->level), 0xFFFFFFFFull);
+        unsigned done = 0;
+        bool known = false;
+        for (;;) {
+            const bool here = z != STOP && lane < width && lane < levels - done;
+            const unsigned word = here ? seen[z >> 5] : 0u, next = here ? queue[z] : STOP, bit = 1u << (z & 31);
+            const unsigned before = __match_any_sync(FULL, z) & lanemask_lt();  // a loop shorter than the warp is wide
+            const unsigned ends = __ballot_sync(FULL, !here), old = __ballot_sync(FULL, here && ((word & bit) || before));
+            const unsigned count = min(ends ? __ffs(ends) - 1 : 32, old ? __ffs(old) - 1 : 32);
+            if (lane < count) atomicOr(&seen[z >> 5], bit);
+            if (count) y = __shfl_sync(FULL, z, count - 1);
+            done += count;
+            if (count < width) {
+                known = (old >> count) & 1;
+                break;
+            }
+            z = next;
+            __syncwarp();
+        }
+        if (lane) return;
+        // (as many tuples as levels, but for the level that ended on a known value; y is in the frontier unless there was one)
+        const unsigned to = at + done;
+        done += known ? 1 : 0;
+        if (!known) queue[to & mask] = (unsigned short)y;
+        sh->head = known ? to + 1 : to;
+        sh->tail = to + 1;
+        sh->level += done;
+        sh->cand += done;
     }
 };
 // The seeds of a row that is given up, for the loop.
@@ -1268,10 +1338,18 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const Out o, const __grid
             uint64_t level = 0, cand = 0, looked = RW_LONG;
             while (ok && head != end && level < max_iterations) {
                 if (end - head == 1 && rules.n == 1) {
-                    if (warp == 0) w.follow(o, rules.r[0].ix[0], max_iterations);
+                    const bool table = sh.queue >> o.lo_bits;  // the ring has an entry for every value
+                    const unsigned from = head;
+                    if (warp == 0) w.follow(o, rules.r[0].ix[0], max_iterations, table ? RW_FOLLOW : ~0u);
                     __syncthreads();
                     head = v->head;
                     end = v->tail;
+                    if (table && head - from == RW_FOLLOW && end - head == 1) {
+                        w.walk(o, rules.r[0].ix[0], max_iterations);
+                        __syncthreads();
+                        head = v->head;
+                        end = v->tail;
+                    }
                     level = v->level;
                     __syncthreads();
                     if (head == end || level >= max_iterations) break;
