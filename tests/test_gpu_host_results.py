@@ -42,3 +42,69 @@ def test_results_are_independent_and_outlive_the_context():
     p.close()
     for h, w in zip(held, want):
         assert np.array_equal(h, w)
+
+
+def expect(p, cols):
+    for g, c in zip(p.download(p.create_buffer_from_slices(cols)), cols):
+        assert np.array_equal(g.view(np.uint8) if c.dtype == np.bool_ else g, c.view(np.uint8) if c.dtype == np.bool_ else c, equal_nan=c.dtype.kind == "f")
+
+
+# First columns of 6 MB and more go as runs where these are long: tiles are 4096 rows, a warp's 512, what a
+# thread fills 65536 (4 bytes) or 32768 (8 bytes) rows, and the staging holds 32766 or 16383 runs.
+@pytest.mark.parametrize("dtype", [np.uint32, np.int64, np.float32])
+@pytest.mark.parametrize("runs", ["one", "last", "edges", "even", "short", "limit", "over"])
+@pytest.mark.parametrize("n", [786431, 3 << 18, (3 << 19) - 1, 3 << 19, (3 << 19) + 4097, 2222222])
+def test_first_columns_of_long_runs(dtype, runs, n):
+    cap = (256 * 1024 - 16) // (2 * np.dtype(dtype).itemsize)
+    if runs == "one":
+        starts = [0]
+    elif runs == "last":
+        starts = [0, n - 1]
+    elif runs == "edges":
+        starts = sorted({x + d for x in (0, 512, 4096, 32768, 65536, 131072, n - 4096) for d in (-1, 0, 1) if 0 <= x + d < n})
+    elif runs == "even":
+        starts = range(0, n, 1000)
+    elif runs == "short":
+        starts = range(0, n, 9)  # more runs than are worth it
+    else:
+        count = min(cap, n // 64) + (runs == "over")
+        starts = np.linspace(0, n - 1, count).astype(np.int64)
+    starts = np.unique(np.array(list(starts)))
+    rng = np.random.default_rng(n)
+    values = rng.standard_normal(len(starts)).astype(dtype) if dtype == np.float32 else rng.permutation(len(starts)).astype(dtype)
+    if dtype == np.float32:
+        values[-1] = np.nan
+    first = np.repeat(values, np.diff(np.append(starts, n)))
+    p = KernelProvider(device=0)
+    expect(p, [first, rng.integers(0, 1 << 32, n, dtype=np.uint32)])
+    expect(p, [first, rng.integers(0, 2, n).astype(np.bool_), first[::-1].copy()])
+    p.close()
+
+
+@pytest.mark.parametrize("offset", [None, 0, 4, 36])
+def test_long_runs_into_memory_of_the_callers(offset):
+    # The C interface takes any memory: what is not page-locked is copied as before, what is need not begin at a
+    # cache line.
+    import ctypes as C
+
+    total = 2200000
+    first, second = np.repeat(np.arange(total // 1000, dtype=np.uint32), 1000), np.arange(total, dtype=np.uint32)
+    p = KernelProvider(device=0)
+    buf = p.create_buffer_from_slices([first, second])
+    for m in (total, total - 49999):  # all rows, and as many as the caller has room for
+        if offset is None:
+            out = [np.zeros(m, dtype=np.uint32) for _ in range(2)]
+        else:
+            block = C.c_void_p()
+            p._check(p._lib.xlb_host_alloc(C.c_uint64(8 * m + 256), C.byref(block)))
+            all_of_it = np.ctypeslib.as_array((C.c_uint32 * (2 * m + 64)).from_address(block.value))
+            all_of_it[:] = 0xABABABAB
+            at = offset // 4
+            out = [all_of_it[at:at + m], all_of_it[at + m + 1:at + 2 * m + 1]]
+        rows = C.c_uint64()
+        p._check(p._lib.xlb_rel_to_host(p._ctx, buf._h, (C.c_void_p * 2)(*[o.ctypes.data for o in out]), m, C.byref(rows)))
+        assert rows.value == total and np.array_equal(out[0], first[:m]) and np.array_equal(out[1], second[:m])
+        if offset is not None:
+            assert np.all(all_of_it[:at] == 0xABABABAB) and all_of_it[at + m] == 0xABABABAB and np.all(all_of_it[at + 2 * m + 1:] == 0xABABABAB)
+            p._lib.xlb_host_free(block)
+    p.close()

@@ -322,7 +322,7 @@ struct xlb_ctx {
     unsigned long long* h_scalar = nullptr;  // SCALAR_WORDS words; read_words uses those from READ_WORDS_AT on
     unsigned long long* h_scalar_dev = nullptr;  // the same words as the device sees them (mapped): a kernel can leave counts there
     unsigned long long publish_seq = 0;          // number of the last set of counts a kernel was asked to leave there
-    char* h_stage = nullptr;      // page-locked staging of small results (made on first use) ...
+    char* h_stage = nullptr;      // page-locked staging of small results and of the runs of large ones (made on first use) ...
     char* h_stage_dev = nullptr;  // ... as the device sees it
     DevStatus* d_status = nullptr;
     unsigned read_seq = 0;      // number of the last read-back (read_words)
@@ -331,6 +331,8 @@ struct xlb_ctx {
     bool leaving = false;       // the last kernel enqueued leaves the status itself (Publish), which nobody has read yet
     unsigned* arrived = nullptr;  // its blocks that are done: zero between kernels
     cudaEvent_t plan_e0 = nullptr, plan_e1 = nullptr;  // around a plan (made on first use)
+    cudaStream_t copy_stream = nullptr;                // copies of a large result, beside the stream (made on first use)
+    cudaEvent_t copy_behind = nullptr;
     int sm_count = 148;
     // executor state
     std::map<uint32_t, std::string> rel_names;
@@ -372,6 +374,7 @@ struct xlb_ctx {
     std::vector<TraceNote> trace;
 };
 
+constexpr uint64_t STAGE_BYTES = 256ull << 10;  // of h_stage
 constexpr int SCALAR_WORDS = 128, READ_WORDS_AT = 64, READ_WORDS_MAX = 16;
 
 // Counts a kernel leaves in pinned memory for the host: low 40 bits the count, top 24 the number

@@ -1,0 +1,256 @@
+// Results of some size, fetched into page-locked host memory.
+//
+// What bounds a large result is the bus (55 GB/s against the 6.5 TB/s at which the device wrote it), and
+// the first column of a sorted relation is runs of equal values: it crosses the bus as (first row,
+// value) pairs and is written out by host threads while the other columns are copied.  Two columns of 26.8 M
+// rows took 4.1 ms, now 2.0; of 3.9 M rows 570 us, now 330; of 2.2 M rows 320, now 190.
+//   One core writes 19 GB/s around the cache, four 73 (host of a B200, 16 cores).  Four are enough for a column
+// to be there before the next one; more only slow the copies beside them (four 2.0 ms, six 2.1, eight 2.2),
+// and ordinary stores, which read what they overwrite, took 2.6.
+//   The column is read twice on the device (heads counted per tile, then written in order), while the copy of
+// the next column runs on a stream of its own.
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
+
+#include <algorithm>
+#include <atomic>
+#include <exception>
+#include <thread>
+#include <vector>
+
+#include "xlb_common.cuh"
+#include "xlb_host.h"
+#include "xlb_kernels.cuh"
+#include "xlb_ops.h"
+
+using namespace xk;
+
+namespace {
+
+constexpr uint64_t RUNS_TILE = 4096;                     // rows a block looks at, 512 a warp
+constexpr uint64_t RUNS_MIN_BYTES = 6ull << 20;          // below, the 60 us until the runs are there and 11 us a thread are hardly made up for (4 MB: 73 us of bus)
+constexpr uint64_t RUNS_THREAD_BYTES = 3ull << 19;       // of the column, per thread
+constexpr unsigned RUNS_THREADS_MAX = 4, RUNS_CORES_MIN = 4;
+constexpr uint64_t RUNS_CHUNK = 256ull << 10;            // bytes a thread takes at a time
+constexpr uint64_t RUNS_ROWS_MIN = 64;                   // rows a run has to have on average: a run is a few dozen ns of its own
+
+template <class T>
+struct Run {
+    T row, value;
+};
+template <class T>
+__device__ __forceinline__ unsigned warp_heads(const T* __restrict__ col, uint64_t n, uint64_t base, int k) {
+    const uint64_t i = base + k * 32 + lane_id();
+    return __ballot_sync(FULL, i < n && (i == 0 || col[i] != col[i - 1]));
+}
+// counts[t]: runs that begin in tile t
+template <class T>
+__global__ void __launch_bounds__(BLOCK) runs_count_k(const T* __restrict__ col, uint64_t n, unsigned* __restrict__ counts) {
+    __shared__ unsigned warp_s[BLOCK / 32];
+    const uint64_t base = blockIdx.x * RUNS_TILE + (threadIdx.x >> 5) * 512;
+    unsigned c = 0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) c += __popc(warp_heads(col, n, base, k));
+    if (lane_id() == 0) warp_s[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned total = 0;
+        for (int w = 0; w < BLOCK / 32; ++w) total += warp_s[w];
+        counts[blockIdx.x] = total;
+    }
+}
+// The runs in order, into mapped host memory; none when there are more than `cap`.  `total` gets their number.
+template <class T>
+__global__ void __launch_bounds__(BLOCK) runs_write_k(const T* __restrict__ col, uint64_t n, const unsigned* __restrict__ counts, Run<T>* out, uint64_t cap, unsigned long long* total) {
+    __shared__ unsigned long long before_s[BLOCK / 32], all_s[BLOCK / 32];
+    __shared__ unsigned warp_s[BLOCK / 32];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5, mine = counts[blockIdx.x];
+    if (!mine && blockIdx.x) return;
+    unsigned long long before = 0, all = 0;
+    for (unsigned t = threadIdx.x; t < gridDim.x; t += BLOCK) {
+        const unsigned v = counts[t];
+        all += v;
+        if (t < blockIdx.x) before += v;
+    }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) {
+        before += __shfl_xor_sync(FULL, before, d);
+        all += __shfl_xor_sync(FULL, all, d);
+    }
+    const uint64_t base = blockIdx.x * RUNS_TILE + warp * 512;
+    unsigned heads[16], c = 0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        heads[k] = warp_heads(col, n, base, k);
+        c += __popc(heads[k]);
+    }
+    if (lane == 0) {
+        before_s[warp] = before;
+        all_s[warp] = all;
+        warp_s[warp] = c;
+    }
+    __syncthreads();
+    before = all = 0;
+    for (int w = 0; w < BLOCK / 32; ++w) {
+        before += before_s[w];
+        all += all_s[w];
+        if (w < (int)warp) before += warp_s[w];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *total = all;
+    if (all > cap) return;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const uint64_t i = base + k * 32 + lane;
+        if ((heads[k] >> lane) & 1u) out[before + __popc(heads[k] & lanemask_lt())] = {(T)i, col[i]};
+        before += __popc(heads[k]);
+    }
+}
+
+// Rows [lo, hi) of the column, a cache line at a time.  A line that runs meet in is put together first: written
+// in parts, some of them around the cache, it cost 0.3 us.
+template <class T>
+void fill_rows(T* to, const Run<T>* runs, uint64_t n_runs, uint64_t n, uint64_t lo, uint64_t hi) {
+    constexpr uint64_t line = 64 / sizeof(T);
+    uint64_t r = std::upper_bound(runs, runs + n_runs, lo, [](uint64_t row, const Run<T>& x) { return row < x.row; }) - runs - 1;
+    const auto end_of = [&](uint64_t run) { return run + 1 < n_runs ? (uint64_t)runs[run + 1].row : n; };
+    uint64_t end = end_of(r);
+    for (uint64_t at = lo; at < hi;) {
+        alignas(64) T buf[line];
+        const bool whole = (uintptr_t)(to + at) % 64 == 0 && hi - at >= line;
+        const uint64_t m = whole ? line : 1;
+        for (uint64_t k = 0; k < m; ++k) {
+            while (at + k >= end) end = end_of(++r);
+            buf[k] = runs[r].value;
+        }
+        if (!whole) {
+            to[at++] = buf[0];
+            continue;
+        }
+        // this line, and those behind it that lie in the run it ends with
+        const uint64_t lines = end >= at + 2 * line ? (std::min(end, hi) - at) / line : 1;
+#if defined(__SSE2__)
+        __m128i v[4];
+        for (int k = 0; k < 4; ++k) v[k] = _mm_load_si128(reinterpret_cast<const __m128i*>(buf) + k);
+        __m128i* out = reinterpret_cast<__m128i*>(to + at);
+        for (int k = 0; k < 4; ++k) _mm_stream_si128(out + k, v[k]);
+        v[0] = v[1] = v[2] = v[3] = sizeof(T) == 4 ? _mm_set1_epi32((int)buf[line - 1]) : _mm_set1_epi64x((long long)buf[line - 1]);
+        for (out += 4; out < reinterpret_cast<__m128i*>(to + at) + 4 * lines; out += 4)
+            for (int k = 0; k < 4; ++k) _mm_stream_si128(out + k, v[k]);
+#else
+        std::copy(buf, buf + line, to + at);
+        std::fill(to + at + line, to + at + lines * line, buf[line - 1]);
+#endif
+        at += lines * line;
+    }
+#if defined(__SSE2__)
+    _mm_sfence();
+#endif
+}
+// Threads that write a column out.  They are started (11 us each) while the runs are on their way, and wait for them
+// a little before they begin; without any to be had the caller does all of it.
+template <class T>
+class Filler {
+    enum { WAIT, FILL, LEAVE };
+    std::atomic<int> go{WAIT};
+    std::atomic<uint64_t> next{0};
+    T* to = nullptr;
+    const Run<T>* runs = nullptr;
+    uint64_t n_runs = 0, n = 0;
+    std::vector<std::thread> helpers;
+
+    void work() {
+        constexpr uint64_t rows = RUNS_CHUNK / sizeof(T);
+        for (uint64_t at; (at = next.fetch_add(rows, std::memory_order_relaxed)) < n;) fill_rows(to, runs, n_runs, n, at, std::min(n, at + rows));
+    }
+
+   public:
+    explicit Filler(unsigned threads) {
+        try {
+            helpers.reserve(threads);
+            for (unsigned t = 1; t < threads; ++t)
+                helpers.emplace_back([this] {
+                    while (go.load(std::memory_order_acquire) == WAIT) std::this_thread::yield();
+                    if (go.load(std::memory_order_acquire) == FILL) work();
+                });
+        } catch (const std::exception&) {  // no thread (or memory for one) to be had
+        }
+    }
+    void fill(T* column, const Run<T>* r, uint64_t count, uint64_t rows) {
+        to = column;
+        runs = r;
+        n_runs = count;
+        n = rows;
+        go.store(FILL, std::memory_order_release);
+        work();
+    }
+    ~Filler() {
+        int still = WAIT;
+        go.compare_exchange_strong(still, LEAVE, std::memory_order_release, std::memory_order_relaxed);
+        for (auto& t : helpers) t.join();
+    }
+};
+
+// Copies that run beside the context's stream, behind what is on it now.  However the operation ends, they are
+// over before it returns: the memory they write is the caller's.
+struct SideCopies {
+    xlb_ctx* c;
+    explicit SideCopies(xlb_ctx* ctx) : c(ctx) {
+        if (!c->copy_stream) CUDA_OK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+        if (!c->copy_behind) CUDA_OK(cudaEventCreateWithFlags(&c->copy_behind, cudaEventDisableTiming));
+        CUDA_OK(cudaEventRecord(c->copy_behind, c->stream));
+        CUDA_OK(cudaStreamWaitEvent(c->copy_stream, c->copy_behind, 0));
+    }
+    void add(void* to, const void* from, uint64_t bytes) { CUDA_OK(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, c->copy_stream)); }
+    void wait() { CUDA_OK(cudaStreamSynchronize(c->copy_stream)); }
+    ~SideCopies() { CUDA_QUIET(cudaStreamSynchronize(c->copy_stream)); }
+};
+
+bool page_locked(const void* p) {
+    cudaPointerAttributes a{};
+    return cuda_take(cudaPointerGetAttributes(&a, p)) == cudaSuccess && a.type == cudaMemoryTypeHost;
+}
+
+template <class T>
+void fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n, unsigned threads) {
+    const uint64_t tiles = (n + RUNS_TILE - 1) / RUNS_TILE, cap = std::min<uint64_t>((STAGE_BYTES - 16) / sizeof(Run<T>), n / RUNS_ROWS_MIN);
+    char* stage = stage_buffer(c);
+    unsigned long long* total = reinterpret_cast<unsigned long long*>(stage);
+    const Run<T>* runs = reinterpret_cast<const Run<T>*>(stage + 16);
+    Buf counts = make_buf(c, tiles * 4);
+    SideCopies side(c);
+    const T* col = r->cols[0]->as<T>();
+    prof_begin(c, "to_host", n * sizeof(T));
+    runs_count_k<T><<<(unsigned)tiles, BLOCK, 0, c->stream>>>(col, n, counts->as<unsigned>());
+    check_launch(c, "to_host");
+    prof_begin(c, "to_host", n * sizeof(T));
+    runs_write_k<T><<<(unsigned)tiles, BLOCK, 0, c->stream>>>(col, n, counts->as<unsigned>(), reinterpret_cast<Run<T>*>(c->h_stage_dev + 16), cap, reinterpret_cast<unsigned long long*>(c->h_stage_dev));
+    check_launch(c, "to_host");
+    for (uint32_t i = 1; i < r->schema.arity; ++i) side.add(cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]));
+    {
+        Filler<T> filler(threads);
+        stream_wait(c);
+        if (*total > cap) side.add(cols[0], col, n * sizeof(T));
+        else filler.fill(static_cast<T*>(cols[0]), runs, *total, n);
+    }
+    side.wait();
+}
+
+}  // namespace
+
+void ops_fetch_columns(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n) {
+    ops_rel_columns(c, r);
+    const uint32_t arity = r->schema.arity, width = type_width(r->schema.types[0]);
+    // Not with several ranks (whose waits watch the communicator), and not into memory that the driver copies to by
+    // itself: such a copy does not run beside anything.
+    if (arity >= 2 && width >= 4 && n * width >= RUNS_MIN_BYTES && n < 1ull << 32 && !c->wait_hook) {
+        const unsigned cores = host_pool_cores();
+        bool locked = cores >= RUNS_CORES_MIN;
+        for (uint32_t i = 0; i < arity; ++i) locked = locked && page_locked(cols[i]) && (uintptr_t)cols[i] % width == 0;
+        const unsigned threads = (unsigned)std::min<uint64_t>({RUNS_THREADS_MAX, cores / 2, n * width / RUNS_THREAD_BYTES});
+        if (locked && width == 4) return fetch_with_runs<uint32_t>(c, r, cols, n, threads);
+        if (locked) return fetch_with_runs<unsigned long long>(c, r, cols, n, threads);
+    }
+    for (uint32_t i = 0; i < arity; ++i) CUDA_OK(copy_async(c, cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost));
+    CUDA_OK(cudaStreamSynchronize(c->stream));
+}

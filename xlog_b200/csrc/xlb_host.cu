@@ -124,11 +124,14 @@ struct HostPool {
         std::lock_guard<std::mutex> g(mu);
         leaving_bytes -= bytes;
     }
-    uint64_t most() const {
+    unsigned long sharers() const {
         const char* local = getenv("LOCAL_WORLD_SIZE");
         const unsigned long said = local ? strtoul(local, nullptr, 10) : 0;
+        return said ? said : ranks;
+    }
+    uint64_t most() const {
         const uint64_t memory = (uint64_t)sysconf(_SC_PHYS_PAGES) * (uint64_t)sysconf(_SC_PAGESIZE);
-        return std::min<uint64_t>(LIVE_MAX, memory / 8 / (said ? said : ranks));
+        return std::min<uint64_t>(LIVE_MAX, memory / 8 / sharers());
     }
     void* take(uint64_t bytes) {
         if (bytes > LIVE_MAX) return nullptr;
@@ -216,6 +219,11 @@ void host_pool_ranks(unsigned ranks) {
 uint64_t host_pool_most() {
     std::lock_guard<std::mutex> g(pool().mu);
     return pool().most();
+}
+
+unsigned host_pool_cores() {
+    std::lock_guard<std::mutex> g(pool().mu);
+    return std::thread::hardware_concurrency() / (unsigned)pool().sharers();
 }
 
 extern "C" xlb_status xlb_host_alloc(uint64_t bytes, void** out) {

@@ -40,7 +40,6 @@ __global__ void gather_pair_k(const T* __restrict__ in, const uint64_t* __restri
 }
 
 // Columns written into page-locked host memory (16-byte aligned on both sides).
-constexpr uint64_t STAGE_BYTES = 256ull << 10;
 struct StageCols {
     const void* from[XLB_MAX_ARITY];
     void* to[XLB_MAX_ARITY];
@@ -1210,6 +1209,8 @@ extern "C" void xlb_ctx_destroy(xlb_ctx* c) {
     if (c->h_scalar) CUDA_QUIET(cudaFreeHost(c->h_scalar));
     if (c->h_stage) CUDA_QUIET(cudaFreeHost(c->h_stage));
     if (c->d_status) CUDA_QUIET(cudaFree(c->d_status));
+    if (c->copy_behind) CUDA_QUIET(cudaEventDestroy(c->copy_behind));
+    if (c->copy_stream) CUDA_QUIET(cudaStreamDestroy(c->copy_stream));
     if (c->plan_e0) CUDA_QUIET(cudaEventDestroy(c->plan_e0));
     if (c->plan_e1) CUDA_QUIET(cudaEventDestroy(c->plan_e1));
     c->arena.destroy();
@@ -1299,6 +1300,14 @@ extern "C" xlb_status xlb_rel_is_canonical(const xlb_rel* r, int* canonical) {
     return XLB_OK;
 }
 
+char* stage_buffer(xlb_ctx* c) {
+    if (!c->h_stage) {
+        CUDA_OK(cudaHostAlloc((void**)&c->h_stage, STAGE_BYTES, cudaHostAllocMapped));
+        CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_stage_dev, c->h_stage, 0));
+    }
+    return c->h_stage;
+}
+
 extern "C" xlb_status xlb_rel_to_host(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t cap_rows, uint64_t* rows) {
     if (!c || !r) return XLB_ERR_INVALID;
     API_BEGIN(c)
@@ -1314,10 +1323,7 @@ extern "C" xlb_status xlb_rel_to_host(xlb_ctx* c, const xlb_rel* r, void* const*
     if (n && arity && offset[arity] <= STAGE_BYTES) {
         // A small result: one kernel writes all columns into page-locked staging memory across the
         // bus (a copy per column cost 12 us each), the host copies them out of it.
-        if (!c->h_stage) {
-            CUDA_OK(cudaHostAlloc((void**)&c->h_stage, STAGE_BYTES, cudaHostAllocMapped));
-            CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_stage_dev, c->h_stage, 0));
-        }
+        stage_buffer(c);
         const unsigned grid = (unsigned)std::min<uint64_t>((offset[arity] / 4 + BLOCK - 1) / BLOCK, (uint64_t)c->sm_count);
         prof_begin(c, "to_host", offset[arity]);
         if (!r->cols[0]) {
@@ -1336,10 +1342,7 @@ extern "C" xlb_status xlb_rel_to_host(xlb_ctx* c, const xlb_rel* r, void* const*
         stream_wait(c);
         for (uint32_t i = 0; i < arity; ++i) memcpy(cols[i], c->h_stage + offset[i], n * type_width(r->schema.types[i]));
     } else if (n && arity) {
-        ops_rel_columns(c, r);
-        for (uint32_t i = 0; i < arity; ++i)
-            CUDA_OK(copy_async(c, cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost));
-        CUDA_OK(cudaStreamSynchronize(c->stream));
+        ops_fetch_columns(c, r, cols, n);
     } else {
         CUDA_OK(cudaStreamSynchronize(c->stream));
     }

@@ -34,6 +34,8 @@ struct Index {
     bool built() const { return S || cursor; }
 };
 
+char* stage_buffer(xlb_ctx* c);  // h_stage, made if need be
+void ops_fetch_columns(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n);  // the first n rows' columns to host memory (n > 0)
 Keys ops_rel_packed(xlb_ctx* c, const xlb_rel* r);             // packed view (cached on the relation)
 void ops_pack_all(xlb_ctx* c, const std::vector<const xlb_rel*>& rels);  // the packed views of several relations, with one read-back
 // The same for a two-column relation that is not packed yet, with the rows whose column fcol equals
