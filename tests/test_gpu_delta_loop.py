@@ -105,6 +105,64 @@ def test_same_generation(nodes, monkeypatch):
         assert np.array_equal(g, w)
 
 
+def sides(kinds):
+    """p(X,Y) :- s(X,Y), then one rule per kind: both columns led on, the first, the second."""
+    ids = {"s": 0, "a": 1, "b": 2, "p": 3}
+    rules = [CompiledRule("p", Scan(0), U2)]
+    for k in kinds:
+        if k == "both":    # p(X,Y) :- a(P,X), p(P,Q), b(Q,Y)
+            rules.append(CompiledRule("p", Project(Join(Join(Scan(1), Scan(3), [0], [0]), Scan(2), [3], [0]), [1, 5]), U2))
+        elif k == "first":  # p(X,Y) :- a(P,X), p(P,Y)
+            rules.append(CompiledRule("p", Project(Join(Scan(1), Scan(3), [0], [0]), [1, 3]), U2))
+        else:              # p(X,Y) :- p(X,Q), b(Q,Y)
+            rules.append(CompiledRule("p", Project(Join(Scan(3), Scan(2), [1], [0]), [0, 3]), U2))
+    return ExecutionPlan([Scc(0, True, rules)], ids)
+
+
+# heads of 4 to 14 bits a column: too few in all for bit rows, a row of two words, of one per lane, of eight, too long
+@pytest.mark.parametrize("kinds", [("both",), ("first",), ("both", "second"), ("first", "second", "both")], ids="-".join)
+@pytest.mark.parametrize("hi,lo,rows", [(10, 40, 60), (8191, 100, 9000), (8000, 63, 9000), (130, 8191, 3000), (1000, 1023, 1500), (1500, 1500, 2000), (8000, 8191, 9000), (300, 16000, 9000)])
+def test_columns_led_on_apart(hi, lo, rows, kinds, monkeypatch):
+    rng = np.random.default_rng(hi * lo)
+    pairs = lambda n, x, y: [rng.integers(0, x, n).astype(np.uint32), rng.integers(0, y, n).astype(np.uint32)]  # noqa: E731
+    s = pairs(40, hi, lo)
+    s[0][0], s[1][0] = hi - 1, lo - 1
+    both(sides(kinds), {"s": s, "a": pairs(rows, hi, hi), "b": pairs(rows, lo, lo)}, "p", monkeypatch)
+
+
+@pytest.mark.parametrize("fan", [16, 17, 1024, 1025])
+def test_columns_led_on_to_many(fan, monkeypatch):
+    # lists about as long as what a lane takes alone (second column) and as a row is allowed to lead to (first)
+    hub = [np.full(fan, 3, np.uint32), np.arange(10, 10 + fan, dtype=np.uint32)]
+    back = [np.arange(10, 10 + fan, dtype=np.uint32), np.full(fan, 3, np.uint32)]
+    e = [np.concatenate([hub[0], back[0][:9], [2000]]).astype(np.uint32), np.concatenate([hub[1], back[1][:9], [2000]]).astype(np.uint32)]
+    both(sides(("both",)), {"s": [np.array([3, 3], np.uint32), np.array([3, 11], np.uint32)], "a": e, "b": e}, "p", monkeypatch)
+
+
+@pytest.mark.parametrize("n,burst", [(20, 0), (25, 0), (26, 0), (200, 0), (2000, 0), (26, 200), (60, 200)])
+def test_columns_led_on_along_a_path(n, burst, monkeypatch):
+    # one tuple an iteration: after some of them the loop goes on; at the end of the path burst^2 of them at once
+    a = list(chain(n + 1))
+    a = [np.concatenate([a[0], np.full(burst, n), [2000]]).astype(np.uint32), np.concatenate([a[1], np.arange(n + 1, n + 1 + burst), [2000]]).astype(np.uint32)]
+    plan, rels = sides(("both",)), {"s": [np.array([0], np.uint32)] * 2, "a": a, "b": [a[0], a[1]]}
+    both(plan, rels, "p", monkeypatch)
+    for limit in (n - 1, n, n + 1):
+        res = []
+        for off in (False, True):
+            if off:
+                monkeypatch.setenv("XLB_NO_DELTA_LOOP", "1")
+            else:
+                monkeypatch.delenv("XLB_NO_DELTA_LOOP", raising=False)
+            p = KernelProvider(device=0, max_iterations=limit)
+            try:
+                got, stats = run_program(p, plan, rels, ["p"])
+                res.append((len(got["p"][0]), stats["iterations"]))
+            except XlbError as e:
+                res.append(e.status)
+            p.close()
+        assert res[0] == res[1]
+
+
 def test_two_recursive_rules_and_wide_domain(monkeypatch):
     # p(X,Y) :- e(X,Y).  p(X,Z) :- p(X,Y), e(Y,Z).  p(X,Z) :- f(X,Y), p(Y,Z).  ids up to 2^15: 30 bits
     ids = {"e": 0, "f": 1, "p": 2}

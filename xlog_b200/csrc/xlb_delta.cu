@@ -720,6 +720,37 @@ __device__ __forceinline__ void solo(const Out& o, const Rules& rules, Heavy* he
     }
 }
 
+// A bounded wait (one thread): until the word has come to `want`.  An iteration may take any time, so
+// what is bounded is the time in which nothing that the others do can be seen.
+__device__ __forceinline__ unsigned going_on(const Ctl* ctl) {
+    unsigned v = *(const volatile unsigned*)&ctl->beat;
+    for (int k = 0; k < 3; ++k) {
+        const volatile Slot* s = &ctl->slot[k];
+        v += (unsigned)s->count + s->next_heavy + s->next_chunk;
+    }
+    return v;
+}
+__device__ __forceinline__ bool wait_for(const Out& o, const unsigned* word, unsigned want, unsigned sleep, unsigned passed) {
+    unsigned v, seen = going_on(o.ctl);
+    for (unsigned polls = 0;; ++polls) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+        if ((int)(v - want) >= 0) return true;
+        if (polls > o.spin_limit) {
+            const unsigned now = going_on(o.ctl);
+            if (now != seen) {
+                seen = now;
+                polls = 0;
+                continue;
+            }
+            *(volatile unsigned*)&o.ctl->abort = 1;
+            set_status(o.st, XLB_ERR_TIMEOUT, 14, passed);
+            return false;
+        }
+        if (*(volatile unsigned*)&o.ctl->abort) return false;
+        if (sleep) __nanosleep(sleep);
+    }
+}
+
 template <bool SQUARE>
 __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const __grid_constant__ Rules rules, Heavy* heavy, uint64_t max_iterations, const __grid_constant__ Square sq) {
     extern __shared__ uint64_t stage_s[];
@@ -732,36 +763,6 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
     WarpSink sink{o, stage_s + warp * (2 * DL_STAGE)};
     unsigned passed = 0, solo_turns = 0;
     Ctl* ctl = o.ctl;
-    // A bounded wait (one thread): until `done` holds of the word.  An iteration may take any time, so
-    // what is bounded is the time in which nothing that the others do can be seen.
-    auto going_on = [&]() {
-        unsigned v = *(volatile unsigned*)&ctl->beat;
-        for (int k = 0; k < 3; ++k) {
-            const volatile Slot* s = &ctl->slot[k];
-            v += (unsigned)s->count + s->next_heavy + s->next_chunk;
-        }
-        return v;
-    };
-    auto wait_for = [&](const unsigned* word, unsigned sleep, auto done) {
-        unsigned v, seen = going_on();
-        for (unsigned polls = 0;; ++polls) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
-            if (done(v)) return true;
-            if (polls > o.spin_limit) {
-                const unsigned now = going_on();
-                if (now != seen) {
-                    seen = now;
-                    polls = 0;
-                    continue;
-                }
-                *(volatile unsigned*)&ctl->abort = 1;
-                set_status(o.st, XLB_ERR_TIMEOUT, 14, passed);
-                return false;
-            }
-            if (*(volatile unsigned*)&ctl->abort) return false;
-            if (sleep) __nanosleep(sleep);
-        }
-    };
     // All blocks arrive; then thread 0 of each runs `then`, which all threads see the effects of.
     auto barrier = [&](auto then) {
         __syncthreads();
@@ -769,7 +770,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
             passed += gridDim.x;
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->arrived) : "memory");
             const unsigned want = passed;
-            go_s = wait_for(&ctl->arrived, 0, [want](unsigned v) { return (int)(v - want) >= 0; });
+            go_s = wait_for(o, &ctl->arrived, want, 0, passed);
             if (go_s) then(state_s);
         }
         __syncthreads();
@@ -918,7 +919,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const
             } else {
                 if (threadIdx.x == 0) {
                     const unsigned want = ++solo_turns;
-                    go_s = wait_for(&ctl->solo_turns, 100, [want](unsigned v) { return (int)(v - want) >= 0; });
+                    go_s = wait_for(o, &ctl->solo_turns, want, 100, passed);
                     state_s.start = __ldcg(&ctl->solo_start);
                     state_s.end = __ldcg(&ctl->solo_end);
                     state_s.iterations = __ldcg(&ctl->solo_iterations);
@@ -1424,9 +1425,344 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const Out o, const __grid
         if (left) ctl->rows_left = 1;
     }
 }
-// The loop starts over on what was given up.
+// ---- rules that take the head's columns apart: bit rows
+// Where each rule leads a delta row's first column through one stored relation (or none) to the new first column,
+// and its second through another to the new second (same generation: sg(X, Y) :- edge(A, X), sg(A, B),
+// edge(B, Y)), an iteration is two products with sparse matrices: new = A^T delta B.  A block owns every
+// 148th row.  It takes its rows of the delta as bits, leads the bits through B into rows in shared memory, and ORs
+// those into the rows that A leads to; what they gain over the head is found by their own block in the next
+// iteration.  A tuple so costs no atomic in global memory, no entry in a log and no look at a word of its
+// own: same generation over 7001 nodes (26.8 M tuples) took 718 us in the loop, bound by its atomics on single
+// bits, 282 with a warp for each row (five rows in seven have nothing to lead to), and takes 188 here: a phase is
+// some 20 K cycles of dependent steps between two barriers, then atomics on words of shared memory (what neighbours
+// lead to shares words; setting a lane's bits of one word together cost more than it saved).
+//   Rows that nobody reached are passed over by a stamp.  Lists of A are shared out among a block's warps only: where one
+// is longer than BT_ROWS, the loop does it all.  A fixpoint that goes on with next to nothing in an iteration is
+// handed to the loop, whose small iterations meet at no barrier.
+constexpr int BT_BITS_MIN = 5, BT_BITS_MAX = 13;
+constexpr int BT_BITS_BOTH = 20;                    // of both columns: below, the loop is as fast (same generation over 300 and 511 nodes 139 and 149 us of device time by the loop, 155 and 161 here; 1023 nodes 195 and 166)
+constexpr unsigned BT_WORDS = 1u << (BT_BITS_MAX - 5);
+constexpr unsigned BT_OWN = 56;                     // rows of a block
+constexpr unsigned BT_LIST = 16;                    // a value with more matches is a whole warp's work
+constexpr unsigned BT_ROWS = 1024;                  // rows that a row may lead to
+constexpr unsigned BT_SMALL = 1024, BT_LEAVE = 24;  // after so many iterations in a row of fewer tuples the loop goes on
+constexpr unsigned BT_EDGES = 1u << 20;             // rows of A (every block looks through them once)
+constexpr unsigned BT_LISTED = 16384;               // rows of the stored relation whose lists a block keeps in shared memory
+constexpr unsigned BT_SMEM = ((DL_RULES + 2) * BT_WORDS + 2 * BT_OWN * BT_WORDS + DL_WARPS * 256 + (1u << BT_BITS_MAX)) * 4 + BT_LISTED * 2;
+static_assert(BT_SMEM <= (222u << 10), "a block an SM");
+struct BitsRule {
+    Ix a, b;
+    bool a_list, b_list;
+    unsigned listed;  // rows of B's index, if it is the one kept in shared memory
+    unsigned a_rows;  // of A's
+};
+struct BitsRules {
+    BitsRule r[DL_RULES];
+    int n;
+};
+struct Bits {
+    unsigned *next[2], *stamp[2];  // what rows are reached by in this iteration and the next; rows that are
+    unsigned rows, words;          // of the head's bitmap, words of each
+};
+struct Active {  // a row of the delta that A leads on: the block's k-th, its list, the entries of those before it
+    unsigned k;
+    uint32_t at, len, before;
+};
+struct BitsState {
+    unsigned long long tuples, cands, pending, iterations;
+    unsigned slot, small, leaving, over, fix, go;
+};
+__device__ __forceinline__ unsigned warp_sum_before(unsigned mine, unsigned* total) {
+    unsigned incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned v = __shfl_up_sync(FULL, incl, d);
+        if (lane_id() >= (unsigned)d) incl += v;
+    }
+    *total = __shfl_sync(FULL, incl, 31);
+    return incl - mine;
+}
+// B as a block keeps it: per value its matches' start and number, and the matches.
+struct Lists {
+    const unsigned* at;
+    const unsigned short* other;
+};
+// Up to 16 words of a row led through B: where `word` (lane's own, of values from `first` on) has bits, their matches
+// are set in `led`.  Their number, lane by lane.
+template <bool KEPT>
+__device__ __forceinline__ unsigned lead(const Out& o, const Ix& ix, const Lists& kept, unsigned word, unsigned first, unsigned short* queue, unsigned* led) {
+    const unsigned lane = lane_id();
+    unsigned n, c = 0;
+    unsigned to = warp_sum_before(__popc(word), &n);
+    if (!n) return 0;
+    for (; word; word &= word - 1) queue[to++] = (unsigned short)(first + __ffs(word) - 1);
+    __syncwarp();
+    auto other = [&](uint32_t at) { return KEPT ? (uint32_t)kept.other[at] : other_of(ix, at); };
+    auto mark = [&](uint32_t v) {
+        if (v >> o.lo_bits) set_status(o.st, XLB_ERR_CAPACITY, 18, v);
+        else atomicOr(&led[v >> 5], 1u << (v & 31));
+    };
+    for (unsigned base = 0; base < n; base += 64) {  // two values a lane, so that their look-ups are under way together
+        uint32_t s[2], len[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const unsigned i = base + u * 32 + lane;
+            s[u] = len[u] = 0;
+            if (i >= n) continue;
+            if (KEPT) {
+                const unsigned p = kept.at[queue[i]];
+                s[u] = p & 0xFFFF;
+                len[u] = p >> 16;
+            } else find(ix, queue[i], s[u], len[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            c += len[u];
+            for (unsigned far = __ballot_sync(FULL, len[u] > BT_LIST); far; far &= far - 1) {
+                const uint32_t all = __shfl_sync(FULL, len[u], __ffs(far) - 1), from = __shfl_sync(FULL, s[u], __ffs(far) - 1);
+                for (uint32_t j = lane; j < all; j += 32) mark(other(from + j));
+            }
+            if (len[u] > BT_LIST) len[u] = 0;
+        }
+        const unsigned most = __reduce_max_sync(FULL, max(len[0], len[1]));
+        for (unsigned j = 0; j < most; j += 4) {
+            uint32_t v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = j + (u & 3) < len[u >> 2] ? other(s[u >> 2] + j + (u & 3)) : 0u;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (j + (u & 3) < len[u >> 2]) mark(v[u]);
+        }
+    }
+    __syncwarp();
+    return c;
+}
+__global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const Out o, const __grid_constant__ BitsRules rules, const Bits b, uint64_t max_iterations) {
+    extern __shared__ unsigned bt_smem[];
+    __shared__ BitsState st;
+    __shared__ unsigned long long sum_s[2];
+    __shared__ unsigned total_s[BT_OWN];                    // tuples of the block's rows of the delta
+    __shared__ Active act_s[BT_OWN];
+    __shared__ unsigned active_s;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5, W = b.words;
+    constexpr int N = BT_WORDS / 32;
+    unsigned* has = bt_smem;                                // per rule, the values that B leads anywhere
+    unsigned* rows_s = has + DL_RULES * BT_WORDS;           // the block's rows of the delta ...
+    unsigned* led_s = rows_s + BT_OWN * BT_WORDS;           // ... and what B leads them to
+    unsigned* once_s = led_s + BT_OWN * BT_WORDS;           // rows that something leads to,
+    unsigned* more_s = once_s + BT_WORDS;                   // that several things lead to
+    unsigned short* queue = reinterpret_cast<unsigned short*>(more_s + BT_WORDS + warp * 256);
+    unsigned* lists_at = more_s + BT_WORDS + DL_WARPS * 256;
+    unsigned short* lists_other = reinterpret_cast<unsigned short*>(lists_at + (1u << BT_BITS_MAX));
+    const Lists kept{lists_at, lists_other};
+    const unsigned own = b.rows > blockIdx.x ? (b.rows - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const unsigned parts = W > 16 ? 31 - __clz(W / 16) : 0;  // a row is led in 2^parts pieces of work
+    Ctl* ctl = o.ctl;
+    bool bad = false;
+    for (unsigned i = threadIdx.x; i < 2 * BT_WORDS; i += DL_THREADS) once_s[i] = 0;
+    __syncthreads();
+    for (int q = 0; q < rules.n; ++q) {
+        const BitsRule& ru = rules.r[q];
+        constexpr int T = (1 << BT_BITS_MAX) / DL_THREADS;  // (their look-ups are under way together)
+        uint32_t s[T], len[T];
+#pragma unroll
+        for (int i = 0; i < T; ++i) {
+            const unsigned v = threadIdx.x + i * DL_THREADS;
+            s[i] = 0;
+            len[i] = v < W * 32 ? 1 : 0;
+            if (ru.b_list && v < W * 32) find(ru.b, v, s[i], len[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < T; ++i) {
+            const unsigned v = threadIdx.x + i * DL_THREADS, word = __ballot_sync(FULL, len[i] != 0);
+            if (v >= W * 32) continue;
+            if (ru.listed) lists_at[v] = len[i] ? s[i] | (len[i] << 16) : 0u;
+            if (lane == 0) has[q * BT_WORDS + (v >> 5)] = word;
+        }
+#pragma unroll 4
+        for (unsigned i = threadIdx.x; i < ru.listed; i += DL_THREADS) lists_other[i] = (unsigned short)min(other_of(ru.b, i), 0xFFFFu);
+        auto leads_to = [&](uint32_t to) {
+            if (to < b.rows && (atomicOr(&once_s[to >> 5], 1u << (to & 31)) >> (to & 31) & 1u)) atomicOr(&more_s[to >> 5], 1u << (to & 31));
+        };
+        if (!ru.a_list) {
+            for (unsigned v = threadIdx.x; v < b.rows; v += DL_THREADS) leads_to(v);
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < T; ++i) {
+            const unsigned v = threadIdx.x + i * DL_THREADS;
+            len[i] = 0;
+            if (v < b.rows) find(ru.a, v, s[i], len[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < T; ++i) bad |= len[i] > BT_ROWS;
+#pragma unroll 4
+        for (unsigned i = threadIdx.x; i < ru.a_rows; i += DL_THREADS) leads_to(other_of(ru.a, i));
+    }
+    if (threadIdx.x == 0) st = BitsState{};
+    if (__syncthreads_or(bad)) {  // (all blocks find the same)
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->rows_given_up = 1;
+        return;
+    }
+    unsigned passed = 0;
+    for (unsigned phase = 0;; ++phase) {
+        const unsigned cur = phase & 1;
+        const bool leaving = st.leaving != 0;
+        unsigned *next = b.next[cur ^ 1], *reached = b.next[cur];
+        Slot* slot = &ctl->slot[st.slot];
+        if (threadIdx.x < 2) sum_s[threadIdx.x] = 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->slot[st.slot == 2 ? 0 : st.slot + 1] = Slot{};
+        __syncthreads();
+        // the rows of the delta: what they were reached by beyond the head (at first: the seeds)
+        bool some = false;
+        static_assert(BT_OWN <= 2 * DL_WARPS, "a warp has two rows at most");
+        unsigned stamp[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) stamp[i] = warp + i * DL_WARPS < own && phase ? __ldcg(&b.stamp[cur][blockIdx.x + (warp + i * DL_WARPS) * gridDim.x]) : 1u;
+        for (unsigned k = warp; k < own; k += DL_WARPS) {
+            const unsigned row = blockIdx.x + k * gridDim.x;
+            unsigned mine = 0;
+            if (stamp[k >= DL_WARPS]) {
+                unsigned have[N], r[N];
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    const unsigned w = lane + 32 * i;
+                    have[i] = w < W ? __ldcg(&o.visited[(uint64_t)row * W + w]) : 0u;
+                    r[i] = w < W && phase ? __ldcg(&reached[(uint64_t)row * W + w]) : 0u;
+                }
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    const unsigned w = lane + 32 * i, d = phase ? r[i] & ~have[i] : have[i];
+                    if (r[i]) reached[(uint64_t)row * W + w] = 0;
+                    if (r[i] & ~have[i]) o.visited[(uint64_t)row * W + w] = have[i] | d;
+                    if (w < W) rows_s[k * W + w] = d;
+                    mine += __popc(d);
+                }
+                if (lane == 0) b.stamp[cur][row] = 0;
+            }
+            const unsigned all = __reduce_add_sync(FULL, mine);
+            if (lane == 0) {
+                total_s[k] = all;
+                if (all) atomicAdd(&sum_s[0], (unsigned long long)all);
+            }
+            some |= all != 0;
+            if (leaving && all) {
+                unsigned before;
+                before = warp_sum_before(mine, &before);
+                unsigned long long to = 0;
+                if (lane == 0) to = atomicAdd(&ctl->rows_seeds, (unsigned long long)all);
+                to = __shfl_sync(FULL, to, 0) + before;
+                __syncwarp();
+                for (unsigned w = lane; w < W; w += 32)
+                    for (unsigned word = rows_s[k * W + w]; word; word &= word - 1, ++to)
+                        if (to < o.cap) o.log[to] = ((uint64_t)row << 32) | (w * 32 + __ffs(word) - 1);
+            }
+        }
+        some = __syncthreads_or(some) && !leaving;
+        if (some && threadIdx.x == 0) beat(o);
+        unsigned long long cand = 0;
+        for (int q = 0; some && q < rules.n; ++q) {
+            const BitsRule& ru = rules.r[q];
+            if (warp == 0) {  // the rows that A leads anywhere, and how many places those before each are led to
+                unsigned rows = 0, places = 0;
+                for (unsigned k0 = 0; k0 < own; k0 += 32) {
+                    const unsigned k = k0 + lane, all = k < own ? total_s[k] : 0;
+                    uint32_t at = 0, len = all ? 1 : 0;
+                    if (ru.a_list && all) find(ru.a, blockIdx.x + k * gridDim.x, at, len);
+                    if (!ru.b_list) cand += (unsigned long long)all * len;
+                    unsigned more;
+                    const unsigned before = warp_sum_before(len, &more), some = __ballot_sync(FULL, len != 0);
+                    if (len) act_s[rows + __popc(some & lanemask_lt())] = Active{k, at, len, places + before};
+                    rows += __popc(some);
+                    places += more;
+                }
+                if (lane == 0) active_s = rows;
+            }
+            if (ru.b_list)
+                for (unsigned i = threadIdx.x; i < own * W; i += DL_THREADS) led_s[i] = 0;
+            __syncthreads();
+            const unsigned active = active_s;
+            if (ru.b_list) {
+                for (unsigned i = warp; i < active << parts; i += DL_WARPS) {
+                    // (the same part of all rows first: values that lead on may lie in a few parts only)
+                    const Active& on = act_s[i % active];
+                    const unsigned k = on.k, w = i / active * 16 + lane;
+                    const unsigned word = lane < 16 && w < W ? rows_s[k * W + w] & has[q * BT_WORDS + w] : 0u;
+                    cand += (unsigned long long)(ru.listed ? lead<true>(o, ru.b, kept, word, w * 32, queue, led_s + k * W) : lead<false>(o, ru.b, kept, word, w * 32, queue, led_s + k * W)) * on.len;
+                }
+                __syncthreads();
+            }
+            const unsigned* led = ru.b_list ? led_s : rows_s;
+            for (unsigned i = 0; i < active; ++i) {
+                const unsigned k = act_s[i].k;
+                for (unsigned j = (warp - act_s[i].before) % DL_WARPS; j < act_s[i].len; j += DL_WARPS) {  // (a place a warp, one after the other)
+                    const uint32_t to = ru.a_list ? other_of(ru.a, act_s[i].at + j) : blockIdx.x + k * gridDim.x;
+                    if (to >= b.rows) {
+                        if (lane == 0) set_status(o.st, XLB_ERR_CAPACITY, 19, to);
+                        continue;
+                    }
+                    // A row that nothing else leads to is written as it is; it is its own block that looks what is new
+                    // in it.
+                    const bool shared = (more_s[to >> 5] >> (to & 31)) & 1u;
+                    unsigned *out = next + (uint64_t)to * W, any = 0;
+                    if (shared) {
+                        for (unsigned w = lane; w < W; w += 32) {
+                            const unsigned v = led[k * W + w];
+                            // (a word of the head that is being brought up to date only costs an atomic)
+                            if (v & ~__ldcg(&o.visited[(uint64_t)to * W + w])) {
+                                atomicOr(&out[w], v);
+                                any = 1;
+                            }
+                        }
+                    } else {
+                        for (unsigned w = lane; w < W; w += 32) {
+                            const unsigned v = led[k * W + w];
+                            if (v) out[w] = v;
+                            any |= v;
+                        }
+                    }
+                    if (__any_sync(FULL, any) && lane == 0) b.stamp[cur ^ 1][to] = 1;
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int d = 16; d; d >>= 1) cand += __shfl_xor_sync(FULL, cand, d);
+        if (lane == 0 && cand) atomicAdd(&sum_s[1], cand);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (sum_s[0]) atomicAdd(&slot->count, sum_s[0]);
+            if (sum_s[1]) atomicAdd(&slot->cand, sum_s[1]);
+            passed += gridDim.x;
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->arrived) : "memory");
+            st.go = wait_for(o, &ctl->arrived, passed, 0, passed);
+            const unsigned long long found = __ldcg(&slot->count);
+            st.tuples += found;
+            st.cands += st.pending;  // of the joins that found them
+            st.pending = __ldcg(&slot->cand);
+            st.iterations = phase;
+            st.fix = found == 0;
+            st.small = found < BT_SMALL ? st.small + 1 : 0;
+            st.over = st.fix || leaving || phase >= max_iterations;
+            st.leaving = st.small >= BT_LEAVE && st.pending <= o.cap;  // (the log takes whatever the next iteration finds)
+            st.slot = st.slot == 2 ? 0 : st.slot + 1;
+        }
+        __syncthreads();
+        if (!st.go) return;
+        if (st.over) break;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctl->rows_tuples = st.tuples;
+        ctl->rows_candidates = st.cands;
+        ctl->rows_levels = st.iterations ? st.iterations : 1;  // an iteration over nothing finds nothing
+        ctl->rows_left = st.fix ? 0 : 1;
+    }
+}
+// The loop starts on what was given up, or left.
 __global__ void delta_rows_left_k(Ctl* c) {
     c->tail = c->rows_seeds;
+    c->arrived = 0;
+    for (int k = 0; k < 3; ++k) c->slot[k] = Slot{};
     ready(c, false);
 }
 
@@ -1545,12 +1881,72 @@ static bool run_rows(xlb_ctx* c, DeltaLoop& d, const Rules& rs, uint64_t max_ite
     return false;
 }
 
+// Rules whose new first column comes from the old first, and the second from the second, by lists of their own or as
+// they are; from seeds alone.
+static bool bits_apart(const DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, const Keys& known, BitsRules* out) {
+    if (d.square || !d.seeded || known.n || rules.empty() || !variants.empty() || d.lo_bits < BT_BITS_MIN || d.lo_bits > BT_BITS_MAX || d.hi_bits > BT_BITS_MAX || d.hi_bits + d.lo_bits < BT_BITS_BOTH) return false;
+    out->n = (int)rules.size();
+    bool listed = false;  // one rule's B is kept in shared memory
+    for (size_t q = 0; q < rules.size(); ++q) {
+        const DeltaRule& r = rules[q];
+        BitsRule& x = out->r[q];
+        x.a_list = r.hi_src == 2 || r.hi_src == 3;
+        x.b_list = r.lo_src == 2 || r.lo_src == 3;
+        if ((!x.a_list && r.hi_src != 0) || (!x.b_list && r.lo_src != 1) || r.joins != (x.a_list ? 1 : 0) + (x.b_list ? 1 : 0)) return false;
+        if (x.a_list && x.b_list && r.hi_src == r.lo_src) return false;
+        if (x.a_list && r.key_src[r.hi_src - 2] != SRC_HI) return false;
+        if (x.b_list && r.key_src[r.lo_src - 2] != SRC_LO) return false;
+        if (x.a_list) x.a = view_of(*r.ix[r.hi_src - 2]);
+        x.a_rows = x.a_list ? (unsigned)r.ix[r.hi_src - 2]->n : 0;
+        if (x.a_list && r.ix[r.hi_src - 2]->n > BT_EDGES) return false;
+        if (x.b_list) x.b = view_of(*r.ix[r.lo_src - 2]);
+        x.listed = 0;
+        if (x.b_list && !listed && r.ix[r.lo_src - 2]->n <= BT_LISTED) {
+            x.listed = (unsigned)r.ix[r.lo_src - 2]->n;
+            listed = true;
+        }
+    }
+    return true;
+}
+enum class BitsEnd { DONE, DECLINED, LEFT };
+static BitsEnd run_bits(xlb_ctx* c, DeltaLoop& d, BitsRules rules, uint64_t max_iterations, DeltaResult* res, uint64_t* left) {
+    Bits b{};
+    b.rows = 1u << d.hi_bits;
+    b.words = 1u << (d.lo_bits - 5);
+    const uint64_t map = (uint64_t)b.rows * b.words;
+    if (b.rows > BT_OWN * (unsigned)c->sm_count) return BitsEnd::DECLINED;
+    if (c->budget && c->allocated + (map + b.rows) * 8 > c->budget) return BitsEnd::DECLINED;
+    Buf reached = make_buf(c, (map + b.rows) * 8);
+    CUDA_OK(set_async(c, reached->p, 0, reached->bytes));
+    for (int k = 0; k < 2; ++k) {
+        b.next[k] = reached->as<unsigned>() + k * map;
+        b.stamp[k] = reached->as<unsigned>() + 2 * map + k * b.rows;
+    }
+    Out o = out_of(c, d);
+    Ctl* ctl = (Ctl*)d.ctl;
+    void* args[] = {&o, &rules, &b, &max_iterations};
+    prof_begin(c, "expand_mark", 0);
+    CUDA_OK(cudaLaunchCooperativeKernel((const void*)delta_bits_k, dim3((unsigned)c->sm_count), dim3(DL_THREADS), args, BT_SMEM, c->stream));
+    check_launch(c, "expand_mark");
+    unsigned long long w[6];  // tuples, candidates, iterations, left, declined, listed
+    read_words(c, &ctl->rows_tuples, 6, w);
+    if (w[4]) return BitsEnd::DECLINED;
+    res->rows = w[0];
+    res->candidates = w[1];
+    res->iterations = w[2];
+    res->fix = w[3] == 0;
+    *left = w[5];
+    prof_add_bytes(c, "expand_mark", w[0] / 8 + map * 8);
+    return w[5] ? BitsEnd::LEFT : BitsEnd::DONE;
+}
+
 void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
                    DeltaResult* res) {
     if (rules.size() > DL_RULES || variants.size() > SQ_VARIANTS) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules and %zu variants in a delta loop", rules.size(), variants.size());
     if (!c->delta_attr_set) {
         CUDA_OK(cudaFuncSetAttribute(delta_loop_k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DL_SMEM));
         CUDA_OK(cudaFuncSetAttribute(delta_loop_k<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DL_SMEM));
+        CUDA_OK(cudaFuncSetAttribute(delta_bits_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BT_SMEM));
     }
     c->delta_attr_set = true;
     const bool square = d.square;
@@ -1595,14 +1991,33 @@ void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
             r.ix[k] = view_of(*rules[q].ix[k]);
         }
     }
-    Buf by_rows;  // the head after rows were evaluated one by one and some are left
+    Buf by_rows;  // the head after rows were evaluated, and some are left
+    BitsRules bits{};
+    uint64_t earlier = 0;  // iterations before the loop's
+    bool left = false;
     if (rows_apart(d, rules, variants, known)) {
         if (run_rows(c, d, rs, max_iterations, res)) return;
+        left = true;
+    } else if (bits_apart(d, rules, variants, known, &bits)) {
+        uint64_t listed = 0;
+        const BitsEnd end = run_bits(c, d, bits, max_iterations, res, &listed);
+        if (end == BitsEnd::DONE || (end == BitsEnd::LEFT && res->iterations >= max_iterations)) return;
+        if (end == BitsEnd::LEFT) {  // its last tuples are the loop's first delta
+            res->rows -= listed;
+            earlier = res->iterations;
+            max_iterations -= earlier;
+            delta_rows_left_k<<<1, 1, 0, c->stream>>>((Ctl*)d.ctl);
+            check_launch(c, "delta_begin");
+            d.room = listed;
+            left = true;
+        }
+    }
+    if (left) {
         by_rows = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
         CUDA_OK(copy_async(c, by_rows->p, d.visited->p, d.words * 4, cudaMemcpyDeviceToDevice));
     }
     DeltaResult rows_done = *res;
-    if (!by_rows) rows_done.fix = true;
+    if (!by_rows || earlier) rows_done.fix = true;
     Buf heavy = make_buf(c, (uint64_t)DL_HEAVY_MAX * sizeof(Heavy));
     if (!d.seeded) {
         delta_begin_k<<<1, 1, 0, c->stream>>>((Ctl*)d.ctl, square);
@@ -1618,7 +2033,7 @@ void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         unsigned long long w[7];  // tail, start, end, iterations, candidates, fix, overflow
         read_words(c, d.ctl, 7, w);
         res->rows = rows_done.rows + w[0];
-        res->iterations = std::max<uint64_t>(rows_done.iterations, w[3]);
+        res->iterations = earlier ? earlier + w[3] : std::max<uint64_t>(rows_done.iterations, w[3]);
         res->candidates = rows_done.candidates + w[4];
         res->fix = rows_done.fix && w[5] != 0;
         prof_add_bytes(c, "expand_mark", w[4] * 4ull + w[0] * 16ull);
