@@ -86,3 +86,41 @@ def test_small_sorts(p, n):
         order = np.lexsort([c for c in reversed(cols)])
         for g, c in zip(p.download(p.sort(b, keys)), cols + [np.arange(n, dtype=np.uint32)]):
             assert np.array_equal(g, c[order])
+
+
+def joined(left, right, lk, rk):
+    """Matches of the rows of `left`, in their order and each in the order of `right`."""
+    rows = {}
+    for i, k in enumerate(zip(*(right[c].tolist() for c in rk))):
+        rows.setdefault(k, []).append(i)
+    pairs = [(i, j) for i, k in enumerate(zip(*(left[c].tolist() for c in lk))) for j in rows.get(k, [])]
+    l, r = (np.array(x, dtype=np.int64) for x in (zip(*pairs) if pairs else ((), ())))
+    return [c[l] for c in left] + [c[r] for c in right]
+
+
+# groups of up to 64 rows; up to four outputs a build row go out from the chains, more from lists.  Keys of 0 and of all ones.
+@pytest.mark.parametrize("kind", ["u32", "u64", "two"])
+@pytest.mark.parametrize("sizes", [[1], [1, 2, 3, 4], [4, 5, 6], [1, 31, 32, 33, 63, 64], [64]], ids=str)
+@pytest.mark.parametrize("probes", [1, 31, 900, 5000])
+def test_joins_from_chains_and_from_lists(kind, sizes, probes):
+    rng = np.random.default_rng(len(sizes) * probes)
+    sizes = np.resize(sizes, 90)
+    top = (1 << 64) - 1 if kind == "u64" else (1 << 32) - 1
+    dtype = np.uint64 if kind == "u64" else np.uint32
+    names = np.concatenate([np.array([0, top], dtype=dtype), (rng.choice(1 << 31, 98, replace=False) + 1).astype(dtype)])
+    key = rng.permutation(np.repeat(names[:90], sizes))  # (ten names have no rows)
+    ask = names[rng.integers(0, 100, probes)]
+    left, right = [ask, np.arange(probes, dtype=np.uint32)], [np.arange(len(key), dtype=np.uint64), key]
+    lk, rk = [0], [1]
+    if kind == "two":
+        left, right = left + [ask % dtype(3)], right + [key % dtype(3)]
+        lk, rk = [0, 2], [1, 2]
+    p = KernelProvider(device=0)
+    lb, rb = p.create_buffer_from_slices(left), p.create_buffer_from_slices(right)
+    for g, w in zip(p.download(p.hash_join_v2(lb, rb, lk, rk)), joined(left, right, lk, rk)):
+        assert np.array_equal(g, w)
+    there = np.isin(ask, key)
+    for how, keep in ((A.JOIN_SEMI, there), (A.JOIN_ANTI, ~there)):
+        for g, w in zip(p.download(p.hash_join_v2(lb, rb, lk, rk, how)), left):
+            assert np.array_equal(g, w[keep])
+    p.close()

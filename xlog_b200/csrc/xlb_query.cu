@@ -50,27 +50,30 @@ __device__ __forceinline__ void copy_row(const Cols& c, uint64_t left, uint64_t 
     }
 }
 
-// ---- keys of the build side: open addressing, a slot names the first row (plus one) that brought its key
-__device__ __forceinline__ uint64_t claim(const KeyCols& keys, unsigned int* rep, uint64_t mask, uint64_t row, uint64_t key, DevStatus* st) {
-    uint64_t h = mix64(key) & mask;
+// ---- keys of the build side: open addressing over the keys themselves, zero where a slot is free.  The key 0 has
+// the slot behind the last one.  (Slots that named a row, whose key was then looked up: 4 M probes of 400 000 keys
+// 73 us, now 45; their insertion 18, now 14: what is left is a random sector of the L2 a probe, 90 G/s.)
+__device__ __forceinline__ uint64_t slot_of(uint64_t key, uint64_t mask) { return key ? mix64(key) & mask : mask + 1; }
+__device__ __forceinline__ void claim(unsigned long long* slots, uint64_t mask, uint64_t key, DevStatus* st) {
+    uint64_t h = slot_of(key, mask);
+    if (!key) {
+        slots[h] = 1;
+        return;
+    }
     for (uint64_t probe = 0; probe <= mask; ++probe) {  // bounded by the table size
-        unsigned cur = rep[h];
-        if (cur == 0) {
-            cur = atomicCAS(&rep[h], 0u, (unsigned)row + 1);
-            if (cur == 0) return h;
-        }
-        if (keys(cur - 1) == key) return h;
+        unsigned long long cur = slots[h];
+        if (cur == 0) cur = atomicCAS(&slots[h], 0ull, (unsigned long long)key);
+        if (cur == 0 || cur == key) return;
         h = (h + 1) & mask;
     }
-    set_status(st, XLB_ERR_CAPACITY, 20, row);
-    return 0;
+    set_status(st, XLB_ERR_CAPACITY, 20, key);
 }
-__global__ void __launch_bounds__(BLOCK) exists_build_k(KeyCols keys, uint64_t n, unsigned int* __restrict__ rep, uint64_t mask, DevStatus* st) {
-    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) claim(keys, rep, mask, i, keys(i), st);
+__global__ void __launch_bounds__(BLOCK) exists_build_k(KeyCols keys, uint64_t n, unsigned long long* __restrict__ slots, uint64_t mask, DevStatus* st) {
+    for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) claim(slots, mask, keys(i), st);
 }
 // One bit per probe row (has a match == want), and for each tile of SCAN_TILE rows how many were selected before it.
 constexpr int QT_ROUNDS = SCAN_TILE / BLOCK;
-__global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t n, KeyCols keys, const unsigned int* __restrict__ rep, uint64_t mask, bool want,
+__global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t n, const unsigned long long* __restrict__ slots, uint64_t mask, bool want,
                                                        unsigned int* __restrict__ bits, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total,
                                                        const Publish pub) {
     __shared__ uint32_t sm[33];
@@ -79,34 +82,25 @@ __global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t 
     const uint64_t base = (uint64_t)tile * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS;  // a warp's rows side by side
     uint32_t cnt = 0;
     uint64_t key[QT_ROUNDS];
-    unsigned cur[QT_ROUNDS];
+    unsigned long long cur[QT_ROUNDS];
 #pragma unroll
     for (int r = 0; r < QT_ROUNDS; ++r) {
         const uint64_t i = base + r * 32 + lane_id();
         key[r] = i < n ? probe(i) : 0;
     }
 #pragma unroll
-    for (int r = 0; r < QT_ROUNDS; ++r) cur[r] = base + r * 32 + lane_id() < n ? __ldg(&rep[mix64(key[r]) & mask]) : 0u;
-    unsigned same = 0;  // (rounds whose first slot holds the key: all looked at together, 4 M probes 83 us -> 71)
-#pragma unroll
-    for (int r = 0; r < QT_ROUNDS; ++r)
-        if (cur[r] && keys(cur[r] - 1) == key[r]) same |= 1u << r;
+    for (int r = 0; r < QT_ROUNDS; ++r) cur[r] = base + r * 32 + lane_id() < n ? __ldg(&slots[slot_of(key[r], mask)]) : 0ull;
 #pragma unroll
     for (int r = 0; r < QT_ROUNDS; ++r) {
         const uint64_t i = base + r * 32 + lane_id();
-        bool found = (same >> r) & 1u;
-        if (cur[r] && !found) {
+        if (key[r]) {
             uint64_t h = mix64(key[r]) & mask;
-            for (uint64_t p = 0; p < mask; ++p) {  // bounded by the table size
+            for (uint64_t p = 0; p < mask && cur[r] && cur[r] != key[r]; ++p) {  // bounded by the table size
                 h = (h + 1) & mask;
-                const unsigned c = __ldg(&rep[h]);
-                if (!c) break;
-                if (keys(c - 1) == key[r]) {
-                    found = true;
-                    break;
-                }
+                cur[r] = __ldg(&slots[h]);
             }
         }
+        const bool found = cur[r] && (!key[r] || cur[r] == key[r]);
         const unsigned b = __ballot_sync(FULL, i < n && found == want);
         if (lane_id() == 0 && base + r * 32 < n) bits[(base + r * 32) >> 5] = b;
         cnt += __popc(b);
@@ -116,9 +110,12 @@ __global__ void __launch_bounds__(BLOCK) exists_probe_k(KeyCols probe, uint64_t 
     if (threadIdx.x < 32) leave_tile(tiles, tile, tot, tile_offs, total);
     publish_last(pub);
 }
-// The selected rows, all columns, in order.
+// The selected rows, all columns, in order.  (A third of 4 M rows of 16 bytes: 29 us with a lane for every row, selected or
+// not; 20 closed up first.)
 __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned int* __restrict__ bits, uint64_t n, const uint64_t* __restrict__ tile_offs, const Publish pub) {
     __shared__ uint32_t sm[33];
+    __shared__ unsigned char row_s[BLOCK / 32][32 * QT_ROUNDS];
+    static_assert(32 * QT_ROUNDS <= 256, "a row of the warp's is a byte");
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (threadIdx.x & ~31u) * QT_ROUNDS;
     unsigned w[QT_ROUNDS];
     uint32_t cnt = 0;
@@ -129,29 +126,38 @@ __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned
     }
     uint32_t tot;
     uint32_t ex = block_exclusive_scan<uint32_t>(lane_id() == 0 ? cnt : 0u, &tot, sm);
-    uint64_t pos = tile_offs[blockIdx.x] + __shfl_sync(FULL, ex, 0);
+    // The warp's selected rows are closed up first, so that every lane has one to copy.
+    const uint64_t pos = tile_offs[blockIdx.x] + __shfl_sync(FULL, ex, 0);
+    unsigned char* mine = row_s[threadIdx.x >> 5];
+    unsigned at = 0;
+#pragma unroll
     for (int r = 0; r < QT_ROUNDS; ++r) {
-        if ((w[r] >> lane_id()) & 1u) {
-            const uint64_t to = pos + __popc(w[r] & lanemask_lt());
-            copy_row(cols, base + r * 32 + lane_id(), base + r * 32 + lane_id(), to);
-        }
-        pos += __popc(w[r]);
+        if ((w[r] >> lane_id()) & 1u) mine[at + __popc(w[r] & lanemask_lt())] = (unsigned char)(r * 32 + lane_id());
+        at += __popc(w[r]);
     }
+    __syncwarp();
+    for (unsigned t = lane_id(); t < at; t += 32) copy_row(cols, base + mine[t], base + mine[t], pos + t);
     publish_last(pub);
 }
 
 // ---- inner join: the build rows grouped by key
-// Every row finds its key's slot and takes a number in the group there; group starts are the prefix
-// sums of the counts.  The numbers come in no particular order, so each group's rows are put in row
-// order afterwards, which for the usual handful is a few compares.  A group above JOIN_GROUP_MAX rows
-// is reported when it is met, the launches behind end at once, and the caller sorts instead.
+// A slot holds a key, the number of its rows and the last of them; every row names the one before it.  Where the
+// rows go out a few times and groups are short, the chains are followed when they do (join_chains_k), and a
+// handful of rows is put in order by a few compares.  Else lists are made of them first: starts, places,
+// then each group put in row order (three kernels, 92 us for 2 M rows, which used to come before every join).  The
+// line, 1 M build rows, chains / lists: groups of 2, 8 outputs a build row 257 / 322 us, 16 outputs 422 / 503; groups
+// of 8, 8 outputs 249 / 284, 16 outputs 427 / 422; groups of 32, one output 277 / 254 (16 384 rows: 159 / 80).
+//   A group above JOIN_GROUP_MAX rows is reported when it is met, the launches behind end at once, and the caller
+// sorts instead.
 //   The rows of a hub queue for its slot and on its count, some 13 ns each, so a build side of JOIN_SAMPLED
 // rows and more is looked at first: while the other blocks clear the slots, one picks rows evenly and
 // reports a key that it meets JOIN_OFTEN times, which one of JOIN_GROUP_MAX rows cannot be.  (2 M build rows,
-// 4 M probe rows, B200: one key of 1000 rows 947 -> 797 us, one of 1 M that no probe row asks for 1592 -> 685; the
-// sort alone, before there was this route, 768 and 673; keys of at most 64 rows 393 -> 396.  The sample costs
-// some 3 us of 200, so smaller build sides go without: 32 768 rows all of one key 122 us sampled, 138 counted.)
+// 4 M probe rows, B200: one key of 1000 rows 947 us without the sample, 787 with it, one of 1 M that no probe row asks
+// for 1592 and 691; the sort alone 768 and 673; keys of at most 64 rows 330.  The sample costs some 3 us of 200,
+// so smaller build sides go without: 32 768 rows all of one key 122 us sampled, 157 counted.)
 constexpr unsigned JOIN_GROUP_MAX = 64;
+constexpr uint64_t JOIN_CHAIN_OUTPUTS = 8;  // outputs a build row, and rows of the longest group, up to which they
+constexpr unsigned JOIN_CHAIN_ROWS = 16;    // go out from the chains
 constexpr unsigned JOIN_SAMPLE = 1024, JOIN_OFTEN = 16;  // (a row a thread: a chain of latencies as long as the clearing)
 constexpr uint64_t JOIN_SAMPLED = 1ull << 16;
 __global__ void __launch_bounds__(JOIN_SAMPLE) group_clear_k(KeyCols keys, uint64_t n, uint4* __restrict__ slots, uint64_t slot_vecs, uint64_t* __restrict__ words, uint64_t nwords,
@@ -176,33 +182,69 @@ __global__ void __launch_bounds__(JOIN_SAMPLE) group_clear_k(KeyCols keys, uint6
         break;
     }
 }
-__global__ void __launch_bounds__(BLOCK) group_count_k(KeyCols keys, uint64_t n, unsigned int* __restrict__ rep, unsigned int* __restrict__ count, uint64_t mask, uint2* __restrict__ place,
+// (16 bytes at once, of 16-byte aligned memory; what was there)
+__device__ __forceinline__ ulonglong2 cas16(ulonglong2* at, ulonglong2 want, ulonglong2 to) {
+    ulonglong2 was;
+    asm volatile(
+        "{ .reg .b128 w, t, o; mov.b128 w, {%2, %3}; mov.b128 t, {%4, %5}; atom.global.cas.b128 o, [%6], w, t; mov.b128 {%0, %1}, o; }"
+        : "=l"(was.x), "=l"(was.y)
+        : "l"(want.x), "l"(want.y), "l"(to.x), "l"(to.y), "l"(at)
+        : "memory");
+    return was;
+}
+// The first row of a key brings key, count and link by one exchange, the others count and link by one each (an
+// exchange in a loop for them, too, took 1 ms on 32 768 rows of one key, against 157 us).  place: what the lists need.
+// Bound by atomics whose answer is waited for, some 50 G/s on a table of 64 MB: 2 M rows 60 us (an atomic each for key,
+// count and link 71; four rows a thread under way together 60 as well).
+__global__ void __launch_bounds__(BLOCK) group_chain_k(KeyCols keys, uint64_t n, ulonglong2* __restrict__ slots, uint64_t mask, uint32_t* __restrict__ before, uint2* __restrict__ place,
                                                       volatile unsigned int* too_long, DevStatus* st) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
         const unsigned stop = *too_long;
         const uint64_t key = keys(i);
         if (stop) return;
-        const uint64_t h = claim(keys, rep, mask, i, key, st);
-        const unsigned number = atomicAdd(&count[h], 1u);
-        if (number >= JOIN_GROUP_MAX) *too_long = 1;
+        uint64_t h = slot_of(key, mask);
+        unsigned number = 0, link = 0;
+        for (uint64_t probe = 0;; ++probe) {
+            if (probe > mask) {  // bounded by the table size
+                set_status(st, XLB_ERR_CAPACITY, 20, i);
+                break;
+            }
+            unsigned long long there = *(volatile unsigned long long*)&slots[h].x;
+            if (key && !there) {
+                there = cas16(&slots[h], make_ulonglong2(0, 0), make_ulonglong2(key, ((unsigned long long)(i + 1) << 32) | 1)).x;
+                if (!there) break;
+            }
+            if (there == key) {
+                unsigned* entry = reinterpret_cast<unsigned*>(&slots[h].y);  // [0] rows, [1] the last one (plus one)
+                number = atomicAdd(&entry[0], 1u);
+                if (number >= JOIN_GROUP_MAX) {  // (the chain is not used any more)
+                    *too_long = 1;
+                    return;
+                }
+                link = atomicExch(&entry[1], (unsigned)i + 1);
+                break;
+            }
+            h = (h + 1) & mask;
+        }
+        before[i] = link;
         place[i] = make_uint2((unsigned)h, number);
     }
 }
-// A slot's entry: its key, where its rows lie (start << 32) and how many they are.  Groups may lie in any
-// order: a block takes the room for its slots' rows with one atomic.
-__global__ void __launch_bounds__(BLOCK) group_start_k(KeyCols keys, const unsigned int* __restrict__ rep, const unsigned int* __restrict__ count, uint64_t cap, ulonglong2* __restrict__ table,
-                                                      unsigned int* __restrict__ used, const unsigned int* __restrict__ too_long) {
+// Lists, for joins whose rows go out often or whose groups are long: a slot's entry becomes start << 32 | rows, and
+// starts[last row of a chain] is the start as well.  Groups may lie in any order: a block takes the room for its slots'
+// rows with one atomic.
+__global__ void __launch_bounds__(BLOCK) group_start_k(ulonglong2* __restrict__ slots, uint64_t count, uint32_t* __restrict__ starts, unsigned int* __restrict__ used) {
     __shared__ uint32_t sm[33], room_s;
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + threadIdx.x;
-    unsigned len[SCAN_IPT], mine = 0;
-    const unsigned stop = *too_long;
+    unsigned len[SCAN_IPT], last[SCAN_IPT], mine = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_IPT; ++k) {
         const uint64_t h = base + (uint64_t)k * BLOCK;
-        len[k] = h < cap ? count[h] : 0u;
+        const unsigned long long e = h < count ? slots[h].y : 0ull;
+        len[k] = (unsigned)e;
+        last[k] = (unsigned)(e >> 32);
         mine += len[k];
     }
-    if (stop) return;
     uint32_t tot;
     uint32_t at = block_exclusive_scan<uint32_t>(mine, &tot, sm);
     if (threadIdx.x == 0) room_s = tot ? atomicAdd(used, tot) : 0u;
@@ -210,35 +252,31 @@ __global__ void __launch_bounds__(BLOCK) group_start_k(KeyCols keys, const unsig
     at += room_s;
 #pragma unroll
     for (int k = 0; k < SCAN_IPT; ++k) {
-        const uint64_t h = base + (uint64_t)k * BLOCK;
-        if (h >= cap) break;
-        table[h] = len[k] ? make_ulonglong2(keys(rep[h] - 1), ((unsigned long long)at << 32) | len[k]) : make_ulonglong2(0, 0);
+        if (!len[k]) continue;
+        reinterpret_cast<unsigned*>(&slots[base + (uint64_t)k * BLOCK].y)[1] = at;
+        starts[last[k] - 1] = at;
         at += len[k];
     }
 }
-__global__ void __launch_bounds__(BLOCK) group_fill_k(const uint2* __restrict__ place, uint64_t n, const ulonglong2* __restrict__ table, uint32_t* __restrict__ rows,
-                                                     const unsigned int* __restrict__ too_long) {
-    const unsigned stop = *too_long;
+__global__ void __launch_bounds__(BLOCK) group_fill_k(const uint2* __restrict__ place, uint64_t n, const ulonglong2* __restrict__ slots, uint32_t* __restrict__ rows) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
         const uint2 p = place[i];
-        if (stop) return;
-        rows[(uint32_t)(table[p.x].y >> 32) + p.y] = (uint32_t)i;
+        rows[(uint32_t)(slots[p.x].y >> 32) + p.y] = (uint32_t)i;
     }
 }
-// Four slots a thread at a time: a slot is a chain of three loads (60 us one at a time for 4 M slots, against 50).
-__global__ void __launch_bounds__(BLOCK) group_order_k(const unsigned int* __restrict__ count, const ulonglong2* __restrict__ table, uint64_t cap, uint32_t* __restrict__ rows,
-                                                      const unsigned int* __restrict__ too_long) {
-    const unsigned stop = *too_long;
+// Four slots a thread at a time: a slot is a chain of loads (60 us one at a time for 4 M slots, against 50).
+__global__ void __launch_bounds__(BLOCK) group_order_k(const ulonglong2* __restrict__ slots, uint64_t count, uint32_t* __restrict__ rows) {
     constexpr int S = 4, SHORT = 4;
     const uint64_t step = (uint64_t)gridDim.x * BLOCK;
-    for (uint64_t h0 = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; h0 < cap; h0 += S * step) {
+    for (uint64_t h0 = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; h0 < count; h0 += S * step) {
         unsigned len[S], at[S];
         uint32_t v[S][SHORT];
 #pragma unroll
-        for (int s = 0; s < S; ++s) len[s] = h0 + s * step < cap ? count[h0 + s * step] : 0u;
-        if (stop) return;
-#pragma unroll
-        for (int s = 0; s < S; ++s) at[s] = len[s] > 1 ? (unsigned)(table[h0 + s * step].y >> 32) : 0u;
+        for (int s = 0; s < S; ++s) {
+            const unsigned long long e = h0 + s * step < count ? slots[h0 + s * step].y : 0ull;
+            len[s] = (unsigned)e;
+            at[s] = (unsigned)(e >> 32);
+        }
 #pragma unroll
         for (int s = 0; s < S; ++s)
 #pragma unroll
@@ -269,10 +307,10 @@ __global__ void __launch_bounds__(BLOCK) group_order_k(const unsigned int* __res
         }
     }
 }
-// What each probe row meets (start << 32 | rows) and how many outputs come before it: in its tile, and before the tile.
+// What each probe row meets (its slot's entry) and how many outputs come before it: in its tile, and before the tile.
 __global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n, const ulonglong2* __restrict__ table, uint64_t mask, uint64_t* __restrict__ match,
                                                      uint32_t* __restrict__ in_tile, SelectTiles tiles, uint64_t* __restrict__ tile_offs, uint64_t* __restrict__ total,
-                                                     const unsigned int* __restrict__ too_long, const Publish pub) {
+                                                     unsigned int* __restrict__ longest, const unsigned int* __restrict__ too_long, const Publish pub) {
     __shared__ uint64_t sm[33];
     __shared__ unsigned tile_s;
     const unsigned stop = *too_long;
@@ -284,8 +322,9 @@ __global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n,
 #pragma unroll
     for (int r = 0; r < QT_ROUNDS; ++r) key[r] = base + r * 32 < n ? probe(base + r * 32) : 0;
 #pragma unroll
-    for (int r = 0; r < QT_ROUNDS; ++r) m[r] = base + r * 32 < n ? __ldg(&table[mix64(key[r]) & mask]) : make_ulonglong2(0, 0);
+    for (int r = 0; r < QT_ROUNDS; ++r) m[r] = base + r * 32 < n ? __ldg(&table[slot_of(key[r], mask)]) : make_ulonglong2(0, 0);
     uint64_t mine = 0;
+    uint32_t most = 0;
 #pragma unroll
     for (int r = 0; r < QT_ROUNDS; ++r) {
         uint64_t h = mix64(key[r]) & mask;
@@ -295,7 +334,10 @@ __global__ void __launch_bounds__(BLOCK) join_probe_k(KeyCols probe, uint64_t n,
         }
         if (m[r].x != key[r]) m[r].y = 0;
         mine += (uint32_t)m[r].y;
+        most = max(most, (uint32_t)m[r].y);
     }
+    most = __reduce_max_sync(FULL, most);
+    if (lane == 0 && most > *longest) atomicMax(longest, most);  // (a look first: it settles soon)
     for (int d = 16; d; d >>= 1) mine += __shfl_xor_sync(FULL, mine, d);
     uint64_t tot;
     uint64_t at = block_exclusive_scan<uint64_t>(lane == 0 ? mine : 0ull, &tot, sm);
@@ -327,7 +369,7 @@ struct OutputsBefore {
 // before the next; one where that still leaves SMs without a block (1848 outputs: 22 us -> 14; 2.6 M: 71 -> 61).
 template <int IPT>
 __global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict__ match, const OutputsBefore off, uint64_t nrows, uint64_t total, const uint32_t* __restrict__ rows,
-                                                    Cols cols, const Publish pub) {
+                                                    const uint32_t* __restrict__ starts, Cols cols, const Publish pub) {
     constexpr int TILE = BLOCK * IPT;
     __shared__ unsigned rel[TILE + 2];
     __shared__ uint64_t row_s[2];
@@ -373,7 +415,10 @@ __global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict_
         l[u] = r0 + lo - 1;
     }
 #pragma unroll
-    for (int u = 0; u < IPT; ++u) r[u] += match[l[u]] >> 32;
+    for (int u = 0; u < IPT; ++u) {
+        const unsigned t = u * BLOCK + threadIdx.x;
+        if (t < (unsigned)(o1 - o0)) r[u] += starts[(match[l[u]] >> 32) - 1];
+    }
 #pragma unroll
     for (int u = 0; u < IPT; ++u) {
         const unsigned t = u * BLOCK + threadIdx.x;
@@ -383,6 +428,68 @@ __global__ void __launch_bounds__(BLOCK) join_emit_k(const uint64_t* __restrict_
     for (int u = 0; u < IPT; ++u) {
         const unsigned t = u * BLOCK + threadIdx.x;
         if (t < (unsigned)(o1 - o0)) copy_row(cols, l[u], r[u], o0 + t);
+    }
+    publish_last(pub);
+}
+
+// The same from the chains: a warp takes 32 probe rows, follows their chains together, puts the rows in order in
+// shared memory and writes their outputs side by side.  (2.6 M outputs of five columns 64 us, bound by the random
+// sectors of the build side's columns; from lists 57, whose making took 92.)
+constexpr int GL_SHORT = 4;
+constexpr unsigned JC_ROOM = 512;  // outputs at a time; a row's are fewer
+static_assert(JOIN_GROUP_MAX <= JC_ROOM, "a probe row fits");
+__global__ void __launch_bounds__(BLOCK) join_chains_k(const uint64_t* __restrict__ match, const OutputsBefore off, uint64_t nrows, const uint32_t* __restrict__ before, Cols cols,
+                                                      const Publish pub) {
+    __shared__ uint32_t right_s[BLOCK / 32][JC_ROOM];
+    __shared__ unsigned char left_s[BLOCK / 32][JC_ROOM];
+    const unsigned lane = lane_id();
+    uint32_t* right = right_s[threadIdx.x >> 5];
+    unsigned char* left = left_s[threadIdx.x >> 5];
+    const uint64_t base = (uint64_t)blockIdx.x * BLOCK + (threadIdx.x & ~31u);
+    const uint64_t m = base + lane < nrows ? match[base + lane] : 0ull;
+    const unsigned len = (unsigned)m;
+    unsigned incl = len;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned v = __shfl_up_sync(FULL, incl, d);
+        if (lane >= (unsigned)d) incl += v;
+    }
+    const unsigned all = __shfl_sync(FULL, incl, 31);
+    const uint64_t to = all ? off[base] : 0;
+    uint32_t v[GL_SHORT];
+    v[0] = (uint32_t)(m >> 32);
+#pragma unroll
+    for (int k = 1; k < GL_SHORT; ++k) v[k] = k < (int)len ? __ldg(&before[v[k - 1] - 1]) : 0xFFFFFFFFu;
+    for (unsigned done = 0; done < all;) {  // as many rows at a time as there is room for
+        const bool mine = incl > done && incl - done <= JC_ROOM;
+        const unsigned at = incl - len - done, stop = __shfl_sync(FULL, incl, 31 - __clz(__ballot_sync(FULL, mine)));
+        if (mine && len <= GL_SHORT) {  // placed by rank (row numbers differ)
+#pragma unroll
+            for (int k = 0; k < GL_SHORT; ++k) {
+                unsigned rank = 0;
+#pragma unroll
+                for (int q = 0; q < GL_SHORT; ++q) rank += v[q] < v[k];  // (what is past the end is above all)
+                if (k < (int)len) {
+                    right[at + rank] = v[k] - 1;
+                    left[at + k] = (unsigned char)lane;
+                }
+            }
+        } else if (mine) {
+            uint32_t x = v[0];
+            for (unsigned a = 0; a < len; ++a, x = x ? __ldg(&before[x - 1]) : 0) {  // insertion sort in place
+                unsigned b = a;
+                while (b && right[at + b - 1] > x - 1) {
+                    right[at + b] = right[at + b - 1];
+                    --b;
+                }
+                right[at + b] = x - 1;
+                left[at + a] = (unsigned char)lane;
+            }
+        }
+        __syncwarp();
+        for (unsigned t = lane; t < stop - done; t += 32) copy_row(cols, base + left[t], right[t], to + done + t);
+        __syncwarp();
+        done = stop;
     }
     publish_last(pub);
 }
@@ -548,20 +655,21 @@ xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint
     uint64_t cap = 1024;
     while (cap < 2 * r->rows) cap <<= 1;
     const uint64_t n = l->rows, tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    Buf rep = make_buf(c, cap * 4 + sweep_words(tiles) * 8);
-    CUDA_OK(set_async(c, rep->p, 0, cap * 4 + sweep_words(tiles) * 8));
+    const uint64_t words = cap + 1 + sweep_words(tiles);
+    Buf slots = make_buf(c, words * 8);
+    CUDA_OK(set_async(c, slots->p, 0, words * 8));
     const KeyCols build = key_cols(r, rk, nk), probe = key_cols(l, lk, nk);
     if (r->rows) {
         prof_begin(c, "hash_insert", 0);
-        exists_build_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(build, r->rows, rep->as<unsigned int>(), cap - 1, c->d_status);
+        exists_build_k<<<grid_for(c, r->rows), BLOCK, 0, c->stream>>>(build, r->rows, slots->as<unsigned long long>(), cap - 1, c->d_status);
         check_launch(c, "hash_insert");
     }
     Buf bits = make_buf(c, (n + 31) / 32 * 4), offs = make_buf(c, tiles * 8 + 8);
     uint64_t* total = offs->as<uint64_t>() + tiles;
-    Sweep sweep(c, tiles, rep->as<uint64_t>() + cap / 2, offs->as<uint64_t>(), total);
+    Sweep sweep(c, tiles, slots->as<uint64_t>() + cap + 1, offs->as<uint64_t>(), total);
     prof_begin(c, "hash_probe", n * 12ull);
     const Publish pub = sweep.publish(total, 1);
-    exists_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, n, build, rep->as<unsigned int>(), cap - 1, want, bits->as<unsigned int>(), sweep.tiles, sweep.leave_at, total, pub);
+    exists_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, n, slots->as<unsigned long long>(), cap - 1, want, bits->as<unsigned int>(), sweep.tiles, sweep.leave_at, total, pub);
     check_launch(c, "hash_probe");
     sweep.finish();
     unsigned long long m;
@@ -588,39 +696,30 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     uint64_t cap = 1024;
     while (cap < 2 * n) cap <<= 1;
     const KeyCols build = key_cols(r, rk, nk), probe = key_cols(l, lk, nk);
-    const uint64_t tiles = (l->rows + SCAN_TILE - 1) / SCAN_TILE, clear = cap * 8 + (3 + sweep_words(tiles)) * 8;
-    Buf slots = make_buf(c, clear), place = make_buf(c, n * 8), rows = make_buf(c, n * 4), table = make_buf(c, cap * 16);
-    unsigned int *rep = slots->as<unsigned int>(), *count = rep + cap;
-    uint64_t* words = slots->as<uint64_t>() + cap;  // [0] outputs, [1] a group is too long, [2] room taken for groups, then the sweep's
+    const uint64_t tiles = (l->rows + SCAN_TILE - 1) / SCAN_TILE, nwords = 4 + sweep_words(tiles);
+    Buf table = make_buf(c, (cap + 1) * 16 + nwords * 8), before = make_buf(c, n * 4), place = make_buf(c, n * 8);
+    ulonglong2* slots = table->as<ulonglong2>();
+    uint64_t* words = (uint64_t*)(slots + cap + 1);  // [0] outputs, [1] a group is too long, [2] rows of the longest group met, [3] room taken for groups, then the sweep's
     unsigned int* too_long = (unsigned int*)(words + 1);
     if (n < JOIN_SAMPLED) {
-        CUDA_OK(set_async(c, slots->p, 0, clear));
+        CUDA_OK(set_async(c, table->p, 0, (cap + 1) * 16 + nwords * 8));
     } else {
-        prof_begin(c, "group_clear", cap * 8ull);
-        group_clear_k<<<(unsigned)std::min<uint64_t>((cap / 2 + JOIN_SAMPLE - 1) / JOIN_SAMPLE, 2ull * c->sm_count) + 1, JOIN_SAMPLE, 0, c->stream>>>(build, n, slots->as<uint4>(), cap / 2, words, clear / 8 - cap, too_long);
+        prof_begin(c, "group_clear", cap * 16ull);
+        group_clear_k<<<(unsigned)std::min<uint64_t>((cap + JOIN_SAMPLE - 1) / JOIN_SAMPLE, 2ull * c->sm_count) + 1, JOIN_SAMPLE, 0, c->stream>>>(build, n, table->as<uint4>(), cap + 1, words, nwords, too_long);
         check_launch(c, "group_clear");
     }
     prof_begin(c, "hash_insert", n * 8ull);
-    group_count_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, rep, count, cap - 1, place->as<uint2>(), too_long, c->d_status);
+    group_chain_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, slots, cap - 1, before->as<uint32_t>(), place->as<uint2>(), too_long, c->d_status);
     check_launch(c, "hash_insert");
-    prof_begin(c, "group_start", cap * 24ull);
-    group_start_k<<<(unsigned)((cap + SCAN_TILE - 1) / SCAN_TILE), BLOCK, 0, c->stream>>>(build, rep, count, cap, table->as<ulonglong2>(), (unsigned int*)(words + 2), too_long);
-    check_launch(c, "group_start");
-    prof_begin(c, "group_fill", n * 16ull);
-    group_fill_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(place->as<uint2>(), n, table->as<ulonglong2>(), rows->as<uint32_t>(), too_long);
-    check_launch(c, "group_fill");
-    prof_begin(c, "group_order", cap * 4ull);
-    group_order_k<<<grid_for(c, cap), BLOCK, 0, c->stream>>>(count, table->as<ulonglong2>(), cap, rows->as<uint32_t>(), too_long);
-    check_launch(c, "group_order");
     Buf match = make_buf(c, l->rows * 8), in_tile = make_buf(c, l->rows * 4), offs = make_buf(c, tiles * 8);
-    Sweep sweep(c, tiles, words + 3, offs->as<uint64_t>(), words);
+    Sweep sweep(c, tiles, words + 4, offs->as<uint64_t>(), words);
     prof_begin(c, "hash_probe", l->rows * 32ull);
-    const Publish pub = sweep.publish(words, 2);
-    join_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, l->rows, table->as<ulonglong2>(), cap - 1, match->as<uint64_t>(), in_tile->as<uint32_t>(), sweep.tiles, sweep.leave_at, words, too_long, pub);
+    const Publish pub = sweep.publish(words, 3);
+    join_probe_k<<<(unsigned)tiles, BLOCK, 0, c->stream>>>(probe, l->rows, slots, cap - 1, match->as<uint64_t>(), in_tile->as<uint32_t>(), sweep.tiles, sweep.leave_at, words, (unsigned int*)(words + 2), too_long, pub);
     check_launch(c, "hash_probe");
     sweep.finish();
-    unsigned long long w[2];
-    read_published(c, pub, words, 2, w);
+    unsigned long long w[3];
+    read_published(c, pub, words, 3, w);
     if (w[1]) return nullptr;
     std::unique_ptr<xlb_rel> o(new xlb_rel);
     o->ctx = c;
@@ -631,13 +730,27 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     add_columns(c, o.get(), cols, l, w[0]);
     add_columns(c, o.get(), cols, r, w[0]);
     if (w[0]) {
+        const OutputsBefore outputs{offs->as<uint64_t>(), in_tile->as<uint32_t>()};
+        const bool lists = w[0] > JOIN_CHAIN_OUTPUTS * n || w[2] > JOIN_CHAIN_ROWS, few = w[0] <= (uint64_t)c->sm_count * BLOCK * 4;
+        Buf rows;
+        if (lists) {
+            rows = make_buf(c, n * 8);
+            prof_begin(c, "group_start", cap * 16ull);
+            group_start_k<<<(unsigned)((cap + SCAN_TILE) / SCAN_TILE), BLOCK, 0, c->stream>>>(slots, cap + 1, rows->as<uint32_t>() + n, (unsigned int*)(words + 3));
+            check_launch(c, "group_start");
+            prof_begin(c, "group_fill", n * 16ull);
+            group_fill_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(place->as<uint2>(), n, slots, rows->as<uint32_t>());
+            check_launch(c, "group_fill");
+            prof_begin(c, "group_order", cap * 16ull);
+            group_order_k<<<grid_for(c, cap + 1), BLOCK, 0, c->stream>>>(slots, cap + 1, rows->as<uint32_t>());
+            check_launch(c, "group_order");
+        }
         prof_begin(c, "join_emit", 0);
-        const bool few = w[0] <= (uint64_t)c->sm_count * BLOCK * 4;
-        const uint64_t tile = few ? BLOCK : BLOCK * 4, blocks = (w[0] + tile - 1) / tile;
+        const uint64_t tile = !lists || few ? BLOCK : BLOCK * 4, blocks = ((lists ? w[0] : l->rows) + tile - 1) / tile;
         const Publish last = publish_by(c, blocks);
-        const OutputsBefore before{offs->as<uint64_t>(), in_tile->as<uint32_t>()};
-        if (few) join_emit_k<1><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), before, l->rows, w[0], rows->as<uint32_t>(), cols, last);
-        else join_emit_k<4><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), before, l->rows, w[0], rows->as<uint32_t>(), cols, last);
+        if (!lists) join_chains_k<<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), outputs, l->rows, before->as<uint32_t>(), cols, last);
+        else if (few) join_emit_k<1><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), outputs, l->rows, w[0], rows->as<uint32_t>(), rows->as<uint32_t>() + n, cols, last);
+        else join_emit_k<4><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), outputs, l->rows, w[0], rows->as<uint32_t>(), rows->as<uint32_t>() + n, cols, last);
         check_launch(c, "join_emit");
         status_published(c, last);
     }
