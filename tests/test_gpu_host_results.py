@@ -44,12 +44,12 @@ def test_results_are_independent_and_outlive_the_context():
         assert np.array_equal(h, w)
 
 
-def expect(p, cols):
-    for g, c in zip(p.download(p.create_buffer_from_slices(cols)), cols):
+def expect(p, rel, cols):
+    for g, c in zip(p.download(rel), cols):
         assert np.array_equal(g.view(np.uint8) if c.dtype == np.bool_ else g, c.view(np.uint8) if c.dtype == np.bool_ else c, equal_nan=c.dtype.kind == "f")
 
 
-# First columns of 6 MB and more go as runs where these are long: tiles are 4096 rows, a warp's 512, what a
+# First columns of sets, of 6 MB and more, go as runs where these are long: tiles are 4096 rows, a warp's 512, what a
 # thread fills 65536 (4 bytes) or 32768 (8 bytes) rows, and the staging holds 32766 or 16383 runs.
 @pytest.mark.parametrize("dtype", [np.uint32, np.int64, np.float32])
 @pytest.mark.parametrize("runs", ["one", "last", "edges", "even", "short", "limit", "over"])
@@ -71,13 +71,16 @@ def test_first_columns_of_long_runs(dtype, runs, n):
         starts = np.linspace(0, n - 1, count).astype(np.int64)
     starts = np.unique(np.array(list(starts)))
     rng = np.random.default_rng(n)
-    values = rng.standard_normal(len(starts)).astype(dtype) if dtype == np.float32 else rng.permutation(len(starts)).astype(dtype)
+    values = np.sort(rng.standard_normal(len(starts))).astype(dtype) if dtype == np.float32 else np.sort(rng.choice(1 << 30, len(starts), replace=False)).astype(dtype)
     if dtype == np.float32:
         values[-1] = np.nan
-    first = np.repeat(values, np.diff(np.append(starts, n)))
+    cols = [np.repeat(values, np.diff(np.append(starts, n))), np.arange(n, dtype=np.uint32), rng.integers(0, 2, n).astype(np.bool_)]
     p = KernelProvider(device=0)
-    expect(p, [first, rng.integers(0, 1 << 32, n, dtype=np.uint32)])
-    expect(p, [first, rng.integers(0, 2, n).astype(np.bool_), first[::-1].copy()])
+    for k in (2, 3):
+        rel = p.dedup(p.create_buffer_from_slices([c[::-1] for c in cols[:k]]))
+        assert rel.is_canonical()
+        expect(p, rel, cols[:k])
+        expect(p, p.create_buffer_from_slices(cols[:k]), cols[:k])
     p.close()
 
 
@@ -90,7 +93,8 @@ def test_long_runs_into_memory_of_the_callers(offset):
     total = 2200000
     first, second = np.repeat(np.arange(total // 1000, dtype=np.uint32), 1000), np.arange(total, dtype=np.uint32)
     p = KernelProvider(device=0)
-    buf = p.create_buffer_from_slices([first, second])
+    buf = p.dedup(p.create_buffer_from_slices([first, second]))
+    assert buf.is_canonical()
     for m in (total, total - 49999):  # all rows, and as many as the caller has room for
         if offset is None:
             out = [np.zeros(m, dtype=np.uint32) for _ in range(2)]

@@ -241,9 +241,10 @@ void fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n
 void ops_fetch_columns(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n) {
     ops_rel_columns(c, r);
     const uint32_t arity = r->schema.arity, width = type_width(r->schema.types[0]);
-    // Not with several ranks (whose waits watch the communicator), and not into memory that the driver copies to by
-    // itself: such a copy does not run beside anything.
-    if (arity >= 2 && width >= 4 && n * width >= RUNS_MIN_BYTES && n < 1ull << 32 && !c->wait_hook) {
+    // Only of a set, which is in order (in any other relation long runs are a piece of luck, and looking for them in a
+    // sort's result took 11 us of 1500); not with several ranks (whose waits watch the communicator), and not into memory
+    // that the driver copies to by itself: such a copy does not run beside anything.
+    if (r->canonical && arity >= 2 && width >= 4 && n * width >= RUNS_MIN_BYTES && n < 1ull << 32 && !c->wait_hook) {
         const unsigned cores = host_pool_cores();
         bool locked = cores >= RUNS_CORES_MIN;
         for (uint32_t i = 0; i < arity; ++i) locked = locked && page_locked(cols[i]) && (uintptr_t)cols[i] % width == 0;
