@@ -124,3 +124,38 @@ def test_joins_from_chains_and_from_lists(kind, sizes, probes):
         for g, w in zip(p.download(p.hash_join_v2(lb, rb, lk, rk, how)), left):
             assert np.array_equal(g, w[keep])
     p.close()
+
+
+# What one block takes: 4096 build rows, 8192 probe rows, four outputs a probe row and 1024 (2 keys: half of all pairs)
+@pytest.mark.parametrize("nl,nr,keys", [(8191, 4095, 3000), (8192, 4096, 3000), (8193, 4096, 3000), (8192, 4097, 3000), (1, 4096, 4096), (8192, 1, 2), (100, 12, 2), (100, 28, 2),
+                                        (1025, 64, 1), (1024, 65, 1)])
+def test_joins_of_one_block(p, nl, nr, keys):
+    rng = np.random.default_rng(nl * nr)
+    left = [rng.integers(0, keys, nl).astype(np.uint32), np.arange(nl, dtype=np.uint64)]
+    right = [np.arange(nr, dtype=np.float32), (rng.permutation(nr) % keys).astype(np.uint32)]
+    lb, rb = p.create_buffer_from_slices(left), p.create_buffer_from_slices(right)
+    l, r = inner(left[0], right[1])
+    for g, w in zip(p.download(p.hash_join_v2(lb, rb, [0], [1])), [c[l] for c in left] + [c[r] for c in right]):
+        assert np.array_equal(g, w)
+    has = np.isin(left[0], right[1])
+    for kind, keep in ((A.JOIN_SEMI, has), (A.JOIN_ANTI, ~has)):
+        for g, w in zip(p.download(p.hash_join_v2(lb, rb, [0], [1], kind)), left):
+            assert np.array_equal(g, w[keep])
+
+
+# ... and groups whose tables are at most 160 KB (2 tables of 8 bytes and the counts: 2^13 keys)
+@pytest.mark.parametrize("n", [1, 1023, 1025, 8192, 8193])
+@pytest.mark.parametrize("top", [0, 1, 1023, 8191, 8192, 1 << 31])
+@pytest.mark.parametrize("nk", [1, 2])
+def test_groups_of_one_block(p, n, top, nk):
+    rng = np.random.default_rng(n + top)
+    key = rng.integers(0, top, n, endpoint=True).astype(np.uint32)
+    key[0] = top
+    cols = [key, (key >> np.uint32(3)) % np.uint32(5)][:nk] + [rng.integers(0, 1 << 32, n, dtype=np.uint32), rng.integers(0, 1 << 40, n, dtype=np.uint64)]
+    got = p.download(p.groupby_multi_agg(p.create_buffer_from_slices(cols), list(range(nk)), [(nk, A.AGG_COUNT), (nk, A.AGG_SUM), (nk + 1, A.AGG_MIN)]))
+    order = np.lexsort(cols[:nk][::-1])
+    s = [c[order] for c in cols]
+    first = np.flatnonzero(np.concatenate([[True], np.any([k[1:] != k[:-1] for k in s[:nk]], axis=0)])) if n > 1 else np.array([0])
+    want = [k[first] for k in s[:nk]] + [np.diff(np.append(first, n)), np.add.reduceat(s[nk].astype(np.uint64), first), np.minimum.reduceat(s[nk + 1], first)]
+    for g, w in zip(got, want):
+        assert np.array_equal(g.astype(np.uint64), w.astype(np.uint64))

@@ -494,6 +494,180 @@ __global__ void __launch_bounds__(BLOCK) join_chains_k(const uint64_t* __restric
     publish_last(pub);
 }
 
+// ---- a few thousand rows: an operation by one block
+// What a small join or group-by cost was its launches (some 5 us each with the gap before it) and its read-backs (10 us)
+// and nothing of its sizes: 3001 facts through semi join, inner join and group-by took 17 launches and 6
+// read-backs, 164 us; one launch and one read-back each, 87.  Tables lie in shared memory; results go straight into
+// columns with room for the most there can be.  The block takes eight rows a thread: 8192 facts 109 us (by grids 190;
+// 12 000, with the smaller operations still by one block, 150 against 190, 20 000 177 against 203).
+constexpr unsigned SMALL_THREADS = 1024, SMALL_IPT = 8, SMALL_PROBE = SMALL_THREADS * SMALL_IPT, SMALL_BUILD = 4096;
+constexpr unsigned SMALL_SLOTS = 2 * SMALL_BUILD;  // (half of them stay free)
+constexpr uint64_t SMALL_OUTPUTS = 4 * SMALL_PROBE;  // of a join
+constexpr unsigned SMALL_GROUPS_BYTES = 160u << 10;
+__device__ __forceinline__ unsigned small_slots(uint64_t build) {
+    unsigned cap = 64;
+    while (cap < 2 * build) cap <<= 1;
+    return cap;
+}
+// Exclusive sums over the rows of a block that has SMALL_IPT rounds of them (row = round * SMALL_THREADS + thread);
+// warp_s: SMALL_IPT * 32 + 1 words.  `mine` becomes what comes before.
+__device__ __forceinline__ unsigned rounds_before(unsigned (&mine)[SMALL_IPT], unsigned* warp_s) {
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    unsigned len[SMALL_IPT];
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) {
+        len[r] = mine[r];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned v = __shfl_up_sync(FULL, mine[r], d);
+            if (lane >= (unsigned)d) mine[r] += v;
+        }
+        if (lane == 31) warp_s[r * 32 + warp] = mine[r];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        unsigned before = 0;
+        for (unsigned r = 0; r < SMALL_IPT; ++r) {
+            const unsigned v = warp_s[r * 32 + lane];
+            unsigned incl = v;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned x = __shfl_up_sync(FULL, incl, d);
+                if (lane >= (unsigned)d) incl += x;
+            }
+            warp_s[r * 32 + lane] = before + incl - v;
+            before += __shfl_sync(FULL, incl, 31);
+        }
+        if (lane == 0) warp_s[SMALL_IPT * 32] = before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) mine[r] = mine[r] - len[r] + warp_s[r * 32 + warp];
+    return warp_s[SMALL_IPT * 32];
+}
+__device__ __forceinline__ unsigned small_claim(unsigned long long* slots, unsigned mask, uint64_t key) {  // (a slot is free: twice as many as keys)
+    for (unsigned h = (unsigned)mix64(key) & mask;; h = (h + 1) & mask) {
+        const unsigned long long cur = atomicCAS(&slots[h], 0ull, (unsigned long long)key);
+        if (cur == 0 || cur == key) return h;
+    }
+}
+__global__ void __launch_bounds__(SMALL_THREADS, 1) exists_small_k(KeyCols keys, unsigned build, KeyCols probe, unsigned n, bool want, Cols cols, unsigned long long* total, const Publish pub) {
+    extern __shared__ unsigned long long small_s[];
+    __shared__ unsigned warp_s[SMALL_IPT * 32 + 1], zero_s;
+    const unsigned cap = small_slots(build), mask = cap - 1;
+    unsigned short* list = reinterpret_cast<unsigned short*>(small_s + cap);
+    uint64_t key[SMALL_IPT];
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) key[r] = r * SMALL_THREADS + threadIdx.x < n ? probe(r * SMALL_THREADS + threadIdx.x) : 0;
+    for (unsigned h = threadIdx.x; h < cap; h += SMALL_THREADS) small_s[h] = 0;
+    if (threadIdx.x == 0) zero_s = 0;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < build; i += SMALL_THREADS) {
+        const uint64_t k = keys(i);
+        if (k) small_claim(small_s, mask, k);
+        else zero_s = 1;
+    }
+    __syncthreads();
+    unsigned at[SMALL_IPT];
+    bool on[SMALL_IPT];
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) {
+        bool found = zero_s != 0;
+        if (key[r]) {
+            unsigned h = (unsigned)mix64(key[r]) & mask;
+            while (small_s[h] && small_s[h] != key[r]) h = (h + 1) & mask;
+            found = small_s[h] != 0;
+        }
+        on[r] = r * SMALL_THREADS + threadIdx.x < n && found == want;
+        at[r] = on[r];
+    }
+    const unsigned m = rounds_before(at, warp_s);
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r)
+        if (on[r]) list[at[r]] = (unsigned short)(r * SMALL_THREADS + threadIdx.x);
+    __syncthreads();
+    for (unsigned t = threadIdx.x; t < m; t += SMALL_THREADS) copy_row(cols, list[t], list[t], t);
+    if (threadIdx.x == 0) *total = m;
+    publish_now(pub);
+}
+// words: outputs, whether a group is too long.  More outputs than there is room for are only counted.
+__global__ void __launch_bounds__(SMALL_THREADS, 1) join_small_k(KeyCols keys, unsigned build, KeyCols probe, unsigned n, Cols cols, uint64_t room, unsigned long long* words, const Publish pub) {
+    extern __shared__ unsigned long long small_s[];
+    __shared__ unsigned warp_s[SMALL_IPT * 32 + 1], long_s;
+    const unsigned cap = small_slots(build), mask = cap - 1;
+    unsigned* entry = reinterpret_cast<unsigned*>(small_s + cap);  // rows | first row (plus one) << 16, of the key 0 behind the others
+    unsigned short* after = reinterpret_cast<unsigned short*>(entry + cap + 1);
+    uint64_t key[SMALL_IPT];
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) key[r] = r * SMALL_THREADS + threadIdx.x < n ? probe(r * SMALL_THREADS + threadIdx.x) : 0;
+    for (unsigned h = threadIdx.x; h <= cap; h += SMALL_THREADS) {
+        if (h < cap) small_s[h] = 0;
+        entry[h] = 0;
+    }
+    if (threadIdx.x == 0) long_s = 0;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < build; i += SMALL_THREADS) {
+        const uint64_t k = keys(i);
+        const unsigned h = k ? small_claim(small_s, mask, k) : cap;
+        unsigned cur = entry[h];
+        for (;;) {
+            if ((cur & 0xFFFF) >= JOIN_GROUP_MAX) {
+                long_s = 1;
+                break;
+            }
+            after[i] = (unsigned short)(cur >> 16);
+            const unsigned was = atomicCAS(&entry[h], cur, ((i + 1) << 16) | ((cur & 0xFFFF) + 1));
+            if (was == cur) break;
+            cur = was;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) words[1] = long_s;
+    if (long_s) {
+        publish_now(pub);
+        return;
+    }
+    for (unsigned h = threadIdx.x; h <= cap; h += SMALL_THREADS) {  // chains put in row order
+        const unsigned e = entry[h];
+        if ((e & 0xFFFF) < 2) continue;
+        unsigned sorted = 0;
+        for (unsigned x = e >> 16; x;) {
+            const unsigned next = after[x - 1];
+            if (!sorted || sorted > x) {
+                after[x - 1] = (unsigned short)sorted;
+                sorted = x;
+            } else {
+                unsigned p = sorted;
+                while (after[p - 1] && after[p - 1] < x) p = after[p - 1];
+                after[x - 1] = after[p - 1];
+                after[p - 1] = (unsigned short)x;
+            }
+            x = next;
+        }
+        entry[h] = (sorted << 16) | (e & 0xFFFF);
+    }
+    __syncthreads();
+    unsigned at[SMALL_IPT], first[SMALL_IPT];
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) {
+        unsigned e = 0;
+        if (key[r]) {
+            unsigned h = (unsigned)mix64(key[r]) & mask;
+            while (small_s[h] && small_s[h] != key[r]) h = (h + 1) & mask;
+            if (small_s[h]) e = entry[h];
+        } else if (r * SMALL_THREADS + threadIdx.x < n) e = entry[cap];
+        at[r] = e & 0xFFFF;
+        first[r] = e >> 16;
+    }
+    const unsigned m = rounds_before(at, warp_s);
+    if (m <= room)
+#pragma unroll
+        for (unsigned r = 0; r < SMALL_IPT; ++r)
+            for (unsigned x = first[r], to = at[r]; x; x = after[x - 1], ++to) copy_row(cols, r * SMALL_THREADS + threadIdx.x, x - 1, to);
+    if (threadIdx.x == 0) words[0] = m;
+    publish_now(pub);
+}
+
 // ---- group-by over a small domain of keys: tables indexed by the key itself
 // Rows per key (the tile's rows are combined in shared memory first: one hub key would serialise
 // the atomics), whose maximum tells whether the values may be added up by atomics as well.
@@ -607,6 +781,99 @@ __global__ void __launch_bounds__(BLOCK) group_emit_k(const unsigned int* __rest
     publish_last(pub);
 }
 
+// words: bound of the keys, groups.  All ones for the groups: the tables do not fit, nothing was done.
+__global__ void __launch_bounds__(SMALL_THREADS, 1) group_small_k(GroupKey key, unsigned n, Aggs a, int tables, int w0, void* key0, uint32_t* key1, unsigned long long* words, const Publish pub) {
+    extern __shared__ unsigned long long small_s[];
+    __shared__ unsigned long long bound_s;
+    __shared__ unsigned warp_s[33];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    uint64_t k[SMALL_IPT], all = 0;
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) {
+        k[r] = r * SMALL_THREADS + threadIdx.x < n ? key.cols(r * SMALL_THREADS + threadIdx.x) : 0;
+        all |= k[r];
+    }
+    if (threadIdx.x == 0) bound_s = 0;
+    __syncthreads();
+#pragma unroll
+    for (int d = 16; d; d >>= 1) all |= __shfl_xor_sync(FULL, all, d);
+    if (lane == 0 && all) atomicOr(&bound_s, (unsigned long long)all);
+    __syncthreads();
+    const unsigned long long bound = bound_s;
+    int bits = 64 - __clzll(bound);
+    if (key.cols.c1) {
+        key.lo_bits = max(64 - __clzll(bound & 0xFFFFFFFFull), 1);
+        bits = 64 - __clzll(bound >> 32) + key.lo_bits;
+    }
+    if (bits > 20 || ((8u * tables + 4u) << bits) > SMALL_GROUPS_BYTES) {
+        if (threadIdx.x == 0) {
+            words[0] = bound;
+            words[1] = ~0ull;
+        }
+        publish_now(pub);
+        return;
+    }
+    const unsigned domain = 1u << bits;
+    unsigned* count = reinterpret_cast<unsigned*>(small_s + (size_t)tables * domain);
+    int t = 0;
+    for (int q = 0; q < a.n; ++q) {
+        if (a.op[q] == XLB_AGG_COUNT) continue;
+        for (unsigned x = threadIdx.x; x < domain; x += SMALL_THREADS) small_s[t * domain + x] = a.op[q] == XLB_AGG_MIN ? ~0ull : 0ull;
+        ++t;
+    }
+    for (unsigned x = threadIdx.x; x < domain; x += SMALL_THREADS) count[x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (unsigned r = 0; r < SMALL_IPT; ++r) {
+        const unsigned i = r * SMALL_THREADS + threadIdx.x;
+        if (i >= n) break;
+        const unsigned x = key.cols.c1 ? (unsigned)(((k[r] >> 32) << key.lo_bits) | (k[r] & 0xFFFFFFFFull)) : (unsigned)k[r];
+        atomicAdd(&count[x], 1u);
+        t = 0;
+        for (int q = 0; q < a.n; ++q) {
+            if (a.op[q] == XLB_AGG_COUNT) continue;
+            unsigned long long* to = &small_s[t++ * domain + x];
+            const unsigned long long v = a.width[q] == 4 ? __ldg((const uint32_t*)a.val[q] + i) : __ldg((const unsigned long long*)a.val[q] + i);
+            if (a.op[q] == XLB_AGG_SUM) atomicAdd(to, v);
+            else if (a.op[q] == XLB_AGG_MIN) atomicMin(to, v);
+            else atomicMax(to, v);
+        }
+    }
+    __syncthreads();
+    unsigned groups = 0;
+    for (unsigned x0 = 0; x0 < domain; x0 += SMALL_THREADS) {  // in the order of the keys
+        const unsigned x = x0 + threadIdx.x, c = x < domain ? count[x] : 0u, some = __ballot_sync(FULL, c != 0);
+        if (lane == 0) warp_s[warp] = __popc(some);
+        __syncthreads();
+        unsigned before = 0, total = 0;
+        for (unsigned w = 0; w < SMALL_THREADS / 32; ++w) {
+            if (w < warp) before += warp_s[w];
+            total += warp_s[w];
+        }
+        if (c) {
+            const unsigned pos = groups + before + __popc(some & lanemask_lt());
+            if (key1) {
+                ((uint32_t*)key0)[pos] = x >> key.lo_bits;
+                key1[pos] = x & ((1u << key.lo_bits) - 1);
+            } else if (w0 == 4) ((uint32_t*)key0)[pos] = x;
+            else ((unsigned long long*)key0)[pos] = x;
+            t = 0;
+            for (int q = 0; q < a.n; ++q) {
+                const unsigned long long v = a.op[q] == XLB_AGG_COUNT ? c : small_s[t++ * domain + x];
+                if (a.out_width[q] == 4) ((uint32_t*)a.out[q])[pos] = (uint32_t)v;
+                else ((unsigned long long*)a.out[q])[pos] = v;
+            }
+        }
+        groups += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        words[0] = bound;
+        words[1] = groups;
+    }
+    publish_now(pub);
+}
+
 KeyCols key_cols(const xlb_rel* r, const uint32_t* keys, uint32_t nk) {
     KeyCols k{r->cols[keys[0]]->p, nullptr, (int)type_width(r->schema.types[keys[0]])};
     if (nk == 2) k.c1 = r->cols[keys[1]]->as<uint32_t>();
@@ -650,8 +917,42 @@ struct Sweep {
 
 }  // namespace
 
+// Whether one block takes it; the shared memory its kernels may ask for.
+static bool one_block(xlb_ctx* c, uint64_t build, uint64_t probe) {
+    if (!build || build > SMALL_BUILD || !probe || probe > SMALL_PROBE) return false;
+    if (!c->query_attr_set) {
+        CUDA_OK(cudaFuncSetAttribute(exists_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMALL_SLOTS * 8 + SMALL_PROBE * 2)));
+        CUDA_OK(cudaFuncSetAttribute(join_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMALL_SLOTS * 12 + 16 + SMALL_BUILD * 2)));
+        CUDA_OK(cudaFuncSetAttribute(group_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_GROUPS_BYTES));
+        c->query_attr_set = true;
+    }
+    return true;
+}
+static unsigned slots_of(uint64_t build) {
+    unsigned cap = 64;
+    while (cap < 2 * build) cap <<= 1;
+    return cap;
+}
+
 xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, bool want) {
     if (r->rows >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)r->rows);
+    if (one_block(c, r->rows, l->rows)) {
+        std::unique_ptr<xlb_rel> o(new xlb_rel);
+        o->ctx = c;
+        o->schema = l->schema;
+        Cols cols{};
+        add_columns(c, o.get(), cols, l, l->rows);
+        Buf total = make_buf(c, 8);
+        prof_begin(c, "exists_small", 0);
+        const Publish pub = publish_by(c, 1, total->p, 1);
+        exists_small_k<<<1, SMALL_THREADS, slots_of(r->rows) * 8 + SMALL_PROBE * 2, c->stream>>>(key_cols(r, rk, nk), (unsigned)r->rows, key_cols(l, lk, nk), (unsigned)l->rows, want, cols,
+                                                                                              total->as<unsigned long long>(), pub);
+        check_launch(c, "exists_small");
+        unsigned long long m;
+        read_published(c, pub, total->p, 1, &m);
+        o->rows = m;
+        return o.release();
+    }
     uint64_t cap = 1024;
     while (cap < 2 * r->rows) cap <<= 1;
     const uint64_t n = l->rows, tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
@@ -693,6 +994,34 @@ xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint
 xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, const xlb_schema& os) {
     const uint64_t n = r->rows;
     if (n >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)n);
+    if (one_block(c, n, l->rows)) {
+        uint64_t row_bytes = 0;
+        for (uint32_t i = 0; i < os.arity; ++i) row_bytes += type_width(os.types[i]);
+        const uint64_t room = std::min<uint64_t>(SMALL_OUTPUTS, 4 * l->rows + 1024);
+        if (!c->budget || c->allocated + room * row_bytes + (1u << 16) <= c->budget) {
+            std::unique_ptr<xlb_rel> o(new xlb_rel);
+            o->ctx = c;
+            o->schema = os;
+            Cols cols{};
+            cols.left = (int)l->schema.arity;
+            add_columns(c, o.get(), cols, l, room);
+            add_columns(c, o.get(), cols, r, room);
+            Buf words = make_buf(c, 16);
+            prof_begin(c, "join_small", 0);
+            const Publish pub = publish_by(c, 1, words->p, 2);
+            const unsigned cap = slots_of(n);
+            join_small_k<<<1, SMALL_THREADS, cap * 12 + 16 + (unsigned)n * 2, c->stream>>>(key_cols(r, rk, nk), (unsigned)n, key_cols(l, lk, nk), (unsigned)l->rows, cols, room,
+                                                                                         words->as<unsigned long long>(), pub);
+            check_launch(c, "join_small");
+            unsigned long long w[2];
+            read_published(c, pub, words->p, 2, w);
+            if (w[1]) return nullptr;
+            if (w[0] <= room) {
+                o->rows = w[0];
+                return o.release();
+            }
+        }
+    }
     uint64_t cap = 1024;
     while (cap < 2 * n) cap <<= 1;
     const KeyCols build = key_cols(r, rk, nk), probe = key_cols(l, lk, nk);
@@ -768,15 +1097,48 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
     if (nk > 2 || (nk == 2 && (type_width(in->schema.types[key_cols_in[0]]) != 4 || type_width(in->schema.types[key_cols_in[1]]) != 4))) return nullptr;
     const uint64_t n = in->rows;
     GroupKey key{key_cols(in, key_cols_in, nk), 0};
+    uint32_t tables = 0;
+    for (uint32_t a = 0; a < na; ++a) tables += agg_ops[a] != XLB_AGG_COUNT;
+    std::unique_ptr<xlb_rel> o(new xlb_rel);
+    o->ctx = c;
+    o->schema = os;
+    Aggs ag{};
+    ag.n = (int)na;
+    const auto results = [&](uint64_t rows) {
+        for (uint32_t i = 0; i < os.arity; ++i) o->cols[i] = make_buf(c, rows * type_width(os.types[i]));
+        for (uint32_t a = 0; a < na; ++a) {
+            ag.val[a] = in->cols[agg_cols[a]]->p;
+            ag.op[a] = (uint8_t)agg_ops[a];
+            ag.width[a] = (uint8_t)type_width(in->schema.types[agg_cols[a]]);
+            ag.out[a] = o->cols[nk + a]->p;
+            ag.out_width[a] = (uint8_t)type_width(os.types[nk + a]);
+        }
+    };
     Buf words = make_buf(c, 24);  // [0] key bound, [1] groups, [2] rows of the largest
-    CUDA_OK(set_async(c, words->p, 0, 24));
-    prof_begin(c, "group_bound", 0);
-    const unsigned bound_grid = std::min(grid_for(c, n, BLOCK * 4), PUBLISH_BLOCKS_MAX);
-    const Publish bound_pub = publish_by(c, bound_grid, words->p, 1);
-    group_bound_k<<<bound_grid, BLOCK, 0, c->stream>>>(key.cols, n, words->as<unsigned long long>(), bound_pub);
-    check_launch(c, "group_bound");
     unsigned long long w[2];
-    read_published(c, bound_pub, words->p, 1, w);
+    const bool small = one_block(c, 1, n);
+    if (small) {
+        results(n);
+        prof_begin(c, "group_small", 0);
+        const Publish pub = publish_by(c, 1, words->p, 2);
+        group_small_k<<<1, SMALL_THREADS, SMALL_GROUPS_BYTES, c->stream>>>(key, (unsigned)n, ag, (int)tables, (int)type_width(os.types[0]), o->cols[0]->p, nk == 2 ? o->cols[1]->as<uint32_t>() : nullptr,
+                                                                         words->as<unsigned long long>(), pub);
+        check_launch(c, "group_small");
+        read_published(c, pub, words->p, 2, w);
+        if (w[1] != ~0ull) {
+            o->rows = w[1];
+            return o.release();
+        }
+    }
+    CUDA_OK(set_async(c, words->p, 0, 24));
+    if (!small) {
+        prof_begin(c, "group_bound", 0);
+        const unsigned bound_grid = std::min(grid_for(c, n, BLOCK * 4), PUBLISH_BLOCKS_MAX);
+        const Publish bound_pub = publish_by(c, bound_grid, words->p, 1);
+        group_bound_k<<<bound_grid, BLOCK, 0, c->stream>>>(key.cols, n, words->as<unsigned long long>(), bound_pub);
+        check_launch(c, "group_bound");
+        read_published(c, bound_pub, words->p, 1, w);
+    }
     int bits = bit_length(w[0]);
     if (nk == 2) {
         key.lo_bits = std::max(bit_length(w[0] & 0xFFFFFFFFull), 1);
@@ -798,18 +1160,11 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
     sweep.finish();
     read_published(c, pub, words->as<uint64_t>() + 1, 2, w);
     const uint64_t m = w[0];
-    uint32_t tables = 0;
-    for (uint32_t a = 0; a < na; ++a) tables += agg_ops[a] != XLB_AGG_COUNT;
     if (tables && w[1] > GROUP_ROWS_MAX) return nullptr;
-    std::unique_ptr<xlb_rel> o(new xlb_rel);
-    o->ctx = c;
-    o->schema = os;
     o->rows = m;
-    for (uint32_t i = 0; i < os.arity; ++i) o->cols[i] = make_buf(c, m * type_width(os.types[i]));
+    results(m);
     // sums and maxima start from zero, minima from all ones: two fills
     Buf acc = make_buf(c, std::max<uint64_t>(tables * domain * 8, 8));
-    Aggs ag{};
-    ag.n = (int)na;
     uint64_t at = 0, minima = 0;
     for (int pass = 0; pass < 2; ++pass) {
         for (uint32_t a = 0; a < na; ++a) {
@@ -821,13 +1176,6 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
     }
     if (minima) CUDA_OK(set_async(c, acc->p, 0, minima * 8));
     if (at > minima) CUDA_OK(set_async(c, acc->as<uint64_t>() + minima, 0xFF, (at - minima) * 8));
-    for (uint32_t a = 0; a < na; ++a) {
-        ag.val[a] = in->cols[agg_cols[a]]->p;
-        ag.op[a] = (uint8_t)agg_ops[a];
-        ag.width[a] = (uint8_t)type_width(in->schema.types[agg_cols[a]]);
-        ag.out[a] = o->cols[nk + a]->p;
-        ag.out_width[a] = (uint8_t)type_width(os.types[nk + a]);
-    }
     if (tables) {
         prof_begin(c, "groupby_reduce", 0);
         group_add_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(key, n, ag);
