@@ -219,6 +219,46 @@ def test_points_to(scale, monkeypatch):
         assert np.array_equal(g, w)
 
 
+def by_rows(kinds):
+    """p(X,Y) :- s(X,Y), then one rule per kind, each with the stored relation's columns either way round."""
+    ids = {"s": 0, "e": 1, "f": 2, "p": 3}
+    join = lambda l, r, a, b: Join(l, r, [a], [b])  # noqa: E731
+    rules = {
+        "copy": Project(join(Scan(1), Scan(3), 0, 0), [1, 3]),                          # p(X,Y) :- e(P,X), p(P,Y)
+        "copy2": Project(join(Scan(2), Scan(3), 1, 0), [0, 3]),                         # p(X,Y) :- f(X,P), p(P,Y)
+        "step": Project(join(Scan(3), Scan(3), 1, 0), [0, 3]),                          # p(P,Y) :- p(P,Q), p(Q,Y)
+        "steps": Project(join(join(Scan(1), Scan(3), 0, 0), Scan(3), 3, 0), [1, 5]),    # p(X,Y) :- e(P,X), p(P,Q), p(Q,Y)
+        "steps2": Project(join(join(Scan(2), Scan(3), 1, 0), Scan(3), 3, 0), [0, 5]),   # p(X,Y) :- f(X,P), p(P,Q), p(Q,Y)
+        "across": Project(join(join(Scan(1), Scan(3), 0, 0), Scan(3), 1, 0), [3, 5]),   # p(Q,Y) :- e(P,W), p(P,Q), p(W,Y)
+        "across2": Project(join(join(Scan(2), Scan(3), 1, 0), Scan(3), 0, 0), [3, 5]),  # p(Q,Y) :- f(W,P), p(P,Q), p(W,Y)
+    }
+    return ExecutionPlan([Scc(0, True, [CompiledRule("p", Scan(0), U2)] + [CompiledRule("p", rules[k], U2) for k in kinds])], ids)
+
+
+# values of 6 bits (a row of two words) to 13, and of 14, which are too many
+@pytest.mark.parametrize("kinds", [("steps",), ("across",), ("copy", "steps"), ("copy2", "steps2", "across2"), ("copy", "steps", "across", "step")], ids="-".join)
+@pytest.mark.parametrize("top,rows", [(3, 4), (63, 60), (64, 90), (700, 500), (2047, 900), (8191, 2500), (8192, 2500)])
+def test_rules_by_rows(kinds, top, rows, monkeypatch):
+    rng = np.random.default_rng(top)
+    pairs = lambda n: [rng.integers(0, top, n, endpoint=True).astype(np.uint32) for _ in range(2)]  # noqa: E731
+    rels = {"s": pairs(rows), "e": pairs(rows // 3 + 1), "f": pairs(rows // 3 + 1)}
+    rels["s"][0][0] = top
+    got, it, _ = both(by_rows(kinds), rels, "p", monkeypatch)
+    if top <= 700:
+        want, _ = O.run_program(by_rows(kinds), rels, ["p"])
+        for g, w in zip(got, want["p"]):
+            assert np.array_equal(g, w)
+    if it > 1:
+        for limit, fits in ((it, True), (it - 1, False)):
+            p = KernelProvider(device=0, max_iterations=limit)
+            try:
+                run_program(p, by_rows(kinds), rels, ["p"])
+                assert fits
+            except XlbError as e:
+                assert not fits and e.status == A.ERR_ITER_LIMIT
+            p.close()
+
+
 def test_transposed_partner_and_composed_relation(monkeypatch):
     # p(X,Z) :- p(X,Y), p(Z,Y), g(X,Z)-free: the partner by its second column; q-shaped: p(Z,Y) :- g(Z,X), p(X,W), p(W,Y)
     ids = {"e": 0, "g": 1, "p": 2}

@@ -351,6 +351,7 @@ struct xlb_ctx {
     unsigned delta_spin_limit = 1u << 26;  // polls (tens of seconds) for which a block of the delta loop waits without seeing anything go on
     bool frontier_attr_set = false, frontier_many_attr_set = false, frontier_large_attr_set = false;  // the same for the frontier kernels
     bool index_attr_set = false;  // the same for direct_small_k
+    bool delta_wide_attr_set = false;  // the same for the kernel by rows of the head
     bool query_attr_set = false;  // the same for the one-block joins and group-bys
     bool delta_attr_set = false;  // the same for the delta loop's kernel
     bool sort_attr_set = false;  // the scatter kernels' shared-memory opt-in was made on this context's device

@@ -1758,6 +1758,325 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const Out o, const
         ctl->rows_left = st.fix ? 0 : 1;
     }
 }
+// ---- two recursive atoms, by rows of the head
+// The rules of DeltaRows give whole rows of bits to rows of the head, so an iteration is unions of rows: for a value P
+// that a rule has a list for, the rows Q that its row names (of the head where (P, Q) is in the delta, of the
+// delta where it is in the head) are ORed in registers, warp by warp, then in shared memory, and the union goes
+// to the rows it belongs to as far as these gain by it.  (Tuple by tuple, each against bit rows of the head, its
+// transpose and its composites, as delta_loop_k does, a tuple cost an atomic a candidate word, one on the transpose and its
+// place in the log, and few warps had most of them: points-to over 1500 values 395 us, here 190.)  An iteration has two
+// phases: the rows' own warps add what was derived to the head, which makes the delta; then groups of eight warps
+// take the values of all rules in turn, up to four groups a value where there are few of them.  What bounds it is the chain of
+// loads a value costs, some 6 K cycles, and two barriers an iteration.
+//   Against the loop: points-to programs of 150, 600, 1500, 3000 and 6000 values 248, 534, 623, 1242 and 4016 us by the loop, 204,
+// 267, 305, 581 and 1692 by rows, as their relations are skewed.  Over uniform ones the two are close: 2048 values
+// with 300 stored rows a relation 270 and 289, with 2000 787 and 723; 8192 values with 800 346 and 432, with 8000
+// 10.0 and 13.3 ms, with 16 000 43 and 24 ms.  (A warp a value for rows of few tuples, before the groups, did
+// better on sparse relations and took points-to 242.)  h(P, Y) :- h(P, Q), h(Q, Y) stays with the loop: every row is a value
+// then, and on a sparse graph of 8000 nodes rows took 1320 us and the loop 284 (dense, 2000 nodes: 713 and 966).
+constexpr int WD_BITS_MIN = 6, WD_BITS_MAX = 13;
+constexpr unsigned WD_WARPS = 8, WD_THREADS = WD_WARPS * 32, WD_GROUPS = DL_THREADS / WD_THREADS;
+constexpr unsigned WD_SPLIT = 4;  // groups that share a value, at most
+constexpr unsigned WD_FEW = 64;   // tuples of a row up to which it is not
+struct WideRule {
+    Ix ix;
+    int kind;
+};
+struct WideRules {
+    WideRule r[DELTA_ROWS_MAX];
+    int n;
+};
+struct Wide {
+    unsigned *delta, *reached, *stamp;  // bitmaps like the head's; rows that were reached
+    unsigned *n_delta, *n_head;         // tuples of each row
+    unsigned* active[2];                // rows of the delta that hold any, as bits: this iteration's, the next one's
+    unsigned* keys;                     // per rule, the values it has something to do for ...
+    unsigned* n_keys;                   // ... and how many
+    unsigned rows, words;
+};
+// four rows, a list of twice a row's values, counters, items
+__host__ __device__ constexpr size_t wide_group_bytes(unsigned words) { return words * 16 + words * 128 + 16 + WD_THREADS * 4; }
+struct WideGroup {
+    unsigned *led[2], *row_d, *row_h, *count, *items;
+    unsigned short* list;
+    unsigned id, warp, thread;
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(WD_THREADS) : "memory"); }
+};
+// What `led` brings row `to` beyond the head, for up to four rows a warp at a time (entries first, first + step, ... of n).
+template <class Row, class From>
+__device__ __forceinline__ void give(const Out& o, const Wide& b, unsigned first, unsigned step, unsigned n, Row row, From from) {
+    const unsigned W = b.words, lane = lane_id();
+    constexpr int N = 4;
+    for (unsigned e0 = first; e0 < n; e0 += N * step) {
+        unsigned to[N];
+        const unsigned* led[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const bool on = e0 + u * step < n;
+            to[u] = on ? row(e0 + u * step) : ~0u;
+            led[u] = on ? from(e0 + u * step) : nullptr;
+            if (on && to[u] >= b.rows) {
+                if (lane == 0) set_status(o.st, XLB_ERR_CAPACITY, 24, to[u]);
+                to[u] = ~0u;
+            }
+        }
+        for (unsigned w = 2 * lane; w < W; w += 64) {
+            unsigned long long gain[N];
+#pragma unroll
+            for (int u = 0; u < N; ++u) {
+                gain[u] = to[u] != ~0u ? *reinterpret_cast<const unsigned long long*>(led[u] + w) : 0ull;
+                if (gain[u]) gain[u] &= ~__ldcg(reinterpret_cast<const unsigned long long*>(o.visited + (uint64_t)to[u] * W + w));
+            }
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+                if (gain[u]) gain[u] &= ~__ldcg(reinterpret_cast<const unsigned long long*>(b.reached + (uint64_t)to[u] * W + w));  // (found a moment ago)
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+                if (gain[u]) {
+                    atomicOr(reinterpret_cast<unsigned long long*>(b.reached + (uint64_t)to[u] * W + w), gain[u]);
+                    b.stamp[to[u]] = 1;
+                }
+        }
+    }
+}
+// The union of rows: entries of the group's list, a row number and the matrix (bit 15: the delta) each, into led[0].
+__device__ __forceinline__ void unite(const Out& o, const Wide& b, const WideGroup& g, unsigned n) {
+    const unsigned W = b.words, lane = lane_id();
+    constexpr int N = 8;
+    for (unsigned w = 2 * lane; w - 2 * lane < W; w += 64) {
+        unsigned long long acc = 0;
+        for (unsigned e0 = g.warp; e0 < n; e0 += N * WD_WARPS) {
+            unsigned long long v[N];
+#pragma unroll
+            for (int u = 0; u < N; ++u) {
+                const unsigned e = e0 + u * WD_WARPS < n ? g.list[e0 + u * WD_WARPS] : ~0u;
+                const unsigned* m = e & 0x8000u ? b.delta : o.visited;
+                v[u] = e != ~0u && w < W ? __ldcg(reinterpret_cast<const unsigned long long*>(m + (uint64_t)(e & 0x7FFF) * W + w)) : 0ull;
+            }
+#pragma unroll
+            for (int u = 0; u < N; ++u) acc |= v[u];
+        }
+        if (acc) atomicOr(reinterpret_cast<unsigned long long*>(g.led[0] + w), acc);
+    }
+}
+__global__ void __launch_bounds__(DL_THREADS, 1) delta_wide_k(const Out o, const __grid_constant__ WideRules rules, const Wide b, uint64_t max_iterations) {
+    extern __shared__ __align__(16) unsigned char wd_smem[];
+    __shared__ BitsState st;
+    __shared__ unsigned long long sum_s[2];
+    __shared__ unsigned n_keys_s[DELTA_ROWS_MAX];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5, W = b.words;
+    WideGroup g;
+    g.id = warp / WD_WARPS;
+    g.warp = warp % WD_WARPS;
+    g.thread = threadIdx.x % WD_THREADS;
+    unsigned* base = reinterpret_cast<unsigned*>(wd_smem + g.id * wide_group_bytes(W));
+    g.led[0] = base;
+    g.led[1] = base + W;
+    g.row_d = base + 2 * W;
+    g.row_h = base + 3 * W;
+    g.list = reinterpret_cast<unsigned short*>(base + 4 * W);
+    g.count = base + 4 * W + 32 * W;
+    g.items = g.count + 4;
+    Ctl* ctl = o.ctl;
+    if (threadIdx.x == 0) st = BitsState{};
+    // the values each rule has something to do for
+    for (int q = blockIdx.x; q < rules.n; q += gridDim.x)
+        for (unsigned v = threadIdx.x; v < b.rows; v += DL_THREADS) {
+            uint32_t s, len;
+            find(rules.r[q].ix, v, s, len);
+            if (len) b.keys[q * b.rows + atomicAdd(&b.n_keys[q], 1u)] = v;
+        }
+    unsigned passed = 0;
+    const auto meet = [&]() {  // (thread 0)
+        passed += gridDim.x;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->arrived) : "memory");
+        st.go = wait_for(o, &ctl->arrived, passed, 0, passed);
+    };
+    for (unsigned phase = 0;; ++phase) {
+        __syncthreads();
+        if (threadIdx.x < 2) sum_s[threadIdx.x] = 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->slot[st.slot == 2 ? 0 : st.slot + 1] = Slot{};
+        __syncthreads();
+        Slot* slot = &ctl->slot[st.slot];
+        // what was derived joins the head (at first: the seeds are in it)
+        for (unsigned row = warp * gridDim.x + blockIdx.x; row < b.rows; row += gridDim.x * DL_WARPS) {
+            const unsigned held = __ldcg(&b.n_delta[row]), reached = phase ? __ldcg(&b.stamp[row]) : 1u;
+            if (!held && !reached) continue;
+            unsigned mine = 0;
+            for (unsigned w = 2 * lane; w < W; w += 64) {
+                const uint64_t at = (uint64_t)row * W + w;
+                unsigned long long d = 0;
+                if (reached) {
+                    const unsigned long long have = __ldcg(reinterpret_cast<const unsigned long long*>(o.visited + at));
+                    d = have;
+                    if (phase) {
+                        const unsigned long long r = __ldcg(reinterpret_cast<const unsigned long long*>(b.reached + at));
+                        d = r & ~have;
+                        if (r) *reinterpret_cast<unsigned long long*>(b.reached + at) = 0;
+                        if (d) *reinterpret_cast<unsigned long long*>(o.visited + at) = have | d;
+                    }
+                }
+                *reinterpret_cast<unsigned long long*>(b.delta + at) = d;
+                mine += __popcll(d);
+            }
+            const unsigned all = __reduce_add_sync(FULL, mine);
+            if (lane == 0) {
+                if (reached) b.stamp[row] = 0;
+                b.n_delta[row] = all;
+                if (all) {
+                    b.n_head[row] += all;
+                    atomicOr(&b.active[phase & 1][row >> 5], 1u << (row & 31));
+                    atomicAdd(&sum_s[0], (unsigned long long)all);
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (sum_s[0]) atomicAdd(&slot->count, sum_s[0]);
+            meet();
+            const unsigned long long found = __ldcg(&slot->count);
+            st.tuples += found;
+            st.cands += st.pending;  // of the joins that found them
+            st.iterations = phase;
+            st.fix = found == 0;
+            st.over = st.fix || phase >= max_iterations;
+        }
+        __syncthreads();
+        if (!st.go) return;
+        if (st.over) break;
+        if (phase == 0 && threadIdx.x < (unsigned)rules.n) n_keys_s[threadIdx.x] = __ldcg(&b.n_keys[threadIdx.x]);
+        for (unsigned w = blockIdx.x * DL_THREADS + threadIdx.x; w < (b.rows + 31) / 32; w += gridDim.x * DL_THREADS) b.active[(phase & 1) ^ 1][w] = 0;  // (read by nobody now)
+        __syncthreads();
+        const unsigned* active = b.active[phase & 1];
+        unsigned long long cand = 0;
+        const unsigned groups = gridDim.x * WD_GROUPS;
+        unsigned turns = 0;
+        unsigned first = g.id * gridDim.x + blockIdx.x;  // (items are numbered through all rules)
+        for (int q = 0; q < rules.n; ++q) {
+            const WideRule& ru = rules.r[q];
+            unsigned split = ru.kind == DeltaRows::COPY ? 1 : WD_SPLIT;  // (fewer where there are enough values to go round)
+            while (split > 1 && 2 * n_keys_s[q] * split > 3 * groups) split /= 2;
+            const unsigned items = n_keys_s[q] * split;
+            const unsigned all = items > first ? (items - first + groups - 1) / groups : 0;
+            const bool direct = all <= 2;  // (else they are first looked at side by side: what has nothing to do costs no turn)
+            unsigned done = 0, left = direct ? all : 0;
+            while (left || (!direct && done < all)) {
+                if (!left) {
+                    g.sync();
+                    if (g.thread == 0) g.count[2] = 0;
+                    g.sync();
+                    if (done + g.thread < all) {
+                        const unsigned i = first + (done + g.thread) * groups, key = __ldcg(&b.keys[q * b.rows + i / split]), nd = __ldcg(&b.n_delta[key]), nh = __ldcg(&b.n_head[key]);
+                        if ((nd || (nh && ru.kind != DeltaRows::COPY)) && (nh > WD_FEW || i % split == 0)) g.items[atomicAdd(&g.count[2], 1u)] = i;
+                    }
+                    g.sync();
+                    left = g.count[2];
+                    done += WD_THREADS;
+                    continue;
+                }
+                --left;
+                const unsigned item = direct ? first + left * groups : g.items[left];
+                if (++turns % 64 == 0 && g.thread == 0) beat(o);
+                const unsigned key = __ldcg(&b.keys[q * b.rows + item / split]), part = item % split;
+                const unsigned nd = __ldcg(&b.n_delta[key]), nh = __ldcg(&b.n_head[key]);
+                if (!nh || (ru.kind == DeltaRows::COPY && !nd) || (part && nh <= WD_FEW)) continue;
+                uint32_t s, len;
+                find(ru.ix, key, s, len);
+                const unsigned mask = split == 1 || nh <= WD_FEW ? ~0u : (split == 4 ? 0x11111111u : 0x55555555u) << part;  // the values of the row that are this group's
+                g.sync();  // (the one before is done with the rows and the list)
+                if (g.thread == 0) g.count[0] = g.count[1] = 0;
+                for (unsigned w = g.thread; w < W; w += WD_THREADS) {
+                    g.led[0][w] = g.led[1][w] = 0;
+                    g.row_d[w] = nd ? __ldcg(&b.delta[(uint64_t)key * W + w]) : 0u;
+                    g.row_h[w] = ru.kind != DeltaRows::COPY ? __ldcg(&o.visited[(uint64_t)key * W + w]) : 0u;
+                }
+                g.sync();
+                if (ru.kind == DeltaRows::COPY) {
+                    if (g.thread == 0) cand += (unsigned long long)nd * len;
+                    give(o, b, g.warp, WD_WARPS, len, [&](unsigned e) { return other_of(ru.ix, s + e); }, [&](unsigned) { return (const unsigned*)g.row_d; });
+                    continue;
+                }
+                if (ru.kind == DeltaRows::ACROSS) {
+                    // rows listed for the value: of the head into one union, of the delta into the other
+                    unsigned long long all = 0, fresh = 0;
+                    for (unsigned w0 = 0; w0 < W; w0 += 64) {
+                        const unsigned w = w0 + 2 * lane;
+                        unsigned long long x = 0, y = 0;
+                        for (uint32_t j = g.warp; j < len; j += WD_WARPS) {
+                            const uint32_t m = other_of(ru.ix, s + j);
+                            if (m >= b.rows) continue;  // (no row: never derived)
+                            const unsigned mh = __ldcg(&b.n_head[m]), md = __ldcg(&b.n_delta[m]);
+                            if (w0 == 0) {
+                                all += mh;
+                                fresh += md;
+                            }
+                            if (w < W && nd && mh) x |= __ldcg(reinterpret_cast<const unsigned long long*>(o.visited + (uint64_t)m * W + w));
+                            if (w < W && md) y |= __ldcg(reinterpret_cast<const unsigned long long*>(b.delta + (uint64_t)m * W + w));
+                        }
+                        if (x) atomicOr(reinterpret_cast<unsigned long long*>(g.led[0] + w), x);
+                        if (y) atomicOr(reinterpret_cast<unsigned long long*>(g.led[1] + w), y);
+                    }
+                    if (lane == 0 && part == 0) cand += nd * all + nh * fresh;
+                    if (lane == 0 && fresh) g.count[1] = 1;
+                    g.sync();
+                    const bool any_fresh = g.count[1] != 0;
+                    for (unsigned w = g.thread; w < W; w += WD_THREADS) {  // the row's values: those of the delta get the one, the others the other
+                        const unsigned d = g.row_d[w] & mask, h = any_fresh ? g.row_h[w] & ~g.row_d[w] & mask : 0u;
+                        unsigned at = d | h ? atomicAdd(&g.count[0], (unsigned)(__popc(d) + __popc(h))) : 0u;
+                        for (unsigned x = d; x; x &= x - 1) g.list[at++] = (unsigned short)(w * 32 + __ffs(x) - 1);
+                        for (unsigned x = h; x; x &= x - 1) g.list[at++] = (unsigned short)((w * 32 + __ffs(x) - 1) | 0x8000u);
+                    }
+                    g.sync();
+                    give(o, b, g.warp, WD_WARPS, g.count[0], [&](unsigned e) { return (unsigned)(g.list[e] & 0x7FFF); }, [&](unsigned e) { return (const unsigned*)g.led[g.list[e] >> 15]; });
+                    continue;
+                }
+                // STEPS: rows of the head for values of the delta, rows of the delta for values of the head
+                unsigned long long c = 0;
+                for (unsigned w = g.thread; w < W; w += WD_THREADS) {
+                    const unsigned d = g.row_d[w] & mask, h = g.row_h[w] & __ldcg(&active[w]) & mask;
+                    unsigned at = d | h ? atomicAdd(&g.count[0], (unsigned)(__popc(d) + __popc(h))) : 0u;
+                    for (unsigned x = d; x; x &= x - 1) {
+                        const unsigned v = w * 32 + __ffs(x) - 1;
+                        c += __ldcg(&b.n_head[v]);
+                        g.list[at++] = (unsigned short)v;
+                    }
+                    for (unsigned x = h; x; x &= x - 1) {
+                        const unsigned v = w * 32 + __ffs(x) - 1;
+                        c += __ldcg(&b.n_delta[v]);
+                        g.list[at++] = (unsigned short)(v | 0x8000u);
+                    }
+                }
+                cand += c * len;
+                g.sync();
+                const unsigned n = g.count[0];
+                if (!n) continue;
+                unite(o, b, g, n);
+                g.sync();
+                give(o, b, g.warp, WD_WARPS, len, [&](unsigned e) { return other_of(ru.ix, s + e); }, [&](unsigned) { return (const unsigned*)g.led[0]; });
+            }
+            first = (first + groups - items % groups) % groups;
+        }
+#pragma unroll
+        for (int d = 16; d; d >>= 1) cand += __shfl_xor_sync(FULL, cand, d);
+        if (lane == 0 && cand) atomicAdd(&sum_s[1], cand);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (sum_s[1]) atomicAdd(&slot->cand, sum_s[1]);
+            beat(o);
+            meet();
+            st.pending = __ldcg(&slot->cand);
+            st.slot = st.slot == 2 ? 0 : st.slot + 1;
+        }
+        __syncthreads();
+        if (!st.go) return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        ctl->rows_tuples = st.tuples;
+        ctl->rows_candidates = st.cands;
+        ctl->rows_levels = st.iterations ? st.iterations : 1;  // an iteration over nothing finds nothing
+        ctl->rows_left = st.fix ? 0 : 1;
+    }
+}
 // The loop starts on what was given up, or left.
 __global__ void delta_rows_left_k(Ctl* c) {
     c->tail = c->rows_seeds;
@@ -1769,7 +2088,7 @@ __global__ void delta_rows_left_k(Ctl* c) {
 }  // namespace
 
 static Out out_of(xlb_ctx* c, const DeltaLoop& d) {
-    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log->as<uint64_t>(), d.cap, (Ctl*)d.ctl, c->d_status, d.square ? d.visited->as<unsigned int>() + d.words : nullptr, c->delta_spin_limit};
+    return Out{d.visited->as<unsigned int>(), d.words, d.lo_bits, d.log ? d.log->as<uint64_t>() : nullptr, d.cap, (Ctl*)d.ctl, c->d_status, d.square ? d.visited->as<unsigned int>() + d.words : nullptr, c->delta_spin_limit};
 }
 
 DeltaLoop ops_delta_begin(xlb_ctx* c, int hi_bits, int lo_bits, bool square, int composites) {
@@ -2074,4 +2393,54 @@ void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
         delta_resume_k<<<1, 1, 0, c->stream>>>((Ctl*)d.ctl, max_iterations, square);
         check_launch(c, "delta_resume");
     }
+}
+
+static uint64_t wide_bytes(int bits) {
+    const uint64_t rows = 1ull << bits, map = rows * rows / 32;
+    return (2 * map + 3 * rows + 2 * std::max<uint64_t>(rows / 32, 2) + DELTA_ROWS_MAX * rows + DELTA_ROWS_MAX) * 4;
+}
+bool ops_delta_by_rows_fits(xlb_ctx* c, int bits) {
+    return bits >= WD_BITS_MIN && bits <= WD_BITS_MAX && (!c->budget || c->allocated + (1ull << (2 * bits)) / 8 * 2 + wide_bytes(bits) <= c->budget);
+}
+void ops_delta_by_rows(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRows>& rules, uint64_t max_iterations, DeltaResult* res) {
+    for (auto& r : rules)
+        if (rules.size() > DELTA_ROWS_MAX || !r.list) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules by rows", rules.size());
+    Wide b{};
+    b.rows = 1u << d.hi_bits;
+    b.words = b.rows / 32;
+    WideRules rs{};
+    for (auto& r : rules) {
+        WideRule& x = rs.r[rs.n++];
+        x.kind = r.kind;
+        x.ix = view_of(*r.list);
+    }
+    const size_t smem = wide_group_bytes(b.words) * WD_GROUPS;
+    if (!c->delta_wide_attr_set) CUDA_OK(cudaFuncSetAttribute(delta_wide_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(wide_group_bytes(1u << (WD_BITS_MAX - 5)) * WD_GROUPS)));
+    c->delta_wide_attr_set = true;
+    const uint64_t map = (uint64_t)b.rows * b.words, marks = std::max(b.rows / 32, 2u);
+    Buf all = make_buf(c, wide_bytes(d.hi_bits));
+    CUDA_OK(set_async(c, all->p, 0, all->bytes));
+    unsigned* at = all->as<unsigned>();
+    b.delta = at, at += map;
+    b.reached = at, at += map;
+    b.stamp = at, at += b.rows;
+    b.n_delta = at, at += b.rows;
+    b.n_head = at, at += b.rows;
+    b.active[0] = at, at += marks;
+    b.active[1] = at, at += marks;
+    b.keys = at, at += (uint64_t)DELTA_ROWS_MAX * b.rows;
+    b.n_keys = at;
+    Out o = out_of(c, d);
+    Ctl* ctl = (Ctl*)d.ctl;
+    void* args[] = {&o, &rs, &b, &max_iterations};
+    prof_begin(c, "expand_mark", 0);
+    CUDA_OK(cudaLaunchCooperativeKernel((const void*)delta_wide_k, dim3((unsigned)c->sm_count), dim3(DL_THREADS), args, smem, c->stream));
+    check_launch(c, "expand_mark");
+    unsigned long long w[4];  // tuples, candidates, iterations, left
+    read_words(c, &ctl->rows_tuples, 4, w);
+    res->rows = w[0];
+    res->candidates = w[1];
+    res->iterations = w[2];
+    res->fix = w[3] == 0;
+    prof_add_bytes(c, "expand_mark", w[0] / 8 + map * 12);
 }

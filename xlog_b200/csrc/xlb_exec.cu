@@ -1772,8 +1772,16 @@ struct DeltaPlan {
         bool bits_are_hi = false;
         int composed = -1, composed_kc = 0, composed_list_key = 0, composed_row_key = 0;
     };
+    // a rule by rows of the head (see DeltaRows); the stored atom and its column that P is in
+    struct Wide {
+        const FlatRule* fr;
+        DeltaRows::Kind kind;
+        int list, list_kc;
+    };
     std::vector<One> rec;
     std::vector<Two> square;
+    std::vector<Wide> wide;
+    size_t wide_rules = 0;  // recursive rules; all of them are in `wide`, or not
     std::vector<const FlatRule*> seeds;
 };
 constexpr size_t DELTA_RULES_MAX = 4, DELTA_VARIANTS_MAX = 8, DELTA_COMPOSED_MAX = 2;
@@ -1844,6 +1852,36 @@ static bool square_variant(const FlatRule& fr, size_t at, const std::set<std::st
     return true;
 }
 
+// A rule with one or two recursive atoms as one of the kinds of DeltaRows, if it is one.
+static void wide_rule(const FlatRule& fr, const std::set<std::string>& rec, DeltaPlan* plan) {
+    std::vector<const Atom*> own;
+    int stored = -1;
+    for (size_t i = 0; i < fr.atoms.size(); ++i) {
+        if (rec.count(fr.atoms[i].rel)) own.push_back(&fr.atoms[i]);
+        else if (stored >= 0) return;
+        else stored = (int)i;
+    }
+    if (fr.head_vars.size() != 2 || own.empty() || own.size() > 2 || stored < 0) return;
+    const int h = fr.head_vars[0], l = fr.head_vars[1];
+    // the stored atom lists `to` for `from`
+    const auto lists = [&](int from, int to) {
+        const Atom& s = fr.atoms[stored];
+        return from != to && (s.var[0] == from && s.var[1] == to ? 0 : s.var[1] == from && s.var[0] == to ? 1 : -1) >= 0;
+    };
+    const auto add = [&](DeltaRows::Kind kind, int from) { plan->wide.push_back({&fr, kind, stored, fr.atoms[stored].var[0] == from ? 0 : 1}); };
+    if (own.size() == 1) {
+        const int p = own[0]->var[0], y = own[0]->var[1];
+        if (l == y && h != y && lists(p, h)) add(DeltaRows::COPY, p);
+        return;
+    }
+    for (int k = 0; k < 2; ++k) {
+        const int p = own[k]->var[0], q = own[k]->var[1], a = own[1 - k]->var[0], y = own[1 - k]->var[1];
+        if (p == q || a == y || y == p || y == q) continue;
+        if (a == q && l == y && h != p && h != q && h != y && lists(p, h)) return add(DeltaRows::STEPS, p);
+        if (a != q && a != p && l == y && h == q && lists(p, a)) return add(DeltaRows::ACROSS, p);
+    }
+}
+
 static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const std::vector<std::string>& preds, const std::set<std::string>& rec,
                         const std::map<std::string, xlb_schema>& schema, DeltaPlan* plan) {
     if (c->world != 1 || c->comm_world != 1 || (c->flags & (XLB_FLAG_NO_DENSE | XLB_FLAG_KEEP_DELTAS)) || getenv("XLB_NO_DELTA_LOOP")) return false;
@@ -1862,7 +1900,9 @@ static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const st
             plan->seeds.push_back(&fr);
             continue;
         }
+        ++plan->wide_rules;
         if (nrec == 2 && fr.filters.empty() && fr.checks.empty() && fr.atoms.size() <= 3) {
+            wide_rule(fr, rec, plan);
             for (size_t i = 0; i < fr.atoms.size(); ++i)
                 if (rec.count(fr.atoms[i].rel) && !square_variant(fr, i, rec, plan)) return false;
             continue;
@@ -1891,6 +1931,7 @@ static bool delta_shape(xlb_ctx* c, const std::vector<FlatRule>& rules, const st
         one.hi_src = fr.head_vars.size() == 2 ? src(fr.head_vars[0]) : 4;
         one.lo_src = src(fr.head_vars.back());
         if (one.hi_src < 0 || one.lo_src < 0) return false;
+        if (fr.atoms.size() == 2) wide_rule(fr, rec, plan);
         plan->rec.push_back(one);
     }
     size_t composed = 0;
@@ -1964,7 +2005,8 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         if (c->budget && c->allocated + (square ? 8 : 3) * bitmap > c->budget) return false;
         int composed = 0;
         for (auto& t : plan.square) composed += t.composed >= 0 ? 1 : 0;
-        DeltaLoop d = ops_delta_begin(c, hb, lb, square, composed);
+        const bool by_rows = square && plan.wide.size() == plan.wide_rules && plan.wide.size() <= DELTA_ROWS_MAX && ops_delta_by_rows_fits(c, lb);
+        DeltaLoop d = ops_delta_begin(c, hb, lb, square && !by_rows, composed);
         if (from_store) {
             PhaseTimer t(c, &rs.st.ms_join);
             ops_delta_append(c, d, delta);
@@ -1997,8 +2039,17 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
                 ops_delta_seed(c, d, cand);
             }
         }
+        std::vector<DeltaRows> wide;
+        for (auto& w : plan.wide) {
+            if (!by_rows) break;
+            DeltaRows r;
+            r.kind = w.kind;
+            r.list = &get_index(c, w.fr->atoms[w.list].rel, w.list_kc, rs);
+            if (r.list->n) wide.push_back(r);
+        }
         std::vector<DeltaRule> run;
         for (auto& one : plan.rec) {
+            if (by_rows) break;
             DeltaRule r;
             r.joins = one.joins;
             r.hi_src = one.hi_src;
@@ -2013,6 +2064,7 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         }
         std::vector<DeltaVariant> variants;
         for (auto& two : plan.square) {
+            if (by_rows) break;
             DeltaVariant v;
             v.list_key = two.list_key;
             v.rows = two.rows;
@@ -2030,7 +2082,8 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         {
             PhaseTimer t(c, &rs.st.ms_join);
             try {
-                ops_delta_run(c, d, run, variants, c->max_iterations - it, full, &res);
+                if (by_rows) ops_delta_by_rows(c, d, wide, c->max_iterations - it, &res);
+                else ops_delta_run(c, d, run, variants, c->max_iterations - it, full, &res);
             } catch (const XlbError& e) {
                 if (e.st != XLB_ERR_TIMEOUT) throw;
                 rs.st = before;  // a wait inside the loop ran out: the routes without one start over

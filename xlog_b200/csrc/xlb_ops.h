@@ -211,6 +211,16 @@ struct DeltaVariant {
     const Index* composed = nullptr;
     int composed_list_key = 0, composed_row_key = 0;  // halves of a head row (0 high, 1 low): what probes `composed`, what keys its bit rows
 };
+// The same rules by rows of the head: what is derived for a row, as bits, and the rows it belongs to.
+struct DeltaRows {
+    enum Kind {
+        COPY,    // h(X, Y) :- e(P, X), h(P, Y): row P of the delta belongs to the rows listed for P
+        STEPS,   // h(X, Y) :- e(P, X), h(P, Q), h(Q, Y): rows Q of row P to the rows listed for P
+        ACROSS,  // h(Q, Y) :- e(P, W), h(P, Q), h(W, Y): the rows listed for P to the rows Q of row P
+    } kind = COPY;
+    const Index* list = nullptr;  // of P
+};
+constexpr int DELTA_ROWS_MAX = 8;
 struct DeltaLoop {
     Buf visited;            // the head as a bitmap (square components: more of them behind it)
     bool square = false;
@@ -234,6 +244,10 @@ void ops_delta_append(xlb_ctx* c, DeltaLoop& d, const Keys& rows);  // a delta a
 // To the fixpoint.  `known`: what ops_delta_known was given (unique, disjoint from the seeds).
 void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules, const std::vector<DeltaVariant>& variants, uint64_t max_iterations, const Keys& known,
                    DeltaResult* res);
+
+// The same for rules that are all of the kinds of DeltaRows, from seeds alone, over a head of `bits` bits a column.
+bool ops_delta_by_rows_fits(xlb_ctx* c, int bits);
+void ops_delta_by_rows(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRows>& rules, uint64_t max_iterations, DeltaResult* res);
 
 // A whole frontier fixpoint in one launch (xlb_frontier.cu): seeds are the rows of `rel` with a column
 // equal to a constant; from then on rows whose key_col holds a derived value derive their value_col.
