@@ -5,6 +5,9 @@ import gc
 import numpy as np
 import pytest
 
+from xlog_b200 import _abi as A
+from xlog_b200.executor import run_program
+from xlog_b200.plan import CompiledRule, ExecutionPlan, Scan, Scc
 from xlog_b200.provider import KernelProvider
 
 pytestmark = pytest.mark.gpu
@@ -46,41 +49,52 @@ def test_results_are_independent_and_outlive_the_context():
 
 def expect(p, rel, cols):
     for g, c in zip(p.download(rel), cols):
-        assert np.array_equal(g.view(np.uint8) if c.dtype == np.bool_ else g, c.view(np.uint8) if c.dtype == np.bool_ else c, equal_nan=c.dtype.kind == "f")
+        assert np.array_equal(g, c)
 
 
-# First columns of sets, of 6 MB and more, go as runs where these are long: tiles are 4096 rows, a warp's 512, what a
+def rows_from(starts, n):
+    starts = np.unique(starts)
+    return np.diff(np.append(starts, n))
+
+
+# First columns of sets, of 6 MB and more and of few values, go as runs: tiles are 4096 rows, a warp's 512, what a
 # thread fills 65536 (4 bytes) or 32768 (8 bytes) rows, and the staging holds 32766 or 16383 runs.
-@pytest.mark.parametrize("dtype", [np.uint32, np.int64, np.float32])
-@pytest.mark.parametrize("runs", ["one", "last", "edges", "even", "short", "limit", "over"])
-@pytest.mark.parametrize("n", [786431, 3 << 18, (3 << 19) - 1, 3 << 19, (3 << 19) + 4097, 2222222])
-def test_first_columns_of_long_runs(dtype, runs, n):
-    cap = (256 * 1024 - 16) // (2 * np.dtype(dtype).itemsize)
-    if runs == "one":
-        starts = [0]
-    elif runs == "last":
-        starts = [0, n - 1]
-    elif runs == "edges":
-        starts = sorted({x + d for x in (0, 512, 4096, 32768, 65536, 131072, n - 4096) for d in (-1, 0, 1) if 0 <= x + d < n})
-    elif runs == "even":
-        starts = range(0, n, 1000)
-    elif runs == "short":
-        starts = range(0, n, 9)  # more runs than are worth it
-    else:
-        count = min(cap, n // 64) + (runs == "over")
-        starts = np.linspace(0, n - 1, count).astype(np.int64)
-    starts = np.unique(np.array(list(starts)))
-    rng = np.random.default_rng(n)
-    values = np.sort(rng.standard_normal(len(starts))).astype(dtype) if dtype == np.float32 else np.sort(rng.choice(1 << 30, len(starts), replace=False)).astype(dtype)
-    if dtype == np.float32:
-        values[-1] = np.nan
-    cols = [np.repeat(values, np.diff(np.append(starts, n))), np.arange(n, dtype=np.uint32), rng.integers(0, 2, n).astype(np.bool_)]
+@pytest.mark.parametrize("runs", ["one", "last", "edges", "even", "most", "many"])
+@pytest.mark.parametrize("n", [(3 << 19) - 1, 3 << 19, (3 << 19) + 4097, 2222222])
+def test_first_columns_of_long_runs(runs, n):
+    starts = {"one": [0], "last": [0, n - 1], "edges": [x + d for x in (0, 512, 4096, 32768, 65536, 131072, n - 4096) for d in (-1, 0, 1) if 0 <= x + d < n],
+              "even": np.arange(0, n, 1000), "most": np.linspace(0, n - 1, 1 << 14).astype(np.int64), "many": np.arange(0, n, 9)}[runs]
+    first = np.repeat(np.arange(len(np.unique(starts)), dtype=np.uint32), rows_from(starts, n))
+    cols = [first, np.arange(n, dtype=np.uint32)]
     p = KernelProvider(device=0)
-    for k in (2, 3):
-        rel = p.dedup(p.create_buffer_from_slices([c[::-1] for c in cols[:k]]))
-        assert rel.is_canonical()
-        expect(p, rel, cols[:k])
-        expect(p, p.create_buffer_from_slices(cols[:k]), cols[:k])
+    rel = p.dedup(p.create_buffer_from_slices([c[::-1] for c in cols]))
+    assert rel.is_canonical()
+    expect(p, rel, cols)
+    expect(p, p.create_buffer_from_slices(cols), cols)
+    p.close()
+
+
+@pytest.mark.parametrize("dtype", [np.uint64, np.int64, np.float32, np.int32])
+def test_first_columns_of_wide_results(dtype):
+    # of a plan over typed columns: a set of decoded ranks
+    code = {np.uint64: A.U64, np.int64: A.I64, np.float32: A.F32, np.int32: A.I32}[dtype]
+    rng = np.random.default_rng(5)
+    per = rng.integers(1, 4000, 1000)
+    per[::7] = 1
+    values = np.unique(rng.integers(-(1 << 30), 1 << 30, 5000)).astype(dtype)[:4000]
+    if dtype == np.float32:
+        values = np.sort(values)
+    values = np.unique(values) if dtype != np.uint64 else np.unique(np.abs(values.astype(np.int64)).astype(np.uint64))
+    n = len(values)
+    first = np.repeat(values[:1000], np.minimum(per, n))
+    second = np.concatenate([values[: min(k, n)] for k in per])
+    plan = ExecutionPlan([Scc(0, False, [CompiledRule("h", Scan(0), (code, code))])], {"s": 0, "h": 1})
+    order = rng.permutation(len(first))
+    p = KernelProvider(device=0)
+    got, _ = run_program(p, plan, {"s": [first[order], second[order]]}, ["h"])
+    assert len(first) * first.itemsize >= 6 << 20
+    for g, w in zip(got["h"], (first, second)):
+        assert np.array_equal(g, w)
     p.close()
 
 

@@ -659,6 +659,7 @@ struct xlb_rel {
     mutable Buf cols[XLB_MAX_ARITY];
     mutable Buf packed;
     mutable uint64_t or_bound = ~0ull;  // host-known upper bound of the OR of the packed rows (~0: unknown)
+    uint64_t firsts = ~0ull;  // host-known bound of how many different values the first column has (~0: unknown)
     bool canonical = false;
 };
 

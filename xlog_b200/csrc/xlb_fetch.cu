@@ -212,8 +212,10 @@ bool page_locked(const void* p) {
 }
 
 template <class T>
+constexpr uint64_t runs_room() { return (STAGE_BYTES - 16) / sizeof(Run<T>); }
+template <class T>
 void fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n, unsigned threads) {
-    const uint64_t tiles = (n + RUNS_TILE - 1) / RUNS_TILE, cap = std::min<uint64_t>((STAGE_BYTES - 16) / sizeof(Run<T>), n / RUNS_ROWS_MIN);
+    const uint64_t tiles = (n + RUNS_TILE - 1) / RUNS_TILE, cap = runs_room<T>();
     char* stage = stage_buffer(c);
     unsigned long long* total = reinterpret_cast<unsigned long long*>(stage);
     const Run<T>* runs = reinterpret_cast<const Run<T>*>(stage + 16);
@@ -230,8 +232,8 @@ void fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n
     {
         Filler<T> filler(threads);
         stream_wait(c);
-        if (*total > cap) side.add(cols[0], col, n * sizeof(T));
-        else filler.fill(static_cast<T*>(cols[0]), runs, *total, n);
+        if (*total > cap) xlb_fail(XLB_ERR_CUDA, "internal: %llu runs of at most %llu values", *total, (unsigned long long)r->firsts);
+        filler.fill(static_cast<T*>(cols[0]), runs, *total, n);
     }
     side.wait();
 }
@@ -241,10 +243,12 @@ void fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n
 void ops_fetch_columns(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n) {
     ops_rel_columns(c, r);
     const uint32_t arity = r->schema.arity, width = type_width(r->schema.types[0]);
-    // Only of a set, which is in order (in any other relation long runs are a piece of luck, and looking for them in a
-    // sort's result took 11 us of 1500); not with several ranks (whose waits watch the communicator), and not into memory
-    // that the driver copies to by itself: such a copy does not run beside anything.
-    if (r->canonical && arity >= 2 && width >= 4 && n * width >= RUNS_MIN_BYTES && n < 1ull << 32 && !c->wait_hook) {
+    // Only of a set, which is in order, whose first values are known to be few (looking for runs where there are none took
+    // 11 us of a sort's 1500 and 15 of 790 of a union over 2^18 first values); not with several ranks (whose waits watch the
+    // communicator), and not into memory that the driver copies to by itself: such a copy does not run beside anything.
+    const uint64_t bound = rel_packable(r->schema) && r->or_bound != ~0ull ? (r->or_bound >> 32) + 1 : ~0ull, firsts = std::min(bound, r->firsts);
+    if (r->canonical && arity >= 2 && firsts <= std::min(n / RUNS_ROWS_MIN, width == 4 ? runs_room<uint32_t>() : runs_room<unsigned long long>()) && width >= 4 && n * width >= RUNS_MIN_BYTES &&
+        n < 1ull << 32 && !c->wait_hook) {
         const unsigned cores = host_pool_cores();
         bool locked = cores >= RUNS_CORES_MIN;
         for (uint32_t i = 0; i < arity; ++i) locked = locked && page_locked(cols[i]) && (uintptr_t)cols[i] % width == 0;

@@ -734,6 +734,7 @@ xlb_rel* ops_dense_state_columns(xlb_ctx* c, const DenseState& s, const xlb_sche
     o->schema = schema;
     o->rows = s.rows;
     o->canonical = true;
+    if (schema.arity == 2) o->firsts = 1ull << s.hi_bits;
     for (uint32_t i = 0; i < schema.arity; ++i) o->cols[i] = make_buf(c, s.rows * 4);
     dense_state_out(c, s, 0, o->cols);
     return o.release();
@@ -1890,6 +1891,7 @@ xlb_rel* ops_dict_decode(xlb_ctx* c, const xlb_rel* ranks, const xlb_schema& typ
     o->rows = ranks->rows;
     o->schema = types;
     o->canonical = ranks->canonical;
+    o->firsts = dict.n;
     for (uint32_t i = 0; i < types.arity; ++i) {
         const uint32_t w = type_width(types.types[i]);
         o->cols[i] = make_buf(c, ranks->rows * w);
@@ -2091,6 +2093,7 @@ xlb_rel* ops_rank_decode(xlb_ctx* c, const xlb_rel* ranks, const xlb_schema& typ
     o->rows = k.n;
     o->schema = types;
     o->canonical = ranks->canonical;
+    o->firsts = dict.n;
     for (uint32_t i = 0; i < types.arity; ++i) o->cols[i] = make_buf(c, k.n * 4);
     if (k.n) {
         prof_begin(c, "dict_decode", k.n * (8ull + 4 * types.arity));
