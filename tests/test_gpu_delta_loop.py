@@ -88,6 +88,23 @@ def test_iteration_limit_on_a_path(limit):
     p.close()
 
 
+# values with as many matches as a row of the head has words (1, 2, 16, 32, 64; 128 are too many), and fewer; some edges twice
+@pytest.mark.parametrize("nodes,degree", [(20, 8), (60, 4), (500, 40), (500, 12), (1000, 40), (1500, 70), (3000, 130)])
+def test_dense_closures(nodes, degree, monkeypatch):
+    rng = np.random.default_rng(nodes)
+    hubs = rng.integers(0, nodes // 2, nodes * degree)  # a part of the nodes has no successor
+    e = [np.append(hubs, nodes - 1).astype(np.uint32), np.append(rng.integers(0, nodes, nodes * degree), 0).astype(np.uint32)]
+    e = [np.concatenate([c, c[:50]]) for c in e]
+    both(programs.transitive_closure(), {"edge": e}, "reach", monkeypatch)
+    # a path of such blocks: a level for each
+    b = nodes // 10 + 1
+    k = 10 * b
+    src = np.repeat(np.arange(k - b), 2)
+    dst = (src // b + 1) * b + rng.integers(0, b, len(src))
+    dense = [np.concatenate([src, np.repeat(np.arange(b), 9 * b)]).astype(np.uint32), np.concatenate([dst, np.tile(np.arange(b, k), b)]).astype(np.uint32)]
+    both(programs.transitive_closure(), {"edge": dense}, "reach", monkeypatch)
+
+
 def test_many_long_rows(monkeypatch):
     # 70 sources with 1100 matches each twice over: the list of long rows is used by many warps at once
     src = np.repeat(np.arange(70, dtype=np.uint32), 1100)

@@ -46,6 +46,7 @@ struct Rule {
     int key_src[2];  // which half of the delta row is the key: 0 high, 1 low
     int joins;       // 1 or 2
     int hi_src, lo_src;  // output halves: 0 / 1 the delta row's, 2 / 3 the joined rows' other column, 4 zero
+    unsigned long long rows;  // of the first relation
 };
 constexpr int DL_RULES = 4;
 struct Rules {
@@ -1034,11 +1035,13 @@ constexpr unsigned RW_QUEUE = 16384;              // values the frontier of a ro
 constexpr unsigned RW_LONG = 16384;               // candidates of a warp (some 50 us) from which a row may be given up
 constexpr unsigned RW_LIST = 64;                  // a value with so many matches is a warp's work by itself
 constexpr unsigned RW_FOLLOW = 32;                // levels of one value each after which a row is taken for a path
+constexpr int RW_LISTS_BITS = 11;                 // values whose matches are taken as rows of bits: at most 64 words
 constexpr unsigned RW_SQUARED = 16;               // entries a thread of the path's table
 struct RowsShape {
     unsigned rows, words;  // rows of the bitmap, words of each
     unsigned queue;        // entries, a power of two
     unsigned chunk;        // rows taken at a time
+    const unsigned* lists;  // the relation as rows of bits like the head's, or null
 };
 constexpr unsigned rows_queue(int bits) { return 1u << bits < RW_QUEUE ? 1u << bits : RW_QUEUE; }
 constexpr unsigned rows_bytes(int bits) { return (1u << bits) / 8 + rows_queue(bits) * 2; }
@@ -1047,6 +1050,16 @@ struct RowsShared {
     unsigned failed, next;
     unsigned long long level, cand, tuples, cands, levels;
 };
+__device__ __forceinline__ unsigned warp_sum_before(unsigned mine, unsigned* total) {
+    unsigned incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned v = __shfl_up_sync(FULL, incl, d);
+        if (lane_id() >= (unsigned)d) incl += v;
+    }
+    *total = __shfl_sync(FULL, incl, 31);
+    return incl - mine;
+}
 template <int W>
 struct RowsWarp {
     unsigned* seen;
@@ -1165,6 +1178,51 @@ struct RowsWarp {
         }
         for (; from < total; from += 32) dealt<1>(o, ix, from, total, m, before, shift);
         return all + total;
+    }
+    // All matches of up to 32 values [at, at + m) of the queue, as rows of bits: a row is `words` (at most 64) of them, and
+    // narrow rows are taken several at a time.
+    __device__ __forceinline__ void unite(const unsigned* __restrict__ rows, unsigned n_rows, unsigned words, unsigned at, unsigned m) {
+        const unsigned lane = lane_id(), side = words < 32 ? 32 / words : 1, mine = words < 32 ? lane / words : 0;
+        const unsigned w = lane & (min(words, 32u) - 1);
+        constexpr unsigned N = 8;
+        unsigned acc[2] = {0, 0};
+        for (unsigned j0 = mine; j0 - mine < m; j0 += N * side) {
+            unsigned v[N][2];
+#pragma unroll
+            for (unsigned u = 0; u < N; ++u) {
+                const unsigned y = j0 + u * side < m ? queue[(at + j0 + u * side) & mask] : ~0u;
+                const bool on = y < n_rows;
+                v[u][0] = on ? __ldg(&rows[y * words + w]) : 0u;
+                v[u][1] = on && words > 32 ? __ldg(&rows[y * words + 32 + w]) : 0u;
+            }
+#pragma unroll
+            for (unsigned u = 0; u < N; ++u) {
+                acc[0] |= v[u][0];
+                acc[1] |= v[u][1];
+            }
+        }
+        for (unsigned d = words; d < 32; d *= 2) acc[0] |= __shfl_xor_sync(FULL, acc[0], d);
+        unsigned count = 0, all;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (lane != w) acc[k] = 0;  // (the lanes beside hold the same; a second word there is only of rows of 64)
+            if (acc[k] && acc[k] & ~seen[w + 32 * k]) acc[k] &= ~atomicOr(&seen[w + 32 * k], acc[k]);
+            else acc[k] = 0;
+            count += __popc(acc[k]);
+        }
+        const unsigned before = warp_sum_before(count, &all);
+        if (!all) return;
+        unsigned to = 0;
+        if (lane == 0) to = atomicAdd(&sh->tail, all);
+        to = __shfl_sync(FULL, to, 0);
+        if (to + all - head > mask + 1) {  // (the level at hand is still in the ring)
+            if (lane == 0) sh->failed = 1;
+            return;
+        }
+        to += before;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            for (unsigned x = acc[k]; x; x &= x - 1, ++to) queue[to & mask] = (unsigned short)((w + 32 * k) * 32 + __ffs(x) - 1);
     }
     // A frontier of one value, followed by one warp while it stays one, for at most `most` levels: a value's
     // matches are looked up while the test whether it is new is under way.  Leaves the ring's ends and the
@@ -1376,7 +1434,13 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const Out o, const __grid
                 for (unsigned at = head + warp * per; at - head < end - head; at += W * per) {
                     const bool on = lane < per && end - at > lane;
                     const unsigned y = on ? w.queue[(at + lane) & w.mask] : 0u;
-                    for (int q = 0; q < rules.n; ++q) cand += w.expand(o, rules.r[q].ix[0], on, y);
+                    if (sh.lists) {
+                        uint32_t start = 0, len = 0;
+                        if (on) find(rules.r[0].ix[0], y, start, len);
+                        cand += __reduce_add_sync(FULL, len);
+                        w.unite(sh.lists, sh.rows, sh.words, at, min(per, end - at));
+                    } else
+                        for (int q = 0; q < rules.n; ++q) cand += w.expand(o, rules.r[q].ix[0], on, y);
                     if (cand > looked) {
                         looked = cand + 4096;
                         if (lane == 0 && *(volatile unsigned*)&ctl->rows_idle * 4ull > gridDim.x * 3ull) s.failed = 1;
@@ -1472,16 +1536,6 @@ struct BitsState {
     unsigned long long tuples, cands, pending, iterations;
     unsigned slot, small, leaving, over, fix, go;
 };
-__device__ __forceinline__ unsigned warp_sum_before(unsigned mine, unsigned* total) {
-    unsigned incl = mine;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned v = __shfl_up_sync(FULL, incl, d);
-        if (lane_id() >= (unsigned)d) incl += v;
-    }
-    *total = __shfl_sync(FULL, incl, 31);
-    return incl - mine;
-}
 // B as a block keeps it: per value its matches' start and number, and the matches.
 struct Lists {
     const unsigned* at;
@@ -2176,6 +2230,15 @@ static bool run_rows(xlb_ctx* c, DeltaLoop& d, const Rules& rs, uint64_t max_ite
     sh.rows = 1u << d.hi_bits;
     sh.words = 1u << (d.lo_bits - 5);
     sh.queue = rows_queue(d.lo_bits);
+    // Where the seeds are the relation itself and a value has as many matches as a row has words, a level takes the
+    // values' rows and not their matches one by one (four blocks of 128 nodes, 33 M candidates: 62 us, now 20
+    // and 4 for the copy; 2000 nodes of degree 5, rows of 64 words, stay with their matches.)
+    Buf lists;
+    if (d.seeds_listed && d.lo_bits <= RW_LISTS_BITS && (uint64_t)rs.r[0].rows >= d.words) {
+        lists = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
+        CUDA_OK(copy_async(c, lists->p, d.visited->p, d.words * 4, cudaMemcpyDeviceToDevice));
+        sh.lists = lists->as<unsigned>();
+    }
     Ctl* ctl = (Ctl*)d.ctl;
     prof_begin(c, "expand_mark", 0);
     // Four warps a row keep rows of a few thousand candidates short (one: twice the time); eight where an SM
@@ -2309,6 +2372,7 @@ void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
             r.key_src[k] = rules[q].key_src[k];
             r.ix[k] = view_of(*rules[q].ix[k]);
         }
+        r.rows = rules[q].ix[0]->n;
     }
     Buf by_rows;  // the head after rows were evaluated, and some are left
     BitsRules bits{};

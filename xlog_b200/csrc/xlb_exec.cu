@@ -2039,6 +2039,13 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
                 ops_delta_seed(c, d, cand);
             }
         }
+        if (plan.rec.size() == 1 && plan.square.empty() && plan.seeds.size() == 1 && !from_store) {
+            const FlatRule& seed = *plan.seeds[0];
+            const auto& one = plan.rec[0];
+            d.seeds_listed = seed.atoms.size() == 1 && seed.filters.empty() && seed.checks.empty() && seed.atoms[0].arity == 2 && seed.head_vars.size() == 2 &&
+                             seed.atoms[0].var[0] != seed.atoms[0].var[1] && seed.head_vars[0] == seed.atoms[0].var[0] && seed.head_vars[1] == seed.atoms[0].var[1] && one.joins == 1 &&
+                             one.kc[0] == 0 && seed.atoms[0].rel == one.fr->atoms[one.atom[0]].rel;
+        }
         std::vector<DeltaRows> wide;
         for (auto& w : plan.wide) {
             if (!by_rows) break;

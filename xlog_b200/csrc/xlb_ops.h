@@ -230,6 +230,7 @@ struct DeltaLoop {
     uint64_t cap = 0, room = 0;  // tuples the log can hold; that may be in it
     void* ctl = nullptr;    // behind the bitmaps
     bool seeded = false;
+    bool seeds_listed = false;  // the seeds are the rows of the one relation that the one rule joins with, by its first column
 };
 struct DeltaResult {
     uint64_t rows = 0;      // tuples in the log: what was derived beyond the known rows
