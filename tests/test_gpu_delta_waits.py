@@ -57,3 +57,16 @@ def test_a_wait_that_runs_out_falls_back(name, plan, rels, out, monkeypatch):
         assert np.array_equal(g, w) and np.array_equal(b, w)
     assert stats["kernel_launches"] > fast["kernel_launches"]
     assert (stats["iterations"], stats["candidate_tuples"]) == (fast["iterations"], fast["candidate_tuples"])
+
+
+@pytest.mark.parametrize("name,plan,rels,out", [
+    ("same generation", programs.same_generation(), {"edge": list(workloads.tree_dag(1200, 0.05)[:2])}, "sg"),
+    ("points-to", programs.andersen(), {k: list(v) for k, v in workloads.andersen_program(0.0002, 11).items()}, "pt"),
+], ids=lambda x: x if isinstance(x, str) else "")
+def test_waits_of_the_kernels_by_rows(name, plan, rels, out, monkeypatch):
+    # (whether one poll is enough is a matter of luck: the result and the counts are the same either way)
+    got, fast = run(monkeypatch, plan, rels, out)
+    again, stats = run(monkeypatch, plan, rels, out, polls=1)
+    for g, a in zip(got, again):
+        assert np.array_equal(g, a)
+    assert (stats["iterations"], stats["candidate_tuples"]) == (fast["iterations"], fast["candidate_tuples"])

@@ -1036,6 +1036,7 @@ constexpr unsigned RW_LONG = 16384;               // candidates of a warp (some 
 constexpr unsigned RW_LIST = 64;                  // a value with so many matches is a warp's work by itself
 constexpr unsigned RW_FOLLOW = 32;                // levels of one value each after which a row is taken for a path
 constexpr int RW_LISTS_BITS = 11;                 // values whose matches are taken as rows of bits: at most 64 words
+constexpr uint64_t RW_LISTS_MIN = 1u << 13;       // rows of the relation below which the copy costs what it saves (four blocks of 44 nodes, 7744 rows: 162 us by matches, 165 by rows; of 46 162 and 162; of 80 205 and 192)
 constexpr unsigned RW_SQUARED = 16;               // entries a thread of the path's table
 struct RowsShape {
     unsigned rows, words;  // rows of the bitmap, words of each
@@ -2234,7 +2235,7 @@ static bool run_rows(xlb_ctx* c, DeltaLoop& d, const Rules& rs, uint64_t max_ite
     // values' rows and not their matches one by one (four blocks of 128 nodes, 33 M candidates: 62 us, now 20
     // and 4 for the copy; 2000 nodes of degree 5, rows of 64 words, stay with their matches.)
     Buf lists;
-    if (d.seeds_listed && d.lo_bits <= RW_LISTS_BITS && (uint64_t)rs.r[0].rows >= d.words) {
+    if (d.seeds_listed && d.lo_bits <= RW_LISTS_BITS && rs.r[0].rows >= std::max<uint64_t>(d.words, RW_LISTS_MIN)) {
         lists = make_buf(c, std::max<uint64_t>(d.words * 4, 16));
         CUDA_OK(copy_async(c, lists->p, d.visited->p, d.words * 4, cudaMemcpyDeviceToDevice));
         sh.lists = lists->as<unsigned>();
