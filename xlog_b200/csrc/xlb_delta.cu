@@ -753,7 +753,7 @@ __device__ __forceinline__ bool wait_for(const Out& o, const unsigned* word, uns
 }
 
 template <bool SQUARE>
-__global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const Out o, const __grid_constant__ Rules rules, Heavy* heavy, uint64_t max_iterations, const __grid_constant__ Square sq) {
+__global__ void __launch_bounds__(DL_THREADS, 1) delta_loop_k(const __grid_constant__ Out o, const __grid_constant__ Rules rules, Heavy* heavy, uint64_t max_iterations, const __grid_constant__ Square sq) {
     extern __shared__ uint64_t stage_s[];
     __shared__ State state_s;
     __shared__ unsigned go_s;
@@ -968,7 +968,7 @@ __device__ __forceinline__ void ready(Ctl* ctl, bool square) {
     c->phase = n == 0 ? PH_DONE : square ? PH_FULL : PH_ROWS;  // (never solo: a block that starts late would miss it)
 }
 // Rows of a bag into the head: new ones (their bit was clear) are appended to the log.
-__global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict__ rows, uint64_t n, Out o, bool square) {
+__global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict__ rows, uint64_t n, const __grid_constant__ Out o, bool square) {
     __shared__ uint64_t stage_s[BLOCK / 32][64];
     uint64_t* stage = stage_s[threadIdx.x >> 5];
     const uint64_t step = (uint64_t)gridDim.x * BLOCK;
@@ -1365,7 +1365,7 @@ __device__ __noinline__ void rows_give_up(const Out& o, const RowsShape& sh, uns
     if (threadIdx.x == 0) atomicAdd(&o.ctl->rows_given_up, 1ull);
 }
 template <int W>
-__global__ void __launch_bounds__(W * 32) delta_rows_k(const Out o, const __grid_constant__ Rules rules, const RowsShape sh, uint64_t max_iterations) {
+__global__ void __launch_bounds__(W * 32) delta_rows_k(const __grid_constant__ Out o, const __grid_constant__ Rules rules, const __grid_constant__ RowsShape sh, uint64_t max_iterations) {
     extern __shared__ __align__(16) unsigned char rw_smem[];
     __shared__ RowsShared s;
     __shared__ uint2 match_s[W][32];
@@ -1592,7 +1592,7 @@ __device__ __forceinline__ unsigned lead(const Out& o, const Ix& ix, const Lists
     __syncwarp();
     return c;
 }
-__global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const Out o, const __grid_constant__ BitsRules rules, const Bits b, uint64_t max_iterations) {
+__global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_constant__ Out o, const __grid_constant__ BitsRules rules, const __grid_constant__ Bits b, uint64_t max_iterations) {
     extern __shared__ unsigned bt_smem[];
     __shared__ BitsState st;
     __shared__ unsigned long long sum_s[2];
@@ -1914,7 +1914,7 @@ __device__ __forceinline__ void unite(const Out& o, const Wide& b, const WideGro
         if (acc) atomicOr(reinterpret_cast<unsigned long long*>(g.led[0] + w), acc);
     }
 }
-__global__ void __launch_bounds__(DL_THREADS, 1) delta_wide_k(const Out o, const __grid_constant__ WideRules rules, const Wide b, uint64_t max_iterations) {
+__global__ void __launch_bounds__(DL_THREADS, 1) delta_wide_k(const __grid_constant__ Out o, const __grid_constant__ WideRules rules, const __grid_constant__ Wide b, uint64_t max_iterations) {
     extern __shared__ __align__(16) unsigned char wd_smem[];
     __shared__ BitsState st;
     __shared__ unsigned long long sum_s[2];
@@ -2082,7 +2082,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_wide_k(const Out o, const
                         for (unsigned x = h; x; x &= x - 1) g.list[at++] = (unsigned short)((w * 32 + __ffs(x) - 1) | 0x8000u);
                     }
                     g.sync();
-                    give(o, b, g.warp, WD_WARPS, g.count[0], [&](unsigned e) { return (unsigned)(g.list[e] & 0x7FFF); }, [&](unsigned e) { return (const unsigned*)g.led[g.list[e] >> 15]; });
+                    give(o, b, g.warp, WD_WARPS, g.count[0], [&](unsigned e) { return (unsigned)(g.list[e] & 0x7FFF); }, [&](unsigned e) { return (const unsigned*)(g.list[e] >> 15 ? g.led[1] : g.led[0]); });
                     continue;
                 }
                 // STEPS: rows of the head for values of the delta, rows of the delta for values of the head
