@@ -132,7 +132,9 @@ xlb_status xlb_rel_schema(const xlb_rel* rel, xlb_schema* schema);
 /* canonical_full_row_set_certified (memory.rs:1771-1773): sorted by all columns and unique. */
 xlb_status xlb_rel_is_canonical(const xlb_rel* rel, int* canonical);
 /* download_column::<T> for every column (crates/xlog-cuda/src/provider/transfer.rs:22).
- * Copies min(rows, cap_rows) rows into the host arrays and reports the logical row count. */
+ * Copies min(rows, cap_rows) rows into the host arrays and reports the logical row count.  The first
+ * column of a large set into page-locked memory may be written by up to four threads of the process
+ * while the others are copied; everything is there, and no thread left, when the call returns. */
 xlb_status xlb_rel_to_host(xlb_ctx* ctx, const xlb_rel* rel, void* const* cols, uint64_t cap_rows,
                            uint64_t* rows);
 /* Page-locked host memory for results, from a bounded pool that the process shares: copies of

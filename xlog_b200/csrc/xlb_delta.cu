@@ -1498,7 +1498,7 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const __grid_constant__ O
 // those into the rows that A leads to; what they gain over the head is found by their own block in the next
 // iteration.  A tuple so costs no atomic in global memory, no entry in a log and no look at a word of its
 // own: same generation over 7001 nodes (26.8 M tuples) took 718 us in the loop, bound by its atomics on single
-// bits, 282 with a warp for each row (five rows in seven have nothing to lead to), and takes 188 here: a phase is
+// bits, 282 with a warp for each row (five rows in seven have nothing to lead to), and takes 180 here: a phase is
 // some 20 K cycles of dependent steps between two barriers, then atomics on words of shared memory (what neighbours
 // lead to shares words; setting a lane's bits of one word together cost more than it saved).
 //   Rows that nobody reached are passed over by a stamp.  Lists of A are shared out among a block's warps only: where one
@@ -1819,7 +1819,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
 // delta where it is in the head) are ORed in registers, warp by warp, then in shared memory, and the union goes
 // to the rows it belongs to as far as these gain by it.  (Tuple by tuple, each against bit rows of the head, its
 // transpose and its composites, as delta_loop_k does, a tuple cost an atomic a candidate word, one on the transpose and its
-// place in the log, and few warps had most of them: points-to over 1500 values 395 us, here 190.)  An iteration has two
+// place in the log, and few warps had most of them: points-to over 1500 values 395 us, here 184.)  An iteration has two
 // phases: the rows' own warps add what was derived to the head, which makes the delta; then groups of eight warps
 // take the values of all rules in turn, up to four groups a value where there are few of them.  What bounds it is the chain of
 // loads a value costs, some 6 K cycles, and two barriers an iteration.
@@ -2232,7 +2232,7 @@ static bool run_rows(xlb_ctx* c, DeltaLoop& d, const Rules& rs, uint64_t max_ite
     sh.words = 1u << (d.lo_bits - 5);
     sh.queue = rows_queue(d.lo_bits);
     // Where the seeds are the relation itself and a value has as many matches as a row has words, a level takes the
-    // values' rows and not their matches one by one (four blocks of 128 nodes, 33 M candidates: 62 us, now 20
+    // values' rows and not their matches one by one (four blocks of 128 nodes, 33 M candidates: 62 us, now 19
     // and 4 for the copy; 2000 nodes of degree 5, rows of 64 words, stay with their matches.)
     Buf lists;
     if (d.seeds_listed && d.lo_bits <= RW_LISTS_BITS && rs.r[0].rows >= std::max<uint64_t>(d.words, RW_LISTS_MIN)) {
