@@ -1,0 +1,42 @@
+"""Operations whose result fits a memory budget that their quickest route does not: they take the other one."""
+import numpy as np
+import pytest
+
+from xlog_b200 import _abi as A
+from xlog_b200.provider import KernelProvider
+
+pytestmark = pytest.mark.gpu
+
+N = 8192  # rows, the most one block takes
+
+
+def with_spare(cols, spare):
+    """A provider with these relations and `spare` more bytes."""
+    p = KernelProvider(device=0, memory_budget_bytes=sum(c.nbytes for r in cols for c in r) + spare)
+    return p, [p.create_buffer_from_slices(r) for r in cols]
+
+
+@pytest.mark.parametrize("kind", [A.JOIN_SEMI, A.JOIN_ANTI, A.JOIN_INNER])
+def test_small_joins(kind):
+    key = np.arange(N, dtype=np.uint64)
+    left = [key] + [key + np.uint64(k) for k in range(1, 6)]  # 393 KB
+    right = [np.append(key[:3], key[5:] if kind == A.JOIN_ANTI else key[:0])[:4096]]
+    left = [c[:4096] for c in left] if kind == A.JOIN_ANTI else left
+    want = [c[np.isin(left[0], right[0]) != (kind == A.JOIN_ANTI)] for c in left] + ([right[0]] if kind == A.JOIN_INNER else [])
+    assert len(want[0]) < 10
+    # (the inner join's row lists: 8 + 4 bytes a probe row)
+    p, (lb, rb) = with_spare([left, right], 160 << 10)
+    for g, w in zip(p.download(p.hash_join_v2(lb, rb, [0], [0], kind)), want):
+        assert np.array_equal(g, w)
+    p.close()
+
+
+def test_small_groups():
+    key = np.arange(N, dtype=np.uint32) % np.uint32(3)
+    v = np.arange(N, dtype=np.uint64)
+    p, (b,) = with_spare([[key, v]], 32 << 10)
+    got = p.download(p.groupby_multi_agg(b, [0], [(1, op) for op in (A.AGG_SUM, A.AGG_MIN, A.AGG_MAX, A.AGG_COUNT, A.AGG_SUM)]))  # 360 KB for all rows
+    groups = [v[key == k] for k in range(3)]
+    for g, f in zip(got[1:], (np.sum, np.min, np.max, len, np.sum)):
+        assert g.tolist() == [f(x) for x in groups]
+    p.close()

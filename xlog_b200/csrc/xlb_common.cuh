@@ -449,6 +449,9 @@ struct DevBuf {
 };
 using Buf = std::shared_ptr<DevBuf>;
 inline Buf make_buf(xlb_ctx* c, uint64_t bytes) { return std::make_shared<DevBuf>(c, bytes); }
+// Whether the budget leaves room for `bytes` more.  A route that wants more than the result and has another
+// route behind it asks first.
+inline bool within_budget(const xlb_ctx* c, uint64_t bytes) { return !c->budget || (c->allocated <= c->budget && bytes <= c->budget - c->allocated); }
 
 inline void check_launch(xlb_ctx* c, const char* what) {
     const cudaError_t launched = cudaGetLastError();  // (before anything else takes it)

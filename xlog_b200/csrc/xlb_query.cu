@@ -880,6 +880,11 @@ KeyCols key_cols(const xlb_rel* r, const uint32_t* keys, uint32_t nk) {
     return k;
 }
 int bit_length(uint64_t v) { return v ? 64 - __builtin_clzll(v) : 0; }
+uint64_t row_bytes(const xlb_schema& s) {
+    uint64_t bytes = 0;
+    for (uint32_t i = 0; i < s.arity; ++i) bytes += type_width(s.types[i]);
+    return bytes;
+}
 // out: a fresh relation of `rows` rows with the columns of `from` in place `at` and after
 void add_columns(xlb_ctx* c, xlb_rel* out, Cols& cols, const xlb_rel* from, uint64_t rows) {
     for (uint32_t i = 0; i < from->schema.arity; ++i) {
@@ -917,9 +922,10 @@ struct Sweep {
 
 }  // namespace
 
-// Whether one block takes it; the shared memory its kernels may ask for.
-static bool one_block(xlb_ctx* c, uint64_t build, uint64_t probe) {
-    if (!build || build > SMALL_BUILD || !probe || probe > SMALL_PROBE) return false;
+// Whether one block takes it; the shared memory its kernels may ask for.  Its columns have room for the most rows there
+// can be (`room` bytes); where the budget has not, the grids make them as long as the result.
+static bool one_block(xlb_ctx* c, uint64_t build, uint64_t probe, uint64_t room) {
+    if (!build || build > SMALL_BUILD || !probe || probe > SMALL_PROBE || !within_budget(c, room + 64)) return false;
     if (!c->query_attr_set) {
         CUDA_OK(cudaFuncSetAttribute(exists_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMALL_SLOTS * 8 + SMALL_PROBE * 2)));
         CUDA_OK(cudaFuncSetAttribute(join_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMALL_SLOTS * 12 + 16 + SMALL_BUILD * 2)));
@@ -936,7 +942,7 @@ static unsigned slots_of(uint64_t build) {
 
 xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, bool want) {
     if (r->rows >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)r->rows);
-    if (one_block(c, r->rows, l->rows)) {
+    if (one_block(c, r->rows, l->rows, l->rows * row_bytes(l->schema))) {
         std::unique_ptr<xlb_rel> o(new xlb_rel);
         o->ctx = c;
         o->schema = l->schema;
@@ -994,32 +1000,28 @@ xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint
 xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, const xlb_schema& os) {
     const uint64_t n = r->rows;
     if (n >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)n);
-    if (one_block(c, n, l->rows)) {
-        uint64_t row_bytes = 0;
-        for (uint32_t i = 0; i < os.arity; ++i) row_bytes += type_width(os.types[i]);
-        const uint64_t room = std::min<uint64_t>(SMALL_OUTPUTS, 4 * l->rows + 1024);
-        if (!c->budget || c->allocated + room * row_bytes + (1u << 16) <= c->budget) {
-            std::unique_ptr<xlb_rel> o(new xlb_rel);
-            o->ctx = c;
-            o->schema = os;
-            Cols cols{};
-            cols.left = (int)l->schema.arity;
-            add_columns(c, o.get(), cols, l, room);
-            add_columns(c, o.get(), cols, r, room);
-            Buf words = make_buf(c, 16);
-            prof_begin(c, "join_small", 0);
-            const Publish pub = publish_by(c, 1, words->p, 2);
-            const unsigned cap = slots_of(n);
-            join_small_k<<<1, SMALL_THREADS, cap * 12 + 16 + (unsigned)n * 2, c->stream>>>(key_cols(r, rk, nk), (unsigned)n, key_cols(l, lk, nk), (unsigned)l->rows, cols, room,
-                                                                                         words->as<unsigned long long>(), pub);
-            check_launch(c, "join_small");
-            unsigned long long w[2];
-            read_published(c, pub, words->p, 2, w);
-            if (w[1]) return nullptr;
-            if (w[0] <= room) {
-                o->rows = w[0];
-                return o.release();
-            }
+    const uint64_t room = std::min<uint64_t>(SMALL_OUTPUTS, 4 * l->rows + 1024);
+    if (one_block(c, n, l->rows, room * row_bytes(os))) {
+        std::unique_ptr<xlb_rel> o(new xlb_rel);
+        o->ctx = c;
+        o->schema = os;
+        Cols cols{};
+        cols.left = (int)l->schema.arity;
+        add_columns(c, o.get(), cols, l, room);
+        add_columns(c, o.get(), cols, r, room);
+        Buf words = make_buf(c, 16);
+        prof_begin(c, "join_small", 0);
+        const Publish pub = publish_by(c, 1, words->p, 2);
+        const unsigned cap = slots_of(n);
+        join_small_k<<<1, SMALL_THREADS, cap * 12 + 16 + (unsigned)n * 2, c->stream>>>(key_cols(r, rk, nk), (unsigned)n, key_cols(l, lk, nk), (unsigned)l->rows, cols, room,
+                                                                                     words->as<unsigned long long>(), pub);
+        check_launch(c, "join_small");
+        unsigned long long w[2];
+        read_published(c, pub, words->p, 2, w);
+        if (w[1]) return nullptr;
+        if (w[0] <= room) {
+            o->rows = w[0];
+            return o.release();
         }
     }
     uint64_t cap = 1024;
@@ -1116,7 +1118,7 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
     };
     Buf words = make_buf(c, 24);  // [0] key bound, [1] groups, [2] rows of the largest
     unsigned long long w[2];
-    const bool small = one_block(c, 1, n);
+    const bool small = one_block(c, 1, n, n * row_bytes(os));
     if (small) {
         results(n);
         prof_begin(c, "group_small", 0);
@@ -1129,6 +1131,7 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
             o->rows = w[1];
             return o.release();
         }
+        for (uint32_t i = 0; i < os.arity; ++i) o->cols[i].reset();
     }
     CUDA_OK(set_async(c, words->p, 0, 24));
     if (!small) {
