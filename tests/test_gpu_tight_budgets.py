@@ -40,3 +40,20 @@ def test_small_groups():
     for g, f in zip(got[1:], (np.sum, np.min, np.max, len, np.sum)):
         assert g.tolist() == [f(x) for x in groups]
     p.close()
+
+
+def test_large_sets_come_back():
+    # the first column as runs needs a few KB on the device: without them all columns are copied
+    n, budget = 2_200_000, 256 << 20
+    cols = [np.repeat(np.arange(n // 1000, dtype=np.uint32), 1000), np.arange(n, dtype=np.uint32)]
+    p = KernelProvider(device=0, memory_budget_bytes=budget)
+    rel = p.dedup(p.create_buffer_from_slices(cols))
+    assert rel.is_canonical()
+    for full in (False, True):
+        if full:
+            filler = p.create_buffer_from_slices([np.zeros((budget - p.memory_stats()[0] - 256) // 8, dtype=np.uint64)])
+            assert budget - p.memory_stats()[0] < 512
+        for g, c in zip(p.download(rel), cols):
+            assert np.array_equal(g, c)
+    del filler
+    p.close()

@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <atomic>
 #include <exception>
+#include <optional>
 #include <thread>
 #include <vector>
 
@@ -213,14 +214,22 @@ bool page_locked(const void* p) {
 
 template <class T>
 constexpr uint64_t runs_room() { return (STAGE_BYTES - 16) / sizeof(Run<T>); }
+// False: what it needs is not to be had (device memory within the budget, the staging, a stream); nothing was done.
 template <class T>
-void fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n, unsigned threads) {
+bool fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n, unsigned threads) {
     const uint64_t tiles = (n + RUNS_TILE - 1) / RUNS_TILE, cap = runs_room<T>();
-    char* stage = stage_buffer(c);
+    char* stage;
+    Buf counts;
+    std::optional<SideCopies> side;
+    try {
+        stage = stage_buffer(c);
+        counts = make_buf(c, tiles * 4);
+        side.emplace(c);
+    } catch (const XlbError&) {
+        return false;
+    }
     unsigned long long* total = reinterpret_cast<unsigned long long*>(stage);
     const Run<T>* runs = reinterpret_cast<const Run<T>*>(stage + 16);
-    Buf counts = make_buf(c, tiles * 4);
-    SideCopies side(c);
     const T* col = r->cols[0]->as<T>();
     prof_begin(c, "to_host", n * sizeof(T));
     runs_count_k<T><<<(unsigned)tiles, BLOCK, 0, c->stream>>>(col, n, counts->as<unsigned>());
@@ -228,14 +237,15 @@ void fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n
     prof_begin(c, "to_host", n * sizeof(T));
     runs_write_k<T><<<(unsigned)tiles, BLOCK, 0, c->stream>>>(col, n, counts->as<unsigned>(), reinterpret_cast<Run<T>*>(c->h_stage_dev + 16), cap, reinterpret_cast<unsigned long long*>(c->h_stage_dev));
     check_launch(c, "to_host");
-    for (uint32_t i = 1; i < r->schema.arity; ++i) side.add(cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]));
+    for (uint32_t i = 1; i < r->schema.arity; ++i) side->add(cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]));
     {
         Filler<T> filler(threads);
         stream_wait(c);
         if (*total > cap) xlb_fail(XLB_ERR_CUDA, "internal: %llu runs of at most %llu values", *total, (unsigned long long)r->firsts);
         filler.fill(static_cast<T*>(cols[0]), runs, *total, n);
     }
-    side.wait();
+    side->wait();
+    return true;
 }
 
 }  // namespace
@@ -253,8 +263,7 @@ void ops_fetch_columns(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t
         bool locked = cores >= RUNS_CORES_MIN;
         for (uint32_t i = 0; i < arity; ++i) locked = locked && page_locked(cols[i]) && (uintptr_t)cols[i] % width == 0;
         const unsigned threads = (unsigned)std::min<uint64_t>({RUNS_THREADS_MAX, cores / 2, n * width / RUNS_THREAD_BYTES});
-        if (locked && width == 4) return fetch_with_runs<uint32_t>(c, r, cols, n, threads);
-        if (locked) return fetch_with_runs<unsigned long long>(c, r, cols, n, threads);
+        if (locked && (width == 4 ? fetch_with_runs<uint32_t>(c, r, cols, n, threads) : fetch_with_runs<unsigned long long>(c, r, cols, n, threads))) return;
     }
     for (uint32_t i = 0; i < arity; ++i) CUDA_OK(copy_async(c, cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost));
     CUDA_OK(cudaStreamSynchronize(c->stream));

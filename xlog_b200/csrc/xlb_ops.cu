@@ -1303,8 +1303,13 @@ extern "C" xlb_status xlb_rel_is_canonical(const xlb_rel* r, int* canonical) {
 
 char* stage_buffer(xlb_ctx* c) {
     if (!c->h_stage) {
-        CUDA_OK(cudaHostAlloc((void**)&c->h_stage, STAGE_BYTES, cudaHostAllocMapped));
-        CUDA_OK(cudaHostGetDevicePointer((void**)&c->h_stage_dev, c->h_stage, 0));
+        char *p = nullptr, *dev = nullptr;
+        CUDA_OK(cudaHostAlloc((void**)&p, STAGE_BYTES, cudaHostAllocMapped));
+        const cudaError_t e = cuda_take(cudaHostGetDevicePointer((void**)&dev, p, 0));
+        if (e != cudaSuccess) CUDA_QUIET(cudaFreeHost(p));
+        CUDA_OK(e);
+        c->h_stage = p;
+        c->h_stage_dev = dev;
     }
     return c->h_stage;
 }
