@@ -8,6 +8,7 @@ from xlog_b200.provider import KernelProvider
 pytestmark = pytest.mark.gpu
 
 N = 8192  # rows, the most one block takes
+REST = 16 << 10  # bytes a column may hold beyond its rows
 
 
 def with_spare(cols, spare):
@@ -56,4 +57,27 @@ def test_large_sets_come_back():
         for g, c in zip(p.download(rel), cols):
             assert np.array_equal(g, c)
     del filler
+    p.close()
+
+
+@pytest.mark.parametrize("rows", [0, 1, 130, 4096])
+def test_small_results_keep_what_they_need(rows):
+    probe = [np.arange(N, dtype=np.uint32), np.arange(N, dtype=np.uint64), np.zeros(N, dtype=np.float32)]
+    build = [np.arange(N - rows, 2 * N - rows, dtype=np.uint32)[:4096], np.arange(4096, dtype=np.uint32)]
+    p = KernelProvider(device=0)
+    lb, rb = p.create_buffer_from_slices(probe), p.create_buffer_from_slices(build)
+    for kind, width in ((A.JOIN_SEMI, 16), (A.JOIN_ANTI, 16), (A.JOIN_INNER, 24)):
+        before = p.memory_stats()[0]
+        out = p.hash_join_v2(lb, rb, [0], [0], kind)
+        assert out.num_rows() == (N - rows if kind == A.JOIN_ANTI else rows)
+        assert width * out.num_rows() <= p.memory_stats()[0] - before <= width * out.num_rows() + 5 * REST
+        again = p.hash_join_v2(lb, rb, [0], [0], kind)  # (in what the first did not keep)
+        for g, w in zip(p.download(out), p.download(again)):
+            assert np.array_equal(g, w)
+        del out, again
+    before = p.memory_stats()[0]
+    g = p.create_buffer_from_slices([np.arange(N, dtype=np.uint32) % np.uint32(max(rows, 1)), probe[1]])
+    own = p.memory_stats()[0] - before
+    out = p.groupby_multi_agg(g, [0], [(1, A.AGG_SUM)])
+    assert out.num_rows() == max(rows, 1) and 0 <= p.memory_stats()[0] - before - own - 12 * out.num_rows() <= 2 * REST
     p.close()

@@ -444,6 +444,15 @@ struct DevBuf {
     }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
+    // Only the first n bytes are kept; the others are free for later work on the stream.
+    void keep(uint64_t n) {
+        if (!p || n >= bytes) return;
+        const uint64_t held = Arena::round_up(n);
+        if (held < bytes) ctx->arena.release((char*)p + held, bytes - held);
+        ctx->allocated -= bytes - n;
+        bytes = n;
+        if (!n) p = nullptr;
+    }
     template <class T>
     T* as() const { return (T*)p; }
 };

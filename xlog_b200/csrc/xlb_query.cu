@@ -895,6 +895,17 @@ void add_columns(xlb_ctx* c, xlb_rel* out, Cols& cols, const xlb_rel* from, uint
         cols.out[k] = out->cols[k]->p;
     }
 }
+// A relation whose columns had room for more rows than there are.  Giving a rest back costs 0.2 us, and as much when the
+// relation goes (semi join, inner join and group-by of 3001 facts 87 us, 90 with every rest): only those worth it.
+constexpr uint64_t REST_KEPT = 16u << 10;  // bytes a column
+xlb_rel* with_rows(std::unique_ptr<xlb_rel>& o, uint64_t rows) {
+    o->rows = rows;
+    for (uint32_t i = 0; i < o->schema.arity; ++i) {
+        const uint64_t bytes = rows * type_width(o->schema.types[i]);
+        if (o->cols[i]->bytes - bytes > REST_KEPT) o->cols[i]->keep(bytes);
+    }
+    return o.release();
+}
 
 // The sums before each tile of a kernel that calls leave_tile: the kernel's own doing, or by a scan after it.
 struct Sweep {
@@ -956,8 +967,7 @@ xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint
         check_launch(c, "exists_small");
         unsigned long long m;
         read_published(c, pub, total->p, 1, &m);
-        o->rows = m;
-        return o.release();
+        return with_rows(o, m);
     }
     uint64_t cap = 1024;
     while (cap < 2 * r->rows) cap <<= 1;
@@ -1019,10 +1029,7 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
         unsigned long long w[2];
         read_published(c, pub, words->p, 2, w);
         if (w[1]) return nullptr;
-        if (w[0] <= room) {
-            o->rows = w[0];
-            return o.release();
-        }
+        if (w[0] <= room) return with_rows(o, w[0]);
     }
     uint64_t cap = 1024;
     while (cap < 2 * n) cap <<= 1;
@@ -1127,10 +1134,7 @@ xlb_rel* query_groupby(xlb_ctx* c, const xlb_rel* in, const uint32_t* key_cols_i
                                                                          words->as<unsigned long long>(), pub);
         check_launch(c, "group_small");
         read_published(c, pub, words->p, 2, w);
-        if (w[1] != ~0ull) {
-            o->rows = w[1];
-            return o.release();
-        }
+        if (w[1] != ~0ull) return with_rows(o, w[1]);
         for (uint32_t i = 0; i < os.arity; ++i) o->cols[i].reset();
     }
     CUDA_OK(set_async(c, words->p, 0, 24));
