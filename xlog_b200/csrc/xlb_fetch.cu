@@ -9,18 +9,11 @@
 // and ordinary stores, which read what they overwrite, took 2.6.
 //   The column is read twice on the device (heads counted per tile, then written in order), while the copy of
 // the next column runs on a stream of its own.
-#if defined(__SSE2__)
-#include <emmintrin.h>
-#endif
-
 #include <algorithm>
-#include <atomic>
-#include <exception>
 #include <optional>
-#include <thread>
-#include <vector>
 
 #include "xlb_common.cuh"
+#include "xlb_fill.h"
 #include "xlb_host.h"
 #include "xlb_kernels.cuh"
 #include "xlb_ops.h"
@@ -33,13 +26,8 @@ constexpr uint64_t RUNS_TILE = 4096;                     // rows a block looks a
 constexpr uint64_t RUNS_MIN_BYTES = 6ull << 20;          // below, the 60 us until the runs are there and 11 us a thread are hardly made up for (4 MB: 73 us of bus)
 constexpr uint64_t RUNS_THREAD_BYTES = 3ull << 19;       // of the column, per thread
 constexpr unsigned RUNS_THREADS_MAX = 4, RUNS_CORES_MIN = 4;
-constexpr uint64_t RUNS_CHUNK = 256ull << 10;            // bytes a thread takes at a time
 constexpr uint64_t RUNS_ROWS_MIN = 64;                   // rows a run has to have on average: a run is a few dozen ns of its own
 
-template <class T>
-struct Run {
-    T row, value;
-};
 template <class T>
 __device__ __forceinline__ unsigned warp_heads(const T* __restrict__ col, uint64_t n, uint64_t base, int k) {
     const uint64_t i = base + k * 32 + lane_id();
@@ -107,90 +95,6 @@ __global__ void __launch_bounds__(BLOCK) runs_write_k(const T* __restrict__ col,
         before += __popc(heads[k]);
     }
 }
-
-// Rows [lo, hi) of the column, a cache line at a time.  A line that runs meet in is put together first: written
-// in parts, some of them around the cache, it cost 0.3 us.
-template <class T>
-void fill_rows(T* to, const Run<T>* runs, uint64_t n_runs, uint64_t n, uint64_t lo, uint64_t hi) {
-    constexpr uint64_t line = 64 / sizeof(T);
-    uint64_t r = std::upper_bound(runs, runs + n_runs, lo, [](uint64_t row, const Run<T>& x) { return row < x.row; }) - runs - 1;
-    const auto end_of = [&](uint64_t run) { return run + 1 < n_runs ? (uint64_t)runs[run + 1].row : n; };
-    uint64_t end = end_of(r);
-    for (uint64_t at = lo; at < hi;) {
-        alignas(64) T buf[line];
-        const bool whole = (uintptr_t)(to + at) % 64 == 0 && hi - at >= line;
-        const uint64_t m = whole ? line : 1;
-        for (uint64_t k = 0; k < m; ++k) {
-            while (at + k >= end) end = end_of(++r);
-            buf[k] = runs[r].value;
-        }
-        if (!whole) {
-            to[at++] = buf[0];
-            continue;
-        }
-        // this line, and those behind it that lie in the run it ends with
-        const uint64_t lines = end >= at + 2 * line ? (std::min(end, hi) - at) / line : 1;
-#if defined(__SSE2__)
-        __m128i v[4];
-        for (int k = 0; k < 4; ++k) v[k] = _mm_load_si128(reinterpret_cast<const __m128i*>(buf) + k);
-        __m128i* out = reinterpret_cast<__m128i*>(to + at);
-        for (int k = 0; k < 4; ++k) _mm_stream_si128(out + k, v[k]);
-        v[0] = v[1] = v[2] = v[3] = sizeof(T) == 4 ? _mm_set1_epi32((int)buf[line - 1]) : _mm_set1_epi64x((long long)buf[line - 1]);
-        for (out += 4; out < reinterpret_cast<__m128i*>(to + at) + 4 * lines; out += 4)
-            for (int k = 0; k < 4; ++k) _mm_stream_si128(out + k, v[k]);
-#else
-        std::copy(buf, buf + line, to + at);
-        std::fill(to + at + line, to + at + lines * line, buf[line - 1]);
-#endif
-        at += lines * line;
-    }
-#if defined(__SSE2__)
-    _mm_sfence();
-#endif
-}
-// Threads that write a column out.  They are started (11 us each) while the runs are on their way, and wait for them
-// a little before they begin; without any to be had the caller does all of it.
-template <class T>
-class Filler {
-    enum { WAIT, FILL, LEAVE };
-    std::atomic<int> go{WAIT};
-    std::atomic<uint64_t> next{0};
-    T* to = nullptr;
-    const Run<T>* runs = nullptr;
-    uint64_t n_runs = 0, n = 0;
-    std::vector<std::thread> helpers;
-
-    void work() {
-        constexpr uint64_t rows = RUNS_CHUNK / sizeof(T);
-        for (uint64_t at; (at = next.fetch_add(rows, std::memory_order_relaxed)) < n;) fill_rows(to, runs, n_runs, n, at, std::min(n, at + rows));
-    }
-
-   public:
-    explicit Filler(unsigned threads) {
-        try {
-            helpers.reserve(threads);
-            for (unsigned t = 1; t < threads; ++t)
-                helpers.emplace_back([this] {
-                    while (go.load(std::memory_order_acquire) == WAIT) std::this_thread::yield();
-                    if (go.load(std::memory_order_acquire) == FILL) work();
-                });
-        } catch (const std::exception&) {  // no thread (or memory for one) to be had
-        }
-    }
-    void fill(T* column, const Run<T>* r, uint64_t count, uint64_t rows) {
-        to = column;
-        runs = r;
-        n_runs = count;
-        n = rows;
-        go.store(FILL, std::memory_order_release);
-        work();
-    }
-    ~Filler() {
-        int still = WAIT;
-        go.compare_exchange_strong(still, LEAVE, std::memory_order_release, std::memory_order_relaxed);
-        for (auto& t : helpers) t.join();
-    }
-};
 
 // Copies that run beside the context's stream, behind what is on it now.  However the operation ends, they are
 // over before it returns: the memory they write is the caller's.
