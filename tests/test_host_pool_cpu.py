@@ -26,6 +26,8 @@ extern "C" int device_here() { return fake_device; }
 extern "C" void device_is(int d) { fake_device = d; }
 extern "C" void registration_takes(int ms) { fake.register_ms = ms; }
 extern "C" uint64_t most() { return host_pool_most(); }
+extern "C" unsigned cores() { return host_pool_cores(); }
+extern "C" unsigned quota(const char* groups, const char* mount) { return host_cores_quota(groups, mount); }
 extern "C" void ranks(unsigned n) { host_pool_ranks(n); }
 extern "C" void fail(int r, int u) { fake.fail_register = r; fake.fail_unregister = u; }
 """, "xlb_host.cu")
@@ -135,3 +137,30 @@ def test_without_a_context_the_thread_decides(pool):
     assert pool.last_device() == 3
     pool.xlb_host_free(p)
     assert pool.registered() == 0 and pool.touched_devices() == 1 << 3
+
+
+@pytest.mark.parametrize("groups,files,cores", [
+    ("0::/\n", {}, 0),
+    ("0::/\n", {"cpu.max": "max 100000"}, 0),
+    ("0::/\n", {"cpu.max": "350000 100000"}, 3),
+    ("0::/\n", {"cpu.max": "50000 100000"}, 1),
+    ("0::/a/b\n", {"a/b/cpu.max": "max 100000", "a/cpu.max": "200000 100000", "cpu.max": "900000 100000"}, 2),
+    ("3:cpuset:/x\n2:cpuacct,cpu:/x\n1:memory:/x\n", {"cpu/x/cpu.cfs_quota_us": "400000", "cpu/x/cpu.cfs_period_us": "100000"}, 4),
+    ("2:cpu:/x\n0::/\n", {"cpu/x/cpu.cfs_quota_us": "-1", "cpu/x/cpu.cfs_period_us": "100000", "cpu/cpu.cfs_quota_us": "-1"}, 0),
+    ("nonsense\n\n4:\n0::\n", {"cpu.max": "oops"}, 0),
+])
+def test_cores_under_a_quota(pool, tmp_path, groups, files, cores):
+    (tmp_path / "cgroup").write_text(groups)
+    for name, text in files.items():
+        f = tmp_path / "mount" / name
+        f.parent.mkdir(parents=True, exist_ok=True)
+        f.write_text(text + "\n")
+    assert pool.quota(str(tmp_path / "cgroup").encode(), str(tmp_path / "mount").encode()) == cores
+    assert pool.quota(b"/nowhere", b"/nowhere") == 0
+
+
+def test_cores_of_this_process(pool, monkeypatch):
+    cores = pool.cores()
+    assert 1 <= cores <= len(os.sched_getaffinity(0))
+    monkeypatch.setenv("LOCAL_WORLD_SIZE", "2")
+    assert pool.cores() == cores // 2

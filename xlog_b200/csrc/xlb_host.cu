@@ -20,9 +20,11 @@
 #include <algorithm>
 #include <cstdlib>
 #include <exception>
+#include <fstream>
 #include <list>
 #include <mutex>
 #include <new>
+#include <string>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -221,9 +223,38 @@ uint64_t host_pool_most() {
     return pool().most();
 }
 
+// What the control groups of this process, and those above them, allow it of the cores (0: no bound is set).  `groups` is
+// /proc/self/cgroup, `mount` where the groups' files are; version 2 has one tree, version 1 one for the processor.
+unsigned host_cores_quota(const char* groups, const char* mount) {
+    double least = 0;
+    std::ifstream lines(groups);
+    for (std::string line; std::getline(lines, line);) {
+        const size_t a = line.find(':'), b = a == std::string::npos ? a : line.find(':', a + 1);
+        if (b == std::string::npos) continue;
+        const std::string kinds = "," + line.substr(a + 1, b - a - 1) + ",";
+        const bool v2 = kinds == ",,";
+        if (!v2 && kinds.find(",cpu,") == std::string::npos) continue;
+        for (std::string path = line.substr(b + 1);; path.erase(path.find_last_of('/'))) {
+            if (path == "/") path.clear();
+            double quota = 0, period = 0;
+            const std::string at = std::string(mount) + (v2 ? "" : "/cpu") + path;
+            if (v2) std::ifstream(at + "/cpu.max") >> quota >> period;  // ("max": no number, none set)
+            else {
+                std::ifstream(at + "/cpu.cfs_quota_us") >> quota;  // (-1: none set)
+                std::ifstream(at + "/cpu.cfs_period_us") >> period;
+            }
+            if (quota > 0 && period > 0 && (least == 0 || quota / period < least)) least = quota / period;
+            if (path.empty() || path.find('/') == std::string::npos) break;
+        }
+    }
+    return least > 0 ? std::max(1u, (unsigned)std::min(least, 1e6)) : 0;
+}
+
 unsigned host_pool_cores() {
+    static const unsigned quota = host_cores_quota("/proc/self/cgroup", "/sys/fs/cgroup");
+    const unsigned cores = std::thread::hardware_concurrency();
     std::lock_guard<std::mutex> g(pool().mu);
-    return std::thread::hardware_concurrency() / (unsigned)pool().sharers();
+    return (quota ? std::min(quota, cores) : cores) / (unsigned)pool().sharers();
 }
 
 extern "C" xlb_status xlb_host_alloc(uint64_t bytes, void** out) {
