@@ -159,3 +159,21 @@ def test_groups_of_one_block(p, n, top, nk):
     want = [k[first] for k in s[:nk]] + [np.diff(np.append(first, n)), np.add.reduceat(s[nk].astype(np.uint64), first), np.minimum.reduceat(s[nk + 1], first)]
     for g, w in zip(got, want):
         assert np.array_equal(g.astype(np.uint64), w.astype(np.uint64))
+
+
+# rows of one key next to each other in a warp, alone in it, all of them, in a warp that is not full
+@pytest.mark.parametrize("n", [1, 3, 31, 33, 1000, 1025, 8191, 8192])
+@pytest.mark.parametrize("kind", ["one", "two", "ten", "hub", "runs", "all", "late"])
+def test_few_groups_of_one_block(p, n, kind):
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    key = {"one": i * 0, "two": rng.integers(0, 2, n), "ten": rng.integers(0, 10, n), "hub": np.where(rng.integers(0, 10, n), 777, rng.integers(0, 4096, n)), "runs": i // 5, "all": i,
+           "late": np.where(i % 32 > 27, 5, i % 32)}[kind].astype(np.uint32)
+    cols = [key, rng.integers(0, 1 << 32, n, dtype=np.uint32), rng.integers(1 << 63, 1 << 64, n, dtype=np.uint64, endpoint=False)]
+    got = p.download(p.groupby_multi_agg(p.create_buffer_from_slices(cols), [0], [(1, A.AGG_SUM), (2, A.AGG_MAX), (1, A.AGG_COUNT), (2, A.AGG_MIN), (2, A.AGG_SUM)][: 5 if kind != "all" else 2]))
+    order = np.argsort(key, kind="stable")
+    u, at = np.unique(key[order], return_index=True)
+    v, w = cols[1][order].astype(np.uint64), cols[2][order]
+    want = [u, np.add.reduceat(v, at), np.maximum.reduceat(w, at), np.diff(np.append(at, n)).astype(np.uint64), np.minimum.reduceat(w, at), np.add.reduceat(w, at)]
+    for g, x in zip(got, want):
+        assert np.array_equal(g.astype(np.uint64), x.astype(np.uint64))
