@@ -177,3 +177,17 @@ def test_few_groups_of_one_block(p, n, kind):
     want = [u, np.add.reduceat(v, at), np.maximum.reduceat(w, at), np.diff(np.append(at, n)).astype(np.uint64), np.minimum.reduceat(w, at), np.add.reduceat(w, at)]
     for g, x in zip(got, want):
         assert np.array_equal(g.astype(np.uint64), x.astype(np.uint64))
+
+
+# Groups of a key and outputs beyond the room that one block's columns have, up to and past the longest group; key 0 among them
+@pytest.mark.parametrize("npr,nb,keys", [(100, 100, 2), (300, 300, 10), (1025, 64, 1), (1100, 4096, 64), (8192, 4096, 64), (8192, 4000, 400), (8192, 64, 1), (18, 4096, 64), (8191, 129, 2), (8191, 130, 2), (1, 4096, 1), (100, 256, 1), (100, 257, 1), (500, 4096, 300), (500, 3600, 300), (500, 3900, 300), (8192, 3840, 15)])
+@pytest.mark.parametrize("dtype", [np.uint32, np.uint64])
+def test_more_outputs_than_one_block_has_room_for(p, npr, nb, keys, dtype):
+    rng = np.random.default_rng(npr + nb)
+    left = [rng.integers(0, keys + 1, npr).astype(dtype), np.arange(npr, dtype=np.uint64)]
+    right = [np.arange(nb, dtype=np.float32), (rng.permutation(nb) % keys).astype(dtype)]
+    lb, rb = p.create_buffer_from_slices(left), p.create_buffer_from_slices(right)
+    l, r = inner(left[0], right[1])
+    for _ in range(2):
+        for g, w in zip(p.download(p.hash_join_v2(lb, rb, [0], [1])), [c[l] for c in left] + [c[r] for c in right]):
+            assert np.array_equal(g, w)

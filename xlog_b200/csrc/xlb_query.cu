@@ -502,7 +502,9 @@ __global__ void __launch_bounds__(BLOCK) join_chains_k(const uint64_t* __restric
 // 12 000, with the smaller operations still by one block, 150 against 190, 20 000 177 against 203).
 constexpr unsigned SMALL_THREADS = 1024, SMALL_IPT = 8, SMALL_PROBE = SMALL_THREADS * SMALL_IPT, SMALL_BUILD = 4096;
 constexpr unsigned SMALL_SLOTS = 2 * SMALL_BUILD;  // (half of them stay free)
-constexpr uint64_t SMALL_OUTPUTS = 4 * SMALL_PROBE;  // of a join
+constexpr unsigned SMALL_CHAIN = 12;   // rows of a key up to which a thread puts them in order by itself (groups of 20: 98 us, ranked row by row 45; by grids 75)
+constexpr unsigned SMALL_GROUP = 256;  // rows of a key, at most: each is ranked among the others
+constexpr uint64_t SMALL_OUTPUTS = 3 * SMALL_PROBE / 2;  // of a join; more go out by a grid
 constexpr unsigned SMALL_GROUPS_BYTES = 160u << 10;
 constexpr unsigned GROUP_PEERS = 4;  // lanes of one key from which a warp puts their values together first ...
 constexpr unsigned GROUP_HUB = 256;  // ... where some group has more rows than this (looking for them costs 7 us for 8192 rows; 30 groups of 273: 38 us either way)
@@ -592,81 +594,130 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) exists_small_k(KeyCols keys,
     if (threadIdx.x == 0) *total = m;
     publish_now(pub);
 }
-// words: outputs, whether a group is too long.  More outputs than there is room for are only counted.
-__global__ void __launch_bounds__(SMALL_THREADS, 1) join_small_k(KeyCols keys, unsigned build, KeyCols probe, unsigned n, Cols cols, uint64_t room, unsigned long long* words, const Publish pub) {
+// What is left for join_emit_k where there are more outputs than room or a key has many rows, so that the grids need
+// not find it out again (8000 probe rows, 80 000 outputs: 98 us when they did, 66 without the attempt, 45 now; 32 000
+// written by the one block 82 to 96, now 44; 100 rows of one key on either side 107, by a sort of all, now 36).  Per probe row, the outputs before it, its group and the group's start ...
+struct SmallLists {
+    uint64_t* match;
+    uint32_t *before, *start;
+    uint64_t* tile;  // (nothing: `before` counts from the first row)
+    uint32_t* rows;  // ... in the build rows by group
+};
+// words: outputs; what became of them: 0 written, 1 listed, 2 nothing, as a group is too long.
+__global__ void __launch_bounds__(SMALL_THREADS, 1) join_small_k(KeyCols keys, unsigned build, KeyCols probe, unsigned n, Cols cols, uint64_t room, SmallLists lists, unsigned long long* words,
+                                                               const Publish pub) {
     extern __shared__ unsigned long long small_s[];
-    __shared__ unsigned warp_s[SMALL_IPT * 32 + 1], long_s;
+    __shared__ unsigned warp_s[SMALL_IPT * 32 + 1], long_s, too_long_s;
     const unsigned cap = small_slots(build), mask = cap - 1;
-    unsigned* entry = reinterpret_cast<unsigned*>(small_s + cap);  // rows | first row (plus one) << 16, of the key 0 behind the others
-    unsigned short* after = reinterpret_cast<unsigned short*>(entry + cap + 1);
+    unsigned* count = reinterpret_cast<unsigned*>(small_s + cap);  // rows of a slot's key (of the key 0: behind the others) ...
+    unsigned* chain = count + cap + 1;                             // ... the first of them, plus one
+    unsigned short* after = reinterpret_cast<unsigned short*>(chain + cap + 1);
     uint64_t key[SMALL_IPT];
 #pragma unroll
     for (unsigned r = 0; r < SMALL_IPT; ++r) key[r] = r * SMALL_THREADS + threadIdx.x < n ? probe(r * SMALL_THREADS + threadIdx.x) : 0;
     for (unsigned h = threadIdx.x; h <= cap; h += SMALL_THREADS) {
         if (h < cap) small_s[h] = 0;
-        entry[h] = 0;
+        count[h] = chain[h] = 0;
     }
-    if (threadIdx.x == 0) long_s = 0;
+    if (threadIdx.x == 0) long_s = too_long_s = 0;
     __syncthreads();
     for (unsigned i = threadIdx.x; i < build; i += SMALL_THREADS) {
         const uint64_t k = keys(i);
         const unsigned h = k ? small_claim(small_s, mask, k) : cap;
-        unsigned cur = entry[h];
-        for (;;) {
-            if ((cur & 0xFFFF) >= JOIN_GROUP_MAX) {
-                long_s = 1;
-                break;
-            }
-            after[i] = (unsigned short)(cur >> 16);
-            const unsigned was = atomicCAS(&entry[h], cur, ((i + 1) << 16) | ((cur & 0xFFFF) + 1));
-            if (was == cur) break;
-            cur = was;
-        }
+        // (both by one native atomic each: a compare-and-swap of both together cost 40 us where all rows have one key)
+        const unsigned number = atomicAdd(&count[h], 1u);
+        if (number >= SMALL_CHAIN) long_s = 1;
+        if (number >= SMALL_GROUP) too_long_s = 1;
+        if (number < SMALL_GROUP) after[i] = (unsigned short)atomicExch(&chain[h], i + 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) words[1] = long_s;
-    if (long_s) {
+    if (too_long_s) {
+        if (threadIdx.x == 0) words[1] = 2;
         publish_now(pub);
         return;
     }
-    for (unsigned h = threadIdx.x; h <= cap; h += SMALL_THREADS) {  // chains put in row order
-        const unsigned e = entry[h];
-        if ((e & 0xFFFF) < 2) continue;
-        unsigned sorted = 0;
-        for (unsigned x = e >> 16; x;) {
-            const unsigned next = after[x - 1];
-            if (!sorted || sorted > x) {
-                after[x - 1] = (unsigned short)sorted;
-                sorted = x;
-            } else {
-                unsigned p = sorted;
-                while (after[p - 1] && after[p - 1] < x) p = after[p - 1];
-                after[x - 1] = after[p - 1];
-                after[p - 1] = (unsigned short)x;
-            }
-            x = next;
-        }
-        entry[h] = (sorted << 16) | (e & 0xFFFF);
-    }
-    __syncthreads();
-    unsigned at[SMALL_IPT], first[SMALL_IPT];
+    constexpr unsigned NONE = ~0u;
+    unsigned at[SMALL_IPT], slot[SMALL_IPT];
 #pragma unroll
     for (unsigned r = 0; r < SMALL_IPT; ++r) {
-        unsigned e = 0;
+        slot[r] = NONE;
         if (key[r]) {
             unsigned h = (unsigned)mix64(key[r]) & mask;
             while (small_s[h] && small_s[h] != key[r]) h = (h + 1) & mask;
-            if (small_s[h]) e = entry[h];
-        } else if (r * SMALL_THREADS + threadIdx.x < n) e = entry[cap];
-        at[r] = e & 0xFFFF;
-        first[r] = e >> 16;
+            if (small_s[h]) slot[r] = h;
+        } else if (r * SMALL_THREADS + threadIdx.x < n) slot[r] = cap;
+        at[r] = slot[r] != NONE ? count[slot[r]] : 0u;
     }
     const unsigned m = rounds_before(at, warp_s);
-    if (m <= room)
+    const bool listed = m > room || long_s;
+    if (!listed) {
+        for (unsigned h = threadIdx.x; h <= cap; h += SMALL_THREADS) {  // chains put in row order
+            if (count[h] < 2) continue;
+            unsigned sorted = 0;
+            for (unsigned x = chain[h]; x;) {
+                const unsigned next = after[x - 1];
+                if (!sorted || sorted > x) {
+                    after[x - 1] = (unsigned short)sorted;
+                    sorted = x;
+                } else {
+                    unsigned p = sorted;
+                    while (after[p - 1] && after[p - 1] < x) p = after[p - 1];
+                    after[x - 1] = after[p - 1];
+                    after[p - 1] = (unsigned short)x;
+                }
+                x = next;
+            }
+            chain[h] = sorted;
+        }
+        __syncthreads();
 #pragma unroll
         for (unsigned r = 0; r < SMALL_IPT; ++r)
-            for (unsigned x = first[r], to = at[r]; x; x = after[x - 1], ++to) copy_row(cols, r * SMALL_THREADS + threadIdx.x, x - 1, to);
-    if (threadIdx.x == 0) words[0] = m;
+            for (unsigned x = slot[r] != NONE ? chain[slot[r]] : 0u, to = at[r]; x; x = after[x - 1], ++to) copy_row(cols, r * SMALL_THREADS + threadIdx.x, x - 1, to);
+    } else {
+        unsigned start[SMALL_IPT];  // of each slot's rows
+        static_assert(SMALL_SLOTS <= SMALL_PROBE, "rounds of slots");
+        __syncthreads();  // (warp_s)
+#pragma unroll
+        for (unsigned r = 0; r < SMALL_IPT; ++r) start[r] = r * SMALL_THREADS + threadIdx.x < cap ? count[r * SMALL_THREADS + threadIdx.x] : 0u;
+        const unsigned others = rounds_before(start, warp_s);
+        unsigned rank[SMALL_BUILD / SMALL_THREADS], in[SMALL_BUILD / SMALL_THREADS];
+#pragma unroll
+        for (unsigned r = 0; r < SMALL_BUILD / SMALL_THREADS; ++r) {  // of each build row in its chain
+            const unsigned i = r * SMALL_THREADS + threadIdx.x;
+            in[r] = NONE;
+            rank[r] = 0;
+            if (i >= build) continue;
+            const uint64_t k = keys(i);
+            unsigned h = cap;
+            if (k)
+                for (h = (unsigned)mix64(k) & mask; small_s[h] != k;) h = (h + 1) & mask;
+            in[r] = h;
+            for (unsigned x = chain[h]; x; x = after[x - 1]) rank[r] += x - 1 < i;
+        }
+        __syncthreads();
+        unsigned* starts = reinterpret_cast<unsigned*>(small_s);  // (the keys have been looked up)
+#pragma unroll
+        for (unsigned r = 0; r < SMALL_IPT; ++r)
+            if (r * SMALL_THREADS + threadIdx.x < cap) starts[r * SMALL_THREADS + threadIdx.x] = start[r];
+        if (threadIdx.x == 0) starts[cap] = others;
+        __syncthreads();
+#pragma unroll
+        for (unsigned r = 0; r < SMALL_BUILD / SMALL_THREADS; ++r)
+            if (in[r] != NONE) lists.rows[starts[in[r]] + rank[r]] = r * SMALL_THREADS + threadIdx.x;
+#pragma unroll
+        for (unsigned r = 0; r < SMALL_IPT; ++r) {
+            const unsigned i = r * SMALL_THREADS + threadIdx.x;
+            if (i >= n) break;
+            lists.match[i] = ((uint64_t)(i + 1) << 32) | (slot[r] != NONE ? count[slot[r]] : 0u);
+            lists.before[i] = at[r];
+            lists.start[i] = slot[r] != NONE ? starts[slot[r]] : 0u;
+            if (i % SCAN_TILE == 0) lists.tile[i / SCAN_TILE] = 0;
+        }
+    }
+    if (threadIdx.x == 0) {
+        words[0] = m;
+        words[1] = listed;
+    }
     publish_now(pub);
 }
 
@@ -993,7 +1044,7 @@ static bool one_block(xlb_ctx* c, uint64_t build, uint64_t probe, uint64_t room)
     if (!build || build > SMALL_BUILD || !probe || probe > SMALL_PROBE || !within_budget(c, room + 64)) return false;
     if (!c->query_attr_set) {
         CUDA_OK(cudaFuncSetAttribute(exists_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMALL_SLOTS * 8 + SMALL_PROBE * 2)));
-        CUDA_OK(cudaFuncSetAttribute(join_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMALL_SLOTS * 12 + 16 + SMALL_BUILD * 2)));
+        CUDA_OK(cudaFuncSetAttribute(join_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMALL_SLOTS * 16 + 16 + SMALL_BUILD * 2)));
         CUDA_OK(cudaFuncSetAttribute(group_small_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_GROUPS_BYTES));
         c->query_attr_set = true;
     }
@@ -1061,11 +1112,23 @@ xlb_rel* query_exists(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint
     return o.release();
 }
 
+// The outputs of a join from its rows by group.
+static void emit_joined(xlb_ctx* c, const uint64_t* match, const OutputsBefore& outputs, uint64_t probes, uint64_t total, const uint32_t* rows, const uint32_t* starts, const Cols& cols) {
+    const bool few = total <= (uint64_t)c->sm_count * BLOCK * 4;
+    const uint64_t tile = few ? BLOCK : BLOCK * 4, blocks = (total + tile - 1) / tile;
+    prof_begin(c, "join_emit", 0);
+    const Publish last = publish_by(c, blocks);
+    if (few) join_emit_k<1><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match, outputs, probes, total, rows, starts, cols, last);
+    else join_emit_k<4><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match, outputs, probes, total, rows, starts, cols, last);
+    check_launch(c, "join_emit");
+    status_published(c, last);
+}
+
 xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32_t* lk, const uint32_t* rk, uint32_t nk, const xlb_schema& os) {
     const uint64_t n = r->rows;
     if (n >= 0xFFFFFFFFull) xlb_fail(XLB_ERR_CAPACITY, "join build side of %llu rows exceeds the 2^32 - 1 row limit", (unsigned long long)n);
     const uint64_t room = std::min<uint64_t>(SMALL_OUTPUTS, 4 * l->rows + 1024);
-    if (one_block(c, n, l->rows, room * row_bytes(os))) {
+    if (one_block(c, n, l->rows, room * row_bytes(os) + l->rows * 24 + n * 4)) {
         std::unique_ptr<xlb_rel> o(new xlb_rel);
         o->ctx = c;
         o->schema = os;
@@ -1073,17 +1136,32 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
         cols.left = (int)l->schema.arity;
         add_columns(c, o.get(), cols, l, room);
         add_columns(c, o.get(), cols, r, room);
-        Buf words = make_buf(c, 16);
+        const uint64_t tiles = (l->rows + SCAN_TILE - 1) / SCAN_TILE;
+        Buf words = make_buf(c, 16 + (tiles + l->rows * 2) * 8 + n * 4);
+        SmallLists lists{};
+        lists.tile = words->as<uint64_t>() + 2;
+        lists.match = lists.tile + tiles;
+        lists.before = (uint32_t*)(lists.match + l->rows);
+        lists.start = lists.before + l->rows;
+        lists.rows = lists.start + l->rows;
         prof_begin(c, "join_small", 0);
         const Publish pub = publish_by(c, 1, words->p, 2);
         const unsigned cap = slots_of(n);
-        join_small_k<<<1, SMALL_THREADS, cap * 12 + 16 + (unsigned)n * 2, c->stream>>>(key_cols(r, rk, nk), (unsigned)n, key_cols(l, lk, nk), (unsigned)l->rows, cols, room,
+        join_small_k<<<1, SMALL_THREADS, cap * 16 + 16 + (unsigned)n * 2, c->stream>>>(key_cols(r, rk, nk), (unsigned)n, key_cols(l, lk, nk), (unsigned)l->rows, cols, room, lists,
                                                                                      words->as<unsigned long long>(), pub);
         check_launch(c, "join_small");
         unsigned long long w[2];
         read_published(c, pub, words->p, 2, w);
-        if (w[1]) return nullptr;
-        if (w[0] <= room) return with_rows(o, w[0]);
+        if (w[1] == 2) return nullptr;
+        if (w[1] == 0 || w[0] == 0) return with_rows(o, w[0]);
+        if (w[0] > room) {
+            for (uint32_t i = 0; i < os.arity; ++i) o->cols[i].reset();
+            cols.n = 0;
+            add_columns(c, o.get(), cols, l, w[0]);
+            add_columns(c, o.get(), cols, r, w[0]);
+        }
+        emit_joined(c, lists.match, OutputsBefore{lists.tile, lists.before}, l->rows, w[0], lists.rows, lists.start, cols);
+        return with_rows(o, w[0]);
     }
     uint64_t cap = 1024;
     while (cap < 2 * n) cap <<= 1;
@@ -1123,10 +1201,8 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     add_columns(c, o.get(), cols, r, w[0]);
     if (w[0]) {
         const OutputsBefore outputs{offs->as<uint64_t>(), in_tile->as<uint32_t>()};
-        const bool lists = w[0] > JOIN_CHAIN_OUTPUTS * n || w[2] > JOIN_CHAIN_ROWS, few = w[0] <= (uint64_t)c->sm_count * BLOCK * 4;
-        Buf rows;
-        if (lists) {
-            rows = make_buf(c, n * 8);
+        if (w[0] > JOIN_CHAIN_OUTPUTS * n || w[2] > JOIN_CHAIN_ROWS) {
+            Buf rows = make_buf(c, n * 8);
             prof_begin(c, "group_start", cap * 16ull);
             group_start_k<<<(unsigned)((cap + SCAN_TILE) / SCAN_TILE), BLOCK, 0, c->stream>>>(slots, cap + 1, rows->as<uint32_t>() + n, (unsigned int*)(words + 3));
             check_launch(c, "group_start");
@@ -1136,15 +1212,15 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
             prof_begin(c, "group_order", cap * 16ull);
             group_order_k<<<grid_for(c, cap + 1), BLOCK, 0, c->stream>>>(slots, cap + 1, rows->as<uint32_t>());
             check_launch(c, "group_order");
+            emit_joined(c, match->as<uint64_t>(), outputs, l->rows, w[0], rows->as<uint32_t>(), rows->as<uint32_t>() + n, cols);
+        } else {
+            prof_begin(c, "join_emit", 0);
+            const uint64_t blocks = (l->rows + BLOCK - 1) / BLOCK;
+            const Publish last = publish_by(c, blocks);
+            join_chains_k<<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), outputs, l->rows, before->as<uint32_t>(), cols, last);
+            check_launch(c, "join_emit");
+            status_published(c, last);
         }
-        prof_begin(c, "join_emit", 0);
-        const uint64_t tile = !lists || few ? BLOCK : BLOCK * 4, blocks = ((lists ? w[0] : l->rows) + tile - 1) / tile;
-        const Publish last = publish_by(c, blocks);
-        if (!lists) join_chains_k<<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), outputs, l->rows, before->as<uint32_t>(), cols, last);
-        else if (few) join_emit_k<1><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), outputs, l->rows, w[0], rows->as<uint32_t>(), rows->as<uint32_t>() + n, cols, last);
-        else join_emit_k<4><<<(unsigned)blocks, BLOCK, 0, c->stream>>>(match->as<uint64_t>(), outputs, l->rows, w[0], rows->as<uint32_t>(), rows->as<uint32_t>() + n, cols, last);
-        check_launch(c, "join_emit");
-        status_published(c, last);
     }
     return o.release();
 }
