@@ -180,6 +180,31 @@ def test_columns_led_on_along_a_path(n, burst, monkeypatch):
         assert res[0] == res[1]
 
 
+def crowd(rels, rows):
+    """Seeds given so often that bit rows are begun: one and a half for every row of the head, whatever they lead to."""
+    n = -(-3 * (1 << (rows - 1).bit_length()) // (2 * len(rels["s"][0])))
+    return {**rels, "s": [np.tile(c, n) for c in rels["s"]]}
+
+
+# As above, begun as bit rows; (2000, 2000, 20000) more rows of a relation than are looked through for rows led to once
+@pytest.mark.parametrize("kinds", [("both",), ("first",), ("both", "second"), ("first", "second", "both")], ids="-".join)
+@pytest.mark.parametrize("hi,lo,rows", [(8191, 100, 9000), (8000, 130, 9000), (130, 8191, 3000), (1000, 1023, 1500), (1500, 1500, 2000), (8000, 8191, 9000), (2000, 2000, 20000)])
+def test_columns_led_on_apart_by_bit_rows(hi, lo, rows, kinds, monkeypatch):
+    rng = np.random.default_rng(hi * lo)
+    pairs = lambda n, x, y: [rng.integers(0, x, n).astype(np.uint32), rng.integers(0, y, n).astype(np.uint32)]  # noqa: E731
+    s = pairs(40, hi, lo)
+    s[0][0], s[1][0] = hi - 1, lo - 1
+    both(sides(kinds), crowd({"s": s, "a": pairs(rows, hi, hi), "b": pairs(rows, lo, lo)}, hi), "p", monkeypatch)
+
+
+@pytest.mark.parametrize("fan", [16, 17, 1024, 1025])
+def test_columns_led_on_to_many_by_bit_rows(fan, monkeypatch):
+    hub = [np.full(fan, 3, np.uint32), np.arange(10, 10 + fan, dtype=np.uint32)]
+    back = [np.arange(10, 10 + fan, dtype=np.uint32), np.full(fan, 3, np.uint32)]
+    e = [np.concatenate([hub[0], back[0][:9], [2000]]).astype(np.uint32), np.concatenate([hub[1], back[1][:9], [2000]]).astype(np.uint32)]
+    both(sides(("both",)), crowd({"s": [np.array([3, 3], np.uint32), np.array([3, 11], np.uint32)], "a": e, "b": e}, 2001), "p", monkeypatch)
+
+
 def test_two_recursive_rules_and_wide_domain(monkeypatch):
     # p(X,Y) :- e(X,Y).  p(X,Z) :- p(X,Y), e(Y,Z).  p(X,Z) :- f(X,Y), p(Y,Z).  ids up to 2^15: 30 bits
     ids = {"e": 0, "f": 1, "p": 2}

@@ -1511,7 +1511,7 @@ constexpr unsigned BT_OWN = 56;                     // rows of a block
 constexpr unsigned BT_LIST = 16;                    // a value with more matches is a whole warp's work
 constexpr unsigned BT_ROWS = 1024;                  // rows that a row may lead to
 constexpr unsigned BT_SMALL = 1024, BT_LEAVE = 24;  // after so many iterations in a row of fewer tuples the loop goes on
-constexpr unsigned BT_EDGES = 1u << 20;             // rows of A (every block looks through them once)
+constexpr unsigned BT_SCANNED = 1u << 14;           // rows of A that every block looks through, for the rows that only one leads to (more: none is taken for such a row)
 constexpr unsigned BT_LISTED = 16384;               // rows of the stored relation whose lists a block keeps in shared memory
 constexpr unsigned BT_SMEM = ((DL_RULES + 2) * BT_WORDS + 2 * BT_OWN * BT_WORDS + DL_WARPS * 256 + (1u << BT_BITS_MAX)) * 4 + BT_LISTED * 2;
 static_assert(BT_SMEM <= (222u << 10), "a block an SM");
@@ -1651,6 +1651,10 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
         }
 #pragma unroll
         for (int i = 0; i < T; ++i) bad |= len[i] > BT_ROWS;
+        if (ru.a_rows > BT_SCANNED) {
+            for (unsigned i = threadIdx.x; i < BT_WORDS; i += DL_THREADS) more_s[i] = ~0u;
+            continue;
+        }
 #pragma unroll 4
         for (unsigned i = threadIdx.x; i < ru.a_rows; i += DL_THREADS) leads_to(other_of(ru.a, i));
     }
@@ -1761,13 +1765,21 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
                     const bool shared = (more_s[to >> 5] >> (to & 31)) & 1u;
                     unsigned *out = next + (uint64_t)to * W, any = 0;
                     if (shared) {
-                        for (unsigned w = lane; w < W; w += 32) {
-                            const unsigned v = led[k * W + w];
+                        constexpr unsigned H = 4;  // words a lane has under way
+                        for (unsigned w0 = lane; w0 < W; w0 += 32 * H) {
+                            unsigned v[H];
+#pragma unroll
+                            for (unsigned u = 0; u < H; ++u) v[u] = w0 + 32 * u < W ? led[k * W + w0 + 32 * u] : 0u;
                             // (a word of the head that is being brought up to date only costs an atomic)
-                            if (v & ~__ldcg(&o.visited[(uint64_t)to * W + w])) {
-                                atomicOr(&out[w], v);
-                                any = 1;
-                            }
+#pragma unroll
+                            for (unsigned u = 0; u < H; ++u)
+                                if (v[u]) v[u] &= ~__ldcg(&o.visited[(uint64_t)to * W + w0 + 32 * u]);
+#pragma unroll
+                            for (unsigned u = 0; u < H; ++u)
+                                if (v[u]) {
+                                    atomicOr(&out[w0 + 32 * u], v[u]);
+                                    any = 1;
+                                }
                         }
                     } else {
                         for (unsigned w = lane; w < W; w += 32) {
@@ -2281,7 +2293,6 @@ static bool bits_apart(const DeltaLoop& d, const std::vector<DeltaRule>& rules, 
         if (x.b_list && r.key_src[r.lo_src - 2] != SRC_LO) return false;
         if (x.a_list) x.a = view_of(*r.ix[r.hi_src - 2]);
         x.a_rows = x.a_list ? (unsigned)r.ix[r.hi_src - 2]->n : 0;
-        if (x.a_list && r.ix[r.hi_src - 2]->n > BT_EDGES) return false;
         if (x.b_list) x.b = view_of(*r.ix[r.lo_src - 2]);
         x.listed = 0;
         if (x.b_list && !listed && r.ix[r.lo_src - 2]->n <= BT_LISTED) {
