@@ -205,6 +205,27 @@ def test_columns_led_on_to_many_by_bit_rows(fan, monkeypatch):
     both(sides(("both",)), crowd({"s": [np.array([3, 3], np.uint32), np.array([3, 11], np.uint32)], "a": e, "b": e}, 2001), "p", monkeypatch)
 
 
+# Handed to the loop after 32 small iterations, as `rows` rows or `rows` tuples of one row; at the end of the path each of them meets `burst` values at once
+@pytest.mark.parametrize("n,rows,burst", [(30, 1, 0), (31, 1, 0), (32, 1, 0), (33, 1, 0), (32, 1, 200), (60, 1, 200), (300, 40, 0), (300, 1500, 0), (40, 1500, 60)])
+@pytest.mark.parametrize("turned", [False, True])
+def test_bit_rows_left_for_the_loop(n, rows, burst, turned, monkeypatch):
+    path = list(chain(n + 1))
+    path = [np.concatenate([path[0], np.full(burst, n), [2000]]).astype(np.uint32), np.concatenate([path[1], np.arange(n + 1, n + 1 + burst), [2000]]).astype(np.uint32)]
+    still = [np.append(np.arange(rows), 2000).astype(np.uint32)] * 2
+    s = [np.zeros(rows, np.uint32), np.arange(rows, dtype=np.uint32)]
+    rels = {"s": s[::-1] if turned else s, "a": still if turned else path, "b": path if turned else still}
+    rels = crowd(rels, 2001)
+    both(sides(("both",)), rels, "p", monkeypatch)
+    for limit, fits in ((n - 1, False), (n + 1 + (burst > 0), True)):
+        p = KernelProvider(device=0, max_iterations=limit)
+        try:
+            run_program(p, sides(("both",)), rels, ["p"])
+            assert fits
+        except XlbError as e:
+            assert not fits and e.status == A.ERR_ITER_LIMIT
+        p.close()
+
+
 def test_two_recursive_rules_and_wide_domain(monkeypatch):
     # p(X,Y) :- e(X,Y).  p(X,Z) :- p(X,Y), e(Y,Z).  p(X,Z) :- f(X,Y), p(Y,Z).  ids up to 2^15: 30 bits
     ids = {"e": 0, "f": 1, "p": 2}

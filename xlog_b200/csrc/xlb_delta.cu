@@ -92,7 +92,7 @@ enum Phase { PH_ROWS = 0, PH_HEAVY = 1, PH_SOLO = 2, PH_DONE = 3, PH_FULL = 4 };
 // that is late.  A solo phase that ends an iteration by itself touches none.
 struct Slot {
     unsigned long long count, cand;  // tuples appended to the log; candidates
-    unsigned long long heavy_n;      // pieces of long rows, listed or not (rows that found the list full go on raising it)
+    unsigned long long heavy_n;      // pieces of long rows, listed or not (rows that found the list full go on raising it); of bit rows: rows that the delta's were led to
     unsigned next_heavy;             // pieces taken
     unsigned next_chunk;             // rows are taken in batches
 };
@@ -1502,15 +1502,18 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const __grid_constant__ O
 // some 20 K cycles of dependent steps between two barriers, then atomics on words of shared memory (what neighbours
 // lead to shares words; setting a lane's bits of one word together cost more than it saved).
 //   Rows that nobody reached are passed over by a stamp.  Lists of A are shared out among a block's warps only: where one
-// is longer than BT_ROWS, the loop does it all.  A fixpoint that goes on with next to nothing in an iteration is
-// handed to the loop, whose small iterations meet at no barrier.
+// is longer than BT_ROWS, the loop does it all.  A fixpoint whose iterations come out cheaper there is handed to the
+// loop, whose small ones meet at no barrier.
 constexpr int BT_BITS_MIN = 5, BT_BITS_MAX = 13;
 constexpr int BT_BITS_BOTH = 20;                    // of both columns: below, the loop is as fast (same generation over 300 and 511 nodes 139 and 149 us of device time by the loop, 155 and 161 here; 1023 nodes 195 and 166)
 constexpr unsigned BT_WORDS = 1u << (BT_BITS_MAX - 5);
 constexpr unsigned BT_OWN = 56;                     // rows of a block
 constexpr unsigned BT_LIST = 16;                    // a value with more matches is a whole warp's work
 constexpr unsigned BT_ROWS = 1024;                  // rows that a row may lead to
-constexpr unsigned BT_SMALL = 1024, BT_LEAVE = 24;  // after so many iterations in a row of fewer tuples the loop goes on
+// What an iteration takes beside what it would take the loop, counted in candidates of the loop (80 a ns).  One of next
+// to nothing took 1.4 us more with heads of 11 bits a column, 1.7 with 12 and 4 to 11 with 13: the rows every block looks
+// through.  Then a word a lane of every place.  Going on in the loop costs some 40 us.
+constexpr float BT_FIXED = 80e3f, BT_MAP = 0.16f, BT_WORD = 1 / 16.f, BT_CHANGE = 3200e3f;
 // Seeds, times the matches of a value, a row of the head has to have for bit rows to be begun.  Same generation over
 // trees has 1.8 to 3.6 (gains of 1.2 to 2.6 x), 2000 nodes of degree 2 3.8 (338 us by the loop, 252), of degree 1.1
 // 1.15 (262 and 302; 8000 nodes 690 and 865), a path 1 or less (8000 nodes 38 and 72 ms), 5 values led on by a relation of
@@ -1540,7 +1543,16 @@ struct Active {  // a row of the delta that A leads on: the block's k-th, its li
 };
 struct BitsState {
     unsigned long long tuples, cands, pending, iterations;
-    unsigned slot, small, leaving, over, fix, go;
+    float regret, before;  // time lost to the loop so far, in its candidates; tuples of the iteration before
+    unsigned slot, leaving, over, fix, go;
+    // Whether the loop should go on, after an iteration of so many tuples, candidates and words written (of `all` there
+    // can be; the head's bitmap has `map`).  Looks two iterations ahead by the growth of this one: a few seeds may be about to fill the head.
+    __device__ __forceinline__ bool leave(float found, float cand, float words, float all, float map) {
+        const float fixed = BT_FIXED + map * BT_MAP, growth = iterations ? found / fmaxf(before, 1.f) : cand / fmaxf(found, 1.f);
+        regret = fmaxf(0.f, regret + fixed + words * BT_WORD - cand);
+        before = found;
+        return regret >= BT_CHANGE && fixed + fminf(words * growth, all) * BT_WORD > cand * growth * fmaxf(growth, 1.f);
+    }
 };
 // B as a block keeps it: per value its matches' start and number, and the matches.
 struct Lists {
@@ -1600,7 +1612,7 @@ __device__ __forceinline__ unsigned lead(const Out& o, const Ix& ix, const Lists
 __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_constant__ Out o, const __grid_constant__ BitsRules rules, const __grid_constant__ Bits b, uint64_t max_iterations) {
     extern __shared__ unsigned bt_smem[];
     __shared__ BitsState st;
-    __shared__ unsigned long long sum_s[2];
+    __shared__ unsigned long long sum_s[3];
     __shared__ unsigned total_s[BT_OWN];                    // tuples of the block's rows of the delta
     __shared__ Active act_s[BT_OWN];
     __shared__ unsigned active_s;
@@ -1619,6 +1631,8 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
     const unsigned parts = W > 16 ? 31 - __clz(W / 16) : 0;  // a row is led in 2^parts pieces of work
     Ctl* ctl = o.ctl;
     bool bad = false;
+    float all_places = 0;
+    for (int q = 0; q < rules.n; ++q) all_places += rules.r[q].a_list ? rules.r[q].a_rows : b.rows;
     for (unsigned i = threadIdx.x; i < 2 * BT_WORDS; i += DL_THREADS) once_s[i] = 0;
     __syncthreads();
     for (int q = 0; q < rules.n; ++q) {
@@ -1674,7 +1688,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
         const bool leaving = st.leaving != 0;
         unsigned *next = b.next[cur ^ 1], *reached = b.next[cur];
         Slot* slot = &ctl->slot[st.slot];
-        if (threadIdx.x < 2) sum_s[threadIdx.x] = 0;
+        if (threadIdx.x < 3) sum_s[threadIdx.x] = 0;
         if (blockIdx.x == 0 && threadIdx.x == 0) ctl->slot[st.slot == 2 ? 0 : st.slot + 1] = Slot{};
         __syncthreads();
         // the rows of the delta: what they were reached by beyond the head (at first: the seeds)
@@ -1740,7 +1754,10 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
                     rows += __popc(some);
                     places += more;
                 }
-                if (lane == 0) active_s = rows;
+                if (lane == 0) {
+                    active_s = rows;
+                    sum_s[2] += places;  // (nobody else's until the iteration is over)
+                }
             }
             if (ru.b_list)
                 for (unsigned i = threadIdx.x; i < own * W; i += DL_THREADS) led_s[i] = 0;
@@ -1805,6 +1822,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
         if (threadIdx.x == 0) {
             if (sum_s[0]) atomicAdd(&slot->count, sum_s[0]);
             if (sum_s[1]) atomicAdd(&slot->cand, sum_s[1]);
+            if (sum_s[2]) atomicAdd(&slot->heavy_n, sum_s[2]);
             passed += gridDim.x;
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->arrived) : "memory");
             st.go = wait_for(o, &ctl->arrived, passed, 0, passed);
@@ -1814,9 +1832,9 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
             st.pending = __ldcg(&slot->cand);
             st.iterations = phase;
             st.fix = found == 0;
-            st.small = found < BT_SMALL ? st.small + 1 : 0;
             st.over = st.fix || leaving || phase >= max_iterations;
-            st.leaving = st.small >= BT_LEAVE && st.pending <= o.cap;  // (the log takes whatever the next iteration finds)
+            // (the log takes whatever the next iteration finds)
+            st.leaving = st.leave((float)found, (float)st.pending, (float)__ldcg(&slot->heavy_n) * W, all_places * W, (float)b.rows * W) && st.pending <= o.cap;
             st.slot = st.slot == 2 ? 0 : st.slot + 1;
         }
         __syncthreads();
