@@ -1509,7 +1509,7 @@ constexpr int BT_BITS_BOTH = 20;                    // of both columns: below, t
 constexpr unsigned BT_WORDS = 1u << (BT_BITS_MAX - 5);
 constexpr unsigned BT_OWN = 56;                     // rows of a block
 constexpr unsigned BT_LIST = 16;                    // a value with more matches is a whole warp's work
-constexpr unsigned BT_ROWS = 1024;                  // rows that a row may lead to
+constexpr unsigned BT_ROWS = 1024;                  // rows that a row may lead to; where the head has more than four times as many, a quarter of those (7000 nodes of degree 2 and 2000 more into one: 2.39 ms by the loop, 2.02; 4000 into one 2.48 and 3.67; 2000 nodes and 1900 into one 0.72 and 0.85)
 // What an iteration takes beside what it would take the loop, counted in candidates of the loop (80 a ns).  One of next
 // to nothing took 1.4 us more with heads of 11 bits a column, 1.7 with 12 and 4 to 11 with 13: the rows every block looks
 // through.  Then a word a lane of every place.  Going on in the loop costs some 40 us.
@@ -1669,7 +1669,7 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
             if (v < b.rows) find(ru.a, v, s[i], len[i]);
         }
 #pragma unroll
-        for (int i = 0; i < T; ++i) bad |= len[i] > BT_ROWS;
+        for (int i = 0; i < T; ++i) bad |= len[i] > max(BT_ROWS, b.rows / 4);
         if (ru.a_rows > BT_SCANNED) {
             for (unsigned i = threadIdx.x; i < BT_WORDS; i += DL_THREADS) more_s[i] = ~0u;
             continue;
