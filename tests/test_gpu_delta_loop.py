@@ -322,6 +322,30 @@ def test_rules_by_rows(kinds, top, rows, monkeypatch):
             p.close()
 
 
+# From 12 bits on (ACROSS alone: 11) rows are taken where the lists are long or many: `hubs` values with 60 of them each, one row
+# for every fourth value (few: the loop), or for every one and the other way round
+@pytest.mark.parametrize("kinds", [("across",), ("steps",), ("copy", "steps"), ("copy2", "steps2", "across2")], ids="-".join)
+@pytest.mark.parametrize("top", [2047, 4095, 8191])
+@pytest.mark.parametrize("hubs", [0, 2, 60])
+def test_rules_by_rows_where_they_pay(kinds, top, hubs, monkeypatch):
+    rng = np.random.default_rng(top + hubs)
+    pairs = lambda n: [rng.integers(0, top, n, endpoint=True).astype(np.uint32) for _ in range(2)]  # noqa: E731
+    lists = lambda way: [np.concatenate(c).astype(np.uint32) for c in zip(pairs(top // 4), [np.repeat(np.arange(hubs) * 30, 60), rng.integers(0, top, 60 * hubs)][::way])]  # noqa: E731
+    rels = {"s": pairs(top // 3), "e": lists(1), "f": lists(-1)}
+    rels["s"][0][0] = top
+    got, it, cand = both(by_rows(kinds), rels, "p", monkeypatch)
+    monkeypatch.delenv("XLB_NO_DELTA_LOOP")
+    p = KernelProvider(device=0)
+    p.profile_enable("list_squares")
+    again, _ = run_program(p, by_rows(kinds), rels, ["p"])
+    asked = "list_squares" in p.profile_read()
+    p.close()
+    if hubs < 60:  # (rows enough decide by their number)
+        assert asked == (top > 2047 or kinds == ("across",))
+    for a, b in zip(again["p"], got):
+        assert np.array_equal(a, b)
+
+
 def test_transposed_partner_and_composed_relation(monkeypatch):
     # p(X,Z) :- p(X,Y), p(Z,Y), g(X,Z)-free: the partner by its second column; q-shaped: p(Z,Y) :- g(Z,X), p(X,W), p(W,Y)
     ids = {"e": 0, "g": 1, "p": 2}

@@ -1858,13 +1858,23 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_bits_k(const __grid_const
 // phases: the rows' own warps add what was derived to the head, which makes the delta; then groups of eight warps
 // take the values of all rules in turn, up to four groups a value where there are few of them.  What bounds it is the chain of
 // loads a value costs, some 6 K cycles, and two barriers an iteration.
-//   Against the loop: points-to programs of 150, 600, 1500, 3000 and 6000 values 248, 534, 623, 1242 and 4016 us by the loop, 204,
-// 267, 305, 581 and 1692 by rows, as their relations are skewed.  Over uniform ones the two are close: 2048 values
-// with 300 stored rows a relation 270 and 289, with 2000 787 and 723; 8192 values with 800 346 and 432, with 8000
-// 10.0 and 13.3 ms, with 16 000 43 and 24 ms.  (A warp a value for rows of few tuples, before the groups, did
+//   Against the loop: points-to programs of 300, 600, 1500, 3000 and 6000 values 328, 530, 623, 1236 and 3937 us by the loop, 198,
+// 237, 287, 502 and 1506 by rows, as their relations are skewed.  An item costs whole rows, which are long where the head has
+// many bits, whatever is in them; so from 12 bits on there has to be enough (ops_delta_by_rows_pays): seeds a
+// value of the head, times the sum of the squares of the lists' lengths a value and rule, since a tuple is led on by
+// a list of average length weighted by itself.  Over uniform relations, by the loop and by rows: COPY and STEPS over 8192
+// values 1.0 seeds and 0.3 rows a value (0.4 by this measure) 416 and 509 us, 0.3 and 1.0 (0.6) 2.95 and 2.63 ms, 1.0 and
+// 1.0 (2) 13.9 and 6.7; COPY, STEPS and ACROSS 0.4 14.2 and 20.5, 0.6 9.8 and 10.7, 2 31.8 and 22.4; STEPS 0.6 1.02 and
+// 1.20; ACROSS alone, whose values have a row or none, 0.6 0.84 and 1.86, 2 8.7 and 9.7, 6 18.8 and 12.7.  Over 4096 values
+// 0.12 183 and 204 us, 0.39 289 and 309, 3.02 and 2.54 ms, 0.6 995 and 866 us; ACROSS 1.8 604 and 796 us, 2 1.84 and
+// 1.92 ms, 6 3.43 and 2.45.  Points-to over uniform relations of 6000 values 0.1 2.08 and 2.52, 0.3 3.90 and 4.86, 0.9 5.28 and 3.40; over skewed ones
+// the measure is 1.2 to 10.  Up to 11 bits the two differ by a tenth at most where rows lose (ACROSS by a
+// quarter); long copy chains in such programs, 2000 iterations of next to nothing, 17.4 and 20.0 ms.
+//   (A warp a value for rows of few tuples, before the groups, did
 // better on sparse relations and took points-to 242.)  h(P, Y) :- h(P, Q), h(Q, Y) stays with the loop: every row is a value
 // then, and on a sparse graph of 8000 nodes rows took 1320 us and the loop 284 (dense, 2000 nodes: 713 and 966).
 constexpr int WD_BITS_MIN = 6, WD_BITS_MAX = 13;
+constexpr int WD_ALWAYS = 11;     // bits up to which rows are taken whatever is stored (but for ACROSS alone)
 constexpr unsigned WD_WARPS = 8, WD_THREADS = WD_WARPS * 32, WD_GROUPS = DL_THREADS / WD_THREADS;
 constexpr unsigned WD_SPLIT = 4;  // groups that share a value, at most
 constexpr unsigned WD_FEW = 64;   // tuples of a row up to which it is not
@@ -2166,6 +2176,26 @@ __global__ void __launch_bounds__(DL_THREADS, 1) delta_wide_k(const __grid_const
         ctl->rows_levels = st.iterations ? st.iterations : 1;  // an iteration over nothing finds nothing
         ctl->rows_left = st.fix ? 0 : 1;
     }
+}
+// Squares of the lists' lengths, of all rules: what a tuple is led on to, summed over the stored rows.
+__global__ void __launch_bounds__(DL_THREADS) list_squares_k(const __grid_constant__ WideRules rules, unsigned rows, unsigned long long* sum, const Publish pub) {
+    __shared__ unsigned long long sum_s;
+    if (threadIdx.x == 0) sum_s = 0;
+    __syncthreads();
+    unsigned long long mine = 0;
+    for (int q = 0; q < rules.n; ++q)
+#pragma unroll 4
+        for (unsigned v = threadIdx.x; v < rows; v += DL_THREADS) {
+            uint32_t s, len;
+            find(rules.r[q].ix, v, s, len);
+            mine += (unsigned long long)len * len;
+        }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) mine += __shfl_xor_sync(FULL, mine, d);
+    if (lane_id() == 0 && mine) atomicAdd(&sum_s, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) *sum = sum_s;
+    publish_now(pub);
 }
 // The loop starts on what was given up, or left.
 __global__ void delta_rows_left_k(Ctl* c) {
@@ -2501,21 +2531,48 @@ static uint64_t wide_bytes(int bits) {
     const uint64_t rows = 1ull << bits, map = rows * rows / 32;
     return (2 * map + 3 * rows + 2 * std::max<uint64_t>(rows / 32, 2) + DELTA_ROWS_MAX * rows + DELTA_ROWS_MAX) * 4;
 }
-bool ops_delta_by_rows_fits(xlb_ctx* c, int bits) {
-    return bits >= WD_BITS_MIN && bits <= WD_BITS_MAX && (!c->budget || c->allocated + (1ull << (2 * bits)) / 8 * 2 + wide_bytes(bits) <= c->budget);
-}
-void ops_delta_by_rows(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRows>& rules, uint64_t max_iterations, DeltaResult* res) {
-    for (auto& r : rules)
-        if (rules.size() > DELTA_ROWS_MAX || !r.list) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules by rows", rules.size());
-    Wide b{};
-    b.rows = 1u << d.hi_bits;
-    b.words = b.rows / 32;
+static WideRules wide_rules(const std::vector<DeltaRows>& rules) {
     WideRules rs{};
     for (auto& r : rules) {
+        if (rules.size() > DELTA_ROWS_MAX || !r.list) xlb_fail(XLB_ERR_INVALID, "internal: %zu rules by rows", rules.size());
         WideRule& x = rs.r[rs.n++];
         x.kind = r.kind;
         x.ix = view_of(*r.list);
     }
+    return rs;
+}
+bool ops_delta_by_rows_pays(xlb_ctx* c, int bits, double seeds, const std::vector<DeltaRows>& rules) {
+    bool across = true;
+    for (auto& r : rules) across = across && r.kind == DeltaRows::ACROSS;
+    const double least = across ? (bits <= WD_ALWAYS - 1 ? 0 : bits <= WD_ALWAYS ? 2 : 4) : bits <= WD_ALWAYS ? 0 : bits <= WD_ALWAYS + 1 ? 0.25 : 0.7;
+    if (least == 0 || rules.empty()) return true;
+    // (what the squares are between: rows as even as they can be, and all of one value)
+    const double values = (double)(1u << bits), scale = seeds / values / (values * rules.size());
+    double low = 0, high = 0;
+    for (auto& r : rules) {
+        const double n = (double)r.list->n;
+        low += n * std::max(1.0, n / values);
+        high += n * n;
+    }
+    if (low * scale >= least || high * scale < least) return low * scale >= least;
+    const WideRules rs = wide_rules(rules);
+    Buf sum = make_buf(c, 8);
+    prof_begin(c, "list_squares", 0);
+    const Publish pub = publish_by(c, 1, sum->p, 1);
+    list_squares_k<<<1, DL_THREADS, 0, c->stream>>>(rs, 1u << bits, sum->as<unsigned long long>(), pub);
+    check_launch(c, "list_squares");
+    unsigned long long squares;
+    read_published(c, pub, sum->p, 1, &squares);
+    return squares * scale >= least;
+}
+bool ops_delta_by_rows_fits(xlb_ctx* c, int bits) {
+    return bits >= WD_BITS_MIN && bits <= WD_BITS_MAX && (!c->budget || c->allocated + (1ull << (2 * bits)) / 8 * 2 + wide_bytes(bits) <= c->budget);
+}
+void ops_delta_by_rows(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRows>& rules, uint64_t max_iterations, DeltaResult* res) {
+    Wide b{};
+    b.rows = 1u << d.hi_bits;
+    b.words = b.rows / 32;
+    WideRules rs = wide_rules(rules);
     const size_t smem = wide_group_bytes(b.words) * WD_GROUPS;
     if (!c->delta_wide_attr_set) CUDA_OK(cudaFuncSetAttribute(delta_wide_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(wide_group_bytes(1u << (WD_BITS_MAX - 5)) * WD_GROUPS)));
     c->delta_wide_attr_set = true;

@@ -1979,6 +1979,17 @@ static bool delta_bounds(xlb_ctx* c, const std::vector<FlatRule>& rules, const s
     return true;
 }
 
+// About how many seeds there will be: the rows of a relation that is copied; a join's are not known yet, and taken for one
+// a value.
+static double delta_seeds(xlb_ctx* c, const DeltaPlan& plan, int bits) {
+    double seeds = 0;
+    for (const FlatRule* fr : plan.seeds) {
+        const xlb_rel* r = fr->atoms.size() == 1 && fr->filters.empty() && fr->checks.empty() ? store_get(c, fr->atoms[0].rel) : nullptr;
+        seeds += r ? (double)r->rows : (double)(1u << bits);
+    }
+    return seeds;
+}
+
 // Seeds the component (unless `from_store`: then the stored head and "__delta_<head>" are where it
 // stands) and runs it to its fixpoint.  False: not taken, nothing changed.
 static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<FlatRule>& rules, const std::string& p, const xlb_schema& hs, bool from_store, RunState& rs,
@@ -2005,7 +2016,16 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         if (c->budget && c->allocated + (square ? 8 : 3) * bitmap > c->budget) return false;
         int composed = 0;
         for (auto& t : plan.square) composed += t.composed >= 0 ? 1 : 0;
-        const bool by_rows = square && plan.wide.size() == plan.wide_rules && plan.wide.size() <= DELTA_ROWS_MAX && ops_delta_by_rows_fits(c, lb);
+        bool by_rows = square && plan.wide.size() == plan.wide_rules && plan.wide.size() <= DELTA_ROWS_MAX && ops_delta_by_rows_fits(c, lb);
+        std::vector<DeltaRows> wide;
+        for (auto& w : plan.wide) {
+            if (!by_rows) break;
+            DeltaRows r;
+            r.kind = w.kind;
+            r.list = &get_index(c, w.fr->atoms[w.list].rel, w.list_kc, rs);
+            if (r.list->n) wide.push_back(r);
+        }
+        by_rows = by_rows && ops_delta_by_rows_pays(c, lb, delta_seeds(c, plan, lb), wide);
         DeltaLoop d = ops_delta_begin(c, hb, lb, square && !by_rows, composed);
         if (from_store) {
             PhaseTimer t(c, &rs.st.ms_join);
@@ -2045,14 +2065,6 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
             d.seeds_listed = seed.atoms.size() == 1 && seed.filters.empty() && seed.checks.empty() && seed.atoms[0].arity == 2 && seed.head_vars.size() == 2 &&
                              seed.atoms[0].var[0] != seed.atoms[0].var[1] && seed.head_vars[0] == seed.atoms[0].var[0] && seed.head_vars[1] == seed.atoms[0].var[1] && one.joins == 1 &&
                              one.kc[0] == 0 && seed.atoms[0].rel == one.fr->atoms[one.atom[0]].rel;
-        }
-        std::vector<DeltaRows> wide;
-        for (auto& w : plan.wide) {
-            if (!by_rows) break;
-            DeltaRows r;
-            r.kind = w.kind;
-            r.list = &get_index(c, w.fr->atoms[w.list].rel, w.list_kc, rs);
-            if (r.list->n) wide.push_back(r);
         }
         std::vector<DeltaRule> run;
         for (auto& one : plan.rec) {

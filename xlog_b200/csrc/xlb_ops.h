@@ -247,6 +247,7 @@ void ops_delta_run(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRule>& rules
                    DeltaResult* res);
 
 // The same for rules that are all of the kinds of DeltaRows, from seeds alone, over a head of `bits` bits a column.
+bool ops_delta_by_rows_pays(xlb_ctx* c, int bits, double seeds, const std::vector<DeltaRows>& rules);  // rather than the loop
 bool ops_delta_by_rows_fits(xlb_ctx* c, int bits);
 void ops_delta_by_rows(xlb_ctx* c, DeltaLoop& d, const std::vector<DeltaRows>& rules, uint64_t max_iterations, DeltaResult* res);
 
