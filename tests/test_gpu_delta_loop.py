@@ -75,6 +75,18 @@ def test_rows_that_follow_a_path(tail, top, monkeypatch):
     both(programs.transitive_closure(), {"edge": edge}, "reach", monkeypatch)
 
 
+# Followed for 32 levels and more (a level for 96 values: 85 of 13 bits, 170 of 14), walked, cut short by a twig, later tried again
+@pytest.mark.parametrize("top", [1000, 8191, (1 << 14) - 1])
+@pytest.mark.parametrize("every", [33, 40, 72, 73, 200, 500])
+@pytest.mark.parametrize("back", [None, 0, 590, 600])
+def test_rows_that_are_walked(top, every, back, monkeypatch):
+    n = 600
+    twigs = np.arange(every // 2, n, every)
+    src = [np.arange(n), twigs, [top]] + ([] if back is None else [[n]])
+    dst = [np.arange(1, n + 1), n + 1 + np.arange(len(twigs)), [0]] + ([] if back is None else [[back]])
+    both(programs.transitive_closure(), {"edge": [np.concatenate(c).astype(np.uint32) for c in (src, dst)]}, "reach", monkeypatch)
+
+
 @pytest.mark.parametrize("limit", [31, 32, 33, 34, 69, 70])
 def test_iteration_limit_on_a_path(limit):
     p = KernelProvider(device=0, max_iterations=limit)

@@ -1034,7 +1034,7 @@ constexpr int RW_BITS_MIN = 5, RW_BITS_MAX = 16;  // of the second column: a row
 constexpr unsigned RW_QUEUE = 16384;              // values the frontier of a row may hold (and the row's seeds)
 constexpr unsigned RW_LONG = 16384;               // candidates of a warp (some 50 us) from which a row may be given up
 constexpr unsigned RW_LIST = 64;                  // a value with so many matches is a warp's work by itself
-constexpr unsigned RW_FOLLOW = 32;                // levels of one value each after which a row is taken for a path
+constexpr unsigned RW_FOLLOW = 32, RW_PATH = 96;  // levels of one value each after which a row is taken for a path, and entries of the table for each
 constexpr int RW_LISTS_BITS = 11;                 // values whose matches are taken as rows of bits: at most 64 words
 constexpr uint64_t RW_LISTS_MIN = 1u << 13;       // rows of the relation below which the copy costs what it saves (four blocks of 44 nodes, 7744 rows: 162 us by matches, 165 by rows; of 46 162 and 162; of 80 205 and 192)
 constexpr unsigned RW_SQUARED = 16;               // entries a thread of the path's table
@@ -1292,17 +1292,28 @@ struct RowsWarp {
     // table has more, one lane goes alone.)  Ends where a value has no or several matches (its level is not done),
     // where a value is known, or at the limit.  What bounds `follow` is some 600 cycles of dependent instructions a
     // level, one warp an SM partition; here 32 levels share them (chain of 1500 nodes, the whole kernel: 484 us
-    // with `follow` alone, 135 with one lane on the table, 70 with 32).
+    // with `follow` alone, 135 with one lane on the table, 70 with 32).  Making the table takes what 40 levels of `follow` do,
+    // with more values more: a path with a twig after every 40 of 7000 nodes, each of which ended a walk of eight
+    // levels, took 22.0 ms, 8.1 now that a row whose walk was cut short is followed further before its next (7.9 by
+    // `follow` alone); paths of 80 nodes, 8000 in all, 297 us, 222 since more values want more levels (217 by `follow` alone).
     __device__ __forceinline__ void walk(const Out& o, const Ix& ix, uint64_t max_iterations) {
         constexpr unsigned short STOP = 0xFFFF;  // (no value: the ring has fewer entries)
         const unsigned lane = lane_id(), at = sh->head, values = 1u << o.lo_bits;
         unsigned y = queue[at & mask];
         __syncthreads();
-        for (unsigned v = threadIdx.x; v < values; v += W * 32) {
-            uint32_t start, len;
-            find(ix, v, start, len);
-            const uint32_t z = len == 1 ? other_of(ix, start) : ~0u;
-            queue[v] = z >> o.lo_bits ? STOP : (unsigned short)z;  // (a match outside the domain is left to the other paths to report)
+        constexpr unsigned N = 8;  // values a thread looks up together
+        for (unsigned v0 = threadIdx.x; v0 < values; v0 += N * W * 32) {
+            uint32_t start[N], len[N];
+#pragma unroll
+            for (unsigned u = 0; u < N; ++u) {
+                start[u] = len[u] = 0;
+                if (v0 + u * W * 32 < values) find(ix, v0 + u * W * 32, start[u], len[u]);
+            }
+#pragma unroll
+            for (unsigned u = 0; u < N; ++u) start[u] = len[u] == 1 ? other_of(ix, start[u]) : ~0u;
+#pragma unroll
+            for (unsigned u = 0; u < N; ++u)
+                if (v0 + u * W * 32 < values) queue[v0 + u * W * 32] = start[u] >> o.lo_bits ? STOP : (unsigned short)start[u];  // (a match outside the domain is left to the other paths to report)
         }
         __syncthreads();
         const unsigned width = values <= RW_SQUARED * W * 32 ? 32 : 1;
@@ -1411,19 +1422,22 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const __grid_constant__ O
             __syncthreads();  // (read by all before a warp adds to it)
             bool ok = tried && end <= sh.queue;
             uint64_t level = 0, cand = 0, looked = RW_LONG;
+            const unsigned least = max(RW_FOLLOW, sh.queue / RW_PATH);
+            unsigned path = least;  // levels of one value each after which the row is taken for a path
             while (ok && head != end && level < max_iterations) {
                 if (end - head == 1 && rules.n == 1) {
                     const bool table = sh.queue >> o.lo_bits;  // the ring has an entry for every value
                     const unsigned from = head;
-                    if (warp == 0) w.follow(o, rules.r[0].ix[0], max_iterations, table ? RW_FOLLOW : ~0u);
+                    if (warp == 0) w.follow(o, rules.r[0].ix[0], max_iterations, table ? path : ~0u);
                     __syncthreads();
                     head = v->head;
                     end = v->tail;
-                    if (table && head - from == RW_FOLLOW && end - head == 1) {
+                    if (table && head - from == path && end - head == 1) {
                         w.walk(o, rules.r[0].ix[0], max_iterations);
                         __syncthreads();
                         head = v->head;
                         end = v->tail;
+                        path = head - from < least * 9 / 4 ? 2 * path : least;  // (a short one, as the next may be: later)
                     }
                     level = v->level;
                     __syncthreads();
