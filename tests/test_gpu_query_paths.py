@@ -191,3 +191,16 @@ def test_more_outputs_than_one_block_has_room_for(p, npr, nb, keys, dtype):
     for _ in range(2):
         for g, w in zip(p.download(p.hash_join_v2(lb, rb, [0], [1])), [c[l] for c in left] + [c[r] for c in right]):
             assert np.array_equal(g, w)
+
+
+# Many build rows: groups of 9 to 16 go out from lists where they go out often
+@pytest.mark.parametrize("group,ratio", [(8, 8), (9, 5), (9, 6), (13, 4), (16, 3), (16, 4), (17, 1)])
+def test_joins_of_many_rows_from_chains_and_from_lists(p, group, ratio):
+    rng = np.random.default_rng(group)
+    n = (1 << 18) + 5000
+    key = rng.permutation(np.arange(n, dtype=np.uint64) // np.uint64(group) * np.uint64(977) + np.uint64(1))
+    ask = key[rng.integers(0, n, n * ratio // group)]
+    left, right = [ask, np.arange(len(ask), dtype=np.uint32)], [np.arange(n, dtype=np.uint32), key]
+    l, r = inner(ask, key)
+    for g, w in zip(p.download(p.hash_join_v2(p.create_buffer_from_slices(left), p.create_buffer_from_slices(right), [0], [1])), [c[l] for c in left] + [c[r] for c in right]):
+        assert np.array_equal(g, w)

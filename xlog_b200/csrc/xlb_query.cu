@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned
 constexpr unsigned JOIN_GROUP_MAX = 64;
 constexpr uint64_t JOIN_CHAIN_OUTPUTS = 8;  // outputs a build row, and rows of the longest group, up to which they
 constexpr unsigned JOIN_CHAIN_ROWS = 16;    // go out from the chains
+constexpr uint64_t JOIN_CHAIN_NEAR = 1ull << 18, JOIN_CHAIN_FAR = 52;  // above so many build rows, outputs a build row times rows of the longest group (1 M rows by chains / lists: groups of 16 two outputs 162 / 214, four 253 / 244, eight 373 / 298; groups of 12 four 161 / 234, eight 290 / 290; 131 072 rows, groups of 16, eight 85 / 116)
 constexpr unsigned JOIN_SAMPLE = 1024, JOIN_OFTEN = 16;  // (a row a thread: a chain of latencies as long as the clearing)
 constexpr uint64_t JOIN_SAMPLED = 1ull << 16;
 __global__ void __launch_bounds__(JOIN_SAMPLE) group_clear_k(KeyCols keys, uint64_t n, uint4* __restrict__ slots, uint64_t slot_vecs, uint64_t* __restrict__ words, uint64_t nwords,
@@ -217,11 +218,11 @@ __global__ void __launch_bounds__(BLOCK) group_chain_k(KeyCols keys, uint64_t n,
             if (there == key) {
                 unsigned* entry = reinterpret_cast<unsigned*>(&slots[h].y);  // [0] rows, [1] the last one (plus one)
                 number = atomicAdd(&entry[0], 1u);
-                if (number >= JOIN_GROUP_MAX) {  // (the chain is not used any more)
+                if (number >= JOIN_GROUP_MAX) {
                     *too_long = 1;
                     return;
                 }
-                link = atomicExch(&entry[1], (unsigned)i + 1);
+                if (number < JOIN_CHAIN_ROWS) link = atomicExch(&entry[1], (unsigned)i + 1);  // (longer chains are not followed)
                 break;
             }
             h = (h + 1) & mask;
@@ -1201,7 +1202,8 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
     add_columns(c, o.get(), cols, r, w[0]);
     if (w[0]) {
         const OutputsBefore outputs{offs->as<uint64_t>(), in_tile->as<uint32_t>()};
-        if (w[0] > JOIN_CHAIN_OUTPUTS * n || w[2] > JOIN_CHAIN_ROWS) {
+        const bool far = n > JOIN_CHAIN_NEAR && w[2] > JOIN_CHAIN_ROWS / 2;
+        if (w[0] > JOIN_CHAIN_OUTPUTS * n || w[2] > JOIN_CHAIN_ROWS || (far && w[0] * w[2] > JOIN_CHAIN_FAR * n)) {
             Buf rows = make_buf(c, n * 8);
             prof_begin(c, "group_start", cap * 16ull);
             group_start_k<<<(unsigned)((cap + SCAN_TILE) / SCAN_TILE), BLOCK, 0, c->stream>>>(slots, cap + 1, rows->as<uint32_t>() + n, (unsigned int*)(words + 3));
