@@ -60,7 +60,7 @@ def rows_from(starts, n):
 # First columns of sets, of 6 MB and more and of few values, go as runs: tiles are 4096 rows, a warp's 512, what a
 # thread fills 65536 (4 bytes) or 32768 (8 bytes) rows, and the staging holds 32766 or 16383 runs.
 @pytest.mark.parametrize("runs", ["one", "last", "edges", "even", "most", "many"])
-@pytest.mark.parametrize("n", [(3 << 19) - 1, 3 << 19, (3 << 19) + 4097, 2222222])
+@pytest.mark.parametrize("n", [(3 << 19) - 1, 3 << 19, (3 << 19) + 4097, (1 << 21) - 1, 1 << 21, 2222222])
 def test_first_columns_of_long_runs(runs, n):
     starts = {"one": [0], "last": [0, n - 1], "edges": [x + d for x in (0, 512, 4096, 32768, 65536, 131072, n - 4096) for d in (-1, 0, 1) if 0 <= x + d < n],
               "even": np.arange(0, n, 1000), "most": np.linspace(0, n - 1, 1 << 14).astype(np.int64), "many": np.arange(0, n, 9)}[runs]

@@ -26,7 +26,7 @@ constexpr uint64_t RUNS_TILE = 4096;                     // rows a block looks a
 constexpr uint64_t RUNS_MIN_BYTES = 6ull << 20;          // below, the 60 us until the runs are there and 11 us a thread are hardly made up for (4 MB: 73 us of bus)
 constexpr uint64_t RUNS_THREAD_BYTES = 3ull << 19;       // of the column, per thread
 constexpr unsigned RUNS_THREADS_MAX = 4, RUNS_CORES_MIN = 4;
-constexpr uint64_t RUNS_ROWS_MIN = 64;                   // rows a run has to have on average: a run is a few dozen ns of its own
+constexpr uint64_t RUNS_ROWS_MIN = 128;                  // rows a run has to have on average: a run is a few dozen ns of its own (16 384 runs: of 96 rows 244 us copied, 274 to 296 as runs; of 128 317, 277 to 328; of 146 360, 296 to 354)
 
 template <class T>
 __device__ __forceinline__ unsigned warp_heads(const T* __restrict__ col, uint64_t n, uint64_t base, int k) {
