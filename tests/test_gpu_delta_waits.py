@@ -59,6 +59,23 @@ def test_a_wait_that_runs_out_falls_back(name, plan, rels, out, monkeypatch):
     assert (stats["iterations"], stats["candidate_tuples"]) == (fast["iterations"], fast["candidate_tuples"])
 
 
+# No wait of any block is given a second look: of some 2000, all would have to be over at the first for the kernel to finish
+@pytest.mark.parametrize("name,plan,rels,out", [
+    ("same generation", programs.same_generation(), {"edge": list(workloads.tree_dag(1200, 0.05)[:2])}, "sg"),
+    ("same generation of 13 bits", programs.same_generation(), {"edge": list(workloads.tree_dag(5000, 0.05)[:2])}, "sg"),
+    ("points-to", programs.andersen(), {k: list(v) for k, v in workloads.andersen_program(0.0002, 11).items()}, "pt"),
+    ("points-to of 12 bits", programs.andersen(), {k: list(v) for k, v in workloads.andersen_program(0.001, 11).items()}, "pt"),
+    ("ladder", two_rules(), hub_ladder(50, 1, 3, 4), "p"),
+], ids=lambda x: x if isinstance(x, str) else "")
+def test_a_wait_that_is_not_over_falls_back(name, plan, rels, out, monkeypatch):
+    by_kernel, fast = run(monkeypatch, plan, rels, out)
+    got, stats = run(monkeypatch, plan, rels, out, polls=0)
+    for g, b in zip(got, by_kernel):
+        assert np.array_equal(g, b)
+    assert stats["kernel_launches"] > fast["kernel_launches"] + 10  # iteration by iteration
+    assert (stats["iterations"], stats["candidate_tuples"]) == (fast["iterations"], fast["candidate_tuples"])
+
+
 @pytest.mark.parametrize("name,plan,rels,out", [
     ("same generation", programs.same_generation(), {"edge": list(workloads.tree_dag(1200, 0.05)[:2])}, "sg"),
     ("points-to", programs.andersen(), {k: list(v) for k, v in workloads.andersen_program(0.0002, 11).items()}, "pt"),

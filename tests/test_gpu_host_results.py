@@ -1,11 +1,13 @@
 """Results fetched into staged and into page-locked memory: sizes around the limit of the staging
 buffer, columns of every width, results that outlive their context, blocks used again."""
 import gc
+import threading
 
 import numpy as np
 import pytest
 
 from xlog_b200 import _abi as A
+from xlog_b200 import programs
 from xlog_b200.executor import run_program
 from xlog_b200.plan import CompiledRule, ExecutionPlan, Scan, Scc
 from xlog_b200.provider import KernelProvider
@@ -96,6 +98,48 @@ def test_first_columns_of_wide_results(dtype):
     for g, w in zip(got["h"], (first, second)):
         assert np.array_equal(g, w)
     p.close()
+
+
+def cycle_of_blocks(ids, blocks):
+    """Every value of a block leads to every one of the next: the closure is all pairs."""
+    b = np.array_split(ids, blocks)
+    return [np.concatenate([np.repeat(x, len(y)) for x, y in zip(b, b[1:] + b[:1])]), np.concatenate([np.tile(y, len(x)) for x, y in zip(b, b[1:] + b[:1])])]
+
+
+def test_first_columns_of_decoded_ranks():
+    # ids of 30 bits, which a plan runs over as ranks: the result's first values are as many as there are ranks
+    rng = np.random.default_rng(3)
+    ids = np.sort(rng.choice(1 << 30, 1400, replace=False)).astype(np.uint32)
+    p = KernelProvider(device=0)
+    got, _ = run_program(p, programs.transitive_closure(), {"edge": cycle_of_blocks(ids, 10)}, ["reach"])
+    assert 4 * len(got["reach"][0]) >= 6 << 20
+    assert np.array_equal(got["reach"][0], np.repeat(ids, len(ids))) and np.array_equal(got["reach"][1], np.tile(ids, len(ids)))
+    p.close()
+
+
+def test_two_contexts_fetch_at_once():
+    n, wrong = 2_200_000, []
+
+    def work(seed):
+        try:
+            p = KernelProvider(device=0)
+            cols = [np.repeat(np.arange(n // 1000, dtype=np.uint32) * np.uint32(3 + seed), 1000), np.arange(n, dtype=np.uint32) * np.uint32(7)]
+            rel = p.dedup(p.create_buffer_from_slices([c[::-1] for c in cols]))
+            assert rel.is_canonical()
+            cols[1] = cols[1].reshape(-1, 1000)
+            cols[1] = np.sort(cols[1], axis=1).reshape(-1)
+            for _ in range(25):
+                expect(p, rel, cols)
+            p.close()
+        except BaseException as e:  # noqa: BLE001
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
 
 
 @pytest.mark.parametrize("offset", [None, 0, 4, 36])

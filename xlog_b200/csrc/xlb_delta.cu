@@ -736,9 +736,9 @@ __device__ __forceinline__ bool wait_for(const Out& o, const unsigned* word, uns
     for (unsigned polls = 0;; ++polls) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
         if ((int)(v - want) >= 0) return true;
-        if (polls > o.spin_limit) {
+        if (polls >= o.spin_limit) {
             const unsigned now = going_on(o.ctl);
-            if (now != seen) {
+            if (now != seen && o.spin_limit) {  // (a limit of 0: what is not over when it is first looked at has run out)
                 seen = now;
                 polls = 0;
                 continue;
