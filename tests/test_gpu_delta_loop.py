@@ -117,6 +117,24 @@ def test_dense_closures(nodes, degree, monkeypatch):
     both(programs.transitive_closure(), {"edge": dense}, "reach", monkeypatch)
 
 
+# Dense, with rows that are done at once (no successor, or the last of a band) beside rows that are not
+@pytest.mark.parametrize("kind", ["band", "skewed", "bipartite", "bipartite and back"])
+@pytest.mark.parametrize("nodes,degree", [(128, 70), (600, 40), (2000, 70)])
+def test_dense_closures_of_uneven_rows(kind, nodes, degree, monkeypatch):
+    rng = np.random.default_rng(nodes)
+    n = nodes * degree
+    if kind == "band":
+        u = rng.integers(0, nodes, n)
+        v = np.minimum(u + rng.integers(1, 40, n), nodes - 1)
+    elif kind == "skewed":
+        u, v = (np.minimum((rng.random(n) ** 6 * nodes).astype(int), nodes - 1) for _ in range(2))
+    else:
+        u, v = rng.integers(0, nodes // 20 + 1, n), rng.integers(nodes // 20 + 1, nodes, n)
+        if kind != "bipartite":
+            u, v = np.append(u, rng.integers(0, nodes, 50)), np.append(v, rng.integers(0, nodes, 50))
+    both(programs.transitive_closure(), {"edge": [np.append(u, 0).astype(np.uint32), np.append(v, nodes - 1).astype(np.uint32)]}, "reach", monkeypatch)
+
+
 def test_many_long_rows(monkeypatch):
     # 70 sources with 1100 matches each twice over: the list of long rows is used by many warps at once
     src = np.repeat(np.arange(70, dtype=np.uint32), 1100)

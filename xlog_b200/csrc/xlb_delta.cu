@@ -1033,6 +1033,7 @@ constexpr int RW_UNROLL = 4;
 constexpr int RW_BITS_MIN = 5, RW_BITS_MAX = 16;  // of the second column: a row is whole words, a value 16 bits
 constexpr unsigned RW_QUEUE = 16384;              // values the frontier of a row may hold (and the row's seeds)
 constexpr unsigned RW_LONG = 16384;               // candidates of a warp (some 50 us) from which a row may be given up
+constexpr unsigned RW_UNITED = 4;                 // words of rows of bits that take as long as a candidate (counted by their candidates, rows were given up long before they took long: band of 2000 nodes of degree 66 876 us, now 280; by matches 732)
 constexpr unsigned RW_LIST = 64;                  // a value with so many matches is a warp's work by itself
 constexpr unsigned RW_FOLLOW = 32, RW_PATH = 96;  // levels of one value each after which a row is taken for a path, and entries of the table for each
 constexpr int RW_LISTS_BITS = 11;                 // values whose matches are taken as rows of bits: at most 64 words
@@ -1421,7 +1422,8 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const __grid_constant__ O
             unsigned head = 0, end = v->tail;
             __syncthreads();  // (read by all before a warp adds to it)
             bool ok = tried && end <= sh.queue;
-            uint64_t level = 0, cand = 0, looked = RW_LONG;
+            uint64_t level = 0, cand = 0;
+            int patience = RW_LONG;  // candidates (or what takes as long) until it is asked whether the others are done
             const unsigned least = max(RW_FOLLOW, sh.queue / RW_PATH);
             unsigned path = least;  // levels of one value each after which the row is taken for a path
             while (ok && head != end && level < max_iterations) {
@@ -1452,12 +1454,20 @@ __global__ void __launch_bounds__(W * 32) delta_rows_k(const __grid_constant__ O
                     if (sh.lists) {
                         uint32_t start = 0, len = 0;
                         if (on) find(rules.r[0].ix[0], y, start, len);
-                        cand += __reduce_add_sync(FULL, len);
-                        w.unite(sh.lists, sh.rows, sh.words, at, min(per, end - at));
+                        const unsigned all = __reduce_add_sync(FULL, len), m = min(per, end - at);
+                        cand += all;
+                        if (all) {
+                            patience -= (int)(m * sh.words / RW_UNITED);
+                            w.unite(sh.lists, sh.rows, sh.words, at, m);
+                        }
                     } else
-                        for (int q = 0; q < rules.n; ++q) cand += w.expand(o, rules.r[q].ix[0], on, y);
-                    if (cand > looked) {
-                        looked = cand + 4096;
+                        for (int q = 0; q < rules.n; ++q) {
+                            const uint32_t all = w.expand(o, rules.r[q].ix[0], on, y);
+                            cand += all;
+                            patience -= (int)min(all, 1u << 20);
+                        }
+                    if (patience < 0) {
+                        patience = 4096;
                         if (lane == 0 && *(volatile unsigned*)&ctl->rows_idle * 4ull > gridDim.x * 3ull) s.failed = 1;
                     }
                     if (__any_sync(FULL, v->failed)) break;
