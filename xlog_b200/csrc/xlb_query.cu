@@ -4,6 +4,7 @@
 
 #include "xlb_kernels.cuh"
 #include "xlb_ops.h"
+#include "xlb_place.h"
 
 using namespace xk;
 
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(BLOCK) select_rows_k(Cols cols, const unsigned
 // for 1592 and 691; the sort alone 768 and 673; keys of at most 64 rows 330.  The sample costs some 3 us of 200,
 // so smaller build sides go without: 32 768 rows all of one key 122 us sampled, 157 counted.)
 constexpr unsigned JOIN_GROUP_MAX = 64;
+static_assert(JOIN_GROUP_MAX <= 1u << PLACE_NUMBER_BITS, "a row's number in its group");
 constexpr uint64_t JOIN_CHAIN_OUTPUTS = 8;  // outputs a build row, and rows of the longest group, up to which they
 constexpr unsigned JOIN_CHAIN_ROWS = 16;    // go out from the chains
 constexpr uint64_t JOIN_CHAIN_NEAR = 1ull << 18, JOIN_CHAIN_FAR = 52;  // above so many build rows, outputs a build row times rows of the longest group (1 M rows by chains / lists: groups of 16 two outputs 162 / 214, four 253 / 244, eight 373 / 298; groups of 12 four 161 / 234, eight 290 / 290; 131 072 rows, groups of 16, eight 85 / 116)
@@ -197,7 +199,7 @@ __device__ __forceinline__ ulonglong2 cas16(ulonglong2* at, ulonglong2 want, ulo
 // exchange in a loop for them, too, took 1 ms on 32 768 rows of one key, against 157 us).  place: what the lists need.
 // Bound by atomics whose answer is waited for, some 50 G/s on a table of 64 MB: 2 M rows 60 us (an atomic each for key,
 // count and link 71; four rows a thread under way together 60 as well).
-__global__ void __launch_bounds__(BLOCK) group_chain_k(KeyCols keys, uint64_t n, ulonglong2* __restrict__ slots, uint64_t mask, uint32_t* __restrict__ before, uint2* __restrict__ place,
+__global__ void __launch_bounds__(BLOCK) group_chain_k(KeyCols keys, uint64_t n, ulonglong2* __restrict__ slots, uint64_t mask, uint32_t* __restrict__ before, uint64_t* __restrict__ place,
                                                       volatile unsigned int* too_long, DevStatus* st) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
         const unsigned stop = *too_long;
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(BLOCK) group_chain_k(KeyCols keys, uint64_t n,
             h = (h + 1) & mask;
         }
         before[i] = link;
-        place[i] = make_uint2((unsigned)h, number);
+        place[i] = place_of(h, number);
     }
 }
 // Lists, for joins whose rows go out often or whose groups are long: a slot's entry becomes start << 32 | rows, and
@@ -259,10 +261,10 @@ __global__ void __launch_bounds__(BLOCK) group_start_k(ulonglong2* __restrict__ 
         at += len[k];
     }
 }
-__global__ void __launch_bounds__(BLOCK) group_fill_k(const uint2* __restrict__ place, uint64_t n, const ulonglong2* __restrict__ slots, uint32_t* __restrict__ rows) {
+__global__ void __launch_bounds__(BLOCK) group_fill_k(const uint64_t* __restrict__ place, uint64_t n, const ulonglong2* __restrict__ slots, uint32_t* __restrict__ rows) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n; i += (uint64_t)gridDim.x * BLOCK) {
-        const uint2 p = place[i];
-        rows[(uint32_t)(slots[p.x].y >> 32) + p.y] = (uint32_t)i;
+        const uint64_t p = place[i];
+        rows[(uint32_t)(slots[place_slot(p)].y >> 32) + place_number(p)] = (uint32_t)i;
     }
 }
 // Four slots a thread at a time: a slot is a chain of loads (60 us one at a time for 4 M slots, against 50).
@@ -1180,7 +1182,7 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
         check_launch(c, "group_clear");
     }
     prof_begin(c, "hash_insert", n * 8ull);
-    group_chain_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, slots, cap - 1, before->as<uint32_t>(), place->as<uint2>(), too_long, c->d_status);
+    group_chain_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(build, n, slots, cap - 1, before->as<uint32_t>(), place->as<uint64_t>(), too_long, c->d_status);
     check_launch(c, "hash_insert");
     Buf match = make_buf(c, l->rows * 8), in_tile = make_buf(c, l->rows * 4), offs = make_buf(c, tiles * 8);
     Sweep sweep(c, tiles, words + 4, offs->as<uint64_t>(), words);
@@ -1209,7 +1211,7 @@ xlb_rel* query_join(xlb_ctx* c, const xlb_rel* l, const xlb_rel* r, const uint32
             group_start_k<<<(unsigned)((cap + SCAN_TILE) / SCAN_TILE), BLOCK, 0, c->stream>>>(slots, cap + 1, rows->as<uint32_t>() + n, (unsigned int*)(words + 3));
             check_launch(c, "group_start");
             prof_begin(c, "group_fill", n * 16ull);
-            group_fill_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(place->as<uint2>(), n, slots, rows->as<uint32_t>());
+            group_fill_k<<<grid_for(c, n), BLOCK, 0, c->stream>>>(place->as<uint64_t>(), n, slots, rows->as<uint32_t>());
             check_launch(c, "group_fill");
             prof_begin(c, "group_order", cap * 16ull);
             group_order_k<<<grid_for(c, cap + 1), BLOCK, 0, c->stream>>>(slots, cap + 1, rows->as<uint32_t>());
