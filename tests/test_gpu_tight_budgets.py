@@ -2,7 +2,10 @@
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from xlog_b200 import _abi as A
+from xlog_b200 import programs, workloads
+from xlog_b200.executor import run_program
 from xlog_b200.provider import KernelProvider
 
 pytestmark = pytest.mark.gpu
@@ -81,3 +84,20 @@ def test_small_results_keep_what_they_need(rows):
     out = p.groupby_multi_agg(g, [0], [(1, A.AGG_SUM)])
     assert out.num_rows() == max(rows, 1) and 0 <= p.memory_stats()[0] - before - own - 12 * out.num_rows() <= 2 * REST
     p.close()
+
+
+def test_rules_by_rows_without_a_log():
+    # values of 9 bits: a bitmap of 32 KB, where a log of all there could be takes 2 MB
+    rels = {k: list(v) for k, v in workloads.andersen_program(0.0001, 5).items()}
+    want, _ = O.run_program(programs.andersen(), rels, ["pt"])
+    assert max(int(c.max()) for c in want["pt"]) < 512
+    launches = []
+    for budget in (1 << 30, 1536 << 10):
+        p = KernelProvider(device=0, memory_budget_bytes=budget)
+        got, stats = run_program(p, programs.andersen(), rels, ["pt"])
+        launches.append(stats["kernel_launches"])
+        assert p.memory_stats()[1] < 1536 << 10
+        p.close()
+        for g, w in zip(got["pt"], want["pt"]):
+            assert np.array_equal(g, w)
+    assert launches[0] == launches[1] < 40  # (iteration by iteration several hundred)

@@ -967,7 +967,7 @@ __device__ __forceinline__ void ready(Ctl* ctl, bool square) {
     c->fix = n == 0 ? 1 : 0;
     c->phase = n == 0 ? PH_DONE : square ? PH_FULL : PH_ROWS;  // (never solo: a block that starts late would miss it)
 }
-// Rows of a bag into the head: new ones (their bit was clear) are appended to the log.
+// Rows of a bag into the head: new ones (their bit was clear) are appended to the log, where there is one.
 __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict__ rows, uint64_t n, const __grid_constant__ Out o, bool square) {
     __shared__ uint64_t stage_s[BLOCK / 32][64];
     uint64_t* stage = stage_s[threadIdx.x >> 5];
@@ -985,6 +985,7 @@ __global__ void __launch_bounds__(BLOCK) delta_seed_k(const uint64_t* __restrict
         const unsigned bit = 1u << (at & 31);
         on = on && !(o.visited[at >> 5] & bit) && !(atomicOr(&o.visited[at >> 5], bit) & bit);
         if (on && o.visited_t) mark_transposed(o, k);
+        if (!o.log) continue;
         const unsigned b = __ballot_sync(FULL, on);
         if (on) stage[staged + __popc(b & lanemask_lt())] = k;
         staged += __popc(b);
@@ -2275,7 +2276,7 @@ static void log_room(xlb_ctx* c, DeltaLoop& d, uint64_t more) {
 
 void ops_delta_seed(xlb_ctx* c, DeltaLoop& d, const Keys& bag) {
     if (!bag.n) return;
-    log_room(c, d, bag.n);
+    if (d.logged) log_room(c, d, bag.n);
     prof_begin(c, "dense_mark", bag.n * 16ull);
     delta_seed_k<<<grid_for(c, bag.n), BLOCK, 0, c->stream>>>(bag.ptr(), bag.n, out_of(c, d), d.square);
     d.seeded = true;

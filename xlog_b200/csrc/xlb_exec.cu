@@ -2027,6 +2027,7 @@ static bool delta_loop(xlb_ctx* c, const DeltaPlan& plan, const std::vector<Flat
         }
         by_rows = by_rows && ops_delta_by_rows_pays(c, lb, delta_seeds(c, plan, lb), wide);
         DeltaLoop d = ops_delta_begin(c, hb, lb, square && !by_rows, composed);
+        d.logged = !by_rows;
         if (from_store) {
             PhaseTimer t(c, &rs.st.ms_join);
             ops_delta_append(c, d, delta);

@@ -230,6 +230,7 @@ struct DeltaLoop {
     uint64_t cap = 0, room = 0;  // tuples the log can hold; that may be in it
     void* ctl = nullptr;    // behind the bitmaps
     bool seeded = false;
+    bool logged = true;     // (set before any seed) rules that run by rows of the head need no log, 512 MB of a large budget
     bool seeds_listed = false;  // the seeds are the rows of the one relation that the one rule joins with, by its first column
 };
 struct DeltaResult {
