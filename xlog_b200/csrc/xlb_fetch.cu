@@ -145,8 +145,8 @@ bool fetch_with_runs(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t n
     {
         Filler<T> filler(threads);
         stream_wait(c);
-        if (*total > cap) xlb_fail(XLB_ERR_CUDA, "internal: %llu runs of at most %llu values", *total, (unsigned long long)r->firsts);
-        filler.fill(static_cast<T*>(cols[0]), runs, *total, n);
+        if (*total <= cap) filler.fill(static_cast<T*>(cols[0]), runs, *total, n);
+        else side->add(cols[0], col, n * sizeof(T));  // (more values than were announced)
     }
     side->wait();
     return true;
