@@ -24,7 +24,6 @@ namespace {
 
 constexpr uint64_t RUNS_TILE = 4096;                     // rows a block looks at, 512 a warp
 constexpr uint64_t RUNS_MIN_BYTES = 6ull << 20;          // below, the 60 us until the runs are there and 11 us a thread are hardly made up for (4 MB: 73 us of bus)
-constexpr uint64_t RUNS_THREAD_BYTES = 3ull << 19;       // of the column, per thread
 constexpr unsigned RUNS_THREADS_MAX = 4, RUNS_CORES_MIN = 4;
 constexpr uint64_t RUNS_ROWS_MIN = 128;                  // rows a run has to have on average: a run is a few dozen ns of its own (16 384 runs: of 96 rows 244 us copied, 274 to 296 as runs; of 128 317, 277 to 328; of 146 360, 296 to 354)
 
@@ -166,7 +165,7 @@ void ops_fetch_columns(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t
         const unsigned cores = host_pool_cores();
         bool locked = cores >= RUNS_CORES_MIN;
         for (uint32_t i = 0; i < arity; ++i) locked = locked && page_locked(cols[i]) && (uintptr_t)cols[i] % width == 0;
-        const unsigned threads = (unsigned)std::min<uint64_t>({RUNS_THREADS_MAX, cores / 2, n * width / RUNS_THREAD_BYTES});
+        const unsigned threads = std::min(RUNS_THREADS_MAX, cores / 2);  // (two or more)
         if (locked && (width == 4 ? fetch_with_runs<uint32_t>(c, r, cols, n, threads) : fetch_with_runs<unsigned long long>(c, r, cols, n, threads))) return;
     }
     for (uint32_t i = 0; i < arity; ++i) CUDA_OK(copy_async(c, cols[i], r->cols[i]->p, n * type_width(r->schema.types[i]), cudaMemcpyDeviceToHost));
