@@ -204,3 +204,19 @@ def test_joins_of_many_rows_from_chains_and_from_lists(p, group, ratio):
     l, r = inner(ask, key)
     for g, w in zip(p.download(p.hash_join_v2(p.create_buffer_from_slices(left), p.create_buffer_from_slices(right), [0], [1])), [c[l] for c in left] + [c[r] for c in right]):
         assert np.array_equal(g, w)
+
+
+# Rows of a key next to each other in the build side: a warp's lanes claim one slot, count and link on it at once
+@pytest.mark.parametrize("group", [2, 3, 8, 15, 16, 17, 31, 32, 64])
+@pytest.mark.parametrize("apart", [1, 32, 256, 5000])
+def test_rows_of_one_key_side_by_side(p, group, apart):
+    n = 60_000
+    i = np.arange(n, dtype=np.uint64)
+    key = (i // np.uint64(apart * group) * np.uint64(apart) + i % np.uint64(apart)) * np.uint64(3)  # (`group` rows each, `apart` rows from one to the next)
+    rng = np.random.default_rng(group)
+    left, right = [rng.integers(0, int(key.max()) + 1, 9000, dtype=np.uint64), np.arange(9000, dtype=np.uint32)], [i.astype(np.uint32), key]
+    l, r = inner(left[0], key)
+    lb, rb = p.create_buffer_from_slices(left), p.create_buffer_from_slices(right)
+    for _ in range(5):
+        for g, w in zip(p.download(p.hash_join_v2(lb, rb, [0], [1])), [c[l] for c in left] + [c[r] for c in right]):
+            assert np.array_equal(g, w)

@@ -197,6 +197,11 @@ __device__ __forceinline__ ulonglong2 cas16(ulonglong2* at, ulonglong2 want, ulo
 }
 // The first row of a key brings key, count and link by one exchange, the others count and link by one each (an
 // exchange in a loop for them, too, took 1 ms on 32 768 rows of one key, against 157 us).  place: what the lists need.
+// A slot is met by accesses of three sizes: the exchange of 16 bytes, the look at its key, and the additions and
+// exchanges on the halves of its entry.  The PTX memory model promises nothing for overlapping accesses of different
+// sizes, so this rests on the hardware: atomics, and volatile loads, of one sector are served one by one at the L2, and
+// a row adds to an entry only after its look, or its exchange, has brought the key back.  (Within the model: a
+// key claimed by 8 bytes and an atomic each for count and link, 71 us for the 60 below.)
 // Bound by atomics whose answer is waited for, some 50 G/s on a table of 64 MB: 2 M rows 60 us (an atomic each for key,
 // count and link 71; four rows a thread under way together 60 as well).
 __global__ void __launch_bounds__(BLOCK) group_chain_k(KeyCols keys, uint64_t n, ulonglong2* __restrict__ slots, uint64_t mask, uint32_t* __restrict__ before, uint64_t* __restrict__ place,
