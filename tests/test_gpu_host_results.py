@@ -1,6 +1,8 @@
 """Results fetched into staged and into page-locked memory: sizes around the limit of the staging
 buffer, columns of every width, results that outlive their context, blocks used again."""
 import gc
+import glob
+import os
 import threading
 
 import numpy as np
@@ -54,6 +56,19 @@ def expect(p, rel, cols):
         assert np.array_equal(g, c)
 
 
+CORES = min([len(os.sched_getaffinity(0))] + [int(q[0]) // int(q[1]) for q in [open(f).read().split() for f in glob.glob("/sys/fs/cgroup/cpu.max")] if q[0] != "max"])
+
+
+def went_as_runs(p, fetch):
+    """Whether `fetch` brought a first column as runs: two kernels, of which plain copies have none."""
+    p.profile_enable("to_host")
+    fetch()
+    launches = p.profile_read().get("to_host", {"launches": 0})["launches"]
+    p.profile_enable(None)
+    assert launches in (0, 2)
+    return launches == 2
+
+
 def rows_from(starts, n):
     starts = np.unique(starts)
     return np.diff(np.append(starts, n))
@@ -71,8 +86,8 @@ def test_first_columns_of_long_runs(runs, n):
     p = KernelProvider(device=0)
     rel = p.dedup(p.create_buffer_from_slices([c[::-1] for c in cols]))
     assert rel.is_canonical()
-    expect(p, rel, cols)
-    expect(p, p.create_buffer_from_slices(cols), cols)
+    assert went_as_runs(p, lambda: expect(p, rel, cols)) == (CORES >= 4 and n >= 3 << 19 and 1 << len(bin(int(first[-1]))) - 2 <= n // 128)
+    assert not went_as_runs(p, lambda: expect(p, p.create_buffer_from_slices(cols), cols))  # (not known to be in order)
     p.close()
 
 
@@ -93,8 +108,10 @@ def test_first_columns_of_wide_results(dtype):
     plan = ExecutionPlan([Scc(0, False, [CompiledRule("h", Scan(0), (code, code))])], {"s": 0, "h": 1})
     order = rng.permutation(len(first))
     p = KernelProvider(device=0)
-    got, _ = run_program(p, plan, {"s": [first[order], second[order]]}, ["h"])
+    res = []
+    assert went_as_runs(p, lambda: res.append(run_program(p, plan, {"s": [first[order], second[order]]}, ["h"])[0])) == (CORES >= 4)
     assert len(first) * first.itemsize >= 6 << 20
+    got = res[0]
     for g, w in zip(got["h"], (first, second)):
         assert np.array_equal(g, w)
     p.close()
@@ -111,7 +128,9 @@ def test_first_columns_of_decoded_ranks():
     rng = np.random.default_rng(3)
     ids = np.sort(rng.choice(1 << 30, 1400, replace=False)).astype(np.uint32)
     p = KernelProvider(device=0)
-    got, _ = run_program(p, programs.transitive_closure(), {"edge": cycle_of_blocks(ids, 10)}, ["reach"])
+    res = []
+    assert went_as_runs(p, lambda: res.append(run_program(p, programs.transitive_closure(), {"edge": cycle_of_blocks(ids, 10)}, ["reach"])[0])) == (CORES >= 4)
+    got = res[0]
     assert 4 * len(got["reach"][0]) >= 6 << 20
     assert np.array_equal(got["reach"][0], np.repeat(ids, len(ids))) and np.array_equal(got["reach"][1], np.tile(ids, len(ids)))
     p.close()
@@ -164,7 +183,8 @@ def test_long_runs_into_memory_of_the_callers(offset):
             at = offset // 4
             out = [all_of_it[at:at + m], all_of_it[at + m + 1:at + 2 * m + 1]]
         rows = C.c_uint64()
-        p._check(p._lib.xlb_rel_to_host(p._ctx, buf._h, (C.c_void_p * 2)(*[o.ctypes.data for o in out]), m, C.byref(rows)))
+        fetch = lambda: p._check(p._lib.xlb_rel_to_host(p._ctx, buf._h, (C.c_void_p * 2)(*[o.ctypes.data for o in out]), m, C.byref(rows)))  # noqa: E731, B023
+        assert went_as_runs(p, fetch) == (offset is not None and CORES >= 4)
         assert rows.value == total and np.array_equal(out[0], first[:m]) and np.array_equal(out[1], second[:m])
         if offset is not None:
             assert np.all(all_of_it[:at] == 0xABABABAB) and all_of_it[at + m] == 0xABABABAB and np.all(all_of_it[at + 2 * m + 1:] == 0xABABABAB)
