@@ -86,7 +86,7 @@ def test_first_columns_of_long_runs(runs, n):
     p = KernelProvider(device=0)
     rel = p.dedup(p.create_buffer_from_slices([c[::-1] for c in cols]))
     assert rel.is_canonical()
-    assert went_as_runs(p, lambda: expect(p, rel, cols)) == (CORES >= 4 and n >= 3 << 19 and 1 << len(bin(int(first[-1]))) - 2 <= n // 128)
+    assert went_as_runs(p, lambda: expect(p, rel, cols)) == (CORES >= 4 and n >= 3 << 19 and 400 << len(bin(int(first[-1]))) - 2 <= 4 * n)
     assert not went_as_runs(p, lambda: expect(p, p.create_buffer_from_slices(cols), cols))  # (not known to be in order)
     p.close()
 
@@ -113,6 +113,21 @@ def test_first_columns_of_wide_results(dtype):
     assert len(first) * first.itemsize >= 6 << 20
     got = res[0]
     for g, w in zip(got["h"], (first, second)):
+        assert np.array_equal(g, w)
+    p.close()
+
+
+# 4-byte runs are worth their while from 100 rows on, 8-byte ones from 50
+@pytest.mark.parametrize("dtype,runs,rows", [(np.uint32, 16384, 99), (np.uint32, 16384, 100), (np.uint64, 16000, 50), (np.uint64, 8000, 99)])
+def test_short_runs(dtype, runs, rows):
+    ids = np.arange(runs, dtype=dtype) * dtype(1 if dtype == np.uint32 else 1 << 33)
+    first, second = np.repeat(ids, rows), np.tile(ids[:rows], runs)
+    code = A.U32 if dtype == np.uint32 else A.U64
+    plan = ExecutionPlan([Scc(0, False, [CompiledRule("h", Scan(0), (code, code))])], {"s": 0, "h": 1})
+    p = KernelProvider(device=0)
+    res = []
+    assert went_as_runs(p, lambda: res.append(run_program(p, plan, {"s": [first, second]}, ["h"])[0])) == (CORES >= 4 and rows * first.itemsize >= 400)
+    for g, w in zip(res[0]["h"], (first, second)):
         assert np.array_equal(g, w)
     p.close()
 

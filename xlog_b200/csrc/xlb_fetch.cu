@@ -25,7 +25,7 @@ namespace {
 constexpr uint64_t RUNS_TILE = 4096;                     // rows a block looks at, 512 a warp
 constexpr uint64_t RUNS_MIN_BYTES = 6ull << 20;          // below, the 60 us until the runs are there and 11 us a thread are hardly made up for (4 MB: 73 us of bus)
 constexpr unsigned RUNS_THREADS_MAX = 4, RUNS_CORES_MIN = 4;
-constexpr uint64_t RUNS_ROWS_MIN = 128;                  // rows a run has to have on average: a run is a few dozen ns of its own (16 384 runs: of 96 rows 244 us copied, 274 to 296 as runs; of 128 317, 277 to 328; of 146 360, 296 to 354)
+constexpr uint64_t RUNS_RUN_BYTES = 400;                 // a run has to have on average: it is 10 to 15 ns of its own, whatever its rows' width (16 384 runs of 4-byte rows: of 96 rows 244 us copied, 249 to 269 as runs; of 104 263, 237; of 112 281, 233; of 128 318, 255; 16 000 of 8-byte rows: of 50 rows 460, 315; of 80 526, 315)
 
 template <class T>
 __device__ __forceinline__ unsigned warp_heads(const T* __restrict__ col, uint64_t n, uint64_t base, int k) {
@@ -160,7 +160,7 @@ void ops_fetch_columns(xlb_ctx* c, const xlb_rel* r, void* const* cols, uint64_t
     // 11 us of a sort's 1500 and 15 of 790 of a union over 2^18 first values); not with several ranks (whose waits watch the
     // communicator), and not into memory that the driver copies to by itself: such a copy does not run beside anything.
     const uint64_t bound = rel_packable(r->schema) && r->or_bound != ~0ull ? (r->or_bound >> 32) + 1 : ~0ull, firsts = std::min(bound, r->firsts);
-    if (r->canonical && arity >= 2 && firsts <= std::min(n / RUNS_ROWS_MIN, width == 4 ? runs_room<uint32_t>() : runs_room<unsigned long long>()) && width >= 4 && n * width >= RUNS_MIN_BYTES &&
+    if (r->canonical && arity >= 2 && firsts <= std::min(n * width / RUNS_RUN_BYTES, width == 4 ? runs_room<uint32_t>() : runs_room<unsigned long long>()) && width >= 4 && n * width >= RUNS_MIN_BYTES &&
         n < 1ull << 32 && !c->wait_hook) {
         const unsigned cores = host_pool_cores();
         bool locked = cores >= RUNS_CORES_MIN;
