@@ -73,6 +73,9 @@ def test_a_wait_that_is_not_over_falls_back(name, plan, rels, out, monkeypatch):
     for g, b in zip(got, by_kernel):
         assert np.array_equal(g, b)
     assert stats["kernel_launches"] > fast["kernel_launches"] + 10  # iteration by iteration
+    if "bits" not in name:  # (the others take the oracle long)
+        for g, w in zip(got, O.run_program(plan, rels, [out])[0][out]):
+            assert np.array_equal(g, w)
     assert (stats["iterations"], stats["candidate_tuples"]) == (fast["iterations"], fast["candidate_tuples"])
 
 

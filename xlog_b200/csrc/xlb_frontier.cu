@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) frontier_many_k(const __grid_con
 // in global memory, past what the head holds and past a small cache of what the block marked
 // lately.  Looked up in the L1 (one line a cycle), the bitmaps and not the stream were what the
 // launch-by-launch loop paid for: 16 M edges took it 190 us in six scans and 350 us in all, and take
-// this kernel 178 us from launch to end.  Of that, by the clock inside it, 19 the seed, 76 the first stream, 21
+// this kernel 178 us from launch to end (160 to 190 from process to process; 4 more with the L2 flushed).  Of that, by the clock inside it, 19 the seed, 76 the first stream, 21
 // the second, 4 each iteration after; the rest is the launch, the barriers and the list written off.  (Looking
 // at what all blocks have marked before sending an atomic evens the blocks out but costs as much.)
 constexpr int FL_BITS = 20, FL_CACHE = 1 << 14, FL_ITERATIONS = 48;
